@@ -6,7 +6,8 @@
 // the chunk places each slot at base + (its rank among the equal ids seen so
 // far), which keeps slots of an expert in ascending order.  The ranks inside a
 // group of 32 slots come from __match_any_sync.
-#include "common.cuh"
+#include "align.cuh"
+#include "pair.cuh"
 
 namespace fmoe {
 namespace {
@@ -14,10 +15,47 @@ namespace {
 constexpr int kThreads = 1024;
 constexpr int kWarps = kThreads / 32;
 
+// One warp: exclusive scan of the padded row counts -> s_start[E + 1] and num_post_pad; with `table`, also the experts'
+// first rows, rows and token tiles for the CTA-pair GEMMs (pair.cuh).  E <= 1024: 32 experts per step.
+__device__ __forceinline__ void scan_experts_warp(const int* s_total, int* s_start, int E, int block, int lane,
+                                                  int32_t* num_post_pad, int32_t* table) {
+  int carry = 0, tile_carry = 0;
+  for (int base = 0; base < E; base += 32) {
+    const int e = base + lane;
+    const int rows = (e < E) ? s_total[e] : 0;
+    const int padded = ceil_div(rows, block) * block, tiles = ceil_div(rows, kPairTokens);
+    int incl = padded, tile_incl = tiles;
+#pragma unroll
+    for (int off = 1; off < 32; off <<= 1) {
+      const int v = __shfl_up_sync(0xffffffffu, incl, off), w = __shfl_up_sync(0xffffffffu, tile_incl, off);
+      if (lane >= off) {
+        incl += v;
+        tile_incl += w;
+      }
+    }
+    if (e < E) {
+      s_start[e] = carry + incl - padded;
+      if (table) {
+        table[e] = carry + incl - padded;
+        table[E + e] = rows;
+        table[2 * E + e] = tile_carry + tile_incl - tiles;
+      }
+    }
+    carry += __shfl_sync(0xffffffffu, incl, 31);
+    tile_carry += __shfl_sync(0xffffffffu, tile_incl, 31);
+  }
+  if (lane == 0) {
+    s_start[E] = carry;
+    num_post_pad[0] = carry;
+    if (table) table[3 * E] = tile_carry;
+  }
+}
+
 __global__ void __launch_bounds__(kThreads)
 moe_align_kernel(const int32_t* __restrict__ topk_ids, int numel, int E, int block,
                  int32_t* __restrict__ sorted_ids, int sorted_cap, int32_t* __restrict__ expert_ids,
-                 int expert_cap, int32_t* __restrict__ num_post_pad) {
+                 int expert_cap, int32_t* __restrict__ num_post_pad, int32_t* __restrict__ table,
+                 int32_t* __restrict__ zero_words, int num_zero) {
   pdl_entry();
   extern __shared__ int s_mem[];
   int* s_cnt = s_mem;                  // [kWarps][E] counts, then running output positions
@@ -27,6 +65,7 @@ moe_align_kernel(const int32_t* __restrict__ topk_ids, int numel, int E, int blo
 
   for (int i = tid; i < kWarps * E; i += kThreads) s_cnt[i] = 0;
   for (int i = tid; i < sorted_cap; i += kThreads) sorted_ids[i] = numel;
+  for (int i = tid; i < num_zero; i += kThreads) zero_words[i] = 0;
   __syncthreads();
 
   const int chunk = ceil_div(ceil_div(numel, kWarps), 32) * 32;  // multiple of 32 per warp
@@ -55,26 +94,7 @@ moe_align_kernel(const int32_t* __restrict__ topk_ids, int numel, int E, int blo
   }
   __syncthreads();
 
-  // padded exclusive scan over experts (E <= 1024: warp 0, 32 experts per step)
-  if (warp == 0) {
-    int carry = 0;
-    for (int base = 0; base < E; base += 32) {
-      int e = base + lane;
-      int padded = (e < E) ? ceil_div(s_total[e], block) * block : 0;
-      int incl = padded;
-#pragma unroll
-      for (int off = 1; off < 32; off <<= 1) {
-        int v = __shfl_up_sync(0xffffffffu, incl, off);
-        if (lane >= off) incl += v;
-      }
-      if (e < E) s_start[e] = carry + incl - padded;
-      carry += __shfl_sync(0xffffffffu, incl, 31);
-    }
-    if (lane == 0) {
-      s_start[E] = carry;
-      num_post_pad[0] = carry;
-    }
-  }
+  if (warp == 0) scan_experts_warp(s_total, s_start, E, block, lane, num_post_pad, table);
   __syncthreads();
 
   // block -> expert map (-1 after the used blocks)
@@ -131,11 +151,13 @@ align_count_kernel(const int32_t* __restrict__ topk_ids, int numel, int E, int32
 
 __global__ void __launch_bounds__(kThreads)
 align_scan_kernel(int chunks, int E, int block, int32_t* __restrict__ cnt, int32_t* __restrict__ expert_ids,
-                  int expert_cap, int32_t* __restrict__ num_post_pad) {
+                  int expert_cap, int32_t* __restrict__ num_post_pad, int32_t* __restrict__ table,
+                  int32_t* __restrict__ zero_words, int num_zero) {
   extern __shared__ int s_mem[];
   int* s_total = s_mem;      // [E]
   int* s_start = s_mem + E;  // [E+1]
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  for (int i = tid; i < num_zero; i += kThreads) zero_words[i] = 0;
   for (int e = tid; e < E; e += kThreads) {
     int run = 0;
     for (int c = 0; c < chunks; ++c) {
@@ -146,25 +168,7 @@ align_scan_kernel(int chunks, int E, int block, int32_t* __restrict__ cnt, int32
     s_total[e] = run;
   }
   __syncthreads();
-  if (warp == 0) {
-    int carry = 0;
-    for (int base = 0; base < E; base += 32) {
-      int e = base + lane;
-      int padded = (e < E) ? ceil_div(s_total[e], block) * block : 0;
-      int incl = padded;
-#pragma unroll
-      for (int off = 1; off < 32; off <<= 1) {
-        int v = __shfl_up_sync(0xffffffffu, incl, off);
-        if (lane >= off) incl += v;
-      }
-      if (e < E) s_start[e] = carry + incl - padded;
-      carry += __shfl_sync(0xffffffffu, incl, 31);
-    }
-    if (lane == 0) {
-      s_start[E] = carry;
-      num_post_pad[0] = carry;
-    }
-  }
+  if (warp == 0) scan_experts_warp(s_total, s_start, E, block, lane, num_post_pad, table);
   __syncthreads();
   const int used_blocks = s_start[E] / block;
   for (int e = tid; e < E; e += kThreads) {
@@ -218,6 +222,54 @@ align_scatter_kernel(const int32_t* __restrict__ topk_ids, int numel, int E, con
 }
 
 }  // namespace
+
+namespace {
+int check_align(const AlignArgs& a) {
+  FMOE_REQUIRE(a.E >= 1 && a.E <= 1024, "moe_align_block_size: need 1 <= E <= 1024 (got %d)", a.E);
+  FMOE_REQUIRE(a.block >= 1, "moe_align_block_size: block must be >= 1 (got %d)", a.block);
+  FMOE_REQUIRE(a.numel >= 0 && a.numel < (1ll << 30), "moe_align_block_size: numel out of range");
+  // worst case: every non-empty expert wastes block-1 positions
+  const int64_t need = a.numel + (a.numel < a.E ? a.numel : (int64_t)a.E) * (a.block - 1);
+  FMOE_REQUIRE(a.sorted_cap >= need, "moe_align_block_size: sorted_token_ids too small (%lld < %lld)",
+               (long long)a.sorted_cap, (long long)need);
+  FMOE_REQUIRE(a.sorted_cap < (1ll << 31), "moe_align_block_size: sorted_cap out of range");
+  FMOE_REQUIRE(a.expert_cap >= ceil_div<int64_t>(a.sorted_cap, a.block),
+               "moe_align_block_size: expert_ids too small (%lld < %lld)", (long long)a.expert_cap,
+               (long long)ceil_div<int64_t>(a.sorted_cap, a.block));
+  FMOE_REQUIRE(a.sorted_ids && a.expert_ids && a.num_post_pad && (a.topk_ids || a.numel == 0),
+               "moe_align_block_size: null pointer");
+  return FMOE_OK;
+}
+}  // namespace
+
+int run_align(const AlignArgs& a, cudaStream_t st) {
+  int rc = check_align(a);
+  if (rc) return rc;
+  if (a.numel < 2 * kChunk || !a.workspace) {  // small inputs, or no scratch: the single-CTA kernel
+    const size_t smem = ((size_t)kWarps * a.E + 2 * (size_t)a.E + 1) * sizeof(int);
+    if (smem > 48 * 1024)
+      FMOE_CUDA_OK(cudaFuncSetAttribute(moe_align_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    launch_pdl(moe_align_kernel, dim3(1), dim3(kThreads), smem, st, a.topk_ids, (int)a.numel, a.E, a.block, a.sorted_ids,
+               (int)a.sorted_cap, a.expert_ids, (int)a.expert_cap, a.num_post_pad, a.table, a.zero_words, a.num_zero);
+    return launch_status("moe_align_kernel");
+  }
+  FMOE_REQUIRE(a.workspace_bytes >= fmoe_moe_align_workspace_bytes(a.numel, a.E), "moe_align_block_size: workspace too small");
+  const int chunks = (int)ceil_div<int64_t>(a.numel, kChunk);
+  int32_t* cnt = static_cast<int32_t*>(a.workspace);
+  align_count_kernel<<<chunks, kThreads, a.E * sizeof(int), st>>>(a.topk_ids, (int)a.numel, a.E, a.sorted_ids, (int)a.sorted_cap, cnt);
+  rc = launch_status("align_count_kernel");
+  if (rc) return rc;
+  align_scan_kernel<<<1, kThreads, (2 * a.E + 1) * sizeof(int), st>>>(chunks, a.E, a.block, cnt, a.expert_ids, (int)a.expert_cap,
+                                                                     a.num_post_pad, a.table, a.zero_words, a.num_zero);
+  rc = launch_status("align_scan_kernel");
+  if (rc) return rc;
+  const size_t smem = (size_t)kWarps * a.E * sizeof(int);
+  if (smem > 48 * 1024)
+    FMOE_CUDA_OK(cudaFuncSetAttribute(align_scatter_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  align_scatter_kernel<<<chunks, kThreads, smem, st>>>(a.topk_ids, (int)a.numel, a.E, cnt, a.sorted_ids, (int)a.sorted_cap);
+  return launch_status("align_scatter_kernel");
+}
+
 }  // namespace fmoe
 
 extern "C" int64_t fmoe_moe_align_workspace_bytes(int64_t numel, int E) {
@@ -228,59 +280,25 @@ extern "C" int fmoe_moe_align_block_size_ws(const int32_t* topk_ids, int64_t num
                                             int32_t* sorted_token_ids, int64_t sorted_cap, int32_t* expert_ids,
                                             int64_t expert_cap, int32_t* num_tokens_post_padded, void* workspace,
                                             int64_t workspace_bytes, void* stream) {
-  using namespace fmoe;
-  // small inputs, or no scratch: the single-CTA kernel
-  if (numel < 2 * kChunk || !workspace)
-    return fmoe_moe_align_block_size(topk_ids, numel, E, block, sorted_token_ids, sorted_cap, expert_ids, expert_cap,
-                                     num_tokens_post_padded, stream);
-  FMOE_REQUIRE(E >= 1 && E <= 1024, "moe_align_block_size: need 1 <= E <= 1024 (got %d)", E);
-  FMOE_REQUIRE(block >= 1, "moe_align_block_size: block must be >= 1 (got %d)", block);
-  FMOE_REQUIRE(numel < (1ll << 30), "moe_align_block_size: numel out of range");
-  const int64_t need = numel + (numel < E ? numel : (int64_t)E) * (block - 1);
-  FMOE_REQUIRE(sorted_cap >= need && sorted_cap < (1ll << 31), "moe_align_block_size: sorted_token_ids too small (%lld < %lld)",
-               (long long)sorted_cap, (long long)need);
-  FMOE_REQUIRE(expert_cap >= ceil_div<int64_t>(sorted_cap, block), "moe_align_block_size: expert_ids too small");
-  FMOE_REQUIRE(sorted_token_ids && expert_ids && num_tokens_post_padded && topk_ids, "moe_align_block_size: null pointer");
-  FMOE_REQUIRE(workspace_bytes >= fmoe_moe_align_workspace_bytes(numel, E), "moe_align_block_size: workspace too small");
-  const int chunks = (int)ceil_div<int64_t>(numel, kChunk);
-  auto st = (cudaStream_t)stream;
-  int32_t* cnt = static_cast<int32_t*>(workspace);
-  align_count_kernel<<<chunks, kThreads, E * sizeof(int), st>>>(topk_ids, (int)numel, E, sorted_token_ids, (int)sorted_cap, cnt);
-  int rc = launch_status("align_count_kernel");
-  if (rc) return rc;
-  align_scan_kernel<<<1, kThreads, (2 * E + 1) * sizeof(int), st>>>(chunks, E, block, cnt, expert_ids, (int)expert_cap,
-                                                                   num_tokens_post_padded);
-  rc = launch_status("align_scan_kernel");
-  if (rc) return rc;
-  size_t smem = (size_t)kWarps * E * sizeof(int);
-  if (smem > 48 * 1024)
-    FMOE_CUDA_OK(cudaFuncSetAttribute(align_scatter_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-  align_scatter_kernel<<<chunks, kThreads, smem, st>>>(topk_ids, (int)numel, E, cnt, sorted_token_ids, (int)sorted_cap);
-  return launch_status("align_scatter_kernel");
+  fmoe::AlignArgs a;
+  a.topk_ids = topk_ids;
+  a.numel = numel;
+  a.E = E;
+  a.block = block;
+  a.sorted_ids = sorted_token_ids;
+  a.sorted_cap = sorted_cap;
+  a.expert_ids = expert_ids;
+  a.expert_cap = expert_cap;
+  a.num_post_pad = num_tokens_post_padded;
+  a.workspace = workspace;
+  a.workspace_bytes = workspace_bytes;
+  return fmoe::run_align(a, (cudaStream_t)stream);
 }
 
 extern "C" int fmoe_moe_align_block_size(const int32_t* topk_ids, int64_t numel, int E, int block,
                                          int32_t* sorted_token_ids, int64_t sorted_cap,
                                          int32_t* expert_ids, int64_t expert_cap,
                                          int32_t* num_tokens_post_padded, void* stream) {
-  using namespace fmoe;
-  FMOE_REQUIRE(E >= 1 && E <= 1024, "moe_align_block_size: need 1 <= E <= 1024 (got %d)", E);
-  FMOE_REQUIRE(block >= 1, "moe_align_block_size: block must be >= 1 (got %d)", block);
-  FMOE_REQUIRE(numel >= 0 && numel < (1ll << 30), "moe_align_block_size: numel out of range");
-  // worst case: every non-empty expert wastes block-1 positions
-  const int64_t need = numel + (numel < E ? numel : (int64_t)E) * (block - 1);
-  FMOE_REQUIRE(sorted_cap >= need, "moe_align_block_size: sorted_token_ids too small (%lld < %lld)",
-               (long long)sorted_cap, (long long)need);
-  FMOE_REQUIRE(sorted_cap < (1ll << 31), "moe_align_block_size: sorted_cap out of range");
-  FMOE_REQUIRE(expert_cap >= ceil_div<int64_t>(sorted_cap, block),
-               "moe_align_block_size: expert_ids too small (%lld < %lld)", (long long)expert_cap,
-               (long long)ceil_div<int64_t>(sorted_cap, block));
-  FMOE_REQUIRE(sorted_token_ids && expert_ids && num_tokens_post_padded && (topk_ids || numel == 0),
-               "moe_align_block_size: null pointer");
-  size_t smem = ((size_t)kWarps * E + 2 * (size_t)E + 1) * sizeof(int);
-  if (smem > 48 * 1024)
-    FMOE_CUDA_OK(cudaFuncSetAttribute(moe_align_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-  launch_pdl(moe_align_kernel, dim3(1), dim3(kThreads), smem, (cudaStream_t)stream, topk_ids, (int)numel, E, block,
-             sorted_token_ids, (int)sorted_cap, expert_ids, (int)expert_cap, num_tokens_post_padded);
-  return launch_status("moe_align_kernel");
+  return fmoe_moe_align_block_size_ws(topk_ids, numel, E, block, sorted_token_ids, sorted_cap, expert_ids, expert_cap,
+                                      num_tokens_post_padded, nullptr, 0, stream);
 }

@@ -1,0 +1,24 @@
+// Internal interface of moe_align (align.cu): the public outputs, and what the one-call layer asks for besides.
+#pragma once
+#include "common.cuh"
+
+namespace fmoe {
+
+struct AlignArgs {
+  const int32_t* topk_ids = nullptr;
+  int64_t numel = 0;
+  int E = 0, block = 0;
+  int32_t* sorted_ids = nullptr;
+  int64_t sorted_cap = 0;
+  int32_t* expert_ids = nullptr;
+  int64_t expert_cap = 0;
+  int32_t* num_post_pad = nullptr;
+  void* workspace = nullptr;  // scratch of the multi-CTA variant (NULL: single CTA)
+  int64_t workspace_bytes = 0;
+  int32_t* table = nullptr;       // optional: expert table of the CTA-pair GEMMs (pair.cuh)
+  int32_t* zero_words = nullptr;  // optional: counters of later kernels, set to zero
+  int num_zero = 0;
+};
+int run_align(const AlignArgs& a, cudaStream_t st);
+
+}  // namespace fmoe

@@ -71,16 +71,23 @@ int dispatch_gemm(const fmoe_gemm_args* args, bool gated, void* stream, const ch
   if (args->struct_size != sizeof(fmoe_gemm_args))
     return fail(FMOE_ERR_INVALID_ARG, "%s: fmoe_gemm_args.struct_size is %u, this library's struct has %zu bytes "
                 "(binding built against another header?)", who, args->struct_size, sizeof(fmoe_gemm_args));
-  const GemmParams& a = *args;
+  GemmParams p;
+  static_cast<fmoe_gemm_args&>(p) = *args;
+  return run_gemm(p, gated, (cudaStream_t)stream);
+}
+
+}  // namespace
+
+int run_gemm(const GemmParams& a, bool gated, cudaStream_t st) {
+  const char* who = gated ? "gemm1_silu" : "gemm2";
   int rc = validate_gemm(a, gated, who);
   if (rc) return rc;
   if (a.max_blocks == 0 || a.numel == 0) return FMOE_OK;
-  auto st = (cudaStream_t)stream;
   int variant = a.variant;
   if (a.w_layout == FMOE_W_N_MAJOR || (a.dtype == FMOE_E4M3 && a.scale_mode == FMOE_SCALE_CHANNEL)) {
     variant = FMOE_VARIANT_TCGEN05;
   } else if (variant == FMOE_VARIANT_AUTO) {
-    if (gemm_tcgen05_supports(a, gated) || gemm_tcgen05_fp8_supports(a, gated))
+    if (gemm_pair_supports(a, gated) || gemm_tcgen05_fp8_supports(a, gated))
       variant = FMOE_VARIANT_TCGEN05;
     else if (gemm_stream_supports(a, gated))
       variant = FMOE_VARIANT_STREAM;
@@ -92,17 +99,16 @@ int dispatch_gemm(const fmoe_gemm_args* args, bool gated, void* stream, const ch
     case FMOE_VARIANT_STREAM: return gemm_stream(a, gated, st);
     case FMOE_VARIANT_TCGEN05:
       return (a.dtype == FMOE_E4M3 && a.scale_mode == FMOE_SCALE_BLOCK128) ? gemm_tcgen05_fp8(a, gated, st)
-                                                                           : gemm_tcgen05(a, gated, st);
+                                                                           : gemm_pair(a, gated, st);
   }
   return fail(FMOE_ERR_INVALID_ARG, "%s: unknown variant %d", who, a.variant);
 }
 
-}  // namespace
 }  // namespace fmoe
 
 extern "C" int fmoe_version(void) { return 4; }
 
-extern "C" int64_t fmoe_gemm_split_workspace_bytes(void) { return fmoe::gemm_tcgen05_split_workspace_bytes(); }
+extern "C" int64_t fmoe_gemm_split_workspace_bytes(void) { return fmoe::gemm_pair_split_workspace_bytes(); }
 
 extern "C" int fmoe_debug_tail_plan(int64_t total_tiles, int k_steps, int max_split, int grid, int cta, int64_t unit,
                                     int64_t* host_out) {

@@ -1,6 +1,9 @@
 // fmoe_fused_experts: the whole expert computation behind one C call.  Host-side orchestration only:
 // it carves the caller's workspace and enqueues the kernels of the other files on the given stream.
+#include "align.cuh"
 #include "fused.cuh"
+#include "pair.cuh"
+#include "rows.cuh"
 
 #include <nvtx3/nvToolsExt.h>
 
@@ -125,6 +128,10 @@ int plan_fused(const fmoe_fused_args& a, FusedPlan* pl) {
   p.off_npp = take(16);
   p.align_ws_bytes = fmoe_moe_align_workspace_bytes(p.numel, a.num_experts);
   p.off_align_ws = take(p.align_ws_bytes);
+  // the CTA-pair GEMMs read the experts' rows from one table, and their tail split counts arrivals in words that the
+  // align kernel clears: both GEMMs of a call have their own, so no memset stands between the kernels
+  p.off_table = tc ? take(pair_table_bytes(a.num_experts)) : -1;
+  p.off_counters = tc ? take(2 * kSplitCounters * 4) : -1;
   p.off_xs = p.off_xs_scale = p.off_xt = p.off_xt_scale = p.off_actq = p.off_actq_scale = p.off_split = -1;
   p.split_bytes = 0;
   if (channel) {
@@ -219,13 +226,29 @@ int run_fused(const fmoe_fused_args& a, const FusedPlan& p, uint8_t* ws, void* s
   auto st = (cudaStream_t)stream;
 
   mark(0);
-  int rc = fmoe_moe_align_block_size_ws(a.topk_ids, p.numel, a.num_experts, p.block, sorted, p.cap, experts, p.nblk, npp,
-                                        ws + p.off_align_ws, p.align_ws_bytes, stream);
+  int32_t* table = p.off_table >= 0 ? reinterpret_cast<int32_t*>(ws + p.off_table) : nullptr;
+  int32_t* counters = p.off_counters >= 0 ? reinterpret_cast<int32_t*>(ws + p.off_counters) : nullptr;
+  AlignArgs al;
+  al.topk_ids = a.topk_ids;
+  al.numel = p.numel;
+  al.E = a.num_experts;
+  al.block = p.block;
+  al.sorted_ids = sorted;
+  al.sorted_cap = p.cap;
+  al.expert_ids = experts;
+  al.expert_cap = p.nblk;
+  al.num_post_pad = npp;
+  al.workspace = ws + p.off_align_ws;
+  al.workspace_bytes = p.align_ws_bytes;
+  al.table = table;
+  al.zero_words = counters;
+  al.num_zero = counters ? 2 * kSplitCounters : 0;
+  int rc = run_align(al, st);
   if (rc) return rc;
   mark(1);
   if (a.zero_dropped) FMOE_CUDA_OK(cudaMemsetAsync(z, 0, (size_t)(p.numel * a.H * eb), st));
 
-  fmoe_gemm_args g{};
+  GemmParams g{};
   g.struct_size = (uint32_t)sizeof(fmoe_gemm_args);
   g.w_layout = a.w_layout;
   g.variant = p.variant;
@@ -243,7 +266,11 @@ int run_fused(const fmoe_fused_args& a, const FusedPlan& p, uint8_t* ws, void* s
     g.split_ws = ws + p.off_split;
     g.split_ws_bytes = p.split_bytes;
   }
-  fmoe_gemm_args g1 = g, g2 = g;
+  g.expert_table = table;
+  g.skip_padding = true;  // nothing below reads a padding row's values
+  GemmParams g1 = g, g2 = g;
+  g1.split_counters = counters;
+  g2.split_counters = counters ? counters + kSplitCounters : nullptr;
   g1.n = a.I;
   g1.activation = a.activation;
   g1.act_alpha = a.act_alpha;
@@ -268,7 +295,7 @@ int run_fused(const fmoe_fused_args& a, const FusedPlan& p, uint8_t* ws, void* s
     g1.dtype = g1.out_dtype = g2.dtype = a.dtype;
     if (tc && p.off_xs >= 0) {
       void* xs = ws + p.off_xs;
-      rc = fmoe_gather_rows(a.hidden, (int)eb, p.cap, a.H, sorted, a.top_k, p.numel, npp, xs, stream);
+      rc = run_gather_rows(a.hidden, (int)eb, p.cap, a.H, sorted, a.top_k, p.numel, npp, xs, false, st);
       if (rc) return rc;
       g1.a = xs;
       g1.a_rows = p.cap;
@@ -289,7 +316,7 @@ int run_fused(const fmoe_fused_args& a, const FusedPlan& p, uint8_t* ws, void* s
       float* xtsc = reinterpret_cast<float*>(ws + p.off_xt_scale);
       rc = fmoe_quant_fp8_per_token(a.hidden, FMOE_BF16, a.T, a.H, nullptr, 1, 0, nullptr, xt, xtsc, stream);
       if (rc) return rc;
-      rc = fmoe_gather_rows(xt, 1, p.cap, a.H, sorted, a.top_k, p.numel, npp, xq, stream);
+      rc = run_gather_rows(xt, 1, p.cap, a.H, sorted, a.top_k, p.numel, npp, xq, false, st);
       xsc = xtsc;  // the gate/up GEMM looks the scale up by token
       g1.a_scale_gather = 1;
     } else if (channel) {
@@ -319,7 +346,7 @@ int run_fused(const fmoe_fused_args& a, const FusedPlan& p, uint8_t* ws, void* s
     g2.w_scale = a.w2_scale;
   }
   mark(2);
-  rc = fmoe_gemm1_silu(&g1, stream);
+  rc = run_gemm(g1, true, st);
   if (rc) return rc;
   mark(3);
   if (fp8) {
@@ -333,7 +360,7 @@ int run_fused(const fmoe_fused_args& a, const FusedPlan& p, uint8_t* ws, void* s
     if (rc) return rc;
   }
   mark(4);
-  rc = fmoe_gemm2(&g2, stream);
+  rc = run_gemm(g2, false, st);
   if (rc) return rc;
   mark(5);
   if (a.no_combine) return FMOE_OK;

@@ -7,21 +7,28 @@
 
 namespace fmoe {
 
-using GemmParams = fmoe_gemm_args;
+// Arguments of one grouped GEMM: the public ones, and what only the one-call layer hands over (fused.cu).
+struct GemmParams : fmoe_gemm_args {
+  const int32_t* expert_table = nullptr;  // pair_table_words(E) words written by moe_align (see pair.cuh); NULL: derived
+  int32_t* split_counters = nullptr;      // zeroed arrival counters of the tail split; NULL: cleared by the launcher
+  bool skip_padding = false;              // gate/up: rows between an expert's last row and its block's end stay unwritten
+};
 
 // gated = true : gemm1, w has 2*n rows per expert (gate rows then up rows), output
 //                silu(gate)*up of width n, written at the sorted position p.
 // gated = false: gemm2, w has n rows per expert, output written at row slot(p).
 int gemm_simt(const GemmParams& p, bool gated, cudaStream_t st);
 int gemm_stream(const GemmParams& p, bool gated, cudaStream_t st);
-int gemm_tcgen05(const GemmParams& p, bool gated, cudaStream_t st);
+int gemm_pair(const GemmParams& p, bool gated, cudaStream_t st);
 int gemm_tcgen05_fp8(const GemmParams& p, bool gated, cudaStream_t st);
 
 // true when the variant can run these arguments (shape / alignment / dtype rules)
 bool gemm_stream_supports(const GemmParams& p, bool gated);
-bool gemm_tcgen05_supports(const GemmParams& p, bool gated);
-int64_t gemm_tcgen05_split_workspace_bytes();
+bool gemm_pair_supports(const GemmParams& p, bool gated);
+int64_t gemm_pair_split_workspace_bytes();
 int tail_plan_unit(int64_t total_tiles, int k_steps, int max_split, int grid, int cta, int64_t it, int64_t* out);
+// validates the arguments and launches the kernel family they ask for
+int run_gemm(const GemmParams& p, bool gated, cudaStream_t st);
 bool gemm_tcgen05_fp8_supports(const GemmParams& p, bool gated);
 
 // Tile order of the persistent kernels: expert by expert, and inside an expert in groups of at most
@@ -98,7 +105,7 @@ inline int pick_group_m(int64_t block_rows, int64_t k_bytes_per_row) {
   return (int)(g < 8 ? 8 : (g > 64 ? 64 : g));
 }
 
-// device status word written by bounded waits (gemm_tcgen05.cu)
+// device status word written by bounded waits (gemm_pair.cu)
 int read_and_clear_device_status(cudaStream_t st, int* status_out);
 
 }  // namespace fmoe

@@ -1,0 +1,806 @@
+// Grouped GEMM on CTA pairs (cluster of 2, tcgen05 cta_group::2) for bf16 operands, and for e4m3 operands with one scale
+// per token and one per output channel.
+//
+//   tile      : 256 weight rows (M, 128 in each CTA) x up to 256 tokens of one expert (N, half of them loaded by each CTA)
+//   K step    : 128 bytes per row (64 bf16 / 128 e4m3), one 128-byte swizzle atom; 4 MMAs per step
+//   pipeline  : 6 shared-memory stages of 16 KB of weights + at most 16 KB of tokens per CTA
+//   TMEM      : 512 columns per CTA = two 128 x 256 fp32 accumulators, so the epilogue of a tile overlaps the next tile
+//   warps     : 0-7 epilogue (TMEM lane quarter = warp % 4; the two halves take alternate 16-token chunks),
+//               8 TMA producer (each CTA its own weight rows and its own half of the tokens), 9 MMA issuer (CTA 0)
+//
+// Why pairs: with one CTA per 128 x 256 tile an MMA reads 12 KB of shared memory for every 8 KB here, and TMA writes as
+// much; fill and operand reads of one SM together ran into its 128 bytes per clock.  Why weights on M: see pair.cuh.
+//
+// gate/up GEMM: a CTA's 128 weight rows are 64 gate and the matching 64 up rows, alternating in groups of 16, so that in
+// the 16 x 256b read-out of TMEM a gate value and its up value land in the same thread; the activation is applied there
+// and only [rows, I] is written.  Output is transposed 16 tokens at a time through a strip of shared memory private to the
+// warp (stmatrix.trans), so that stores are 16 bytes of consecutive channels.
+//
+// Weights given as [E, K, N] (N contiguous) are read in place as an M-major operand, in 64-channel boxes: there the gate
+// rows are lanes 0-63 and the up rows lanes 64-127, and the pairs meet through shared memory.
+//
+// Every mbarrier wait is bounded; on expiry the warp records a code in a device status word, leaves its loops, and the CTA
+// frees its TMEM and returns.  The two cluster-wide barriers are reached by every thread on every path.  Every load has a
+// single destination CTA.
+#include "pair.cuh"
+
+#include <cstdlib>
+#include <mutex>
+
+namespace fmoe {
+
+__device__ int g_device_status = 0;  // 0 = fine; otherwise (role << 8 | site) of the first wait that gave up
+// Optional wait-time profile (FMOE_TC_PROFILE=1): per CTA {tiles, mma wait acc, mma wait data, producer wait, epilogue wait, epilogue busy}
+__device__ long long g_wait_prof[256 * 8];
+
+namespace {
+
+constexpr int KBYTES = 128;
+constexpr int STAGES = 6;
+constexpr int W_BYTES = 128 * KBYTES;               // this CTA's weight rows of a stage
+constexpr int T_BYTES = kPairTokens / 2 * KBYTES;   // this CTA's half of the tokens
+constexpr int STAGE_BYTES = W_BYTES + T_BYTES;
+constexpr int TMEM_COLS = 512;
+constexpr int ACC_COLS = 256;
+constexpr int kEpiWarps = 8;
+constexpr int kThreads = (kEpiWarps + 2) * 32;
+constexpr int BOX_TOKENS = 32;                      // token rows per TMA box
+constexpr int STRIP_BYTES = 16 * 80;                // per warp: 16 tokens x (32 channels + 8 of padding: no bank conflicts)
+constexpr int EX_PITCH = 20;                        // floats per lane row of the gate/up exchange (16 tokens + padding)
+constexpr int EX_BYTES = 128 * EX_PITCH * 4;        // per half of the epilogue warps
+constexpr int BAR_BYTES = 256;
+constexpr int smem_bytes(int num_experts, bool exchange) {
+  return 1024 + STAGES * STAGE_BYTES + BAR_BYTES + (exchange ? 2 * EX_BYTES : kEpiWarps * STRIP_BYTES) + pair_table_bytes(num_experts);
+}
+static_assert(smem_bytes(1024, true) <= 227 * 1024, "shared memory");
+
+struct PairParams {
+  const int32_t* sorted_token_ids;
+  const int32_t* expert_ids;
+  const int32_t* num_tokens_post_padded;
+  const int32_t* expert_table;  // written by moe_align (NULL: derived from the block tables)
+  const float* row_scale;
+  const float* a_scale;   // F8: one scale per row of the sorted order, or per token (a_scale_gather)
+  const float* w_scale;   // F8: [E, w_rows], one scale per output channel
+  const float* bias;      // optional [E, w_rows]
+  void* out;
+  void* const* out_rows;  // down projection: optional per-slot row addresses (may be peer memory)
+  float* split_partials;    // tail split: [workers][2 CTAs][128][256] f32 partial accumulators (NULL: no split)
+  int32_t* split_counters;  // tail split: [workers][2] arrivals, zero at launch
+  int64_t numel;
+  int64_t n;              // gemm1: I, gemm2: H
+  int64_t w_rows;         // rows of W per expert
+  float act_alpha, act_limit;
+  int32_t a_scale_gather;
+  int32_t num_experts;
+  int32_t k_steps;
+  int32_t w_tiles;
+  int32_t max_blocks;
+  int32_t activation;
+  int32_t group;
+  int32_t profile;
+  int32_t split_max;      // tail split: most K slices per tile (< 2: no split)
+  int32_t top_k;
+  int32_t a_rows;         // gather mode: rows of the input tensor (a row index >= a_rows reads zeros)
+  int32_t zero_padding;   // gemm1: rows between an expert's last token and its block's end are written as zeros
+};
+
+__device__ __forceinline__ void report(int code) { atomicCAS(&g_device_status, 0, code); }
+
+// Bounded wait whose verdict is uniform across the warp, so that the epilogue never diverges around __syncwarp().
+__device__ __forceinline__ bool warp_wait_relaxed(uint64_t* bar, uint32_t parity) {
+  return __all_sync(0xffffffffu, ptx::mbar_wait_relaxed(bar, parity));
+}
+__device__ __forceinline__ int32_t ld_acquire_gpu(const int32_t* p) {
+  int32_t v;
+  asm volatile("ld.acquire.gpu.global.s32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
+  return v;
+}
+
+template <bool GATED, bool F8, bool EXTRA, bool WMN, bool GATHER>
+__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 1)
+grouped_gemm_pair_kernel(const __grid_constant__ CUtensorMap map_t, const __grid_constant__ CUtensorMap map_w,
+                         const PairParams p) {
+  extern __shared__ uint8_t smem_raw[];
+  uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
+  uint64_t* bars = reinterpret_cast<uint64_t*>(smem + STAGES * STAGE_BYTES);
+  uint64_t* full_bar = bars;                    // [STAGES] used in CTA 0: the bytes of both CTAs' loads -> MMA
+  uint64_t* empty_bar = bars + STAGES;          // [STAGES] per CTA: MMA -> this CTA's producer
+  uint64_t* acc_full = bars + 2 * STAGES;       // [2] per CTA: MMA -> this CTA's epilogue
+  uint64_t* acc_empty = bars + 2 * STAGES + 2;  // [2] used in CTA 0: both epilogues -> MMA
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 2 * STAGES + 4);
+  uint8_t* strips = smem + STAGES * STAGE_BYTES + BAR_BYTES;
+  int32_t* table = reinterpret_cast<int32_t*>(strips + (GATED && WMN ? 2 * EX_BYTES : kEpiWarps * STRIP_BYTES));
+
+  const int warp = ptx::uniform_warp_id(), lane = threadIdx.x & 31;
+  const int rank = (int)ptx::cluster_ctarank();
+  const int worker = blockIdx.x >> 1, workers = gridDim.x >> 1;
+
+  if (threadIdx.x == 0) {
+    for (int s = 0; s < STAGES; ++s) {
+      ptx::mbar_init(&full_bar[s], 1);   // CTA 0's producer arms it with the bytes of both CTAs
+      ptx::mbar_init(&empty_bar[s], 1);  // one tcgen05.commit
+    }
+    for (int a = 0; a < 2; ++a) {
+      ptx::mbar_init(&acc_full[a], 1);
+      ptx::mbar_init(&acc_empty[a], 2 * kEpiWarps);  // one arrival per epilogue warp of both CTAs
+    }
+    ptx::fence_barrier_init();
+  }
+  if (warp == kEpiWarps && lane == 0) {
+    ptx::prefetch_tensormap(&map_t);
+    ptx::prefetch_tensormap(&map_w);
+  }
+  if (warp == kEpiWarps + 1) {
+    ptx::tmem_alloc_pair(tmem_slot, TMEM_COLS);
+    ptx::tmem_relinquish_pair();
+  }
+  ptx::tc_fence_before_sync();
+  pdl_entry();  // everything above is independent of the kernels before this one on the stream
+  const int used_blocks = min((int)(*p.num_tokens_post_padded / 128), p.max_blocks);
+  pair_build_table(table, p.num_experts, p.expert_table, p.expert_ids, p.sorted_token_ids, p.numel, 128, used_blocks);
+  ptx::cluster_sync_all();  // the other CTA's barriers exist before anything is signalled across
+  ptx::tc_fence_after_sync();
+  const uint32_t tmem_base = *tmem_slot;
+
+  const int k_steps = p.k_steps;
+  UnitPlan plan;
+  plan.init((int64_t)table[3 * p.num_experts] * p.w_tiles, k_steps, p.split_max, workers, worker);
+  PairCursor cursor;
+  PairTile tl;
+
+  if (warp == kEpiWarps) {
+    // ---------------- TMA producer (both CTAs) ----------------
+    if (ptx::elect_one()) {
+      int stage = 0;
+      uint32_t phase = 0;
+      bool alive = true;
+      long long prof_p = 0;
+      int64_t tile;
+      int ks0, ks1, slice;
+      const uint32_t ring = ptx::smem_u32(smem), bar_full0 = ptx::smem_u32(full_bar) & ~ptx::kPeerRankBit;
+      for (int64_t it = 0; alive && plan.get(it, &tile, &ks0, &ks1, &slice); ++it) {
+        cursor.locate(tile, p.w_tiles, p.group, p.num_experts, table, &tl);
+        const int half_n = tl.n >> 1;                       // tokens this CTA loads
+        const int row_t = tl.row0 + rank * half_n;
+        const int boxes = (half_n + BOX_TOKENS - 1) / BOX_TOKENS;
+        const uint32_t t_bytes = GATHER ? half_n * KBYTES : boxes * (BOX_TOKENS * KBYTES);
+        const int32_t c0 = GATED ? tl.w_tile * 128 + rank * 64 : tl.w_tile * 256 + rank * 128;
+        for (int ks = ks0; ks < ks1; ++ks) {
+          const long long tp0 = p.profile ? clock64() : 0;
+          const bool okp = ptx::mbar_wait(&empty_bar[stage], phase ^ 1);
+          if (p.profile) prof_p += clock64() - tp0;
+          if (!okp) {
+            report(0x100 | stage);
+            alive = false;
+            break;
+          }
+          const uint32_t sw = ring + stage * STAGE_BYTES, stok = sw + W_BYTES, bar0 = bar_full0 + stage * 8;
+          const int32_t x = ks * (KBYTES / (F8 ? 1 : 2));  // element coordinate along K
+          if (rank == 0) ptx::mbar_arrive_expect_tx(&full_bar[stage], 2 * (W_BYTES + t_bytes));
+          if constexpr (WMN) {
+            ptx::tma_load_3d_pair(sw, &map_w, c0, x, tl.expert, bar0);
+            ptx::tma_load_3d_pair(sw + W_BYTES / 2, &map_w, GATED ? c0 + (int32_t)p.n : c0 + 64, x, tl.expert, bar0);
+          } else if constexpr (GATED) {
+            ptx::tma_load_5d_pair(sw, &map_w, x, 0, 0, c0 >> 4, tl.expert, bar0);
+          } else {
+            ptx::tma_load_3d_pair(sw, &map_w, x, c0, tl.expert, bar0);
+          }
+          if constexpr (GATHER) {
+            auto row = [&](int32_t slot) { return (slot >= 0 && slot < p.numel) ? slot / p.top_k : p.a_rows; };
+            for (int r = 0; r < half_n; r += 4) {
+              const int4 s = *reinterpret_cast<const int4*>(p.sorted_token_ids + row_t + r);
+              ptx::tma_gather4_pair(stok + r * KBYTES, &map_t, x, row(s.x), row(s.y), row(s.z), row(s.w), bar0);
+            }
+          } else {
+            for (int b = 0; b < boxes; ++b)
+              ptx::tma_load_2d_pair(stok + b * (BOX_TOKENS * KBYTES), &map_t, x, row_t + b * BOX_TOKENS, bar0);
+          }
+          if (++stage == STAGES) {
+            stage = 0;
+            phase ^= 1;
+          }
+        }
+      }
+      if (p.profile && blockIdx.x < 256) g_wait_prof[blockIdx.x * 8 + 3] = prof_p;
+      if (alive) {  // drain: every stage this CTA filled has been consumed before the CTA may end
+        for (int s = 0; s < STAGES; ++s) {
+          if (!ptx::mbar_wait(&empty_bar[stage], phase ^ 1)) {
+            report(0x180 | stage);
+            break;
+          }
+          if (++stage == STAGES) {
+            stage = 0;
+            phase ^= 1;
+          }
+        }
+      }
+    }
+  } else if (warp == kEpiWarps + 1) {
+    // ---------------- MMA issuer (CTA 0 only) ----------------
+    if (rank == 0 && ptx::elect_one()) {
+      int stage = 0;
+      uint32_t phase = 0;
+      int local = 0;
+      bool alive = true;
+      long long prof_acc = 0, prof_data = 0;
+      int64_t tile;
+      int ks0, ks1, slice;
+      const uint32_t ring = ptx::smem_u32(smem);
+      const uint64_t db0 = ptx::smem_desc_sw128(ring + W_BYTES);
+      // M-major: 64 channels (128 B) x 8 K rows per swizzle atom; the next 8 K rows 1 KB on, the next 64 channels 8 KB on
+      const uint64_t da0 = WMN ? ptx::smem_desc_sw128_lbo(ring, W_BYTES / 2, 1024) : ptx::smem_desc_sw128(ring);
+      constexpr int a_step = WMN ? (2048 >> 4) : 2;  // one MMA's K: 16 K rows of 128 B, or 32 bytes of each row
+      for (int64_t it = 0; alive && plan.get(it, &tile, &ks0, &ks1, &slice); ++it) {
+        cursor.locate(tile, p.w_tiles, p.group, p.num_experts, table, &tl);
+        // bit 15: the M-side operand is M-major
+        const uint32_t idesc = ptx::make_idesc(F8 ? /*e4m3*/ 0 : /*bf16*/ 1, 256, (uint32_t)tl.n) | (WMN ? (1u << 15) : 0u);
+        const int acc = local & 1;
+        const uint32_t acc_phase = (local >> 1) & 1;
+        ++local;
+        const long long tm0 = p.profile ? clock64() : 0;
+        const bool oka = ptx::mbar_wait(&acc_empty[acc], acc_phase ^ 1);
+        if (p.profile) prof_acc += clock64() - tm0;
+        if (!oka) {
+          report(0x200 | acc);
+          alive = false;
+          break;
+        }
+        ptx::tc_fence_after_sync();
+        const uint32_t d_tmem = tmem_base + acc * ACC_COLS;
+        for (int ks = ks0; ks < ks1; ++ks) {
+          const long long tm1 = p.profile ? clock64() : 0;
+          const bool okd = ptx::mbar_wait(&full_bar[stage], phase);
+          if (p.profile) prof_data += clock64() - tm1;
+          if (!okd) {
+            report(0x240 | stage);
+            alive = false;
+            break;
+          }
+          ptx::tc_fence_after_sync();
+          const uint64_t da = da0 + (uint64_t)(stage * (STAGE_BYTES >> 4)), db = db0 + (uint64_t)(stage * (STAGE_BYTES >> 4));
+#pragma unroll
+          for (int kk = 0; kk < KBYTES / 32; ++kk) {
+            if constexpr (F8) ptx::mma_f8f6f4_ss_pair(d_tmem, da + a_step * kk, db + 2 * kk, idesc, ((ks - ks0) | kk) != 0);
+            else ptx::mma_f16_ss_pair(d_tmem, da + a_step * kk, db + 2 * kk, idesc, ((ks - ks0) | kk) != 0);
+          }
+          ptx::mma_commit_both(&empty_bar[stage]);  // the stage is free in both CTAs once these MMAs have read it
+          if (++stage == STAGES) {
+            stage = 0;
+            phase ^= 1;
+          }
+        }
+        if (alive) ptx::mma_commit_both(&acc_full[acc]);
+      }
+      if (p.profile && blockIdx.x < 256) {
+        g_wait_prof[blockIdx.x * 8 + 0] = local;
+        g_wait_prof[blockIdx.x * 8 + 1] = prof_acc;
+        g_wait_prof[blockIdx.x * 8 + 2] = prof_data;
+      }
+    }
+  } else {
+    // ---------------- epilogue (warps 0-7 of both CTAs, each its CTA's 128 weight rows) ----------------
+    const int quarter = warp & 3, half = warp >> 2;
+    const int g = lane >> 2, t = lane & 3;
+    uint8_t* strip = strips + warp * STRIP_BYTES;
+    int local = 0;
+    bool alive = true;
+    long long prof_wait = 0, prof_busy = 0;
+    int64_t tile;
+    int ks0, ks1, slice;
+    for (int64_t it = 0; alive && plan.get(it, &tile, &ks0, &ks1, &slice); ++it) {
+      cursor.locate(tile, p.w_tiles, p.group, p.num_experts, table, &tl);
+      const int acc = local & 1;
+      const uint32_t acc_phase = (local >> 1) & 1;
+      ++local;
+      const int chunks = tl.n >> 4;  // 16-token chunks; this warp takes those with the parity of `half`
+      // token f = 16 * c + u of the warp's c-th chunk sits in register f / 32 of lane f % 32
+      int32_t slot_r[4];
+      float rs_r[4];
+#pragma unroll
+      for (int r = 0; r < 4; ++r) {
+        const int f = r * 32 + lane;
+        const int tok = (2 * (f >> 4) + half) * 16 + (f & 15);
+        slot_r[r] = -1;
+        rs_r[r] = 1.0f;
+        if (tok < tl.cols) {
+          const int32_t s = p.sorted_token_ids[tl.row0 + tok];
+          if (s >= 0 && s < p.numel) {
+            slot_r[r] = s;
+            if (p.row_scale) rs_r[r] = p.row_scale[s];
+            if constexpr (F8) rs_r[r] *= p.a_scale_gather ? p.a_scale[s / p.top_k] : p.a_scale[tl.row0 + tok];
+          }
+        }
+      }
+      // first output channel of this warp, and per-channel factors / biases of its rows: gated {gate g, gate g+8, up g,
+      // up g+8}, plain {g, g+8, g+16, g+24}
+      const int ch0 = GATED ? tl.w_tile * 128 + rank * 64 + quarter * 16 : tl.w_tile * 256 + rank * 128 + quarter * 32;
+      float cv[4] = {0.f, 0.f, 0.f, 0.f};
+      if constexpr ((F8 || EXTRA) && !WMN) {
+        const float* vec = F8 ? p.w_scale : p.bias;
+        if (vec) {
+          vec += (int64_t)tl.expert * p.w_rows;
+#pragma unroll
+          for (int i = 0; i < 4; ++i) {
+            const int64_t c = GATED ? ch0 + g + 8 * (i & 1) : ch0 + g + 8 * i;
+            if (c < p.n) cv[i] = vec[c + (GATED && i >= 2 ? p.n : 0)];
+          }
+        }
+      }
+      const long long te0 = p.profile ? clock64() : 0;
+      const bool oke = warp_wait_relaxed(&acc_full[acc], acc_phase);
+      const long long te1 = p.profile ? clock64() : 0;
+      prof_wait += te1 - te0;
+      if (!oke) {
+        report(0x300 | acc);
+        alive = false;
+        break;
+      }
+      ptx::tc_fence_after_sync();
+      const uint32_t taddr = tmem_base + acc * ACC_COLS + ((uint32_t)(quarter * 32) << 16);
+      const bool split = plan.is_split(it);
+      const int S = split ? plan.S : 1;
+      const int c_begin = chunks * slice / S, c_end = chunks * (slice + 1) / S;
+      const int tail_index = plan.b / plan.S;
+      // fragment (slice o, chunk j) of this thread: four float4, 512 bytes apart so that a warp stores whole lines
+      auto partial = [&](int o, int j) {
+        return reinterpret_cast<float4*>(p.split_partials) +
+               ((((int64_t)(tail_index * S + o) * 2 + rank) * 16 + j) * 4 + quarter) * 128 + lane;
+      };
+      if (split) {
+#pragma unroll 1
+        for (int j = half; j < chunks; j += 2) {
+          if (j >= c_begin && j < c_end) continue;
+          uint32_t lo[8], hi[8];
+          ptx::tmem_ld_16x256b_x2(taddr + j * 16, lo);
+          ptx::tmem_ld_16x256b_x2(taddr + (16u << 16) + j * 16, hi);
+          ptx::tmem_ld_wait();
+          float4* dst = partial(slice, j);
+#pragma unroll
+          for (int q = 0; q < 4; ++q) {
+            const uint32_t* v = q < 2 ? lo + 4 * q : hi + 4 * (q - 2);
+            __stcg(dst + 32 * q, make_float4(__uint_as_float(v[0]), __uint_as_float(v[1]), __uint_as_float(v[2]),
+                                             __uint_as_float(v[3])));
+          }
+        }
+        __threadfence();  // the strips are visible device-wide before this warp counts as arrived
+        __syncwarp();
+        int32_t* counter = p.split_counters + tail_index * 2 + rank;
+        if (lane == 0) atomicAdd(counter, 1);
+        const long long t0 = clock64();
+        bool ok = true;
+        while (ld_acquire_gpu(counter) < kEpiWarps * S) {  // every epilogue warp of every slice has published
+          if (clock64() - t0 > 2000000000ll) {
+            ok = false;
+            break;
+          }
+          __nanosleep(64);
+        }
+        if (!__all_sync(0xffffffffu, ok)) {
+          report(0x380 | acc);
+          alive = false;
+          break;
+        }
+      }
+#pragma unroll 1
+      for (int j = half; j < chunks; j += 2) {
+        if (j < c_begin || j >= c_end) continue;
+        uint32_t lo[8], hi[8];
+        ptx::tmem_ld_16x256b_x2(taddr + j * 16, lo);                // rows 0-15 of the quarter (gated: gate)
+        ptx::tmem_ld_16x256b_x2(taddr + (16u << 16) + j * 16, hi);  // rows 16-31 (gated: up)
+        ptx::tmem_ld_wait();
+        if (S > 1) {
+          for (int o = 0; o < S; ++o) {
+            if (o == slice) continue;
+            const float4* src = partial(o, j);
+#pragma unroll
+            for (int q = 0; q < 4; ++q) {
+              const float4 v = __ldcg(src + 32 * q);
+              uint32_t* d = q < 2 ? lo + 4 * q : hi + 4 * (q - 2);
+              d[0] = __float_as_uint(__uint_as_float(d[0]) + v.x);
+              d[1] = __float_as_uint(__uint_as_float(d[1]) + v.y);
+              d[2] = __float_as_uint(__uint_as_float(d[2]) + v.z);
+              d[3] = __float_as_uint(__uint_as_float(d[3]) + v.w);
+            }
+          }
+        }
+        // the chunk's 16 slots and row scales, from the lanes that hold them
+        const int c = j >> 1;
+        const int32_t slot_c = (c >> 1) == 0 ? slot_r[0] : (c >> 1) == 1 ? slot_r[1] : (c >> 1) == 2 ? slot_r[2] : slot_r[3];
+        const float rs_c = (c >> 1) == 0 ? rs_r[0] : (c >> 1) == 1 ? rs_r[1] : (c >> 1) == 2 ? rs_r[2] : rs_r[3];
+        const int src_lane = (c & 1) * 16;
+        if constexpr (GATED && WMN) {
+          // gate rows are lanes 0-63, up rows 64-127: the four warps of a half meet in shared memory
+          float* ex = reinterpret_cast<float*>(strips + half * EX_BYTES);
+#pragma unroll
+          for (int q = 0; q < 4; ++q) {
+            const int row = quarter * 32 + g + 8 * (q & 1) + 16 * (q >> 1);
+            const uint32_t* v = (q >> 1) ? hi : lo;
+            *reinterpret_cast<float2*>(ex + row * EX_PITCH + 2 * t) =
+                make_float2(__uint_as_float(v[2 * (q & 1)]), __uint_as_float(v[2 * (q & 1) + 1]));
+            *reinterpret_cast<float2*>(ex + row * EX_PITCH + 8 + 2 * t) =
+                make_float2(__uint_as_float(v[4 + 2 * (q & 1)]), __uint_as_float(v[4 + 2 * (q & 1) + 1]));
+          }
+          asm volatile("bar.sync %0, 128;" ::"r"(1 + half) : "memory");
+          const int i = quarter * 32 + lane, u = i >> 3, oct = i & 7;  // token of the chunk, 8 channels
+          const int tok = j * 16 + u;
+          const float rs = __shfl_sync(0xffffffffu, rs_c, src_lane + u);
+          const int64_t ch = tl.w_tile * 128 + rank * 64 + oct * 8;
+          if (tok < tl.cols && ch < p.n) {
+            uint32_t w[4];
+#pragma unroll
+            for (int v = 0; v < 4; ++v) {
+              const float* e0 = ex + (oct * 8 + 2 * v) * EX_PITCH + u;
+              const float g0 = e0[0], g1 = e0[EX_PITCH], u0 = e0[64 * EX_PITCH], u1 = e0[65 * EX_PITCH];
+              w[v] = pack_bf16x2(act_mul_fast(g0 * rs, u0 * rs, p.activation), act_mul_fast(g1 * rs, u1 * rs, p.activation));
+            }
+            *reinterpret_cast<uint4*>(reinterpret_cast<__nv_bfloat16*>(p.out) + (int64_t)(tl.row0 + tok) * p.n + ch) =
+                make_uint4(w[0], w[1], w[2], w[3]);
+          }
+          asm volatile("bar.sync %0, 128;" ::"r"(1 + half) : "memory");
+        } else {
+          float rs[4];  // columns 2t, 2t+1, 8+2t, 9+2t
+#pragma unroll
+          for (int q = 0; q < 4; ++q) rs[q] = __shfl_sync(0xffffffffu, rs_c, src_lane + (q >> 1) * 8 + 2 * t + (q & 1));
+          if constexpr (GATED) {
+            uint32_t m[4];
+#pragma unroll
+            for (int q = 0; q < 4; ++q) {  // q = 2 * (column group) + (row half)
+              const int i = 4 * (q >> 1) + 2 * (q & 1);
+              float o[2];
+#pragma unroll
+              for (int v = 0; v < 2; ++v) {
+                const float gv = __uint_as_float(lo[i + v]), uv = __uint_as_float(hi[i + v]), r = rs[2 * (q >> 1) + v];
+                if constexpr (EXTRA)
+                  o[v] = gated_output<true>(gv, uv, cv[q & 1], cv[2 + (q & 1)], r, p.activation, p.act_alpha, p.act_limit);
+                else if constexpr (F8)  // (accumulator * row scale) * channel scale, then the activation
+                  o[v] = act_mul_fast(gv * r * cv[q & 1], uv * r * cv[2 + (q & 1)], p.activation);
+                else
+                  o[v] = act_mul_fast(gv * r, uv * r, p.activation);
+              }
+              m[q] = pack_bf16x2(o[0], o[1]);
+            }
+            constexpr int PITCH = 48;  // 16 channels + 8 of padding
+            const int tok_l = (lane & 7) + (lane >> 4) * 8, ch_l = ((lane >> 3) & 1) * 8;
+            ptx::stmatrix_x4_trans(ptx::smem_u32(strip + tok_l * PITCH + ch_l * 2), m[0], m[1], m[2], m[3]);
+            __syncwarp();
+            const int u = lane >> 1, part = (lane & 1) * 8;
+            const uint4 v = *reinterpret_cast<const uint4*>(strip + u * PITCH + part * 2);
+            const int tok = j * 16 + u;
+            if (tok < tl.cols && ch0 + part < p.n)
+              *reinterpret_cast<uint4*>(reinterpret_cast<__nv_bfloat16*>(p.out) + (int64_t)(tl.row0 + tok) * p.n + ch0 + part) = v;
+            __syncwarp();
+          } else {
+            constexpr int PITCH = 80;  // 32 channels + 8 of padding
+            const int tok_l = (lane & 7) + (lane >> 4) * 8, ch_l = ((lane >> 3) & 1) * 8;
+#pragma unroll
+            for (int h = 0; h < 2; ++h) {
+              uint32_t m[4];
+#pragma unroll
+              for (int q = 0; q < 4; ++q) {
+                const int i = 4 * (q >> 1) + 2 * (q & 1);
+                const uint32_t* a = h ? hi : lo;
+                const float v0 = __uint_as_float(a[i]), v1 = __uint_as_float(a[i + 1]);
+                const float r0 = rs[2 * (q >> 1)], r1 = rs[2 * (q >> 1) + 1], c0 = cv[2 * h + (q & 1)];
+                if constexpr (F8) m[q] = pack_bf16x2(v0 * r0 * c0, v1 * r1 * c0);
+                else m[q] = pack_bf16x2((v0 + c0) * r0, (v1 + c0) * r1);
+              }
+              ptx::stmatrix_x4_trans(ptx::smem_u32(strip + tok_l * PITCH + (16 * h + ch_l) * 2), m[0], m[1], m[2], m[3]);
+            }
+            __syncwarp();
+#pragma unroll
+            for (int h = 0; h < 2; ++h) {
+              const int u = (lane >> 2) + 8 * h, part = (lane & 3) * 8;
+              const uint4 v = *reinterpret_cast<const uint4*>(strip + u * PITCH + part * 2);
+              const int32_t slot = __shfl_sync(0xffffffffu, slot_c, src_lane + u);
+              if (slot >= 0 && ch0 + part < p.n) {
+                __nv_bfloat16* orow = p.out_rows ? reinterpret_cast<__nv_bfloat16*>(p.out_rows[slot])
+                                                 : reinterpret_cast<__nv_bfloat16*>(p.out) + (int64_t)slot * p.n;
+                if (orow) *reinterpret_cast<uint4*>(orow + ch0 + part) = v;
+              }
+            }
+            __syncwarp();
+          }
+        }
+      }
+      // the accumulator may be overwritten from here on: tell CTA 0's MMA warp
+      ptx::tc_fence_before_sync();
+      __syncwarp();
+      if (lane == 0) ptx::mbar_arrive_cluster(ptx::smem_u32(&acc_empty[acc]) & ~ptx::kPeerRankBit);
+      if constexpr (GATED) {
+        if (p.zero_padding && tl.last && slice == 0) {
+          const int end = (tl.row0 + tl.cols + 127) & ~127;  // blocks start at multiples of 128 rows
+          const int tile_ch = tl.w_tile * 128 + rank * 64;
+          for (int i = threadIdx.x; i < (end - tl.row0 - tl.cols) * 8; i += kEpiWarps * 32) {
+            const int64_t row = tl.row0 + tl.cols + (i >> 3), ch = tile_ch + (i & 7) * 8;
+            if (ch < p.n)
+              *reinterpret_cast<uint4*>(reinterpret_cast<__nv_bfloat16*>(p.out) + row * p.n + ch) = make_uint4(0, 0, 0, 0);
+          }
+        }
+      }
+      if (p.profile) prof_busy += clock64() - te1;
+    }
+    if (p.out_rows) __threadfence_system();  // rows stored to a peer are complete before the kernel ends
+    if (p.profile && threadIdx.x == 0 && blockIdx.x < 256) {
+      g_wait_prof[blockIdx.x * 8 + 4] = prof_wait;
+      g_wait_prof[blockIdx.x * 8 + 5] = prof_busy;
+    }
+  }
+
+  ptx::tc_fence_before_sync();
+  __syncthreads();
+  ptx::cluster_sync_all();  // nobody signals into a CTA that has left, and both are done with TMEM
+  if (warp == kEpiWarps + 1) {
+    ptx::tc_fence_after_sync();
+    ptx::tmem_dealloc_pair(tmem_base, TMEM_COLS);
+  }
+}
+
+// ---- host side ----------------------------------------------------------------
+using EncodeTiledFn = CUresult (*)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*,
+                                   const cuuint64_t*, const cuuint32_t*, const cuuint32_t*, CUtensorMapInterleave,
+                                   CUtensorMapSwizzle, CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
+
+EncodeTiledFn encode_tiled_fn() {
+  static EncodeTiledFn fn = nullptr;
+  static std::once_flag once;
+  std::call_once(once, [] {
+    void* ptr = nullptr;
+    cudaDriverEntryPointQueryResult qres;
+    if (cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &ptr, cudaEnableDefault, &qres) == cudaSuccess &&
+        qres == cudaDriverEntryPointSuccess)
+      fn = reinterpret_cast<EncodeTiledFn>(ptr);
+  });
+  return fn;
+}
+
+int encode(CUtensorMap* map, const void* base, int elem_bytes, int rank, const cuuint64_t* dims, const cuuint64_t* strides,
+           const cuuint32_t* box, bool weights, const char* what) {
+  EncodeTiledFn fn = encode_tiled_fn();
+  if (!fn) return fail(FMOE_ERR_CUDA, "cuTensorMapEncodeTiled is not available from the driver");
+  const cuuint32_t estr[5] = {1, 1, 1, 1, 1};
+  CUresult r = fn(map, elem_bytes == 2 ? CU_TENSOR_MAP_DATA_TYPE_BFLOAT16 : CU_TENSOR_MAP_DATA_TYPE_UINT8, (cuuint32_t)rank,
+                  const_cast<void*>(base), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
+                  CU_TENSOR_MAP_SWIZZLE_128B,
+                  weights ? CU_TENSOR_MAP_L2_PROMOTION_L2_256B : CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
+                  CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+  if (r != CUDA_SUCCESS) return fail(FMOE_ERR_CUDA, "cuTensorMapEncodeTiled (%s) failed with code %d", what, (int)r);
+  return FMOE_OK;
+}
+
+}  // namespace
+
+// SM count of the current device (cached per device ordinal).
+int device_sm_count() {
+  static std::mutex mu;
+  static int sm_count[kMaxDevices] = {};
+  int dev = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess) return 0;
+  if (dev < 0 || dev >= kMaxDevices) {
+    int n = 0;
+    cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev);
+    return n;
+  }
+  std::lock_guard<std::mutex> lock(mu);
+  if (sm_count[dev] == 0) cudaDeviceGetAttribute(&sm_count[dev], cudaDevAttrMultiProcessorCount, dev);
+  return sm_count[dev];
+}
+
+// Host-side view of the work-unit plan (the same code the kernels run), for tests.
+int tail_plan_unit(int64_t total_tiles, int k_steps, int max_split, int grid, int cta, int64_t it, int64_t* out) {
+  UnitPlan plan;
+  plan.init(total_tiles, k_steps, max_split, grid, cta);
+  int64_t tile = 0;
+  int ks0 = 0, ks1 = 0, slice = 0;
+  if (!plan.get(it, &tile, &ks0, &ks1, &slice)) return 0;
+  out[0] = tile;
+  out[1] = ks0;
+  out[2] = ks1;
+  out[3] = slice;
+  out[4] = plan.is_split(it) ? plan.S : 1;
+  return 1;
+}
+
+int64_t gemm_pair_split_workspace_bytes() {
+  const int sms = device_sm_count();
+  return 1024 + (int64_t)std::min(std::max(sms, 1), 256) * 128 * 256 * 4;
+}
+
+// tokens: row-major [rows, cols]; box = 128 bytes x box_rows
+int pair_map_tokens(CUtensorMap* map, const void* base, int64_t rows, int64_t cols, int elem_bytes, int box_rows) {
+  const cuuint64_t dims[2] = {(cuuint64_t)cols, (cuuint64_t)rows};
+  const cuuint64_t strides[1] = {(cuuint64_t)cols * elem_bytes};
+  const cuuint32_t box[2] = {(cuuint32_t)(KBYTES / elem_bytes), (cuuint32_t)box_rows};
+  return encode(map, base, elem_bytes, 2, dims, strides, box, false, "tokens");
+}
+
+int make_tensor_map_2d(CUtensorMap* map, const void* base, int64_t rows, int64_t cols, int elem_bytes, int box_rows,
+                       bool weights, int kbytes) {
+  const cuuint64_t dims[2] = {(cuuint64_t)cols, (cuuint64_t)rows};
+  const cuuint64_t strides[1] = {(cuuint64_t)cols * elem_bytes};
+  const cuuint32_t box[2] = {(cuuint32_t)(kbytes / elem_bytes), (cuuint32_t)box_rows};
+  return encode(map, base, elem_bytes, 2, dims, strides, box, weights, "2d");
+}
+
+// weights [E, rows, K], K contiguous.  gated: rows = n gate rows then n up rows; the box takes 4 groups of 16 gate rows and
+// the 16 matching up rows (K, 16 rows, gate/up, row groups, expert: rows past n read as zeros).  plain: rows = n, 128 rows.
+int pair_map_weights(CUtensorMap* map, const void* base, int64_t experts, int64_t n, int64_t k, int elem_bytes, bool gated) {
+  const cuuint64_t row = (cuuint64_t)k * elem_bytes;
+  if (gated) {
+    const cuuint64_t dims[5] = {(cuuint64_t)k, 16, 2, (cuuint64_t)(n / 16), (cuuint64_t)experts};
+    const cuuint64_t strides[4] = {row, row * n, row * 16, row * 2 * n};
+    const cuuint32_t box[5] = {(cuuint32_t)(KBYTES / elem_bytes), 16, 2, 4, 1};
+    return encode(map, base, elem_bytes, 5, dims, strides, box, true, "gate/up weights");
+  }
+  const cuuint64_t dims[3] = {(cuuint64_t)k, (cuuint64_t)n, (cuuint64_t)experts};
+  const cuuint64_t strides[2] = {row, row * n};
+  const cuuint32_t box[3] = {(cuuint32_t)(KBYTES / elem_bytes), 128, 1};
+  return encode(map, base, elem_bytes, 3, dims, strides, box, true, "down weights");
+}
+
+// bf16 weights [E, K, w_rows] with w_rows contiguous; box = 64 channels (128 bytes, the swizzle width) x 64 K rows.
+int pair_map_weights_nmajor(CUtensorMap* map, const void* base, int64_t experts, int64_t k, int64_t w_rows) {
+  const cuuint64_t dims[3] = {(cuuint64_t)w_rows, (cuuint64_t)k, (cuuint64_t)experts};
+  const cuuint64_t strides[2] = {(cuuint64_t)w_rows * 2, (cuuint64_t)w_rows * (cuuint64_t)k * 2};
+  const cuuint32_t box[3] = {64, 64, 1};
+  return encode(map, base, 2, 3, dims, strides, box, true, "N-major weights");
+}
+
+namespace {
+
+template <bool GATED, bool F8, bool EXTRA, bool WMN, bool GATHER>
+int launch(const GemmParams& g, cudaStream_t st) {
+  constexpr int ELEM = F8 ? 1 : 2;
+  constexpr int MAX_SMEM = smem_bytes(1024, GATED && WMN);
+  auto kernel = grouped_gemm_pair_kernel<GATED, F8, EXTRA, WMN, GATHER>;
+  const int smem = smem_bytes(g.num_experts, GATED && WMN);
+  static PerDeviceOnce once_attr;  // the opt-in to > 48 KB of dynamic shared memory is per device
+  const cudaError_t attr_err = per_device_once(once_attr, [&] {
+    return cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, MAX_SMEM);
+  });
+  if (attr_err != cudaSuccess)
+    return fail(FMOE_ERR_CUDA, "cudaFuncSetAttribute(smem=%d) failed: %s", MAX_SMEM, cudaGetErrorString(attr_err));
+
+  const int64_t w_rows = GATED ? 2 * g.n : g.n;
+  CUtensorMap map_t, map_w;
+  int rc = pair_map_tokens(&map_t, g.a, g.a_rows, g.k, ELEM, GATHER ? 1 : BOX_TOKENS);
+  if (rc) return rc;
+  if constexpr (WMN) rc = pair_map_weights_nmajor(&map_w, g.w, g.num_experts, g.k, w_rows);
+  else rc = pair_map_weights(&map_w, g.w, g.num_experts, g.n, g.k, ELEM, GATED);
+  if (rc) return rc;
+
+  PairParams p;
+  p.sorted_token_ids = g.sorted_token_ids;
+  p.expert_ids = g.expert_ids;
+  p.num_tokens_post_padded = g.num_tokens_post_padded;
+  p.expert_table = g.expert_table;
+  p.row_scale = g.row_scale;
+  p.a_scale = g.a_scale;
+  p.a_scale_gather = g.a_scale_gather;
+  p.w_scale = g.w_scale;
+  p.bias = g.bias;
+  p.act_alpha = g.act_alpha;
+  p.act_limit = g.act_limit;
+  p.out = g.out;
+  p.out_rows = GATED ? nullptr : g.out_rows;
+  p.numel = g.numel;
+  p.n = g.n;
+  p.w_rows = w_rows;
+  p.num_experts = g.num_experts;
+  p.k_steps = (int)ceil_div<int64_t>(g.k * ELEM, KBYTES);
+  p.w_tiles = (int)ceil_div<int64_t>(g.n, GATED ? 128 : 256);
+  p.max_blocks = (int)g.max_blocks;
+  p.activation = g.activation;
+  p.top_k = g.top_k;
+  p.a_rows = (int32_t)g.a_rows;
+  p.zero_padding = !g.skip_padding;
+  p.group = pick_group_m(kPairTokens, g.k * ELEM);
+  static const bool profile = getenv("FMOE_TC_PROFILE") != nullptr;
+  p.profile = profile;
+
+  const int64_t max_tiles = g.max_blocks * p.w_tiles;  // an expert has no more 256-token tiles than 128-row blocks
+  const int sms = device_sm_count();
+  const int workers = (int)std::max<int64_t>(1, std::min<int64_t>((sms > 0 ? sms : 148) / 2, max_tiles));
+  p.split_partials = nullptr;
+  p.split_counters = nullptr;
+  p.split_max = 0;
+  const char* split_env = getenv("FMOE_TC_SPLIT_TAIL");  // "0": off (read per launch, tests flip it)
+  const bool split_off = split_env && split_env[0] == '0';
+  const bool split_fits = g.split_ws_bytes >= 1024 + (int64_t)workers * 2 * 128 * 256 * 4 && workers <= 128;
+  if (g.split_ws && !split_off && split_fits && aligned16(g.split_ws)) {
+    p.split_partials = reinterpret_cast<float*>(reinterpret_cast<uint8_t*>(g.split_ws) + 1024);
+    p.split_max = GATED ? 4 : 8;
+    if (g.split_counters) {
+      p.split_counters = g.split_counters;
+    } else {
+      p.split_counters = reinterpret_cast<int32_t*>(g.split_ws);
+      FMOE_CUDA_OK(cudaMemsetAsync(g.split_ws, 0, 1024, st));
+    }
+  }
+  launch_pdl(kernel, dim3(2 * workers), dim3(kThreads), smem, st, map_t, map_w, p);
+  return launch_status("grouped_gemm_pair_kernel");
+}
+
+}  // namespace
+
+bool gemm_pair_supports(const GemmParams& p, bool gated) {
+  const bool f8 = p.dtype == FMOE_E4M3 && p.scale_mode == FMOE_SCALE_CHANNEL;
+  if ((p.dtype != FMOE_BF16 && !f8) || p.out_dtype != FMOE_BF16) return false;
+  // e4m3 with per-row / per-channel scales: plain kernels, K-major weights, sorted input rows
+  if (f8 && (p.a_gather || p.bias || p.w_layout != FMOE_W_K_MAJOR || !p.a_scale || !p.w_scale || !aligned16(p.w_scale) ||
+             (gated && p.activation == FMOE_ACT_SWIGLU_OAI)))
+    return false;
+  if (p.block_size != 128) return false;
+  // gather mode: gate/up GEMM only; one int4 of sorted ids per lane
+  if (p.a_gather && (!gated || p.top_k < 1 || !aligned16(p.sorted_token_ids))) return false;
+  if (p.w_layout != FMOE_W_K_MAJOR && p.w_layout != FMOE_W_N_MAJOR) return false;
+  // weights in the reference operator's [E, K, N] layout: plain kernels only (no row gather, bias or swiglu_oai)
+  if (p.w_layout == FMOE_W_N_MAJOR && (p.a_gather || p.bias || (gated && p.activation == FMOE_ACT_SWIGLU_OAI))) return false;
+  if (p.k <= 0 || (p.k * (f8 ? 1 : 2)) % 16 != 0) return false;  // TMA row stride must be a multiple of 16 bytes
+  if (p.n <= 0 || p.n % 32 != 0) return false;  // gate/up row groups of 16, 16-byte stores
+  if (!aligned16(p.a) || !aligned16(p.w) || !(aligned16(p.out) && (p.out || (!gated && p.out_rows)))) return false;
+  if ((int64_t)p.num_experts * (gated ? 2 * p.n : p.n) >= (1ll << 31) || p.a_rows >= (1ll << 31)) return false;
+  if (p.max_blocks >= (1ll << 24) || p.num_experts > 1024) return false;
+  return true;
+}
+
+int gemm_pair(const GemmParams& p, bool gated, cudaStream_t st) {
+  if (!gemm_pair_supports(p, gated))
+    return fail(FMOE_ERR_UNSUPPORTED,
+                "tcgen05 gemm: needs bf16 in/out (or e4m3 in with per-channel scales), block_size 128, input-row gather only for the gate/up gemm, "
+                "n %% %d == 0, 16-byte aligned pointers (got dtype=%d block=%d a_gather=%d n=%lld k=%lld)",
+                32, p.dtype, p.block_size, p.a_gather, (long long)p.n, (long long)p.k);
+  if (p.max_blocks <= 0) return FMOE_OK;
+  const bool extra = p.bias != nullptr || (gated && p.activation == FMOE_ACT_SWIGLU_OAI);
+  //                                      GATED  F8    EXTRA  WMN    GATHER
+  if (p.dtype == FMOE_E4M3)
+    return gated ? launch<true, true, false, false, false>(p, st) : launch<false, true, false, false, false>(p, st);
+  if (p.w_layout == FMOE_W_N_MAJOR)
+    return gated ? launch<true, false, false, true, false>(p, st) : launch<false, false, false, true, false>(p, st);
+  if (p.a_gather) return extra ? launch<true, false, true, false, true>(p, st) : launch<true, false, false, false, true>(p, st);
+  if (gated) return extra ? launch<true, false, true, false, false>(p, st) : launch<true, false, false, false, false>(p, st);
+  return extra ? launch<false, false, true, false, false>(p, st) : launch<false, false, false, false, false>(p, st);
+}
+
+namespace {
+// Self-test of the time-out path: waits on a barrier that nobody signals, with a short limit.
+__global__ void bounded_wait_selftest_kernel(long long limit_cycles) {
+  __shared__ uint64_t bar;
+  if (threadIdx.x == 0) {
+    ptx::mbar_init(&bar, 1);
+    ptx::fence_barrier_init();
+  }
+  __syncthreads();
+  if (!ptx::mbar_wait_limit(&bar, 0, limit_cycles) && threadIdx.x == 0) report(0xE00);
+}
+}  // namespace
+
+int launch_bounded_wait_selftest(long long limit_cycles, cudaStream_t st) {
+  bounded_wait_selftest_kernel<<<1, 32, 0, st>>>(limit_cycles);
+  return launch_status("bounded_wait_selftest_kernel");
+}
+
+int read_wait_profile(long long* host_out, int n) {
+  FMOE_CUDA_OK(cudaMemcpyFromSymbol(host_out, g_wait_prof, sizeof(long long) * (size_t)n));
+  return FMOE_OK;
+}
+
+int status_word_fp8(int* out, bool clear);
+int status_word_ep(int* out, bool clear);
+
+// First non-zero status word of the translation units that keep one (tcgen05 kernels, expert-parallel
+// exchange); all are cleared.
+int read_and_clear_device_status(cudaStream_t st, int* status_out) {
+  int zero = 0, a = 0, b = 0, d = 0;
+  FMOE_CUDA_OK(cudaStreamSynchronize(st));
+  FMOE_CUDA_OK(cudaMemcpyFromSymbol(&a, g_device_status, sizeof(int)));
+  if (a != 0) FMOE_CUDA_OK(cudaMemcpyToSymbol(g_device_status, &zero, sizeof(int)));
+  int rc = status_word_fp8(&b, true);
+  if (rc) return rc;
+  rc = status_word_ep(&d, true);
+  if (rc) return rc;
+  *status_out = a ? a : (b ? b : d);
+  return FMOE_OK;
+}
+
+}  // namespace fmoe

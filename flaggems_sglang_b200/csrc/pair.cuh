@@ -1,0 +1,181 @@
+// What the CTA-pair grouped GEMMs (gemm_pair.cu, gemm_pair_fold.cu) share: the table of experts, the tile order, the work
+// units of a cluster and the TMA maps.
+//
+// Both kernels put the WEIGHTS on the M side of the tensor cores (256 weight rows per tile, 128 in each CTA of a pair)
+// and the tokens on the N side.  N is any multiple of 16 up to 256, so an expert with 9 tokens costs a 16-column tile and
+// one with 300 costs two of 160: no work is done for padding beyond 15 columns, and the weights are read once per 256
+// tokens.  The rows between an expert's last token and the next multiple of the moe_align block are never touched.
+#pragma once
+#include "gemm.cuh"
+#include "ptx_sm100.cuh"
+
+namespace fmoe {
+
+constexpr int kPairTokens = 256;     // most tokens of a tile
+constexpr int kSplitCounters = 256;  // tail-split arrival counters of one launch: one per CTA
+
+// int32 words of the expert table: first row [E], rows [E], exclusive prefix sum of the token tiles [E + 1]
+__host__ __device__ constexpr int pair_table_words(int num_experts) { return 3 * num_experts + 1; }
+__host__ __device__ constexpr int pair_table_bytes(int num_experts) { return (pair_table_words(num_experts) * 4 + 15) & ~15; }
+
+#if defined(__CUDACC__)
+// Exclusive prefix sum over the experts' token tiles by one warp; rows[e] -> prefix[e], total in prefix[E].
+__device__ __forceinline__ void pair_prefix_warp(const int32_t* rows, int32_t* prefix, int num_experts, int lane) {
+  int carry = 0;
+  for (int base = 0; base < num_experts; base += 32) {
+    const int e = base + lane;
+    const int tiles = e < num_experts ? (rows[e] + kPairTokens - 1) / kPairTokens : 0;
+    int incl = tiles;
+#pragma unroll
+    for (int off = 1; off < 32; off <<= 1) {
+      const int v = __shfl_up_sync(0xffffffffu, incl, off);
+      if (lane >= off) incl += v;
+    }
+    if (e < num_experts) prefix[e] = carry + incl - tiles;
+    carry += __shfl_sync(0xffffffffu, incl, 31);
+  }
+  if (lane == 0) prefix[num_experts] = carry;
+}
+
+// All threads of the CTA fill `table` (shared memory): a copy of the one moe_align wrote, or, for callers of the plain
+// C entry points, derived from the block tables (rows of an expert = up to the last real slot of its last block).
+// Ends with __syncthreads().
+__device__ __forceinline__ void pair_build_table(int32_t* table, int num_experts, const int32_t* __restrict__ global_table,
+                                                 const int32_t* __restrict__ expert_ids,
+                                                 const int32_t* __restrict__ sorted_ids, int64_t numel, int block_rows,
+                                                 int used_blocks) {
+  if (global_table) {
+    for (int i = threadIdx.x; i < pair_table_words(num_experts); i += blockDim.x) table[i] = global_table[i];
+    __syncthreads();
+    return;
+  }
+  int32_t* first = table;
+  int32_t* rows = table + num_experts;
+  for (int e = threadIdx.x; e < num_experts; e += blockDim.x) {
+    first[e] = 0x7fffffff;
+    rows[e] = 0;
+  }
+  __syncthreads();
+  for (int b = threadIdx.x; b < used_blocks; b += blockDim.x) {
+    const int e = expert_ids[b];
+    if (e >= 0 && e < num_experts) {
+      atomicMin(&first[e], b);
+      atomicAdd(&rows[e], 1);
+    }
+  }
+  __syncthreads();
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  for (int e = warp; e < num_experts; e += blockDim.x >> 5) {
+    const int b0 = first[e], nb = rows[e];
+    __syncwarp();
+    int last = 0;
+    if (nb > 0) {
+      const int64_t base = (int64_t)(b0 + nb - 1) * block_rows;
+      for (int i = lane; i < block_rows; i += 32) {
+        const int32_t s = sorted_ids[base + i];
+        if (s >= 0 && s < numel) last = i + 1;
+      }
+      last = __reduce_max_sync(0xffffffffu, last);
+    }
+    if (lane == 0) {
+      first[e] = nb > 0 ? b0 * block_rows : 0;
+      rows[e] = nb > 0 ? (nb - 1) * block_rows + last : 0;
+    }
+  }
+  __syncthreads();
+  if (warp == 0) pair_prefix_warp(rows, table + 2 * num_experts, num_experts, lane);
+  __syncthreads();
+}
+
+// One tile: `cols` real tokens (rows [row0, row0 + cols) of the sorted order) x weight tile `w_tile` of `expert`;
+// n = cols rounded up to the 16 columns that an MMA of M = 256 steps by.
+struct PairTile {
+  int row0, cols, n, w_tile, expert;
+  bool last;  // holds the expert's last token
+};
+
+// Tile order: expert by expert, inside an expert in groups of at most `group` token tiles, inside a group the token tile
+// varies fastest: the tiles that run at the same time share weight rows through L2, and the group's token rows stay hot.
+struct PairCursor {
+  int expert = 0;
+  __device__ __forceinline__ void locate(int64_t tile, int w_tiles, int group, int num_experts, const int32_t* table,
+                                         PairTile* out) {
+    const int32_t* prefix = table + 2 * num_experts;
+    const int q = (int)(tile / w_tiles);
+    if (!(prefix[expert] <= q && q < prefix[expert + 1])) {
+      int lo = 0, hi = num_experts - 1;  // last expert whose prefix is <= q (one with tiles, as q < prefix[E])
+      while (lo < hi) {
+        const int mid = (lo + hi + 1) >> 1;
+        if (prefix[mid] <= q) lo = mid;
+        else hi = mid - 1;
+      }
+      expert = lo;
+    }
+    const int tiles = prefix[expert + 1] - prefix[expert];
+    const int rows = table[num_experts + expert];
+    const int64_t local = tile - (int64_t)prefix[expert] * w_tiles;
+    const int64_t per_group = (int64_t)group * w_tiles;
+    const int g = (int)(local / per_group), r = (int)(local % per_group);
+    const int in_group = min(group, tiles - g * group);
+    out->w_tile = r / in_group;
+    const int t = g * group + r % in_group;
+    const int step = (((rows + tiles - 1) / tiles) + 15) & ~15;  // the expert's tokens in equal tiles (<= 256)
+    out->row0 = table[expert] + t * step;
+    out->cols = min(step, rows - t * step);
+    out->n = (out->cols + 15) & ~15;
+    out->expert = expert;
+    out->last = t == tiles - 1;
+  }
+};
+#endif
+
+// Work units of one worker (a CTA pair).  Tiles are dealt round-robin; when the last round has work for at most half of
+// the workers (they are bound by their own rate, so a part-filled round costs as much as a full one), each of its tiles
+// is cut into S slices along K (S a power of two) that S neighbouring workers compute.  The S partial accumulators are
+// then summed by all S workers together: worker s owns the s-th strip of the tile's columns, publishes the other strips
+// of its partial in global memory, waits until all S have done so, adds the others' partials of its strip in slice
+// order (a fixed order: results do not depend on timing) and runs the epilogue on the strip.
+struct UnitPlan {
+  int64_t total, rounds, left;
+  int grid, b, S, k_steps;
+  __host__ __device__ __forceinline__ void init(int64_t total_tiles, int k_steps_, int max_split, int grid_, int b_) {
+    total = total_tiles;
+    k_steps = k_steps_;
+    grid = grid_;
+    b = b_;
+    S = 1;
+    rounds = (total + grid - 1) / grid;
+    left = total - (rounds - 1) * grid;
+    if (total > 0 && max_split >= 2 && left * 2 <= grid) {
+      int s = (int)(max_split < grid / left ? max_split : grid / left);
+      s = s < k_steps / 8 ? s : k_steps / 8;
+      while (s & (s - 1)) s &= s - 1;  // largest power of two below
+      if (s >= 2) S = s;
+    }
+  }
+  // unit `it` of this worker: tile, K steps [ks0, ks1), slice (always 0 for whole tiles); false past the last unit
+  __host__ __device__ __forceinline__ bool get(int64_t it, int64_t* tile, int* ks0, int* ks1, int* slice) const {
+    *ks0 = 0;
+    *ks1 = k_steps;
+    *slice = 0;
+    if (S == 1 || it < rounds - 1) {
+      *tile = b + it * grid;
+      return *tile < total;
+    }
+    if (it > rounds - 1 || b >= left * S) return false;
+    *tile = (rounds - 1) * grid + b / S;
+    *slice = b % S;
+    *ks0 = (int)((int64_t)k_steps * *slice / S);
+    *ks1 = (int)((int64_t)k_steps * (*slice + 1) / S);
+    return true;
+  }
+  __host__ __device__ __forceinline__ bool is_split(int64_t it) const { return S > 1 && it == rounds - 1; }
+};
+
+// TMA maps (gemm_pair.cu)
+int pair_map_tokens(CUtensorMap* map, const void* base, int64_t rows, int64_t cols, int elem_bytes, int box_rows);
+int pair_map_weights(CUtensorMap* map, const void* base, int64_t experts, int64_t n, int64_t k, int elem_bytes, bool gated);
+int pair_map_weights_nmajor(CUtensorMap* map, const void* base, int64_t experts, int64_t k, int64_t w_rows);
+int device_sm_count();
+
+}  // namespace fmoe

@@ -2,7 +2,7 @@
 //   fmoe_quant_fp8_group128 : per-row, per-128-channel e4m3 quantisation (+ optional row gather)
 //   fmoe_gather_rows        : copy rows into the padded expert-sorted order
 //   fmoe_moe_sum            : out[t] = sum_j z[t,j], optional post-scale
-#include "common.cuh"
+#include "rows.cuh"
 
 namespace fmoe {
 namespace {
@@ -207,11 +207,12 @@ quant_row_kernel(const __nv_bfloat16* __restrict__ x, int64_t rows_out, int64_t 
 __global__ void __launch_bounds__(256)
 gather_rows_kernel(const uint4* __restrict__ x, int64_t rows_out, int64_t vec_per_row,
                    const int32_t* __restrict__ row_map, int map_div, int64_t sentinel,
-                   const int32_t* __restrict__ num_rows_dev, uint4* __restrict__ out) {
+                   const int32_t* __restrict__ num_rows_dev, uint4* __restrict__ out, int zero_padding) {
   pdl_entry();
   const int64_t limit = num_rows_dev ? min((int64_t)*num_rows_dev, rows_out) : rows_out;
   for (int64_t p = blockIdx.x; p < limit; p += gridDim.x) {
     const int64_t r = mapped_row(row_map, map_div, sentinel, p);
+    if (r < 0 && !zero_padding) continue;
     for (int64_t c = threadIdx.x; c < vec_per_row; c += blockDim.x)
       out[p * vec_per_row + c] = (r >= 0) ? __ldg(x + r * vec_per_row + c) : make_uint4(0, 0, 0, 0);
   }
@@ -302,19 +303,24 @@ extern "C" int fmoe_quant_fp8_per_token(const void* x, int in_dtype, int64_t row
   return launch_status("quant_row_kernel");
 }
 
-extern "C" int fmoe_gather_rows(const void* x, int elem_bytes, int64_t rows_out, int64_t K,
-                                const int32_t* row_map, int map_div, int64_t map_sentinel,
-                                const int32_t* num_rows_dev, void* out, void* stream) {
-  using namespace fmoe;
+int fmoe::run_gather_rows(const void* x, int elem_bytes, int64_t rows_out, int64_t K, const int32_t* row_map, int map_div,
+                          int64_t map_sentinel, const int32_t* num_rows_dev, void* out, bool zero_padding, cudaStream_t st) {
   FMOE_REQUIRE(elem_bytes == 2 || elem_bytes == 4 || elem_bytes == 1, "gather_rows: elem_bytes must be 1, 2 or 4");
   FMOE_REQUIRE(K > 0 && (K * elem_bytes) % 16 == 0, "gather_rows: row size must be a multiple of 16 bytes");
   FMOE_REQUIRE(row_map && map_div >= 1, "gather_rows: row_map required");
   if (rows_out <= 0) return FMOE_OK;
   FMOE_REQUIRE(x && out && aligned16(x) && aligned16(out), "gather_rows: null or misaligned pointer");
   unsigned grid = (unsigned)std::min<int64_t>(rows_out, 148 * 8);
-  launch_pdl(gather_rows_kernel, dim3(grid), dim3(256), 0, (cudaStream_t)stream, (const uint4*)x, rows_out,
-             K * elem_bytes / 16, row_map, map_div, map_sentinel, num_rows_dev, (uint4*)out);
+  launch_pdl(gather_rows_kernel, dim3(grid), dim3(256), 0, st, (const uint4*)x, rows_out, K * elem_bytes / 16, row_map,
+             map_div, map_sentinel, num_rows_dev, (uint4*)out, (int)zero_padding);
   return launch_status("gather_rows_kernel");
+}
+
+extern "C" int fmoe_gather_rows(const void* x, int elem_bytes, int64_t rows_out, int64_t K,
+                                const int32_t* row_map, int map_div, int64_t map_sentinel,
+                                const int32_t* num_rows_dev, void* out, void* stream) {
+  return fmoe::run_gather_rows(x, elem_bytes, rows_out, K, row_map, map_div, map_sentinel, num_rows_dev, out, true,
+                               (cudaStream_t)stream);
 }
 
 extern "C" int fmoe_moe_sum(const void* z, int dtype, int64_t T, int k, int64_t H, float scale, void* out,
