@@ -7,7 +7,6 @@
 // far), which keeps slots of an expert in ascending order.  The ranks inside a
 // group of 32 slots come from __match_any_sync.
 #include "align.cuh"
-#include "pair.cuh"
 
 namespace fmoe {
 namespace {
@@ -18,12 +17,12 @@ constexpr int kWarps = kThreads / 32;
 // One warp: exclusive scan of the padded row counts -> s_start[E + 1] and num_post_pad; with `table`, also the experts'
 // first rows, rows and token tiles for the CTA-pair GEMMs (pair.cuh).  E <= 1024: 32 experts per step.
 __device__ __forceinline__ void scan_experts_warp(const int* s_total, int* s_start, int E, int block, int lane,
-                                                  int32_t* num_post_pad, int32_t* table) {
+                                                  int32_t* num_post_pad, int32_t* table, int token_tile) {
   int carry = 0, tile_carry = 0;
   for (int base = 0; base < E; base += 32) {
     const int e = base + lane;
     const int rows = (e < E) ? s_total[e] : 0;
-    const int padded = ceil_div(rows, block) * block, tiles = ceil_div(rows, kPairTokens);
+    const int padded = ceil_div(rows, block) * block, tiles = ceil_div(rows, token_tile);
     int incl = padded, tile_incl = tiles;
 #pragma unroll
     for (int off = 1; off < 32; off <<= 1) {
@@ -54,7 +53,7 @@ __device__ __forceinline__ void scan_experts_warp(const int* s_total, int* s_sta
 __global__ void __launch_bounds__(kThreads)
 moe_align_kernel(const int32_t* __restrict__ topk_ids, int numel, int E, int block,
                  int32_t* __restrict__ sorted_ids, int sorted_cap, int32_t* __restrict__ expert_ids,
-                 int expert_cap, int32_t* __restrict__ num_post_pad, int32_t* __restrict__ table,
+                 int expert_cap, int32_t* __restrict__ num_post_pad, int32_t* __restrict__ table, int token_tile,
                  int32_t* __restrict__ zero_words, int num_zero) {
   pdl_entry();
   extern __shared__ int s_mem[];
@@ -94,7 +93,7 @@ moe_align_kernel(const int32_t* __restrict__ topk_ids, int numel, int E, int blo
   }
   __syncthreads();
 
-  if (warp == 0) scan_experts_warp(s_total, s_start, E, block, lane, num_post_pad, table);
+  if (warp == 0) scan_experts_warp(s_total, s_start, E, block, lane, num_post_pad, table, token_tile);
   __syncthreads();
 
   // block -> expert map (-1 after the used blocks)
@@ -151,7 +150,7 @@ align_count_kernel(const int32_t* __restrict__ topk_ids, int numel, int E, int32
 
 __global__ void __launch_bounds__(kThreads)
 align_scan_kernel(int chunks, int E, int block, int32_t* __restrict__ cnt, int32_t* __restrict__ expert_ids,
-                  int expert_cap, int32_t* __restrict__ num_post_pad, int32_t* __restrict__ table,
+                  int expert_cap, int32_t* __restrict__ num_post_pad, int32_t* __restrict__ table, int token_tile,
                   int32_t* __restrict__ zero_words, int num_zero) {
   extern __shared__ int s_mem[];
   int* s_total = s_mem;      // [E]
@@ -168,7 +167,7 @@ align_scan_kernel(int chunks, int E, int block, int32_t* __restrict__ cnt, int32
     s_total[e] = run;
   }
   __syncthreads();
-  if (warp == 0) scan_experts_warp(s_total, s_start, E, block, lane, num_post_pad, table);
+  if (warp == 0) scan_experts_warp(s_total, s_start, E, block, lane, num_post_pad, table, token_tile);
   __syncthreads();
   const int used_blocks = s_start[E] / block;
   for (int e = tid; e < E; e += kThreads) {
@@ -250,7 +249,7 @@ int run_align(const AlignArgs& a, cudaStream_t st) {
     if (smem > 48 * 1024)
       FMOE_CUDA_OK(cudaFuncSetAttribute(moe_align_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
     launch_pdl(moe_align_kernel, dim3(1), dim3(kThreads), smem, st, a.topk_ids, (int)a.numel, a.E, a.block, a.sorted_ids,
-               (int)a.sorted_cap, a.expert_ids, (int)a.expert_cap, a.num_post_pad, a.table, a.zero_words, a.num_zero);
+               (int)a.sorted_cap, a.expert_ids, (int)a.expert_cap, a.num_post_pad, a.table, a.token_tile, a.zero_words, a.num_zero);
     return launch_status("moe_align_kernel");
   }
   FMOE_REQUIRE(a.workspace_bytes >= fmoe_moe_align_workspace_bytes(a.numel, a.E), "moe_align_block_size: workspace too small");
@@ -260,7 +259,7 @@ int run_align(const AlignArgs& a, cudaStream_t st) {
   rc = launch_status("align_count_kernel");
   if (rc) return rc;
   align_scan_kernel<<<1, kThreads, (2 * a.E + 1) * sizeof(int), st>>>(chunks, a.E, a.block, cnt, a.expert_ids, (int)a.expert_cap,
-                                                                     a.num_post_pad, a.table, a.zero_words, a.num_zero);
+                                                                     a.num_post_pad, a.table, a.token_tile, a.zero_words, a.num_zero);
   rc = launch_status("align_scan_kernel");
   if (rc) return rc;
   const size_t smem = (size_t)kWarps * a.E * sizeof(int);

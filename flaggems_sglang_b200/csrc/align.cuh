@@ -15,7 +15,8 @@ struct AlignArgs {
   int32_t* num_post_pad = nullptr;
   void* workspace = nullptr;  // scratch of the multi-CTA variant (NULL: single CTA)
   int64_t workspace_bytes = 0;
-  int32_t* table = nullptr;       // optional: expert table of the CTA-pair GEMMs (pair.cuh)
+  int32_t* table = nullptr;       // optional: expert table of the CTA-pair GEMMs (pair.cuh), for tiles of
+  int token_tile = 256;           //   at most this many tokens
   int32_t* zero_words = nullptr;  // optional: counters of later kernels, set to zero
   int num_zero = 0;
 };

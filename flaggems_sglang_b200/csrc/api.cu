@@ -87,7 +87,7 @@ int run_gemm(const GemmParams& a, bool gated, cudaStream_t st) {
   if (a.w_layout == FMOE_W_N_MAJOR || (a.dtype == FMOE_E4M3 && a.scale_mode == FMOE_SCALE_CHANNEL)) {
     variant = FMOE_VARIANT_TCGEN05;
   } else if (variant == FMOE_VARIANT_AUTO) {
-    if (gemm_pair_supports(a, gated) || gemm_tcgen05_fp8_supports(a, gated))
+    if (gemm_pair_supports(a, gated) || gemm_pair_fold_supports(a, gated))
       variant = FMOE_VARIANT_TCGEN05;
     else if (gemm_stream_supports(a, gated))
       variant = FMOE_VARIANT_STREAM;
@@ -98,7 +98,7 @@ int run_gemm(const GemmParams& a, bool gated, cudaStream_t st) {
     case FMOE_VARIANT_SIMT: return gemm_simt(a, gated, st);
     case FMOE_VARIANT_STREAM: return gemm_stream(a, gated, st);
     case FMOE_VARIANT_TCGEN05:
-      return (a.dtype == FMOE_E4M3 && a.scale_mode == FMOE_SCALE_BLOCK128) ? gemm_tcgen05_fp8(a, gated, st)
+      return (a.dtype == FMOE_E4M3 && a.scale_mode == FMOE_SCALE_BLOCK128) ? gemm_pair_fold(a, gated, st)
                                                                            : gemm_pair(a, gated, st);
   }
   return fail(FMOE_ERR_INVALID_ARG, "%s: unknown variant %d", who, a.variant);

@@ -23,21 +23,20 @@ int pick_variant(int dtype, int64_t numel, int E, int64_t I, int64_t H, int forc
   // bf16: the tensor-core kernels cut their last column tile / zero-fill their last K step, the streaming kernel
   // masks its last 128-k chunk, so sizes such as 2880 (GPT-OSS) stay off the plain CUDA-core kernel
   const bool stream_ok = dtype == FMOE_BF16 ? (H % 16 == 0 && I % 16 == 0) : (H % 128 == 0 && I % 128 == 0);
-  // e4m3: a tile's block scales are staged in shared memory, which bounds the reduction length at 8192
   const bool tc_ok = dtype == FMOE_BF16 ? (I % 32 == 0 && H % 32 == 0)
-                                        : (I % 128 == 0 && H % 128 == 0 && I <= 8192 && H <= 8192);
+                                        : (I % 128 == 0 && H % 128 == 0);
   int v = forced;
   if (v == FMOE_VARIANT_AUTO) {
     // measured on B200: up to 4 rows per expert the two families tie (both stream the weights once at ~90 % of
     // HBM bandwidth) and the streaming kernel wins on tile quantisation for a handful of experts; above that the
     // 128-row tensor-core tiles win (DeepSeek-V3 T=256: 1.49 against 2.11 ms)
-    if (stream_ok && (rows <= 4.0 || !tc_ok)) v = FMOE_VARIANT_STREAM;
+    if (stream_ok && ((dtype == FMOE_BF16 ? rows <= 4.0 : rows < 4.0) || !tc_ok)) v = FMOE_VARIANT_STREAM;
     else if (tc_ok) v = FMOE_VARIANT_TCGEN05;
     else v = FMOE_VARIANT_SIMT;
   }
   switch (v) {
     case FMOE_VARIANT_TCGEN05:
-      if (!tc_ok) return fail(FMOE_ERR_UNSUPPORTED, "tcgen05 kernels need I %% 32 == 0 and H %% 32 == 0 (e4m3: multiples of 128, up to 8192)");
+      if (!tc_ok) return fail(FMOE_ERR_UNSUPPORTED, "tcgen05 kernels need I %% 32 == 0 and H %% 32 == 0 (e4m3: multiples of 128)");
       *block = 128;
       break;
     case FMOE_VARIANT_STREAM:
@@ -241,6 +240,8 @@ int run_fused(const fmoe_fused_args& a, const FusedPlan& p, uint8_t* ws, void* s
   al.workspace = ws + p.off_align_ws;
   al.workspace_bytes = p.align_ws_bytes;
   al.table = table;
+  const bool fold = fp8 && a.scale_mode == FMOE_SCALE_BLOCK128;
+  al.token_tile = fold ? pick_fold_token_tile(p.numel, a.num_experts) : pick_token_tile(p.numel, a.num_experts);
   al.zero_words = counters;
   al.num_zero = counters ? 2 * kSplitCounters : 0;
   int rc = run_align(al, st);
@@ -267,6 +268,7 @@ int run_fused(const fmoe_fused_args& a, const FusedPlan& p, uint8_t* ws, void* s
     g.split_ws_bytes = p.split_bytes;
   }
   g.expert_table = table;
+  g.token_tile = al.token_tile;
   g.skip_padding = true;  // nothing below reads a padding row's values
   GemmParams g1 = g, g2 = g;
   g1.split_counters = counters;
@@ -326,9 +328,9 @@ int run_fused(const fmoe_fused_args& a, const FusedPlan& p, uint8_t* ws, void* s
       float* xtsc = reinterpret_cast<float*>(ws + p.off_xt_scale);
       rc = fmoe_quant_fp8_group128(a.hidden, FMOE_BF16, a.T, a.H, nullptr, 1, 0, nullptr, xt, xtsc, stream);
       if (rc) return rc;
-      rc = fmoe_gather_rows(xt, 1, p.cap, a.H, sorted, a.top_k, p.numel, npp, xq, stream);
-      if (rc) return rc;
-      rc = fmoe_gather_rows(xtsc, 4, p.cap, a.H / 128, sorted, a.top_k, p.numel, npp, xsc, stream);
+      rc = run_gather_rows(xt, 1, p.cap, a.H, sorted, a.top_k, p.numel, npp, xq, false, st);
+      xsc = xtsc;  // the gate/up GEMM looks the scales up by token
+      g1.a_scale_gather = 1;
     } else if (tc)
       rc = fmoe_quant_fp8_group128(a.hidden, FMOE_BF16, p.cap, a.H, sorted, a.top_k, p.numel, npp, xq, xsc, stream);
     else

@@ -13,10 +13,10 @@ struct FusedPlan {
   int64_t off_table, off_counters;  // expert table and tail-split counters of the CTA-pair GEMMs
 };
 
-// e4m3 with the tcgen05 kernels: quantise each token row once ([T,H]) and copy bytes and scales into the sorted
-// order, instead of quantising every one of the T*top_k sorted rows (the quantiser is division-bound, the copy is
-// not).  The scale rows must be a multiple of 16 bytes for the copy kernel.
-inline bool fp8_quant_once(int64_t top_k, int64_t H) { return top_k >= 2 && H % 512 == 0; }
+// e4m3 with the tcgen05 kernels: quantise each token row once ([T,H]) and copy the bytes into the sorted order, instead
+// of quantising every one of the T*top_k sorted rows (the quantiser is division-bound, the copy is not); the GEMM finds
+// the scales by token.
+inline bool fp8_quant_once(int64_t top_k, int64_t) { return top_k >= 2; }
 
 int pick_variant(int dtype, int64_t numel, int E, int64_t I, int64_t H, int forced, int* variant, int* block);
 int plan_fused(const fmoe_fused_args& a, FusedPlan* plan);

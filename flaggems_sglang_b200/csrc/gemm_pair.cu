@@ -1,9 +1,9 @@
 // Grouped GEMM on CTA pairs (cluster of 2, tcgen05 cta_group::2) for bf16 operands, and for e4m3 operands with one scale
 // per token and one per output channel.
 //
-//   tile      : 256 weight rows (M, 128 in each CTA) x up to 256 tokens of one expert (N, half of them loaded by each CTA)
+//   tile      : 256 weight rows (M, 128 in each CTA) x up to 64, 128 or 256 tokens of one expert (N, half loaded by each CTA)
 //   K step    : 128 bytes per row (64 bf16 / 128 e4m3), one 128-byte swizzle atom; 4 MMAs per step
-//   pipeline  : 6 shared-memory stages of 16 KB of weights + at most 16 KB of tokens per CTA
+//   pipeline  : 192 KB ring of 6, 8 or 9 stages (16 KB of weights + 16, 8 or 4 KB of tokens) per CTA
 //   TMEM      : 512 columns per CTA = two 128 x 256 fp32 accumulators, so the epilogue of a tile overlaps the next tile
 //   warps     : 0-7 epilogue (TMEM lane quarter = warp % 4; the two halves take alternate 16-token chunks),
 //               8 TMA producer (each CTA its own weight rows and its own half of the tokens), 9 MMA issuer (CTA 0)
@@ -36,10 +36,10 @@ __device__ long long g_wait_prof[256 * 8];
 namespace {
 
 constexpr int KBYTES = 128;
-constexpr int STAGES = 6;
 constexpr int W_BYTES = 128 * KBYTES;               // this CTA's weight rows of a stage
-constexpr int T_BYTES = kPairTokens / 2 * KBYTES;   // this CTA's half of the tokens
-constexpr int STAGE_BYTES = W_BYTES + T_BYTES;
+constexpr int RING_BYTES = 6 * 32 * 1024;           // stages of 16 KB of weights + half a token tile
+constexpr int MAX_STAGES = 9;
+constexpr int stage_bytes(int token_tile) { return W_BYTES + token_tile / 2 * KBYTES; }
 constexpr int TMEM_COLS = 512;
 constexpr int ACC_COLS = 256;
 constexpr int kEpiWarps = 8;
@@ -50,7 +50,7 @@ constexpr int EX_PITCH = 20;                        // floats per lane row of th
 constexpr int EX_BYTES = 128 * EX_PITCH * 4;        // per half of the epilogue warps
 constexpr int BAR_BYTES = 256;
 constexpr int smem_bytes(int num_experts, bool exchange) {
-  return 1024 + STAGES * STAGE_BYTES + BAR_BYTES + (exchange ? 2 * EX_BYTES : kEpiWarps * STRIP_BYTES) + pair_table_bytes(num_experts);
+  return RING_BYTES + BAR_BYTES + (exchange ? 2 * EX_BYTES : kEpiWarps * STRIP_BYTES) + pair_table_bytes(num_experts);
 }
 static_assert(smem_bytes(1024, true) <= 227 * 1024, "shared memory");
 
@@ -82,6 +82,8 @@ struct PairParams {
   int32_t split_max;      // tail split: most K slices per tile (< 2: no split)
   int32_t top_k;
   int32_t a_rows;         // gather mode: rows of the input tensor (a row index >= a_rows reads zeros)
+  int32_t token_tile;     // most tokens per tile
+  int32_t stages, stage_bytes;
   int32_t zero_padding;   // gemm1: rows between an expert's last token and its block's end are written as zeros
 };
 
@@ -101,15 +103,15 @@ template <bool GATED, bool F8, bool EXTRA, bool WMN, bool GATHER>
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 1)
 grouped_gemm_pair_kernel(const __grid_constant__ CUtensorMap map_t, const __grid_constant__ CUtensorMap map_w,
                          const PairParams p) {
-  extern __shared__ uint8_t smem_raw[];
-  uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
-  uint64_t* bars = reinterpret_cast<uint64_t*>(smem + STAGES * STAGE_BYTES);
-  uint64_t* full_bar = bars;                    // [STAGES] used in CTA 0: the bytes of both CTAs' loads -> MMA
-  uint64_t* empty_bar = bars + STAGES;          // [STAGES] per CTA: MMA -> this CTA's producer
-  uint64_t* acc_full = bars + 2 * STAGES;       // [2] per CTA: MMA -> this CTA's epilogue
-  uint64_t* acc_empty = bars + 2 * STAGES + 2;  // [2] used in CTA 0: both epilogues -> MMA
-  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 2 * STAGES + 4);
-  uint8_t* strips = smem + STAGES * STAGE_BYTES + BAR_BYTES;
+  extern __shared__ __align__(1024) uint8_t smem[];  // aligned by declaration: every address below is a constant
+  const int stages = p.stages, stage_size = p.stage_bytes;
+  uint64_t* bars = reinterpret_cast<uint64_t*>(smem + RING_BYTES);
+  uint64_t* full_bar = bars;                    // [stages] used in CTA 0: the bytes of both CTAs' loads -> MMA
+  uint64_t* empty_bar = bars + MAX_STAGES;          // [stages] per CTA: MMA -> this CTA's producer
+  uint64_t* acc_full = bars + 2 * MAX_STAGES;       // [2] per CTA: MMA -> this CTA's epilogue
+  uint64_t* acc_empty = bars + 2 * MAX_STAGES + 2;  // [2] used in CTA 0: both epilogues -> MMA
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 2 * MAX_STAGES + 4);
+  uint8_t* strips = smem + RING_BYTES + BAR_BYTES;
   int32_t* table = reinterpret_cast<int32_t*>(strips + (GATED && WMN ? 2 * EX_BYTES : kEpiWarps * STRIP_BYTES));
 
   const int warp = ptx::uniform_warp_id(), lane = threadIdx.x & 31;
@@ -117,7 +119,7 @@ grouped_gemm_pair_kernel(const __grid_constant__ CUtensorMap map_t, const __grid
   const int worker = blockIdx.x >> 1, workers = gridDim.x >> 1;
 
   if (threadIdx.x == 0) {
-    for (int s = 0; s < STAGES; ++s) {
+    for (int s = 0; s < stages; ++s) {
       ptx::mbar_init(&full_bar[s], 1);   // CTA 0's producer arms it with the bytes of both CTAs
       ptx::mbar_init(&empty_bar[s], 1);  // one tcgen05.commit
     }
@@ -138,7 +140,8 @@ grouped_gemm_pair_kernel(const __grid_constant__ CUtensorMap map_t, const __grid
   ptx::tc_fence_before_sync();
   pdl_entry();  // everything above is independent of the kernels before this one on the stream
   const int used_blocks = min((int)(*p.num_tokens_post_padded / 128), p.max_blocks);
-  pair_build_table(table, p.num_experts, p.expert_table, p.expert_ids, p.sorted_token_ids, p.numel, 128, used_blocks);
+  pair_build_table(table, p.num_experts, p.expert_table, p.expert_ids, p.sorted_token_ids, p.numel, 128,
+                   p.token_tile, used_blocks);
   ptx::cluster_sync_all();  // the other CTA's barriers exist before anything is signalled across
   ptx::tc_fence_after_sync();
   const uint32_t tmem_base = *tmem_slot;
@@ -175,7 +178,7 @@ grouped_gemm_pair_kernel(const __grid_constant__ CUtensorMap map_t, const __grid
             alive = false;
             break;
           }
-          const uint32_t sw = ring + stage * STAGE_BYTES, stok = sw + W_BYTES, bar0 = bar_full0 + stage * 8;
+          const uint32_t sw = ring + stage * stage_size, stok = sw + W_BYTES, bar0 = bar_full0 + stage * 8;
           const int32_t x = ks * (KBYTES / (F8 ? 1 : 2));  // element coordinate along K
           if (rank == 0) ptx::mbar_arrive_expect_tx(&full_bar[stage], 2 * (W_BYTES + t_bytes));
           if constexpr (WMN) {
@@ -196,7 +199,7 @@ grouped_gemm_pair_kernel(const __grid_constant__ CUtensorMap map_t, const __grid
             for (int b = 0; b < boxes; ++b)
               ptx::tma_load_2d_pair(stok + b * (BOX_TOKENS * KBYTES), &map_t, x, row_t + b * BOX_TOKENS, bar0);
           }
-          if (++stage == STAGES) {
+          if (++stage == stages) {
             stage = 0;
             phase ^= 1;
           }
@@ -204,12 +207,12 @@ grouped_gemm_pair_kernel(const __grid_constant__ CUtensorMap map_t, const __grid
       }
       if (p.profile && blockIdx.x < 256) g_wait_prof[blockIdx.x * 8 + 3] = prof_p;
       if (alive) {  // drain: every stage this CTA filled has been consumed before the CTA may end
-        for (int s = 0; s < STAGES; ++s) {
+        for (int s = 0; s < stages; ++s) {
           if (!ptx::mbar_wait(&empty_bar[stage], phase ^ 1)) {
             report(0x180 | stage);
             break;
           }
-          if (++stage == STAGES) {
+          if (++stage == stages) {
             stage = 0;
             phase ^= 1;
           }
@@ -258,14 +261,14 @@ grouped_gemm_pair_kernel(const __grid_constant__ CUtensorMap map_t, const __grid
             break;
           }
           ptx::tc_fence_after_sync();
-          const uint64_t da = da0 + (uint64_t)(stage * (STAGE_BYTES >> 4)), db = db0 + (uint64_t)(stage * (STAGE_BYTES >> 4));
+          const uint64_t da = da0 + (uint64_t)(stage * (stage_size >> 4)), db = db0 + (uint64_t)(stage * (stage_size >> 4));
 #pragma unroll
           for (int kk = 0; kk < KBYTES / 32; ++kk) {
             if constexpr (F8) ptx::mma_f8f6f4_ss_pair(d_tmem, da + a_step * kk, db + 2 * kk, idesc, ((ks - ks0) | kk) != 0);
             else ptx::mma_f16_ss_pair(d_tmem, da + a_step * kk, db + 2 * kk, idesc, ((ks - ks0) | kk) != 0);
           }
           ptx::mma_commit_both(&empty_bar[stage]);  // the stage is free in both CTAs once these MMAs have read it
-          if (++stage == STAGES) {
+          if (++stage == stages) {
             stage = 0;
             phase ^= 1;
           }
@@ -614,14 +617,6 @@ int pair_map_tokens(CUtensorMap* map, const void* base, int64_t rows, int64_t co
   return encode(map, base, elem_bytes, 2, dims, strides, box, false, "tokens");
 }
 
-int make_tensor_map_2d(CUtensorMap* map, const void* base, int64_t rows, int64_t cols, int elem_bytes, int box_rows,
-                       bool weights, int kbytes) {
-  const cuuint64_t dims[2] = {(cuuint64_t)cols, (cuuint64_t)rows};
-  const cuuint64_t strides[1] = {(cuuint64_t)cols * elem_bytes};
-  const cuuint32_t box[2] = {(cuuint32_t)(kbytes / elem_bytes), (cuuint32_t)box_rows};
-  return encode(map, base, elem_bytes, 2, dims, strides, box, weights, "2d");
-}
-
 // weights [E, rows, K], K contiguous.  gated: rows = n gate rows then n up rows; the box takes 4 groups of 16 gate rows and
 // the 16 matching up rows (K, 16 rows, gate/up, row groups, expert: rows past n read as zeros).  plain: rows = n, 128 rows.
 int pair_map_weights(CUtensorMap* map, const void* base, int64_t experts, int64_t n, int64_t k, int elem_bytes, bool gated) {
@@ -694,11 +689,14 @@ int launch(const GemmParams& g, cudaStream_t st) {
   p.top_k = g.top_k;
   p.a_rows = (int32_t)g.a_rows;
   p.zero_padding = !g.skip_padding;
-  p.group = pick_group_m(kPairTokens, g.k * ELEM);
+  p.token_tile = g.token_tile ? g.token_tile : pick_token_tile(g.numel, g.num_experts);
+  p.stage_bytes = stage_bytes(p.token_tile);
+  p.stages = std::min(RING_BYTES / p.stage_bytes, MAX_STAGES);
+  p.group = pick_group_m(p.token_tile, g.k * ELEM);
   static const bool profile = getenv("FMOE_TC_PROFILE") != nullptr;
   p.profile = profile;
 
-  const int64_t max_tiles = g.max_blocks * p.w_tiles;  // an expert has no more 256-token tiles than 128-row blocks
+  const int64_t max_tiles = g.max_blocks * ceil_div(128, p.token_tile) * p.w_tiles;
   const int sms = device_sm_count();
   const int workers = (int)std::max<int64_t>(1, std::min<int64_t>((sms > 0 ? sms : 148) / 2, max_tiles));
   p.split_partials = nullptr;

@@ -1,0 +1,1004 @@
+// Grouped GEMM on CTA pairs for e4m3 operands with 128x128 weight scales and 1x128 activation scales.
+//
+// tcgen05 accumulates in fp32 inside TMEM and cannot apply a different scale to every 128-wide K block, so every K block
+// (128 bytes = 128 e4m3 = one scale block) is multiplied into a FRESH TMEM partial (4 MMAs of K = 32, the first one
+// overwriting), and the fold warps add it into register accumulators:
+//     acc[channel, token] += partial[channel, token] * (a_scale[token, kb] * w_scale[channel / 128, kb])
+//
+// Two kernels: the narrow one (64-token tiles, few rows per expert) and the wide one (below).  The narrow one:
+//   tile      : 256 weight rows (128 per CTA) x up to 64 tokens of one expert, as in gemm_pair.cu (same tile order, same
+//               row interleave of gate and up, same transposed stores)
+//   TMEM      : 512 columns per CTA as eight partials of 64 tokens: the MMAs of the next K blocks run while one is folded
+//   warps 0-15: fold + epilogue.  Warp w reads TMEM lanes 32 * (w % 4).. and the 16-token piece w / 4.  16 x 256b read-out puts two tokens of one channel side by side, which is
+//               what the packed fma.rn.f32x2 takes with one pair of factors for two channels
+//   warp 16   : TMA producer      warp 17 : MMA issuer (CTA 0)
+//   warps 18-19: factors.  For four K blocks at a time they multiply the tokens' scales with the tile's one or two weight
+//               scales and leave the products in a 3-slot ring in shared memory, next to the tile's slots and row weights:
+//               the fold warps read one 8-byte pair per two tokens and keep no pointers
+// What bounds it: HBM (the weights stream through a 9-stage ring of 20 KB); the fold of a 64-token partial costs a warp
+// about 300 cycles from wait to hand-over, with eight partials in flight.
+#include "pair.cuh"
+
+#include <cstdlib>
+#include <type_traits>
+
+namespace fmoe {
+
+// This translation unit's status word (device code is not linked across files); read by status_word_fp8().
+__device__ int g_device_status_fp8 = 0;
+// Wait-time profile of the instrumented build of the kernel (FMOE_TC_PROFILE=1): per CTA
+// {tiles, fold waits for the MMAs, fold busy, fold waits for staged scales, epilogue, kernel cycles, MMA warp waits for a
+// partial, MMA warp waits for data};
+// [0]: down GEMM, [1]: gate/up GEMM
+__device__ long long g_wait_prof_fp8[2 * 256 * 8];
+
+namespace {
+
+constexpr int KBYTES = 128;
+constexpr int W_BYTES = 128 * KBYTES;
+constexpr int TMEM_COLS = 512;
+constexpr int kFoldWarps = 16;
+constexpr int kThreads = (kFoldWarps + 4) * 32;
+constexpr int BOX_TOKENS = 32;
+constexpr int SC_SLOTS = 4;                      // factor ring: slots of 4 K blocks
+constexpr int META_TILES = 8;                    // more than the SC_SLOTS tiles that the factor warps may be ahead of the fold
+constexpr int BAR_BYTES = 512;
+constexpr int kMaxSmem = 227 * 1024;
+// Geometry of the narrow kernel
+constexpr int TOK = 64;
+template <bool GATED>
+struct Geo {
+  static constexpr int STAGE_BYTES = W_BYTES + TOK / 2 * KBYTES;
+  static constexpr int STAGES = 9;
+  static constexpr int BUFS = TMEM_COLS / TOK;                 // TMEM partials
+  static constexpr int KB_BYTES = (GATED ? 2 : 1) * TOK * 4;   // factors of one K block
+  static constexpr int STRIP_BYTES = GATED ? 16 * 48 : 16 * 80;
+  static constexpr int FACTOR_BYTES = SC_SLOTS * 4 * KB_BYTES;
+  static constexpr int META_BYTES = GATED ? 0 : META_TILES * TOK * 8;  // slots and row weights of the tile's tokens
+  static constexpr int bytes(int num_experts) {
+    return STAGES * STAGE_BYTES + BAR_BYTES + kFoldWarps * STRIP_BYTES + FACTOR_BYTES + META_BYTES + pair_table_bytes(num_experts);
+  }
+};
+static_assert(Geo<true>::bytes(1024) <= kMaxSmem && Geo<false>::bytes(1024) <= kMaxSmem, "shared memory");
+
+struct FoldParams {
+  const int32_t* sorted_token_ids;
+  const int32_t* expert_ids;
+  const int32_t* num_tokens_post_padded;
+  const int32_t* expert_table;
+  const float* row_scale;
+  const float* a_scale;  // [a_rows, kblocks], or [tokens, kblocks] (a_scale_gather)
+  const float* w_scale;  // [E, w_rows/128, kblocks]
+  void* out;
+  void* const* out_rows;  // down projection: optional per-slot row addresses (may be peer memory)
+  int64_t numel;
+  int64_t n;
+  int64_t w_rows;
+  int32_t a_scale_gather;
+  int32_t top_k;
+  int32_t num_experts;
+  int32_t kblocks;
+  int32_t w_tiles;
+  int32_t max_blocks;
+  int32_t activation;
+  int32_t group;
+  int32_t zero_padding;
+};
+
+__device__ __forceinline__ void report(int code) { atomicCAS(&g_device_status_fp8, 0, code); }
+__device__ __forceinline__ bool warp_wait(uint64_t* bar, uint32_t parity) {
+  return __all_sync(0xffffffffu, ptx::mbar_wait(bar, parity));
+}
+
+// acc (two packed floats) += v * f, both lanes
+__device__ __forceinline__ void fma2(unsigned long long& acc, uint32_t v0, uint32_t v1, unsigned long long ff) {
+  unsigned long long v;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(v) : "r"(v0), "r"(v1));
+  asm("fma.rn.f32x2 %0, %1, %2, %0;" : "+l"(acc) : "l"(v), "l"(ff));
+}
+__device__ __forceinline__ float lds32(uint32_t addr) {
+  float v;
+  asm volatile("ld.shared.f32 %0, [%1];" : "=f"(v) : "r"(addr) : "memory");
+  return v;
+}
+__device__ __forceinline__ void unpack2(unsigned long long v, float& a, float& b) {
+  asm("mov.b64 {%0, %1}, %2;" : "=f"(a), "=f"(b) : "l"(v));
+}
+// weight of the tile's token u when top-k weights go to the gate/up GEMM
+__device__ __forceinline__ float row_weight(const FoldParams& p, const PairTile& tl, int u) {
+  const int32_t s = u < tl.cols ? p.sorted_token_ids[tl.row0 + u] : -1;
+  return (s >= 0 && s < p.numel) ? p.row_scale[s] : 1.0f;
+}
+__device__ __forceinline__ unsigned long long lds64(uint32_t addr) {
+  unsigned long long v;
+  asm volatile("ld.shared.b64 %0, [%1];" : "=l"(v) : "r"(addr) : "memory");
+  return v;
+}
+
+// PROF: instrumented build with wait-time counters (reading the clock is slow enough to distort the fold loop).
+template <bool GATED, bool PROF>
+__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 1)
+grouped_gemm_pair_fold_kernel(const __grid_constant__ CUtensorMap map_t, const __grid_constant__ CUtensorMap map_w,
+                              const FoldParams p) {
+  using G = Geo<GATED>;
+  constexpr int STAGES = G::STAGES, STAGE_BYTES = G::STAGE_BYTES, BUFS = G::BUFS, KB_BYTES = G::KB_BYTES;
+  extern __shared__ __align__(1024) uint8_t smem[];  // aligned by declaration: every address below is a constant
+  uint64_t* bars = reinterpret_cast<uint64_t*>(smem + STAGES * STAGE_BYTES);
+  uint64_t* full_bar = bars;                            // [STAGES] used in CTA 0: both CTAs' loads -> MMA
+  uint64_t* empty_bar = bars + STAGES;              // [STAGES] per CTA: MMA -> producer
+  uint64_t* part_full = bars + 2 * STAGES;          // [bufs] per CTA: MMA -> fold
+  uint64_t* part_empty = part_full + BUFS;              // [bufs] used in CTA 0: folds of both CTAs -> MMA
+  uint64_t* sc_full = part_empty + BUFS;                // [slots] factor warps -> fold
+  uint64_t* sc_empty = sc_full + SC_SLOTS;              // [slots] fold -> factor warps
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(sc_empty + SC_SLOTS);
+  uint8_t* strips = smem + STAGES * STAGE_BYTES + BAR_BYTES;
+  uint8_t* factors = strips + kFoldWarps * G::STRIP_BYTES;                      // [slot][K block][gate | up][token]
+  int32_t* meta = reinterpret_cast<int32_t*>(factors + G::FACTOR_BYTES);        // [tile][slot ids | row weights]
+  int32_t* table = reinterpret_cast<int32_t*>(factors + G::FACTOR_BYTES + G::META_BYTES);
+
+  const int warp = ptx::uniform_warp_id(), lane = threadIdx.x & 31;
+  const int rank = (int)ptx::cluster_ctarank();
+  const int worker = blockIdx.x >> 1, workers = gridDim.x >> 1;
+  const long long t_kernel0 = PROF ? clock64() : 0;
+
+  if (threadIdx.x == 0) {
+    for (int s = 0; s < STAGES; ++s) {
+      ptx::mbar_init(&full_bar[s], 1);
+      ptx::mbar_init(&empty_bar[s], 1);
+    }
+    for (int b = 0; b < BUFS; ++b) {
+      ptx::mbar_init(&part_full[b], 1);
+      ptx::mbar_init(&part_empty[b], 2 * kFoldWarps);  // one arrival per fold warp of both CTAs
+    }
+    for (int s = 0; s < SC_SLOTS; ++s) {
+      ptx::mbar_init(&sc_full[s], 1);
+      ptx::mbar_init(&sc_empty[s], kFoldWarps);
+    }
+    ptx::fence_barrier_init();
+  }
+  if (warp == kFoldWarps && lane == 0) {
+    ptx::prefetch_tensormap(&map_t);
+    ptx::prefetch_tensormap(&map_w);
+  }
+  if (warp == kFoldWarps + 1) {
+    ptx::tmem_alloc_pair(tmem_slot, TMEM_COLS);
+    ptx::tmem_relinquish_pair();
+  }
+  ptx::tc_fence_before_sync();
+  pdl_entry();  // everything above is independent of the kernels before this one on the stream
+  const int used_blocks = min((int)(*p.num_tokens_post_padded / 128), p.max_blocks);
+  pair_build_table(table, p.num_experts, p.expert_table, p.expert_ids, p.sorted_token_ids, p.numel, 128, TOK,
+                   used_blocks);
+  ptx::cluster_sync_all();
+  ptx::tc_fence_after_sync();
+  const uint32_t tmem_base = *tmem_slot;
+  const int kblocks = p.kblocks;
+  const int total_tiles = table[3 * p.num_experts] * p.w_tiles;
+  PairCursor cursor;
+  PairTile tl;
+
+  if (warp == kFoldWarps) {
+    // ---------------- TMA producer (both CTAs) ----------------
+    if (ptx::elect_one()) {
+      int stage = 0;
+      uint32_t phase = 0;
+      bool alive = true;
+      const uint32_t ring = ptx::smem_u32(smem), bar_full0 = ptx::smem_u32(full_bar) & ~ptx::kPeerRankBit;
+      for (int tile = worker; tile < total_tiles && alive; tile += workers) {
+        cursor.locate(tile, p.w_tiles, p.group, p.num_experts, table, &tl);
+        const int half_n = tl.n >> 1;
+        const int row_t = tl.row0 + rank * half_n;
+        const int boxes = (half_n + BOX_TOKENS - 1) / BOX_TOKENS;
+        const uint32_t bytes = 2 * (W_BYTES + boxes * (BOX_TOKENS * KBYTES));
+        const int32_t c0 = GATED ? tl.w_tile * 128 + rank * 64 : tl.w_tile * 256 + rank * 128;
+        for (int kb = 0; kb < kblocks; ++kb) {
+          if (!ptx::mbar_wait(&empty_bar[stage], phase ^ 1)) {
+            report(0x500 | stage);
+            alive = false;
+            break;
+          }
+          const uint32_t sw = ring + stage * STAGE_BYTES, stok = sw + W_BYTES, bar0 = bar_full0 + stage * 8;
+          const int32_t x = kb * KBYTES;  // element coordinate (1-byte elements)
+          if (rank == 0) ptx::mbar_arrive_expect_tx(&full_bar[stage], bytes);
+          if constexpr (GATED) ptx::tma_load_5d_pair(sw, &map_w, x, 0, 0, c0 >> 4, tl.expert, bar0);
+          else ptx::tma_load_3d_pair(sw, &map_w, x, c0, tl.expert, bar0);
+          for (int b = 0; b < boxes; ++b)
+            ptx::tma_load_2d_pair(stok + b * (BOX_TOKENS * KBYTES), &map_t, x, row_t + b * BOX_TOKENS, bar0);
+          if (++stage == STAGES) {
+            stage = 0;
+            phase ^= 1;
+          }
+        }
+      }
+      if (alive) {  // drain our own bulk copies before leaving
+        for (int s = 0; s < STAGES; ++s) {
+          if (!ptx::mbar_wait(&empty_bar[stage], phase ^ 1)) {
+            report(0x580 | stage);
+            break;
+          }
+          if (++stage == STAGES) {
+            stage = 0;
+            phase ^= 1;
+          }
+        }
+      }
+    }
+  } else if (warp == kFoldWarps + 1) {
+    // ---------------- MMA issuer (CTA 0): one fresh partial per K block ----------------
+    if (rank == 0 && ptx::elect_one()) {
+      int stage = 0;
+      uint32_t phase = 0, step = 0;  // step: K blocks issued so far (selects the partial and its phase)
+      bool alive = true;
+      long long prof_mp = 0, prof_md = 0;
+      const uint32_t ring = ptx::smem_u32(smem);
+      const uint64_t da0 = ptx::smem_desc_sw128(ring), db0 = ptx::smem_desc_sw128(ring + W_BYTES);
+      for (int tile = worker; tile < total_tiles && alive; tile += workers) {
+        cursor.locate(tile, p.w_tiles, p.group, p.num_experts, table, &tl);
+        const uint32_t idesc = ptx::make_idesc(/*e4m3*/ 0, 256, (uint32_t)tl.n);
+        for (int kb = 0; kb < kblocks; ++kb, ++step) {
+          const int buf = step % BUFS;
+          const long long tm0 = PROF ? clock64() : 0;
+          if (!ptx::mbar_wait(&part_empty[buf], ((step / BUFS) & 1) ^ 1)) {
+            report(0x600 | buf);
+            alive = false;
+            break;
+          }
+          const long long tm1 = PROF ? clock64() : 0;
+          if (!ptx::mbar_wait(&full_bar[stage], phase)) {
+            report(0x640 | stage);
+            alive = false;
+            break;
+          }
+          if (PROF) {
+            prof_mp += tm1 - tm0;
+            prof_md += clock64() - tm1;
+          }
+          ptx::tc_fence_after_sync();
+          const uint64_t da = da0 + (uint64_t)(stage * (STAGE_BYTES >> 4)), db = db0 + (uint64_t)(stage * (STAGE_BYTES >> 4));
+          const uint32_t d_tmem = tmem_base + buf * TOK;
+#pragma unroll
+          for (int kk = 0; kk < KBYTES / 32; ++kk)
+            ptx::mma_f8f6f4_ss_pair(d_tmem, da + 2 * kk, db + 2 * kk, idesc, kk != 0);
+          ptx::mma_commit_both(&part_full[buf]);
+          ptx::mma_commit_both(&empty_bar[stage]);
+          if (++stage == STAGES) {
+            stage = 0;
+            phase ^= 1;
+          }
+        }
+      }
+      if (PROF && blockIdx.x < 256) {
+        g_wait_prof_fp8[(GATED ? 2048 : 0) + blockIdx.x * 8 + 6] = prof_mp;
+        g_wait_prof_fp8[(GATED ? 2048 : 0) + blockIdx.x * 8 + 7] = prof_md;
+      }
+    }
+  } else if (warp >= kFoldWarps + 2) {
+    // ---------------- factors: two warps take alternate groups of four K blocks, one tile after the other ----------------
+    constexpr int LANES = TOK / 32;  // tokens per lane
+    const int me = warp - (kFoldWarps + 2);
+    uint32_t group = 0;  // groups so far (selects the slot and its phase)
+    bool alive = true;
+    int ltile = 0;
+    const bool vec = (kblocks & 3) == 0 && aligned16(p.a_scale) && aligned16(p.w_scale);
+    const int wblocks = (int)(p.w_rows / 128);
+    for (int tile = worker; tile < total_tiles && alive; tile += workers, ++ltile) {
+      cursor.locate(tile, p.w_tiles, p.group, p.num_experts, table, &tl);
+      int32_t ids[LANES], row[LANES];  // slot and scale row of token lane + 32 j
+#pragma unroll
+      for (int j = 0; j < LANES; ++j) {
+        const int u = lane + 32 * j;
+        ids[j] = u < tl.cols ? p.sorted_token_ids[tl.row0 + u] : -1;
+      }
+#pragma unroll
+      for (int j = 0; j < LANES; ++j) {
+        if (ids[j] >= p.numel) ids[j] = -1;
+        row[j] = ids[j] < 0 ? 0 : (p.a_scale_gather ? ids[j] / p.top_k : tl.row0 + lane + 32 * j);
+      }
+      const int w0 = GATED ? tl.w_tile : min(tl.w_tile * 2 + rank, wblocks - 1), w1 = GATED ? tl.w_tile + wblocks / 2 : w0;
+      const float* sw0 = p.w_scale + ((int64_t)tl.expert * wblocks + w0) * kblocks;
+      const float* sw1 = p.w_scale + ((int64_t)tl.expert * wblocks + w1) * kblocks;
+      for (int kb0 = 0; kb0 < kblocks; kb0 += 4, ++group) {
+        if ((int)(group & 1) != me) continue;
+        float4 a[LANES], f0, f1;
+        if (vec) {
+          f0 = __ldg(reinterpret_cast<const float4*>(sw0 + kb0));
+          f1 = GATED ? __ldg(reinterpret_cast<const float4*>(sw1 + kb0)) : f0;
+#pragma unroll
+          for (int j = 0; j < LANES; ++j)  // a tile's unused lanes read row 0 and store factors that nobody uses
+            if (32 * j < tl.n) a[j] = __ldg(reinterpret_cast<const float4*>(p.a_scale + (int64_t)row[j] * kblocks + kb0));
+        } else {
+          const int left = kblocks - kb0;
+          auto load4 = [&](const float* src) {
+            return make_float4(src[0], left > 1 ? src[1] : 0.f, left > 2 ? src[2] : 0.f, left > 3 ? src[3] : 0.f);
+          };
+          f0 = load4(sw0 + kb0);
+          f1 = GATED ? load4(sw1 + kb0) : f0;
+#pragma unroll
+          for (int j = 0; j < LANES; ++j)
+            if (32 * j < tl.n) a[j] = load4(p.a_scale + (int64_t)row[j] * kblocks + kb0);
+        }
+        const int slot = group % SC_SLOTS;
+        if (!warp_wait(&sc_empty[slot], ((group / SC_SLOTS) & 1) ^ 1)) {
+          report(0x780 | slot);
+          alive = false;
+          break;
+        }
+        if constexpr (!GATED) {
+          if (kb0 == 0) {  // the slot just granted also frees this tile's meta entry
+            int32_t* m = meta + (ltile % META_TILES) * TOK * 2;
+#pragma unroll
+            for (int j = 0; j < LANES; ++j) {
+              m[lane + 32 * j] = ids[j];
+              m[TOK + lane + 32 * j] = __float_as_int((ids[j] >= 0 && p.row_scale) ? p.row_scale[ids[j]] : 1.0f);
+            }
+          }
+        }
+        float* dst = reinterpret_cast<float*>(factors + slot * 4 * KB_BYTES) + lane;
+        constexpr int KB_STEP = KB_BYTES / 4;
+#pragma unroll
+        for (int j = 0; j < LANES; ++j) {
+          if (32 * j < tl.n) {
+            float* d = dst + 32 * j;
+            d[0] = a[j].x * f0.x;
+            d[KB_STEP] = a[j].y * f0.y;
+            d[2 * KB_STEP] = a[j].z * f0.z;
+            d[3 * KB_STEP] = a[j].w * f0.w;
+            if constexpr (GATED) {
+              d[TOK] = a[j].x * f1.x;
+              d[KB_STEP + TOK] = a[j].y * f1.y;
+              d[2 * KB_STEP + TOK] = a[j].z * f1.z;
+              d[3 * KB_STEP + TOK] = a[j].w * f1.w;
+            }
+          }
+        }
+        __syncwarp();
+        if (lane == 0) ptx::mbar_arrive(&sc_full[slot]);
+      }
+    }
+  } else {
+    // ---------------- fold + epilogue (warps 0-15) ----------------
+    const int quarter = warp & 3, cgroup = warp >> 2;
+    const int t = lane & 3;
+    const uint32_t factor_addr = ptx::smem_u32(factors) + (16 * cgroup + 2 * t) * 4;
+    const uint32_t lane_addr = tmem_base + ((uint32_t)(quarter * 32) << 16) + 16 * cgroup;
+    const uint32_t empty0 = ptx::smem_u32(part_empty) & ~ptx::kPeerRankBit;
+    uint32_t step = 0, gkb = 0;  // K blocks folded so far; the same, rounded up to whole groups at the end of each tile
+    int ltile = 0;
+    bool alive = true;
+    long long prof_fw = 0, prof_fb = 0, prof_sw = 0, prof_epi = 0;
+    for (int tile = worker; tile < total_tiles && alive; tile += workers, ++ltile) {
+      cursor.locate(tile, p.w_tiles, p.group, p.num_experts, table, &tl);
+      const bool mine = cgroup < (tl.n >> 4);  // this warp has a 16-token piece
+      unsigned long long acc[8];  // [0..3] rows 0-15 of the quarter, [4..7] rows 16-31
+#pragma unroll
+      for (int q = 0; q < 8; ++q) acc[q] = 0ull;
+#pragma unroll 1
+      for (int kb = 0; kb < kblocks; ++kb, ++step, ++gkb) {
+        const long long tf0 = PROF ? clock64() : 0;
+        if ((kb & 3) == 0) {
+          if (!warp_wait(&sc_full[(gkb >> 2) % SC_SLOTS], (gkb >> 2) / SC_SLOTS & 1)) {
+            report(0x740);
+            alive = false;
+            break;
+          }
+        }
+        const uint32_t fsrc = factor_addr + (gkb % (4 * SC_SLOTS)) * KB_BYTES;
+        const long long tf1 = PROF ? clock64() : 0;
+        if (!warp_wait(&part_full[step % BUFS], (step / BUFS) & 1)) {
+          report(0x700);
+          alive = false;
+          break;
+        }
+        const long long tf2 = PROF ? clock64() : 0;
+        ptx::tc_fence_after_sync();
+        const uint32_t taddr = lane_addr + (step % BUFS) * TOK;
+        if (mine) {
+          uint32_t lo[8], hi[8];
+          ptx::tmem_ld_16x256b_x2(taddr, lo);
+          ptx::tmem_ld_16x256b_x2(taddr + (16u << 16), hi);
+          const unsigned long long g0 = lds64(fsrc), g1 = lds64(fsrc + 32);
+          unsigned long long u0 = g0, u1 = g1;
+          if constexpr (GATED) {
+            u0 = lds64(fsrc + TOK * 4);
+            u1 = lds64(fsrc + TOK * 4 + 32);
+          }
+          ptx::tmem_ld_wait();
+          fma2(acc[0], lo[0], lo[1], g0);
+          fma2(acc[1], lo[2], lo[3], g0);
+          fma2(acc[2], lo[4], lo[5], g1);
+          fma2(acc[3], lo[6], lo[7], g1);
+          fma2(acc[4], hi[0], hi[1], u0);
+          fma2(acc[5], hi[2], hi[3], u0);
+          fma2(acc[6], hi[4], hi[5], u1);
+          fma2(acc[7], hi[6], hi[7], u1);
+        }
+        ptx::tc_fence_before_sync();
+        __syncwarp();
+        if (lane == 0) {
+          ptx::mbar_arrive_cluster(empty0 + (step % BUFS) * 8);
+          if ((kb & 3) == 3 || kb + 1 == kblocks) ptx::mbar_arrive(&sc_empty[(gkb >> 2) % SC_SLOTS]);
+        }
+        if (PROF) {
+          prof_sw += tf1 - tf0;
+          prof_fw += tf2 - tf1;
+          prof_fb += clock64() - tf2;
+        }
+      }
+      gkb = (gkb + 3) & ~3u;
+      if (!alive) break;
+
+      const long long te0 = PROF ? clock64() : 0;
+      const int32_t* m = meta + (ltile % META_TILES) * TOK * 2;
+      uint8_t* strip = strips + warp * G::STRIP_BYTES;
+      const int ch0 = GATED ? tl.w_tile * 128 + rank * 64 + quarter * 16 : tl.w_tile * 256 + rank * 128 + quarter * 32;
+      if (mine) {
+        const int tok0 = 16 * cgroup;
+        float2 r0 = make_float2(1.f, 1.f), r1 = r0;
+        if constexpr (!GATED) {
+          r0 = *reinterpret_cast<const float2*>(m + TOK + tok0 + 2 * t);
+          r1 = *reinterpret_cast<const float2*>(m + TOK + tok0 + 8 + 2 * t);
+        } else if (p.row_scale) {  // top-k weight on the input side: not the usual case, looked up in place
+          r0 = make_float2(row_weight(p, tl, tok0 + 2 * t), row_weight(p, tl, tok0 + 2 * t + 1));
+          r1 = make_float2(row_weight(p, tl, tok0 + 8 + 2 * t), row_weight(p, tl, tok0 + 9 + 2 * t));
+        }
+        float lo[8], hi[8];
+#pragma unroll
+        for (int q = 0; q < 4; ++q) {
+          unpack2(acc[q], lo[2 * q], lo[2 * q + 1]);
+          unpack2(acc[4 + q], hi[2 * q], hi[2 * q + 1]);
+        }
+        const float rs[4] = {r0.x, r0.y, r1.x, r1.y};
+        if constexpr (GATED) {
+          uint32_t v[4];
+#pragma unroll
+          for (int q = 0; q < 4; ++q) {
+            const int j = 4 * (q >> 1) + 2 * (q & 1);
+            v[q] = pack_bf16x2(act_mul_fast(lo[j] * rs[2 * (q >> 1)], hi[j] * rs[2 * (q >> 1)], p.activation),
+                               act_mul_fast(lo[j + 1] * rs[2 * (q >> 1) + 1], hi[j + 1] * rs[2 * (q >> 1) + 1], p.activation));
+          }
+          strip_put16(strip, 48, 0, lane, v);
+          strip_store_sorted(strip, lane, reinterpret_cast<__nv_bfloat16*>(p.out) + (int64_t)(tl.row0 + tok0) * p.n, p.n, ch0,
+                             tl.cols - tok0);
+        } else {
+#pragma unroll
+          for (int h = 0; h < 2; ++h) {
+            uint32_t v[4];
+#pragma unroll
+            for (int q = 0; q < 4; ++q) {
+              const int j = 4 * (q >> 1) + 2 * (q & 1);
+              const float a0 = h ? hi[j] : lo[j], a1 = h ? hi[j + 1] : lo[j + 1];
+              v[q] = pack_bf16x2(a0 * rs[2 * (q >> 1)], a1 * rs[2 * (q >> 1) + 1]);
+            }
+            strip_put16(strip, 80, 16 * h, lane, v);
+          }
+          strip_store_slots(strip, lane, p.out, p.out_rows, p.n, ch0, m[tok0 + (lane >> 2)], m[tok0 + 8 + (lane >> 2)]);
+        }
+      }
+      if constexpr (GATED) {
+        if (p.zero_padding && tl.last) zero_block_rows(tl, p.out, p.n, tl.w_tile * 128 + rank * 64, kFoldWarps * 32);
+      }
+      if (PROF) prof_epi += clock64() - te0;
+    }
+    if (p.out_rows) __threadfence_system();  // rows stored to a peer are complete before the kernel ends
+    if (PROF && threadIdx.x == 0 && blockIdx.x < 256) {
+      long long* out = g_wait_prof_fp8 + (GATED ? 2048 : 0) + blockIdx.x * 8;
+      out[0] = ltile;
+      out[1] = prof_fw;
+      out[2] = prof_fb;
+      out[3] = prof_sw;
+      out[4] = prof_epi;
+    }
+  }
+
+  ptx::tc_fence_before_sync();
+  __syncthreads();
+  ptx::cluster_sync_all();  // nobody signals into a CTA that has left, and both are done with TMEM
+  if (warp == kFoldWarps + 1) {
+    ptx::tc_fence_after_sync();
+    ptx::tmem_dealloc_pair(tmem_base, TMEM_COLS);
+  }
+  if (PROF && threadIdx.x == 0 && blockIdx.x < 256)
+    g_wait_prof_fp8[(GATED ? 2048 : 0) + blockIdx.x * 8 + 5] = clock64() - t_kernel0;
+}
+
+// ---------------------------------------------------------------------------------------------------------------------
+// Wide tiles (experts with many rows): the same fold with the TOKENS on the M side, 256 of one expert (128 in each CTA) x
+// 256 weight rows (CTA 0 loads the first 128: gate, or the tile's first half; CTA 1 the other 128).  A thread of the fold
+// then owns one token: its activation scale is ONE value per K block and the weight scale one value per 128 columns, and
+// TMEM is read 32 lanes wide.  With tokens on N every thread needs one factor per column: a 16-lane read-out with packed
+// factors takes 512 cycles of TMEM and 128-256 shared-memory loads per 128 x 256 partial, a 32-lane one 256 cycles and 1024
+// cycles of broadcast loads (both measured), against 310 cycles and 32 loads here.  In exchange M is always 256: tokens short of that
+// are lanes without work, so experts with few rows stay on the narrow kernel.
+//   warps 0-15: fold + epilogue: TMEM lanes 32 * (w % 4).., columns 32 * (w / 4).. of each half: 64 accumulators per thread
+//   warp 16 TMA, warp 17 MMA (CTA 0), warps 18-19 factors: products of token and weight scales in a ring of 4 slots of 8 K
+//   blocks, one slot wait per 8 K blocks of the fold
+// ---------------------------------------------------------------------------------------------------------------------
+struct WideGeo {
+  static constexpr int STAGE_BYTES = 2 * W_BYTES;  // 128 token rows + 128 weight rows per CTA
+  static constexpr int STAGES = 5;
+  static constexpr int GROUP = 8;                  // K blocks per factor slot
+  static constexpr int KB_BYTES = 2 * 128 * 4;     // factors of one K block: [first | second 128 columns][token]
+  static constexpr int SLOT_BYTES = GROUP * KB_BYTES;
+  static constexpr int META_WORDS = 2 * 128 + 4;   // slot ids, row weights, {first row, rows of this CTA, weight tile}
+  static constexpr int META_BYTES = META_TILES * META_WORDS * 4;
+  static constexpr int bytes(int num_experts) {
+    return STAGES * STAGE_BYTES + BAR_BYTES + SC_SLOTS * SLOT_BYTES + META_BYTES + pair_table_bytes(num_experts);
+  }
+};
+static_assert(WideGeo::bytes(1024) <= kMaxSmem, "shared memory");
+
+template <bool GATED, bool PROF>
+__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 1)
+grouped_gemm_pair_fold_wide_kernel(const __grid_constant__ CUtensorMap map_t, const __grid_constant__ CUtensorMap map_w,
+                                   const FoldParams p) {
+  using G = WideGeo;
+  constexpr int STAGES = G::STAGES, STAGE_BYTES = G::STAGE_BYTES;
+  extern __shared__ __align__(1024) uint8_t smem[];  // aligned by declaration: every address below is a constant
+  uint64_t* bars = reinterpret_cast<uint64_t*>(smem + STAGES * STAGE_BYTES);
+  uint64_t* full_bar = bars;                 // [STAGES] used in CTA 0: both CTAs' loads -> MMA
+  uint64_t* empty_bar = bars + STAGES;       // [STAGES] per CTA: MMA -> producer
+  uint64_t* part_full = bars + 2 * STAGES;   // [2] per CTA: MMA -> fold
+  uint64_t* part_empty = part_full + 2;      // [2] used in CTA 0: folds of both CTAs -> MMA
+  uint64_t* sc_full = part_empty + 2;        // [slots] scale warps -> fold
+  uint64_t* sc_empty = sc_full + SC_SLOTS;   // [slots] fold -> scale warps
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(sc_empty + SC_SLOTS);
+  uint8_t* scales = smem + STAGES * STAGE_BYTES + BAR_BYTES;  // [slot][K block][half][token]
+  int32_t* meta = reinterpret_cast<int32_t*>(scales + SC_SLOTS * G::SLOT_BYTES);  // [tile]
+  int32_t* table = reinterpret_cast<int32_t*>(scales + SC_SLOTS * G::SLOT_BYTES + G::META_BYTES);
+
+  const int warp = ptx::uniform_warp_id(), lane = threadIdx.x & 31;
+  const int rank = (int)ptx::cluster_ctarank();
+  const int worker = blockIdx.x >> 1, workers = gridDim.x >> 1;
+  const long long t_kernel0 = PROF ? clock64() : 0;
+
+  if (threadIdx.x == 0) {
+    for (int s = 0; s < STAGES; ++s) {
+      ptx::mbar_init(&full_bar[s], 1);
+      ptx::mbar_init(&empty_bar[s], 1);
+    }
+    for (int b = 0; b < 2; ++b) {
+      ptx::mbar_init(&part_full[b], 1);
+      ptx::mbar_init(&part_empty[b], 2 * kFoldWarps);
+    }
+    for (int s = 0; s < SC_SLOTS; ++s) {
+      ptx::mbar_init(&sc_full[s], 1);
+      ptx::mbar_init(&sc_empty[s], kFoldWarps);
+    }
+    ptx::fence_barrier_init();
+  }
+  if (warp == kFoldWarps && lane == 0) {
+    ptx::prefetch_tensormap(&map_t);
+    ptx::prefetch_tensormap(&map_w);
+  }
+  if (warp == kFoldWarps + 1) {
+    ptx::tmem_alloc_pair(tmem_slot, TMEM_COLS);
+    ptx::tmem_relinquish_pair();
+  }
+  ptx::tc_fence_before_sync();
+  pdl_entry();
+  const int used_blocks = min((int)(*p.num_tokens_post_padded / 128), p.max_blocks);
+  pair_build_table(table, p.num_experts, p.expert_table, p.expert_ids, p.sorted_token_ids, p.numel, 128, 256, used_blocks);
+  ptx::cluster_sync_all();
+  ptx::tc_fence_after_sync();
+  const uint32_t tmem_base = *tmem_slot;
+  const int kblocks = p.kblocks;
+  const int total_tiles = table[3 * p.num_experts] * p.w_tiles;
+  PairCursor cursor;
+  PairTile tl;
+
+  if (warp == kFoldWarps) {
+    // ---------------- TMA producer (both CTAs): its half of the tile's tokens, its 128 weight rows ----------------
+    if (ptx::elect_one()) {
+      int stage = 0;
+      uint32_t phase = 0;
+      bool alive = true;
+      const uint32_t ring = ptx::smem_u32(smem), bar_full0 = ptx::smem_u32(full_bar) & ~ptx::kPeerRankBit;
+      for (int tile = worker; tile < total_tiles && alive; tile += workers) {
+        cursor.locate(tile, p.w_tiles, p.group, p.num_experts, table, &tl);
+        const int half_n = tl.n >> 1;
+        const int row_t = tl.row0 + rank * half_n;
+        const int boxes = (half_n + BOX_TOKENS - 1) / BOX_TOKENS;  // lanes past them multiply what an earlier stage left
+        const uint32_t bytes = 2 * (W_BYTES + boxes * (BOX_TOKENS * KBYTES));
+        const int32_t row_w = GATED ? tl.w_tile * 128 + rank * (int32_t)p.n : tl.w_tile * 256 + rank * 128;
+        for (int kb = 0; kb < kblocks; ++kb) {
+          if (!ptx::mbar_wait(&empty_bar[stage], phase ^ 1)) {
+            report(0x500 | stage);
+            alive = false;
+            break;
+          }
+          const uint32_t stok = ring + stage * STAGE_BYTES, bar0 = bar_full0 + stage * 8;
+          const int32_t x = kb * KBYTES;
+          if (rank == 0) ptx::mbar_arrive_expect_tx(&full_bar[stage], bytes);
+          ptx::tma_load_3d_pair(stok + W_BYTES, &map_w, x, row_w, tl.expert, bar0);
+          for (int b = 0; b < boxes; ++b)
+            ptx::tma_load_2d_pair(stok + b * (BOX_TOKENS * KBYTES), &map_t, x, row_t + b * BOX_TOKENS, bar0);
+          if (++stage == STAGES) {
+            stage = 0;
+            phase ^= 1;
+          }
+        }
+      }
+      if (alive) {
+        for (int s = 0; s < STAGES; ++s) {
+          if (!ptx::mbar_wait(&empty_bar[stage], phase ^ 1)) {
+            report(0x580 | stage);
+            break;
+          }
+          if (++stage == STAGES) {
+            stage = 0;
+            phase ^= 1;
+          }
+        }
+      }
+    }
+  } else if (warp == kFoldWarps + 1) {
+    // ---------------- MMA issuer (CTA 0): one fresh partial per K block ----------------
+    if (rank == 0 && ptx::elect_one()) {
+      constexpr uint32_t idesc = ptx::make_idesc(/*e4m3*/ 0, 256, 256);
+      int stage = 0;
+      uint32_t phase = 0, step = 0;
+      bool alive = true;
+      long long prof_mp = 0, prof_md = 0;
+      const uint32_t ring = ptx::smem_u32(smem);
+      const uint64_t da0 = ptx::smem_desc_sw128(ring), db0 = ptx::smem_desc_sw128(ring + W_BYTES);
+      for (int tile = worker; tile < total_tiles && alive; tile += workers) {
+        for (int kb = 0; kb < kblocks; ++kb, ++step) {
+          const int buf = step & 1;
+          const long long tm0 = PROF ? clock64() : 0;
+          if (!ptx::mbar_wait(&full_bar[stage], phase)) {  // the data is there long before the partial is folded
+            report(0x640 | stage);
+            alive = false;
+            break;
+          }
+          const long long tm1 = PROF ? clock64() : 0;
+          if (!ptx::mbar_wait(&part_empty[buf], ((step >> 1) & 1) ^ 1)) {
+            report(0x600 | buf);
+            alive = false;
+            break;
+          }
+          if (PROF) {
+            prof_md += tm1 - tm0;
+            prof_mp += clock64() - tm1;
+          }
+          ptx::tc_fence_after_sync();
+          const uint64_t da = da0 + (uint64_t)(stage * (STAGE_BYTES >> 4)), db = db0 + (uint64_t)(stage * (STAGE_BYTES >> 4));
+#pragma unroll
+          for (int kk = 0; kk < KBYTES / 32; ++kk)
+            ptx::mma_f8f6f4_ss_pair(tmem_base + buf * 256, da + 2 * kk, db + 2 * kk, idesc, kk != 0);
+          ptx::mma_commit_both(&part_full[buf]);
+          ptx::mma_commit_both(&empty_bar[stage]);
+          if (++stage == STAGES) {
+            stage = 0;
+            phase ^= 1;
+          }
+        }
+      }
+      if (PROF && blockIdx.x < 256) {
+        g_wait_prof_fp8[(GATED ? 2048 : 0) + blockIdx.x * 8 + 6] = prof_mp;
+        g_wait_prof_fp8[(GATED ? 2048 : 0) + blockIdx.x * 8 + 7] = prof_md;
+      }
+    }
+  } else if (warp >= kFoldWarps + 2) {
+    // ---------------- factors: two warps take alternate groups of eight K blocks ----------------
+    const int me = warp - (kFoldWarps + 2);
+    uint32_t group = 0;
+    bool alive = true;
+    int ltile = 0;
+    const bool vec = (kblocks & 3) == 0 && aligned16(p.a_scale) && aligned16(p.w_scale);
+    const int wblocks = (int)(p.w_rows / 128);
+    for (int tile = worker; tile < total_tiles && alive; tile += workers, ++ltile) {
+      cursor.locate(tile, p.w_tiles, p.group, p.num_experts, table, &tl);
+      const int half_n = tl.n >> 1, first = tl.row0 + rank * half_n;
+      int32_t ids[4], row[4];  // slot and scale row of this CTA's token lane + 32 j
+#pragma unroll
+      for (int j = 0; j < 4; ++j) {
+        const int u = lane + 32 * j;
+        ids[j] = (u < half_n && rank * half_n + u < tl.cols) ? p.sorted_token_ids[first + u] : -1;
+      }
+#pragma unroll
+      for (int j = 0; j < 4; ++j) {
+        if (ids[j] >= p.numel) ids[j] = -1;
+        row[j] = ids[j] < 0 ? 0 : (p.a_scale_gather ? ids[j] / p.top_k : first + lane + 32 * j);
+      }
+      const int w0 = GATED ? tl.w_tile : tl.w_tile * 2, w1 = GATED ? tl.w_tile + wblocks / 2 : min(tl.w_tile * 2 + 1, wblocks - 1);
+      const float* sw0 = p.w_scale + ((int64_t)tl.expert * wblocks + w0) * kblocks;
+      const float* sw1 = p.w_scale + ((int64_t)tl.expert * wblocks + w1) * kblocks;
+      for (int kb0 = 0; kb0 < kblocks; kb0 += G::GROUP, ++group) {
+        if ((int)(group & 1) != me) continue;
+        const int slot = group % SC_SLOTS;
+        bool granted = false;
+#pragma unroll
+        for (int q = 0; q < G::GROUP / 4; ++q) {
+          const int kb = kb0 + 4 * q, left = kblocks - kb;
+          if (left <= 0) break;
+          float4 a[4], f0, f1;
+          if (vec) {
+            f0 = __ldg(reinterpret_cast<const float4*>(sw0 + kb));
+            f1 = __ldg(reinterpret_cast<const float4*>(sw1 + kb));
+#pragma unroll
+            for (int j = 0; j < 4; ++j)  // tokens that are not there read row 0
+              if (32 * j < half_n) a[j] = __ldg(reinterpret_cast<const float4*>(p.a_scale + (int64_t)row[j] * kblocks + kb));
+          } else {
+            auto load4 = [&](const float* src) {
+              return make_float4(src[0], left > 1 ? src[1] : 0.f, left > 2 ? src[2] : 0.f, left > 3 ? src[3] : 0.f);
+            };
+            f0 = load4(sw0 + kb);
+            f1 = load4(sw1 + kb);
+#pragma unroll
+            for (int j = 0; j < 4; ++j)
+              if (32 * j < half_n) a[j] = load4(p.a_scale + (int64_t)row[j] * kblocks + kb);
+          }
+          if (!granted) {
+            if (!warp_wait(&sc_empty[slot], ((group / SC_SLOTS) & 1) ^ 1)) {
+              report(0x780 | slot);
+              alive = false;
+              break;
+            }
+            granted = true;
+            if (kb0 == 0) {  // the slot just granted also frees this tile's meta entry
+              int32_t* m = meta + (ltile % META_TILES) * G::META_WORDS;
+#pragma unroll
+              for (int j = 0; j < 4; ++j) {
+                m[lane + 32 * j] = ids[j];
+                m[128 + lane + 32 * j] = __float_as_int((ids[j] >= 0 && p.row_scale) ? p.row_scale[ids[j]] : 1.0f);
+              }
+              if (lane == 0) {
+                m[256] = first;
+                m[257] = half_n;
+                m[258] = tl.w_tile;
+              }
+            }
+          }
+          float* dst = reinterpret_cast<float*>(scales + slot * G::SLOT_BYTES + 4 * q * G::KB_BYTES) + lane;
+#pragma unroll
+          for (int j = 0; j < 4; ++j) {
+            if (32 * j < half_n) {
+              float* d = dst + 32 * j;
+              d[0] = a[j].x * f0.x;
+              d[128] = a[j].x * f1.x;
+              d[256] = a[j].y * f0.y;
+              d[384] = a[j].y * f1.y;
+              d[512] = a[j].z * f0.z;
+              d[640] = a[j].z * f1.z;
+              d[768] = a[j].w * f0.w;
+              d[896] = a[j].w * f1.w;
+            }
+          }
+        }
+        if (!alive) break;
+        __syncwarp();
+        if (lane == 0) ptx::mbar_arrive(&sc_full[slot]);
+      }
+      if constexpr (GATED) {
+        if (p.zero_padding && tl.last && me == 0) {  // rows between the expert's last token and its block's end
+          const int from = tl.row0 + tl.cols, end = (from + 127) & ~127;
+          for (int i = lane; i < (end - from) * 8; i += 32)
+            *reinterpret_cast<uint4*>(reinterpret_cast<__nv_bfloat16*>(p.out) + (int64_t)(from + (i >> 3)) * p.n +
+                                      tl.w_tile * 128 + rank * 64 + (i & 7) * 8) = make_uint4(0, 0, 0, 0);
+        }
+      }
+    }
+  } else {
+    // ---------------- fold + epilogue (warps 0-15) ----------------
+    // This loop runs at the 96 registers that 20 warps leave a thread: the tile is described by its meta entry, shared
+    // memory addresses are constants, everything else is derived from three counters.
+    const uint32_t lane_addr = tmem_base + ((uint32_t)((warp & 3) * 32) << 16) + 32 * (warp >> 2);
+    uint32_t step = 0;  // K blocks folded so far
+    int ltile = 0;
+    bool alive = true;
+    long long prof_fw = 0, prof_fb = 0, prof_sw = 0, prof_epi = 0;
+    for (; worker + ltile * workers < total_tiles; ++ltile) {
+      float acc[64];  // [0,32): first half's 32 columns, [32,64): second half's
+#pragma unroll
+      for (int i = 0; i < 64; ++i) acc[i] = 0.f;
+      bool mine = false;  // some of this warp's lanes hold tokens
+      uint32_t src = 0;
+#pragma unroll 1
+      for (int kb = 0; kb < kblocks; ++kb, ++step) {
+        if ((kb & (G::GROUP - 1)) == 0) {
+          const long long tf0 = PROF ? clock64() : 0;
+          const uint32_t group = ltile * ((kblocks + G::GROUP - 1) / G::GROUP) + kb / G::GROUP;
+          if (kb > 0 && lane == 0) ptx::mbar_arrive(&sc_empty[(group - 1) % SC_SLOTS]);
+          if (!warp_wait(&sc_full[group % SC_SLOTS], (group / SC_SLOTS) & 1)) {
+            report(0x740);
+            alive = false;
+            break;
+          }
+          mine = (warp & 3) * 32 < meta[(ltile % META_TILES) * G::META_WORDS + 257];
+          src = ptx::smem_u32(scales) + (group % SC_SLOTS) * G::SLOT_BYTES + ((warp & 3) * 32 + lane) * 4;
+          if (PROF) prof_sw += clock64() - tf0;
+        }
+        const long long tf1 = PROF ? clock64() : 0;
+        if (!warp_wait(&part_full[step & 1], (step >> 1) & 1)) {
+          report(0x700);
+          alive = false;
+          break;
+        }
+        const long long tf2 = PROF ? clock64() : 0;
+        ptx::tc_fence_after_sync();
+        if (mine) {
+          const float f0 = lds32(src), f1 = lds32(src + 512);
+#pragma unroll
+          for (int c = 0; c < 4; ++c) {
+            // 16 columns at a time keeps the staging registers small (the 64 accumulators stay live)
+            uint32_t v[16];
+            ptx::tmem_ld_32x32b_x16(lane_addr + (step & 1) * 256 + (c >> 1) * 128 + (c & 1) * 16, v);
+            ptx::tmem_ld_wait();
+#pragma unroll
+            for (int i = 0; i < 16; ++i) acc[16 * c + i] = fmaf(__uint_as_float(v[i]), c < 2 ? f0 : f1, acc[16 * c + i]);
+          }
+        }
+        src += G::KB_BYTES;
+        ptx::tc_fence_before_sync();
+        __syncwarp();
+        if (lane == 0) ptx::mbar_arrive_cluster((ptx::smem_u32(part_empty) & ~ptx::kPeerRankBit) + (step & 1) * 8);
+        if (PROF) {
+          prof_fw += tf2 - tf1;
+          prof_fb += clock64() - tf2;
+        }
+      }
+      if (!alive) break;
+      if (lane == 0) ptx::mbar_arrive(&sc_empty[((ltile + 1) * ((kblocks + G::GROUP - 1) / G::GROUP) - 1) % SC_SLOTS]);
+
+      const long long te0 = PROF ? clock64() : 0;
+      const int32_t* m = meta + (ltile % META_TILES) * G::META_WORDS;
+      const int32_t slot = m[(warp & 3) * 32 + lane];
+      const float rs = __int_as_float(m[128 + (warp & 3) * 32 + lane]);
+      if (mine && slot >= 0) {
+        const int cpart = warp >> 2;
+        if constexpr (GATED) {
+          // acc[0..31] gate, acc[32..63] up -> output columns w_tile*128 + 32*cpart + [0,32)
+          const int64_t pos = m[256] + (warp & 3) * 32 + lane;
+          uint4* dst = reinterpret_cast<uint4*>(reinterpret_cast<__nv_bfloat16*>(p.out) + pos * p.n + (int64_t)m[258] * 128 +
+                                                32 * cpart);
+#pragma unroll
+          for (int v = 0; v < 4; ++v) {
+            uint32_t w[4];
+#pragma unroll
+            for (int j = 0; j < 4; ++j) {
+              const int i = 8 * v + 2 * j;
+              w[j] = pack_bf16x2(act_mul_fast(acc[i] * rs, acc[32 + i] * rs, p.activation),
+                                 act_mul_fast(acc[i + 1] * rs, acc[33 + i] * rs, p.activation));
+            }
+            dst[v] = make_uint4(w[0], w[1], w[2], w[3]);
+          }
+        } else {
+          // acc[0..31]: columns n0 + 32*cpart + [0,32); acc[32..63]: columns n0 + 128 + 32*cpart + [0,32)
+          __nv_bfloat16* obase = p.out_rows ? reinterpret_cast<__nv_bfloat16*>(p.out_rows[slot])
+                                            : reinterpret_cast<__nv_bfloat16*>(p.out) + (int64_t)slot * p.n;
+#pragma unroll
+          for (int h = 0; h < 2; ++h) {
+            const int64_t colg = (int64_t)m[258] * 256 + 128 * h + 32 * cpart;
+            if (obase && colg < p.n) {
+              uint4* dst = reinterpret_cast<uint4*>(obase + colg);
+#pragma unroll
+              for (int v = 0; v < 4; ++v) {
+                uint32_t w[4];
+#pragma unroll
+                for (int j = 0; j < 4; ++j) {
+                  const int i = 32 * h + 8 * v + 2 * j;
+                  w[j] = pack_bf16x2(acc[i] * rs, acc[i + 1] * rs);
+                }
+                dst[v] = make_uint4(w[0], w[1], w[2], w[3]);
+              }
+            }
+          }
+        }
+      }
+      if (PROF) prof_epi += clock64() - te0;
+    }
+    if (p.out_rows) __threadfence_system();  // rows stored to a peer are complete before the kernel ends
+    if (PROF && threadIdx.x == 0 && blockIdx.x < 256) {
+      long long* out = g_wait_prof_fp8 + (GATED ? 2048 : 0) + blockIdx.x * 8;
+      out[0] = ltile;
+      out[1] = prof_fw;
+      out[2] = prof_fb;
+      out[3] = prof_sw;
+      out[4] = prof_epi;
+    }
+  }
+
+  ptx::tc_fence_before_sync();
+  __syncthreads();
+  ptx::cluster_sync_all();
+  if (warp == kFoldWarps + 1) {
+    ptx::tc_fence_after_sync();
+    ptx::tmem_dealloc_pair(tmem_base, TMEM_COLS);
+  }
+  if (PROF && threadIdx.x == 0 && blockIdx.x < 256)
+    g_wait_prof_fp8[(GATED ? 2048 : 0) + blockIdx.x * 8 + 5] = clock64() - t_kernel0;
+}
+
+template <bool GATED, bool WIDE, bool PROF>
+int launch(const GemmParams& g, cudaStream_t st) {
+  auto kernel = WIDE ? grouped_gemm_pair_fold_wide_kernel<GATED, PROF> : grouped_gemm_pair_fold_kernel<GATED, PROF>;
+  static PerDeviceOnce once_attr;  // the opt-in to > 48 KB of dynamic shared memory is per device
+  const cudaError_t attr_err = per_device_once(once_attr, [&] {
+    return cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kMaxSmem);
+  });
+  if (attr_err != cudaSuccess)
+    return fail(FMOE_ERR_CUDA, "cudaFuncSetAttribute(smem=%d) failed: %s", kMaxSmem, cudaGetErrorString(attr_err));
+  const int64_t w_rows = GATED ? 2 * g.n : g.n;
+  constexpr int tile = WIDE ? 256 : TOK;
+  CUtensorMap map_t, map_w;
+  int rc = pair_map_tokens(&map_t, g.a, g.a_rows, g.k, 1, BOX_TOKENS);
+  if (rc) return rc;
+  // wide: gate and up rows are whole boxes of 128 of one [w_rows, K] matrix per expert
+  rc = pair_map_weights(&map_w, g.w, g.num_experts, WIDE ? w_rows : g.n, g.k, 1, GATED && !WIDE);
+  if (rc) return rc;
+  FoldParams p;
+  p.sorted_token_ids = g.sorted_token_ids;
+  p.expert_ids = g.expert_ids;
+  p.num_tokens_post_padded = g.num_tokens_post_padded;
+  p.expert_table = g.expert_table;
+  p.row_scale = g.row_scale;
+  p.a_scale = g.a_scale;
+  p.w_scale = g.w_scale;
+  p.out = g.out;
+  p.out_rows = GATED ? nullptr : g.out_rows;
+  p.numel = g.numel;
+  p.n = g.n;
+  p.w_rows = w_rows;
+  p.a_scale_gather = g.a_scale_gather;
+  p.top_k = g.top_k;
+  p.num_experts = g.num_experts;
+  p.kblocks = (int)(g.k / 128);
+  p.w_tiles = (int)ceil_div<int64_t>(g.n, GATED ? 128 : 256);
+  p.max_blocks = (int)g.max_blocks;
+  p.activation = g.activation;
+  p.group = pick_group_m(tile, g.k);
+  p.zero_padding = !g.skip_padding;
+
+  const int64_t max_tiles = g.max_blocks * ceil_div(128, tile) * p.w_tiles;
+  const int sms = device_sm_count();
+  const int workers = (int)std::max<int64_t>(1, std::min<int64_t>((sms > 0 ? sms : 148) / 2, max_tiles));
+  launch_pdl(kernel, dim3(2 * workers), dim3(kThreads),
+             WIDE ? WideGeo::bytes(g.num_experts) : Geo<GATED>::bytes(g.num_experts), st, map_t, map_w, p);
+  return launch_status("grouped_gemm_pair_fold_kernel");
+}
+
+}  // namespace
+
+bool gemm_pair_fold_supports(const GemmParams& p, bool gated) {
+  if (p.dtype != FMOE_E4M3 || p.out_dtype != FMOE_BF16) return false;
+  if (p.bias || p.activation == FMOE_ACT_SWIGLU_OAI) return false;  // bf16-only variant
+  if (p.block_size != 128 || p.a_gather) return false;
+  if (p.k <= 0 || p.k % 128 != 0 || p.n <= 0 || p.n % 128 != 0) return false;
+  if (!p.a_scale || !p.w_scale) return false;
+  if (!aligned16(p.a) || !aligned16(p.w) || !(aligned16(p.out) && (p.out || (!gated && p.out_rows)))) return false;
+  if ((int64_t)p.num_experts * (gated ? 2 * p.n : p.n) >= (1ll << 31) || p.a_rows >= (1ll << 31)) return false;
+  if (2 * p.max_blocks * ceil_div<int64_t>(p.n, gated ? 128 : 256) >= (1ll << 30) || p.num_experts > 1024) return false;
+  return true;
+}
+
+int read_wait_profile_fp8(long long* host_out, int n) {
+  FMOE_CUDA_OK(cudaMemcpyFromSymbol(host_out, g_wait_prof_fp8, sizeof(long long) * (size_t)n));
+  return FMOE_OK;
+}
+
+int status_word_fp8(int* out, bool clear) {
+  int zero = 0;
+  FMOE_CUDA_OK(cudaMemcpyFromSymbol(out, g_device_status_fp8, sizeof(int)));
+  if (clear && *out != 0) FMOE_CUDA_OK(cudaMemcpyToSymbol(g_device_status_fp8, &zero, sizeof(int)));
+  return FMOE_OK;
+}
+
+int gemm_pair_fold(const GemmParams& p, bool gated, cudaStream_t st) {
+  if (!gemm_pair_fold_supports(p, gated))
+    return fail(FMOE_ERR_UNSUPPORTED,
+                "tcgen05 fp8 gemm: needs e4m3 in, bf16 out, block_size 128, sorted input rows, n and k multiples of 128");
+  if (p.max_blocks <= 0) return FMOE_OK;
+  static const bool profile = getenv("FMOE_TC_PROFILE") != nullptr;
+  // the table's tile width decides: 64-token tiles for the narrow kernel, 256 for the wide one
+  const bool wide = (p.token_tile ? p.token_tile : pick_fold_token_tile(p.numel, p.num_experts)) == 256;
+  auto go = [&](auto gated_c, auto wide_c) {
+    constexpr bool G = decltype(gated_c)::value, W = decltype(wide_c)::value;
+    return profile ? launch<G, W, true>(p, st) : launch<G, W, false>(p, st);
+  };
+  using T = std::true_type;
+  using F = std::false_type;
+  if (gated) return wide ? go(T{}, T{}) : go(T{}, F{});
+  return wide ? go(F{}, T{}) : go(F{}, F{});
+}
+
+}  // namespace fmoe

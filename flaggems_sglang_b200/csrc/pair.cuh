@@ -2,29 +2,41 @@
 // units of a cluster and the TMA maps.
 //
 // Both kernels put the WEIGHTS on the M side of the tensor cores (256 weight rows per tile, 128 in each CTA of a pair)
-// and the tokens on the N side.  N is any multiple of 16 up to 256, so an expert with 9 tokens costs a 16-column tile and
-// one with 300 costs two of 160: no work is done for padding beyond 15 columns, and the weights are read once per 256
-// tokens.  The rows between an expert's last token and the next multiple of the moe_align block are never touched.
+// and the tokens on the N side.  N is any multiple of 16 up to the launch's token tile (64, 128 or 256), so an expert with
+// 9 tokens costs a 16-column tile and one with 300 costs two of 160: no work is done for padding beyond 15 columns.  The
+// rows between an expert's last token and the next multiple of the moe_align block are never touched.
 #pragma once
 #include "gemm.cuh"
 #include "ptx_sm100.cuh"
 
 namespace fmoe {
 
-constexpr int kPairTokens = 256;     // most tokens of a tile
+// Most tokens of a tile, by the rows an expert has on average.  A narrow tile leaves shared memory for a deeper ring of
+// weights (what a launch needs whose time is the reading of weights) and TMEM for more partials (gemm_pair_fold.cu); a wide
+// one reads the weights from L2 less often.  Experts well above the average are cut into several tiles either way.
+inline int pick_token_tile(int64_t numel, int num_experts) {
+  const double rows = (double)numel / (double)(numel < num_experts ? (numel > 0 ? numel : 1) : num_experts);
+  return rows <= 40.0 ? 64 : (rows <= 88.0 ? 128 : 256);
+}
 constexpr int kSplitCounters = 256;  // tail-split arrival counters of one launch: one per CTA
 
 // int32 words of the expert table: first row [E], rows [E], exclusive prefix sum of the token tiles [E + 1]
 __host__ __device__ constexpr int pair_table_words(int num_experts) { return 3 * num_experts + 1; }
 __host__ __device__ constexpr int pair_table_bytes(int num_experts) { return (pair_table_words(num_experts) * 4 + 15) & ~15; }
+// The e4m3 block-scale kernels (gemm_pair_fold.cu) are built for two widths.
+inline int pick_fold_token_tile(int64_t numel, int num_experts) {
+  const double rows = (double)numel / (double)(numel < num_experts ? (numel > 0 ? numel : 1) : num_experts);
+  return rows <= 48.0 ? 64 : 256;
+}
 
 #if defined(__CUDACC__)
 // Exclusive prefix sum over the experts' token tiles by one warp; rows[e] -> prefix[e], total in prefix[E].
-__device__ __forceinline__ void pair_prefix_warp(const int32_t* rows, int32_t* prefix, int num_experts, int lane) {
+__device__ __forceinline__ void pair_prefix_warp(const int32_t* rows, int32_t* prefix, int num_experts, int token_tile,
+                                                 int lane) {
   int carry = 0;
   for (int base = 0; base < num_experts; base += 32) {
     const int e = base + lane;
-    const int tiles = e < num_experts ? (rows[e] + kPairTokens - 1) / kPairTokens : 0;
+    const int tiles = e < num_experts ? (rows[e] + token_tile - 1) / token_tile : 0;
     int incl = tiles;
 #pragma unroll
     for (int off = 1; off < 32; off <<= 1) {
@@ -43,7 +55,7 @@ __device__ __forceinline__ void pair_prefix_warp(const int32_t* rows, int32_t* p
 __device__ __forceinline__ void pair_build_table(int32_t* table, int num_experts, const int32_t* __restrict__ global_table,
                                                  const int32_t* __restrict__ expert_ids,
                                                  const int32_t* __restrict__ sorted_ids, int64_t numel, int block_rows,
-                                                 int used_blocks) {
+                                                 int token_tile, int used_blocks) {
   if (global_table) {
     for (int i = threadIdx.x; i < pair_table_words(num_experts); i += blockDim.x) table[i] = global_table[i];
     __syncthreads();
@@ -83,7 +95,7 @@ __device__ __forceinline__ void pair_build_table(int32_t* table, int num_experts
     }
   }
   __syncthreads();
-  if (warp == 0) pair_prefix_warp(rows, table + 2 * num_experts, num_experts, lane);
+  if (warp == 0) pair_prefix_warp(rows, table + 2 * num_experts, num_experts, token_tile, lane);
   __syncthreads();
 }
 
@@ -119,7 +131,7 @@ struct PairCursor {
     const int in_group = min(group, tiles - g * group);
     out->w_tile = r / in_group;
     const int t = g * group + r % in_group;
-    const int step = (((rows + tiles - 1) / tiles) + 15) & ~15;  // the expert's tokens in equal tiles (<= 256)
+    const int step = (((rows + tiles - 1) / tiles) + 15) & ~15;  // the expert's tokens in equal tiles
     out->row0 = table[expert] + t * step;
     out->cols = min(step, rows - t * step);
     out->n = (out->cols + 15) & ~15;
@@ -127,6 +139,54 @@ struct PairCursor {
     out->last = t == tiles - 1;
   }
 };
+
+// ---- transposed stores ------------------------------------------------------------------------------
+// A warp's strip of shared memory holds 16 tokens x (up to 32 channels + 8 of padding, so that neither the column stores
+// nor the row loads conflict).
+constexpr int kStripBytes = 16 * 80;
+
+// 16 channels x 16 tokens in the fragment layout of tmem_ld_16x256b_x2, packed to bf16 (v[2 * token half + channel half]),
+// into channels [ch, ch + 16) of a strip with `pitch` bytes per token.
+__device__ __forceinline__ void strip_put16(uint8_t* strip, int pitch, int ch, int lane, const uint32_t (&v)[4]) {
+  const int tok = (lane & 7) + (lane >> 4) * 8, c = ch + ((lane >> 3) & 1) * 8;
+  ptx::stmatrix_x4_trans(ptx::smem_u32(strip + tok * pitch + c * 2), v[0], v[1], v[2], v[3]);
+}
+// 16 tokens x 16 channels of a strip (pitch 48) to consecutive rows; `rows` of them are real.
+__device__ __forceinline__ void strip_store_sorted(const uint8_t* strip, int lane, __nv_bfloat16* out, int64_t n, int ch0,
+                                                   int rows) {
+  __syncwarp();
+  const int u = lane >> 1, part = (lane & 1) * 8;
+  const uint4 v = *reinterpret_cast<const uint4*>(strip + u * 48 + part * 2);
+  if (u < rows && ch0 + part < n) *reinterpret_cast<uint4*>(out + u * n + ch0 + part) = v;
+  __syncwarp();
+}
+// 16 tokens x 32 channels of a strip (pitch 80) to the rows of their slots; slot_a / slot_b: of tokens lane / 4 and
+// 8 + lane / 4 (negative: none).
+__device__ __forceinline__ void strip_store_slots(const uint8_t* strip, int lane, void* out, void* const* out_rows, int64_t n,
+                                                  int ch0, int32_t slot_a, int32_t slot_b) {
+  __syncwarp();
+  const int part = (lane & 3) * 8;
+#pragma unroll
+  for (int h = 0; h < 2; ++h) {
+    const uint4 v = *reinterpret_cast<const uint4*>(strip + ((lane >> 2) + 8 * h) * 80 + part * 2);
+    const int32_t slot = h ? slot_b : slot_a;
+    if (slot >= 0 && ch0 + part < n) {
+      __nv_bfloat16* row = out_rows ? reinterpret_cast<__nv_bfloat16*>(out_rows[slot])
+                                    : reinterpret_cast<__nv_bfloat16*>(out) + (int64_t)slot * n;
+      if (row) *reinterpret_cast<uint4*>(row + ch0 + part) = v;
+    }
+  }
+  __syncwarp();
+}
+// gate/up GEMM through the plain C entry point: the rows between the expert's last token and the end of its 128-row block
+// are zeros in this CTA's 64 channels.  All `threads` epilogue threads.
+__device__ __forceinline__ void zero_block_rows(const PairTile& tl, void* out, int64_t n, int ch, int threads) {
+  const int from = tl.row0 + tl.cols, end = (from + 127) & ~127;  // blocks start at multiples of 128 rows
+  for (int i = threadIdx.x; i < (end - from) * 8; i += threads) {
+    const int64_t row = from + (i >> 3), c = ch + (i & 7) * 8;
+    if (c < n) *reinterpret_cast<uint4*>(reinterpret_cast<__nv_bfloat16*>(out) + row * n + c) = make_uint4(0, 0, 0, 0);
+  }
+}
 #endif
 
 // Work units of one worker (a CTA pair).  Tiles are dealt round-robin; when the last round has work for at most half of
