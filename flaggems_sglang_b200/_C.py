@@ -74,6 +74,13 @@ class FusedArgs(_SizedStructure):
     ]
 
 
+class RouteArgs(Structure):
+    """Mirror of struct fmoe_route_args."""
+
+    _fields_ = [("logits", c_void_p), ("correction_bias", c_void_p), ("grouped", c_int32), ("renormalize", c_int32),
+                ("n_group", c_int32), ("topk_group", c_int32)]
+
+
 # name -> (restype, argtypes); every symbol include/fmoe_b200.h declares
 SIGNATURES = {
     "fmoe_version": (c_int, []),
@@ -102,6 +109,8 @@ SIGNATURES = {
     "fmoe_pick_variant": (c_int, [c_int, c_int64, c_int, c_int64, c_int64, c_int, POINTER(c_int), POINTER(c_int)]),
     "fmoe_fused_experts_workspace_bytes": (c_int64, [POINTER(FusedArgs)]),
     "fmoe_fused_experts": (c_int, [POINTER(FusedArgs), c_void_p]),
+    "fmoe_fused_moe_workspace_bytes": (c_int64, [POINTER(FusedArgs), POINTER(RouteArgs)]),
+    "fmoe_fused_moe": (c_int, [POINTER(FusedArgs), POINTER(RouteArgs), c_void_p]),
     "fmoe_static_scratch_bytes": (c_int64, []),
     "fmoe_fused_experts_static": (c_int, [POINTER(FusedArgs), c_void_p]),
     "fmoe_ep_buffer_create": (c_int, [c_int64, POINTER(c_void_p), c_void_p]),

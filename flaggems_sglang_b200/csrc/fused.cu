@@ -67,7 +67,7 @@ inline bool tc_gathers_input(int variant, int dtype) {
 }
 }
 
-int plan_fused(const fmoe_fused_args& a, FusedPlan* pl) {
+int plan_fused(const fmoe_fused_args& a, const RouteArgs& route, FusedPlan* pl) {
   if (a.struct_size != sizeof(fmoe_fused_args))
     return fail(FMOE_ERR_INVALID_ARG, "fused_experts: fmoe_fused_args.struct_size is %u, this library's struct has %zu "
                 "bytes (binding built against another header?)", a.struct_size, sizeof(fmoe_fused_args));
@@ -122,6 +122,16 @@ int plan_fused(const fmoe_fused_args& a, FusedPlan* pl) {
     off += up256(bytes);
     return o;
   };
+  p.off_route_ids = p.off_route_weights = -1;
+  p.use_decode = plan_decode(a, route, &p.decode);
+  if (p.use_decode) {
+    p.total = p.decode.total;
+    return FMOE_OK;
+  }
+  if (route.logits) {
+    p.off_route_ids = take(p.numel * 4);
+    p.off_route_weights = take(p.numel * 4);
+  }
   p.off_sorted = take(p.cap * 4);
   p.off_expert = take(p.nblk * 4);
   p.off_npp = take(16);
@@ -195,7 +205,8 @@ const char* const kStageNames[7] = {"fmoe.align",       "fmoe.gather_quant", "fm
                                     "fmoe.gemm2",       "fmoe.moe_sum",      "fmoe.done"};
 }  // namespace
 
-int run_fused(const fmoe_fused_args& a, const FusedPlan& p, uint8_t* ws, void* stream) {
+int run_fused(const fmoe_fused_args& args, const RouteArgs& route, const FusedPlan& p, uint8_t* ws, void* stream) {
+  fmoe_fused_args a = args;
   void* const* stage_ev = t_stage_events;
   const int stage_n = t_stage_count;
   t_stage_events = nullptr;
@@ -206,6 +217,23 @@ int run_fused(const fmoe_fused_args& a, const FusedPlan& p, uint8_t* ws, void* s
     if (i < 6) range.next(kStageNames[i]);
   };
   if (a.T == 0) return FMOE_OK;
+  auto st = (cudaStream_t)stream;
+  if (p.use_decode) {
+    mark(0);
+    const int rc = run_decode(a, route, p.decode, ws, st);
+    for (int i = 1; i <= 6; ++i) mark(i);
+    return rc;
+  }
+  if (route.logits) {
+    int32_t* ids = reinterpret_cast<int32_t*>(ws + p.off_route_ids);
+    float* weights = reinterpret_cast<float*>(ws + p.off_route_weights);
+    const int rc = route.grouped ? fmoe_topk_grouped(route.logits, route.bias, a.T, a.num_experts, a.top_k, route.n_group,
+                                                     route.topk_group, route.renorm, 1.0f, weights, ids, stream)
+                                 : fmoe_topk_softmax(route.logits, a.T, a.num_experts, a.top_k, route.renorm, weights, ids, stream);
+    if (rc) return rc;
+    a.topk_ids = ids;
+    a.topk_weights = weights;
+  }
   FMOE_REQUIRE(a.hidden && a.w1 && a.w2 && a.topk_weights && a.topk_ids && (a.out || a.out_rows), "fused_experts: null pointer");
   if (a.out_rows) {
     FMOE_REQUIRE(a.no_combine && !a.zero_dropped, "fused_experts: out_rows needs no_combine = 1 and zero_dropped = 0");
@@ -222,7 +250,6 @@ int run_fused(const fmoe_fused_args& a, const FusedPlan& p, uint8_t* ws, void* s
   int32_t* npp = reinterpret_cast<int32_t*>(ws + p.off_npp);
   void* act = ws + p.off_act;
   void* z = a.no_combine ? a.out : (void*)(ws + p.off_z);
-  auto st = (cudaStream_t)stream;
 
   mark(0);
   int32_t* table = p.off_table >= 0 ? reinterpret_cast<int32_t*>(ws + p.off_table) : nullptr;
@@ -371,6 +398,18 @@ int run_fused(const fmoe_fused_args& a, const FusedPlan& p, uint8_t* ws, void* s
   return rc;
 }
 
+int run_with_workspace(const fmoe_fused_args& args, const RouteArgs& route, void* stream) {
+  FusedPlan p;
+  int rc = plan_fused(args, route, &p);
+  if (rc) return rc;
+  if (args.T == 0) return FMOE_OK;
+  FMOE_REQUIRE(args.workspace && (reinterpret_cast<uintptr_t>(args.workspace) & 255u) == 0,
+               "fused_experts: workspace must be non-null and 256-byte aligned");
+  FMOE_REQUIRE(args.workspace_bytes >= p.total, "fused_experts: workspace too small (%lld < %lld bytes)",
+               (long long)args.workspace_bytes, (long long)p.total);
+  return run_fused(args, route, p, reinterpret_cast<uint8_t*>(args.workspace), stream);
+}
+
 }  // namespace fmoe
 
 extern "C" int fmoe_pick_variant(int dtype, int64_t numel, int E, int64_t I, int64_t H, int forced_variant,
@@ -393,20 +432,56 @@ extern "C" int64_t fmoe_fused_experts_workspace_bytes(const fmoe_fused_args* arg
     return -1;
   }
   fmoe::FusedPlan p;
-  if (fmoe::plan_fused(*args, &p)) return -1;
+  if (fmoe::plan_fused(*args, fmoe::RouteArgs{}, &p)) return -1;
   return p.total;
 }
 
 extern "C" int fmoe_fused_experts(const fmoe_fused_args* args, void* stream) {
   using namespace fmoe;
   if (!args) return fail(FMOE_ERR_INVALID_ARG, "fused_experts: args is null");
-  FusedPlan p;
-  int rc = plan_fused(*args, &p);
+  return run_with_workspace(*args, RouteArgs{}, stream);
+}
+
+namespace {
+fmoe::RouteArgs route_args(const fmoe_route_args& r) {
+  fmoe::RouteArgs out;
+  out.logits = r.logits;
+  out.bias = r.correction_bias;
+  out.grouped = r.grouped;
+  out.renorm = r.renormalize;
+  out.n_group = r.n_group;
+  out.topk_group = r.topk_group;
+  return out;
+}
+int check_route(const fmoe_fused_args& a, const fmoe_route_args& r) {
+  using namespace fmoe;
+  FMOE_REQUIRE(r.logits, "fused_moe: logits is null");
+  FMOE_REQUIRE(a.num_experts >= 1 && a.num_experts <= 1024 && a.top_k >= 1 && a.top_k <= 32 && a.top_k <= a.num_experts,
+               "fused_moe: need 1 <= k <= min(32,E), E <= 1024 (got k=%d, E=%d)", a.top_k, a.num_experts);
+  if (r.grouped) {
+    FMOE_REQUIRE(r.n_group >= 1 && r.n_group <= 32 && a.num_experts % r.n_group == 0,
+                 "fused_moe: need 1 <= n_group <= 32 dividing E (got n_group=%d, E=%d)", r.n_group, a.num_experts);
+    FMOE_REQUIRE(r.topk_group >= 1 && r.topk_group <= r.n_group, "fused_moe: bad topk_group=%d", r.topk_group);
+    FMOE_REQUIRE(a.top_k <= r.topk_group * (a.num_experts / r.n_group), "fused_moe: k=%d exceeds the experts of the kept groups",
+                 a.top_k);
+  }
+  return FMOE_OK;
+}
+}  // namespace
+
+extern "C" int64_t fmoe_fused_moe_workspace_bytes(const fmoe_fused_args* args, const fmoe_route_args* route) {
+  if (!args || !route) {
+    fmoe::fail(FMOE_ERR_INVALID_ARG, "fused_moe: args or route is null");
+    return -1;
+  }
+  fmoe::FusedPlan p;
+  if (check_route(*args, *route) || fmoe::plan_fused(*args, route_args(*route), &p)) return -1;
+  return p.total;
+}
+
+extern "C" int fmoe_fused_moe(const fmoe_fused_args* args, const fmoe_route_args* route, void* stream) {
+  if (!args || !route) return fmoe::fail(FMOE_ERR_INVALID_ARG, "fused_moe: args or route is null");
+  const int rc = check_route(*args, *route);
   if (rc) return rc;
-  if (args->T == 0) return FMOE_OK;
-  FMOE_REQUIRE(args->workspace && (reinterpret_cast<uintptr_t>(args->workspace) & 255u) == 0,
-               "fused_experts: workspace must be non-null and 256-byte aligned");
-  FMOE_REQUIRE(args->workspace_bytes >= p.total, "fused_experts: workspace too small (%lld < %lld bytes)",
-               (long long)args->workspace_bytes, (long long)p.total);
-  return run_fused(*args, p, reinterpret_cast<uint8_t*>(args->workspace), stream);
+  return fmoe::run_with_workspace(*args, route_args(*route), stream);
 }

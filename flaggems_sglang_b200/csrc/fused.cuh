@@ -1,6 +1,7 @@
 // Internal: workspace plan and launcher of the one-call expert computation (fused.cu).
 #pragma once
 #include "common.cuh"
+#include "decode.cuh"
 
 namespace fmoe {
 
@@ -10,6 +11,9 @@ struct FusedPlan {
   // byte offsets into the workspace (-1: not used)
   int64_t off_sorted, off_expert, off_npp, off_align_ws, align_ws_bytes, off_xs, off_xs_scale, off_xt, off_xt_scale, off_act, off_actq, off_actq_scale, off_z;
   int64_t off_split, split_bytes;  // tail-split scratch of the tcgen05 GEMMs
+  bool use_decode;                  // the two decode kernels take the call (decode.cu); the fields above are then unused
+  DecodePlan decode;
+  int64_t off_route_ids, off_route_weights;  // calls from logits: where the router's results go (-1: not used)
   int64_t off_table, off_counters;  // expert table and tail-split counters of the CTA-pair GEMMs
 };
 
@@ -19,8 +23,8 @@ struct FusedPlan {
 inline bool fp8_quant_once(int64_t top_k, int64_t) { return top_k >= 2; }
 
 int pick_variant(int dtype, int64_t numel, int E, int64_t I, int64_t H, int forced, int* variant, int* block);
-int plan_fused(const fmoe_fused_args& a, FusedPlan* plan);
+int plan_fused(const fmoe_fused_args& a, const RouteArgs& route, FusedPlan* plan);
 // Enqueues the whole computation using `ws` (at least plan.total bytes, 256-byte aligned) as scratch.
-int run_fused(const fmoe_fused_args& a, const FusedPlan& plan, uint8_t* ws, void* stream);
+int run_fused(const fmoe_fused_args& a, const RouteArgs& route, const FusedPlan& plan, uint8_t* ws, void* stream);
 
 }  // namespace fmoe

@@ -50,7 +50,7 @@ extern "C" int fmoe_fused_experts_static(const fmoe_fused_args* args, void* stre
   using namespace fmoe;
   if (!args) return fail(FMOE_ERR_INVALID_ARG, "fused_experts_static: args is null");
   FusedPlan plan;
-  int rc = plan_fused(*args, &plan);
+  int rc = plan_fused(*args, RouteArgs{}, &plan);
   if (rc) return rc;
   if (plan.total > kStaticScratchBytes)
     return fail(FMOE_ERR_UNSUPPORTED,
@@ -61,5 +61,5 @@ extern "C" int fmoe_fused_experts_static(const fmoe_fused_args* args, void* stre
   uint8_t* scratch = nullptr;
   rc = static_scratch_for_current_device(&scratch);
   if (rc) return rc;
-  return run_fused(*args, plan, scratch, stream);
+  return run_fused(*args, RouteArgs{}, plan, scratch, stream);
 }

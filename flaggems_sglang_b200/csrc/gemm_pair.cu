@@ -557,7 +557,9 @@ EncodeTiledFn encode_tiled_fn() {
   return fn;
 }
 
-int encode(CUtensorMap* map, const void* base, int elem_bytes, int rank, const cuuint64_t* dims, const cuuint64_t* strides,
+}  // namespace
+
+int encode_tensor_map(CUtensorMap* map, const void* base, int elem_bytes, int rank, const cuuint64_t* dims, const cuuint64_t* strides,
            const cuuint32_t* box, bool weights, const char* what) {
   EncodeTiledFn fn = encode_tiled_fn();
   if (!fn) return fail(FMOE_ERR_CUDA, "cuTensorMapEncodeTiled is not available from the driver");
@@ -570,8 +572,6 @@ int encode(CUtensorMap* map, const void* base, int elem_bytes, int rank, const c
   if (r != CUDA_SUCCESS) return fail(FMOE_ERR_CUDA, "cuTensorMapEncodeTiled (%s) failed with code %d", what, (int)r);
   return FMOE_OK;
 }
-
-}  // namespace
 
 // SM count of the current device (cached per device ordinal).
 int device_sm_count() {
@@ -614,7 +614,7 @@ int pair_map_tokens(CUtensorMap* map, const void* base, int64_t rows, int64_t co
   const cuuint64_t dims[2] = {(cuuint64_t)cols, (cuuint64_t)rows};
   const cuuint64_t strides[1] = {(cuuint64_t)cols * elem_bytes};
   const cuuint32_t box[2] = {(cuuint32_t)(KBYTES / elem_bytes), (cuuint32_t)box_rows};
-  return encode(map, base, elem_bytes, 2, dims, strides, box, false, "tokens");
+  return encode_tensor_map(map, base, elem_bytes, 2, dims, strides, box, false, "tokens");
 }
 
 // weights [E, rows, K], K contiguous.  gated: rows = n gate rows then n up rows; the box takes 4 groups of 16 gate rows and
@@ -625,12 +625,12 @@ int pair_map_weights(CUtensorMap* map, const void* base, int64_t experts, int64_
     const cuuint64_t dims[5] = {(cuuint64_t)k, 16, 2, (cuuint64_t)(n / 16), (cuuint64_t)experts};
     const cuuint64_t strides[4] = {row, row * n, row * 16, row * 2 * n};
     const cuuint32_t box[5] = {(cuuint32_t)(KBYTES / elem_bytes), 16, 2, 4, 1};
-    return encode(map, base, elem_bytes, 5, dims, strides, box, true, "gate/up weights");
+    return encode_tensor_map(map, base, elem_bytes, 5, dims, strides, box, true, "gate/up weights");
   }
   const cuuint64_t dims[3] = {(cuuint64_t)k, (cuuint64_t)n, (cuuint64_t)experts};
   const cuuint64_t strides[2] = {row, row * n};
   const cuuint32_t box[3] = {(cuuint32_t)(KBYTES / elem_bytes), 128, 1};
-  return encode(map, base, elem_bytes, 3, dims, strides, box, true, "down weights");
+  return encode_tensor_map(map, base, elem_bytes, 3, dims, strides, box, true, "down weights");
 }
 
 // bf16 weights [E, K, w_rows] with w_rows contiguous; box = 64 channels (128 bytes, the swizzle width) x 64 K rows.
@@ -638,7 +638,7 @@ int pair_map_weights_nmajor(CUtensorMap* map, const void* base, int64_t experts,
   const cuuint64_t dims[3] = {(cuuint64_t)w_rows, (cuuint64_t)k, (cuuint64_t)experts};
   const cuuint64_t strides[2] = {(cuuint64_t)w_rows * 2, (cuuint64_t)w_rows * (cuuint64_t)k * 2};
   const cuuint32_t box[3] = {64, 64, 1};
-  return encode(map, base, 2, 3, dims, strides, box, true, "N-major weights");
+  return encode_tensor_map(map, base, 2, 3, dims, strides, box, true, "N-major weights");
 }
 
 namespace {
@@ -785,19 +785,22 @@ int read_wait_profile(long long* host_out, int n) {
 
 int status_word_fp8(int* out, bool clear);
 int status_word_ep(int* out, bool clear);
+int status_word_decode(int* out, bool clear);
 
-// First non-zero status word of the translation units that keep one (tcgen05 kernels, expert-parallel
-// exchange); all are cleared.
+// First non-zero status word of the translation units that keep one (tcgen05 kernels, decode layer,
+// expert-parallel exchange); all are cleared.
 int read_and_clear_device_status(cudaStream_t st, int* status_out) {
-  int zero = 0, a = 0, b = 0, d = 0;
+  int zero = 0, a = 0, b = 0, c = 0, d = 0;
   FMOE_CUDA_OK(cudaStreamSynchronize(st));
   FMOE_CUDA_OK(cudaMemcpyFromSymbol(&a, g_device_status, sizeof(int)));
   if (a != 0) FMOE_CUDA_OK(cudaMemcpyToSymbol(g_device_status, &zero, sizeof(int)));
   int rc = status_word_fp8(&b, true);
   if (rc) return rc;
+  rc = status_word_decode(&c, true);
+  if (rc) return rc;
   rc = status_word_ep(&d, true);
   if (rc) return rc;
-  *status_out = a ? a : (b ? b : d);
+  *status_out = a ? a : (b ? b : (c ? c : d));
   return FMOE_OK;
 }
 

@@ -26,7 +26,7 @@ template <typename InT>
 __global__ void __launch_bounds__(256)
 quant_group128_kernel(const InT* __restrict__ x, int64_t rows_out, int64_t K, const int32_t* __restrict__ row_map,
                       int map_div, int64_t sentinel, const int32_t* __restrict__ num_rows_dev,
-                      uint8_t* __restrict__ q, float* __restrict__ scale) {
+                      uint8_t* __restrict__ q, float* __restrict__ scale, int zero_padding) {
   pdl_entry();
   constexpr int kIlp = 4;
   const int sub = threadIdx.x & 15;  // lane inside the 16-lane team
@@ -88,32 +88,14 @@ quant_group128_kernel(const InT* __restrict__ x, int64_t rows_out, int64_t K, co
       for (int off = 8; off > 0; off >>= 1) amax = fmaxf(amax, __shfl_xor_sync(hmask, amax, off));
       if (pu[u] >= limit) continue;  // uniform over the 16 lanes of the team
       uint2* dst = reinterpret_cast<uint2*>(q + pu[u] * K + (int64_t)gu[u] * 128 + sub * 8);
-      if (!real[u]) {  // padding position: zeros with a unit scale
+      if (!real[u]) {  // padding position: zeros with a unit scale, or nothing
+        if (!zero_padding) continue;
         *dst = make_uint2(0, 0);
         if (sub == 0) scale[pu[u] * groups + gu[u]] = 1.0f;
         continue;
       }
-      const float s = __fdiv_rn(fmaxf(amax, 1e-10f), 448.0f);
-      uint32_t lo = 0, hi = 0;
-      if (amax <= 3.0e38f) {
-        const float r = __frcp_rn(s);
-        float qv[8];
-#pragma unroll
-        for (int i = 0; i < 8; ++i) qv[i] = div_by_shared(v[u][i], s, r);
-        // two values per conversion instruction (low byte = first value)
-        auto pair = [](float a, float b) {
-          return (uint32_t)__nv_cvt_float2_to_fp8x2(make_float2(a, b), __NV_SATFINITE, __NV_E4M3);
-        };
-        lo = pair(qv[0], qv[1]) | (pair(qv[2], qv[3]) << 16);
-        hi = pair(qv[4], qv[5]) | (pair(qv[6], qv[7]) << 16);
-      } else {
-#pragma unroll
-        for (int i = 0; i < 4; ++i) {
-          lo |= (uint32_t)f32_to_e4m3_bits(__fdiv_rn(v[u][i], s)) << (8 * i);
-          hi |= (uint32_t)f32_to_e4m3_bits(__fdiv_rn(v[u][4 + i], s)) << (8 * i);
-        }
-      }
-      *dst = make_uint2(lo, hi);
+      const float s = group_scale(amax);
+      *dst = quant8(v[u], s, __frcp_rn(s), amax <= 3.0e38f);
       if (sub == 0) scale[pu[u] * groups + gu[u]] = s;
     }
   }
@@ -127,7 +109,7 @@ template <int TEAM, int VECS>
 __global__ void __launch_bounds__(256)
 quant_row_kernel(const __nv_bfloat16* __restrict__ x, int64_t rows_out, int64_t K, const int32_t* __restrict__ row_map,
                  int map_div, int64_t sentinel, const int32_t* __restrict__ num_rows_dev, uint8_t* __restrict__ q,
-                 float* __restrict__ scale) {
+                 float* __restrict__ scale, int zero_padding) {
   pdl_entry();
   __shared__ float s_max[8];
   constexpr int kTeams = 256 / TEAM;
@@ -138,7 +120,8 @@ quant_row_kernel(const __nv_bfloat16* __restrict__ x, int64_t rows_out, int64_t 
   for (int64_t p = (int64_t)blockIdx.x * kTeams + threadIdx.x / TEAM; p < limit; p += (int64_t)gridDim.x * kTeams) {
     const int64_t r = mapped_row(row_map, map_div, sentinel, p);
     uint2* dst = reinterpret_cast<uint2*>(q + p * K);
-    if (r < 0) {  // padding position: zeros with a unit scale
+    if (r < 0) {  // padding position: zeros with a unit scale, or nothing
+      if (!zero_padding) continue;
       for (int c = lane; c < vecs; c += TEAM) dst[c] = make_uint2(0, 0);
       if (lane == 0) scale[p] = 1.0f;
       continue;
@@ -181,24 +164,7 @@ quant_row_kernel(const __nv_bfloat16* __restrict__ x, int64_t rows_out, int64_t 
         v[2 * j] = __low2float(h[j]);
         v[2 * j + 1] = __high2float(h[j]);
       }
-      uint32_t lo = 0, hi = 0;
-      if (finite) {
-        float qv[8];
-#pragma unroll
-        for (int j = 0; j < 8; ++j) qv[j] = div_by_shared(v[j], s, rcp);
-        auto pair = [](float a, float b) {
-          return (uint32_t)__nv_cvt_float2_to_fp8x2(make_float2(a, b), __NV_SATFINITE, __NV_E4M3);
-        };
-        lo = pair(qv[0], qv[1]) | (pair(qv[2], qv[3]) << 16);
-        hi = pair(qv[4], qv[5]) | (pair(qv[6], qv[7]) << 16);
-      } else {
-#pragma unroll
-        for (int j = 0; j < 4; ++j) {
-          lo |= (uint32_t)f32_to_e4m3_bits(__fdiv_rn(v[j], s)) << (8 * j);
-          hi |= (uint32_t)f32_to_e4m3_bits(__fdiv_rn(v[4 + j], s)) << (8 * j);
-        }
-      }
-      dst[c] = make_uint2(lo, hi);
+      dst[c] = quant8(v, s, rcp, finite);
     }
     if (lane == 0) scale[p] = s;
   }
@@ -259,10 +225,9 @@ moe_sum_kernel(const T* __restrict__ z, int64_t Tn, int k, int64_t H, float scal
 }  // namespace
 }  // namespace fmoe
 
-extern "C" int fmoe_quant_fp8_group128(const void* x, int in_dtype, int64_t rows_out, int64_t K,
-                                       const int32_t* row_map, int map_div, int64_t map_sentinel,
-                                       const int32_t* num_rows_dev, void* q, float* scale, void* stream) {
-  using namespace fmoe;
+int fmoe::run_quant_group128(const void* x, int in_dtype, int64_t rows_out, int64_t K, const int32_t* row_map, int map_div,
+                             int64_t map_sentinel, const int32_t* num_rows_dev, void* q, float* scale, bool zero_padding,
+                             cudaStream_t st) {
   FMOE_REQUIRE(K > 0 && K % 128 == 0, "quant_fp8_group128: K must be a positive multiple of 128 (got %lld)", (long long)K);
   FMOE_REQUIRE(in_dtype == FMOE_BF16 || in_dtype == FMOE_F32, "quant_fp8_group128: in_dtype must be bf16 or f32");
   FMOE_REQUIRE(!row_map || map_div >= 0, "quant_fp8_group128: map_div must be >= 0");
@@ -271,20 +236,25 @@ extern "C" int fmoe_quant_fp8_group128(const void* x, int in_dtype, int64_t rows
   FMOE_REQUIRE(aligned16(x) && (reinterpret_cast<uintptr_t>(q) & 7u) == 0, "quant_fp8_group128: misaligned pointer");
   // 16 teams per CTA, 4 items per team and pass
   unsigned grid = (unsigned)std::max<int64_t>(1, std::min<int64_t>(ceil_div<int64_t>(rows_out * (K / 128), 64), 148 * 8));
-  auto st = (cudaStream_t)stream;
   if (in_dtype == FMOE_BF16)
     launch_pdl(quant_group128_kernel<__nv_bfloat16>, dim3(grid), dim3(256), 0, st, (const __nv_bfloat16*)x, rows_out, K,
-               row_map, map_div, map_sentinel, num_rows_dev, (uint8_t*)q, scale);
+               row_map, map_div, map_sentinel, num_rows_dev, (uint8_t*)q, scale, (int)zero_padding);
   else
     launch_pdl(quant_group128_kernel<float>, dim3(grid), dim3(256), 0, st, (const float*)x, rows_out, K, row_map,
-               map_div, map_sentinel, num_rows_dev, (uint8_t*)q, scale);
+               map_div, map_sentinel, num_rows_dev, (uint8_t*)q, scale, (int)zero_padding);
   return launch_status("quant_group128_kernel");
 }
 
-extern "C" int fmoe_quant_fp8_per_token(const void* x, int in_dtype, int64_t rows_out, int64_t K,
-                                        const int32_t* row_map, int map_div, int64_t map_sentinel,
-                                        const int32_t* num_rows_dev, void* q, float* scale, void* stream) {
-  using namespace fmoe;
+extern "C" int fmoe_quant_fp8_group128(const void* x, int in_dtype, int64_t rows_out, int64_t K,
+                                       const int32_t* row_map, int map_div, int64_t map_sentinel,
+                                       const int32_t* num_rows_dev, void* q, float* scale, void* stream) {
+  return fmoe::run_quant_group128(x, in_dtype, rows_out, K, row_map, map_div, map_sentinel, num_rows_dev, q, scale, true,
+                                  (cudaStream_t)stream);
+}
+
+int fmoe::run_quant_per_token(const void* x, int in_dtype, int64_t rows_out, int64_t K, const int32_t* row_map, int map_div,
+                              int64_t map_sentinel, const int32_t* num_rows_dev, void* q, float* scale, bool zero_padding,
+                              cudaStream_t st) {
   FMOE_REQUIRE(K > 0 && K % 8 == 0 && K <= 16384, "quant_fp8_per_token: K must be a multiple of 8 up to 16384 (got %lld)",
                (long long)K);
   FMOE_REQUIRE(in_dtype == FMOE_BF16, "quant_fp8_per_token: in_dtype must be bf16");
@@ -294,13 +264,20 @@ extern "C" int fmoe_quant_fp8_per_token(const void* x, int in_dtype, int64_t row
   FMOE_REQUIRE(aligned16(x) && (reinterpret_cast<uintptr_t>(q) & 7u) == 0, "quant_fp8_per_token: misaligned pointer");
   auto go = [&](auto kernel, int teams) {
     unsigned grid = (unsigned)std::min<int64_t>(ceil_div<int64_t>(rows_out, teams), 148 * 8);
-    launch_pdl(kernel, dim3(grid), dim3(256), 0, (cudaStream_t)stream, (const __nv_bfloat16*)x, rows_out, K, row_map,
-               map_div, map_sentinel, num_rows_dev, (uint8_t*)q, scale);
+    launch_pdl(kernel, dim3(grid), dim3(256), 0, st, (const __nv_bfloat16*)x, rows_out, K, row_map, map_div, map_sentinel,
+               num_rows_dev, (uint8_t*)q, scale, (int)zero_padding);
   };
   if (K <= 2048) go(quant_row_kernel<32, 8>, 8);         // a warp per row, 8 rows per CTA
   else if (K <= 4096) go(quant_row_kernel<32, 16>, 8);
   else go(quant_row_kernel<256, 8>, 1);                  // a CTA per row
   return launch_status("quant_row_kernel");
+}
+
+extern "C" int fmoe_quant_fp8_per_token(const void* x, int in_dtype, int64_t rows_out, int64_t K,
+                                        const int32_t* row_map, int map_div, int64_t map_sentinel,
+                                        const int32_t* num_rows_dev, void* q, float* scale, void* stream) {
+  return fmoe::run_quant_per_token(x, in_dtype, rows_out, K, row_map, map_div, map_sentinel, num_rows_dev, q, scale, true,
+                                   (cudaStream_t)stream);
 }
 
 int fmoe::run_gather_rows(const void* x, int elem_bytes, int64_t rows_out, int64_t K, const int32_t* row_map, int map_div,

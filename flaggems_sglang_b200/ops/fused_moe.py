@@ -26,6 +26,7 @@ import torch
 
 from .. import _C
 from .moe_align_block_size import moe_align_block_size
+from .topk import _prep_logits
 from .topk import topk as _route
 
 logger = logging.getLogger(__name__)
@@ -179,6 +180,17 @@ def fused_experts(
     src/flaggems_sglang/ops/fused_moe.py:192-199), read in place by the bf16 tensor-core kernels as an N-major
     operand; see `n_major_supported` for the shapes this covers.
     """
+    return _experts(hidden_states, w1, w2, topk_weights, topk_ids, None, topk_ids.shape[1] if topk_ids.ndim == 2 else 0, inplace,
+                    activation, apply_router_weight_on_input, use_fp8_w8a8, per_channel_quant, w1_scale, w2_scale, a1_scale,
+                    a2_scale, block_shape, no_combine, routed_scaling_factor, expert_map, variant, out_rows, b1, b2, gemm1_alpha,
+                    gemm1_clamp_limit, weights_n_major)
+
+
+def _experts(hidden_states, w1, w2, topk_weights, topk_ids, route, k, inplace=False, activation="silu",
+             apply_router_weight_on_input=False, use_fp8_w8a8=False, per_channel_quant=False, w1_scale=None, w2_scale=None,
+             a1_scale=None, a2_scale=None, block_shape=None, no_combine=False, routed_scaling_factor=None, expert_map=None,
+             variant=None, out_rows=None, b1=None, b2=None, gemm1_alpha=None, gemm1_clamp_limit=None, weights_n_major=False):
+    """`fused_experts`, or with `route` (a filled _C.RouteArgs: logits of [T,E]) the router and the experts in one call."""
     logger.debug("FLAGGEMS_SGLANG_B200 FUSED_EXPERTS")
     assert inplace is False, "Inplace is not supported"
     assert a1_scale is None, _UNSUPPORTED_FEATURE_MSG.format(name="a1_scale")
@@ -200,8 +212,7 @@ def fused_experts(
     I = twoI // 2
     assert Hw == H, "hidden size mismatch"
     assert w2.shape[0] == E and w2.shape[1] == H and w2.shape[2] == I, "intermediate size mismatch"
-    assert topk_ids.shape == topk_weights.shape and topk_ids.shape[0] == T, "topk shape mismatch"
-    k = topk_ids.shape[1]
+    assert route is not None or (topk_ids.shape == topk_weights.shape and topk_ids.shape[0] == T), "topk shape mismatch"
     numel = T * k
 
     if per_channel_quant:
@@ -235,11 +246,12 @@ def fused_experts(
     if not weights_n_major:
         w1 = w1.contiguous()
         w2 = w2.contiguous()
-    wts = topk_weights.float().contiguous()
-    ids = topk_ids
-    if expert_map is not None:
-        ids = expert_map.to(torch.int32)[topk_ids.long()]
-    ids = ids.to(torch.int32).contiguous()
+    if route is None:
+        wts = topk_weights.float().contiguous()
+        ids = topk_ids
+        if expert_map is not None:
+            ids = expert_map.to(torch.int32)[topk_ids.long()]
+        ids = ids.to(torch.int32).contiguous()
 
     if b1 is not None or b2 is not None or activation == "swiglu_oai":
         assert not use_fp8_w8a8, "bias / swiglu_oai are not available with fp8 weights"
@@ -274,14 +286,15 @@ def fused_experts(
             zero_dropped=int(expert_map is not None), activation=_C.ACTIVATIONS[activation], T=T, H=H, I=I,
             routed_scaling_factor=1.0 if routed_scaling_factor is None else float(routed_scaling_factor),
             hidden=x.data_ptr(), w1=w1.data_ptr(), w2=w2.data_ptr(), w1_scale=_C.ptr(w1_scale),
-            w2_scale=_C.ptr(w2_scale), topk_weights=wts.data_ptr(), topk_ids=ids.data_ptr(), out=_C.ptr(out),
+            w2_scale=_C.ptr(w2_scale), topk_weights=None if route is not None else wts.data_ptr(),
+            topk_ids=None if route is not None else ids.data_ptr(), out=_C.ptr(out),
             out_rows=_C.ptr(out_rows), b1=_C.ptr(b1), b2=_C.ptr(b2), act_alpha=act_alpha, act_limit=act_limit)
-        need = lib.fmoe_fused_experts_workspace_bytes(fa)
+        need = lib.fmoe_fused_experts_workspace_bytes(fa) if route is None else lib.fmoe_fused_moe_workspace_bytes(fa, route)
         if need < 0:
             _C.check(_C.ERR_INVALID_ARG)
         ws = torch.empty(max(int(need), 256), dtype=torch.uint8, device=dev)
         fa.workspace, fa.workspace_bytes = ws.data_ptr(), ws.numel()
-        _C.check(lib.fmoe_fused_experts(fa, st))
+        _C.check(lib.fmoe_fused_experts(fa, st) if route is None else lib.fmoe_fused_moe(fa, route, st))
         return out
 
     # profiling path (STAGE_EVENTS set): the same kernels launched one by one with events around each launch
@@ -410,6 +423,12 @@ def fused_experts(
     return out
 
 
+# fused_experts' options that the one-call layer takes (global_num_experts is accepted there and has no effect)
+_EXPERT_OPTIONS = frozenset(("inplace", "activation", "apply_router_weight_on_input", "use_fp8_w8a8", "per_channel_quant",
+                             "w1_scale", "w2_scale", "a1_scale", "a2_scale", "block_shape", "no_combine", "variant", "b1", "b2",
+                             "gemm1_alpha", "gemm1_clamp_limit", "weights_n_major"))
+
+
 def fused_moe(
     hidden_states: torch.Tensor,
     w1: torch.Tensor,
@@ -429,6 +448,23 @@ def fused_moe(
     `routed_scaling_factor` is applied exactly once, after the combine
     (as the reference hook does, src/flaggems_sglang/ops/fused_moe.py:415-420).
     """
+    if STAGE_EVENTS is None and kwargs.get("expert_map") is None and gating_output.ndim == 2 and \
+            gating_output.shape[1] == w1.shape[0] and (not use_grouped_topk or (num_expert_group and topk_group)) and \
+            all(name in _EXPERT_OPTIONS for name in kwargs):
+        # router and experts in one library call
+        g = _prep_logits(gating_output)
+        T, E = g.shape
+        if hidden_states.shape[0] != T:
+            raise ValueError("Number of tokens mismatch")
+        bias = None
+        if use_grouped_topk and correction_bias is not None:
+            _C.require_cuda(correction_bias)
+            bias = correction_bias.float().contiguous()
+            if bias.numel() != E:
+                raise ValueError("correction_bias must have num_experts entries")
+        route = _C.RouteArgs(g.data_ptr(), _C.ptr(bias), int(use_grouped_topk), int(renormalize),
+                             num_expert_group if use_grouped_topk else 1, topk_group if use_grouped_topk else 1)
+        return _experts(hidden_states, w1, w2, None, None, route, topk, routed_scaling_factor=routed_scaling_factor, **kwargs)
     w, ids = _route(hidden_states, gating_output, topk, renormalize, use_grouped_topk, num_expert_group,
                     topk_group, correction_bias, None)
     return fused_experts(hidden_states, w1, w2, w, ids, routed_scaling_factor=routed_scaling_factor, **kwargs)

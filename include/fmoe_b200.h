@@ -290,6 +290,21 @@ int64_t fmoe_fused_experts_workspace_bytes(const fmoe_fused_args* args);
 int fmoe_fused_experts(const fmoe_fused_args* args, void* stream);
 
 /*
+ * The whole layer from router logits: router (fmoe_topk_softmax or fmoe_topk_grouped with scale 1), then
+ * fmoe_fused_experts on its result; args->topk_weights / topk_ids are ignored.  Takes over what the reference's caller
+ * does before the operator (tests/test_fused_moe.py:38-41) together with the operator.
+ */
+typedef struct fmoe_route_args {
+  const float* logits;          /* [T,E] f32                                                              */
+  const float* correction_bias; /* grouped: optional [E] f32                                              */
+  int32_t grouped;              /* 0: softmax top-k; 1: sigmoid scores, group-limited                     */
+  int32_t renormalize;
+  int32_t n_group, topk_group;  /* grouped only                                                           */
+} fmoe_route_args;
+int64_t fmoe_fused_moe_workspace_bytes(const fmoe_fused_args* args, const fmoe_route_args* route);
+int fmoe_fused_moe(const fmoe_fused_args* args, const fmoe_route_args* route, void* stream);
+
+/*
  * fmoe_fused_experts for callers that cannot allocate device memory.  It has no counterpart in the
  * reference, which allocates its intermediates with torch on every call.
  *
