@@ -5,8 +5,8 @@
 //   K step    : 128 bytes per row (64 bf16 / 128 e4m3), one 128-byte swizzle atom; 4 MMAs per step
 //   pipeline  : 192 KB ring of 6, 8 or 9 stages (16 KB of weights + 16, 8 or 4 KB of tokens) per CTA
 //   TMEM      : 512 columns per CTA = two 128 x 256 fp32 accumulators, so the epilogue of a tile overlaps the next tile
-//   warps     : 0-7 epilogue (TMEM lane quarter = warp % 4; the two halves take alternate 16-token chunks),
-//               8 TMA producer (each CTA its own weight rows and its own half of the tokens), 9 MMA issuer (CTA 0)
+//   warps     : 0-15 epilogue (TMEM lane quarter = warp % 4; the four of a quarter take 16-token chunks in turn),
+//               16 TMA producer (each CTA its own weight rows and its own half of the tokens), 17 MMA issuer (CTA 0)
 //
 // Why pairs: with one CTA per 128 x 256 tile an MMA reads 12 KB of shared memory for every 8 KB here, and TMA writes as
 // much; fill and operand reads of one SM together ran into its 128 bytes per clock.  Why weights on M: see pair.cuh.
@@ -42,15 +42,17 @@ constexpr int MAX_STAGES = 9;
 constexpr int stage_bytes(int token_tile) { return W_BYTES + token_tile / 2 * KBYTES; }
 constexpr int TMEM_COLS = 512;
 constexpr int ACC_COLS = 256;
-constexpr int kEpiWarps = 8;
-constexpr int kThreads = (kEpiWarps + 2) * 32;
+// Epilogue warps: 16 (4 per TMEM lane quarter), so that their TMEM, shuffle, shared-memory and store latencies overlap;
+// with 8 a short main loop waited for them (7.3k cycles per tile against 6.1k of MMAs at K = 768).  The gate/up exchange of
+// M-major weights needs shared memory per group of four, so that kernel keeps 8.
+constexpr int epi_warps(bool exchange) { return exchange ? 8 : 16; }
 constexpr int BOX_TOKENS = 32;                      // token rows per TMA box
-constexpr int STRIP_BYTES = 16 * 80;                // per warp: 16 tokens x (32 channels + 8 of padding: no bank conflicts)
+constexpr int STRIP_BYTES = kStripBytes;
 constexpr int EX_PITCH = 20;                        // floats per lane row of the gate/up exchange (16 tokens + padding)
 constexpr int EX_BYTES = 128 * EX_PITCH * 4;        // per half of the epilogue warps
 constexpr int BAR_BYTES = 256;
 constexpr int smem_bytes(int num_experts, bool exchange) {
-  return RING_BYTES + BAR_BYTES + (exchange ? 2 * EX_BYTES : kEpiWarps * STRIP_BYTES) + pair_table_bytes(num_experts);
+  return RING_BYTES + BAR_BYTES + (exchange ? 2 * EX_BYTES : epi_warps(false) * STRIP_BYTES) + pair_table_bytes(num_experts);
 }
 static_assert(smem_bytes(1024, true) <= 227 * 1024, "shared memory");
 
@@ -100,9 +102,10 @@ __device__ __forceinline__ int32_t ld_acquire_gpu(const int32_t* p) {
 }
 
 template <bool GATED, bool F8, bool EXTRA, bool WMN, bool GATHER>
-__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 1)
+__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__((epi_warps(GATED && WMN) + 2) * 32, 1)
 grouped_gemm_pair_kernel(const __grid_constant__ CUtensorMap map_t, const __grid_constant__ CUtensorMap map_w,
                          const PairParams p) {
+  constexpr int kEpiWarps = epi_warps(GATED && WMN), HALVES = kEpiWarps / 4;  // warps per lane quarter
   extern __shared__ __align__(1024) uint8_t smem[];  // aligned by declaration: every address below is a constant
   const int stages = p.stages, stage_size = p.stage_bytes;
   uint64_t* bars = reinterpret_cast<uint64_t*>(smem + RING_BYTES);
@@ -282,7 +285,7 @@ grouped_gemm_pair_kernel(const __grid_constant__ CUtensorMap map_t, const __grid
       }
     }
   } else {
-    // ---------------- epilogue (warps 0-7 of both CTAs, each its CTA's 128 weight rows) ----------------
+    // ---------------- epilogue (both CTAs, each its CTA's 128 weight rows) ----------------
     const int quarter = warp & 3, half = warp >> 2;
     const int g = lane >> 2, t = lane & 3;
     uint8_t* strip = strips + warp * STRIP_BYTES;
@@ -296,14 +299,15 @@ grouped_gemm_pair_kernel(const __grid_constant__ CUtensorMap map_t, const __grid
       const int acc = local & 1;
       const uint32_t acc_phase = (local >> 1) & 1;
       ++local;
-      const int chunks = tl.n >> 4;  // 16-token chunks; this warp takes those with the parity of `half`
+      const int chunks = tl.n >> 4;  // 16-token chunks; this warp takes those that are `half` modulo HALVES
       // token f = 16 * c + u of the warp's c-th chunk sits in register f / 32 of lane f % 32
-      int32_t slot_r[4];
-      float rs_r[4];
+      constexpr int REGS = 8 / HALVES;
+      int32_t slot_r[REGS];
+      float rs_r[REGS];
 #pragma unroll
-      for (int r = 0; r < 4; ++r) {
+      for (int r = 0; r < REGS; ++r) {
         const int f = r * 32 + lane;
-        const int tok = (2 * (f >> 4) + half) * 16 + (f & 15);
+        const int tok = (HALVES * (f >> 4) + half) * 16 + (f & 15);
         slot_r[r] = -1;
         rs_r[r] = 1.0f;
         if (tok < tl.cols) {
@@ -352,7 +356,7 @@ grouped_gemm_pair_kernel(const __grid_constant__ CUtensorMap map_t, const __grid
       };
       if (split) {
 #pragma unroll 1
-        for (int j = half; j < chunks; j += 2) {
+        for (int j = half; j < chunks; j += HALVES) {
           if (j >= c_begin && j < c_end) continue;
           uint32_t lo[8], hi[8];
           ptx::tmem_ld_16x256b_x2(taddr + j * 16, lo);
@@ -385,13 +389,26 @@ grouped_gemm_pair_kernel(const __grid_constant__ CUtensorMap map_t, const __grid
           break;
         }
       }
+      // first chunk of this warp inside the strip; the next one's TMEM read-out is in flight while a chunk is stored
+      int j = half + ((max(c_begin - half, 0) + HALVES - 1) / HALVES) * HALVES;
+      uint32_t nlo[8], nhi[8];
+      if (j < c_end) {
+        ptx::tmem_ld_16x256b_x2(taddr + j * 16, nlo);                // rows 0-15 of the quarter (gated: gate)
+        ptx::tmem_ld_16x256b_x2(taddr + (16u << 16) + j * 16, nhi);  // rows 16-31 (gated: up)
+      }
 #pragma unroll 1
-      for (int j = half; j < chunks; j += 2) {
-        if (j < c_begin || j >= c_end) continue;
+      for (; j < c_end; j += HALVES) {
         uint32_t lo[8], hi[8];
-        ptx::tmem_ld_16x256b_x2(taddr + j * 16, lo);                // rows 0-15 of the quarter (gated: gate)
-        ptx::tmem_ld_16x256b_x2(taddr + (16u << 16) + j * 16, hi);  // rows 16-31 (gated: up)
         ptx::tmem_ld_wait();
+#pragma unroll
+        for (int i = 0; i < 8; ++i) {
+          lo[i] = nlo[i];
+          hi[i] = nhi[i];
+        }
+        if (j + HALVES < c_end) {
+          ptx::tmem_ld_16x256b_x2(taddr + (j + HALVES) * 16, nlo);
+          ptx::tmem_ld_16x256b_x2(taddr + (16u << 16) + (j + HALVES) * 16, nhi);
+        }
         if (S > 1) {
           for (int o = 0; o < S; ++o) {
             if (o == slice) continue;
@@ -408,9 +425,16 @@ grouped_gemm_pair_kernel(const __grid_constant__ CUtensorMap map_t, const __grid
           }
         }
         // the chunk's 16 slots and row scales, from the lanes that hold them
-        const int c = j >> 1;
-        const int32_t slot_c = (c >> 1) == 0 ? slot_r[0] : (c >> 1) == 1 ? slot_r[1] : (c >> 1) == 2 ? slot_r[2] : slot_r[3];
-        const float rs_c = (c >> 1) == 0 ? rs_r[0] : (c >> 1) == 1 ? rs_r[1] : (c >> 1) == 2 ? rs_r[2] : rs_r[3];
+        const int c = j / HALVES;
+        int32_t slot_c = slot_r[0];
+        float rs_c = rs_r[0];
+#pragma unroll
+        for (int r = 1; r < REGS; ++r) {
+          if ((c >> 1) == r) {
+            slot_c = slot_r[r];
+            rs_c = rs_r[r];
+          }
+        }
         const int src_lane = (c & 1) * 16;
         if constexpr (GATED && WMN) {
           // gate rows are lanes 0-63, up rows 64-127: the four warps of a half meet in shared memory
@@ -463,19 +487,10 @@ grouped_gemm_pair_kernel(const __grid_constant__ CUtensorMap map_t, const __grid
               }
               m[q] = pack_bf16x2(o[0], o[1]);
             }
-            constexpr int PITCH = 48;  // 16 channels + 8 of padding
-            const int tok_l = (lane & 7) + (lane >> 4) * 8, ch_l = ((lane >> 3) & 1) * 8;
-            ptx::stmatrix_x4_trans(ptx::smem_u32(strip + tok_l * PITCH + ch_l * 2), m[0], m[1], m[2], m[3]);
-            __syncwarp();
-            const int u = lane >> 1, part = (lane & 1) * 8;
-            const uint4 v = *reinterpret_cast<const uint4*>(strip + u * PITCH + part * 2);
-            const int tok = j * 16 + u;
-            if (tok < tl.cols && ch0 + part < p.n)
-              *reinterpret_cast<uint4*>(reinterpret_cast<__nv_bfloat16*>(p.out) + (int64_t)(tl.row0 + tok) * p.n + ch0 + part) = v;
-            __syncwarp();
+            strip_put16(strip, 48, 0, lane, m);
+            strip_store_sorted(strip, lane, reinterpret_cast<__nv_bfloat16*>(p.out) + (int64_t)(tl.row0 + j * 16) * p.n, p.n, ch0,
+                               tl.cols - j * 16);
           } else {
-            constexpr int PITCH = 80;  // 32 channels + 8 of padding
-            const int tok_l = (lane & 7) + (lane >> 4) * 8, ch_l = ((lane >> 3) & 1) * 8;
 #pragma unroll
             for (int h = 0; h < 2; ++h) {
               uint32_t m[4];
@@ -488,21 +503,10 @@ grouped_gemm_pair_kernel(const __grid_constant__ CUtensorMap map_t, const __grid
                 if constexpr (F8) m[q] = pack_bf16x2(v0 * r0 * c0, v1 * r1 * c0);
                 else m[q] = pack_bf16x2((v0 + c0) * r0, (v1 + c0) * r1);
               }
-              ptx::stmatrix_x4_trans(ptx::smem_u32(strip + tok_l * PITCH + (16 * h + ch_l) * 2), m[0], m[1], m[2], m[3]);
+              strip_put16(strip, 80, 16 * h, lane, m);
             }
-            __syncwarp();
-#pragma unroll
-            for (int h = 0; h < 2; ++h) {
-              const int u = (lane >> 2) + 8 * h, part = (lane & 3) * 8;
-              const uint4 v = *reinterpret_cast<const uint4*>(strip + u * PITCH + part * 2);
-              const int32_t slot = __shfl_sync(0xffffffffu, slot_c, src_lane + u);
-              if (slot >= 0 && ch0 + part < p.n) {
-                __nv_bfloat16* orow = p.out_rows ? reinterpret_cast<__nv_bfloat16*>(p.out_rows[slot])
-                                                 : reinterpret_cast<__nv_bfloat16*>(p.out) + (int64_t)slot * p.n;
-                if (orow) *reinterpret_cast<uint4*>(orow + ch0 + part) = v;
-              }
-            }
-            __syncwarp();
+            strip_store_slots(strip, lane, p.out, p.out_rows, p.n, ch0, __shfl_sync(0xffffffffu, slot_c, src_lane + (lane >> 2)),
+                              __shfl_sync(0xffffffffu, slot_c, src_lane + 8 + (lane >> 2)));
           }
         }
       }
@@ -511,15 +515,8 @@ grouped_gemm_pair_kernel(const __grid_constant__ CUtensorMap map_t, const __grid
       __syncwarp();
       if (lane == 0) ptx::mbar_arrive_cluster(ptx::smem_u32(&acc_empty[acc]) & ~ptx::kPeerRankBit);
       if constexpr (GATED) {
-        if (p.zero_padding && tl.last && slice == 0) {
-          const int end = (tl.row0 + tl.cols + 127) & ~127;  // blocks start at multiples of 128 rows
-          const int tile_ch = tl.w_tile * 128 + rank * 64;
-          for (int i = threadIdx.x; i < (end - tl.row0 - tl.cols) * 8; i += kEpiWarps * 32) {
-            const int64_t row = tl.row0 + tl.cols + (i >> 3), ch = tile_ch + (i & 7) * 8;
-            if (ch < p.n)
-              *reinterpret_cast<uint4*>(reinterpret_cast<__nv_bfloat16*>(p.out) + row * p.n + ch) = make_uint4(0, 0, 0, 0);
-          }
-        }
+        if (p.zero_padding && tl.last && slice == 0)
+          zero_block_rows(tl, p.out, p.n, tl.w_tile * 128 + rank * 64, kEpiWarps * 32);
       }
       if (p.profile) prof_busy += clock64() - te1;
     }
@@ -715,7 +712,7 @@ int launch(const GemmParams& g, cudaStream_t st) {
       FMOE_CUDA_OK(cudaMemsetAsync(g.split_ws, 0, 1024, st));
     }
   }
-  launch_pdl(kernel, dim3(2 * workers), dim3(kThreads), smem, st, map_t, map_w, p);
+  launch_pdl(kernel, dim3(2 * workers), dim3((epi_warps(GATED && WMN) + 2) * 32), smem, st, map_t, map_w, p);
   return launch_status("grouped_gemm_pair_kernel");
 }
 
