@@ -111,6 +111,8 @@ SIGNATURES = {
     "fmoe_fused_experts": (c_int, [POINTER(FusedArgs), c_void_p]),
     "fmoe_fused_moe_workspace_bytes": (c_int64, [POINTER(FusedArgs), POINTER(RouteArgs)]),
     "fmoe_fused_moe": (c_int, [POINTER(FusedArgs), POINTER(RouteArgs), c_void_p]),
+    "fmoe_fused_experts_sorted_workspace_bytes": (c_int64, [POINTER(FusedArgs)]),
+    "fmoe_fused_experts_sorted": (c_int, [POINTER(FusedArgs), c_void_p, c_void_p, c_void_p, c_void_p]),
     "fmoe_static_scratch_bytes": (c_int64, []),
     "fmoe_fused_experts_static": (c_int, [POINTER(FusedArgs), c_void_p]),
     "fmoe_ep_buffer_create": (c_int, [c_int64, POINTER(c_void_p), c_void_p]),

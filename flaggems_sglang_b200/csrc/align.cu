@@ -4,8 +4,8 @@
 // counts its chunk per expert, a scan over (expert, warp) turns the counts into
 // the first output position of every (warp, expert) pair, and a second pass over
 // the chunk places each slot at base + (its rank among the equal ids seen so
-// far), which keeps slots of an expert in ascending order.  The ranks inside a
-// group of 32 slots come from __match_any_sync.
+// far), which keeps slots of an expert in ascending order.  The ranks inside
+// a group of 32 slots come from warp ballots.
 #include "align.cuh"
 
 namespace fmoe {
@@ -13,6 +13,25 @@ namespace {
 
 constexpr int kThreads = 1024;
 constexpr int kWarps = kThreads / 32;
+constexpr int kBatch = 4;
+
+// Lanes of the warp whose id equals this lane's (ids below 2^bits; lanes without an id pass -1 and get the other such
+// lanes).  One ballot per id bit: __match_any_sync took most of the 21 us of a single-CTA sort of 8192 slots.
+__device__ __forceinline__ unsigned warp_peers(int id, int bits) {
+  const bool on = id >= 0;
+  unsigned peers = __ballot_sync(0xffffffffu, on);
+  if (!on) peers = ~peers;
+  for (int b = 0; b < bits; ++b) {
+    const unsigned m = __ballot_sync(0xffffffffu, (id >> b) & 1);
+    peers &= ((id >> b) & 1) ? m : ~m;
+  }
+  return peers;
+}
+__host__ __device__ inline int id_bits(int E) {
+  int b = 0;
+  while ((1 << b) < E) ++b;
+  return b;
+}
 
 // One warp: exclusive scan of the padded row counts -> s_start[E + 1] and num_post_pad; with `table`, also the experts'
 // first rows, rows and token tiles for the CTA-pair GEMMs (pair.cuh).  E <= 1024: 32 experts per step.
@@ -60,30 +79,39 @@ moe_align_kernel(const int32_t* __restrict__ topk_ids, int numel, int E, int blo
   int* s_cnt = s_mem;                  // [kWarps][E] counts, then running output positions
   int* s_total = s_mem + kWarps * E;   // [E] per-expert count
   int* s_start = s_total + E;          // [E+1] padded start of each expert
-  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, bits = id_bits(E);
 
   for (int i = tid; i < kWarps * E; i += kThreads) s_cnt[i] = 0;
-  for (int i = tid; i < sorted_cap; i += kThreads) sorted_ids[i] = numel;
   for (int i = tid; i < num_zero; i += kThreads) zero_words[i] = 0;
   __syncthreads();
 
   const int chunk = ceil_div(ceil_div(numel, kWarps), 32) * 32;  // multiple of 32 per warp
   const int lo = min(warp * chunk, numel), hi = min(lo + chunk, numel);
 
-  // pass 1: per-warp histogram
-  for (int base = lo; base < hi; base += 32) {
-    int s = base + lane;
-    int e = (s < hi) ? topk_ids[s] : -1;
-    bool ok = (e >= 0 && e < E);
-    unsigned peers = __match_any_sync(0xffffffffu, ok ? e : -1);
-    if (ok && (__ffs(peers) - 1) == lane) s_cnt[warp * E + e] += __popc(peers);
-    __syncwarp();
+  // pass 1: per-warp histogram (kBatch ids per lane loaded before the first is counted)
+  for (int base = lo; base < hi; base += 32 * kBatch) {
+    int id[kBatch];
+#pragma unroll
+    for (int i = 0; i < kBatch; ++i) {
+      const int s = base + 32 * i + lane;
+      id[i] = (s < hi) ? topk_ids[s] : -1;
+    }
+#pragma unroll
+    for (int i = 0; i < kBatch; ++i) {
+      if (base + 32 * i >= hi) break;
+      const int e = id[i];
+      const bool ok = (e >= 0 && e < E);
+      const unsigned peers = warp_peers(ok ? e : -1, bits);
+      if (ok && (__ffs(peers) - 1) == lane) s_cnt[warp * E + e] += __popc(peers);
+      __syncwarp();
+    }
   }
   __syncthreads();
 
   // scan over warps for each expert: s_cnt[w][e] <- number of slots of e in warps < w
   for (int e = tid; e < E; e += kThreads) {
     int run = 0;
+#pragma unroll 8
     for (int w = 0; w < kWarps; ++w) {
       int c = s_cnt[w * E + e];
       s_cnt[w * E + e] = run;
@@ -103,21 +131,34 @@ moe_align_kernel(const int32_t* __restrict__ topk_ids, int numel, int E, int blo
     for (int b = b0; b < b1 && b < expert_cap; ++b) expert_ids[b] = e;
   }
   for (int b = used_blocks + tid; b < expert_cap; b += kThreads) expert_ids[b] = -1;
+  // sentinels: the padding of every expert, and everything past the used blocks
+  for (int e = warp; e < E; e += kWarps)
+    for (int i = s_start[e] + s_total[e] + lane; i < s_start[e + 1]; i += 32) sorted_ids[i] = numel;
+  for (int i = s_start[E] + tid; i < sorted_cap; i += kThreads) sorted_ids[i] = numel;
 
   // pass 2: stable scatter
-  for (int base = lo; base < hi; base += 32) {
-    int s = base + lane;
-    int e = (s < hi) ? topk_ids[s] : -1;
-    bool ok = (e >= 0 && e < E);
-    unsigned peers = __match_any_sync(0xffffffffu, ok ? e : -1);
-    if (ok) {
-      int rank = __popc(peers & ((1u << lane) - 1u));
-      int pos = s_start[e] + s_cnt[warp * E + e] + rank;
-      if (pos < sorted_cap) sorted_ids[pos] = s;
+  for (int base = lo; base < hi; base += 32 * kBatch) {
+    int id[kBatch];
+#pragma unroll
+    for (int i = 0; i < kBatch; ++i) {
+      const int s = base + 32 * i + lane;
+      id[i] = (s < hi) ? topk_ids[s] : -1;
     }
-    __syncwarp();
-    if (ok && (__ffs(peers) - 1) == lane) s_cnt[warp * E + e] += __popc(peers);
-    __syncwarp();
+#pragma unroll
+    for (int i = 0; i < kBatch; ++i) {
+      if (base + 32 * i >= hi) break;
+      const int s = base + 32 * i + lane, e = id[i];
+      const bool ok = (e >= 0 && e < E);
+      const unsigned peers = warp_peers(ok ? e : -1, bits);
+      if (ok) {
+        const int rank = __popc(peers & ((1u << lane) - 1u));
+        const int pos = s_start[e] + s_cnt[warp * E + e] + rank;
+        if (pos < sorted_cap) sorted_ids[pos] = s;
+      }
+      __syncwarp();
+      if (ok && (__ffs(peers) - 1) == lane) s_cnt[warp * E + e] += __popc(peers);
+      __syncwarp();
+    }
   }
 }
 
@@ -126,13 +167,16 @@ moe_align_kernel(const int32_t* __restrict__ topk_ids, int numel, int E, int blo
 //   count   : per-chunk histogram -> cnt[chunk][E]; sentinel fill of sorted_token_ids
 //   scan    : one CTA: exclusive scan over chunks per expert, padded starts, expert_ids, total
 //   scatter : every CTA redoes its chunk's per-warp histogram and places its slots (stable)
-// cnt lives in caller scratch (chunks * E ints).
+// cnt and the experts' starts live in caller scratch ((chunks + 1) * E ints).
 // ---------------------------------------------------------------------------------------------
 constexpr int kChunk = 4096;
+// Up to here one CTA is faster than three dependent launches.
+constexpr int kSingleCtaSlots = 4 * kChunk;
 
 __global__ void __launch_bounds__(kThreads)
 align_count_kernel(const int32_t* __restrict__ topk_ids, int numel, int E, int32_t* __restrict__ sorted_ids,
                    int sorted_cap, int32_t* __restrict__ cnt) {
+  pdl_entry();
   extern __shared__ int s_mem[];  // [E]
   const int tid = threadIdx.x;
   for (int e = tid; e < E; e += kThreads) s_mem[e] = 0;
@@ -140,18 +184,25 @@ align_count_kernel(const int32_t* __restrict__ topk_ids, int numel, int E, int32
     sorted_ids[i] = numel;
   __syncthreads();
   const int lo = blockIdx.x * kChunk, hi = min(lo + kChunk, numel);
-  for (int s = lo + tid; s < hi; s += kThreads) {
-    int e = topk_ids[s];
-    if (e >= 0 && e < E) atomicAdd(&s_mem[e], 1);
+  int id[kChunk / kThreads];
+#pragma unroll
+  for (int i = 0; i < kChunk / kThreads; ++i) {
+    const int s = lo + tid + i * kThreads;
+    id[i] = s < hi ? topk_ids[s] : -1;
   }
+#pragma unroll
+  for (int i = 0; i < kChunk / kThreads; ++i)
+    if (id[i] >= 0 && id[i] < E) atomicAdd(&s_mem[id[i]], 1);
   __syncthreads();
   for (int e = tid; e < E; e += kThreads) cnt[blockIdx.x * E + e] = s_mem[e];
 }
 
 __global__ void __launch_bounds__(kThreads)
-align_scan_kernel(int chunks, int E, int block, int32_t* __restrict__ cnt, int32_t* __restrict__ expert_ids,
+align_scan_kernel(int chunks, int E, int block, int32_t* __restrict__ cnt, int32_t* __restrict__ starts,
+                  int32_t* __restrict__ expert_ids,
                   int expert_cap, int32_t* __restrict__ num_post_pad, int32_t* __restrict__ table, int token_tile,
                   int32_t* __restrict__ zero_words, int num_zero) {
+  pdl_entry();
   extern __shared__ int s_mem[];
   int* s_total = s_mem;      // [E]
   int* s_start = s_mem + E;  // [E+1]
@@ -159,10 +210,15 @@ align_scan_kernel(int chunks, int E, int block, int32_t* __restrict__ cnt, int32
   for (int i = tid; i < num_zero; i += kThreads) zero_words[i] = 0;
   for (int e = tid; e < E; e += kThreads) {
     int run = 0;
-    for (int c = 0; c < chunks; ++c) {
-      int v = cnt[c * E + e];
-      cnt[c * E + e] = run;  // slots of e in earlier chunks
-      run += v;
+    for (int c0 = 0; c0 < chunks; c0 += 8) {
+      int v[8];
+#pragma unroll
+      for (int i = 0; i < 8; ++i) v[i] = c0 + i < chunks ? cnt[(c0 + i) * E + e] : 0;
+#pragma unroll
+      for (int i = 0; i < 8; ++i) {
+        if (c0 + i < chunks) cnt[(c0 + i) * E + e] = run;  // slots of e in earlier chunks
+        run += v[i];
+      }
     }
     s_total[e] = run;
   }
@@ -173,31 +229,39 @@ align_scan_kernel(int chunks, int E, int block, int32_t* __restrict__ cnt, int32
   for (int e = tid; e < E; e += kThreads) {
     int b0 = s_start[e] / block, b1 = s_start[e + 1] / block;
     for (int b = b0; b < b1 && b < expert_cap; ++b) expert_ids[b] = e;
-    for (int c = 0; c < chunks; ++c) cnt[c * E + e] += s_start[e];  // absolute first position per (chunk, expert)
+    starts[e] = s_start[e];  // first position of the expert, for the scatter
   }
   for (int b = used_blocks + tid; b < expert_cap; b += kThreads) expert_ids[b] = -1;
 }
 
 __global__ void __launch_bounds__(kThreads)
 align_scatter_kernel(const int32_t* __restrict__ topk_ids, int numel, int E, const int32_t* __restrict__ cnt,
-                     int32_t* __restrict__ sorted_ids, int sorted_cap) {
+                     const int32_t* __restrict__ starts, int32_t* __restrict__ sorted_ids, int sorted_cap) {
+  pdl_entry();
   extern __shared__ int s_mem[];  // [kWarps][E] per-warp counts -> running positions
-  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, bits = id_bits(E);
   for (int i = tid; i < kWarps * E; i += kThreads) s_mem[i] = 0;
   __syncthreads();
   constexpr int per_warp = kChunk / kWarps;  // 128 contiguous slots per warp
   const int lo = min(blockIdx.x * kChunk + warp * per_warp, numel), hi = min(lo + per_warp, numel);
-  for (int base = lo; base < hi; base += 32) {
-    int s = base + lane;
-    int e = (s < hi) ? topk_ids[s] : -1;
-    bool ok = (e >= 0 && e < E);
-    unsigned peers = __match_any_sync(0xffffffffu, ok ? e : -1);
-    if (ok && (__ffs(peers) - 1) == lane) s_mem[warp * E + e] += __popc(peers);
+  int id[per_warp / 32];
+  unsigned peers[per_warp / 32];
+#pragma unroll
+  for (int i = 0; i < per_warp / 32; ++i) {
+    const int s = lo + 32 * i + lane;
+    id[i] = s < hi ? topk_ids[s] : -1;
+    if (id[i] >= E) id[i] = -1;
+  }
+#pragma unroll
+  for (int i = 0; i < per_warp / 32; ++i) {
+    peers[i] = warp_peers(max(id[i], -1), bits);
+    if (id[i] >= 0 && (__ffs(peers[i]) - 1) == lane) s_mem[warp * E + id[i]] += __popc(peers[i]);
     __syncwarp();
   }
   __syncthreads();
   for (int e = tid; e < E; e += kThreads) {
-    int run = cnt[blockIdx.x * E + e];
+    int run = cnt[blockIdx.x * E + e] + starts[e];
+#pragma unroll 8
     for (int w = 0; w < kWarps; ++w) {
       int c = s_mem[w * E + e];
       s_mem[w * E + e] = run;
@@ -205,19 +269,85 @@ align_scatter_kernel(const int32_t* __restrict__ topk_ids, int numel, int E, con
     }
   }
   __syncthreads();
-  for (int base = lo; base < hi; base += 32) {
-    int s = base + lane;
-    int e = (s < hi) ? topk_ids[s] : -1;
-    bool ok = (e >= 0 && e < E);
-    unsigned peers = __match_any_sync(0xffffffffu, ok ? e : -1);
-    if (ok) {
-      int pos = s_mem[warp * E + e] + __popc(peers & ((1u << lane) - 1u));
-      if (pos < sorted_cap) sorted_ids[pos] = s;
+#pragma unroll
+  for (int i = 0; i < per_warp / 32; ++i) {
+    if (id[i] >= 0) {
+      const int pos = s_mem[warp * E + id[i]] + __popc(peers[i] & ((1u << lane) - 1u));
+      if (pos < sorted_cap) sorted_ids[pos] = lo + 32 * i + lane;
     }
     __syncwarp();
-    if (ok && (__ffs(peers) - 1) == lane) s_mem[warp * E + e] += __popc(peers);
+    if (id[i] >= 0 && (__ffs(peers[i]) - 1) == lane) s_mem[warp * E + id[i]] += __popc(peers[i]);
     __syncwarp();
   }
+}
+
+// ---------------------------------------------------------------------------------------------
+// The same tables from slots that the caller already holds in expert order (the reference operator's routing triple:
+// sorted position -> slot, rows per expert, weights in sorted order): nothing is counted or sorted, every CTA scans the
+// E row counts and copies its share of the positions to their padded places.  Also writes expert and weight by slot.
+// ---------------------------------------------------------------------------------------------
+constexpr int kSortedThreads = 256;
+
+__global__ void __launch_bounds__(kSortedThreads)
+align_sorted_kernel(const int32_t* __restrict__ slot_of, const int32_t* __restrict__ hist, const float* __restrict__ gate, int numel,
+                    int E, int block, int32_t* __restrict__ sorted_ids, int sorted_cap, int32_t* __restrict__ expert_ids,
+                    int expert_cap, int32_t* __restrict__ num_post_pad, int32_t* __restrict__ table, int token_tile,
+                    int32_t* __restrict__ zero_words, int num_zero, int32_t* __restrict__ ids, float* __restrict__ weights) {
+  pdl_entry();
+  extern __shared__ int s_mem[];
+  int* s_total = s_mem;            // [E]
+  int* s_start = s_mem + E;        // [E+1] padded
+  int* s_first = s_start + E + 1;  // [E+1] unpadded
+  __shared__ int s_npp;
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, block_id = blockIdx.x;
+  for (int e = tid; e < E; e += kSortedThreads) s_total[e] = max(hist[e], 0);
+  __syncthreads();
+  if (warp == 0) scan_experts_warp(s_total, s_start, E, block, lane,
+                                   block_id == 0 && num_post_pad ? num_post_pad : &s_npp, block_id == 0 ? table : nullptr, token_tile);
+  if (warp == 1) {
+    int carry = 0;
+    for (int base = 0; base < E; base += 32) {
+      const int e = base + lane, v = e < E ? s_total[e] : 0;
+      int incl = v;
+#pragma unroll
+      for (int off = 1; off < 32; off <<= 1) {
+        const int w = __shfl_up_sync(0xffffffffu, incl, off);
+        if (lane >= off) incl += w;
+      }
+      if (e < E) s_first[e] = carry + incl - v;
+      carry += __shfl_sync(0xffffffffu, incl, 31);
+    }
+    if (lane == 0) s_first[E] = carry;
+  }
+  __syncthreads();
+  const int stride = gridDim.x * kSortedThreads;
+  for (int p = block_id * kSortedThreads + tid; p < numel; p += stride) {
+    const int slot = slot_of[p];
+    if (slot < 0 || slot >= numel) continue;
+    if (p >= s_first[E]) {  // a histogram that does not cover every position: the rest belongs to no expert
+      ids[slot] = -1;
+      weights[slot] = 0.f;
+      continue;
+    }
+    int lo = 0, hi = E - 1;  // last expert that starts at or before p
+    while (lo < hi) {
+      const int mid = (lo + hi + 1) >> 1;
+      if (s_first[mid] <= p) lo = mid;
+      else hi = mid - 1;
+    }
+    const int pos = s_start[lo] + p - s_first[lo];
+    if (pos < sorted_cap && sorted_ids) sorted_ids[pos] = slot;
+    ids[slot] = lo;
+    weights[slot] = gate[p];
+  }
+  if (!sorted_ids) return;  // only experts and weights by slot were asked for
+  for (int e = block_id * (kSortedThreads / 32) + warp; e < E; e += gridDim.x * (kSortedThreads / 32)) {
+    for (int i = s_start[e] + s_total[e] + lane; i < min(s_start[e + 1], sorted_cap); i += 32) sorted_ids[i] = numel;
+    for (int b = s_start[e] / block + lane; b < s_start[e + 1] / block && b < expert_cap; b += 32) expert_ids[b] = e;
+  }
+  for (int i = s_start[E] + block_id * kSortedThreads + tid; i < sorted_cap; i += stride) sorted_ids[i] = numel;
+  for (int b = s_start[E] / block + block_id * kSortedThreads + tid; b < expert_cap; b += stride) expert_ids[b] = -1;
+  for (int i = block_id * kSortedThreads + tid; i < num_zero; i += stride) zero_words[i] = 0;
 }
 
 }  // namespace
@@ -235,7 +365,7 @@ int check_align(const AlignArgs& a) {
   FMOE_REQUIRE(a.expert_cap >= ceil_div<int64_t>(a.sorted_cap, a.block),
                "moe_align_block_size: expert_ids too small (%lld < %lld)", (long long)a.expert_cap,
                (long long)ceil_div<int64_t>(a.sorted_cap, a.block));
-  FMOE_REQUIRE(a.sorted_ids && a.expert_ids && a.num_post_pad && (a.topk_ids || a.numel == 0),
+  FMOE_REQUIRE(a.sorted_ids && a.expert_ids && a.num_post_pad && (a.topk_ids || a.numel == 0 || a.from_sorted),
                "moe_align_block_size: null pointer");
   return FMOE_OK;
 }
@@ -244,7 +374,7 @@ int check_align(const AlignArgs& a) {
 int run_align(const AlignArgs& a, cudaStream_t st) {
   int rc = check_align(a);
   if (rc) return rc;
-  if (a.numel < 2 * kChunk || !a.workspace) {  // small inputs, or no scratch: the single-CTA kernel
+  if (a.numel < kSingleCtaSlots || !a.workspace) {  // small inputs, or no scratch: the single-CTA kernel
     const size_t smem = ((size_t)kWarps * a.E + 2 * (size_t)a.E + 1) * sizeof(int);
     if (smem > 48 * 1024)
       FMOE_CUDA_OK(cudaFuncSetAttribute(moe_align_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
@@ -255,24 +385,41 @@ int run_align(const AlignArgs& a, cudaStream_t st) {
   FMOE_REQUIRE(a.workspace_bytes >= fmoe_moe_align_workspace_bytes(a.numel, a.E), "moe_align_block_size: workspace too small");
   const int chunks = (int)ceil_div<int64_t>(a.numel, kChunk);
   int32_t* cnt = static_cast<int32_t*>(a.workspace);
-  align_count_kernel<<<chunks, kThreads, a.E * sizeof(int), st>>>(a.topk_ids, (int)a.numel, a.E, a.sorted_ids, (int)a.sorted_cap, cnt);
+  int32_t* starts = cnt + (int64_t)chunks * a.E;
+  launch_pdl(align_count_kernel, dim3(chunks), dim3(kThreads), a.E * sizeof(int), st, a.topk_ids, (int)a.numel, a.E, a.sorted_ids,
+             (int)a.sorted_cap, cnt);
   rc = launch_status("align_count_kernel");
   if (rc) return rc;
-  align_scan_kernel<<<1, kThreads, (2 * a.E + 1) * sizeof(int), st>>>(chunks, a.E, a.block, cnt, a.expert_ids, (int)a.expert_cap,
-                                                                     a.num_post_pad, a.table, a.token_tile, a.zero_words, a.num_zero);
+  launch_pdl(align_scan_kernel, dim3(1), dim3(kThreads), (2 * a.E + 1) * sizeof(int), st, chunks, a.E, a.block, cnt, starts,
+             a.expert_ids, (int)a.expert_cap, a.num_post_pad, a.table, a.token_tile, a.zero_words, a.num_zero);
   rc = launch_status("align_scan_kernel");
   if (rc) return rc;
   const size_t smem = (size_t)kWarps * a.E * sizeof(int);
   if (smem > 48 * 1024)
     FMOE_CUDA_OK(cudaFuncSetAttribute(align_scatter_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-  align_scatter_kernel<<<chunks, kThreads, smem, st>>>(a.topk_ids, (int)a.numel, a.E, cnt, a.sorted_ids, (int)a.sorted_cap);
+  launch_pdl(align_scatter_kernel, dim3(chunks), dim3(kThreads), smem, st, a.topk_ids, (int)a.numel, a.E,
+             (const int32_t*)cnt, (const int32_t*)starts, a.sorted_ids, (int)a.sorted_cap);
   return launch_status("align_scatter_kernel");
+}
+
+int run_align_sorted(const AlignArgs& a, const SortedSlots& s, cudaStream_t st) {
+  FMOE_REQUIRE(a.E >= 1 && a.E <= 1024 && a.numel >= 1 && a.numel < (1ll << 30), "routing triple: bad E or slot count");
+  FMOE_REQUIRE(s.slot_of && s.hist && s.gate && s.ids && s.weights, "routing triple: null pointer");
+  if (a.sorted_ids) {
+    const int rc = check_align(a);
+    if (rc) return rc;
+  }
+  const unsigned grid = (unsigned)std::min<int64_t>(ceil_div<int64_t>(std::max(a.numel, a.sorted_ids ? a.sorted_cap / 4 : 0), kSortedThreads), 148);
+  launch_pdl(align_sorted_kernel, dim3(grid), dim3(kSortedThreads), (3 * (size_t)a.E + 2) * sizeof(int), st, s.slot_of, s.hist, s.gate,
+             (int)a.numel, a.E, a.block, a.sorted_ids, (int)a.sorted_cap, a.expert_ids, (int)a.expert_cap, a.num_post_pad, a.table,
+             a.token_tile, a.zero_words, a.num_zero, s.ids, s.weights);
+  return launch_status("align_sorted_kernel");
 }
 
 }  // namespace fmoe
 
 extern "C" int64_t fmoe_moe_align_workspace_bytes(int64_t numel, int E) {
-  return fmoe::ceil_div<int64_t>(numel > 0 ? numel : 1, fmoe::kChunk) * E * (int64_t)sizeof(int32_t);
+  return (fmoe::ceil_div<int64_t>(numel > 0 ? numel : 1, fmoe::kChunk) + 1) * E * (int64_t)sizeof(int32_t);
 }
 
 extern "C" int fmoe_moe_align_block_size_ws(const int32_t* topk_ids, int64_t numel, int E, int block,

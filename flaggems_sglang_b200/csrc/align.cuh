@@ -19,7 +19,19 @@ struct AlignArgs {
   int token_tile = 256;           //   at most this many tokens
   int32_t* zero_words = nullptr;  // optional: counters of later kernels, set to zero
   int num_zero = 0;
+  bool from_sorted = false;       // topk_ids is not read (run_align_sorted)
 };
 int run_align(const AlignArgs& a, cudaStream_t st);
+
+// Slots that are already in expert order, and where their experts and weights go by slot.
+struct SortedSlots {
+  const int32_t* slot_of = nullptr;  // [numel] sorted position -> slot
+  const int32_t* hist = nullptr;     // [E] rows per expert
+  const float* gate = nullptr;       // [numel] weights in sorted order
+  int32_t* ids = nullptr;            // [numel]
+  float* weights = nullptr;          // [numel]
+};
+// The outputs of run_align from sorted slots; with sorted_ids == NULL only ids and weights.
+int run_align_sorted(const AlignArgs& a, const SortedSlots& s, cudaStream_t st);
 
 }  // namespace fmoe

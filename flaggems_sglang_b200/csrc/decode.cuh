@@ -11,6 +11,10 @@ struct RouteArgs {
   const float* logits = nullptr;  // [T, E]
   const float* bias = nullptr;    // grouped: [E] or NULL
   int grouped = 0, renorm = 1, n_group = 1, topk_group = 1;
+  // or slots in expert order (sorted position -> slot, rows per expert, weights in sorted order)
+  const int32_t* slot_of = nullptr;
+  const int32_t* hist = nullptr;
+  const float* gate = nullptr;
 };
 
 struct DecodePlan {

@@ -125,10 +125,15 @@ int plan_fused(const fmoe_fused_args& a, const RouteArgs& route, FusedPlan* pl) 
   p.off_route_ids = p.off_route_weights = -1;
   p.use_decode = plan_decode(a, route, &p.decode);
   if (p.use_decode) {
-    p.total = p.decode.total;
+    off = p.decode.total;
+    if (route.slot_of) {
+      p.off_route_ids = take(p.numel * 4);
+      p.off_route_weights = take(p.numel * 4);
+    }
+    p.total = off;
     return FMOE_OK;
   }
-  if (route.logits) {
+  if (route.logits || route.slot_of) {
     p.off_route_ids = take(p.numel * 4);
     p.off_route_weights = take(p.numel * 4);
   }
@@ -218,8 +223,26 @@ int run_fused(const fmoe_fused_args& args, const RouteArgs& route, const FusedPl
   };
   if (a.T == 0) return FMOE_OK;
   auto st = (cudaStream_t)stream;
+  SortedSlots slots;
+  if (route.slot_of) {
+    slots.slot_of = route.slot_of;
+    slots.hist = route.hist;
+    slots.gate = route.gate;
+    slots.ids = reinterpret_cast<int32_t*>(ws + p.off_route_ids);
+    slots.weights = reinterpret_cast<float*>(ws + p.off_route_weights);
+    a.topk_ids = slots.ids;
+    a.topk_weights = slots.weights;
+  }
   if (p.use_decode) {
     mark(0);
+    if (route.slot_of) {
+      AlignArgs al;
+      al.numel = p.numel;
+      al.E = a.num_experts;
+      al.block = 1;
+      const int rc = run_align_sorted(al, slots, st);
+      if (rc) return rc;
+    }
     const int rc = run_decode(a, route, p.decode, ws, st);
     for (int i = 1; i <= 6; ++i) mark(i);
     return rc;
@@ -271,7 +294,8 @@ int run_fused(const fmoe_fused_args& args, const RouteArgs& route, const FusedPl
   al.token_tile = fold ? pick_fold_token_tile(p.numel, a.num_experts) : pick_token_tile(p.numel, a.num_experts);
   al.zero_words = counters;
   al.num_zero = counters ? 2 * kSplitCounters : 0;
-  int rc = run_align(al, st);
+  al.from_sorted = route.slot_of != nullptr;
+  int rc = route.slot_of ? run_align_sorted(al, slots, st) : run_align(al, st);
   if (rc) return rc;
   mark(1);
   if (a.zero_dropped) FMOE_CUDA_OK(cudaMemsetAsync(z, 0, (size_t)(p.numel * a.H * eb), st));
@@ -468,6 +492,30 @@ int check_route(const fmoe_fused_args& a, const fmoe_route_args& r) {
   return FMOE_OK;
 }
 }  // namespace
+
+extern "C" int64_t fmoe_fused_experts_sorted_workspace_bytes(const fmoe_fused_args* args) {
+  if (!args) {
+    fmoe::fail(FMOE_ERR_INVALID_ARG, "fused_experts_sorted: args is null");
+    return -1;
+  }
+  fmoe::RouteArgs r;
+  const int32_t present = 0;  // the plan asks only whether there are sorted slots
+  r.slot_of = &present;
+  fmoe::FusedPlan p;
+  if (fmoe::plan_fused(*args, r, &p)) return -1;
+  return p.total;
+}
+
+extern "C" int fmoe_fused_experts_sorted(const fmoe_fused_args* args, const int32_t* topk_indx, const int32_t* expt_hist,
+                                         const float* gate_scal, void* stream) {
+  if (!args) return fmoe::fail(FMOE_ERR_INVALID_ARG, "fused_experts_sorted: args is null");
+  if (!topk_indx || !expt_hist || !gate_scal) return fmoe::fail(FMOE_ERR_INVALID_ARG, "fused_experts_sorted: null pointer");
+  fmoe::RouteArgs r;
+  r.slot_of = topk_indx;
+  r.hist = expt_hist;
+  r.gate = gate_scal;
+  return fmoe::run_with_workspace(*args, r, stream);
+}
 
 extern "C" int64_t fmoe_fused_moe_workspace_bytes(const fmoe_fused_args* args, const fmoe_route_args* route) {
   if (!args || !route) {

@@ -4,6 +4,8 @@
 //   fmoe_moe_sum            : out[t] = sum_j z[t,j], optional post-scale
 #include "rows.cuh"
 
+#include <type_traits>
+
 namespace fmoe {
 namespace {
 
@@ -170,23 +172,46 @@ quant_row_kernel(const __nv_bfloat16* __restrict__ x, int64_t rows_out, int64_t 
   }
 }
 
+// A warp per output row, eight 16-byte loads per lane in flight, the next row's map entry fetched ahead: 16384 rows of 4 KB
+// and 65536 of 4 KB went from 2.8 to about 5 TB/s against a CTA per row with one load per thread.
 __global__ void __launch_bounds__(256)
 gather_rows_kernel(const uint4* __restrict__ x, int64_t rows_out, int64_t vec_per_row,
                    const int32_t* __restrict__ row_map, int map_div, int64_t sentinel,
                    const int32_t* __restrict__ num_rows_dev, uint4* __restrict__ out, int zero_padding) {
   pdl_entry();
+  constexpr int kIlp = 8;
+  const int lane = threadIdx.x & 31;
   const int64_t limit = num_rows_dev ? min((int64_t)*num_rows_dev, rows_out) : rows_out;
-  for (int64_t p = blockIdx.x; p < limit; p += gridDim.x) {
-    const int64_t r = mapped_row(row_map, map_div, sentinel, p);
-    if (r < 0 && !zero_padding) continue;
-    for (int64_t c = threadIdx.x; c < vec_per_row; c += blockDim.x)
-      out[p * vec_per_row + c] = (r >= 0) ? __ldg(x + r * vec_per_row + c) : make_uint4(0, 0, 0, 0);
+  const int64_t stride = (int64_t)gridDim.x * 8;
+  int64_t p = (int64_t)blockIdx.x * 8 + (threadIdx.x >> 5);
+  int64_t r = p < limit ? mapped_row(row_map, map_div, sentinel, p) : -1;
+  for (; p < limit; p += stride) {
+    const int64_t next = p + stride < limit ? mapped_row(row_map, map_div, sentinel, p + stride) : -1;
+    if (r >= 0 || zero_padding) {
+      const uint4* src = x + r * vec_per_row;
+      uint4* dst = out + p * vec_per_row;
+      for (int64_t c0 = lane; c0 < vec_per_row; c0 += 32 * kIlp) {
+        uint4 v[kIlp];
+#pragma unroll
+        for (int i = 0; i < kIlp; ++i) {
+          const int64_t c = c0 + 32 * i;
+          v[i] = (r >= 0 && c < vec_per_row) ? __ldg(src + c) : make_uint4(0, 0, 0, 0);
+        }
+#pragma unroll
+        for (int i = 0; i < kIlp; ++i) {
+          const int64_t c = c0 + 32 * i;
+          if (c < vec_per_row) dst[c] = v[i];
+        }
+      }
+    }
+    r = next;
   }
 }
 
-// each thread owns 8 bf16 (or 4 f32) columns of one token and adds the k slots in order
-template <typename T>
-__global__ void __launch_bounds__(256)
+// each thread owns 8 bf16 (or 4 f32) columns of one token and adds the k slots in order; kIlp slots' loads are issued
+// before the first is added
+template <typename T, int kIlp>
+__global__ void __launch_bounds__(256, kIlp <= 2 ? 8 : 4)
 moe_sum_kernel(const T* __restrict__ z, int64_t Tn, int k, int64_t H, float scale, const T* __restrict__ addend,
                T* __restrict__ out) {
   pdl_entry();
@@ -195,14 +220,23 @@ moe_sum_kernel(const T* __restrict__ z, int64_t Tn, int k, int64_t H, float scal
   const int64_t total = Tn * vec_per_row;
   for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < total; i += (int64_t)gridDim.x * blockDim.x) {
     const int64_t t = i / vec_per_row, c = i % vec_per_row;
+    const uint4* src = reinterpret_cast<const uint4*>(z + t * k * H) + c;
     float acc[V];
 #pragma unroll
     for (int v = 0; v < V; ++v) acc[v] = 0.f;
-    for (int j = 0; j < k; ++j) {
-      uint4 raw = __ldg(reinterpret_cast<const uint4*>(z + ((t * k + j) * H)) + c);
-      const T* e = reinterpret_cast<const T*>(&raw);
+    for (int j0 = 0; j0 < k; j0 += kIlp) {
+      uint4 raw[kIlp];
 #pragma unroll
-      for (int v = 0; v < V; ++v) acc[v] += to_f32(e[v]);
+      for (int j = 0; j < kIlp; ++j)
+        if (j0 + j < k) raw[j] = __ldg(src + (int64_t)(j0 + j) * vec_per_row);
+#pragma unroll
+      for (int j = 0; j < kIlp; ++j) {
+        if (j0 + j < k) {
+          const T* e = reinterpret_cast<const T*>(&raw[j]);
+#pragma unroll
+          for (int v = 0; v < V; ++v) acc[v] += to_f32(e[v]);
+        }
+      }
     }
     uint4 res;
     T* o = reinterpret_cast<T*>(&res);
@@ -287,7 +321,7 @@ int fmoe::run_gather_rows(const void* x, int elem_bytes, int64_t rows_out, int64
   FMOE_REQUIRE(row_map && map_div >= 1, "gather_rows: row_map required");
   if (rows_out <= 0) return FMOE_OK;
   FMOE_REQUIRE(x && out && aligned16(x) && aligned16(out), "gather_rows: null or misaligned pointer");
-  unsigned grid = (unsigned)std::min<int64_t>(rows_out, 148 * 8);
+  unsigned grid = (unsigned)std::min<int64_t>(ceil_div<int64_t>(rows_out, 8), 148 * 8);
   launch_pdl(gather_rows_kernel, dim3(grid), dim3(256), 0, st, (const uint4*)x, rows_out, K * elem_bytes / 16, row_map,
              map_div, map_sentinel, num_rows_dev, (uint4*)out, (int)zero_padding);
   return launch_status("gather_rows_kernel");
@@ -316,11 +350,11 @@ extern "C" int fmoe_moe_sum_add(const void* z, int dtype, int64_t T, int k, int6
   int64_t total = T * (H * eb / 16);
   unsigned grid = (unsigned)std::min<int64_t>(ceil_div<int64_t>(total, 256), 148 * 16);
   auto st = (cudaStream_t)stream;
-  if (dtype == FMOE_BF16)
-    launch_pdl(moe_sum_kernel<__nv_bfloat16>, dim3(grid), dim3(256), 0, st, (const __nv_bfloat16*)z, T, k, H, scale,
-               (const __nv_bfloat16*)addend, (__nv_bfloat16*)out);
-  else
-    launch_pdl(moe_sum_kernel<float>, dim3(grid), dim3(256), 0, st, (const float*)z, T, k, H, scale,
-               (const float*)addend, (float*)out);
+  auto go = [&](auto kernel, auto* zt) {
+    using E = std::remove_pointer_t<decltype(zt)>;
+    launch_pdl(kernel, dim3(grid), dim3(256), 0, st, (const E*)z, T, k, H, scale, (const E*)addend, (E*)out);
+  };
+  if (dtype == FMOE_BF16) k <= 2 ? go(moe_sum_kernel<__nv_bfloat16, 2>, (__nv_bfloat16*)nullptr) : go(moe_sum_kernel<__nv_bfloat16, 4>, (__nv_bfloat16*)nullptr);
+  else k <= 2 ? go(moe_sum_kernel<float, 2>, (float*)nullptr) : go(moe_sum_kernel<float, 4>, (float*)nullptr);
   return launch_status("moe_sum_kernel");
 }

@@ -189,8 +189,10 @@ def fused_experts(
 def _experts(hidden_states, w1, w2, topk_weights, topk_ids, route, k, inplace=False, activation="silu",
              apply_router_weight_on_input=False, use_fp8_w8a8=False, per_channel_quant=False, w1_scale=None, w2_scale=None,
              a1_scale=None, a2_scale=None, block_shape=None, no_combine=False, routed_scaling_factor=None, expert_map=None,
-             variant=None, out_rows=None, b1=None, b2=None, gemm1_alpha=None, gemm1_clamp_limit=None, weights_n_major=False):
-    """`fused_experts`, or with `route` (a filled _C.RouteArgs: logits of [T,E]) the router and the experts in one call."""
+             variant=None, out_rows=None, b1=None, b2=None, gemm1_alpha=None, gemm1_clamp_limit=None, weights_n_major=False,
+             triple=None):
+    """`fused_experts`; with `route` (a filled _C.RouteArgs: logits of [T,E]) the router and the experts in one call, with
+    `triple` (positions -> slots, rows per expert, weights of the sorted positions) a routing that is already in expert order."""
     logger.debug("FLAGGEMS_SGLANG_B200 FUSED_EXPERTS")
     assert inplace is False, "Inplace is not supported"
     assert a1_scale is None, _UNSUPPORTED_FEATURE_MSG.format(name="a1_scale")
@@ -212,7 +214,8 @@ def _experts(hidden_states, w1, w2, topk_weights, topk_ids, route, k, inplace=Fa
     I = twoI // 2
     assert Hw == H, "hidden size mismatch"
     assert w2.shape[0] == E and w2.shape[1] == H and w2.shape[2] == I, "intermediate size mismatch"
-    assert route is not None or (topk_ids.shape == topk_weights.shape and topk_ids.shape[0] == T), "topk shape mismatch"
+    routed_here = route is not None or triple is not None
+    assert routed_here or (topk_ids.shape == topk_weights.shape and topk_ids.shape[0] == T), "topk shape mismatch"
     numel = T * k
 
     if per_channel_quant:
@@ -246,7 +249,7 @@ def _experts(hidden_states, w1, w2, topk_weights, topk_ids, route, k, inplace=Fa
     if not weights_n_major:
         w1 = w1.contiguous()
         w2 = w2.contiguous()
-    if route is None:
+    if not routed_here:
         wts = topk_weights.float().contiguous()
         ids = topk_ids
         if expert_map is not None:
@@ -286,15 +289,22 @@ def _experts(hidden_states, w1, w2, topk_weights, topk_ids, route, k, inplace=Fa
             zero_dropped=int(expert_map is not None), activation=_C.ACTIVATIONS[activation], T=T, H=H, I=I,
             routed_scaling_factor=1.0 if routed_scaling_factor is None else float(routed_scaling_factor),
             hidden=x.data_ptr(), w1=w1.data_ptr(), w2=w2.data_ptr(), w1_scale=_C.ptr(w1_scale),
-            w2_scale=_C.ptr(w2_scale), topk_weights=None if route is not None else wts.data_ptr(),
-            topk_ids=None if route is not None else ids.data_ptr(), out=_C.ptr(out),
+            w2_scale=_C.ptr(w2_scale), topk_weights=None if routed_here else wts.data_ptr(),
+            topk_ids=None if routed_here else ids.data_ptr(), out=_C.ptr(out),
             out_rows=_C.ptr(out_rows), b1=_C.ptr(b1), b2=_C.ptr(b2), act_alpha=act_alpha, act_limit=act_limit)
-        need = lib.fmoe_fused_experts_workspace_bytes(fa) if route is None else lib.fmoe_fused_moe_workspace_bytes(fa, route)
+        if triple is not None:
+            need = lib.fmoe_fused_experts_sorted_workspace_bytes(fa)
+        else:
+            need = lib.fmoe_fused_experts_workspace_bytes(fa) if route is None else lib.fmoe_fused_moe_workspace_bytes(fa, route)
         if need < 0:
             _C.check(_C.ERR_INVALID_ARG)
         ws = torch.empty(max(int(need), 256), dtype=torch.uint8, device=dev)
         fa.workspace, fa.workspace_bytes = ws.data_ptr(), ws.numel()
-        _C.check(lib.fmoe_fused_experts(fa, st) if route is None else lib.fmoe_fused_moe(fa, route, st))
+        if triple is not None:
+            slot_of, hist, gate = triple
+            _C.check(lib.fmoe_fused_experts_sorted(fa, slot_of.data_ptr(), hist.data_ptr(), gate.data_ptr(), st))
+        else:
+            _C.check(lib.fmoe_fused_experts(fa, st) if route is None else lib.fmoe_fused_moe(fa, route, st))
         return out
 
     # profiling path (STAGE_EVENTS set): the same kernels launched one by one with events around each launch
@@ -484,6 +494,31 @@ def n_major_supported(w1: torch.Tensor, w2: torch.Tensor, activation: str = "sil
     return H % 32 == 0 and twoI % 64 == 0 and w1.data_ptr() % 16 == 0 and w2.data_ptr() % 16 == 0
 
 
+def _from_triple(hidden_states, w1, w2, routing_data, gather_indx, scatter_indx, activation, **kw):
+    """The experts for a routing triple; `scatter_indx=None` returns the rows in expert-sorted order."""
+    T, H = hidden_states.shape
+    k = routing_data.n_expts_act
+    E = w1.shape[0]
+    M = T * k
+    slot_of, hist = gather_indx.src_indx, routing_data.expt_hist
+    if STAGE_EVENTS is None:
+        triple = (slot_of.to(torch.int32).contiguous(), hist.to(torch.int32).contiguous(), routing_data.gate_scal.float().contiguous())
+        _C.require_cuda(hidden_states, *triple)
+        assert triple[0].numel() == M and triple[1].numel() == E and triple[2].numel() == M, "routing triple: size mismatch"
+        out = _experts(hidden_states, w1, w2, None, None, None, k, activation=activation, no_combine=scatter_indx is None,
+                       triple=triple, **kw)
+    else:  # per-stage profiling: expert and weight by slot, for the kernels launched one by one
+        dev = hidden_states.device
+        pos = slot_of.long()
+        ids = torch.empty(M, dtype=torch.int32, device=dev)
+        ids[pos] = torch.repeat_interleave(torch.arange(E, device=dev), hist.long(), output_size=M).to(torch.int32)
+        w = torch.empty(M, dtype=torch.float32, device=dev)
+        w[pos] = routing_data.gate_scal.float()
+        out = fused_experts(hidden_states, w1, w2, w.view(T, k), ids.view(T, k), activation=activation,
+                            no_combine=scatter_indx is None, **kw)
+    return out.view(M, H)[slot_of.long()] if scatter_indx is None else out.view(T, H)
+
+
 def _k_major(w: torch.Tensor) -> torch.Tensor:
     """[E, K, N] (reference layout) -> [E, N, K] contiguous.  Free when the caller passes
     the transposed view of a serving-side weight, a copy otherwise."""
@@ -537,31 +572,12 @@ def triton_kernel_fused_experts(
     if activation not in _C.ACTIVATIONS:
         raise ValueError(f"Unsupported FusedMoe activation: {activation}")
 
-    T, H = hidden_states.shape
-    k = routing_data.n_expts_act
-    E = w1.shape[0]
-    M = T * k
-    dev = hidden_states.device
-    topk_indx = gather_indx.src_indx.long()          # sorted position -> flat slot
-    hist = routing_data.expt_hist.long()
-    expert_of_pos = torch.repeat_interleave(torch.arange(E, device=dev), hist, output_size=M)
-    ids_flat = torch.empty(M, dtype=torch.int32, device=dev)
-    ids_flat[topk_indx] = expert_of_pos.to(torch.int32)
-    w_flat = torch.empty(M, dtype=torch.float32, device=dev)
-    w_flat[topk_indx] = routing_data.gate_scal.float()
     # contiguous reference-layout weights (what the reference's own tests and benchmarks pass) are read in place;
     # transposed views of serving-side weights are used as they are; anything else costs a transposed copy
     in_place = n_major_supported(w1, w2, activation) and os.environ.get("FMOE_N_MAJOR", "1") != "0"
-    z_or_out = fused_experts(
-        hidden_states, w1 if in_place else _k_major(w1), w2 if in_place else _k_major(w2), w_flat.view(T, k),
-        ids_flat.view(T, k), weights_n_major=in_place,
-        activation=activation, apply_router_weight_on_input=apply_router_weight_on_input,
-        no_combine=scatter_indx is None,
-    )
-    if scatter_indx is None:
-        # reference returns rows in sorted order p; ours are by flat slot
-        return z_or_out.view(M, H)[topk_indx]
-    return z_or_out.view(T, H)
+    return _from_triple(hidden_states, w1 if in_place else _k_major(w1), w2 if in_place else _k_major(w2), routing_data,
+                        gather_indx, scatter_indx, activation, weights_n_major=in_place,
+                        apply_router_weight_on_input=apply_router_weight_on_input)
 
 
 def _split_interleaved(w13_rows: torch.Tensor, b13: Optional[torch.Tensor]):
@@ -613,27 +629,10 @@ def triton_kernel_fused_experts_with_bias(
         raise ValueError(f"Unsupported FusedMoe activation: {activation}")
     assert w1.dtype == torch.bfloat16 and w2.dtype == torch.bfloat16, "w1/w2 must be bfloat16"
     assert hidden_states.shape[-1] == w1.shape[-2], "hidden size mismatch"
-    T, H = hidden_states.shape
-    k = routing_data.n_expts_act
-    E = w1.shape[0]
-    M = T * k
-    dev = hidden_states.device
-    topk_indx = gather_indx.src_indx.long()          # sorted position -> flat slot
-    hist = routing_data.expt_hist.long()
-    expert_of_pos = torch.repeat_interleave(torch.arange(E, device=dev), hist, output_size=M)
-    ids_flat = torch.empty(M, dtype=torch.int32, device=dev)
-    ids_flat[topk_indx] = expert_of_pos.to(torch.int32)
-    w_flat = torch.empty(M, dtype=torch.float32, device=dev)
-    w_flat[topk_indx] = routing_data.gate_scal.float()
     w1_split, b1_split = _split_interleaved(w1.transpose(1, 2), b1)
-    z_or_out = fused_experts(
-        hidden_states, w1_split, _k_major(w2), w_flat.view(T, k), ids_flat.view(T, k), activation="swiglu_oai",
-        apply_router_weight_on_input=apply_router_weight_on_input, no_combine=scatter_indx is None,
-        b1=b1_split, b2=b2, gemm1_alpha=gemm1_alpha, gemm1_clamp_limit=gemm1_clamp_limit,
-    )
-    if scatter_indx is None:
-        return z_or_out.view(M, H)[topk_indx]
-    return z_or_out.view(T, H)
+    return _from_triple(hidden_states, w1_split, _k_major(w2), routing_data, gather_indx, scatter_indx, "swiglu_oai",
+                        apply_router_weight_on_input=apply_router_weight_on_input, b1=b1_split, b2=b2,
+                        gemm1_alpha=gemm1_alpha, gemm1_clamp_limit=gemm1_clamp_limit)
 
 
 @dataclass

@@ -105,7 +105,7 @@ int fmoe_moe_align_block_size(const int32_t* topk_ids, int64_t numel, int E, int
                               int32_t* num_tokens_post_padded, void* stream);
 
 /*
- * Same result with caller scratch: inputs of 8192 slots or more are processed by one CTA per 4096 slots
+ * Same result with caller scratch: inputs of 16384 slots or more are processed by one CTA per 4096 slots
  * (three launches) instead of a single CTA.  workspace needs fmoe_moe_align_workspace_bytes(numel, E) bytes;
  * with workspace == NULL or a small input this is fmoe_moe_align_block_size.
  */
@@ -303,6 +303,15 @@ typedef struct fmoe_route_args {
 } fmoe_route_args;
 int64_t fmoe_fused_moe_workspace_bytes(const fmoe_fused_args* args, const fmoe_route_args* route);
 int fmoe_fused_moe(const fmoe_fused_args* args, const fmoe_route_args* route, void* stream);
+
+/*
+ * fmoe_fused_experts for a routing that is already in expert order, as the reference operator takes it
+ * (src/flaggems_sglang/ops/fused_moe.py:119-146): topk_indx [T*k] sorted position -> flat slot, expt_hist [E] rows per
+ * expert, gate_scal [T*k] weights in sorted order; args->topk_weights / topk_ids are ignored.
+ */
+int64_t fmoe_fused_experts_sorted_workspace_bytes(const fmoe_fused_args* args);
+int fmoe_fused_experts_sorted(const fmoe_fused_args* args, const int32_t* topk_indx, const int32_t* expt_hist,
+                              const float* gate_scal, void* stream);
 
 /*
  * fmoe_fused_experts for callers that cannot allocate device memory.  It has no counterpart in the

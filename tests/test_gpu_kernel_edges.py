@@ -1,0 +1,154 @@
+"""GPU: the kernels at the sizes where a tile, a chunk or a dispatch rule ends, against the CPU oracle."""
+import numpy as np
+import pytest
+import torch
+
+from oracle import experts as OE
+from oracle import quant as OQ
+from oracle import routing as OR
+from tests.util import assert_close_moe
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.fixture(scope="module")
+def fg():
+    import flaggems_sglang_b200 as fg
+
+    return fg
+
+
+@pytest.fixture(autouse=True)
+def _device_status():
+    yield
+    from flaggems_sglang_b200 import _C
+
+    _C.check_device_status()
+
+
+def _layer(T, H, I, E, seed):
+    g = torch.Generator().manual_seed(seed)
+    x = torch.randn(T, H, generator=g).to(torch.bfloat16)
+    w1 = (torch.randn(E, 2 * I, H, generator=g) * H ** -0.5).to(torch.bfloat16)
+    w2 = (torch.randn(E, H, I, generator=g) * I ** -0.5).to(torch.bfloat16)
+    return x, w1, w2, g
+
+
+# rows per expert around the edges of 8-row groups and of the 64-, 128- and 256-token tiles; the mean picks the tile
+ROWS = {"64": [1, 0, 7, 8, 9, 15, 16, 17, 31, 33, 63, 64, 65, 80], "128": [1, 63, 64, 65, 127, 128, 129, 0],
+        "256": [1, 127, 129, 255, 256, 257, 400, 513]}
+
+
+@pytest.mark.parametrize("tile", ROWS)
+@pytest.mark.parametrize("kind", ["bf16", "n_major", "bias", "channel", "block"])
+def test_rows_per_expert_at_tile_edges(fg, tile, kind):
+    """CTA-pair GEMMs: every expert's last token tile is cut by its row count.  I and H leave a part-filled weight tile."""
+    rows = ROWS[tile]
+    E, T = len(rows), sum(rows)
+    H, I = (384, 384) if kind == "block" else (320, 352)
+    x, w1, w2, g = _layer(T, H, I, E, 7)
+    ids = torch.repeat_interleave(torch.arange(E), torch.tensor(rows))[torch.randperm(T, generator=g)].to(torch.int32).view(T, 1)
+    tw = torch.rand(T, 1, generator=g) + 0.5
+    xd, twd, idd = x.cuda(), tw.cuda(), ids.cuda()
+    if kind in ("bf16", "bias"):
+        kw, okw = dict(variant="tcgen05"), {}
+        ref = OE.fused_experts(x, w1, w2, tw, ids)
+        if kind == "bias":
+            b1, b2 = torch.randn(E, 2 * I, generator=g), torch.randn(E, H, generator=g)
+            kw.update(b1=b1.cuda(), b2=b2.cuda(), activation="swiglu_oai", gemm1_clamp_limit=7.0)
+            ref = OE.fused_experts_with_bias(x, w1, b1, w2, b2, tw, ids, limit=7.0)
+        out = fg.fused_experts(xd, w1.cuda(), w2.cuda(), twd, idd, **kw)
+    elif kind == "n_major":
+        out = fg.fused_experts(xd, w1.transpose(1, 2).contiguous().cuda(), w2.transpose(1, 2).contiguous().cuda(), twd, idd,
+                               weights_n_major=True)
+        ref = OE.fused_experts(x, w1, w2, tw, ids)
+    else:
+        q = OQ.quant_weight_per_channel if kind == "channel" else OQ.quant_weight_block128
+        (w1q, w1s), (w2q, w2s) = q(w1), q(w2)
+        kw = dict(per_channel_quant=True) if kind == "channel" else dict(block_shape=[128, 128], variant="tcgen05")
+        out = fg.fused_experts(xd, w1q.cuda(), w2q.cuda(), twd, idd, use_fp8_w8a8=True, w1_scale=w1s.cuda(),
+                               w2_scale=w2s.cuda(), **kw)
+        ref = (OE.fused_experts_fp8_per_channel if kind == "channel" else OE.fused_experts_fp8)(x, w1q, w1s, w2q, w2s, tw, ids)
+    assert_close_moe(out, ref, "fp8" if kind in ("channel", "block") else "bf16", f"{kind} tile {tile}")
+
+
+@pytest.mark.parametrize("T", [1, 2, 3, 5, 8, 9])
+@pytest.mark.parametrize("kind", ["bf16", "bias", "block"])
+def test_decode_layer(fg, T, kind):
+    """Up to 8 tokens run in the two decode kernels (T = 9 is the first call that does not): shared experts, ids outside
+    the range, and the router inside the call."""
+    E, H, I, k = 16, 640, 384, 4
+    x, w1, w2, g = _layer(T, H, I, E, 20 + T)
+    logits = torch.randn(T, E, generator=g)
+    tw, ids = OR.softmax_topk(logits, k, True)
+    kw, wts = {}, (w1, w2)
+    if kind == "block":
+        (w1q, w1s), (w2q, w2s) = OQ.quant_weight_block128(w1), OQ.quant_weight_block128(w2)
+        wts, kw = (w1q, w2q), dict(use_fp8_w8a8=True, w1_scale=w1s.cuda(), w2_scale=w2s.cuda(), block_shape=[128, 128])
+        oracle = lambda w, i, **o: OE.fused_experts_fp8(x, w1q, w1s, w2q, w2s, w, i, **o)  # noqa: E731
+    elif kind == "bias":
+        b1, b2 = torch.randn(E, 2 * I, generator=g), torch.randn(E, H, generator=g)
+        kw = dict(b1=b1.cuda(), b2=b2.cuda(), activation="swiglu_oai", gemm1_clamp_limit=7.0)
+        oracle = lambda w, i, **o: OE.fused_experts_with_bias(x, w1, b1, w2, b2, w, i, limit=7.0, **o)  # noqa: E731
+    else:
+        oracle = lambda w, i, **o: OE.fused_experts(x, w1, w2, w, i, **o)  # noqa: E731
+    d = [x.cuda(), wts[0].cuda(), wts[1].cuda()]
+    tol = "fp8" if kind == "block" else "bf16"
+    out = fg.fused_experts(*d, tw.cuda(), ids.cuda(), routed_scaling_factor=1.5, **kw)
+    assert_close_moe(out, oracle(tw, ids).float() * 1.5, tol, f"{kind} T={T}")
+    routed = fg.fused_moe(*d, logits.cuda(), k, True, routed_scaling_factor=1.5, **kw)
+    assert_close_moe(routed, oracle(tw, ids).float() * 1.5, tol, f"{kind} T={T} with the router")
+    z = fg.fused_experts(*d, tw.cuda(), ids.cuda(), no_combine=True, **kw)
+    assert_close_moe(z.float().sum(1), oracle(tw, ids), tol, f"{kind} T={T} rows")
+    if T > 8:
+        return
+    bad = ids.clone()
+    bad[:, 1] = -1
+    bad[0, 2] = E + 3
+    if T > 1:
+        bad[1] = bad[0]
+    assert_close_moe(fg.fused_experts(*d, tw.cuda(), bad.cuda(), **kw), oracle(tw, bad), tol, f"{kind} T={T} dropped ids")
+
+
+@pytest.mark.parametrize("E", [1, 8, 255, 257])
+@pytest.mark.parametrize("numel", [1, 127, 128, 129, 4097, 16383, 16384, 16385])
+def test_align_at_chunk_edges(fg, numel, E):
+    g = torch.Generator().manual_seed(numel + E)
+    ids = torch.randint(-1, E + 1, (numel, 1), generator=g, dtype=torch.int32)
+    s, e, n = fg.moe_align_block_size(ids.cuda(), 64, E)
+    os_, oe, on = OR.moe_align_block_size(ids, 64, E)
+    np.testing.assert_array_equal(n.cpu().numpy(), on)
+    np.testing.assert_array_equal(s.cpu().numpy(), os_)
+    np.testing.assert_array_equal(e.cpu().numpy(), oe)
+
+
+@pytest.mark.parametrize("T", [1, 8, 9, 100, 2049])
+def test_sorted_routing_equals_routing_by_slot(fg, T):
+    """The routing triple goes to the kernels as it is; the results are those of the same routing by slot."""
+    E, H, I, k = 24, 256, 192, 3
+    x, w1, w2, g = _layer(T, H, I, E, 50 + T)
+    logits = torch.randn(T, E, generator=g)
+    tw, ids = OR.softmax_topk(logits, k, True)
+    tw, ids = tw.cuda(), ids.cuda()
+    rd, gi, si = fg.standard_topk_to_routing(tw, ids, E)
+    ids2, perm = torch.sort(ids, dim=1)  # the triple's slots hold a token's experts in ascending order
+    tw2 = torch.gather(tw, 1, perm)
+    d = [x.cuda(), w1.cuda(), w2.cuda()]
+    views = [d[1].transpose(1, 2), d[2].transpose(1, 2)]
+    assert torch.equal(fg.triton_kernel_fused_experts(d[0], *views, rd, gi, si), fg.fused_experts(*d, tw2, ids2))
+    nm = [v.contiguous() for v in views]
+    assert torch.equal(fg.triton_kernel_fused_experts(d[0], *nm, rd, gi, si),
+                       fg.fused_experts(d[0], *nm, tw2, ids2, weights_n_major=True))
+    rows = fg.triton_kernel_fused_experts(d[0], *nm, rd, gi, None)
+    ref = fg.fused_experts(d[0], *nm, tw2, ids2, weights_n_major=True, no_combine=True).view(T * k, H)[gi.src_indx.long()]
+    assert torch.equal(rows, ref)
+
+
+@pytest.mark.parametrize("k", [1, 2, 3, 4, 5, 9])
+def test_combine_slot_counts(fg, k):
+    """moe_sum issues the loads of up to 2 or 4 slots before the first is added."""
+    z = torch.randn(37, k, 264, generator=torch.Generator().manual_seed(k))
+    for dt in (torch.bfloat16, torch.float32):
+        out = torch.empty(37, 264, dtype=dt, device="cuda")
+        fg.moe_sum(z.to(dt).cuda(), out)
+        assert torch.equal(out.cpu(), OE.moe_sum(z.to(dt)).to(dt))
