@@ -170,8 +170,10 @@ int plan_fused(const fmoe_fused_args& a, const RouteArgs& route, FusedPlan* pl) 
       p.off_xt = take(a.T * a.H);
       p.off_xt_scale = take(a.T * (a.H / 128) * 4);
     }
-    p.act_elem = tc ? 2 : 4;  // bf16 from the tcgen05 epilogue, fp32 from the streaming kernel
-    p.off_act = take(p.cap * a.I * p.act_elem);
+    // the wide tensor-core kernel quantises its 128-channel groups itself; the others write fp32 for the quantiser
+    const bool wide = tc && pick_fold_token_tile(p.numel, a.num_experts) == 256;
+    p.act_elem = wide ? 1 : 4;
+    p.off_act = wide ? -1 : take(p.cap * a.I * 4);
     p.off_actq = take(p.cap * a.I);
     p.off_actq_scale = take(p.cap * (a.I / 128) * 4);
   } else {
@@ -271,7 +273,7 @@ int run_fused(const fmoe_fused_args& args, const RouteArgs& route, const FusedPl
   int32_t* sorted = reinterpret_cast<int32_t*>(ws + p.off_sorted);
   int32_t* experts = reinterpret_cast<int32_t*>(ws + p.off_expert);
   int32_t* npp = reinterpret_cast<int32_t*>(ws + p.off_npp);
-  void* act = ws + p.off_act;
+  void* act = p.off_act >= 0 ? ws + p.off_act : nullptr;
   void* z = a.no_combine ? a.out : (void*)(ws + p.off_z);
 
   mark(0);
@@ -373,7 +375,7 @@ int run_fused(const fmoe_fused_args& args, const RouteArgs& route, const FusedPl
       xsc = xtsc;  // the gate/up GEMM looks the scale up by token
       g1.a_scale_gather = 1;
     } else if (channel) {
-      rc = fmoe_quant_fp8_per_token(a.hidden, FMOE_BF16, p.cap, a.H, sorted, a.top_k, p.numel, npp, xq, xsc, stream);
+      rc = run_quant_per_token(a.hidden, FMOE_BF16, p.cap, a.H, sorted, a.top_k, p.numel, npp, xq, xsc, false, st);
     } else if (tc && p.off_xt >= 0) {
       void* xt = ws + p.off_xt;
       float* xtsc = reinterpret_cast<float*>(ws + p.off_xt_scale);
@@ -383,12 +385,16 @@ int run_fused(const fmoe_fused_args& args, const RouteArgs& route, const FusedPl
       xsc = xtsc;  // the gate/up GEMM looks the scales up by token
       g1.a_scale_gather = 1;
     } else if (tc)
-      rc = fmoe_quant_fp8_group128(a.hidden, FMOE_BF16, p.cap, a.H, sorted, a.top_k, p.numel, npp, xq, xsc, stream);
+      rc = run_quant_group128(a.hidden, FMOE_BF16, p.cap, a.H, sorted, a.top_k, p.numel, npp, xq, xsc, false, st);
     else
       rc = fmoe_quant_fp8_group128(a.hidden, FMOE_BF16, a.T, a.H, nullptr, 1, 0, nullptr, xq, xsc, stream);
     if (rc) return rc;
     g1.dtype = g2.dtype = FMOE_E4M3;
-    g1.out_dtype = p.act_elem == 2 ? FMOE_BF16 : FMOE_F32;
+    g1.out_dtype = channel ? FMOE_BF16 : (p.act_elem == 1 ? FMOE_E4M3 : FMOE_F32);
+    if (g1.out_dtype == FMOE_E4M3) {
+      g1.out = ws + p.off_actq;
+      g1.out_scale = reinterpret_cast<float*>(ws + p.off_actq_scale);
+    }
     g1.a = xq;
     g1.a_scale = xsc;
     g1.a_rows = tc ? p.cap : a.T;
@@ -402,14 +408,12 @@ int run_fused(const fmoe_fused_args& args, const RouteArgs& route, const FusedPl
   rc = run_gemm(g1, true, st);
   if (rc) return rc;
   mark(3);
-  if (fp8) {
-    // padding positions of the sorted order (most of the rows at small T) are zero-filled, not quantised
+  if (fp8 && act) {
+    float* scale = reinterpret_cast<float*>(ws + p.off_actq_scale);
     if (a.scale_mode == FMOE_SCALE_CHANNEL)
-      rc = fmoe_quant_fp8_per_token(act, FMOE_BF16, p.cap, a.I, sorted, 0, p.numel, npp, ws + p.off_actq,
-                                    reinterpret_cast<float*>(ws + p.off_actq_scale), stream);
+      rc = run_quant_per_token(act, FMOE_BF16, p.cap, a.I, sorted, 0, p.numel, npp, ws + p.off_actq, scale, false, st);
     else
-      rc = fmoe_quant_fp8_group128(act, g1.out_dtype, p.cap, a.I, sorted, 0, p.numel, npp, ws + p.off_actq,
-                                   reinterpret_cast<float*>(ws + p.off_actq_scale), stream);
+      rc = run_quant_group128(act, FMOE_F32, p.cap, a.I, sorted, 0, p.numel, npp, ws + p.off_actq, scale, !tc, st);
     if (rc) return rc;
   }
   mark(4);

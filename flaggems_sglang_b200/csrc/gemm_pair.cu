@@ -516,7 +516,7 @@ grouped_gemm_pair_kernel(const __grid_constant__ CUtensorMap map_t, const __grid
       if (lane == 0) ptx::mbar_arrive_cluster(ptx::smem_u32(&acc_empty[acc]) & ~ptx::kPeerRankBit);
       if constexpr (GATED) {
         if (p.zero_padding && tl.last && slice == 0)
-          zero_block_rows(tl, p.out, p.n, tl.w_tile * 128 + rank * 64, kEpiWarps * 32);
+          zero_block_rows(tl, p.out, p.n, tl.w_tile * 128 + rank * 64, 2, threadIdx.x, kEpiWarps * 32);
       }
       if (p.profile) prof_busy += clock64() - te1;
     }

@@ -18,6 +18,7 @@
 // What bounds it: HBM (the weights stream through a 9-stage ring of 20 KB); the fold of a 64-token partial costs a warp
 // about 300 cycles from wait to hand-over, with eight partials in flight.
 #include "pair.cuh"
+#include "rows.cuh"
 
 #include <cstdlib>
 #include <type_traits>
@@ -83,6 +84,8 @@ struct FoldParams {
   int32_t activation;
   int32_t group;
   int32_t zero_padding;
+  int32_t out_dtype;  // gate/up: FMOE_F32, FMOE_BF16 or (wide) FMOE_E4M3 with out_scale
+  float* out_scale;   // [rows, n / 128]
 };
 
 __device__ __forceinline__ void report(int code) { atomicCAS(&g_device_status_fp8, 0, code); }
@@ -113,6 +116,15 @@ __device__ __forceinline__ unsigned long long lds64(uint32_t addr) {
   unsigned long long v;
   asm volatile("ld.shared.b64 %0, [%1];" : "=l"(v) : "r"(addr) : "memory");
   return v;
+}
+
+// 16 values times s as bf16
+__device__ __forceinline__ void store16(__nv_bfloat16* dst, const float* v, float s) {
+  uint32_t w[8];
+#pragma unroll
+  for (int j = 0; j < 8; ++j) w[j] = pack_bf16x2(v[2 * j] * s, v[2 * j + 1] * s);
+  reinterpret_cast<uint4*>(dst)[0] = make_uint4(w[0], w[1], w[2], w[3]);
+  reinterpret_cast<uint4*>(dst)[1] = make_uint4(w[4], w[5], w[6], w[7]);
 }
 
 // PROF: instrumented build with wait-time counters (reading the clock is slow enough to distort the fold loop).
@@ -449,16 +461,24 @@ grouped_gemm_pair_fold_kernel(const __grid_constant__ CUtensorMap map_t, const _
         }
         const float rs[4] = {r0.x, r0.y, r1.x, r1.y};
         if constexpr (GATED) {
-          uint32_t v[4];
+          // element j: token tok0 + 8 * (j >> 2) + 2 t + (j & 1), channel ch0 + lane / 4 + 8 * ((j >> 1) & 1)
 #pragma unroll
-          for (int q = 0; q < 4; ++q) {
-            const int j = 4 * (q >> 1) + 2 * (q & 1);
-            v[q] = pack_bf16x2(act_mul_fast(lo[j] * rs[2 * (q >> 1)], hi[j] * rs[2 * (q >> 1)], p.activation),
-                               act_mul_fast(lo[j + 1] * rs[2 * (q >> 1) + 1], hi[j + 1] * rs[2 * (q >> 1) + 1], p.activation));
+          for (int j = 0; j < 8; ++j) lo[j] = act_mul(lo[j] * rs[2 * (j >> 2) + (j & 1)], hi[j] * rs[2 * (j >> 2) + (j & 1)], p.activation);
+          if (p.out_dtype == FMOE_F32) {  // eight lanes store one token's 32 bytes
+            float* out = reinterpret_cast<float*>(p.out) + (int64_t)(tl.row0 + tok0) * p.n + ch0 + (lane >> 2);
+#pragma unroll
+            for (int j = 0; j < 8; ++j) {
+              const int u = 8 * (j >> 2) + 2 * t + (j & 1);
+              if (u < tl.cols - tok0) out[(int64_t)u * p.n + 8 * ((j >> 1) & 1)] = lo[j];
+            }
+          } else {
+            uint32_t v[4];
+#pragma unroll
+            for (int q = 0; q < 4; ++q) v[q] = pack_bf16x2(lo[2 * q], lo[2 * q + 1]);
+            strip_put16(strip, 48, 0, lane, v);
+            strip_store_sorted(strip, lane, reinterpret_cast<__nv_bfloat16*>(p.out) + (int64_t)(tl.row0 + tok0) * p.n, p.n, ch0,
+                               tl.cols - tok0);
           }
-          strip_put16(strip, 48, 0, lane, v);
-          strip_store_sorted(strip, lane, reinterpret_cast<__nv_bfloat16*>(p.out) + (int64_t)(tl.row0 + tok0) * p.n, p.n, ch0,
-                             tl.cols - tok0);
         } else {
 #pragma unroll
           for (int h = 0; h < 2; ++h) {
@@ -475,7 +495,8 @@ grouped_gemm_pair_fold_kernel(const __grid_constant__ CUtensorMap map_t, const _
         }
       }
       if constexpr (GATED) {
-        if (p.zero_padding && tl.last) zero_block_rows(tl, p.out, p.n, tl.w_tile * 128 + rank * 64, kFoldWarps * 32);
+        if (p.zero_padding && tl.last) 
+          zero_block_rows(tl, p.out, p.n, tl.w_tile * 128 + rank * 64, p.out_dtype == FMOE_F32 ? 4 : 2, threadIdx.x, kFoldWarps * 32);
       }
       if (PROF) prof_epi += clock64() - te0;
     }
@@ -521,8 +542,9 @@ struct WideGeo {
   static constexpr int SLOT_BYTES = GROUP * KB_BYTES;
   static constexpr int META_WORDS = 2 * 128 + 4;   // slot ids, row weights, {first row, rows of this CTA, weight tile}
   static constexpr int META_BYTES = META_TILES * META_WORDS * 4;
+  static constexpr int AMAX_BYTES = 2 * 4 * 128 * 4;  // two tiles' [column piece][token] largest magnitudes
   static constexpr int bytes(int num_experts) {
-    return STAGES * STAGE_BYTES + BAR_BYTES + SC_SLOTS * SLOT_BYTES + META_BYTES + pair_table_bytes(num_experts);
+    return STAGES * STAGE_BYTES + BAR_BYTES + SC_SLOTS * SLOT_BYTES + META_BYTES + AMAX_BYTES + pair_table_bytes(num_experts);
   }
 };
 static_assert(WideGeo::bytes(1024) <= kMaxSmem, "shared memory");
@@ -537,14 +559,16 @@ grouped_gemm_pair_fold_wide_kernel(const __grid_constant__ CUtensorMap map_t, co
   uint64_t* bars = reinterpret_cast<uint64_t*>(smem + STAGES * STAGE_BYTES);
   uint64_t* full_bar = bars;                 // [STAGES] used in CTA 0: both CTAs' loads -> MMA
   uint64_t* empty_bar = bars + STAGES;       // [STAGES] per CTA: MMA -> producer
-  uint64_t* part_full = bars + 2 * STAGES;   // [2] per CTA: MMA -> fold
-  uint64_t* part_empty = part_full + 2;      // [2] used in CTA 0: folds of both CTAs -> MMA
-  uint64_t* sc_full = part_empty + 2;        // [slots] scale warps -> fold
+  uint64_t* part_full = bars + 2 * STAGES;   // [4] per CTA: MMA -> fold
+  uint64_t* part_empty = part_full + 4;      // [4] used in CTA 0: folds of both CTAs -> MMA
+  uint64_t* sc_full = part_empty + 4;        // [slots] scale warps -> fold
   uint64_t* sc_empty = sc_full + SC_SLOTS;   // [slots] fold -> scale warps
-  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(sc_empty + SC_SLOTS);
+  uint64_t* amax_bar = sc_empty + SC_SLOTS;  // [4] the four warps that hold a token's 128 channels
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(amax_bar + 4);
   uint8_t* scales = smem + STAGES * STAGE_BYTES + BAR_BYTES;  // [slot][K block][half][token]
   int32_t* meta = reinterpret_cast<int32_t*>(scales + SC_SLOTS * G::SLOT_BYTES);  // [tile]
-  int32_t* table = reinterpret_cast<int32_t*>(scales + SC_SLOTS * G::SLOT_BYTES + G::META_BYTES);
+  float* amax_buf = reinterpret_cast<float*>(scales + SC_SLOTS * G::SLOT_BYTES + G::META_BYTES);
+  int32_t* table = reinterpret_cast<int32_t*>(scales + SC_SLOTS * G::SLOT_BYTES + G::META_BYTES + G::AMAX_BYTES);
 
   const int warp = ptx::uniform_warp_id(), lane = threadIdx.x & 31;
   const int rank = (int)ptx::cluster_ctarank();
@@ -556,9 +580,10 @@ grouped_gemm_pair_fold_wide_kernel(const __grid_constant__ CUtensorMap map_t, co
       ptx::mbar_init(&full_bar[s], 1);
       ptx::mbar_init(&empty_bar[s], 1);
     }
-    for (int b = 0; b < 2; ++b) {
+    for (int b = 0; b < 4; ++b) {
       ptx::mbar_init(&part_full[b], 1);
       ptx::mbar_init(&part_empty[b], 2 * kFoldWarps);
+      ptx::mbar_init(&amax_bar[b], 4);
     }
     for (int s = 0; s < SC_SLOTS; ++s) {
       ptx::mbar_init(&sc_full[s], 1);
@@ -586,6 +611,8 @@ grouped_gemm_pair_fold_wide_kernel(const __grid_constant__ CUtensorMap map_t, co
   PairCursor cursor;
   PairTile tl;
 
+  // 16 * 104 + 4 * 64 registers per lane are the launch's 20 * 96
+  if (warp >= kFoldWarps) asm volatile("setmaxnreg.dec.sync.aligned.u32 64;");
   if (warp == kFoldWarps) {
     // ---------------- TMA producer (both CTAs): its half of the tile's tokens, its 128 weight rows ----------------
     if (ptx::elect_one()) {
@@ -634,7 +661,7 @@ grouped_gemm_pair_fold_wide_kernel(const __grid_constant__ CUtensorMap map_t, co
   } else if (warp == kFoldWarps + 1) {
     // ---------------- MMA issuer (CTA 0): one fresh partial per K block ----------------
     if (rank == 0 && ptx::elect_one()) {
-      constexpr uint32_t idesc = ptx::make_idesc(/*e4m3*/ 0, 256, 256);
+      constexpr uint32_t idesc = ptx::make_idesc(/*e4m3*/ 0, 256, 128);
       int stage = 0;
       uint32_t phase = 0, step = 0;
       bool alive = true;
@@ -643,29 +670,31 @@ grouped_gemm_pair_fold_wide_kernel(const __grid_constant__ CUtensorMap map_t, co
       const uint64_t da0 = ptx::smem_desc_sw128(ring), db0 = ptx::smem_desc_sw128(ring + W_BYTES);
       for (int tile = worker; tile < total_tiles && alive; tile += workers) {
         for (int kb = 0; kb < kblocks; ++kb, ++step) {
-          const int buf = step & 1;
           const long long tm0 = PROF ? clock64() : 0;
           if (!ptx::mbar_wait(&full_bar[stage], phase)) {  // the data is there long before the partial is folded
             report(0x640 | stage);
             alive = false;
             break;
           }
-          const long long tm1 = PROF ? clock64() : 0;
-          if (!ptx::mbar_wait(&part_empty[buf], ((step >> 1) & 1) ^ 1)) {
-            report(0x600 | buf);
-            alive = false;
-            break;
-          }
-          if (PROF) {
-            prof_md += tm1 - tm0;
-            prof_mp += clock64() - tm1;
-          }
-          ptx::tc_fence_after_sync();
+          if (PROF) prof_md += clock64() - tm0;
           const uint64_t da = da0 + (uint64_t)(stage * (STAGE_BYTES >> 4)), db = db0 + (uint64_t)(stage * (STAGE_BYTES >> 4));
 #pragma unroll
-          for (int kk = 0; kk < KBYTES / 32; ++kk)
-            ptx::mma_f8f6f4_ss_pair(tmem_base + buf * 256, da + 2 * kk, db + 2 * kk, idesc, kk != 0);
-          ptx::mma_commit_both(&part_full[buf]);
+          for (int h = 0; h < 2; ++h) {  // half h: rows 64 h.. of both CTAs' weight rows
+            const int buf = 2 * (step & 1) + h;
+            const long long tm1 = PROF ? clock64() : 0;
+            if (!ptx::mbar_wait(&part_empty[buf], ((step >> 1) & 1) ^ 1)) {
+              report(0x600 | buf);
+              alive = false;
+              break;
+            }
+            if (PROF) prof_mp += clock64() - tm1;
+            ptx::tc_fence_after_sync();
+#pragma unroll
+            for (int kk = 0; kk < KBYTES / 32; ++kk)
+              ptx::mma_f8f6f4_ss_pair(tmem_base + buf * 128, da + 2 * kk, db + h * (64 * KBYTES >> 4) + 2 * kk, idesc, kk != 0);
+            ptx::mma_commit_both(&part_full[buf]);
+          }
+          if (!alive) break;
           ptx::mma_commit_both(&empty_bar[stage]);
           if (++stage == STAGES) {
             stage = 0;
@@ -771,24 +800,23 @@ grouped_gemm_pair_fold_wide_kernel(const __grid_constant__ CUtensorMap map_t, co
       }
       if constexpr (GATED) {
         if (p.zero_padding && tl.last && me == 0) {  // rows between the expert's last token and its block's end
-          const int from = tl.row0 + tl.cols, end = (from + 127) & ~127;
-          for (int i = lane; i < (end - from) * 8; i += 32)
-            *reinterpret_cast<uint4*>(reinterpret_cast<__nv_bfloat16*>(p.out) + (int64_t)(from + (i >> 3)) * p.n +
-                                      tl.w_tile * 128 + rank * 64 + (i & 7) * 8) = make_uint4(0, 0, 0, 0);
+          zero_block_rows(tl, p.out, p.n, tl.w_tile * 128 + rank * 64,
+                          p.out_dtype == FMOE_F32 ? 4 : (p.out_dtype == FMOE_BF16 ? 2 : 1), lane, 32);
         }
       }
     }
   } else {
     // ---------------- fold + epilogue (warps 0-15) ----------------
+    asm volatile("setmaxnreg.inc.sync.aligned.u32 104;");
     // This loop runs at the 96 registers that 20 warps leave a thread: the tile is described by its meta entry, shared
     // memory addresses are constants, everything else is derived from three counters.
-    const uint32_t lane_addr = tmem_base + ((uint32_t)((warp & 3) * 32) << 16) + 32 * (warp >> 2);
+    const uint32_t lane_addr = tmem_base + ((uint32_t)((warp & 3) * 32) << 16) + 16 * (warp >> 2);
     uint32_t step = 0;  // K blocks folded so far
     int ltile = 0;
     bool alive = true;
     long long prof_fw = 0, prof_fb = 0, prof_sw = 0, prof_epi = 0;
     for (; worker + ltile * workers < total_tiles; ++ltile) {
-      float acc[64];  // [0,32): first half's 32 columns, [32,64): second half's
+      float acc[64];  // [32 h + i]: half h, i < 16 first 128 rows' (gate's) columns, i >= 16 the second's (up's)
 #pragma unroll
       for (int i = 0; i < 64; ++i) acc[i] = 0.f;
       bool mine = false;  // some of this warp's lanes hold tokens
@@ -808,34 +836,39 @@ grouped_gemm_pair_fold_wide_kernel(const __grid_constant__ CUtensorMap map_t, co
           src = ptx::smem_u32(scales) + (group % SC_SLOTS) * G::SLOT_BYTES + ((warp & 3) * 32 + lane) * 4;
           if (PROF) prof_sw += clock64() - tf0;
         }
-        const long long tf1 = PROF ? clock64() : 0;
-        if (!warp_wait(&part_full[step & 1], (step >> 1) & 1)) {
-          report(0x700);
-          alive = false;
-          break;
-        }
-        const long long tf2 = PROF ? clock64() : 0;
-        ptx::tc_fence_after_sync();
-        if (mine) {
-          const float f0 = lds32(src), f1 = lds32(src + 512);
 #pragma unroll
-          for (int c = 0; c < 4; ++c) {
-            // 16 columns at a time keeps the staging registers small (the 64 accumulators stay live)
-            uint32_t v[16];
-            ptx::tmem_ld_32x32b_x16(lane_addr + (step & 1) * 256 + (c >> 1) * 128 + (c & 1) * 16, v);
+        for (int h = 0; h < 2; ++h) {
+          const int buf = 2 * (step & 1) + h;
+          const long long tf1 = PROF ? clock64() : 0;
+          if (!warp_wait(&part_full[buf], (step >> 1) & 1)) {
+            report(0x700);
+            alive = false;
+            break;
+          }
+          const long long tf2 = PROF ? clock64() : 0;
+          ptx::tc_fence_after_sync();
+          if (mine) {
+            uint32_t v[16], w[16];
+            ptx::tmem_ld_32x32b_x16(lane_addr + buf * 128, v);
+            ptx::tmem_ld_32x32b_x16(lane_addr + buf * 128 + 64, w);
+            const float f0 = lds32(src), f1 = lds32(src + 512);
             ptx::tmem_ld_wait();
 #pragma unroll
-            for (int i = 0; i < 16; ++i) acc[16 * c + i] = fmaf(__uint_as_float(v[i]), c < 2 ? f0 : f1, acc[16 * c + i]);
+            for (int i = 0; i < 16; ++i) {
+              acc[32 * h + i] = fmaf(__uint_as_float(v[i]), f0, acc[32 * h + i]);
+              acc[32 * h + 16 + i] = fmaf(__uint_as_float(w[i]), f1, acc[32 * h + 16 + i]);
+            }
+          }
+          ptx::tc_fence_before_sync();
+          __syncwarp();
+          if (lane == 0) ptx::mbar_arrive_cluster((ptx::smem_u32(part_empty) & ~ptx::kPeerRankBit) + buf * 8);
+          if (PROF) {
+            prof_fw += tf2 - tf1;
+            prof_fb += clock64() - tf2;
           }
         }
+        if (!alive) break;
         src += G::KB_BYTES;
-        ptx::tc_fence_before_sync();
-        __syncwarp();
-        if (lane == 0) ptx::mbar_arrive_cluster((ptx::smem_u32(part_empty) & ~ptx::kPeerRankBit) + (step & 1) * 8);
-        if (PROF) {
-          prof_fw += tf2 - tf1;
-          prof_fb += clock64() - tf2;
-        }
       }
       if (!alive) break;
       if (lane == 0) ptx::mbar_arrive(&sc_empty[((ltile + 1) * ((kblocks + G::GROUP - 1) / G::GROUP) - 1) % SC_SLOTS]);
@@ -844,45 +877,68 @@ grouped_gemm_pair_fold_wide_kernel(const __grid_constant__ CUtensorMap map_t, co
       const int32_t* m = meta + (ltile % META_TILES) * G::META_WORDS;
       const int32_t slot = m[(warp & 3) * 32 + lane];
       const float rs = __int_as_float(m[128 + (warp & 3) * 32 + lane]);
-      if (mine && slot >= 0) {
-        const int cpart = warp >> 2;
-        if constexpr (GATED) {
-          // acc[0..31] gate, acc[32..63] up -> output columns w_tile*128 + 32*cpart + [0,32)
-          const int64_t pos = m[256] + (warp & 3) * 32 + lane;
-          uint4* dst = reinterpret_cast<uint4*>(reinterpret_cast<__nv_bfloat16*>(p.out) + pos * p.n + (int64_t)m[258] * 128 +
-                                                32 * cpart);
+      const int cpart = warp >> 2;
+      if constexpr (GATED) {
+        // output columns w_tile * 128 + 64 h + 16 cpart + [0,16), in place of the gate accumulators
+        const int64_t pos = m[256] + (warp & 3) * 32 + lane, col = (int64_t)m[258] * 128 + 16 * cpart;
+        float amax = 0.f;
 #pragma unroll
-          for (int v = 0; v < 4; ++v) {
-            uint32_t w[4];
+        for (int h = 0; h < 2; ++h) {
 #pragma unroll
-            for (int j = 0; j < 4; ++j) {
-              const int i = 8 * v + 2 * j;
-              w[j] = pack_bf16x2(act_mul_fast(acc[i] * rs, acc[32 + i] * rs, p.activation),
-                                 act_mul_fast(acc[i + 1] * rs, acc[33 + i] * rs, p.activation));
-            }
-            dst[v] = make_uint4(w[0], w[1], w[2], w[3]);
+          for (int i = 0; i < 16; ++i) {
+            acc[32 * h + i] = act_mul_fast(acc[32 * h + i] * rs, acc[32 * h + 16 + i] * rs, p.activation);
+            amax = fmaxf(amax, fabsf(acc[32 * h + i]));
           }
-        } else {
-          // acc[0..31]: columns n0 + 32*cpart + [0,32); acc[32..63]: columns n0 + 128 + 32*cpart + [0,32)
-          __nv_bfloat16* obase = p.out_rows ? reinterpret_cast<__nv_bfloat16*>(p.out_rows[slot])
-                                            : reinterpret_cast<__nv_bfloat16*>(p.out) + (int64_t)slot * p.n;
+        }
+        if (p.out_dtype == FMOE_E4M3) {
+          // the tile's 128 channels are one quantisation group, held by four warps
+          float* am = amax_buf + (ltile & 1) * 512 + (warp & 3) * 32 + lane;
+          am[cpart * 128] = amax;
+          __syncwarp();
+          if (lane == 0) ptx::mbar_arrive(&amax_bar[warp & 3]);
+          if (!warp_wait(&amax_bar[warp & 3], ltile & 1)) {
+            report(0x7c0);
+            break;
+          }
+          amax = fmaxf(fmaxf(am[0], am[128]), fmaxf(am[256], am[384]));
+          if (mine && slot >= 0) {
+            const float s = group_scale(amax), r = __frcp_rn(s);
+#pragma unroll
+            for (int h = 0; h < 2; ++h) {
+              float v[8];
+              uint2 q[2];
+#pragma unroll
+              for (int u = 0; u < 2; ++u) {
+#pragma unroll
+                for (int i = 0; i < 8; ++i) v[i] = acc[32 * h + 8 * u + i];
+                q[u] = quant8(v, s, r, amax <= 3.0e38f);
+              }
+              *reinterpret_cast<uint4*>(reinterpret_cast<uint8_t*>(p.out) + pos * p.n + col + 64 * h) =
+                  make_uint4(q[0].x, q[0].y, q[1].x, q[1].y);
+            }
+            if (cpart == 0) p.out_scale[pos * (p.n / 128) + m[258]] = s;
+          }
+        } else if (mine && slot >= 0) {
 #pragma unroll
           for (int h = 0; h < 2; ++h) {
-            const int64_t colg = (int64_t)m[258] * 256 + 128 * h + 32 * cpart;
-            if (obase && colg < p.n) {
-              uint4* dst = reinterpret_cast<uint4*>(obase + colg);
+            if (p.out_dtype == FMOE_F32) {
+              float4* dst = reinterpret_cast<float4*>(reinterpret_cast<float*>(p.out) + pos * p.n + col + 64 * h);
 #pragma unroll
-              for (int v = 0; v < 4; ++v) {
-                uint32_t w[4];
-#pragma unroll
-                for (int j = 0; j < 4; ++j) {
-                  const int i = 32 * h + 8 * v + 2 * j;
-                  w[j] = pack_bf16x2(acc[i] * rs, acc[i + 1] * rs);
-                }
-                dst[v] = make_uint4(w[0], w[1], w[2], w[3]);
-              }
+              for (int v = 0; v < 4; ++v)
+                dst[v] = make_float4(acc[32 * h + 4 * v], acc[32 * h + 4 * v + 1], acc[32 * h + 4 * v + 2], acc[32 * h + 4 * v + 3]);
+            } else {
+              store16(reinterpret_cast<__nv_bfloat16*>(p.out) + pos * p.n + col + 64 * h, &acc[32 * h], 1.0f);
             }
           }
+        }
+      } else if (mine && slot >= 0) {
+        // columns w_tile * 256 + 128 c + 64 h + 16 cpart + [0,16)
+        __nv_bfloat16* obase = p.out_rows ? reinterpret_cast<__nv_bfloat16*>(p.out_rows[slot])
+                                          : reinterpret_cast<__nv_bfloat16*>(p.out) + (int64_t)slot * p.n;
+#pragma unroll
+        for (int q = 0; q < 4; ++q) {
+          const int64_t colg = (int64_t)m[258] * 256 + 128 * (q & 1) + 64 * (q >> 1) + 16 * cpart;
+          if (obase && colg < p.n) store16(obase + colg, &acc[16 * q], rs);
         }
       }
       if (PROF) prof_epi += clock64() - te0;
@@ -948,6 +1004,8 @@ int launch(const GemmParams& g, cudaStream_t st) {
   p.activation = g.activation;
   p.group = pick_group_m(tile, g.k);
   p.zero_padding = !g.skip_padding;
+  p.out_dtype = g.out_dtype;
+  p.out_scale = g.out_scale;
 
   const int64_t max_tiles = g.max_blocks * ceil_div(128, tile) * p.w_tiles;
   const int sms = device_sm_count();
@@ -960,7 +1018,8 @@ int launch(const GemmParams& g, cudaStream_t st) {
 }  // namespace
 
 bool gemm_pair_fold_supports(const GemmParams& p, bool gated) {
-  if (p.dtype != FMOE_E4M3 || p.out_dtype != FMOE_BF16) return false;
+  if (p.dtype != FMOE_E4M3) return false;
+  if (p.out_dtype != FMOE_BF16 && !(gated && (p.out_dtype == FMOE_F32 || (p.out_dtype == FMOE_E4M3 && p.out_scale)))) return false;
   if (p.bias || p.activation == FMOE_ACT_SWIGLU_OAI) return false;  // bf16-only variant
   if (p.block_size != 128 || p.a_gather) return false;
   if (p.k <= 0 || p.k % 128 != 0 || p.n <= 0 || p.n % 128 != 0) return false;
@@ -986,11 +1045,15 @@ int status_word_fp8(int* out, bool clear) {
 int gemm_pair_fold(const GemmParams& p, bool gated, cudaStream_t st) {
   if (!gemm_pair_fold_supports(p, gated))
     return fail(FMOE_ERR_UNSUPPORTED,
-                "tcgen05 fp8 gemm: needs e4m3 in, bf16 out, block_size 128, sorted input rows, n and k multiples of 128");
+                "tcgen05 fp8 gemm: needs e4m3 in, bf16 out (gate/up: or f32, or e4m3 with out_scale), block_size 128, sorted "
+                "input rows, n and k multiples of 128");
   if (p.max_blocks <= 0) return FMOE_OK;
   static const bool profile = getenv("FMOE_TC_PROFILE") != nullptr;
   // the table's tile width decides: 64-token tiles for the narrow kernel, 256 for the wide one
-  const bool wide = (p.token_tile ? p.token_tile : pick_fold_token_tile(p.numel, p.num_experts)) == 256;
+  // (e4m3 output needs the wide one: a narrow tile's 128 channels are spread over both CTAs)
+  const bool e4m3_out = gated && p.out_dtype == FMOE_E4M3;
+  const bool wide = p.token_tile ? p.token_tile == 256 : e4m3_out || pick_fold_token_tile(p.numel, p.num_experts) == 256;
+  FMOE_REQUIRE(wide || !e4m3_out, "tcgen05 fp8 gemm: e4m3 output needs 256-token tiles");
   auto go = [&](auto gated_c, auto wide_c) {
     constexpr bool G = decltype(gated_c)::value, W = decltype(wide_c)::value;
     return profile ? launch<G, W, true>(p, st) : launch<G, W, false>(p, st);

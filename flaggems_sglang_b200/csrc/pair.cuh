@@ -179,12 +179,14 @@ __device__ __forceinline__ void strip_store_slots(const uint8_t* strip, int lane
   __syncwarp();
 }
 // gate/up GEMM through the plain C entry point: the rows between the expert's last token and the end of its 128-row block
-// are zeros in this CTA's 64 channels.  All `threads` epilogue threads.
-__device__ __forceinline__ void zero_block_rows(const PairTile& tl, void* out, int64_t n, int ch, int threads) {
+// are zeros in this CTA's 64 channels (of elem_bytes each).  All `threads` epilogue threads.
+__device__ __forceinline__ void zero_block_rows(const PairTile& tl, void* out, int64_t n, int ch, int elem_bytes, int thread,
+                                                int threads) {
   const int from = tl.row0 + tl.cols, end = (from + 127) & ~127;  // blocks start at multiples of 128 rows
-  for (int i = threadIdx.x; i < (end - from) * 8; i += threads) {
-    const int64_t row = from + (i >> 3), c = ch + (i & 7) * 8;
-    if (c < n) *reinterpret_cast<uint4*>(reinterpret_cast<__nv_bfloat16*>(out) + row * n + c) = make_uint4(0, 0, 0, 0);
+  const int per_row = 4 * elem_bytes;                              // 16-byte pieces
+  for (int i = thread; i < (end - from) * per_row; i += threads) {
+    const int64_t row = from + i / per_row, c = ch * elem_bytes + i % per_row * 16;
+    if (c < n * elem_bytes) *reinterpret_cast<uint4*>(reinterpret_cast<uint8_t*>(out) + row * n * elem_bytes + c) = make_uint4(0, 0, 0, 0);
   }
 }
 #endif

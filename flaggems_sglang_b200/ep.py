@@ -269,9 +269,8 @@ class PeerExchange:
         self.expert_ids = torch.empty(cap // blk, dtype=torch.int32, device=dev)
         self.npp = torch.zeros(1, dtype=torch.int32, device=dev)
         self.out_rows = torch.zeros(cap, dtype=torch.int64, device=dev)
-        tc = self.variant.startswith("tcgen05")
         if self.fp8:
-            self.act = torch.empty(cap, self.I, dtype=torch.bfloat16 if tc else torch.float32, device=dev)
+            self.act = torch.empty(cap, self.I, dtype=torch.float32, device=dev)
             self.actq = torch.empty(cap, self.I, dtype=torch.float8_e4m3fn, device=dev)
             self.act_scale = torch.empty(cap, self.I // 128, dtype=torch.float32, device=dev)
         else:

@@ -397,16 +397,16 @@ def _experts(hidden_states, w1, w2, topk_weights, topk_ids, route, k, inplace=Fa
                 with _stage("quant_input"):
                     _C.check(lib.fmoe_quant_fp8_group128(x.data_ptr(), _C.BF16, cap, H, sorted_ids.data_ptr(), k, numel,
                                                          num_post.data_ptr(), xq.data_ptr(), xsc.data_ptr(), st))
-            a_rows, gather, act_dtype, act_code = cap, 0, torch.bfloat16, _C.BF16
+            a_rows, gather = cap, 0
         else:
             xq = torch.empty((T, H), dtype=torch.float8_e4m3fn, device=dev)
             xsc = torch.empty((T, H // 128), dtype=torch.float32, device=dev)
             with _stage("quant_input"):
                 _C.check(lib.fmoe_quant_fp8_group128(x.data_ptr(), _C.BF16, T, H, None, 1, 0, None, xq.data_ptr(),
                                                      xsc.data_ptr(), st))
-            a_rows, gather, act_dtype, act_code = T, 1, torch.float32, _C.F32
-        act = torch.empty((cap, I), dtype=act_dtype, device=dev)
-        g1 = _gemm_args(dtype=_C.E4M3, out_dtype=act_code, a_gather=gather, n=I, k=H, a_rows=a_rows, a=xq.data_ptr(),
+            a_rows, gather = T, 1
+        act = torch.empty((cap, I), dtype=torch.float32, device=dev)
+        g1 = _gemm_args(dtype=_C.E4M3, out_dtype=_C.F32, a_gather=gather, n=I, k=H, a_rows=a_rows, a=xq.data_ptr(),
                         a_scale=xsc.data_ptr(), w=w1.data_ptr(), w_scale=w1_scale.data_ptr(),
                         row_scale=row_w if apply_router_weight_on_input else None, out=act.data_ptr(), **common)
         with _stage("gemm1_fp8_" + name):
@@ -414,7 +414,7 @@ def _experts(hidden_states, w1, w2, topk_weights, topk_ids, route, k, inplace=Fa
         aq = torch.empty((cap, I), dtype=torch.float8_e4m3fn, device=dev)
         asc = torch.empty((cap, I // 128), dtype=torch.float32, device=dev)
         with _stage("quant_act"):
-            _C.check(lib.fmoe_quant_fp8_group128(act.data_ptr(), act_code, cap, I, sorted_ids.data_ptr(), 0, numel, num_post.data_ptr(),
+            _C.check(lib.fmoe_quant_fp8_group128(act.data_ptr(), _C.F32, cap, I, sorted_ids.data_ptr(), 0, numel, num_post.data_ptr(),
                                                  aq.data_ptr(), asc.data_ptr(), st))
         g2 = _gemm_args(dtype=_C.E4M3, out_dtype=_C.BF16, a_gather=0, n=H, k=I, a_rows=cap, a=aq.data_ptr(),
                         a_scale=asc.data_ptr(), w=w2.data_ptr(), w_scale=w2_scale.data_ptr(),
