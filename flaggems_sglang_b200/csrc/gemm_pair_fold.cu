@@ -9,8 +9,9 @@
 //   tile      : 256 weight rows (128 per CTA) x up to 64 tokens of one expert, as in gemm_pair.cu (same tile order, same
 //               row interleave of gate and up, same transposed stores)
 //   TMEM      : 512 columns per CTA as eight partials of 64 tokens: the MMAs of the next K blocks run while one is folded
-//   warps 0-15: fold + epilogue.  Warp w reads TMEM lanes 32 * (w % 4).. and the 16-token piece w / 4.  16 x 256b read-out puts two tokens of one channel side by side, which is
-//               what the packed fma.rn.f32x2 takes with one pair of factors for two channels
+//   warps 0-15: fold + epilogue.  Warp w reads TMEM lanes 32 * (w % 4).. and the 16-token piece w / 4.  The 16 x 256b
+//               read-out puts two tokens of one channel side by side, which is what the packed fma.rn.f32x2 takes with one
+//               pair of factors for two channels.  The gate/up output is fp32, for the quantiser behind it
 //   warp 16   : TMA producer      warp 17 : MMA issuer (CTA 0)
 //   warps 18-19: factors.  For four K blocks at a time they multiply the tokens' scales with the tile's one or two weight
 //               scales and leave the products in a 3-slot ring in shared memory, next to the tile's slots and row weights:
@@ -118,13 +119,15 @@ __device__ __forceinline__ unsigned long long lds64(uint32_t addr) {
   return v;
 }
 
-// 16 values times s as bf16
-__device__ __forceinline__ void store16(__nv_bfloat16* dst, const float* v, float s) {
-  uint32_t w[8];
+// 32 values times s as bf16
+__device__ __forceinline__ void store32(__nv_bfloat16* dst, const float* v, float s) {
 #pragma unroll
-  for (int j = 0; j < 8; ++j) w[j] = pack_bf16x2(v[2 * j] * s, v[2 * j + 1] * s);
-  reinterpret_cast<uint4*>(dst)[0] = make_uint4(w[0], w[1], w[2], w[3]);
-  reinterpret_cast<uint4*>(dst)[1] = make_uint4(w[4], w[5], w[6], w[7]);
+  for (int q = 0; q < 4; ++q) {
+    uint32_t w[4];
+#pragma unroll
+    for (int j = 0; j < 4; ++j) w[j] = pack_bf16x2(v[8 * q + 2 * j] * s, v[8 * q + 2 * j + 1] * s);
+    reinterpret_cast<uint4*>(dst)[q] = make_uint4(w[0], w[1], w[2], w[3]);
+  }
 }
 
 // PROF: instrumented build with wait-time counters (reading the clock is slow enough to distort the fold loop).
@@ -528,11 +531,21 @@ grouped_gemm_pair_fold_kernel(const __grid_constant__ CUtensorMap map_t, const _
 // then owns one token: its activation scale is ONE value per K block and the weight scale one value per 128 columns, and
 // TMEM is read 32 lanes wide.  With tokens on N every thread needs one factor per column: a 16-lane read-out with packed
 // factors takes 512 cycles of TMEM and 128-256 shared-memory loads per 128 x 256 partial, a 32-lane one 256 cycles and 1024
-// cycles of broadcast loads (both measured), against 310 cycles and 32 loads here.  In exchange M is always 256: tokens short of that
-// are lanes without work, so experts with few rows stay on the narrow kernel.
-//   warps 0-15: fold + epilogue: TMEM lanes 32 * (w % 4).., columns 32 * (w / 4).. of each half: 64 accumulators per thread
+// cycles of broadcast loads (both measured), against 310 cycles and 32 loads here.  In exchange M is always 256: tokens short
+// of that are lanes without work, so experts with few rows stay on the narrow kernel.
+//   TMEM: four partials of 128 columns.  A K block's MMAs go to two of them: the first holds rows 0-63 of both CTAs' weights,
+//   the second rows 64-127.
+//   warps 0-15: fold + epilogue.  Eight warps fold each half, so that one half's TMEM reads run beside the other's FMAs and a
+//   partial is handed back while the other half is still being multiplied (one partial of 256 columns per K block, folded by
+//   all sixteen warps at once: gate/up + down of DeepSeek-V3, 4096 tokens, 3.43 ms; this split 3.25 ms).  Warp w: TMEM lanes
+//   32 * (w % 4).., half w / 8, columns 32 * (w / 4 % 2).. of gate and of up: 64 accumulators per thread.  The loop keeps
+//   its addresses in two registers; every spill inside it shows (44 bytes of them: 3.76 ms)
 //   warp 16 TMA, warp 17 MMA (CTA 0), warps 18-19 factors: products of token and weight scales in a ring of 4 slots of 8 K
 //   blocks, one slot wait per 8 K blocks of the fold
+// The gate/up kernel quantises its output: the tile's 128 channels of a token are one group, spread over four warps, which
+// exchange their largest magnitudes through shared memory.  (A bf16 activation and a quantiser pass took 135 us of that case.)
+// What bounds it: the power limit (980 W, SM clock 1.4 GHz of 1.965) and the fold, about 800 cycles per K block against 512
+// of MMA.
 // ---------------------------------------------------------------------------------------------------------------------
 struct WideGeo {
   static constexpr int STAGE_BYTES = 2 * W_BYTES;  // 128 token rows + 128 weight rows per CTA
@@ -582,7 +595,7 @@ grouped_gemm_pair_fold_wide_kernel(const __grid_constant__ CUtensorMap map_t, co
     }
     for (int b = 0; b < 4; ++b) {
       ptx::mbar_init(&part_full[b], 1);
-      ptx::mbar_init(&part_empty[b], 2 * kFoldWarps);
+      ptx::mbar_init(&part_empty[b], kFoldWarps);  // the half's 8 warps of both CTAs
       ptx::mbar_init(&amax_bar[b], 4);
     }
     for (int s = 0; s < SC_SLOTS; ++s) {
@@ -611,6 +624,7 @@ grouped_gemm_pair_fold_wide_kernel(const __grid_constant__ CUtensorMap map_t, co
   PairCursor cursor;
   PairTile tl;
 
+  // 16 * 104 + 4 * 64 registers per lane are the launch's 20 * 96
   // 16 * 104 + 4 * 64 registers per lane are the launch's 20 * 96
   if (warp >= kFoldWarps) asm volatile("setmaxnreg.dec.sync.aligned.u32 64;");
   if (warp == kFoldWarps) {
@@ -810,37 +824,35 @@ grouped_gemm_pair_fold_wide_kernel(const __grid_constant__ CUtensorMap map_t, co
     asm volatile("setmaxnreg.inc.sync.aligned.u32 104;");
     // This loop runs at the 96 registers that 20 warps leave a thread: the tile is described by its meta entry, shared
     // memory addresses are constants, everything else is derived from three counters.
-    const uint32_t lane_addr = tmem_base + ((uint32_t)((warp & 3) * 32) << 16) + 16 * (warp >> 2);
-    uint32_t step = 0;  // K blocks folded so far
+    const uint32_t lane_addr = tmem_base + ((uint32_t)((warp & 3) * 32) << 16) + 128 * (warp >> 3) + 32 * ((warp >> 2) & 1);
+    const uint32_t my_full = ptx::smem_u32(part_full) + 8 * (warp >> 3);  // the warp's half of the even K blocks
+    constexpr uint32_t kToEmpty = 4 * 8;                                   // from part_full to part_empty
+    uint32_t step = 0, group = 0;  // K blocks folded so far; factor slots used
     int ltile = 0;
     bool alive = true;
     long long prof_fw = 0, prof_fb = 0, prof_sw = 0, prof_epi = 0;
     for (; worker + ltile * workers < total_tiles; ++ltile) {
-      float acc[64];  // [32 h + i]: half h, i < 16 first 128 rows' (gate's) columns, i >= 16 the second's (up's)
+      float acc[64];  // 32 columns of the first 128 weight rows (gate), then the same 32 of the second (up)
 #pragma unroll
       for (int i = 0; i < 64; ++i) acc[i] = 0.f;
       bool mine = false;  // some of this warp's lanes hold tokens
-      uint32_t src = 0;
 #pragma unroll 1
-      for (int kb = 0; kb < kblocks; ++kb, ++step) {
-        if ((kb & (G::GROUP - 1)) == 0) {
-          const long long tf0 = PROF ? clock64() : 0;
-          const uint32_t group = ltile * ((kblocks + G::GROUP - 1) / G::GROUP) + kb / G::GROUP;
-          if (kb > 0 && lane == 0) ptx::mbar_arrive(&sc_empty[(group - 1) % SC_SLOTS]);
-          if (!warp_wait(&sc_full[group % SC_SLOTS], (group / SC_SLOTS) & 1)) {
-            report(0x740);
-            alive = false;
-            break;
-          }
-          mine = (warp & 3) * 32 < meta[(ltile % META_TILES) * G::META_WORDS + 257];
-          src = ptx::smem_u32(scales) + (group % SC_SLOTS) * G::SLOT_BYTES + ((warp & 3) * 32 + lane) * 4;
-          if (PROF) prof_sw += clock64() - tf0;
+      for (int left = kblocks; left > 0; left -= G::GROUP, ++group) {
+        const long long tf0 = PROF ? clock64() : 0;
+        if (!warp_wait(&sc_full[group % SC_SLOTS], (group / SC_SLOTS) & 1)) {
+          report(0x740);
+          alive = false;
+          break;
         }
-#pragma unroll
-        for (int h = 0; h < 2; ++h) {
-          const int buf = 2 * (step & 1) + h;
+        if (PROF) prof_sw += clock64() - tf0;
+        mine = (warp & 3) * 32 < meta[(ltile % META_TILES) * G::META_WORDS + 257];
+        uint32_t src = ptx::smem_u32(scales) + (group % SC_SLOTS) * G::SLOT_BYTES + ((warp & 3) * 32 + lane) * 4;
+        const uint32_t end = step + min(left, G::GROUP);
+#pragma unroll 1
+        for (; step != end; ++step, src += G::KB_BYTES) {
+          const uint32_t odd = step & 1;
           const long long tf1 = PROF ? clock64() : 0;
-          if (!warp_wait(&part_full[buf], (step >> 1) & 1)) {
+          if (!__all_sync(0xffffffffu, ptx::mbar_wait_addr(my_full + odd * 16, (step >> 1) & 1))) {
             report(0x700);
             alive = false;
             break;
@@ -848,30 +860,29 @@ grouped_gemm_pair_fold_wide_kernel(const __grid_constant__ CUtensorMap map_t, co
           const long long tf2 = PROF ? clock64() : 0;
           ptx::tc_fence_after_sync();
           if (mine) {
-            uint32_t v[16], w[16];
-            ptx::tmem_ld_32x32b_x16(lane_addr + buf * 128, v);
-            ptx::tmem_ld_32x32b_x16(lane_addr + buf * 128 + 64, w);
-            const float f0 = lds32(src), f1 = lds32(src + 512);
-            ptx::tmem_ld_wait();
 #pragma unroll
-            for (int i = 0; i < 16; ++i) {
-              acc[32 * h + i] = fmaf(__uint_as_float(v[i]), f0, acc[32 * h + i]);
-              acc[32 * h + 16 + i] = fmaf(__uint_as_float(w[i]), f1, acc[32 * h + 16 + i]);
+            for (int c = 0; c < 4; ++c) {
+              // 16 columns at a time keeps the staging registers few (the 64 accumulators stay live)
+              const float f = lds32(src + (c >> 1) * 512);
+              uint32_t v[16];
+              ptx::tmem_ld_32x32b_x16(lane_addr + odd * 256 + (c >> 1) * 64 + (c & 1) * 16, v);
+              ptx::tmem_ld_wait();
+#pragma unroll
+              for (int i = 0; i < 16; ++i) acc[16 * c + i] = fmaf(__uint_as_float(v[i]), f, acc[16 * c + i]);
             }
           }
           ptx::tc_fence_before_sync();
           __syncwarp();
-          if (lane == 0) ptx::mbar_arrive_cluster((ptx::smem_u32(part_empty) & ~ptx::kPeerRankBit) + buf * 8);
+          if (ptx::elect_one()) ptx::mbar_arrive_cluster(((my_full + odd * 16) & ~ptx::kPeerRankBit) + kToEmpty);
           if (PROF) {
             prof_fw += tf2 - tf1;
             prof_fb += clock64() - tf2;
           }
         }
         if (!alive) break;
-        src += G::KB_BYTES;
+        if (lane == 0) ptx::mbar_arrive(&sc_empty[group % SC_SLOTS]);
       }
       if (!alive) break;
-      if (lane == 0) ptx::mbar_arrive(&sc_empty[((ltile + 1) * ((kblocks + G::GROUP - 1) / G::GROUP) - 1) % SC_SLOTS]);
 
       const long long te0 = PROF ? clock64() : 0;
       const int32_t* m = meta + (ltile % META_TILES) * G::META_WORDS;
@@ -879,16 +890,13 @@ grouped_gemm_pair_fold_wide_kernel(const __grid_constant__ CUtensorMap map_t, co
       const float rs = __int_as_float(m[128 + (warp & 3) * 32 + lane]);
       const int cpart = warp >> 2;
       if constexpr (GATED) {
-        // output columns w_tile * 128 + 64 h + 16 cpart + [0,16), in place of the gate accumulators
-        const int64_t pos = m[256] + (warp & 3) * 32 + lane, col = (int64_t)m[258] * 128 + 16 * cpart;
+        // output columns w_tile * 128 + 32 cpart + [0,32), in place of the gate accumulators
+        const int64_t at = (int64_t)(m[256] + (warp & 3) * 32 + lane) * p.n + m[258] * 128 + 32 * cpart;
         float amax = 0.f;
 #pragma unroll
-        for (int h = 0; h < 2; ++h) {
-#pragma unroll
-          for (int i = 0; i < 16; ++i) {
-            acc[32 * h + i] = act_mul_fast(acc[32 * h + i] * rs, acc[32 * h + 16 + i] * rs, p.activation);
-            amax = fmaxf(amax, fabsf(acc[32 * h + i]));
-          }
+        for (int i = 0; i < 32; ++i) {
+          acc[i] = act_mul_fast(acc[i] * rs, acc[32 + i] * rs, p.activation);
+          amax = fmaxf(amax, fabsf(acc[i]));
         }
         if (p.out_dtype == FMOE_E4M3) {
           // the tile's 128 channels are one quantisation group, held by four warps
@@ -903,6 +911,7 @@ grouped_gemm_pair_fold_wide_kernel(const __grid_constant__ CUtensorMap map_t, co
           amax = fmaxf(fmaxf(am[0], am[128]), fmaxf(am[256], am[384]));
           if (mine && slot >= 0) {
             const float s = group_scale(amax), r = __frcp_rn(s);
+            uint4* dst = reinterpret_cast<uint4*>(reinterpret_cast<uint8_t*>(p.out) + at);
 #pragma unroll
             for (int h = 0; h < 2; ++h) {
               float v[8];
@@ -910,35 +919,30 @@ grouped_gemm_pair_fold_wide_kernel(const __grid_constant__ CUtensorMap map_t, co
 #pragma unroll
               for (int u = 0; u < 2; ++u) {
 #pragma unroll
-                for (int i = 0; i < 8; ++i) v[i] = acc[32 * h + 8 * u + i];
+                for (int i = 0; i < 8; ++i) v[i] = acc[16 * h + 8 * u + i];
                 q[u] = quant8(v, s, r, amax <= 3.0e38f);
               }
-              *reinterpret_cast<uint4*>(reinterpret_cast<uint8_t*>(p.out) + pos * p.n + col + 64 * h) =
-                  make_uint4(q[0].x, q[0].y, q[1].x, q[1].y);
+              dst[h] = make_uint4(q[0].x, q[0].y, q[1].x, q[1].y);
             }
-            if (cpart == 0) p.out_scale[pos * (p.n / 128) + m[258]] = s;
+            if (cpart == 0) p.out_scale[at >> 7] = s;  // n is a multiple of 128
           }
         } else if (mine && slot >= 0) {
+          if (p.out_dtype == FMOE_F32) {
+            float4* dst = reinterpret_cast<float4*>(reinterpret_cast<float*>(p.out) + at);
 #pragma unroll
-          for (int h = 0; h < 2; ++h) {
-            if (p.out_dtype == FMOE_F32) {
-              float4* dst = reinterpret_cast<float4*>(reinterpret_cast<float*>(p.out) + pos * p.n + col + 64 * h);
-#pragma unroll
-              for (int v = 0; v < 4; ++v)
-                dst[v] = make_float4(acc[32 * h + 4 * v], acc[32 * h + 4 * v + 1], acc[32 * h + 4 * v + 2], acc[32 * h + 4 * v + 3]);
-            } else {
-              store16(reinterpret_cast<__nv_bfloat16*>(p.out) + pos * p.n + col + 64 * h, &acc[32 * h], 1.0f);
-            }
+            for (int v = 0; v < 8; ++v) dst[v] = make_float4(acc[4 * v], acc[4 * v + 1], acc[4 * v + 2], acc[4 * v + 3]);
+          } else {
+            store32(reinterpret_cast<__nv_bfloat16*>(p.out) + at, acc, 1.0f);
           }
         }
       } else if (mine && slot >= 0) {
-        // columns w_tile * 256 + 128 c + 64 h + 16 cpart + [0,16)
+        // columns w_tile * 256 + 32 cpart + [0,32), and the same 128 further
         __nv_bfloat16* obase = p.out_rows ? reinterpret_cast<__nv_bfloat16*>(p.out_rows[slot])
                                           : reinterpret_cast<__nv_bfloat16*>(p.out) + (int64_t)slot * p.n;
 #pragma unroll
-        for (int q = 0; q < 4; ++q) {
-          const int64_t colg = (int64_t)m[258] * 256 + 128 * (q & 1) + 64 * (q >> 1) + 16 * cpart;
-          if (obase && colg < p.n) store16(obase + colg, &acc[16 * q], rs);
+        for (int h = 0; h < 2; ++h) {
+          const int64_t colg = (int64_t)m[258] * 256 + 128 * h + 32 * cpart;
+          if (obase && colg < p.n) store32(obase + colg, &acc[32 * h], rs);
         }
       }
       if (PROF) prof_epi += clock64() - te0;

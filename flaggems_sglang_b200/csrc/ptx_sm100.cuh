@@ -29,29 +29,32 @@ __device__ __forceinline__ void mbar_arrive_expect_tx(uint64_t* bar, uint32_t by
 __device__ __forceinline__ void mbar_arrive(uint64_t* bar) {
   asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_u32(bar)) : "memory");
 }
-__device__ __forceinline__ bool mbar_try_wait(uint64_t* bar, uint32_t parity) {
+__device__ __forceinline__ bool mbar_try_wait(uint32_t addr, uint32_t parity) {
   uint32_t ok;
   asm volatile(
       "{\n\t.reg .pred p;\n\t"
       "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
       "selp.u32 %0, 1, 0, p;\n\t}"
       : "=r"(ok)
-      : "r"(smem_u32(bar)), "r"(parity)
+      : "r"(addr), "r"(parity)
       : "memory");
   return ok != 0;
 }
+__device__ __forceinline__ bool mbar_try_wait(uint64_t* bar, uint32_t parity) { return mbar_try_wait(smem_u32(bar), parity); }
 // Bounded wait for the phase with the given parity.  Returns false on time-out.
-__device__ __forceinline__ bool mbar_wait_limit(uint64_t* bar, uint32_t parity, long long limit_cycles) {
-  if (mbar_try_wait(bar, parity)) return true;
+__device__ __forceinline__ bool mbar_wait_limit(uint32_t addr, uint32_t parity, long long limit_cycles) {
+  if (mbar_try_wait(addr, parity)) return true;
   const long long t0 = clock64();
   while (true) {
-    if (mbar_try_wait(bar, parity)) return true;
+    if (mbar_try_wait(addr, parity)) return true;
     if (clock64() - t0 > limit_cycles) return false;
   }
 }
-__device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity) {
-  return mbar_wait_limit(bar, parity, kWaitCycles);
+__device__ __forceinline__ bool mbar_wait_limit(uint64_t* bar, uint32_t parity, long long limit_cycles) {
+  return mbar_wait_limit(smem_u32(bar), parity, limit_cycles);
 }
+__device__ __forceinline__ bool mbar_wait_addr(uint32_t addr, uint32_t parity) { return mbar_wait_limit(addr, parity, kWaitCycles); }
+__device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity) { return mbar_wait_addr(smem_u32(bar), parity); }
 
 // Non-suspending poll (mbarrier.test_wait): for waits that sit on a kernel's critical path and are short, where the
 // wake-up time of a suspended try_wait would be paid on every hand-over.  Bounded like the others.
