@@ -73,7 +73,7 @@ __global__ void __launch_bounds__(kThreads)
 moe_align_kernel(const int32_t* __restrict__ topk_ids, int numel, int E, int block,
                  int32_t* __restrict__ sorted_ids, int sorted_cap, int32_t* __restrict__ expert_ids,
                  int expert_cap, int32_t* __restrict__ num_post_pad, int32_t* __restrict__ table, int token_tile,
-                 int32_t* __restrict__ zero_words, int num_zero) {
+                 int32_t* __restrict__ zero_words, int num_zero, int32_t* __restrict__ slot_pos, int rows_only) {
   pdl_entry();
   extern __shared__ int s_mem[];
   int* s_cnt = s_mem;                  // [kWarps][E] counts, then running output positions
@@ -124,17 +124,19 @@ moe_align_kernel(const int32_t* __restrict__ topk_ids, int numel, int E, int blo
   if (warp == 0) scan_experts_warp(s_total, s_start, E, block, lane, num_post_pad, table, token_tile);
   __syncthreads();
 
-  // block -> expert map (-1 after the used blocks)
-  const int used_blocks = s_start[E] / block;
-  for (int e = tid; e < E; e += kThreads) {
-    int b0 = s_start[e] / block, b1 = s_start[e + 1] / block;
-    for (int b = b0; b < b1 && b < expert_cap; ++b) expert_ids[b] = e;
+  if (!rows_only) {
+    // block -> expert map (-1 after the used blocks)
+    const int used_blocks = s_start[E] / block;
+    for (int e = tid; e < E; e += kThreads) {
+      int b0 = s_start[e] / block, b1 = s_start[e + 1] / block;
+      for (int b = b0; b < b1 && b < expert_cap; ++b) expert_ids[b] = e;
+    }
+    for (int b = used_blocks + tid; b < expert_cap; b += kThreads) expert_ids[b] = -1;
+    // sentinels: the padding of every expert, and everything past the used blocks
+    for (int e = warp; e < E; e += kWarps)
+      for (int i = s_start[e] + s_total[e] + lane; i < s_start[e + 1]; i += 32) sorted_ids[i] = numel;
+    for (int i = s_start[E] + tid; i < sorted_cap; i += kThreads) sorted_ids[i] = numel;
   }
-  for (int b = used_blocks + tid; b < expert_cap; b += kThreads) expert_ids[b] = -1;
-  // sentinels: the padding of every expert, and everything past the used blocks
-  for (int e = warp; e < E; e += kWarps)
-    for (int i = s_start[e] + s_total[e] + lane; i < s_start[e + 1]; i += 32) sorted_ids[i] = numel;
-  for (int i = s_start[E] + tid; i < sorted_cap; i += kThreads) sorted_ids[i] = numel;
 
   // pass 2: stable scatter
   for (int base = lo; base < hi; base += 32 * kBatch) {
@@ -150,11 +152,12 @@ moe_align_kernel(const int32_t* __restrict__ topk_ids, int numel, int E, int blo
       const int s = base + 32 * i + lane, e = id[i];
       const bool ok = (e >= 0 && e < E);
       const unsigned peers = warp_peers(ok ? e : -1, bits);
+      int pos = -1;
       if (ok) {
-        const int rank = __popc(peers & ((1u << lane) - 1u));
-        const int pos = s_start[e] + s_cnt[warp * E + e] + rank;
+        pos = s_start[e] + s_cnt[warp * E + e] + __popc(peers & ((1u << lane) - 1u));
         if (pos < sorted_cap) sorted_ids[pos] = s;
       }
+      if (slot_pos && s < hi) slot_pos[s] = pos;
       __syncwarp();
       if (ok && (__ffs(peers) - 1) == lane) s_cnt[warp * E + e] += __popc(peers);
       __syncwarp();
@@ -175,13 +178,13 @@ constexpr int kSingleCtaSlots = 4 * kChunk;
 
 __global__ void __launch_bounds__(kThreads)
 align_count_kernel(const int32_t* __restrict__ topk_ids, int numel, int E, int32_t* __restrict__ sorted_ids,
-                   int sorted_cap, int32_t* __restrict__ cnt) {
+                   int sorted_cap, int32_t* __restrict__ cnt, int rows_only) {
   pdl_entry();
   extern __shared__ int s_mem[];  // [E]
   const int tid = threadIdx.x;
   for (int e = tid; e < E; e += kThreads) s_mem[e] = 0;
-  for (int64_t i = (int64_t)blockIdx.x * kThreads + tid; i < sorted_cap; i += (int64_t)gridDim.x * kThreads)
-    sorted_ids[i] = numel;
+  if (!rows_only)
+    for (int64_t i = (int64_t)blockIdx.x * kThreads + tid; i < sorted_cap; i += (int64_t)gridDim.x * kThreads) sorted_ids[i] = numel;
   __syncthreads();
   const int lo = blockIdx.x * kChunk, hi = min(lo + kChunk, numel);
   int id[kChunk / kThreads];
@@ -201,7 +204,7 @@ __global__ void __launch_bounds__(kThreads)
 align_scan_kernel(int chunks, int E, int block, int32_t* __restrict__ cnt, int32_t* __restrict__ starts,
                   int32_t* __restrict__ expert_ids,
                   int expert_cap, int32_t* __restrict__ num_post_pad, int32_t* __restrict__ table, int token_tile,
-                  int32_t* __restrict__ zero_words, int num_zero) {
+                  int32_t* __restrict__ zero_words, int num_zero, int rows_only) {
   pdl_entry();
   extern __shared__ int s_mem[];
   int* s_total = s_mem;      // [E]
@@ -226,17 +229,19 @@ align_scan_kernel(int chunks, int E, int block, int32_t* __restrict__ cnt, int32
   if (warp == 0) scan_experts_warp(s_total, s_start, E, block, lane, num_post_pad, table, token_tile);
   __syncthreads();
   const int used_blocks = s_start[E] / block;
+  for (int e = tid; e < E; e += kThreads) starts[e] = s_start[e];  // first position of the expert, for the scatter
+  if (rows_only) return;
   for (int e = tid; e < E; e += kThreads) {
     int b0 = s_start[e] / block, b1 = s_start[e + 1] / block;
     for (int b = b0; b < b1 && b < expert_cap; ++b) expert_ids[b] = e;
-    starts[e] = s_start[e];  // first position of the expert, for the scatter
   }
   for (int b = used_blocks + tid; b < expert_cap; b += kThreads) expert_ids[b] = -1;
 }
 
 __global__ void __launch_bounds__(kThreads)
 align_scatter_kernel(const int32_t* __restrict__ topk_ids, int numel, int E, const int32_t* __restrict__ cnt,
-                     const int32_t* __restrict__ starts, int32_t* __restrict__ sorted_ids, int sorted_cap) {
+                     const int32_t* __restrict__ starts, int32_t* __restrict__ sorted_ids, int sorted_cap,
+                     int32_t* __restrict__ slot_pos) {
   pdl_entry();
   extern __shared__ int s_mem[];  // [kWarps][E] per-warp counts -> running positions
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, bits = id_bits(E);
@@ -271,10 +276,13 @@ align_scatter_kernel(const int32_t* __restrict__ topk_ids, int numel, int E, con
   __syncthreads();
 #pragma unroll
   for (int i = 0; i < per_warp / 32; ++i) {
+    const int s = lo + 32 * i + lane;
+    int pos = -1;
     if (id[i] >= 0) {
-      const int pos = s_mem[warp * E + id[i]] + __popc(peers[i] & ((1u << lane) - 1u));
-      if (pos < sorted_cap) sorted_ids[pos] = lo + 32 * i + lane;
+      pos = s_mem[warp * E + id[i]] + __popc(peers[i] & ((1u << lane) - 1u));
+      if (pos < sorted_cap) sorted_ids[pos] = s;
     }
+    if (slot_pos && s < hi) slot_pos[s] = pos;
     __syncwarp();
     if (id[i] >= 0 && (__ffs(peers[i]) - 1) == lane) s_mem[warp * E + id[i]] += __popc(peers[i]);
     __syncwarp();
@@ -292,7 +300,8 @@ __global__ void __launch_bounds__(kSortedThreads)
 align_sorted_kernel(const int32_t* __restrict__ slot_of, const int32_t* __restrict__ hist, const float* __restrict__ gate, int numel,
                     int E, int block, int32_t* __restrict__ sorted_ids, int sorted_cap, int32_t* __restrict__ expert_ids,
                     int expert_cap, int32_t* __restrict__ num_post_pad, int32_t* __restrict__ table, int token_tile,
-                    int32_t* __restrict__ zero_words, int num_zero, int32_t* __restrict__ ids, float* __restrict__ weights) {
+                    int32_t* __restrict__ zero_words, int num_zero, int32_t* __restrict__ ids, float* __restrict__ weights,
+                    int32_t* __restrict__ slot_pos, int rows_only) {
   pdl_entry();
   extern __shared__ int s_mem[];
   int* s_total = s_mem;            // [E]
@@ -327,6 +336,7 @@ align_sorted_kernel(const int32_t* __restrict__ slot_of, const int32_t* __restri
     if (p >= s_first[E]) {  // a histogram that does not cover every position: the rest belongs to no expert
       ids[slot] = -1;
       weights[slot] = 0.f;
+      if (slot_pos) slot_pos[slot] = -1;
       continue;
     }
     int lo = 0, hi = E - 1;  // last expert that starts at or before p
@@ -337,17 +347,18 @@ align_sorted_kernel(const int32_t* __restrict__ slot_of, const int32_t* __restri
     }
     const int pos = s_start[lo] + p - s_first[lo];
     if (pos < sorted_cap && sorted_ids) sorted_ids[pos] = slot;
+    if (slot_pos) slot_pos[slot] = pos;
     ids[slot] = lo;
     weights[slot] = gate[p];
   }
-  if (!sorted_ids) return;  // only experts and weights by slot were asked for
+  for (int i = block_id * kSortedThreads + tid; i < num_zero; i += stride) zero_words[i] = 0;
+  if (!sorted_ids || rows_only) return;
   for (int e = block_id * (kSortedThreads / 32) + warp; e < E; e += gridDim.x * (kSortedThreads / 32)) {
     for (int i = s_start[e] + s_total[e] + lane; i < min(s_start[e + 1], sorted_cap); i += 32) sorted_ids[i] = numel;
     for (int b = s_start[e] / block + lane; b < s_start[e + 1] / block && b < expert_cap; b += 32) expert_ids[b] = e;
   }
   for (int i = s_start[E] + block_id * kSortedThreads + tid; i < sorted_cap; i += stride) sorted_ids[i] = numel;
   for (int b = s_start[E] / block + block_id * kSortedThreads + tid; b < expert_cap; b += stride) expert_ids[b] = -1;
-  for (int i = block_id * kSortedThreads + tid; i < num_zero; i += stride) zero_words[i] = 0;
 }
 
 }  // namespace
@@ -379,7 +390,8 @@ int run_align(const AlignArgs& a, cudaStream_t st) {
     if (smem > 48 * 1024)
       FMOE_CUDA_OK(cudaFuncSetAttribute(moe_align_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
     launch_pdl(moe_align_kernel, dim3(1), dim3(kThreads), smem, st, a.topk_ids, (int)a.numel, a.E, a.block, a.sorted_ids,
-               (int)a.sorted_cap, a.expert_ids, (int)a.expert_cap, a.num_post_pad, a.table, a.token_tile, a.zero_words, a.num_zero);
+               (int)a.sorted_cap, a.expert_ids, (int)a.expert_cap, a.num_post_pad, a.table, a.token_tile, a.zero_words, a.num_zero,
+               a.slot_pos, (int)a.rows_only);
     return launch_status("moe_align_kernel");
   }
   FMOE_REQUIRE(a.workspace_bytes >= fmoe_moe_align_workspace_bytes(a.numel, a.E), "moe_align_block_size: workspace too small");
@@ -387,18 +399,18 @@ int run_align(const AlignArgs& a, cudaStream_t st) {
   int32_t* cnt = static_cast<int32_t*>(a.workspace);
   int32_t* starts = cnt + (int64_t)chunks * a.E;
   launch_pdl(align_count_kernel, dim3(chunks), dim3(kThreads), a.E * sizeof(int), st, a.topk_ids, (int)a.numel, a.E, a.sorted_ids,
-             (int)a.sorted_cap, cnt);
+             (int)a.sorted_cap, cnt, (int)a.rows_only);
   rc = launch_status("align_count_kernel");
   if (rc) return rc;
   launch_pdl(align_scan_kernel, dim3(1), dim3(kThreads), (2 * a.E + 1) * sizeof(int), st, chunks, a.E, a.block, cnt, starts,
-             a.expert_ids, (int)a.expert_cap, a.num_post_pad, a.table, a.token_tile, a.zero_words, a.num_zero);
+             a.expert_ids, (int)a.expert_cap, a.num_post_pad, a.table, a.token_tile, a.zero_words, a.num_zero, (int)a.rows_only);
   rc = launch_status("align_scan_kernel");
   if (rc) return rc;
   const size_t smem = (size_t)kWarps * a.E * sizeof(int);
   if (smem > 48 * 1024)
     FMOE_CUDA_OK(cudaFuncSetAttribute(align_scatter_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
   launch_pdl(align_scatter_kernel, dim3(chunks), dim3(kThreads), smem, st, a.topk_ids, (int)a.numel, a.E,
-             (const int32_t*)cnt, (const int32_t*)starts, a.sorted_ids, (int)a.sorted_cap);
+             (const int32_t*)cnt, (const int32_t*)starts, a.sorted_ids, (int)a.sorted_cap, a.slot_pos);
   return launch_status("align_scatter_kernel");
 }
 
@@ -409,10 +421,10 @@ int run_align_sorted(const AlignArgs& a, const SortedSlots& s, cudaStream_t st) 
     const int rc = check_align(a);
     if (rc) return rc;
   }
-  const unsigned grid = (unsigned)std::min<int64_t>(ceil_div<int64_t>(std::max(a.numel, a.sorted_ids ? a.sorted_cap / 4 : 0), kSortedThreads), 148);
+  const unsigned grid = (unsigned)std::min<int64_t>(ceil_div<int64_t>(std::max(a.numel, a.sorted_ids && !a.rows_only ? a.sorted_cap / 4 : 0), kSortedThreads), 148);
   launch_pdl(align_sorted_kernel, dim3(grid), dim3(kSortedThreads), (3 * (size_t)a.E + 2) * sizeof(int), st, s.slot_of, s.hist, s.gate,
              (int)a.numel, a.E, a.block, a.sorted_ids, (int)a.sorted_cap, a.expert_ids, (int)a.expert_cap, a.num_post_pad, a.table,
-             a.token_tile, a.zero_words, a.num_zero, s.ids, s.weights);
+             a.token_tile, a.zero_words, a.num_zero, s.ids, s.weights, a.slot_pos, (int)a.rows_only);
   return launch_status("align_sorted_kernel");
 }
 

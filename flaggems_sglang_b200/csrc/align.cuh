@@ -19,6 +19,8 @@ struct AlignArgs {
   int token_tile = 256;           //   at most this many tokens
   int32_t* zero_words = nullptr;  // optional: counters of later kernels, set to zero
   int num_zero = 0;
+  int32_t* slot_pos = nullptr;    // optional: [numel] position of every slot in the sorted order, -1 for dropped ids
+  bool rows_only = false;         // padding positions and expert_ids are not read by anyone: they stay unwritten
   bool from_sorted = false;       // topk_ids is not read (run_align_sorted)
 };
 int run_align(const AlignArgs& a, cudaStream_t st);

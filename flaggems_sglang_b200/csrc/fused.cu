@@ -146,16 +146,13 @@ int plan_fused(const fmoe_fused_args& a, const RouteArgs& route, FusedPlan* pl) 
   // align kernel clears: both GEMMs of a call have their own, so no memset stands between the kernels
   p.off_table = tc ? take(pair_table_bytes(a.num_experts)) : -1;
   p.off_counters = tc ? take(2 * kSplitCounters * 4) : -1;
-  p.off_xs = p.off_xs_scale = p.off_xt = p.off_xt_scale = p.off_actq = p.off_actq_scale = p.off_split = -1;
+  p.off_slot_pos = tc ? take(p.numel * 4) : -1;
+  p.off_xs = p.off_xs_scale = p.off_actq = p.off_actq_scale = p.off_split = -1;
   p.split_bytes = 0;
   if (channel) {
-    // every sorted row is quantised with its own scale; the activation likewise
+    // token rows quantised straight into the sorted order, one scale per token; every row of the activation with its own
     p.off_xs = take(p.cap * a.H);
-    p.off_xs_scale = take(p.cap * 4);
-    if (a.top_k >= 2 && a.H % 16 == 0) {  // each token row quantised once, its bytes copied into the sorted order
-      p.off_xt = take(a.T * a.H);
-      p.off_xt_scale = take(a.T * 4);
-    }
+    p.off_xs_scale = take(a.T * 4);
     p.act_elem = 2;
     p.off_act = take(p.cap * a.I * 2);
     p.off_actq = take(p.cap * a.I);
@@ -163,13 +160,8 @@ int plan_fused(const fmoe_fused_args& a, const RouteArgs& route, FusedPlan* pl) 
     p.split_bytes = fmoe_gemm_split_workspace_bytes();
     p.off_split = take(p.split_bytes);
   } else if (fp8) {
-    const int64_t xrows = tc ? p.cap : a.T;
-    p.off_xs = take(xrows * a.H);
-    p.off_xs_scale = take(xrows * (a.H / 128) * 4);
-    if (tc && fp8_quant_once(a.top_k, a.H)) {
-      p.off_xt = take(a.T * a.H);
-      p.off_xt_scale = take(a.T * (a.H / 128) * 4);
-    }
+    p.off_xs = take((tc ? p.cap : a.T) * a.H);
+    p.off_xs_scale = take(a.T * (a.H / 128) * 4);
     // the wide tensor-core kernel quantises its 128-channel groups itself; the others write fp32 for the quantiser
     const bool wide = tc && pick_fold_token_tile(p.numel, a.num_experts) == 256;
     p.act_elem = wide ? 1 : 4;
@@ -296,6 +288,9 @@ int run_fused(const fmoe_fused_args& args, const RouteArgs& route, const FusedPl
   al.token_tile = fold ? pick_fold_token_tile(p.numel, a.num_experts) : pick_token_tile(p.numel, a.num_experts);
   al.zero_words = counters;
   al.num_zero = counters ? 2 * kSplitCounters : 0;
+  int32_t* slot_pos = tc ? reinterpret_cast<int32_t*>(ws + p.off_slot_pos) : nullptr;
+  al.slot_pos = slot_pos;
+  al.rows_only = tc && (fp8 || p.off_xs >= 0);  // the GEMMs go by the table, the row passes by slot_pos
   al.from_sorted = route.slot_of != nullptr;
   int rc = route.slot_of ? run_align_sorted(al, slots, st) : run_align(al, st);
   if (rc) return rc;
@@ -350,7 +345,7 @@ int run_fused(const fmoe_fused_args& args, const RouteArgs& route, const FusedPl
     g1.dtype = g1.out_dtype = g2.dtype = a.dtype;
     if (tc && p.off_xs >= 0) {
       void* xs = ws + p.off_xs;
-      rc = run_gather_rows(a.hidden, (int)eb, p.cap, a.H, sorted, a.top_k, p.numel, npp, xs, false, st);
+      rc = run_scatter_rows(a.hidden, (int)eb, a.T, a.top_k, a.H, slot_pos, xs, st);
       if (rc) return rc;
       g1.a = xs;
       g1.a_rows = p.cap;
@@ -366,28 +361,12 @@ int run_fused(const fmoe_fused_args& args, const RouteArgs& route, const FusedPl
     float* xsc = reinterpret_cast<float*>(ws + p.off_xs_scale);
     const bool channel = a.scale_mode == FMOE_SCALE_CHANNEL;
     g1.scale_mode = g2.scale_mode = a.scale_mode;
-    if (channel && p.off_xt >= 0) {
-      void* xt = ws + p.off_xt;
-      float* xtsc = reinterpret_cast<float*>(ws + p.off_xt_scale);
-      rc = fmoe_quant_fp8_per_token(a.hidden, FMOE_BF16, a.T, a.H, nullptr, 1, 0, nullptr, xt, xtsc, stream);
-      if (rc) return rc;
-      rc = run_gather_rows(xt, 1, p.cap, a.H, sorted, a.top_k, p.numel, npp, xq, false, st);
-      xsc = xtsc;  // the gate/up GEMM looks the scale up by token
-      g1.a_scale_gather = 1;
-    } else if (channel) {
-      rc = run_quant_per_token(a.hidden, FMOE_BF16, p.cap, a.H, sorted, a.top_k, p.numel, npp, xq, xsc, false, st);
-    } else if (tc && p.off_xt >= 0) {
-      void* xt = ws + p.off_xt;
-      float* xtsc = reinterpret_cast<float*>(ws + p.off_xt_scale);
-      rc = fmoe_quant_fp8_group128(a.hidden, FMOE_BF16, a.T, a.H, nullptr, 1, 0, nullptr, xt, xtsc, stream);
-      if (rc) return rc;
-      rc = run_gather_rows(xt, 1, p.cap, a.H, sorted, a.top_k, p.numel, npp, xq, false, st);
-      xsc = xtsc;  // the gate/up GEMM looks the scales up by token
-      g1.a_scale_gather = 1;
-    } else if (tc)
-      rc = run_quant_group128(a.hidden, FMOE_BF16, p.cap, a.H, sorted, a.top_k, p.numel, npp, xq, xsc, false, st);
-    else
+    if (tc) {
+      rc = run_quant_scatter(a.hidden, a.T, a.top_k, a.H, slot_pos, channel, xq, xsc, st);
+      g1.a_scale_gather = 1;  // the gate/up GEMM looks the scales up by token
+    } else {
       rc = fmoe_quant_fp8_group128(a.hidden, FMOE_BF16, a.T, a.H, nullptr, 1, 0, nullptr, xq, xsc, stream);
+    }
     if (rc) return rc;
     g1.dtype = g2.dtype = FMOE_E4M3;
     g1.out_dtype = channel ? FMOE_BF16 : (p.act_elem == 1 ? FMOE_E4M3 : FMOE_F32);
@@ -410,10 +389,8 @@ int run_fused(const fmoe_fused_args& args, const RouteArgs& route, const FusedPl
   mark(3);
   if (fp8 && act) {
     float* scale = reinterpret_cast<float*>(ws + p.off_actq_scale);
-    if (a.scale_mode == FMOE_SCALE_CHANNEL)
-      rc = run_quant_per_token(act, FMOE_BF16, p.cap, a.I, sorted, 0, p.numel, npp, ws + p.off_actq, scale, false, st);
-    else
-      rc = run_quant_group128(act, FMOE_F32, p.cap, a.I, sorted, 0, p.numel, npp, ws + p.off_actq, scale, !tc, st);
+    rc = tc ? run_quant_slots(act, g1.out_dtype, p.numel, a.I, slot_pos, a.scale_mode == FMOE_SCALE_CHANNEL, ws + p.off_actq, scale, st)
+            : fmoe_quant_fp8_group128(act, FMOE_F32, p.cap, a.I, sorted, 0, p.numel, npp, ws + p.off_actq, scale, stream);
     if (rc) return rc;
   }
   mark(4);

@@ -9,18 +9,14 @@ struct FusedPlan {
   int variant, block, act_elem;
   int64_t numel, cap, nblk, max_blocks, total;
   // byte offsets into the workspace (-1: not used)
-  int64_t off_sorted, off_expert, off_npp, off_align_ws, align_ws_bytes, off_xs, off_xs_scale, off_xt, off_xt_scale, off_act, off_actq, off_actq_scale, off_z;
+  int64_t off_sorted, off_expert, off_npp, off_align_ws, align_ws_bytes, off_xs, off_xs_scale, off_act, off_actq, off_actq_scale, off_z;
   int64_t off_split, split_bytes;  // tail-split scratch of the tcgen05 GEMMs
   bool use_decode;                  // the two decode kernels take the call (decode.cu); the fields above are then unused
   DecodePlan decode;
   int64_t off_route_ids, off_route_weights;  // calls from logits: where the router's results go (-1: not used)
   int64_t off_table, off_counters;  // expert table and tail-split counters of the CTA-pair GEMMs
+  int64_t off_slot_pos;             // position of every slot in the sorted order
 };
-
-// e4m3 with the tcgen05 kernels: quantise each token row once ([T,H]) and copy the bytes into the sorted order, instead
-// of quantising every one of the T*top_k sorted rows (the quantiser is division-bound, the copy is not); the GEMM finds
-// the scales by token.
-inline bool fp8_quant_once(int64_t top_k, int64_t) { return top_k >= 2; }
 
 int pick_variant(int dtype, int64_t numel, int E, int64_t I, int64_t H, int forced, int* variant, int* block);
 int plan_fused(const fmoe_fused_args& a, const RouteArgs& route, FusedPlan* plan);

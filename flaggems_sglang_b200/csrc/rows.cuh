@@ -4,17 +4,16 @@
 
 namespace fmoe {
 
-// fmoe_gather_rows; without zero_padding the padding positions stay unwritten
-int run_gather_rows(const void* x, int elem_bytes, int64_t rows_out, int64_t K, const int32_t* row_map, int map_div,
-                    int64_t map_sentinel, const int32_t* num_rows_dev, void* out, bool zero_padding, cudaStream_t st);
-
-// fmoe_quant_fp8_group128 / fmoe_quant_fp8_per_token, likewise
-int run_quant_group128(const void* x, int in_dtype, int64_t rows_out, int64_t K, const int32_t* row_map, int map_div,
-                       int64_t map_sentinel, const int32_t* num_rows_dev, void* q, float* scale, bool zero_padding,
-                       cudaStream_t st);
-int run_quant_per_token(const void* x, int in_dtype, int64_t rows_out, int64_t K, const int32_t* row_map, int map_div,
-                        int64_t map_sentinel, const int32_t* num_rows_dev, void* q, float* scale, bool zero_padding,
-                        cudaStream_t st);
+// The layer's passes, by slot: slot_pos [T * k] is every slot's position in the sorted order (-1: none), as run_align
+// writes it; padding positions are neither read nor written.
+// token rows -> the positions of their k slots
+int run_scatter_rows(const void* x, int elem_bytes, int64_t T, int k, int64_t K, const int32_t* slot_pos, void* out, cudaStream_t st);
+// bf16 token rows -> e4m3 at the positions of their k slots; scales by token: [T, K/128], or [T] with per_row
+int run_quant_scatter(const void* x, int64_t T, int k, int64_t K, const int32_t* slot_pos, bool per_row, void* q, float* scale,
+                      cudaStream_t st);
+// sorted rows (f32; bf16 with per_row) -> e4m3 in the same positions, scales by position
+int run_quant_slots(const void* x, int in_dtype, int64_t numel, int64_t K, const int32_t* slot_pos, bool per_row, void* q,
+                    float* scale, cudaStream_t st);
 
 #if defined(__CUDACC__)
 // Scale of a group of 128 channels with this largest magnitude.
