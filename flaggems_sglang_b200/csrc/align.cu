@@ -1,11 +1,9 @@
-// moe_align_block_size: histogram -> scan -> stable scatter, one CTA.
+// moe_align_block_size: histogram -> scan -> stable scatter.
 //
-// The slots [0, numel) are split into one contiguous chunk per warp.  Each warp
-// counts its chunk per expert, a scan over (expert, warp) turns the counts into
-// the first output position of every (warp, expert) pair, and a second pass over
-// the chunk places each slot at base + (its rank among the equal ids seen so
-// far), which keeps slots of an expert in ascending order.  The ranks inside
-// a group of 32 slots come from warp ballots.
+// Up to kOneLaunchSlots slots (and for any number without scratch) one launch does all of it: CTA b owns slots
+// [1024 b, 1024 (b + 1)), one per thread, and counts ALL slots per expert, those before its own apart, so that no CTA waits
+// for another.  Slots of an expert keep their ascending order: position = expert's start + slots before this CTA + slots in
+// earlier warps + rank among the warp's equal ids (ballots).  Above that, three launches share the counting.
 #include "align.cuh"
 
 namespace fmoe {
@@ -13,7 +11,6 @@ namespace {
 
 constexpr int kThreads = 1024;
 constexpr int kWarps = kThreads / 32;
-constexpr int kBatch = 4;
 
 // Lanes of the warp whose id equals this lane's (ids below 2^bits; lanes without an id pass -1 and get the other such
 // lanes).  One ballot per id bit: __match_any_sync took most of the 21 us of a single-CTA sort of 8192 slots.
@@ -33,13 +30,15 @@ __host__ __device__ inline int id_bits(int E) {
   return b;
 }
 
-// One warp: exclusive scan of the padded row counts -> s_start[E + 1] and num_post_pad; with `table`, also the experts'
-// first rows, rows and token tiles for the CTA-pair GEMMs (pair.cuh).  E <= 1024: 32 experts per step.
-__device__ __forceinline__ void scan_experts_warp(const int* s_total, int* s_start, int E, int block, int lane,
-                                                  int32_t* num_post_pad, int32_t* table, int token_tile) {
+// All NW warps of the CTA: exclusive scan of the padded row counts -> s_start[E + 1] and num_post_pad; with `table`, also the
+// experts' first rows, rows and token tiles for the CTA-pair GEMMs (pair.cuh).  s_sum: [2 * NW].
+template <int NW>
+__device__ __forceinline__ void scan_experts(const int* s_total, int* s_start, int E, int block, int32_t* num_post_pad,
+                                             int32_t* table, int token_tile, int* s_sum) {
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   int carry = 0, tile_carry = 0;
-  for (int base = 0; base < E; base += 32) {
-    const int e = base + lane;
+  for (int base = 0; base < E; base += NW * 32) {
+    const int e = base + tid;
     const int rows = (e < E) ? s_total[e] : 0;
     const int padded = ceil_div(rows, block) * block, tiles = ceil_div(rows, token_tile);
     int incl = padded, tile_incl = tiles;
@@ -51,22 +50,51 @@ __device__ __forceinline__ void scan_experts_warp(const int* s_total, int* s_sta
         tile_incl += w;
       }
     }
+    if (lane == 31) {
+      s_sum[warp] = incl;
+      s_sum[NW + warp] = tile_incl;
+    }
+    __syncthreads();
+    const int warps = min(NW, (E - base + 31) >> 5);  // the others' sums are zero
+    int before = carry, tile_before = tile_carry;
+    for (int w = 0; w < warps; ++w) {
+      const int v = s_sum[w], u = s_sum[NW + w];
+      if (w < warp) {
+        before += v;
+        tile_before += u;
+      }
+      carry += v;
+      tile_carry += u;
+    }
     if (e < E) {
-      s_start[e] = carry + incl - padded;
+      s_start[e] = before + incl - padded;
       if (table) {
-        table[e] = carry + incl - padded;
+        table[e] = before + incl - padded;
         table[E + e] = rows;
-        table[2 * E + e] = tile_carry + tile_incl - tiles;
+        table[2 * E + e] = tile_before + tile_incl - tiles;
       }
     }
-    carry += __shfl_sync(0xffffffffu, incl, 31);
-    tile_carry += __shfl_sync(0xffffffffu, tile_incl, 31);
+    __syncthreads();  // s_sum is free again, s_start is complete
   }
-  if (lane == 0) {
+  if (tid == 0) {
     s_start[E] = carry;
-    num_post_pad[0] = carry;
+    if (num_post_pad) num_post_pad[0] = carry;
     if (table) table[3 * E] = tile_carry;
   }
+  __syncthreads();
+}
+
+// What the block list holds besides the slots, shared out over the grid: block -> expert (-1 after the used blocks), and the
+// sentinel in the padding of every expert and after the used blocks.
+__device__ __forceinline__ void fill_padding(const int* s_total, const int* s_start, int E, int block, int numel,
+                                             int32_t* sorted_ids, int sorted_cap, int32_t* expert_ids, int expert_cap) {
+  const int lane = threadIdx.x & 31, warps = blockDim.x >> 5, at = blockIdx.x * blockDim.x + threadIdx.x, stride = gridDim.x * blockDim.x;
+  for (int e = blockIdx.x * warps + (threadIdx.x >> 5); e < E; e += gridDim.x * warps) {
+    for (int i = s_start[e] + s_total[e] + lane; i < min(s_start[e + 1], sorted_cap); i += 32) sorted_ids[i] = numel;
+    for (int b = s_start[e] / block + lane; b < s_start[e + 1] / block && b < expert_cap; b += 32) expert_ids[b] = e;
+  }
+  for (int i = s_start[E] + at; i < sorted_cap; i += stride) sorted_ids[i] = numel;
+  for (int b = s_start[E] / block + at; b < expert_cap; b += stride) expert_ids[b] = -1;
 }
 
 __global__ void __launch_bounds__(kThreads)
@@ -76,93 +104,54 @@ moe_align_kernel(const int32_t* __restrict__ topk_ids, int numel, int E, int blo
                  int32_t* __restrict__ zero_words, int num_zero, int32_t* __restrict__ slot_pos, int rows_only) {
   pdl_entry();
   extern __shared__ int s_mem[];
-  int* s_cnt = s_mem;                  // [kWarps][E] counts, then running output positions
-  int* s_total = s_mem + kWarps * E;   // [E] per-expert count
-  int* s_start = s_total + E;          // [E+1] padded start of each expert
-  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, bits = id_bits(E);
+  int* s_cnt = s_mem;                 // [kWarps][E] slots of this CTA's warps, then of the warps before
+  int* s_before = s_mem + kWarps * E; // [E] slots of earlier CTAs
+  int* s_total = s_before + E;        // [E]
+  int* s_start = s_total + E;         // [E+1] padded start of each expert
+  __shared__ int s_sum[2 * kWarps];
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, bits = id_bits(E), first = blockIdx.x == 0;
 
-  for (int i = tid; i < kWarps * E; i += kThreads) s_cnt[i] = 0;
-  for (int i = tid; i < num_zero; i += kThreads) zero_words[i] = 0;
+  for (int i = tid; i < (kWarps + 2) * E; i += kThreads) s_mem[i] = 0;
+  const int lo = blockIdx.x * kThreads, slot = lo + tid;
+  int id = slot < numel ? topk_ids[slot] : -1;
+  if (id < 0 || id >= E) id = -1;
+  const unsigned peers = warp_peers(id, bits);
+  const bool leader = id >= 0 && (__ffs(peers) - 1) == lane;
   __syncthreads();
-
-  const int chunk = ceil_div(ceil_div(numel, kWarps), 32) * 32;  // multiple of 32 per warp
-  const int lo = min(warp * chunk, numel), hi = min(lo + chunk, numel);
-
-  // pass 1: per-warp histogram (kBatch ids per lane loaded before the first is counted)
-  for (int base = lo; base < hi; base += 32 * kBatch) {
-    int id[kBatch];
+  if (leader) s_cnt[warp * E + id] = __popc(peers);
+  constexpr int kBatch = 8;
+  for (int base = tid; base < numel; base += kBatch * kThreads) {
+    int v[kBatch];
 #pragma unroll
-    for (int i = 0; i < kBatch; ++i) {
-      const int s = base + 32 * i + lane;
-      id[i] = (s < hi) ? topk_ids[s] : -1;
-    }
+    for (int i = 0; i < kBatch; ++i) v[i] = base + i * kThreads < numel ? topk_ids[base + i * kThreads] : -1;
 #pragma unroll
-    for (int i = 0; i < kBatch; ++i) {
-      if (base + 32 * i >= hi) break;
-      const int e = id[i];
-      const bool ok = (e >= 0 && e < E);
-      const unsigned peers = warp_peers(ok ? e : -1, bits);
-      if (ok && (__ffs(peers) - 1) == lane) s_cnt[warp * E + e] += __popc(peers);
-      __syncwarp();
-    }
+    for (int i = 0; i < kBatch; ++i)
+      if (v[i] >= 0 && v[i] < E) atomicAdd(base + i * kThreads < lo ? &s_before[v[i]] : &s_total[v[i]], 1);
   }
   __syncthreads();
-
-  // scan over warps for each expert: s_cnt[w][e] <- number of slots of e in warps < w
   for (int e = tid; e < E; e += kThreads) {
-    int run = 0;
+    int run = s_before[e];
+    s_total[e] += run;
 #pragma unroll 8
     for (int w = 0; w < kWarps; ++w) {
-      int c = s_cnt[w * E + e];
+      const int c = s_cnt[w * E + e];
       s_cnt[w * E + e] = run;
       run += c;
     }
-    s_total[e] = run;
   }
   __syncthreads();
+  scan_experts<kWarps>(s_total, s_start, E, block, first ? num_post_pad : nullptr, first ? table : nullptr, token_tile, s_sum);
 
-  if (warp == 0) scan_experts_warp(s_total, s_start, E, block, lane, num_post_pad, table, token_tile);
-  __syncthreads();
-
-  if (!rows_only) {
-    // block -> expert map (-1 after the used blocks)
-    const int used_blocks = s_start[E] / block;
-    for (int e = tid; e < E; e += kThreads) {
-      int b0 = s_start[e] / block, b1 = s_start[e + 1] / block;
-      for (int b = b0; b < b1 && b < expert_cap; ++b) expert_ids[b] = e;
+  if (slot < numel) {
+    int pos = -1;
+    if (id >= 0) {
+      pos = s_start[id] + s_cnt[warp * E + id] + __popc(peers & ((1u << lane) - 1u));
+      if (pos < sorted_cap) sorted_ids[pos] = slot;
     }
-    for (int b = used_blocks + tid; b < expert_cap; b += kThreads) expert_ids[b] = -1;
-    // sentinels: the padding of every expert, and everything past the used blocks
-    for (int e = warp; e < E; e += kWarps)
-      for (int i = s_start[e] + s_total[e] + lane; i < s_start[e + 1]; i += 32) sorted_ids[i] = numel;
-    for (int i = s_start[E] + tid; i < sorted_cap; i += kThreads) sorted_ids[i] = numel;
+    if (slot_pos) slot_pos[slot] = pos;
   }
-
-  // pass 2: stable scatter
-  for (int base = lo; base < hi; base += 32 * kBatch) {
-    int id[kBatch];
-#pragma unroll
-    for (int i = 0; i < kBatch; ++i) {
-      const int s = base + 32 * i + lane;
-      id[i] = (s < hi) ? topk_ids[s] : -1;
-    }
-#pragma unroll
-    for (int i = 0; i < kBatch; ++i) {
-      if (base + 32 * i >= hi) break;
-      const int s = base + 32 * i + lane, e = id[i];
-      const bool ok = (e >= 0 && e < E);
-      const unsigned peers = warp_peers(ok ? e : -1, bits);
-      int pos = -1;
-      if (ok) {
-        pos = s_start[e] + s_cnt[warp * E + e] + __popc(peers & ((1u << lane) - 1u));
-        if (pos < sorted_cap) sorted_ids[pos] = s;
-      }
-      if (slot_pos && s < hi) slot_pos[s] = pos;
-      __syncwarp();
-      if (ok && (__ffs(peers) - 1) == lane) s_cnt[warp * E + e] += __popc(peers);
-      __syncwarp();
-    }
-  }
+  for (int i = slot; i < num_zero; i += gridDim.x * kThreads) zero_words[i] = 0;
+  if (!rows_only) fill_padding(s_total, s_start, E, block, numel, sorted_ids, sorted_cap, expert_ids, expert_cap);
 }
 
 // ---------------------------------------------------------------------------------------------
@@ -173,8 +162,8 @@ moe_align_kernel(const int32_t* __restrict__ topk_ids, int numel, int E, int blo
 // cnt and the experts' starts live in caller scratch ((chunks + 1) * E ints).
 // ---------------------------------------------------------------------------------------------
 constexpr int kChunk = 4096;
-// Up to here one CTA is faster than three dependent launches.
-constexpr int kSingleCtaSlots = 4 * kChunk;
+// Up to here every CTA counting all slots is faster than three dependent launches (8192 slots, 64 experts: one CTA 14.4 us).
+constexpr int kOneLaunchSlots = 4 * kChunk;
 
 __global__ void __launch_bounds__(kThreads)
 align_count_kernel(const int32_t* __restrict__ topk_ids, int numel, int E, int32_t* __restrict__ sorted_ids,
@@ -209,7 +198,8 @@ align_scan_kernel(int chunks, int E, int block, int32_t* __restrict__ cnt, int32
   extern __shared__ int s_mem[];
   int* s_total = s_mem;      // [E]
   int* s_start = s_mem + E;  // [E+1]
-  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  __shared__ int s_sum[2 * kWarps];
+  const int tid = threadIdx.x;
   for (int i = tid; i < num_zero; i += kThreads) zero_words[i] = 0;
   for (int e = tid; e < E; e += kThreads) {
     int run = 0;
@@ -226,8 +216,7 @@ align_scan_kernel(int chunks, int E, int block, int32_t* __restrict__ cnt, int32
     s_total[e] = run;
   }
   __syncthreads();
-  if (warp == 0) scan_experts_warp(s_total, s_start, E, block, lane, num_post_pad, table, token_tile);
-  __syncthreads();
+  scan_experts<kWarps>(s_total, s_start, E, block, num_post_pad, table, token_tile, s_sum);
   const int used_blocks = s_start[E] / block;
   for (int e = tid; e < E; e += kThreads) starts[e] = s_start[e];  // first position of the expert, for the scatter
   if (rows_only) return;
@@ -307,12 +296,12 @@ align_sorted_kernel(const int32_t* __restrict__ slot_of, const int32_t* __restri
   int* s_total = s_mem;            // [E]
   int* s_start = s_mem + E;        // [E+1] padded
   int* s_first = s_start + E + 1;  // [E+1] unpadded
-  __shared__ int s_npp;
+  __shared__ int s_sum[2 * kSortedThreads / 32];
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, block_id = blockIdx.x;
   for (int e = tid; e < E; e += kSortedThreads) s_total[e] = max(hist[e], 0);
   __syncthreads();
-  if (warp == 0) scan_experts_warp(s_total, s_start, E, block, lane,
-                                   block_id == 0 && num_post_pad ? num_post_pad : &s_npp, block_id == 0 ? table : nullptr, token_tile);
+  scan_experts<kSortedThreads / 32>(s_total, s_start, E, block, block_id == 0 ? num_post_pad : nullptr,
+                                    block_id == 0 ? table : nullptr, token_tile, s_sum);
   if (warp == 1) {
     int carry = 0;
     for (int base = 0; base < E; base += 32) {
@@ -352,13 +341,7 @@ align_sorted_kernel(const int32_t* __restrict__ slot_of, const int32_t* __restri
     weights[slot] = gate[p];
   }
   for (int i = block_id * kSortedThreads + tid; i < num_zero; i += stride) zero_words[i] = 0;
-  if (!sorted_ids || rows_only) return;
-  for (int e = block_id * (kSortedThreads / 32) + warp; e < E; e += gridDim.x * (kSortedThreads / 32)) {
-    for (int i = s_start[e] + s_total[e] + lane; i < min(s_start[e + 1], sorted_cap); i += 32) sorted_ids[i] = numel;
-    for (int b = s_start[e] / block + lane; b < s_start[e + 1] / block && b < expert_cap; b += 32) expert_ids[b] = e;
-  }
-  for (int i = s_start[E] + block_id * kSortedThreads + tid; i < sorted_cap; i += stride) sorted_ids[i] = numel;
-  for (int b = s_start[E] / block + block_id * kSortedThreads + tid; b < expert_cap; b += stride) expert_ids[b] = -1;
+  if (sorted_ids && !rows_only) fill_padding(s_total, s_start, E, block, numel, sorted_ids, sorted_cap, expert_ids, expert_cap);
 }
 
 }  // namespace
@@ -385,13 +368,16 @@ int check_align(const AlignArgs& a) {
 int run_align(const AlignArgs& a, cudaStream_t st) {
   int rc = check_align(a);
   if (rc) return rc;
-  if (a.numel < kSingleCtaSlots || !a.workspace) {  // small inputs, or no scratch: the single-CTA kernel
-    const size_t smem = ((size_t)kWarps * a.E + 2 * (size_t)a.E + 1) * sizeof(int);
+  if (a.numel <= kOneLaunchSlots || !a.workspace) {
+    const size_t smem = ((size_t)(kWarps + 3) * a.E + 1) * sizeof(int);
     if (smem > 48 * 1024)
       FMOE_CUDA_OK(cudaFuncSetAttribute(moe_align_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    launch_pdl(moe_align_kernel, dim3(1), dim3(kThreads), smem, st, a.topk_ids, (int)a.numel, a.E, a.block, a.sorted_ids,
-               (int)a.sorted_cap, a.expert_ids, (int)a.expert_cap, a.num_post_pad, a.table, a.token_tile, a.zero_words, a.num_zero,
-               a.slot_pos, (int)a.rows_only);
+    // a CTA per 1024 slots; with padding to fill, also one per 8192 positions
+    const int64_t fill = a.rows_only ? 1 : std::min<int64_t>(16, ceil_div<int64_t>(a.sorted_cap, 8 * kThreads));
+    const unsigned grid = (unsigned)std::max<int64_t>(std::max<int64_t>(1, fill), ceil_div<int64_t>(a.numel, kThreads));
+    launch_pdl(moe_align_kernel, dim3(grid), dim3(kThreads), smem, st,
+               a.topk_ids, (int)a.numel, a.E, a.block, a.sorted_ids, (int)a.sorted_cap, a.expert_ids, (int)a.expert_cap,
+               a.num_post_pad, a.table, a.token_tile, a.zero_words, a.num_zero, a.slot_pos, (int)a.rows_only);
     return launch_status("moe_align_kernel");
   }
   FMOE_REQUIRE(a.workspace_bytes >= fmoe_moe_align_workspace_bytes(a.numel, a.E), "moe_align_block_size: workspace too small");

@@ -74,7 +74,8 @@ struct GroupedLauncher {
   static int run(const float* logits, const float* bias, int64_t T, int E, int k, int n_group,
                  int topk_group, int renorm, float scale, float* w, int32_t* ids, cudaStream_t st) {
     size_t smem = (size_t)kWarpsPerBlock * 2 * E * sizeof(float);
-    if (T <= 64) {  // decode-sized: a CTA per token shortens the chain of fp64 sigmoids (13.3 -> 8.7-9.9 us at T = 1, E = 256)
+    if (T <= 592) {  // up to four CTAs per SM: a CTA per token shortens the chain of fp64 sigmoids
+                     // (E = 256: 13.3 -> 8.3 us at 1 token, 12.6 -> 8.4 us at 128 and 512)
       launch_pdl(topk_grouped_kernel<VPT, true>, dim3((unsigned)T), dim3(kWarpsPerBlock * 32), smem, st, logits, bias, T, E,
                  k, n_group, topk_group, renorm, scale, w, ids);
       return launch_status("topk_grouped_kernel");

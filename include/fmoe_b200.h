@@ -105,8 +105,8 @@ int fmoe_moe_align_block_size(const int32_t* topk_ids, int64_t numel, int E, int
                               int32_t* num_tokens_post_padded, void* stream);
 
 /*
- * Same result with caller scratch: inputs of 16384 slots or more are processed by one CTA per 4096 slots
- * (three launches) instead of a single CTA.  workspace needs fmoe_moe_align_workspace_bytes(numel, E) bytes;
+ * Same result with caller scratch: inputs of more than 16384 slots are processed in three launches that share the
+ * counting instead of one launch whose CTAs each count every slot.  workspace needs fmoe_moe_align_workspace_bytes(numel, E) bytes;
  * with workspace == NULL or a small input this is fmoe_moe_align_block_size.
  */
 int64_t fmoe_moe_align_workspace_bytes(int64_t numel, int E);
