@@ -285,7 +285,7 @@ int run_fused(const fmoe_fused_args& args, const RouteArgs& route, const FusedPl
   al.workspace_bytes = p.align_ws_bytes;
   al.table = table;
   const bool fold = fp8 && a.scale_mode == FMOE_SCALE_BLOCK128;
-  al.token_tile = fold ? pick_fold_token_tile(p.numel, a.num_experts) : pick_token_tile(p.numel, a.num_experts);
+  al.token_tile = fold ? pick_fold_token_tile(p.numel, a.num_experts) : pick_token_tile(p.numel, a.num_experts, fp8);
   al.zero_words = counters;
   al.num_zero = counters ? 2 * kSplitCounters : 0;
   int32_t* slot_pos = tc ? reinterpret_cast<int32_t*>(ws + p.off_slot_pos) : nullptr;

@@ -686,7 +686,7 @@ int launch(const GemmParams& g, cudaStream_t st) {
   p.top_k = g.top_k;
   p.a_rows = (int32_t)g.a_rows;
   p.zero_padding = !g.skip_padding;
-  p.token_tile = g.token_tile ? g.token_tile : pick_token_tile(g.numel, g.num_experts);
+  p.token_tile = g.token_tile ? g.token_tile : pick_token_tile(g.numel, g.num_experts, g.dtype == FMOE_E4M3);
   p.stage_bytes = stage_bytes(p.token_tile);
   p.stages = std::min(RING_BYTES / p.stage_bytes, MAX_STAGES);
   p.group = pick_group_m(p.token_tile, g.k * ELEM);

@@ -9,15 +9,18 @@
 //   tile      : 256 weight rows (128 per CTA) x up to 64 tokens of one expert, as in gemm_pair.cu (same tile order, same
 //               row interleave of gate and up, same transposed stores)
 //   TMEM      : 512 columns per CTA as eight partials of 64 tokens: the MMAs of the next K blocks run while one is folded
-//   warps 0-15: fold + epilogue.  Warp w reads TMEM lanes 32 * (w % 4).. and the 16-token piece w / 4.  The 16 x 256b
-//               read-out puts two tokens of one channel side by side, which is what the packed fma.rn.f32x2 takes with one
-//               pair of factors for two channels.  The gate/up output is fp32, for the quantiser behind it
+//   warps 0-15: fold + epilogue.  Warps 0-7 fold the K blocks of even step, 8-15 those of odd step, so that one block's TMEM
+//               reads and waits run beside the other's FMAs; the two sums meet in the epilogue.  Warp w reads TMEM lanes
+//               32 * (w % 4).. and the 16-token pieces w / 4 % 2 and 2 further.  The 16 x 256b read-out puts two tokens of
+//               one channel side by side, which is what the packed fma.rn.f32x2 takes with one pair of factors for two
+//               channels.  A partial is handed back when it is in registers, before the FMAs.  (All sixteen warps on every
+//               block: 722 SM cycles per K block; this split 572.  DeepSeek-V3, 128 tokens 1361 -> 1245 us, 1024 tokens
+//               2190 -> 2005 us per layer.)  The gate/up output is fp32, for the quantiser behind it
 //   warp 16   : TMA producer      warp 17 : MMA issuer (CTA 0)
 //   warps 18-19: factors.  For four K blocks at a time they multiply the tokens' scales with the tile's one or two weight
 //               scales and leave the products in a 3-slot ring in shared memory, next to the tile's slots and row weights:
 //               the fold warps read one 8-byte pair per two tokens and keep no pointers
-// What bounds it: HBM (the weights stream through a 9-stage ring of 20 KB); the fold of a 64-token partial costs a warp
-// about 300 cycles from wait to hand-over, with eight partials in flight.
+// What bounds it: HBM (the weights stream through a ring of 20 KB stages) up to about 8 rows per expert, the fold above.
 #include "pair.cuh"
 #include "rows.cuh"
 
@@ -51,14 +54,16 @@ constexpr int TOK = 64;
 template <bool GATED>
 struct Geo {
   static constexpr int STAGE_BYTES = W_BYTES + TOK / 2 * KBYTES;
-  static constexpr int STAGES = 9;
+  static constexpr int STAGES = GATED ? 8 : 7;
   static constexpr int BUFS = TMEM_COLS / TOK;                 // TMEM partials
   static constexpr int KB_BYTES = (GATED ? 2 : 1) * TOK * 4;   // factors of one K block
   static constexpr int STRIP_BYTES = GATED ? 16 * 48 : 16 * 80;
   static constexpr int FACTOR_BYTES = SC_SLOTS * 4 * KB_BYTES;
+  static constexpr int EX_BYTES = 2 * 1024;                    // per fold warp: sums on their way to the partner warp
   static constexpr int META_BYTES = GATED ? 0 : META_TILES * TOK * 8;  // slots and row weights of the tile's tokens
   static constexpr int bytes(int num_experts) {
-    return STAGES * STAGE_BYTES + BAR_BYTES + kFoldWarps * STRIP_BYTES + FACTOR_BYTES + META_BYTES + pair_table_bytes(num_experts);
+    return STAGES * STAGE_BYTES + BAR_BYTES + kFoldWarps * (STRIP_BYTES + EX_BYTES) + FACTOR_BYTES + META_BYTES +
+           pair_table_bytes(num_experts);
   }
 };
 static_assert(Geo<true>::bytes(1024) <= kMaxSmem && Geo<false>::bytes(1024) <= kMaxSmem, "shared memory");
@@ -130,12 +135,22 @@ __device__ __forceinline__ void store32(__nv_bfloat16* dst, const float* v, floa
   }
 }
 
+__device__ __forceinline__ void sts64(uint32_t addr, unsigned long long v) {
+  asm volatile("st.shared.b64 [%0], %1;" ::"r"(addr), "l"(v) : "memory");
+}
+__device__ __forceinline__ unsigned long long add2(unsigned long long a, unsigned long long b) {
+  unsigned long long v;
+  asm("add.rn.f32x2 %0, %1, %2;" : "=l"(v) : "l"(a), "l"(b));
+  return v;
+}
+
 // PROF: instrumented build with wait-time counters (reading the clock is slow enough to distort the fold loop).
 template <bool GATED, bool PROF>
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 1)
 grouped_gemm_pair_fold_kernel(const __grid_constant__ CUtensorMap map_t, const __grid_constant__ CUtensorMap map_w,
                               const FoldParams p) {
   using G = Geo<GATED>;
+  constexpr int PIECES = TOK / 32;  // 16-token pieces per fold warp: half and half + 2
   constexpr int STAGES = G::STAGES, STAGE_BYTES = G::STAGE_BYTES, BUFS = G::BUFS, KB_BYTES = G::KB_BYTES;
   extern __shared__ __align__(1024) uint8_t smem[];  // aligned by declaration: every address below is a constant
   uint64_t* bars = reinterpret_cast<uint64_t*>(smem + STAGES * STAGE_BYTES);
@@ -145,11 +160,13 @@ grouped_gemm_pair_fold_kernel(const __grid_constant__ CUtensorMap map_t, const _
   uint64_t* part_empty = part_full + BUFS;              // [bufs] used in CTA 0: folds of both CTAs -> MMA
   uint64_t* sc_full = part_empty + BUFS;                // [slots] factor warps -> fold
   uint64_t* sc_empty = sc_full + SC_SLOTS;              // [slots] fold -> factor warps
-  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(sc_empty + SC_SLOTS);
+  uint64_t* pair_bar = sc_empty + SC_SLOTS;             // [8] the two warps that exchange sums
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(pair_bar + 8);
   uint8_t* strips = smem + STAGES * STAGE_BYTES + BAR_BYTES;
   uint8_t* factors = strips + kFoldWarps * G::STRIP_BYTES;                      // [slot][K block][gate | up][token]
   int32_t* meta = reinterpret_cast<int32_t*>(factors + G::FACTOR_BYTES);        // [tile][slot ids | row weights]
-  int32_t* table = reinterpret_cast<int32_t*>(factors + G::FACTOR_BYTES + G::META_BYTES);
+  uint8_t* exchange = factors + G::FACTOR_BYTES + G::META_BYTES;                 // [warp][round parity][4][lane] f32 pairs
+  int32_t* table = reinterpret_cast<int32_t*>(exchange + kFoldWarps * G::EX_BYTES);
 
   const int warp = ptx::uniform_warp_id(), lane = threadIdx.x & 31;
   const int rank = (int)ptx::cluster_ctarank();
@@ -163,12 +180,13 @@ grouped_gemm_pair_fold_kernel(const __grid_constant__ CUtensorMap map_t, const _
     }
     for (int b = 0; b < BUFS; ++b) {
       ptx::mbar_init(&part_full[b], 1);
-      ptx::mbar_init(&part_empty[b], 2 * kFoldWarps);  // one arrival per fold warp of both CTAs
+      ptx::mbar_init(&part_empty[b], kFoldWarps);  // the 8 warps of both CTAs that fold this K block
     }
     for (int s = 0; s < SC_SLOTS; ++s) {
       ptx::mbar_init(&sc_full[s], 1);
       ptx::mbar_init(&sc_empty[s], kFoldWarps);
     }
+    for (int w = 0; w < 8; ++w) ptx::mbar_init(&pair_bar[w], 2);
     ptx::fence_barrier_init();
   }
   if (warp == kFoldWarps && lane == 0) {
@@ -192,6 +210,8 @@ grouped_gemm_pair_fold_kernel(const __grid_constant__ CUtensorMap map_t, const _
   PairCursor cursor;
   PairTile tl;
 
+  // 16 * 104 + 4 * 64 registers per lane are the launch's 20 * 96
+  if (warp >= kFoldWarps) asm volatile("setmaxnreg.dec.sync.aligned.u32 64;");
   if (warp == kFoldWarps) {
     // ---------------- TMA producer (both CTAs) ----------------
     if (ptx::elect_one()) {
@@ -372,133 +392,166 @@ grouped_gemm_pair_fold_kernel(const __grid_constant__ CUtensorMap map_t, const _
     }
   } else {
     // ---------------- fold + epilogue (warps 0-15) ----------------
-    const int quarter = warp & 3, cgroup = warp >> 2;
+    asm volatile("setmaxnreg.inc.sync.aligned.u32 104;");
+    const int quarter = warp & 3, half = (warp >> 2) & 1, kgroup = warp >> 3;
     const int t = lane & 3;
-    const uint32_t factor_addr = ptx::smem_u32(factors) + (16 * cgroup + 2 * t) * 4;
-    const uint32_t lane_addr = tmem_base + ((uint32_t)(quarter * 32) << 16) + 16 * cgroup;
-    const uint32_t empty0 = ptx::smem_u32(part_empty) & ~ptx::kPeerRankBit;
-    uint32_t step = 0, gkb = 0;  // K blocks folded so far; the same, rounded up to whole groups at the end of each tile
+    const uint32_t factor_addr = ptx::smem_u32(factors) + (16 * half + 2 * t) * 4;
+    const uint32_t lane_addr = tmem_base + ((uint32_t)(quarter * 32) << 16) + 16 * half;
+    const uint32_t full0 = ptx::smem_u32(part_full), to_empty = BUFS * 8;  // part_empty follows part_full
+    const uint32_t out_addr = ptx::smem_u32(exchange) + warp * G::EX_BYTES + lane * 8;
+    const uint32_t in_addr = ptx::smem_u32(exchange) + (warp ^ 8) * G::EX_BYTES + lane * 8;
+    uint32_t step0 = 0, slot = 0;  // K blocks before this tile; factor slots used
     int ltile = 0;
     bool alive = true;
     long long prof_fw = 0, prof_fb = 0, prof_sw = 0, prof_epi = 0;
     for (int tile = worker; tile < total_tiles && alive; tile += workers, ++ltile) {
       cursor.locate(tile, p.w_tiles, p.group, p.num_experts, table, &tl);
-      const bool mine = cgroup < (tl.n >> 4);  // this warp has a 16-token piece
-      unsigned long long acc[8];  // [0..3] rows 0-15 of the quarter, [4..7] rows 16-31
+      const int pieces = max(0, ((tl.n >> 4) - half + 1) >> 1);  // 16-token pieces half, half + 2, ..
+      unsigned long long acc[PIECES][8];  // [0..3] rows 0-15 of the quarter, [4..7] rows 16-31
 #pragma unroll
-      for (int q = 0; q < 8; ++q) acc[q] = 0ull;
+      for (int q = 0; q < 8 * PIECES; ++q) acc[q / 8][q % 8] = 0ull;
 #pragma unroll 1
-      for (int kb = 0; kb < kblocks; ++kb, ++step, ++gkb) {
+      for (int kb0 = 0; kb0 < kblocks; kb0 += 4, ++slot) {
         const long long tf0 = PROF ? clock64() : 0;
-        if ((kb & 3) == 0) {
-          if (!warp_wait(&sc_full[(gkb >> 2) % SC_SLOTS], (gkb >> 2) / SC_SLOTS & 1)) {
-            report(0x740);
-            alive = false;
-            break;
-          }
-        }
-        const uint32_t fsrc = factor_addr + (gkb % (4 * SC_SLOTS)) * KB_BYTES;
-        const long long tf1 = PROF ? clock64() : 0;
-        if (!warp_wait(&part_full[step % BUFS], (step / BUFS) & 1)) {
-          report(0x700);
+        if (!warp_wait(&sc_full[slot % SC_SLOTS], (slot / SC_SLOTS) & 1)) {
+          report(0x740);
           alive = false;
           break;
         }
-        const long long tf2 = PROF ? clock64() : 0;
-        ptx::tc_fence_after_sync();
-        const uint32_t taddr = lane_addr + (step % BUFS) * TOK;
-        if (mine) {
-          uint32_t lo[8], hi[8];
-          ptx::tmem_ld_16x256b_x2(taddr, lo);
-          ptx::tmem_ld_16x256b_x2(taddr + (16u << 16), hi);
-          const unsigned long long g0 = lds64(fsrc), g1 = lds64(fsrc + 32);
-          unsigned long long u0 = g0, u1 = g1;
-          if constexpr (GATED) {
-            u0 = lds64(fsrc + TOK * 4);
-            u1 = lds64(fsrc + TOK * 4 + 32);
+        if (PROF) prof_sw += clock64() - tf0;
+        // the K blocks with this group's parity, counted over all tiles: a partial then always belongs to the same group
+#pragma unroll 1
+        for (int kb = kb0 + (int)((kgroup ^ (step0 + kb0)) & 1); kb < min(kb0 + 4, kblocks); kb += 2) {
+          const uint32_t step = step0 + kb, buf = step % BUFS;
+          const long long tf1 = PROF ? clock64() : 0;
+          if (!__all_sync(0xffffffffu, ptx::mbar_wait_addr(full0 + buf * 8, (step / BUFS) & 1))) {
+            report(0x700);
+            alive = false;
+            break;
           }
-          ptx::tmem_ld_wait();
-          fma2(acc[0], lo[0], lo[1], g0);
-          fma2(acc[1], lo[2], lo[3], g0);
-          fma2(acc[2], lo[4], lo[5], g1);
-          fma2(acc[3], lo[6], lo[7], g1);
-          fma2(acc[4], hi[0], hi[1], u0);
-          fma2(acc[5], hi[2], hi[3], u0);
-          fma2(acc[6], hi[4], hi[5], u1);
-          fma2(acc[7], hi[6], hi[7], u1);
+          const long long tf2 = PROF ? clock64() : 0;
+          ptx::tc_fence_after_sync();
+          const uint32_t taddr = lane_addr + buf * TOK;
+          const uint32_t fsrc = factor_addr + ((slot % SC_SLOTS) * 4 + (kb - kb0)) * KB_BYTES;
+          auto hand_back = [&]() {  // the partial is in registers
+            ptx::tc_fence_before_sync();
+            __syncwarp();
+            if (ptx::elect_one()) ptx::mbar_arrive_cluster(((full0 + buf * 8) & ~ptx::kPeerRankBit) + to_empty);
+          };
+          if (pieces > 0) {
+            uint32_t lo[PIECES][8], hi[PIECES][8];
+            unsigned long long g[PIECES][2], u[PIECES][2];
+#pragma unroll
+            for (int q = 0; q < PIECES; ++q) {  // columns past the tile's tokens hold leftovers that nobody stores
+              ptx::tmem_ld_16x256b_x2(taddr + 32 * q, lo[q]);
+              ptx::tmem_ld_16x256b_x2(taddr + 32 * q + (16u << 16), hi[q]);
+              g[q][0] = lds64(fsrc + 128 * q);
+              g[q][1] = lds64(fsrc + 128 * q + 32);
+              u[q][0] = GATED ? lds64(fsrc + 128 * q + TOK * 4) : g[q][0];
+              u[q][1] = GATED ? lds64(fsrc + 128 * q + TOK * 4 + 32) : g[q][1];
+            }
+            ptx::tmem_ld_wait();
+            hand_back();
+#pragma unroll
+            for (int q = 0; q < PIECES; ++q) {
+#pragma unroll
+              for (int c = 0; c < 4; ++c) {
+                fma2(acc[q][c], lo[q][2 * c], lo[q][2 * c + 1], g[q][c >> 1]);
+                fma2(acc[q][4 + c], hi[q][2 * c], hi[q][2 * c + 1], u[q][c >> 1]);
+              }
+            }
+          } else {
+            hand_back();
+          }
+          if (PROF) {
+            prof_fw += tf2 - tf1;
+            prof_fb += clock64() - tf2;
+          }
         }
-        ptx::tc_fence_before_sync();
+        if (!alive) break;
         __syncwarp();
-        if (lane == 0) {
-          ptx::mbar_arrive_cluster(empty0 + (step % BUFS) * 8);
-          if ((kb & 3) == 3 || kb + 1 == kblocks) ptx::mbar_arrive(&sc_empty[(gkb >> 2) % SC_SLOTS]);
-        }
-        if (PROF) {
-          prof_sw += tf1 - tf0;
-          prof_fw += tf2 - tf1;
-          prof_fb += clock64() - tf2;
-        }
+        if (lane == 0) ptx::mbar_arrive(&sc_empty[slot % SC_SLOTS]);
       }
-      gkb = (gkb + 3) & ~3u;
+      step0 += kblocks;
       if (!alive) break;
 
       const long long te0 = PROF ? clock64() : 0;
       const int32_t* m = meta + (ltile % META_TILES) * TOK * 2;
       uint8_t* strip = strips + warp * G::STRIP_BYTES;
       const int ch0 = GATED ? tl.w_tile * 128 + rank * 64 + quarter * 16 : tl.w_tile * 256 + rank * 128 + quarter * 32;
-      if (mine) {
-        const int tok0 = 16 * cgroup;
-        float2 r0 = make_float2(1.f, 1.f), r1 = r0;
-        if constexpr (!GATED) {
-          r0 = *reinterpret_cast<const float2*>(m + TOK + tok0 + 2 * t);
-          r1 = *reinterpret_cast<const float2*>(m + TOK + tok0 + 8 + 2 * t);
-        } else if (p.row_scale) {  // top-k weight on the input side: not the usual case, looked up in place
-          r0 = make_float2(row_weight(p, tl, tok0 + 2 * t), row_weight(p, tl, tok0 + 2 * t + 1));
-          r1 = make_float2(row_weight(p, tl, tok0 + 8 + 2 * t), row_weight(p, tl, tok0 + 9 + 2 * t));
+      // The two K groups' sums meet: each warp hands one piece to its partner (same channels and tokens, other group) and
+      // finishes the other.  Two rounds, two buffers: the partner has read one before it arrives for the next.
+      if (pieces > 0) {
+        unsigned long long sum[8];
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+#pragma unroll
+          for (int c = 0; c < 4; ++c) sts64(out_addr + h * 1024 + c * 256, kgroup ? acc[0][4 * h + c] : acc[1][4 * h + c]);
+          __syncwarp();
+          if (lane == 0) ptx::mbar_arrive(&pair_bar[warp & 7]);
+          if (!warp_wait(&pair_bar[warp & 7], h)) {  // two rounds per tile: h is the phase
+            report(0x7c0);
+            alive = false;
+          }
+#pragma unroll
+          for (int c = 0; c < 4; ++c)
+            sum[4 * h + c] = add2(kgroup ? acc[1][4 * h + c] : acc[0][4 * h + c], lds64(in_addr + h * 1024 + c * 256));
         }
-        float lo[8], hi[8];
+        if (!alive) break;
+        if (kgroup < pieces) {
+          const int tok0 = 16 * half + 32 * kgroup;
+          float2 r0 = make_float2(1.f, 1.f), r1 = r0;
+          if constexpr (!GATED) {
+            r0 = *reinterpret_cast<const float2*>(m + TOK + tok0 + 2 * t);
+            r1 = *reinterpret_cast<const float2*>(m + TOK + tok0 + 8 + 2 * t);
+          } else if (p.row_scale) {  // top-k weight on the input side: not the usual case, looked up in place
+            r0 = make_float2(row_weight(p, tl, tok0 + 2 * t), row_weight(p, tl, tok0 + 2 * t + 1));
+            r1 = make_float2(row_weight(p, tl, tok0 + 8 + 2 * t), row_weight(p, tl, tok0 + 9 + 2 * t));
+          }
+          float lo[8], hi[8];
 #pragma unroll
-        for (int q = 0; q < 4; ++q) {
-          unpack2(acc[q], lo[2 * q], lo[2 * q + 1]);
-          unpack2(acc[4 + q], hi[2 * q], hi[2 * q + 1]);
-        }
-        const float rs[4] = {r0.x, r0.y, r1.x, r1.y};
-        if constexpr (GATED) {
-          // element j: token tok0 + 8 * (j >> 2) + 2 t + (j & 1), channel ch0 + lane / 4 + 8 * ((j >> 1) & 1)
+          for (int q = 0; q < 4; ++q) {
+            unpack2(sum[q], lo[2 * q], lo[2 * q + 1]);
+            unpack2(sum[4 + q], hi[2 * q], hi[2 * q + 1]);
+          }
+          const float rs[4] = {r0.x, r0.y, r1.x, r1.y};
+          if constexpr (GATED) {
+            // element j: token tok0 + 8 * (j >> 2) + 2 t + (j & 1), channel ch0 + lane / 4 + 8 * ((j >> 1) & 1)
 #pragma unroll
-          for (int j = 0; j < 8; ++j) lo[j] = act_mul(lo[j] * rs[2 * (j >> 2) + (j & 1)], hi[j] * rs[2 * (j >> 2) + (j & 1)], p.activation);
-          if (p.out_dtype == FMOE_F32) {  // eight lanes store one token's 32 bytes
-            float* out = reinterpret_cast<float*>(p.out) + (int64_t)(tl.row0 + tok0) * p.n + ch0 + (lane >> 2);
+            for (int j = 0; j < 8; ++j) lo[j] = act_mul(lo[j] * rs[2 * (j >> 2) + (j & 1)], hi[j] * rs[2 * (j >> 2) + (j & 1)], p.activation);
+            if (p.out_dtype == FMOE_F32) {  // eight lanes store one token's 32 bytes
+              float* out = reinterpret_cast<float*>(p.out) + (int64_t)(tl.row0 + tok0) * p.n + ch0 + (lane >> 2);
 #pragma unroll
-            for (int j = 0; j < 8; ++j) {
-              const int u = 8 * (j >> 2) + 2 * t + (j & 1);
-              if (u < tl.cols - tok0) out[(int64_t)u * p.n + 8 * ((j >> 1) & 1)] = lo[j];
+              for (int j = 0; j < 8; ++j) {
+                const int u = 8 * (j >> 2) + 2 * t + (j & 1);
+                if (u < tl.cols - tok0) out[(int64_t)u * p.n + 8 * ((j >> 1) & 1)] = lo[j];
+              }
+            } else {
+              uint32_t v[4];
+#pragma unroll
+              for (int q = 0; q < 4; ++q) v[q] = pack_bf16x2(lo[2 * q], lo[2 * q + 1]);
+              strip_put16(strip, 48, 0, lane, v);
+              strip_store_sorted(strip, lane, reinterpret_cast<__nv_bfloat16*>(p.out) + (int64_t)(tl.row0 + tok0) * p.n, p.n, ch0,
+                                 tl.cols - tok0);
             }
           } else {
-            uint32_t v[4];
 #pragma unroll
-            for (int q = 0; q < 4; ++q) v[q] = pack_bf16x2(lo[2 * q], lo[2 * q + 1]);
-            strip_put16(strip, 48, 0, lane, v);
-            strip_store_sorted(strip, lane, reinterpret_cast<__nv_bfloat16*>(p.out) + (int64_t)(tl.row0 + tok0) * p.n, p.n, ch0,
-                               tl.cols - tok0);
-          }
-        } else {
+            for (int h = 0; h < 2; ++h) {
+              uint32_t v[4];
 #pragma unroll
-          for (int h = 0; h < 2; ++h) {
-            uint32_t v[4];
-#pragma unroll
-            for (int q = 0; q < 4; ++q) {
-              const int j = 4 * (q >> 1) + 2 * (q & 1);
-              const float a0 = h ? hi[j] : lo[j], a1 = h ? hi[j + 1] : lo[j + 1];
-              v[q] = pack_bf16x2(a0 * rs[2 * (q >> 1)], a1 * rs[2 * (q >> 1) + 1]);
+              for (int q = 0; q < 4; ++q) {
+                const int j = 4 * (q >> 1) + 2 * (q & 1);
+                const float a0 = h ? hi[j] : lo[j], a1 = h ? hi[j + 1] : lo[j + 1];
+                v[q] = pack_bf16x2(a0 * rs[2 * (q >> 1)], a1 * rs[2 * (q >> 1) + 1]);
+              }
+              strip_put16(strip, 80, 16 * h, lane, v);
             }
-            strip_put16(strip, 80, 16 * h, lane, v);
+            strip_store_slots(strip, lane, p.out, p.out_rows, p.n, ch0, m[tok0 + (lane >> 2)], m[tok0 + 8 + (lane >> 2)]);
           }
-          strip_store_slots(strip, lane, p.out, p.out_rows, p.n, ch0, m[tok0 + (lane >> 2)], m[tok0 + 8 + (lane >> 2)]);
         }
       }
       if constexpr (GATED) {
-        if (p.zero_padding && tl.last) 
+        if (p.zero_padding && tl.last)
           zero_block_rows(tl, p.out, p.n, tl.w_tile * 128 + rank * 64, p.out_dtype == FMOE_F32 ? 4 : 2, threadIdx.x, kFoldWarps * 32);
       }
       if (PROF) prof_epi += clock64() - te0;
@@ -972,6 +1025,7 @@ grouped_gemm_pair_fold_wide_kernel(const __grid_constant__ CUtensorMap map_t, co
 template <bool GATED, bool WIDE, bool PROF>
 int launch(const GemmParams& g, cudaStream_t st) {
   auto kernel = WIDE ? grouped_gemm_pair_fold_wide_kernel<GATED, PROF> : grouped_gemm_pair_fold_kernel<GATED, PROF>;
+  constexpr int TILE = WIDE ? 256 : TOK;
   static PerDeviceOnce once_attr;  // the opt-in to > 48 KB of dynamic shared memory is per device
   const cudaError_t attr_err = per_device_once(once_attr, [&] {
     return cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kMaxSmem);
@@ -979,7 +1033,6 @@ int launch(const GemmParams& g, cudaStream_t st) {
   if (attr_err != cudaSuccess)
     return fail(FMOE_ERR_CUDA, "cudaFuncSetAttribute(smem=%d) failed: %s", kMaxSmem, cudaGetErrorString(attr_err));
   const int64_t w_rows = GATED ? 2 * g.n : g.n;
-  constexpr int tile = WIDE ? 256 : TOK;
   CUtensorMap map_t, map_w;
   int rc = pair_map_tokens(&map_t, g.a, g.a_rows, g.k, 1, BOX_TOKENS);
   if (rc) return rc;
@@ -1006,12 +1059,12 @@ int launch(const GemmParams& g, cudaStream_t st) {
   p.w_tiles = (int)ceil_div<int64_t>(g.n, GATED ? 128 : 256);
   p.max_blocks = (int)g.max_blocks;
   p.activation = g.activation;
-  p.group = pick_group_m(tile, g.k);
+  p.group = pick_group_m(TILE, g.k);
   p.zero_padding = !g.skip_padding;
   p.out_dtype = g.out_dtype;
   p.out_scale = g.out_scale;
 
-  const int64_t max_tiles = g.max_blocks * ceil_div(128, tile) * p.w_tiles;
+  const int64_t max_tiles = g.max_blocks * ceil_div(128, TILE) * p.w_tiles;
   const int sms = device_sm_count();
   const int workers = (int)std::max<int64_t>(1, std::min<int64_t>((sms > 0 ? sms : 148) / 2, max_tiles));
   launch_pdl(kernel, dim3(2 * workers), dim3(kThreads),
@@ -1053,19 +1106,18 @@ int gemm_pair_fold(const GemmParams& p, bool gated, cudaStream_t st) {
                 "input rows, n and k multiples of 128");
   if (p.max_blocks <= 0) return FMOE_OK;
   static const bool profile = getenv("FMOE_TC_PROFILE") != nullptr;
-  // the table's tile width decides: 64-token tiles for the narrow kernel, 256 for the wide one
-  // (e4m3 output needs the wide one: a narrow tile's 128 channels are spread over both CTAs)
+  // the table's tile width decides; e4m3 output needs the wide kernel (a narrow tile's 128 channels are spread over both CTAs)
   const bool e4m3_out = gated && p.out_dtype == FMOE_E4M3;
-  const bool wide = p.token_tile ? p.token_tile == 256 : e4m3_out || pick_fold_token_tile(p.numel, p.num_experts) == 256;
-  FMOE_REQUIRE(wide || !e4m3_out, "tcgen05 fp8 gemm: e4m3 output needs 256-token tiles");
+  const int tile = p.token_tile ? p.token_tile : (e4m3_out ? 256 : pick_fold_token_tile(p.numel, p.num_experts));
+  FMOE_REQUIRE(tile == 256 || !e4m3_out, "tcgen05 fp8 gemm: e4m3 output needs 256-token tiles");
   auto go = [&](auto gated_c, auto wide_c) {
     constexpr bool G = decltype(gated_c)::value, W = decltype(wide_c)::value;
     return profile ? launch<G, W, true>(p, st) : launch<G, W, false>(p, st);
   };
   using T = std::true_type;
   using F = std::false_type;
-  if (gated) return wide ? go(T{}, T{}) : go(T{}, F{});
-  return wide ? go(F{}, T{}) : go(F{}, F{});
+  if (gated) return tile == 256 ? go(T{}, T{}) : go(T{}, F{});
+  return tile == 256 ? go(F{}, T{}) : go(F{}, F{});
 }
 
 }  // namespace fmoe

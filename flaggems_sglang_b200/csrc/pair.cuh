@@ -12,21 +12,24 @@
 namespace fmoe {
 
 // Most tokens of a tile, by the rows an expert has on average.  A narrow tile leaves shared memory for a deeper ring of
-// weights (what a launch needs whose time is the reading of weights) and TMEM for more partials (gemm_pair_fold.cu); a wide
-// one reads the weights from L2 less often.  Experts well above the average are cut into several tiles either way.
-inline int pick_token_tile(int64_t numel, int num_experts) {
+// weights (what a launch needs whose time is the reading of weights); a wide one reads the weights from L2 less often.
+// Experts well above the average are cut into several tiles either way.  bf16: up to 88 rows the deeper ring wins (Mixtral
+// rank, 83 rows: 287 us per layer against 292; 128 rows: 420 against 359).  e4m3 multiplies a weight byte in half the time,
+// so that the second reading is what counts (DeepSeek-V3, 64 rows on average: 128 tokens 2108 us, 256 tokens 1939 us).
+inline int pick_token_tile(int64_t numel, int num_experts, bool e4m3) {
   const double rows = (double)numel / (double)(numel < num_experts ? (numel > 0 ? numel : 1) : num_experts);
-  return rows <= 40.0 ? 64 : (rows <= 88.0 ? 128 : 256);
+  return rows <= 40.0 ? 64 : (rows <= 88.0 && !e4m3 ? 128 : 256);
 }
 constexpr int kSplitCounters = 256;  // tail-split arrival counters of one launch: one per CTA
 
 // int32 words of the expert table: first row [E], rows [E], exclusive prefix sum of the token tiles [E + 1]
 __host__ __device__ constexpr int pair_table_words(int num_experts) { return 3 * num_experts + 1; }
 __host__ __device__ constexpr int pair_table_bytes(int num_experts) { return (pair_table_words(num_experts) * 4 + 15) & ~15; }
-// The e4m3 block-scale kernels (gemm_pair_fold.cu) are built for two widths.
+// The e4m3 block-scale kernels (gemm_pair_fold.cu) are built for two widths.  DeepSeek-V3, whole layer, narrow against wide:
+// 32 rows 2.00 / 2.52 ms, 48 rows 2.51 / 2.74, 64 rows 2.86 / 2.87, 96 rows 3.84 / 3.45.
 inline int pick_fold_token_tile(int64_t numel, int num_experts) {
   const double rows = (double)numel / (double)(numel < num_experts ? (numel > 0 ? numel : 1) : num_experts);
-  return rows <= 48.0 ? 64 : 256;
+  return rows <= 64.0 ? 64 : 256;
 }
 
 #if defined(__CUDACC__)
