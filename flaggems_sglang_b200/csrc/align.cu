@@ -407,7 +407,8 @@ int run_align_sorted(const AlignArgs& a, const SortedSlots& s, cudaStream_t st) 
     const int rc = check_align(a);
     if (rc) return rc;
   }
-  const unsigned grid = (unsigned)std::min<int64_t>(ceil_div<int64_t>(std::max(a.numel, a.sorted_ids && !a.rows_only ? a.sorted_cap / 4 : 0), kSortedThreads), 148);
+  const int64_t items = std::max(a.numel, a.sorted_ids && !a.rows_only ? a.sorted_cap / 4 : 0);
+  const unsigned grid = (unsigned)std::min<int64_t>(ceil_div<int64_t>(items, kSortedThreads), 148);
   launch_pdl(align_sorted_kernel, dim3(grid), dim3(kSortedThreads), (3 * (size_t)a.E + 2) * sizeof(int), st, s.slot_of, s.hist, s.gate,
              (int)a.numel, a.E, a.block, a.sorted_ids, (int)a.sorted_cap, a.expert_ids, (int)a.expert_cap, a.num_post_pad, a.table,
              a.token_tile, a.zero_words, a.num_zero, s.ids, s.weights, a.slot_pos, (int)a.rows_only);

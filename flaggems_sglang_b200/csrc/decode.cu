@@ -19,9 +19,8 @@
 // warp per slot is also what keeps the barriers' parities unambiguous: a warp free to take any stage could wait for a
 // slot's round r + 1 while round r has not arrived, and pass.)  The stages' partial sums go through a
 // ring in shared memory to the epilogue warps, which take the units in turn and add them in stage order: their fence and
-// counter round trip last longer than a unit's stages and would hold the compute warps up.  A stage is brought by ONE TMA box of 16 KB (sixteen row-wise
-// bulk copies are no slower, but take as many instructions).  The tokens' rows (later the expert's
-// activations) stay in shared memory beside the ring.
+// counter round trip last longer than a unit's stages and would hold the compute warps up.  A stage is brought by one TMA
+// box of 16 KB.  The tokens' rows (later the expert's activations) stay in shared memory beside the ring.
 //
 // The CTAs of decode_layer_kernel wait on one another's counters: there is at most one per SM and all of them are
 // resident, every wait is bounded, and on expiry the status word is set and the CTA finishes without the result.

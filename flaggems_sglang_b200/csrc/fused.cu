@@ -56,11 +56,9 @@ int pick_variant(int dtype, int64_t numel, int E, int64_t I, int64_t H, int forc
 namespace {
 inline int64_t up256(int64_t v) { return (v + 255) & ~int64_t(255); }
 
-// The single-CTA bf16 tcgen05 gate/up kernel can fetch its input rows by TMA gather4 instead of reading a
-// sorted copy of the hidden states.  Measured on B200 the gather costs more than the copy saves (32 four-row
-// TMA instructions per 16 KB stage against one tiled load: gate/up 4.07 ms against 1.67 ms at Mixtral
-// T=4096, 1.03 against 0.39 ms at Qwen3 T=8192), so the copy is the default and FMOE_TC_GATHER4=1 selects
-// the gather (it saves the cap x H workspace).
+// The bf16 gate/up GEMM can fetch its input rows by TMA gather4 instead of reading a sorted copy of the hidden states.  The
+// gather costs about 12 cycles per row and K step, more than the copy (gate/up GEMM at Mixtral T=4096 2.4 times slower), so
+// the copy is the default and FMOE_TC_GATHER4=1 selects the gather (it saves the cap x H workspace).
 inline bool tc_gathers_input(int variant, int dtype) {
   static const bool gather4 = getenv("FMOE_TC_GATHER4") != nullptr;
   return variant == FMOE_VARIANT_TCGEN05 && dtype == FMOE_BF16 && gather4;
@@ -153,7 +151,6 @@ int plan_fused(const fmoe_fused_args& a, const RouteArgs& route, FusedPlan* pl) 
     // token rows quantised straight into the sorted order, one scale per token; every row of the activation with its own
     p.off_xs = take(p.cap * a.H);
     p.off_xs_scale = take(a.T * 4);
-    p.act_elem = 2;
     p.off_act = take(p.cap * a.I * 2);
     p.off_actq = take(p.cap * a.I);
     p.off_actq_scale = take(p.cap * 4);
@@ -163,9 +160,7 @@ int plan_fused(const fmoe_fused_args& a, const RouteArgs& route, FusedPlan* pl) 
     p.off_xs = take((tc ? p.cap : a.T) * a.H);
     p.off_xs_scale = take(a.T * (a.H / 128) * 4);
     // the wide tensor-core kernel quantises its 128-channel groups itself; the others write fp32 for the quantiser
-    const bool wide = tc && pick_fold_token_tile(p.numel, a.num_experts) == 256;
-    p.act_elem = wide ? 1 : 4;
-    p.off_act = wide ? -1 : take(p.cap * a.I * 4);
+    p.off_act = take(p.cap * a.I * 4);
     p.off_actq = take(p.cap * a.I);
     p.off_actq_scale = take(p.cap * (a.I / 128) * 4);
   } else {
@@ -174,7 +169,6 @@ int plan_fused(const fmoe_fused_args& a, const RouteArgs& route, FusedPlan* pl) 
       p.split_bytes = fmoe_gemm_split_workspace_bytes();
       p.off_split = take(p.split_bytes);
     }
-    p.act_elem = (int)eb;
     p.off_act = take(p.cap * a.I * eb);
   }
   p.off_z = a.no_combine ? -1 : take(p.numel * a.H * eb);
@@ -265,7 +259,7 @@ int run_fused(const fmoe_fused_args& args, const RouteArgs& route, const FusedPl
   int32_t* sorted = reinterpret_cast<int32_t*>(ws + p.off_sorted);
   int32_t* experts = reinterpret_cast<int32_t*>(ws + p.off_expert);
   int32_t* npp = reinterpret_cast<int32_t*>(ws + p.off_npp);
-  void* act = p.off_act >= 0 ? ws + p.off_act : nullptr;
+  void* act = ws + p.off_act;
   void* z = a.no_combine ? a.out : (void*)(ws + p.off_z);
 
   mark(0);
@@ -285,7 +279,7 @@ int run_fused(const fmoe_fused_args& args, const RouteArgs& route, const FusedPl
   al.workspace_bytes = p.align_ws_bytes;
   al.table = table;
   const bool fold = fp8 && a.scale_mode == FMOE_SCALE_BLOCK128;
-  al.token_tile = fold ? pick_fold_token_tile(p.numel, a.num_experts) : pick_token_tile(p.numel, a.num_experts, fp8);
+  al.token_tile = fold ? kNarrowRows : pick_token_tile(p.numel, a.num_experts, fp8);
   al.zero_words = counters;
   al.num_zero = counters ? 2 * kSplitCounters : 0;
   int32_t* slot_pos = tc ? reinterpret_cast<int32_t*>(ws + p.off_slot_pos) : nullptr;
@@ -369,11 +363,7 @@ int run_fused(const fmoe_fused_args& args, const RouteArgs& route, const FusedPl
     }
     if (rc) return rc;
     g1.dtype = g2.dtype = FMOE_E4M3;
-    g1.out_dtype = channel ? FMOE_BF16 : (p.act_elem == 1 ? FMOE_E4M3 : FMOE_F32);
-    if (g1.out_dtype == FMOE_E4M3) {
-      g1.out = ws + p.off_actq;
-      g1.out_scale = reinterpret_cast<float*>(ws + p.off_actq_scale);
-    }
+    g1.out_dtype = channel ? FMOE_BF16 : FMOE_F32;
     g1.a = xq;
     g1.a_scale = xsc;
     g1.a_rows = tc ? p.cap : a.T;
@@ -383,14 +373,31 @@ int run_fused(const fmoe_fused_args& args, const RouteArgs& route, const FusedPl
     g2.a_scale = reinterpret_cast<float*>(ws + p.off_actq_scale);
     g2.w_scale = a.w2_scale;
   }
+  const bool both_folds = fold && tc && !fold_narrow_only(p.numel, a.num_experts);
   mark(2);
+  if (both_folds) g1.fold = FoldKernel::kNarrow;
   rc = run_gemm(g1, true, st);
   if (rc) return rc;
+  if (both_folds) {
+    g1.fold = FoldKernel::kWide;
+    g1.out = ws + p.off_actq;
+    g1.out_scale = reinterpret_cast<float*>(ws + p.off_actq_scale);
+    g1.out_dtype = FMOE_E4M3;
+    rc = run_gemm(g1, true, st);
+    if (rc) return rc;
+  }
   mark(3);
-  if (fp8 && act) {
+  if (fp8) {
     float* scale = reinterpret_cast<float*>(ws + p.off_actq_scale);
-    rc = tc ? run_quant_slots(act, g1.out_dtype, p.numel, a.I, slot_pos, a.scale_mode == FMOE_SCALE_CHANNEL, ws + p.off_actq, scale, st)
-            : fmoe_quant_fp8_group128(act, FMOE_F32, p.cap, a.I, sorted, 0, p.numel, npp, ws + p.off_actq, scale, stream);
+    if (a.scale_mode == FMOE_SCALE_CHANNEL) {
+      rc = run_quant_rows(act, p.numel, a.I, slot_pos, ws + p.off_actq, scale, st);
+    } else if (tc && both_folds) {
+      rc = run_quant_experts(static_cast<const float*>(act), p.numel, a.I, a.num_experts, table, kNarrowRows, ws + p.off_actq, scale, st);
+    } else if (tc) {
+      rc = run_quant_slots(static_cast<const float*>(act), p.numel, a.I, slot_pos, ws + p.off_actq, scale, st);
+    } else {
+      rc = fmoe_quant_fp8_group128(act, FMOE_F32, p.cap, a.I, sorted, 0, p.numel, npp, ws + p.off_actq, scale, stream);
+    }
     if (rc) return rc;
   }
   mark(4);

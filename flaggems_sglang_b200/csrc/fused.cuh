@@ -6,7 +6,7 @@
 namespace fmoe {
 
 struct FusedPlan {
-  int variant, block, act_elem;
+  int variant, block;
   int64_t numel, cap, nblk, max_blocks, total;
   // byte offsets into the workspace (-1: not used)
   int64_t off_sorted, off_expert, off_npp, off_align_ws, align_ws_bytes, off_xs, off_xs_scale, off_act, off_actq, off_actq_scale, off_z;

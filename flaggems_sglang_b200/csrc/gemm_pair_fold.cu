@@ -44,6 +44,7 @@ constexpr int W_BYTES = 128 * KBYTES;
 constexpr int TMEM_COLS = 512;
 constexpr int kFoldWarps = 16;
 constexpr int kThreads = (kFoldWarps + 4) * 32;
+constexpr int kFoldRegs = 104, kOtherRegs = 64;  // per thread, out of the launch's 20 * 96 per lane (setmaxnreg)
 constexpr int BOX_TOKENS = 32;
 constexpr int SC_SLOTS = 4;                      // factor ring: slots of 4 K blocks
 constexpr int META_TILES = 8;                    // more than the SC_SLOTS tiles that the factor warps may be ahead of the fold
@@ -92,6 +93,7 @@ struct FoldParams {
   int32_t zero_padding;
   int32_t out_dtype;  // gate/up: FMOE_F32, FMOE_BF16 or (wide) FMOE_E4M3 with out_scale
   float* out_scale;   // [rows, n / 128]
+  int32_t min_rows, max_rows;  // experts of this launch
 };
 
 __device__ __forceinline__ void report(int code) { atomicCAS(&g_device_status_fp8, 0, code); }
@@ -201,7 +203,7 @@ grouped_gemm_pair_fold_kernel(const __grid_constant__ CUtensorMap map_t, const _
   pdl_entry();  // everything above is independent of the kernels before this one on the stream
   const int used_blocks = min((int)(*p.num_tokens_post_padded / 128), p.max_blocks);
   pair_build_table(table, p.num_experts, p.expert_table, p.expert_ids, p.sorted_token_ids, p.numel, 128, TOK,
-                   used_blocks);
+                   used_blocks, p.min_rows, p.max_rows);
   ptx::cluster_sync_all();
   ptx::tc_fence_after_sync();
   const uint32_t tmem_base = *tmem_slot;
@@ -210,8 +212,7 @@ grouped_gemm_pair_fold_kernel(const __grid_constant__ CUtensorMap map_t, const _
   PairCursor cursor;
   PairTile tl;
 
-  // 16 * 104 + 4 * 64 registers per lane are the launch's 20 * 96
-  if (warp >= kFoldWarps) asm volatile("setmaxnreg.dec.sync.aligned.u32 64;");
+  if (warp >= kFoldWarps) asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(kOtherRegs));
   if (warp == kFoldWarps) {
     // ---------------- TMA producer (both CTAs) ----------------
     if (ptx::elect_one()) {
@@ -392,7 +393,7 @@ grouped_gemm_pair_fold_kernel(const __grid_constant__ CUtensorMap map_t, const _
     }
   } else {
     // ---------------- fold + epilogue (warps 0-15) ----------------
-    asm volatile("setmaxnreg.inc.sync.aligned.u32 104;");
+    asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(kFoldRegs));
     const int quarter = warp & 3, half = (warp >> 2) & 1, kgroup = warp >> 3;
     const int t = lane & 3;
     const uint32_t factor_addr = ptx::smem_u32(factors) + (16 * half + 2 * t) * 4;
@@ -668,7 +669,8 @@ grouped_gemm_pair_fold_wide_kernel(const __grid_constant__ CUtensorMap map_t, co
   ptx::tc_fence_before_sync();
   pdl_entry();
   const int used_blocks = min((int)(*p.num_tokens_post_padded / 128), p.max_blocks);
-  pair_build_table(table, p.num_experts, p.expert_table, p.expert_ids, p.sorted_token_ids, p.numel, 128, 256, used_blocks);
+  pair_build_table(table, p.num_experts, p.expert_table, p.expert_ids, p.sorted_token_ids, p.numel, 128, 256, used_blocks,
+                   p.min_rows, p.max_rows);
   ptx::cluster_sync_all();
   ptx::tc_fence_after_sync();
   const uint32_t tmem_base = *tmem_slot;
@@ -677,9 +679,7 @@ grouped_gemm_pair_fold_wide_kernel(const __grid_constant__ CUtensorMap map_t, co
   PairCursor cursor;
   PairTile tl;
 
-  // 16 * 104 + 4 * 64 registers per lane are the launch's 20 * 96
-  // 16 * 104 + 4 * 64 registers per lane are the launch's 20 * 96
-  if (warp >= kFoldWarps) asm volatile("setmaxnreg.dec.sync.aligned.u32 64;");
+  if (warp >= kFoldWarps) asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(kOtherRegs));
   if (warp == kFoldWarps) {
     // ---------------- TMA producer (both CTAs): its half of the tile's tokens, its 128 weight rows ----------------
     if (ptx::elect_one()) {
@@ -874,7 +874,7 @@ grouped_gemm_pair_fold_wide_kernel(const __grid_constant__ CUtensorMap map_t, co
     }
   } else {
     // ---------------- fold + epilogue (warps 0-15) ----------------
-    asm volatile("setmaxnreg.inc.sync.aligned.u32 104;");
+    asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(kFoldRegs));
     // This loop runs at the 96 registers that 20 warps leave a thread: the tile is described by its meta entry, shared
     // memory addresses are constants, everything else is derived from three counters.
     const uint32_t lane_addr = tmem_base + ((uint32_t)((warp & 3) * 32) << 16) + 128 * (warp >> 3) + 32 * ((warp >> 2) & 1);
@@ -1023,15 +1023,20 @@ grouped_gemm_pair_fold_wide_kernel(const __grid_constant__ CUtensorMap map_t, co
 }
 
 template <bool GATED, bool WIDE, bool PROF>
-int launch(const GemmParams& g, cudaStream_t st) {
+int launch(const GemmParams& g, int min_rows, int max_rows, cudaStream_t st) {
   auto kernel = WIDE ? grouped_gemm_pair_fold_wide_kernel<GATED, PROF> : grouped_gemm_pair_fold_kernel<GATED, PROF>;
   constexpr int TILE = WIDE ? 256 : TOK;
   static PerDeviceOnce once_attr;  // the opt-in to > 48 KB of dynamic shared memory is per device
   const cudaError_t attr_err = per_device_once(once_attr, [&] {
+    // setmaxnreg waits for good when the launch has fewer registers than the warps' shares add up to
+    cudaFuncAttributes fa;
+    const cudaError_t err = cudaFuncGetAttributes(&fa, kernel);
+    if (err != cudaSuccess) return err;
+    if (fa.numRegs * kThreads < (kFoldWarps * kFoldRegs + 4 * kOtherRegs) * 32) return cudaErrorInvalidConfiguration;
     return cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kMaxSmem);
   });
   if (attr_err != cudaSuccess)
-    return fail(FMOE_ERR_CUDA, "cudaFuncSetAttribute(smem=%d) failed: %s", kMaxSmem, cudaGetErrorString(attr_err));
+    return fail(FMOE_ERR_CUDA, "set-up of the e4m3 kernel (smem=%d) failed: %s", kMaxSmem, cudaGetErrorString(attr_err));
   const int64_t w_rows = GATED ? 2 * g.n : g.n;
   CUtensorMap map_t, map_w;
   int rc = pair_map_tokens(&map_t, g.a, g.a_rows, g.k, 1, BOX_TOKENS);
@@ -1063,6 +1068,8 @@ int launch(const GemmParams& g, cudaStream_t st) {
   p.zero_padding = !g.skip_padding;
   p.out_dtype = g.out_dtype;
   p.out_scale = g.out_scale;
+  p.min_rows = min_rows;
+  p.max_rows = max_rows;
 
   const int64_t max_tiles = g.max_blocks * ceil_div(128, TILE) * p.w_tiles;
   const int sms = device_sm_count();
@@ -1106,18 +1113,20 @@ int gemm_pair_fold(const GemmParams& p, bool gated, cudaStream_t st) {
                 "input rows, n and k multiples of 128");
   if (p.max_blocks <= 0) return FMOE_OK;
   static const bool profile = getenv("FMOE_TC_PROFILE") != nullptr;
-  // the table's tile width decides; e4m3 output needs the wide kernel (a narrow tile's 128 channels are spread over both CTAs)
-  const bool e4m3_out = gated && p.out_dtype == FMOE_E4M3;
-  const int tile = p.token_tile ? p.token_tile : (e4m3_out ? 256 : pick_fold_token_tile(p.numel, p.num_experts));
-  FMOE_REQUIRE(tile == 256 || !e4m3_out, "tcgen05 fp8 gemm: e4m3 output needs 256-token tiles");
-  auto go = [&](auto gated_c, auto wide_c) {
-    constexpr bool G = decltype(gated_c)::value, W = decltype(wide_c)::value;
-    return profile ? launch<G, W, true>(p, st) : launch<G, W, false>(p, st);
+  auto go = [&](auto wide_c, int min_rows, int max_rows) {
+    constexpr bool W = decltype(wide_c)::value;
+    if (profile) return gated ? launch<true, W, true>(p, min_rows, max_rows, st) : launch<false, W, true>(p, min_rows, max_rows, st);
+    return gated ? launch<true, W, false>(p, min_rows, max_rows, st) : launch<false, W, false>(p, min_rows, max_rows, st);
   };
-  using T = std::true_type;
-  using F = std::false_type;
-  if (gated) return tile == 256 ? go(T{}, T{}) : go(T{}, F{});
-  return tile == 256 ? go(F{}, T{}) : go(F{}, F{});
+  constexpr int kAll = 0x7fffffff;
+  // e4m3 output is the wide kernel's: a narrow tile's 128 channels are spread over both CTAs
+  const bool e4m3_out = gated && p.out_dtype == FMOE_E4M3;
+  if (p.fold == FoldKernel::kWide) return go(std::true_type{}, kNarrowRows + 1, kAll);
+  if (e4m3_out) return go(std::true_type{}, 1, kAll);
+  if (fold_narrow_only(p.numel, p.num_experts)) return go(std::false_type{}, 0, kAll);
+  const int rc = go(std::false_type{}, 0, kNarrowRows);
+  if (rc || p.fold == FoldKernel::kNarrow) return rc;
+  return go(std::true_type{}, kNarrowRows + 1, kAll);
 }
 
 }  // namespace fmoe

@@ -25,11 +25,12 @@ constexpr int kSplitCounters = 256;  // tail-split arrival counters of one launc
 // int32 words of the expert table: first row [E], rows [E], exclusive prefix sum of the token tiles [E + 1]
 __host__ __device__ constexpr int pair_table_words(int num_experts) { return 3 * num_experts + 1; }
 __host__ __device__ constexpr int pair_table_bytes(int num_experts) { return (pair_table_words(num_experts) * 4 + 15) & ~15; }
-// The e4m3 block-scale kernels (gemm_pair_fold.cu) are built for two widths.  DeepSeek-V3, whole layer, narrow against wide:
-// 32 rows 2.00 / 2.52 ms, 48 rows 2.51 / 2.74, 64 rows 2.86 / 2.87, 96 rows 3.84 / 3.45.
-inline int pick_fold_token_tile(int64_t numel, int num_experts) {
-  const double rows = (double)numel / (double)(numel < num_experts ? (numel > 0 ? numel : 1) : num_experts);
-  return rows <= 64.0 ? 64 : 256;
+// The e4m3 block-scale GEMMs (gemm_pair_fold.cu): experts with up to kNarrowRows rows go to the narrow kernel (one 64-token
+// tile: 0.36 us per K block and tile), the others to the wide one (256 tokens: 0.65 us).  A call whose experts have few rows
+// on average is left to the narrow kernel alone: the wide one would find next to nothing.
+constexpr int kNarrowRows = 64;
+inline bool fold_narrow_only(int64_t numel, int num_experts) {
+  return numel <= 16 * (numel < num_experts ? numel : (int64_t)num_experts);
 }
 
 #if defined(__CUDACC__)
@@ -54,18 +55,26 @@ __device__ __forceinline__ void pair_prefix_warp(const int32_t* rows, int32_t* p
 
 // All threads of the CTA fill `table` (shared memory): a copy of the one moe_align wrote, or, for callers of the plain
 // C entry points, derived from the block tables (rows of an expert = up to the last real slot of its last block).
-// Ends with __syncthreads().
+// Experts whose rows are outside [min_rows, max_rows] are left without tiles.  Ends with __syncthreads().
 __device__ __forceinline__ void pair_build_table(int32_t* table, int num_experts, const int32_t* __restrict__ global_table,
                                                  const int32_t* __restrict__ expert_ids,
                                                  const int32_t* __restrict__ sorted_ids, int64_t numel, int block_rows,
-                                                 int token_tile, int used_blocks) {
+                                                 int token_tile, int used_blocks, int min_rows = 0, int max_rows = 0x7fffffff) {
+  int32_t* first = table;
+  int32_t* rows = table + num_experts;
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   if (global_table) {
-    for (int i = threadIdx.x; i < pair_table_words(num_experts); i += blockDim.x) table[i] = global_table[i];
+    const bool all = min_rows <= 0 && max_rows == 0x7fffffff;
+    for (int i = threadIdx.x; i < pair_table_words(num_experts); i += blockDim.x) {
+      const int32_t v = global_table[i];
+      table[i] = !all && i >= num_experts && i < 2 * num_experts && (v < min_rows || v > max_rows) ? 0 : v;
+    }
+    __syncthreads();
+    if (all) return;
+    if (warp == 0) pair_prefix_warp(rows, table + 2 * num_experts, num_experts, token_tile, lane);
     __syncthreads();
     return;
   }
-  int32_t* first = table;
-  int32_t* rows = table + num_experts;
   for (int e = threadIdx.x; e < num_experts; e += blockDim.x) {
     first[e] = 0x7fffffff;
     rows[e] = 0;
@@ -79,7 +88,6 @@ __device__ __forceinline__ void pair_build_table(int32_t* table, int num_experts
     }
   }
   __syncthreads();
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   for (int e = warp; e < num_experts; e += blockDim.x >> 5) {
     const int b0 = first[e], nb = rows[e];
     __syncwarp();
@@ -94,7 +102,8 @@ __device__ __forceinline__ void pair_build_table(int32_t* table, int num_experts
     }
     if (lane == 0) {
       first[e] = nb > 0 ? b0 * block_rows : 0;
-      rows[e] = nb > 0 ? (nb - 1) * block_rows + last : 0;
+      const int r = nb > 0 ? (nb - 1) * block_rows + last : 0;
+      rows[e] = r < min_rows || r > max_rows ? 0 : r;
     }
   }
   __syncthreads();

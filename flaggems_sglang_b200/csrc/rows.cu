@@ -9,7 +9,7 @@
 namespace fmoe {
 namespace {
 
-enum class RowMode { kMap, kScatter, kInPlace };
+enum class RowMode { kMap, kScatter, kInPlace, kExpert };
 
 // Source row of output position p: p itself without a map; with a map, the map's entry divided by map_div,
 // or p when map_div is 0 (the map then only marks padding).  -1 = padding position.
@@ -31,6 +31,8 @@ __device__ __forceinline__ int64_t mapped_row(const int32_t* row_map, int map_di
 //   RowMode::kScatter : row p is token p, read and quantised once and stored at the positions of its map_div slots; its
 //                       scales stay by token (the GEMM looks them up)
 //   RowMode::kInPlace : row p is slot p; the row at its position is quantised into the same position
+//   RowMode::kExpert  : blockIdx.y is an expert; its rows are quantised in place unless they are more than map_div.  `pos` is
+//                       the expert table (first row [E], rows [E], ..)
 // DeepSeek-V3, 128 tokens (1024 rows in 21k positions): 26 -> 10 us before the gate/up GEMM, 38 -> 7 us before the down GEMM;
 // 2048 tokens with one scale per row: 67 -> 42 us.
 template <typename InT, RowMode MODE>
@@ -43,7 +45,13 @@ quant_group128_kernel(const InT* __restrict__ x, int64_t rows_out, int64_t K, co
   const int sub = threadIdx.x & 15;  // lane inside the 16-lane team
   const unsigned hmask = (threadIdx.x & 16) ? 0xffff0000u : 0x0000ffffu;
   const int groups = (int)(K / 128);
-  const int64_t limit = num_rows_dev ? min((int64_t)*num_rows_dev, rows_out) : rows_out;
+  int64_t limit = num_rows_dev ? min((int64_t)*num_rows_dev, rows_out) : rows_out;
+  int64_t base = 0;
+  if constexpr (MODE == RowMode::kExpert) {
+    base = pos[blockIdx.y];
+    limit = pos[gridDim.y + blockIdx.y];
+    if (limit > map_div) return;
+  }
   const int64_t teams = (int64_t)gridDim.x * 16;
   const int64_t team = (int64_t)blockIdx.x * 16 + (threadIdx.x >> 4);
   const int64_t step_p = teams / groups;
@@ -63,8 +71,9 @@ quant_group128_kernel(const InT* __restrict__ x, int64_t rows_out, int64_t K, co
 #pragma unroll
       for (int i = 0; i < 8; ++i) v[u][i] = 0.f;
       if (p < limit) {
-        const int64_t r = MODE == RowMode::kScatter ? p : (MODE == RowMode::kInPlace ? pos[p] : mapped_row(row_map, map_div, sentinel, p));
-        if (MODE == RowMode::kInPlace) pu[u] = r;
+        const int64_t r = MODE == RowMode::kScatter ? p : (MODE == RowMode::kExpert ? base + p
+                          : (MODE == RowMode::kInPlace ? pos[p] : mapped_row(row_map, map_div, sentinel, p)));
+        if (MODE == RowMode::kExpert || MODE == RowMode::kInPlace) pu[u] = r;
         real[u] = r >= 0;
         if (r >= 0) {
           const InT* src = x + r * K + g * 128 + sub * 8;
@@ -235,8 +244,8 @@ gather_rows_kernel(const uint4* __restrict__ x, int64_t rows_out, int64_t vec_pe
   }
 }
 
-// Every token row to the positions of its k slots: read once, k stores (Qwen3, 7777 tokens: 64 -> 46 us, 5.9 TB/s of stores).  A warp per 2 KB piece of a row, so that few long
-// rows still fill the chip.
+// Every token row to the positions of its k slots: read once, k stores (Qwen3, 7777 tokens: 64 -> 46 us, 5.9 TB/s of
+// stores).  A warp per 2 KB piece of a row, so that few long rows still fill the chip.
 __global__ void __launch_bounds__(256)
 scatter_rows_kernel(const uint4* __restrict__ x, int64_t T, int k, int vec_per_row, int pieces, const int32_t* __restrict__ pos,
                     uint4* __restrict__ out) {
@@ -384,21 +393,38 @@ int fmoe::run_quant_scatter(const void* x, int64_t T, int k, int64_t K, const in
   return launch_status("quant_scatter");
 }
 
-int fmoe::run_quant_slots(const void* x, int in_dtype, int64_t numel, int64_t K, const int32_t* slot_pos, bool per_row, void* q,
-                          float* scale, cudaStream_t st) {
-  FMOE_REQUIRE(K > 0 && K % (per_row ? 8 : 128) == 0 && (!per_row || K <= 16384), "quant_slots: bad K %lld", (long long)K);
-  FMOE_REQUIRE(in_dtype == (per_row ? FMOE_BF16 : FMOE_F32), "quant_slots: input is bf16 per row, f32 per group");
-  FMOE_REQUIRE(x && q && scale && aligned16(x) && (reinterpret_cast<uintptr_t>(q) & 7u) == 0, "quant_slots: null or misaligned pointer");
-  auto go = [&](auto kernel, auto* xt, int64_t ctas) {
-    launch_pdl(kernel, dim3((unsigned)std::min<int64_t>(std::max<int64_t>(ctas, 1), 148 * 8)), dim3(256), 0, st, xt, numel, K,
-               nullptr, 1, 0, nullptr, (uint8_t*)q, scale, slot_pos);
+int fmoe::run_quant_rows(const void* x, int64_t numel, int64_t K, const int32_t* slot_pos, void* q, float* scale, cudaStream_t st) {
+  FMOE_REQUIRE(K > 0 && K % 8 == 0 && K <= 16384, "quant_rows: bad K %lld", (long long)K);
+  FMOE_REQUIRE(x && q && scale && aligned16(x) && (reinterpret_cast<uintptr_t>(q) & 7u) == 0, "quant_rows: null or misaligned pointer");
+  auto go = [&](auto kernel, int64_t ctas) {
+    launch_pdl(kernel, dim3((unsigned)std::min<int64_t>(std::max<int64_t>(ctas, 1), 148 * 8)), dim3(256), 0, st,
+               (const __nv_bfloat16*)x, numel, K, nullptr, 1, 0, nullptr, (uint8_t*)q, scale, slot_pos);
   };
-  const auto* xb = (const __nv_bfloat16*)x;
-  if (!per_row) go(quant_group128_kernel<float, RowMode::kInPlace>, (const float*)x, ceil_div<int64_t>(numel * (K / 128), 64));
-  else if (K <= 2048) go(quant_row_kernel<32, 8, RowMode::kInPlace>, xb, ceil_div<int64_t>(numel, 8));
-  else if (K <= 4096) go(quant_row_kernel<32, 16, RowMode::kInPlace>, xb, ceil_div<int64_t>(numel, 8));
-  else go(quant_row_kernel<256, 8, RowMode::kInPlace>, xb, numel);
+  if (K <= 2048) go(quant_row_kernel<32, 8, RowMode::kInPlace>, ceil_div<int64_t>(numel, 8));
+  else if (K <= 4096) go(quant_row_kernel<32, 16, RowMode::kInPlace>, ceil_div<int64_t>(numel, 8));
+  else go(quant_row_kernel<256, 8, RowMode::kInPlace>, numel);
+  return launch_status("quant_rows");
+}
+
+int fmoe::run_quant_slots(const float* x, int64_t numel, int64_t K, const int32_t* slot_pos, void* q, float* scale, cudaStream_t st) {
+  FMOE_REQUIRE(K > 0 && K % 128 == 0, "quant_slots: bad K %lld", (long long)K);
+  FMOE_REQUIRE(x && q && scale && aligned16(x) && (reinterpret_cast<uintptr_t>(q) & 7u) == 0, "quant_slots: null or misaligned pointer");
+  const unsigned grid = (unsigned)std::min<int64_t>(ceil_div<int64_t>(numel * (K / 128), 64), 148 * 8);
+  launch_pdl(quant_group128_kernel<float, RowMode::kInPlace>, dim3(grid), dim3(256), 0, st, x, numel, K, nullptr, 1, 0, nullptr,
+             (uint8_t*)q, scale, slot_pos);
   return launch_status("quant_slots");
+}
+
+int fmoe::run_quant_experts(const float* x, int64_t numel, int64_t K, int num_experts, const int32_t* table, int max_rows, void* q,
+                            float* scale, cudaStream_t st) {
+  FMOE_REQUIRE(K > 0 && K % 128 == 0, "quant_experts: bad K %lld", (long long)K);
+  FMOE_REQUIRE(x && q && scale && aligned16(x) && (reinterpret_cast<uintptr_t>(q) & 7u) == 0, "quant_experts: null or misaligned pointer");
+  // 64 items per CTA and pass; as many CTAs per expert as its rows on average (at most max_rows) ask for
+  const int64_t rows = std::min<int64_t>(ceil_div<int64_t>(numel, num_experts), max_rows);
+  const unsigned per_expert = (unsigned)std::min<int64_t>(std::max<int64_t>(1, rows * (K / 128) / 128), 8);
+  launch_pdl(quant_group128_kernel<float, RowMode::kExpert>, dim3(per_expert, num_experts), dim3(256), 0, st, x, 0, K, nullptr,
+             max_rows, 0, nullptr, (uint8_t*)q, scale, table);
+  return launch_status("quant_experts");
 }
 
 extern "C" int fmoe_gather_rows(const void* x, int elem_bytes, int64_t rows_out, int64_t K,
@@ -437,7 +463,11 @@ extern "C" int fmoe_moe_sum_add(const void* z, int dtype, int64_t T, int k, int6
     using E = std::remove_pointer_t<decltype(zt)>;
     launch_pdl(kernel, dim3(grid), dim3(256), 0, st, (const E*)z, T, k, H, scale, (const E*)addend, (E*)out);
   };
-  if (dtype == FMOE_BF16) k <= 2 ? go(moe_sum_kernel<__nv_bfloat16, 2>, (__nv_bfloat16*)nullptr) : go(moe_sum_kernel<__nv_bfloat16, 4>, (__nv_bfloat16*)nullptr);
-  else k <= 2 ? go(moe_sum_kernel<float, 2>, (float*)nullptr) : go(moe_sum_kernel<float, 4>, (float*)nullptr);
+  __nv_bfloat16* b16 = nullptr;
+  float* f32 = nullptr;
+  if (dtype == FMOE_BF16 && k <= 2) go(moe_sum_kernel<__nv_bfloat16, 2>, b16);  // two slots: more CTAs instead of more loads
+  else if (dtype == FMOE_BF16) go(moe_sum_kernel<__nv_bfloat16, 4>, b16);
+  else if (k <= 2) go(moe_sum_kernel<float, 2>, f32);
+  else go(moe_sum_kernel<float, 4>, f32);
   return launch_status("moe_sum_kernel");
 }

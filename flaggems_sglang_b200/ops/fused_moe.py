@@ -9,10 +9,11 @@ CUDA kernels behind the C ABI (include/fmoe_b200.h); nothing falls back to
 torch or the CPU.
 
 Kernel selection (per call, from shapes only, no host sync):
-  rows per active expert <= 4    -> "stream": small-M weight-streaming kernel,
-                                    moe_align block 8, x gathered on the fly
-  larger                         -> "tcgen05": rows copied into expert-sorted order
-                                    (block 128), TMA + tcgen05/TMEM persistent kernel
+  up to 8 tokens                 -> two decode kernels: routing and block list, then both GEMMs and the combine
+  rows per active expert <= 4    -> "stream" (e4m3: below 4): small-M weight-streaming kernel, moe_align block 8, x gathered
+                                    on the fly
+  larger                         -> "tcgen05": rows copied (e4m3: quantised) into expert-sorted order (block 128), TMA +
+                                    tcgen05/TMEM persistent kernels on CTA pairs
   fp32 inputs                    -> "simt"
 """
 from __future__ import annotations
@@ -335,7 +336,7 @@ def _experts(hidden_states, w1, w2, topk_weights, topk_ids, route, k, inplace=Fa
 
     if not use_fp8_w8a8:
         if name == "tcgen05" and not os.environ.get("FMOE_TC_GATHER4"):
-            # sorted copy of the input rows (FMOE_TC_GATHER4=1: the single-CTA kernel gathers them by TMA instead)
+            # sorted copy of the input rows (FMOE_TC_GATHER4=1: the gate/up GEMM gathers them by TMA instead)
             xs = torch.empty((cap, H), dtype=out_dtype, device=dev)
             with _stage("gather_rows"):
                 _C.check(lib.fmoe_gather_rows(x.data_ptr(), x.element_size(), cap, H, sorted_ids.data_ptr(), k, numel,
