@@ -120,7 +120,8 @@ moe_align_kernel(const int32_t* __restrict__ topk_ids, int numel, int E, int blo
   __syncthreads();
   if (leader) s_cnt[warp * E + id] = __popc(peers);
   constexpr int kBatch = 8;
-  for (int base = tid; base < numel; base += kBatch * kThreads) {
+  const bool alone = gridDim.x == 1;  // this CTA's slots are all there are
+  for (int base = tid; base < numel && !alone; base += kBatch * kThreads) {
     int v[kBatch];
 #pragma unroll
     for (int i = 0; i < kBatch; ++i) v[i] = base + i * kThreads < numel ? topk_ids[base + i * kThreads] : -1;
@@ -138,6 +139,7 @@ moe_align_kernel(const int32_t* __restrict__ topk_ids, int numel, int E, int blo
       s_cnt[w * E + e] = run;
       run += c;
     }
+    if (alone) s_total[e] = run;
   }
   __syncthreads();
   scan_experts<kWarps>(s_total, s_start, E, block, first ? num_post_pad : nullptr, first ? table : nullptr, token_tile, s_sum);

@@ -43,8 +43,8 @@ constexpr int ROW_BYTES = 1024;              // bytes of a weight row per stage
 constexpr int PIECES = ROW_BYTES / 128;
 constexpr int STAGE_BYTES = 16 * ROW_BYTES;  // [8 pieces of 128 bytes along K][16 rows], 128-byte swizzle
 constexpr int MAX_STAGES = kWarps;
-constexpr int kMaxRed = 64;                         // partial sums in flight (16 rows x 2, 4 or 8 tokens each)
-constexpr int HEAD_BYTES = 2048;                    // barriers, flags; then the partial sums
+constexpr int kMaxRed = 160;                        // partial sums in flight (16 rows x 2, 4 or 8 tokens each)
+constexpr int HEAD_BYTES = 4096;                    // barriers, flags; then the partial sums
 constexpr int kMaxSmem = 227 * 1024;
 constexpr int kMaxBlocks = 256;              // blocks <= slots = T * k <= 8 * 32
 constexpr int x_pitch(int64_t row_bytes) { return (int)((row_bytes + 127) / 128 * 128 + 64); }
@@ -640,7 +640,9 @@ bool plan_decode(const fmoe_fused_args& a, const RouteArgs& r, DecodePlan* pl) {
   // Partial sums in flight.  An epilogue warp may wait for the last stage of a unit n_epi units ahead of the oldest one
   // whose stages are still landing (at most two rounds of the ring): that span has to fit, or a parity would repeat.
   const int nst = (int)ceil_div<int64_t>(std::max(a.H, a.I) * eb, ROW_BYTES);
-  pl->n_red = kMaxRed;
+  // Rows of more than 9 stages get a longer ring, for four epilogue warps at work (one, with Mixtral's 28 stages per row of
+  // the down projection, took 213 us for one token).
+  pl->n_red = std::min(kMaxRed, std::max(64, 2 * MAX_STAGES + 4 + 4 * nst));
   pl->n_epi = std::min(kEpiWarps, (pl->n_red - 2 * MAX_STAGES - 4) / nst);
   if (pl->n_epi < 1) return false;
   pl->tp = a.T <= 2 ? 2 : (a.T <= 4 ? 4 : 8);
