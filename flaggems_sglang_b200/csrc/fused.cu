@@ -65,6 +65,23 @@ inline bool tc_gathers_input(int variant, int dtype) {
 }
 }
 
+// The whole layer on the CTA-pair GEMMs although an expert has few rows.  Both families read the weights once; the pair
+// kernels stream them 3-15 % faster but cost a row copy and a longer prologue, 5-15 us.  Measured per layer, stream / pairs
+// in us:
+//   e4m3            DeepSeek-V3 9 tokens 510 / 447, 64 tokens 1203 / 1031, a rank's quarter with 20 tokens 239 / 223
+//   not x128        (the streaming kernel masks its loads) GPT-OSS 9 tokens 257 / 220, half of it 135 / 126
+//   2.8 GB          Mixtral 4 tokens 364 / 360, 16 tokens 486 / 460
+//   1.2-1.5 GB      3 rows and more: Qwen3 52 tokens 210 / 205, reference shape 24 tokens 253 / 252; below: Qwen3 40 tokens
+//                   198 / 200, reference shape 17 tokens 232 / 235, 10 tokens 193 / 199
+//   0.6-0.7 GB      half of Qwen3, 64 tokens 119 / 134; a quarter of Mixtral, 12 tokens 137 / 140
+bool layer_prefers_pairs(const fmoe_fused_args& a, int64_t numel) {
+  if (a.dtype == FMOE_E4M3) return true;  // sizes are multiples of 128
+  if (a.H % 32 || a.I % 32) return false;
+  if (a.H % 128 || a.I % 128) return true;
+  const int64_t active = std::min<int64_t>(a.num_experts, numel), bytes = active * 6 * a.H * a.I;
+  return bytes >= 2400000000ll || (bytes >= 1200000000ll && numel >= 3 * active);
+}
+
 int plan_fused(const fmoe_fused_args& a, const RouteArgs& route, FusedPlan* pl) {
   if (a.struct_size != sizeof(fmoe_fused_args))
     return fail(FMOE_ERR_INVALID_ARG, "fused_experts: fmoe_fused_args.struct_size is %u, this library's struct has %zu "
@@ -106,9 +123,13 @@ int plan_fused(const fmoe_fused_args& a, const RouteArgs& route, FusedPlan* pl) 
   } else {
     rc = pick_variant(a.dtype, p.numel, a.num_experts, a.I, a.H, n_major ? FMOE_VARIANT_TCGEN05 : a.variant, &p.variant,
                       &p.block);
+    if (rc == FMOE_OK && a.variant == FMOE_VARIANT_AUTO && p.variant == FMOE_VARIANT_STREAM && layer_prefers_pairs(a, p.numel)) {
+      p.variant = FMOE_VARIANT_TCGEN05;
+      p.block = 128;
+    }
   }
   if (rc) return rc;
-  p.cap = p.numel + (int64_t)a.num_experts * (p.block - 1);
+  p.cap = p.numel + std::min<int64_t>(a.num_experts, p.numel) * (p.block - 1);
   p.nblk = ceil_div<int64_t>(p.cap, p.block);
   p.max_blocks = std::min<int64_t>(p.cap / p.block, p.numel);
   const int64_t eb = a.dtype == FMOE_F32 ? 4 : 2;  // element size of hidden / out / z

@@ -52,6 +52,16 @@ extern "C" int fmoe_fused_experts_static(const fmoe_fused_args* args, void* stre
   FusedPlan plan;
   int rc = plan_fused(*args, RouteArgs{}, &plan);
   if (rc) return rc;
+  fmoe_fused_args a = *args;
+  if (plan.total > kStaticScratchBytes && a.variant == FMOE_VARIANT_AUTO) {
+    // the streaming kernels need no padded copies: with few rows per expert their plan may fit where the faster one does not
+    int variant = 0, block = 0;
+    FusedPlan streamed;
+    a.variant = FMOE_VARIANT_STREAM;
+    if (pick_variant(a.dtype, a.T * a.top_k, a.num_experts, a.I, a.H, FMOE_VARIANT_STREAM, &variant, &block) == FMOE_OK &&
+        plan_fused(a, RouteArgs{}, &streamed) == FMOE_OK && streamed.total <= kStaticScratchBytes)
+      plan = streamed;
+  }
   if (plan.total > kStaticScratchBytes)
     return fail(FMOE_ERR_UNSUPPORTED,
                 "fused_experts_static: this problem needs %lld bytes of scratch, the built-in array holds %lld; "
@@ -61,5 +71,5 @@ extern "C" int fmoe_fused_experts_static(const fmoe_fused_args* args, void* stre
   uint8_t* scratch = nullptr;
   rc = static_scratch_for_current_device(&scratch);
   if (rc) return rc;
-  return run_fused(*args, RouteArgs{}, plan, scratch, stream);
+  return run_fused(a, RouteArgs{}, plan, scratch, stream);
 }
