@@ -10,8 +10,8 @@ torch or the CPU.
 
 Kernel selection (per call, from shapes only, no host sync):
   up to 8 tokens                 -> two decode kernels: routing and block list, then both GEMMs and the combine
-  rows per active expert <= 4    -> "stream" (e4m3: below 4): small-M weight-streaming kernel, moe_align block 8, x gathered
-                                    on the fly
+  few rows per active expert     -> "stream": small-M weight-streaming kernel, moe_align block 8, x gathered on the fly
+                                    (bf16 layers with little weight to read; see layer_prefers_pairs in csrc/fused.cu)
   larger                         -> "tcgen05": rows copied (e4m3: quantised) into expert-sorted order (block 128), TMA +
                                     tcgen05/TMEM persistent kernels on CTA pairs
   fp32 inputs                    -> "simt"

@@ -36,7 +36,9 @@ def _layer(T, H, I, E, seed):
 
 # rows per expert around the edges of 8-row groups and of the 64-, 128- and 256-token tiles; the mean picks the tile
 ROWS = {"64": [1, 0, 7, 8, 9, 15, 16, 17, 31, 33, 63, 64, 65, 80], "128": [1, 63, 64, 65, 127, 128, 129, 0],
-        "256": [1, 127, 129, 255, 256, 257, 400, 513]}
+        "256": [1, 127, 129, 255, 256, 257, 400, 513],
+        # e4m3 block scales: experts on both sides of the line between the narrow and the wide kernel
+        "mixed": [63, 64, 65, 0, 1, 300, 66, 17, 128]}
 
 
 @pytest.mark.parametrize("tile", ROWS)
@@ -152,3 +154,29 @@ def test_combine_slot_counts(fg, k):
         out = torch.empty(37, 264, dtype=dt, device="cuda")
         fg.moe_sum(z.to(dt).cuda(), out)
         assert torch.equal(out.cpu(), OE.moe_sum(z.to(dt)).to(dt))
+
+
+def test_static_entry_streams_what_does_not_fit(fg):
+    """e4m3 layers with few rows per expert take the padded tensor-core plan; the allocation-free entry keeps the streaming
+    one where only that fits its array."""
+    from flaggems_sglang_b200 import _C
+
+    E, H, I, k, T = 128, 2048, 512, 8, 16
+    g = torch.Generator(device="cuda").manual_seed(3)
+    x = torch.randn(T, H, generator=g, device="cuda").bfloat16()
+    w1 = (torch.randn(E, 2 * I, H, generator=g, device="cuda") * 0.5).to(torch.float8_e4m3fn)
+    w2 = (torch.randn(E, H, I, generator=g, device="cuda") * 0.5).to(torch.float8_e4m3fn)
+    s1 = torch.rand(E, 2 * I // 128, H // 128, generator=g, device="cuda") * 0.04
+    s2 = torch.rand(E, H // 128, I // 128, generator=g, device="cuda") * 0.04
+    tw, ids = fg.fused_topk(x, torch.randn(T, E, generator=g, device="cuda"), k, True)
+    kw = dict(use_fp8_w8a8=True, w1_scale=s1, w2_scale=s2, block_shape=[128, 128])
+    ref, auto = (fg.fused_experts(x, w1, w2, tw, ids, variant=v, **kw) for v in ("stream", None))
+    out = torch.empty_like(ref)
+    a = _C.FusedArgs(dtype=_C.E4M3, variant=_C.VARIANTS["auto"], num_experts=E, top_k=k, T=T, H=H, I=I, routed_scaling_factor=1.0,
+                     hidden=x.data_ptr(), w1=w1.data_ptr(), w2=w2.data_ptr(), w1_scale=s1.data_ptr(), w2_scale=s2.data_ptr(),
+                     topk_weights=tw.data_ptr(), topk_ids=ids.data_ptr(), out=out.data_ptr())
+    lib = _C.lib()
+    assert lib.fmoe_fused_experts_workspace_bytes(a) > lib.fmoe_static_scratch_bytes()
+    _C.check(lib.fmoe_fused_experts_static(a, _C.stream_ptr()))
+    assert torch.equal(out, ref)
+    assert_close_moe(auto, ref.cpu(), "fp8", "auto against stream")
