@@ -5,8 +5,12 @@
 // for another.  Slots of an expert keep their ascending order: position = expert's start + slots before this CTA + slots in
 // earlier warps + rank among the warp's equal ids (ballots).  Above that, three launches share the counting.
 #include "align.cuh"
+#include "ptx_sm100.cuh"
 
 namespace fmoe {
+
+__device__ int g_device_status_align = 0;  // this translation unit's status word; read by status_word_align()
+
 namespace {
 
 constexpr int kThreads = 1024;
@@ -284,10 +288,18 @@ align_scatter_kernel(const int32_t* __restrict__ topk_ids, int numel, int E, con
 // The same tables from slots that the caller already holds in expert order (the reference operator's routing triple:
 // sorted position -> slot, rows per expert, weights in sorted order): nothing is counted or sorted, every CTA scans the
 // E row counts and copies its share of the positions to their padded places.  Also writes expert and weight by slot.
+//
+// The triple is the caller's memory and only the device sees it.  Rows past the last position are clipped, a position whose
+// slot is outside [0, numel) is left out, and ids and slot_pos are -1 for a slot that no position names: no later kernel
+// forms an address from a word that was not written in this call.  Both misuses are recorded for fmoe_check_device_status.
+// The grid is one cluster, so that all of ids and slot_pos can be set to -1 before the first position is stored.
 // ---------------------------------------------------------------------------------------------
-constexpr int kSortedThreads = 256;
+constexpr int kSortedThreads = 1024;
+constexpr int kSortedCtas = 8;
 
-__global__ void __launch_bounds__(kSortedThreads)
+__device__ __forceinline__ void report_triple(int code) { atomicCAS(&g_device_status_align, 0, code); }
+
+__global__ void __cluster_dims__(kSortedCtas, 1, 1) __launch_bounds__(kSortedThreads)
 align_sorted_kernel(const int32_t* __restrict__ slot_of, const int32_t* __restrict__ hist, const float* __restrict__ gate, int numel,
                     int E, int block, int32_t* __restrict__ sorted_ids, int sorted_cap, int32_t* __restrict__ expert_ids,
                     int expert_cap, int32_t* __restrict__ num_post_pad, int32_t* __restrict__ table, int token_tile,
@@ -300,44 +312,57 @@ align_sorted_kernel(const int32_t* __restrict__ slot_of, const int32_t* __restri
   int* s_first = s_start + E + 1;  // [E+1] unpadded
   __shared__ int s_sum[2 * kSortedThreads / 32];
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, block_id = blockIdx.x;
-  for (int e = tid; e < E; e += kSortedThreads) s_total[e] = max(hist[e], 0);
+  constexpr int stride = kSortedCtas * kSortedThreads;
+  for (int i = block_id * kSortedThreads + tid; i < numel; i += stride) {
+    ids[i] = -1;
+    if (slot_pos) slot_pos[i] = -1;
+  }
+  for (int e = tid; e < E; e += kSortedThreads) s_total[e] = hist[e];
   __syncthreads();
-  scan_experts<kSortedThreads / 32>(s_total, s_start, E, block, block_id == 0 ? num_post_pad : nullptr,
-                                    block_id == 0 ? table : nullptr, token_tile, s_sum);
-  if (warp == 1) {
+  // Rows of every expert, and its first position: a prefix sum that stays at numel once it gets there (terms and sums are at
+  // most numel < 2^30, so nothing overflows), so that the rows of all experts together are at most numel.
+  if (warp == 0) {
     int carry = 0;
+    bool over = false;
     for (int base = 0; base < E; base += 32) {
-      const int e = base + lane, v = e < E ? s_total[e] : 0;
+      const int e = base + lane, given = e < E ? s_total[e] : 0, v = min(max(given, 0), numel);
       int incl = v;
 #pragma unroll
       for (int off = 1; off < 32; off <<= 1) {
         const int w = __shfl_up_sync(0xffffffffu, incl, off);
-        if (lane >= off) incl += w;
+        if (lane >= off) incl = min(incl + w, numel);
       }
-      if (e < E) s_first[e] = carry + incl - v;
-      carry += __shfl_sync(0xffffffffu, incl, 31);
+      incl = min(carry + incl, numel);
+      int first = __shfl_up_sync(0xffffffffu, incl, 1);
+      if (lane == 0) first = carry;
+      if (e < E) {
+        s_first[e] = first;
+        s_total[e] = incl - first;
+        over |= incl - first != given;
+      }
+      carry = __shfl_sync(0xffffffffu, incl, 31);
     }
     if (lane == 0) s_first[E] = carry;
+    if (over && block_id == 0) report_triple(0xB01);
   }
   __syncthreads();
-  const int stride = gridDim.x * kSortedThreads;
+  scan_experts<kSortedThreads / 32>(s_total, s_start, E, block, block_id == 0 ? num_post_pad : nullptr,
+                                    block_id == 0 ? table : nullptr, token_tile, s_sum);
+  ptx::cluster_sync_all();
   for (int p = block_id * kSortedThreads + tid; p < numel; p += stride) {
     const int slot = slot_of[p];
-    if (slot < 0 || slot >= numel) continue;
-    if (p >= s_first[E]) {  // a histogram that does not cover every position: the rest belongs to no expert
-      ids[slot] = -1;
-      weights[slot] = 0.f;
-      if (slot_pos) slot_pos[slot] = -1;
-      continue;
-    }
-    int lo = 0, hi = E - 1;  // last expert that starts at or before p
+    const bool named = slot >= 0 && slot < numel;
+    if (!named) report_triple(0xB00);
+    if (p >= s_first[E]) continue;  // a histogram that does not cover every position: the rest belongs to no expert
+    int lo = 0, hi = E - 1;         // last expert that starts at or before p
     while (lo < hi) {
       const int mid = (lo + hi + 1) >> 1;
       if (s_first[mid] <= p) lo = mid;
       else hi = mid - 1;
     }
     const int pos = s_start[lo] + p - s_first[lo];
-    if (pos < sorted_cap && sorted_ids) sorted_ids[pos] = slot;
+    if (sorted_ids) sorted_ids[pos] = named ? slot : numel;  // pos < sorted_cap: at most numel rows (check_align)
+    if (!named) continue;
     if (slot_pos) slot_pos[slot] = pos;
     ids[slot] = lo;
     weights[slot] = gate[p];
@@ -409,12 +434,17 @@ int run_align_sorted(const AlignArgs& a, const SortedSlots& s, cudaStream_t st) 
     const int rc = check_align(a);
     if (rc) return rc;
   }
-  const int64_t items = std::max(a.numel, a.sorted_ids && !a.rows_only ? a.sorted_cap / 4 : 0);
-  const unsigned grid = (unsigned)std::min<int64_t>(ceil_div<int64_t>(items, kSortedThreads), 148);
-  launch_pdl(align_sorted_kernel, dim3(grid), dim3(kSortedThreads), (3 * (size_t)a.E + 2) * sizeof(int), st, s.slot_of, s.hist, s.gate,
+  launch_pdl(align_sorted_kernel, dim3(kSortedCtas), dim3(kSortedThreads), (3 * (size_t)a.E + 2) * sizeof(int), st, s.slot_of, s.hist, s.gate,
              (int)a.numel, a.E, a.block, a.sorted_ids, (int)a.sorted_cap, a.expert_ids, (int)a.expert_cap, a.num_post_pad, a.table,
              a.token_tile, a.zero_words, a.num_zero, s.ids, s.weights, a.slot_pos, (int)a.rows_only);
   return launch_status("align_sorted_kernel");
+}
+
+int status_word_align(int* out, bool clear) {
+  int zero = 0;
+  FMOE_CUDA_OK(cudaMemcpyFromSymbol(out, g_device_status_align, sizeof(int)));
+  if (clear && *out != 0) FMOE_CUDA_OK(cudaMemcpyToSymbol(g_device_status_align, &zero, sizeof(int)));
+  return FMOE_OK;
 }
 
 }  // namespace fmoe

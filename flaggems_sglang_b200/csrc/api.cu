@@ -170,6 +170,10 @@ extern "C" int fmoe_check_device_status(void* stream) {
     return fmoe::fail(FMOE_ERR_INVALID_ARG,
                       "expert-parallel exchange skipped rows (site code 0x%x: 0xA00 expert id out of range, "
                       "0xA01 receive capacity exceeded, 0xA02 bad return address)", status);
+  if ((status & 0xF00) == 0xB00)
+    return fmoe::fail(FMOE_ERR_INVALID_ARG,
+                      "a routing triple was inconsistent (site code 0x%x: 0xB00 sorted position with a slot out of range, "
+                      "0xB01 more rows in the histogram than positions, or a negative count)", status);
   if (status != 0)
     return fmoe::fail(FMOE_ERR_DEVICE_TIMEOUT, "a bounded wait inside a tcgen05 kernel gave up (site code 0x%x)", status);
   return FMOE_OK;

@@ -308,6 +308,11 @@ int fmoe_fused_moe(const fmoe_fused_args* args, const fmoe_route_args* route, vo
  * fmoe_fused_experts for a routing that is already in expert order, as the reference operator takes it
  * (src/flaggems_sglang/ops/fused_moe.py:119-146): topk_indx [T*k] sorted position -> flat slot, expt_hist [E] rows per
  * expert, gate_scal [T*k] weights in sorted order; args->topk_weights / topk_ids are ignored.
+ *
+ * topk_indx is a permutation of [0, T*k) and the counts sum to at most T*k (positions past the sum belong to no expert).
+ * Only the device sees whether they do: a slot outside the range is left out, counts are clipped to the positions that are
+ * left, and fmoe_check_device_status returns FMOE_ERR_INVALID_ARG afterwards.  Nothing outside the buffers is touched then;
+ * the output rows of tokens that have a slot no position names, or two name, are unspecified, all other rows are right.
  */
 int64_t fmoe_fused_experts_sorted_workspace_bytes(const fmoe_fused_args* args);
 int fmoe_fused_experts_sorted(const fmoe_fused_args* args, const int32_t* topk_indx, const int32_t* expt_hist,
@@ -398,8 +403,8 @@ int fmoe_ep_scatter_rows(const void* z_rows, int64_t row_bytes, void* const* out
 
 /*
  * Reads and clears the device-side status word that bounded waits inside the
- * tcgen05 kernels set when they give up, and the one of the expert-parallel
- * exchange kernels.  Synchronises `stream`.
+ * tcgen05 and decode kernels set when they give up, and those of the expert-parallel
+ * exchange kernels and of fmoe_fused_experts_sorted.  Synchronises `stream`.
  * Returns FMOE_OK, FMOE_ERR_DEVICE_TIMEOUT or FMOE_ERR_INVALID_ARG.
  */
 int fmoe_check_device_status(void* stream);

@@ -146,6 +146,59 @@ def test_sorted_routing_equals_routing_by_slot(fg, T):
     assert torch.equal(rows, ref)
 
 
+@pytest.mark.parametrize("T", [2, 30, 700, 3000])
+@pytest.mark.parametrize("fault", ["slot", "duplicate", "hist_over", "hist_negative", "hist_short"])
+def test_inconsistent_triple_stays_inside_its_buffers(fg, fault, T):
+    """Entries of a routing triple that only the device sees: the workspace is filled with words that would be addresses if a
+    kernel took one for a position, and lies between guard bytes.  Tokens whose slots are all named once keep their rows."""
+    from flaggems_sglang_b200 import _C
+
+    E, H, I, k = 24, 256, 192, 3
+    x, w1, w2, g = _layer(T, H, I, E, 70 + T)
+    tw, ids = OR.softmax_topk(torch.randn(T, E, generator=g), k, True)
+    xd, w1d, w2d = x.cuda(), w1.cuda(), w2.cuda()
+    rd, gi, si = fg.standard_topk_to_routing(tw.cuda(), ids.cuda(), E)
+    good = fg.triton_kernel_fused_experts(xd, w1d.transpose(1, 2), w2d.transpose(1, 2), rd, gi, si)
+    slot_of, hist, gate = gi.src_indx.clone(), rd.expt_hist.clone(), rd.gate_scal.contiguous()
+    numel, hit = T * k, torch.zeros(T, dtype=torch.bool)
+    where = [0, numel // 2, numel - 1]
+    if fault == "slot":
+        for p, bad in zip(where, (-7, numel, 2**31 - 1)):
+            hit[int(slot_of[p]) // k] = True
+            slot_of[p] = bad
+    elif fault == "duplicate":
+        for p in where[1:]:
+            hit[int(slot_of[p]) // k] = hit[int(slot_of[0]) // k] = True
+            slot_of[p] = slot_of[0]
+    elif fault == "hist_over":  # the last experts run past the positions: their rows are clipped
+        hist[E - 1] += 2**30
+    elif fault == "hist_negative":
+        hit[:] = True  # every later expert's rows move
+        hist[1] -= 2**31 - 1 - int(hist[1])
+    else:
+        cut = int(hist[hist.nonzero()[-1, 0]])
+        hist[hist.nonzero()[-1, 0]] = 0
+        hit[(slot_of[numel - cut:] // k).long().cpu()] = True
+    lib, out = _C.lib(), torch.empty_like(xd)
+    a = _C.FusedArgs(dtype=_C.BF16, num_experts=E, top_k=k, T=T, H=H, I=I, routed_scaling_factor=1.0, hidden=xd.data_ptr(),
+                     w1=w1d.data_ptr(), w2=w2d.data_ptr(), out=out.data_ptr())
+    need = lib.fmoe_fused_experts_sorted_workspace_bytes(a)
+    guard = 1 << 20
+    area = torch.full(((need + 2 * guard) // 4 + 64,), 0x3F000000, dtype=torch.int32, device="cuda")
+    start = -(-(area.data_ptr() + guard) // 256) * 256
+    a.workspace, a.workspace_bytes = start, need
+    before = [t.clone() for t in (xd, w1d, w2d)]
+    _C.check(lib.fmoe_fused_experts_sorted(a, slot_of.data_ptr(), hist.data_ptr(), gate.data_ptr(), _C.stream_ptr()))
+    torch.cuda.synchronize()
+    lo = (start - area.data_ptr()) // 4
+    assert bool((area[:lo] == 0x3F000000).all()) and bool((area[lo + -(-need // 4):] == 0x3F000000).all())
+    assert all(torch.equal(u, v) for u, v in zip(before, (xd, w1d, w2d)))
+    assert torch.equal(out[~hit.cuda()], good[~hit.cuda()])
+    if fault in ("slot", "hist_over", "hist_negative"):
+        with pytest.raises(_C.FmoeError, match="0xB00" if fault == "slot" else "0xB01"):
+            _C.check_device_status()
+
+
 @pytest.mark.parametrize("k", [1, 2, 3, 4, 5, 9])
 def test_combine_slot_counts(fg, k):
     """moe_sum issues the loads of up to 2 or 4 slots before the first is added."""
