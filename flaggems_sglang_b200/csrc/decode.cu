@@ -22,8 +22,13 @@
 // counter round trip last longer than a unit's stages and would hold the compute warps up.  A stage is brought by one TMA
 // box of 16 KB.  The tokens' rows (later the expert's activations) stay in shared memory beside the ring.
 //
-// The CTAs of decode_layer_kernel wait on one another's counters: there is at most one per SM and all of them are
-// resident, every wait is bounded, and on expiry the status word is set and the CTA finishes without the result.
+// The CTAs of decode_layer_kernel wait on one another's counters, and nothing says that all of them are resident: another
+// stream's kernels may hold SMs.  So the work is cut into one share per CTA and GEMM, and a CTA takes its shares from a
+// counter, all gate/up shares before the first down share.  Only down shares wait, and whoever waits holds a ticket above
+// every gate/up share, so that all of those belong to CTAs that run; a CTA that starts late finds less left to take.  (The
+// ticket is asked for together with the block list, whose latency hides it.  One token, fixed shares / tickets: Qwen3 27.5 /
+// 27.2 us per call, DeepSeek-V3 77.9 / 78.7.)  Every wait is bounded; on expiry the status word is set and the CTA finishes
+// without the result.
 #include "decode.cuh"
 #include "fused.cuh"
 #include "pair.cuh"
@@ -44,7 +49,10 @@ constexpr int PIECES = ROW_BYTES / 128;
 constexpr int STAGE_BYTES = 16 * ROW_BYTES;  // [8 pieces of 128 bytes along K][16 rows], 128-byte swizzle
 constexpr int MAX_STAGES = kWarps;
 constexpr int kMaxRed = 160;                        // partial sums in flight (16 rows x 2, 4 or 8 tokens each)
-constexpr int HEAD_BYTES = 4096;                    // barriers, flags; then the partial sums
+constexpr int HEAD_BYTES = 4096;                    // barriers, flags, tickets; then the partial sums
+constexpr int kMaxShares = 160;                     // shares of a GEMM, at most: one per CTA
+constexpr int kHeadWords = 4 + 2 * kMaxShares + 1;  // flag, the compute warps' ticket (two in turn), all tickets a CTA can hold
+static_assert((2 * kWarps + 2 * kMaxRed) * 8 + kHeadWords * 4 <= HEAD_BYTES, "shared memory");
 constexpr int kMaxSmem = 227 * 1024;
 constexpr int kMaxBlocks = 256;              // blocks <= slots = T * k <= 8 * 32
 constexpr int x_pitch(int64_t row_bytes) { return (int)((row_bytes + 127) / 128 * 128 + 64); }
@@ -191,8 +199,9 @@ struct LayerParams {
   __nv_bfloat16* out;      // [T, H]
   int32_t* ready;          // per block: gate/up units done
   int32_t* done;           // per 16-channel slab: down units done
+  int32_t* tickets;        // next share: gate/up [0, shares), down [shares, 2 shares)
   int64_t H, I;
-  int T, k, E;
+  int T, k, E, shares;
   int on_input, activation, no_combine;
   float act_alpha, act_limit, scale;
   int stages, x_bytes;
@@ -255,7 +264,9 @@ decode_layer_kernel(const __grid_constant__ CUtensorMap map1, const __grid_const
   uint64_t* empty_bar = full_bar + MAX_STAGES;
   uint64_t* red_full = empty_bar + MAX_STAGES;    // [n_red] compute warp -> epilogue warp
   uint64_t* red_empty = red_full + kMaxRed;       // [n_red] epilogue warp -> compute warp
-  int32_t* flag = reinterpret_cast<int32_t*>(red_empty + kMaxRed);  // [0] a wait for activations gave up
+  volatile int32_t* flag = reinterpret_cast<int32_t*>(red_empty + kMaxRed);  // [0] a wait for activations gave up
+  volatile int32_t* seen = flag + 2;     // [2] the compute warps' ticket, in turn
+  volatile int32_t* tickets = flag + 4;  // this CTA's tickets, -1: not taken yet
   float* red = reinterpret_cast<float*>(smem + HEAD_BYTES);
   uint8_t* x_smem = smem + HEAD_BYTES + p.red_bytes;
   const uint32_t x_addr = ptx::smem_u32(x_smem);
@@ -280,31 +291,65 @@ decode_layer_kernel(const __grid_constant__ CUtensorMap map1, const __grid_const
     flag[0] = 0;
     ptx::fence_barrier_init();
   }
+  for (int i = threadIdx.x; i <= 2 * kMaxShares; i += kThreads) tickets[i] = -1;
   __syncthreads();
   pdl_entry();
+  int ticket0 = 0;
+  if (warp == kWarps && lane == 0) ticket0 = atomicAdd(p.tickets, 1);
   const int blocks = p.plan[0];
-  // This CTA's units.  Gate/up: every gridDim-th one, so that all CTAs work on one expert after the other and at the end
-  // only the last expert's activations are still to come.  Down: a contiguous share, so that a CTA sees few experts.
-  const int units1 = (int)(p.I / 8), units2 = (int)(p.H / 16);
-  const int64_t total1 = (int64_t)blocks * units1, total2 = (int64_t)blocks * units2;
-  const int cta = (int)blockIdx.x, ctas = (int)gridDim.x;
-  const int n1 = cta < total1 ? (int)((total1 - cta + ctas - 1) / ctas) : 0;
+  // Units of a share.  Gate/up: every shares-th one, so that all CTAs work on one expert after the other and at the end
+  // only the last expert's activations are still to come.  Down: a contiguous piece, so that a CTA sees few experts.
+  const int units1 = (int)(p.I / 8), units2 = (int)(p.H / 16), shares = p.shares;
   const int pieces1 = (int)(p.H * EB / 128), pieces2 = (int)(p.I * EB / 128);
   const int nst1 = (pieces1 + PIECES - 1) / PIECES, nst2 = (pieces2 + PIECES - 1) / PIECES;  // stages per unit
-  const int lo2 = (int)(total2 * cta / ctas), n2 = (int)(total2 * (cta + 1) / ctas) - lo2;
-  auto unit_of = [&](int gemm, int i) { return gemm ? lo2 + i : cta + i * ctas; };  // the CTA's i-th unit
+  struct Share {
+    int gemm, first, step, count;
+    __device__ __forceinline__ int unit(int i) const { return first + i * step; }
+  };
+  auto share_of = [&](int ticket) {
+    // at most 256 blocks, and a token's row fits shared memory: units * shares stays far below 2^31
+    const int total1 = blocks * units1, total2 = blocks * units2;
+    Share s;
+    s.gemm = ticket >= shares;
+    const int v = ticket - s.gemm * shares;
+    s.first = s.gemm ? total2 * v / shares : v;
+    s.step = s.gemm ? 1 : shares;
+    s.count = s.gemm ? total2 * (v + 1) / shares - s.first : (v < total1 ? (total1 - v + shares - 1) / shares : 0);
+    return s;
+  };
+  // The CTA's idx-th ticket; 2 * shares or more: it has no further share.  Bounded like every wait.
+  auto wait_ticket = [&](int idx) {
+    const long long t0 = clock64();
+    int t;
+    while ((t = tickets[idx]) < 0) {
+      if (clock64() - t0 > ptx::kWaitCycles) {
+        report(0xC44);
+        return 2 * shares;
+      }
+    }
+    return t;
+  };
 
   if (warp == kWarps) {
-    // ---------------- producer: weight rows of the gate/up units, then of the down units ----------------
+    // ---------------- producer: weight rows of the CTA's shares ----------------
+    ticket0 = __shfl_sync(0xffffffffu, ticket0, 0);
     if (ptx::elect_one()) {
       int stage = 0;
       uint32_t phase = 0;
       bool alive = true;
+      int ticket = ticket0;
 #pragma unroll 1
-      for (int gemm = 0; gemm < 2 && alive; ++gemm) {
-        const int units = gemm ? units2 : units1, count = gemm ? n2 : n1, pieces = gemm ? pieces2 : pieces1;
-        for (int i = 0; i < count && alive; ++i) {
-          const int u = unit_of(gemm, i);
+      for (int idx = 0;; ++idx) {
+        if (!alive) ticket = 2 * shares;
+        tickets[idx] = ticket;
+        if (ticket >= 2 * shares) break;
+        const Share sh = share_of(ticket);
+        const int units = sh.gemm ? units2 : units1, pieces = sh.gemm ? pieces2 : pieces1;
+        int next = -1;
+        for (int i = 0; i < sh.count && alive; ++i) {
+          // not earlier, or a CTA would take a gate/up share from one that is just starting
+          if (i == sh.count - 1) next = atomicAdd(p.tickets, 1);
+          const int u = sh.unit(i);
           const int e = p.plan[plan_expert(u / units)], s = u % units;
           for (int piece = 0; piece < pieces; piece += PIECES) {  // pieces past the row's end arrive as zeros
             if (!ptx::mbar_wait(&empty_bar[stage], phase ^ 1)) {
@@ -313,7 +358,7 @@ decode_layer_kernel(const __grid_constant__ CUtensorMap map1, const __grid_const
               break;
             }
             ptx::mbar_arrive_expect_tx(&full_bar[stage], STAGE_BYTES);
-            if (gemm == 0) tma_load_5d(ring + stage * STAGE_BYTES, &map1, 0, 0, 2 * e, s, piece, &full_bar[stage]);
+            if (sh.gemm == 0) tma_load_5d(ring + stage * STAGE_BYTES, &map1, 0, 0, 2 * e, s, piece, &full_bar[stage]);
             else tma_load_4d(ring + stage * STAGE_BYTES, &map2, 0, 0, e * units2 + s, piece, &full_bar[stage]);
             if (++stage == stages) {
               stage = 0;
@@ -321,6 +366,8 @@ decode_layer_kernel(const __grid_constant__ CUtensorMap map1, const __grid_const
             }
           }
         }
+        if (sh.count == 0) next = atomicAdd(p.tickets, 1);
+        ticket = next;
       }
       if (alive) {  // our own bulk copies have landed and been read before the CTA may end
         for (int s = 0; s < stages; ++s) {
@@ -339,93 +386,104 @@ decode_layer_kernel(const __grid_constant__ CUtensorMap map1, const __grid_const
   }
 
   if (warp > kWarps) {
-    // ---------------- epilogue warps: units me, me + 4, ... of this CTA, gate/up then down ----------------
+    // ---------------- epilogue warps: units me, me + n_epi, ... of this CTA ----------------
     const int me = warp - kWarps - 1;
     bool ok = true;
     if (blocks == 0 && !p.no_combine)  // no slot has an expert: the sums are empty
       for (int64_t i = (int64_t)blockIdx.x * (kEpiWarps * 32) + me * 32 + lane; i < p.T * p.H; i += (int64_t)gridDim.x * (kEpiWarps * 32))
         p.out[i] = __float2bfloat16_rn(0.f);
-    for (int n = me; n < n1 + n2 && me < p.n_epi && ok; n += p.n_epi) {
-      const int gemm = n >= n1, units = gemm ? units2 : units1, u = unit_of(gemm, gemm ? n - n1 : n);
-      const int block = u / units, s = u % units;
-      const int expert = p.plan[plan_expert(block)], rows = p.plan[plan_rows(block)];
-      // what the outputs need besides the sums, fetched while the stages are still landing: this lane's outputs are
-      // o = lane + 32 i of [8 channels | 16 rows][tp tokens]
-      const int outs = (gemm ? 16 : 8) * p.tp, tok_i = lane & (p.tp - 1), row_i = lane / p.tp, row_step = 32 / p.tp;
-      const int32_t slot = tok_i < rows ? p.plan[plan_slot(block, tok_i)] : -1;
-      const float wt = (slot >= 0 && p.on_input == !gemm) ? p.topk_w[slot] : 1.0f;
-      // the unit's partial sums, in stage order
-      const uint32_t q0 = gemm ? (uint32_t)(n1 * nst1 + (n - n1) * nst2) : (uint32_t)(n * nst1);
-      const int nst = gemm ? nst2 : nst1;
-      float sum[4] = {0.f, 0.f, 0.f, 0.f}, sum_up[2] = {0.f, 0.f};
-      for (int st = 0; st < nst; ++st) {
-        const uint32_t q = q0 + st;
-        ok = __all_sync(0xffffffffu, ptx::mbar_wait(&red_full[q % n_red], (q / n_red) & 1));
-        if (!ok) {
-          report(0xC10 | me);
-          break;
-        }
-        const float* part = red + (q % n_red) * 16 * p.tp;
+    if (me >= p.n_epi) return;
+    int turn = me;        // units of this CTA until this warp's next one
+    uint32_t q_base = 0;  // stages before the share
+#pragma unroll 1
+    for (int idx = 0; ok; ++idx) {
+      const int ticket = __shfl_sync(0xffffffffu, wait_ticket(idx), 0);
+      if (ticket >= 2 * shares) break;
+      const Share sh = share_of(ticket);
+      const int gemm = sh.gemm, units = gemm ? units2 : units1, nst = gemm ? nst2 : nst1;
+#pragma unroll 1
+      for (; turn < sh.count && ok; turn += p.n_epi) {
+        const int u = sh.unit(turn), block = u / units, s = u % units;
+        const int expert = p.plan[plan_expert(block)], rows = p.plan[plan_rows(block)];
+        // what the outputs need besides the sums, fetched while the stages are still landing: this lane's outputs are
+        // o = lane + 32 i of [8 channels | 16 rows][tp tokens]
+        const int outs = (gemm ? 16 : 8) * p.tp, tok_i = lane & (p.tp - 1), row_i = lane / p.tp, row_step = 32 / p.tp;
+        const int32_t slot = tok_i < rows ? p.plan[plan_slot(block, tok_i)] : -1;
+        const float wt = (slot >= 0 && p.on_input == !gemm) ? p.topk_w[slot] : 1.0f;
+        // the unit's partial sums, in stage order
+        const uint32_t q0 = q_base + (uint32_t)(turn * nst);
+        float sum[4] = {0.f, 0.f, 0.f, 0.f}, sum_up[2] = {0.f, 0.f};
+        for (int st = 0; st < nst; ++st) {
+          const uint32_t q = q0 + st;
+          ok = __all_sync(0xffffffffu, ptx::mbar_wait(&red_full[q % n_red], (q / n_red) & 1));
+          if (!ok) {
+            report(0xC10 | me);
+            break;
+          }
+          const float* part = red + (q % n_red) * 16 * p.tp;
 #pragma unroll
-        for (int i = 0; i < 4; ++i)
-          if (lane + 32 * i < outs) sum[i] += part[lane + 32 * i];
+          for (int i = 0; i < 4; ++i)
+            if (lane + 32 * i < outs) sum[i] += part[lane + 32 * i];
+          if (gemm == 0) {
+#pragma unroll
+            for (int i = 0; i < 2; ++i)
+              if (lane + 32 * i < outs) sum_up[i] += part[8 * p.tp + lane + 32 * i];
+          }
+          __syncwarp();
+          if (lane == 0) ptx::mbar_arrive(&red_empty[q % n_red]);
+        }
+        if (!ok) break;
         if (gemm == 0) {
 #pragma unroll
-          for (int i = 0; i < 2; ++i)
-            if (lane + 32 * i < outs) sum_up[i] += part[8 * p.tp + lane + 32 * i];
-        }
-        __syncwarp();
-        if (lane == 0) ptx::mbar_arrive(&red_empty[q % n_red]);
-      }
-      if (!ok) break;
-      if (gemm == 0) {
-#pragma unroll
-        for (int i = 0; i < 2; ++i) {
-          if (slot >= 0 && lane + 32 * i < outs) {
-            const int64_t ch = (int64_t)s * 8 + row_i + row_step * i;
-            const float* bias = p.b1 ? p.b1 + (int64_t)expert * 2 * p.I + ch : nullptr;
-            const float o = gated_output<false>(sum[i], sum_up[i], bias ? bias[0] : 0.f, bias ? bias[p.I] : 0.f, wt, p.activation,
-                                                p.act_alpha, p.act_limit);
-            const int64_t at = ((int64_t)block * 8 + tok_i) * p.I + ch;
-            if constexpr (EB == 2) reinterpret_cast<__nv_bfloat16*>(p.act)[at] = __float2bfloat16_rn(o);
-            else reinterpret_cast<float*>(p.act)[at] = o;
-          }
-        }
-        __threadfence();  // the activations are visible device-wide before the unit counts
-        __syncwarp();
-        if (lane == 0) atomicAdd(p.ready + block, 1);
-      } else {
-#pragma unroll
-        for (int i = 0; i < 4; ++i) {
-          if (slot >= 0 && lane + 32 * i < outs) {
-            const int64_t ch = (int64_t)s * 16 + row_i + row_step * i;
-            p.z[(int64_t)slot * p.H + ch] = __float2bfloat16_rn((sum[i] + (p.b2 ? p.b2[(int64_t)expert * p.H + ch] : 0.f)) * wt);
-          }
-        }
-        if (p.no_combine) continue;
-        __threadfence();
-        __syncwarp();
-        int last = 0;
-        if (lane == 0) last = atomicAdd(p.done + s, 1) == blocks - 1;
-        if (__shfl_sync(0xffffffffu, last, 0)) {
-          // the slab's last unit: out[t] = sum over the token's slots, in slot order
-          __threadfence();
-          for (int i = lane; i < p.T * 16; i += 32) {
-            const int tok = i >> 4;
-            const int64_t ch = (int64_t)s * 16 + (i & 15);
-            float a = 0.f;
-#pragma unroll 8
-            for (int j = 0; j < p.k; ++j) {
-              const int sl = tok * p.k + j, e = p.ids[sl];
-              const unsigned short v = __ldcg(reinterpret_cast<const unsigned short*>(p.z) + (int64_t)sl * p.H + ch);
-              if (e >= 0 && e < p.E) a += __bfloat162float(__ushort_as_bfloat16(v));
+          for (int i = 0; i < 2; ++i) {
+            if (slot >= 0 && lane + 32 * i < outs) {
+              const int64_t ch = (int64_t)s * 8 + row_i + row_step * i;
+              const float* bias = p.b1 ? p.b1 + (int64_t)expert * 2 * p.I + ch : nullptr;
+              const float o = gated_output<false>(sum[i], sum_up[i], bias ? bias[0] : 0.f, bias ? bias[p.I] : 0.f, wt, p.activation,
+                                                  p.act_alpha, p.act_limit);
+              const int64_t at = ((int64_t)block * 8 + tok_i) * p.I + ch;
+              if constexpr (EB == 2) reinterpret_cast<__nv_bfloat16*>(p.act)[at] = __float2bfloat16_rn(o);
+              else reinterpret_cast<float*>(p.act)[at] = o;
             }
-            __nv_bfloat16 o = __float2bfloat16_rn(a);
-            if (p.scale != 1.0f) o = __float2bfloat16_rn(__bfloat162float(o) * p.scale);
-            p.out[(int64_t)tok * p.H + ch] = o;
+          }
+          __threadfence();  // the activations are visible device-wide before the unit counts
+          __syncwarp();
+          if (lane == 0) atomicAdd(p.ready + block, 1);
+        } else {
+#pragma unroll
+          for (int i = 0; i < 4; ++i) {
+            if (slot >= 0 && lane + 32 * i < outs) {
+              const int64_t ch = (int64_t)s * 16 + row_i + row_step * i;
+              p.z[(int64_t)slot * p.H + ch] = __float2bfloat16_rn((sum[i] + (p.b2 ? p.b2[(int64_t)expert * p.H + ch] : 0.f)) * wt);
+            }
+          }
+          if (p.no_combine) continue;
+          __threadfence();
+          __syncwarp();
+          int last = 0;
+          if (lane == 0) last = atomicAdd(p.done + s, 1) == blocks - 1;
+          if (__shfl_sync(0xffffffffu, last, 0)) {
+            // the slab's last unit: out[t] = sum over the token's slots, in slot order
+            __threadfence();
+            for (int i = lane; i < p.T * 16; i += 32) {
+              const int tok = i >> 4;
+              const int64_t ch = (int64_t)s * 16 + (i & 15);
+              float a = 0.f;
+#pragma unroll 8
+              for (int j = 0; j < p.k; ++j) {
+                const int sl = tok * p.k + j, e = p.ids[sl];
+                const unsigned short v = __ldcg(reinterpret_cast<const unsigned short*>(p.z) + (int64_t)sl * p.H + ch);
+                if (e >= 0 && e < p.E) a += __bfloat162float(__ushort_as_bfloat16(v));
+              }
+              __nv_bfloat16 o = __float2bfloat16_rn(a);
+              if (p.scale != 1.0f) o = __float2bfloat16_rn(__bfloat162float(o) * p.scale);
+              p.out[(int64_t)tok * p.H + ch] = o;
+            }
           }
         }
       }
+      turn -= sh.count;
+      q_base += (uint32_t)(sh.count * nst);
     }
     return;
   }
@@ -433,16 +491,22 @@ decode_layer_kernel(const __grid_constant__ CUtensorMap map1, const __grid_const
   // ---------------- compute warps ----------------
   const int tid = threadIdx.x, g = lane >> 2, t = lane & 3;
   bool ok = true;
+  uint32_t q_base = 0;  // stages before the share
 #pragma unroll 1
-  for (int gemm = 0; gemm < 2; ++gemm) {
-    const int units = gemm ? units2 : units1, count = gemm ? n2 : n1, nst = gemm ? nst2 : nst1;
+  for (int idx = 0;; ++idx) {
+    // One thread waits for the ticket, so that all compute warps act on the same one, also when it does not come
+    if (tid == 0) seen[idx & 1] = wait_ticket(idx);
+    compute_barrier();
+    const int ticket = seen[idx & 1];
+    if (ticket >= 2 * shares) break;
+    const Share sh = share_of(ticket);
+    const int gemm = sh.gemm, units = gemm ? units2 : units1, count = sh.count, nst = gemm ? nst2 : nst1;
     const int pieces = gemm ? pieces2 : pieces1, kblocks = (int)((gemm ? p.I : p.H) / 128);
-    const uint32_t row_bytes = (uint32_t)pieces * 128, q_base = gemm ? (uint32_t)(n1 * nst1) : 0u;
+    const uint32_t row_bytes = (uint32_t)pieces * 128;
     const int xp = x_pitch(row_bytes);
     float* x_scale = nullptr;  // e4m3: scales of the rows in shared memory, [row][kblocks]
     if constexpr (EB == 1) x_scale = reinterpret_cast<float*>(x_smem + p.T * xp);
-    if (gemm == 0 && count > 0) {
-      // the tokens' rows, once
+    if (gemm == 0 && idx == 0) {  // the tokens' rows, once: all gate/up shares come before the first down share
       const int vecs = (int)(row_bytes / 16);
       for (int i = tid; i < p.T * vecs; i += kWarps * 32) {
         const int r = i / vecs, c = i % vecs;
@@ -456,9 +520,9 @@ decode_layer_kernel(const __grid_constant__ CUtensorMap map1, const __grid_const
     // gate/up: all units in one go; down: block by block, each with its expert's activations in shared memory
 #pragma unroll 1
     for (int seg = 0; seg < count;) {
-      const int seg_end = gemm ? min(count, ((lo2 + seg) / units + 1) * units - lo2) : count;
+      const int seg_end = gemm ? min(count, (sh.unit(seg) / units + 1) * units - sh.first) : count;
       if (gemm == 1) {
-        const int block = (lo2 + seg) / units, rows = p.plan[plan_rows(block)];
+        const int block = sh.unit(seg) / units, rows = p.plan[plan_rows(block)];
         if (tid == 0) {  // every gate/up unit of the block has been published
           const long long t0 = clock64();
           while (ld_acquire(p.ready + block) < units1) {
@@ -469,7 +533,7 @@ decode_layer_kernel(const __grid_constant__ CUtensorMap map1, const __grid_const
             }
           }
         }
-        compute_barrier();  // also: the previous block's rows have been read by everyone
+        compute_barrier();  // also: the token rows, or the previous block's, have been read by everyone
         if (flag[0]) ok = false;
         if constexpr (EB == 2) {
           const int vecs = (int)(row_bytes / 16);
@@ -504,7 +568,7 @@ decode_layer_kernel(const __grid_constant__ CUtensorMap map1, const __grid_const
       // stage q lands in ring slot q % stages and belongs to the warp of that number
 #pragma unroll 1
       for (uint32_t q = first + (warp + stages - first % stages) % stages; q < last && warp < stages; q += stages) {
-        const int u = unit_of(gemm, (int)((q - q_base) / nst)), st = (int)((q - q_base) % nst), block = u / units;
+        const int u = sh.unit((int)((q - q_base) / nst)), st = (int)((q - q_base) % nst), block = u / units;
         if (block != cached) {
           cached = block;
           expert = p.plan[plan_expert(block)];
@@ -577,9 +641,11 @@ decode_layer_kernel(const __grid_constant__ CUtensorMap map1, const __grid_const
       }
       seg = seg_end;
     }
-    if (gemm == 0) compute_barrier();  // everyone is done with the token rows
+    q_base += (uint32_t)(count * nst);
   }
 }
+
+thread_local int t_debug_ctas = 0;  // fmoe_debug_decode_ctas
 
 template <int VPT>
 int launch_prepare(const PrepareParams& p, int quant_ctas, size_t smem, cudaStream_t st) {
@@ -609,7 +675,11 @@ int launch_layer(const fmoe_fused_args& a, const LayerParams& p, int smem, cudaS
   rc = encode_tensor_map(&map2, a.w2, EB, 4, dims2, strides2, box2, true, "decode down weights");
   if (rc) return rc;
   const int sms = device_sm_count();
-  launch_pdl(decode_layer_kernel<EB>, dim3(sms > 0 ? sms : 148), dim3(kThreads), (size_t)smem, st, map1, map2, p);
+  LayerParams q = p;
+  q.shares = std::min(sms > 0 ? sms : 148, kMaxShares);
+  const int ctas = t_debug_ctas > 0 ? std::min(t_debug_ctas, q.shares) : q.shares;
+  t_debug_ctas = 0;
+  launch_pdl(decode_layer_kernel<EB>, dim3(ctas), dim3(kThreads), (size_t)smem, st, map1, map2, q);
   return launch_status("decode_layer_kernel");
 }
 
@@ -667,7 +737,7 @@ bool plan_decode(const fmoe_fused_args& a, const RouteArgs& r, DecodePlan* pl) {
   pl->off_xs = fp8 ? take(a.T * (a.H / 128) * 4) : 0;
   pl->off_act = take(blocks * 8 * a.I * (fp8 ? 4 : 2));
   pl->off_z = a.no_combine ? 0 : take(numel * a.H * 2);
-  pl->off_counters = take((kMaxBlocks + a.H / 16) * 4);
+  pl->off_counters = take((kMaxBlocks + a.H / 16 + 1) * 4);
   pl->total = off;
   return true;
 }
@@ -689,7 +759,7 @@ int run_decode(const fmoe_fused_args& a, const RouteArgs& r, const DecodePlan& p
   q.weights = reinterpret_cast<float*>(ws + pl.off_weights);
   q.plan = reinterpret_cast<int32_t*>(ws + pl.off_plan);
   q.counters = reinterpret_cast<int32_t*>(ws + pl.off_counters);
-  q.num_counters = kMaxBlocks + (int)(a.H / 16);
+  q.num_counters = kMaxBlocks + (int)(a.H / 16) + 1;
   q.T = (int)a.T;
   q.k = a.top_k;
   q.E = a.num_experts;
@@ -721,6 +791,7 @@ int run_decode(const fmoe_fused_args& a, const RouteArgs& r, const DecodePlan& p
   p.out = static_cast<__nv_bfloat16*>(a.out);
   p.ready = q.counters;
   p.done = q.counters + kMaxBlocks;
+  p.tickets = p.done + a.H / 16;
   p.H = a.H;
   p.I = a.I;
   p.T = (int)a.T;
@@ -742,3 +813,9 @@ int run_decode(const fmoe_fused_args& a, const RouteArgs& r, const DecodePlan& p
 }
 
 }  // namespace fmoe
+
+extern "C" int fmoe_debug_decode_ctas(int ctas) {
+  if (ctas < 0) return fmoe::fail(FMOE_ERR_INVALID_ARG, "decode CTAs: need 0 (no limit) or more");
+  fmoe::t_debug_ctas = ctas;
+  return FMOE_OK;
+}

@@ -430,6 +430,13 @@ int fmoe_selftest_bounded_wait(int64_t limit_cycles, void* stream);
 int fmoe_debug_stage_events(void* const* events, int n);
 
 /*
+ * Diagnostic: the decode layer kernel of the calling thread's NEXT call of at most 8 tokens is launched with at most `ctas`
+ * CTAs (0: one per SM as usual).  Its work is the same, so this shows the call as it runs when other streams hold the rest
+ * of the SMs.  No counterpart in the reference.
+ */
+int fmoe_debug_decode_ctas(int ctas);
+
+/*
  * Diagnostic: with the environment variable FMOE_TC_PROFILE set, the bf16 tcgen05 kernel records, per
  * CTA, clock cycles spent waiting {tiles, MMA on accumulator, MMA on data, producer on free stage,
  * epilogue on accumulator, epilogue busy, -, -}.  Copies the last launch's n values (8 per CTA, at most

@@ -112,6 +112,48 @@ def test_decode_layer(fg, T, kind):
     assert_close_moe(fg.fused_experts(*d, tw.cuda(), bad.cuda(), **kw), oracle(tw, bad), tol, f"{kind} T={T} dropped ids")
 
 
+def _decode_call(fg, kind, T, seed, E=16, H=640, I=384, k=4):
+    x, w1, w2, g = _layer(T, H, I, E, seed)
+    logits = torch.randn(T, E, generator=g).cuda()
+    if kind == "block":
+        (w1, s1), (w2, s2) = OQ.quant_weight_block128(w1), OQ.quant_weight_block128(w2)
+        kw = dict(use_fp8_w8a8=True, w1_scale=s1.cuda(), w2_scale=s2.cuda(), block_shape=[128, 128])
+    else:
+        kw = {}
+    d = [x.cuda(), w1.cuda(), w2.cuda()]
+    return lambda: fg.fused_moe(*d, logits, k, True, **kw)
+
+
+@pytest.mark.parametrize("ctas", [1, 2, 29, 147])
+@pytest.mark.parametrize("T", [1, 5, 8])
+@pytest.mark.parametrize("kind", ["bf16", "block"])
+def test_decode_layer_needs_no_cta_that_has_not_started(fg, kind, T, ctas):
+    """The decode kernel's CTAs wait on one another.  Launched with fewer CTAs than it has shares of work, those that run take
+    all shares, as they do while another stream holds the other SMs: the call ends and the bits are the same."""
+    from flaggems_sglang_b200 import _C
+
+    call = _decode_call(fg, kind, T, 90 + T)
+    ref = call()
+    _C.check(_C.lib().fmoe_debug_decode_ctas(ctas))
+    out = call()
+    assert torch.equal(out, ref) and torch.equal(call(), ref)
+
+
+@pytest.mark.parametrize("kind", ["bf16", "block"])
+def test_decode_layers_on_streams_of_two_priorities(fg, kind):
+    calls = [_decode_call(fg, kind, T, 110 + T, E=32, H=1024, I=1024) for T in (1, 8)]
+    refs = [c() for c in calls]
+    torch.cuda.synchronize()
+    streams = [torch.cuda.Stream(priority=p) for p in (0, -1)]
+    outs = [[], []]
+    for _ in range(60):
+        for i, st in enumerate(streams):
+            with torch.cuda.stream(st):
+                outs[i].append(calls[i]())
+    torch.cuda.synchronize()
+    assert all(torch.equal(o, refs[i]) for i in range(2) for o in outs[i])
+
+
 @pytest.mark.parametrize("E", [1, 8, 255, 257])
 @pytest.mark.parametrize("numel", [1, 127, 128, 129, 4097, 16383, 16384, 16385])
 def test_align_at_chunk_edges(fg, numel, E):
