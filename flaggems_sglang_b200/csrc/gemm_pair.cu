@@ -68,7 +68,7 @@ struct PairParams {
   void* out;
   void* const* out_rows;  // down projection: optional per-slot row addresses (may be peer memory)
   float* split_partials;    // tail split: [workers][2 CTAs][128][256] f32 partial accumulators (NULL: no split)
-  int32_t* split_counters;  // tail split: [workers][2] arrivals, zero at launch
+  int32_t* split_counters;  // tail split: [tiles][2 CTAs][4 warp groups] arrivals, zero at launch
   int64_t numel;
   int64_t n;              // gemm1: I, gemm2: H
   int64_t w_rows;         // rows of W per expert
@@ -95,10 +95,15 @@ __device__ __forceinline__ void report(int code) { atomicCAS(&g_device_status, 0
 __device__ __forceinline__ bool warp_wait_relaxed(uint64_t* bar, uint32_t parity) {
   return __all_sync(0xffffffffu, ptx::mbar_wait_relaxed(bar, parity));
 }
-__device__ __forceinline__ int32_t ld_acquire_gpu(const int32_t* p) {
-  int32_t v;
-  asm volatile("ld.acquire.gpu.global.s32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
-  return v;
+
+// Whether `pred` holds for any thread of the four epilogue warps (one of each TMEM lane quarter) that share barrier `bar`.
+__device__ __forceinline__ bool any_of_four_warps(int bar, bool pred) {
+  int v = pred;
+  asm volatile("{\n.reg .pred p, q;\nsetp.ne.s32 p, %0, 0;\nbar.red.or.pred q, %1, 128, p;\nselp.s32 %0, 1, 0, q;\n}"
+               : "+r"(v)
+               : "r"(bar)
+               : "memory");
+  return v != 0;
 }
 
 template <bool GATED, bool F8, bool EXTRA, bool WMN, bool GATHER>
@@ -335,7 +340,10 @@ grouped_gemm_pair_kernel(const __grid_constant__ CUtensorMap map_t, const __grid
         }
       }
       const long long te0 = p.profile ? clock64() : 0;
-      const bool oke = warp_wait_relaxed(&acc_full[acc], acc_phase);
+      const bool split = plan.is_split(it);
+      bool oke = warp_wait_relaxed(&acc_full[acc], acc_phase);
+      // warps that meet at a barrier below leave together or not at all
+      if (split || (GATED && WMN)) oke = !any_of_four_warps(1 + half, !oke);
       const long long te1 = p.profile ? clock64() : 0;
       prof_wait += te1 - te0;
       if (!oke) {
@@ -345,19 +353,16 @@ grouped_gemm_pair_kernel(const __grid_constant__ CUtensorMap map_t, const __grid
       }
       ptx::tc_fence_after_sync();
       const uint32_t taddr = tmem_base + acc * ACC_COLS + ((uint32_t)(quarter * 32) << 16);
-      const bool split = plan.is_split(it);
       const int S = split ? plan.S : 1;
-      const int c_begin = chunks * slice / S, c_end = chunks * (slice + 1) / S;
-      const int tail_index = plan.b / plan.S;
       // fragment (slice o, chunk j) of this thread: four float4, 512 bytes apart so that a warp stores whole lines
       auto partial = [&](int o, int j) {
         return reinterpret_cast<float4*>(p.split_partials) +
-               ((((int64_t)(tail_index * S + o) * 2 + rank) * 16 + j) * 4 + quarter) * 128 + lane;
+               ((((int64_t)(plan.b - slice + o) * 2 + rank) * 16 + j) * 4 + quarter) * 128 + lane;
       };
+      bool finish = true;  // these four warps run the epilogue of their chunks
       if (split) {
 #pragma unroll 1
         for (int j = half; j < chunks; j += HALVES) {
-          if (j >= c_begin && j < c_end) continue;
           uint32_t lo[8], hi[8];
           ptx::tmem_ld_16x256b_x2(taddr + j * 16, lo);
           ptx::tmem_ld_16x256b_x2(taddr + (16u << 16) + j * 16, hi);
@@ -370,48 +375,28 @@ grouped_gemm_pair_kernel(const __grid_constant__ CUtensorMap map_t, const __grid
                                              __uint_as_float(v[3])));
           }
         }
-        __threadfence();  // the strips are visible device-wide before this warp counts as arrived
-        __syncwarp();
-        int32_t* counter = p.split_counters + tail_index * 2 + rank;
-        if (lane == 0) atomicAdd(counter, 1);
-        const long long t0 = clock64();
-        bool ok = true;
-        while (ld_acquire_gpu(counter) < kEpiWarps * S) {  // every epilogue warp of every slice has published
-          if (clock64() - t0 > 2000000000ll) {
-            ok = false;
-            break;
-          }
-          __nanosleep(64);
-        }
-        if (!__all_sync(0xffffffffu, ok)) {
-          report(0x380 | acc);
-          alive = false;
-          break;
-        }
+        __threadfence();  // the partials are visible device-wide before these warps count as arrived
+        asm volatile("bar.sync %0, 128;" ::"r"(1 + half) : "memory");
+        finish = any_of_four_warps(1 + half, quarter == 0 && lane == 0 &&
+                                                 atomicAdd(p.split_counters + (plan.b / S * 2 + rank) * 4 + half, 1) == S - 1);
+        __threadfence();  // the other slices' partials are read after the count
       }
-      // first chunk of this warp inside the strip; the next one's TMEM read-out is in flight while a chunk is stored
-      int j = half + ((max(c_begin - half, 0) + HALVES - 1) / HALVES) * HALVES;
+      // the next chunk's TMEM read-out is in flight while a chunk is stored
+      const int c_end = finish ? chunks : 0;
+      int j = half;
       uint32_t nlo[8], nhi[8];
-      if (j < c_end) {
+      if (j < c_end && !split) {
         ptx::tmem_ld_16x256b_x2(taddr + j * 16, nlo);                // rows 0-15 of the quarter (gated: gate)
         ptx::tmem_ld_16x256b_x2(taddr + (16u << 16) + j * 16, nhi);  // rows 16-31 (gated: up)
       }
 #pragma unroll 1
       for (; j < c_end; j += HALVES) {
         uint32_t lo[8], hi[8];
-        ptx::tmem_ld_wait();
+        if (split) {  // all slices' partials in slice order, whoever adds them
 #pragma unroll
-        for (int i = 0; i < 8; ++i) {
-          lo[i] = nlo[i];
-          hi[i] = nhi[i];
-        }
-        if (j + HALVES < c_end) {
-          ptx::tmem_ld_16x256b_x2(taddr + (j + HALVES) * 16, nlo);
-          ptx::tmem_ld_16x256b_x2(taddr + (16u << 16) + (j + HALVES) * 16, nhi);
-        }
-        if (S > 1) {
+          for (int i = 0; i < 8; ++i) lo[i] = hi[i] = 0u;
+#pragma unroll 1
           for (int o = 0; o < S; ++o) {
-            if (o == slice) continue;
             const float4* src = partial(o, j);
 #pragma unroll
             for (int q = 0; q < 4; ++q) {
@@ -422,6 +407,17 @@ grouped_gemm_pair_kernel(const __grid_constant__ CUtensorMap map_t, const __grid
               d[2] = __float_as_uint(__uint_as_float(d[2]) + v.z);
               d[3] = __float_as_uint(__uint_as_float(d[3]) + v.w);
             }
+          }
+        } else {
+          ptx::tmem_ld_wait();
+#pragma unroll
+          for (int i = 0; i < 8; ++i) {
+            lo[i] = nlo[i];
+            hi[i] = nhi[i];
+          }
+          if (j + HALVES < c_end) {
+            ptx::tmem_ld_16x256b_x2(taddr + (j + HALVES) * 16, nlo);
+            ptx::tmem_ld_16x256b_x2(taddr + (16u << 16) + (j + HALVES) * 16, nhi);
           }
         }
         // the chunk's 16 slots and row scales, from the lanes that hold them
@@ -603,7 +599,7 @@ int tail_plan_unit(int64_t total_tiles, int k_steps, int max_split, int grid, in
 
 int64_t gemm_pair_split_workspace_bytes() {
   const int sms = device_sm_count();
-  return 1024 + (int64_t)std::min(std::max(sms, 1), 256) * 128 * 256 * 4;
+  return kSplitCounters * 4 + (int64_t)std::min(std::max(sms, 1), 256) * 128 * 256 * 4;
 }
 
 // tokens: row-major [rows, cols]; box = 128 bytes x box_rows
@@ -701,15 +697,15 @@ int launch(const GemmParams& g, cudaStream_t st) {
   p.split_max = 0;
   const char* split_env = getenv("FMOE_TC_SPLIT_TAIL");  // "0": off (read per launch, tests flip it)
   const bool split_off = split_env && split_env[0] == '0';
-  const bool split_fits = g.split_ws_bytes >= 1024 + (int64_t)workers * 2 * 128 * 256 * 4 && workers <= 128;
+  const bool split_fits = g.split_ws_bytes >= kSplitCounters * 4 + (int64_t)workers * 2 * 128 * 256 * 4 && workers <= 128;
   if (g.split_ws && !split_off && split_fits && aligned16(g.split_ws)) {
-    p.split_partials = reinterpret_cast<float*>(reinterpret_cast<uint8_t*>(g.split_ws) + 1024);
+    p.split_partials = reinterpret_cast<float*>(reinterpret_cast<uint8_t*>(g.split_ws) + kSplitCounters * 4);
     p.split_max = GATED ? 4 : 8;
     if (g.split_counters) {
       p.split_counters = g.split_counters;
     } else {
       p.split_counters = reinterpret_cast<int32_t*>(g.split_ws);
-      FMOE_CUDA_OK(cudaMemsetAsync(g.split_ws, 0, 1024, st));
+      FMOE_CUDA_OK(cudaMemsetAsync(g.split_ws, 0, kSplitCounters * 4, st));
     }
   }
   launch_pdl(kernel, dim3(2 * workers), dim3((epi_warps(GATED && WMN) + 2) * 32), smem, st, map_t, map_w, p);

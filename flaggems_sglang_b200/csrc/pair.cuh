@@ -20,7 +20,8 @@ inline int pick_token_tile(int64_t numel, int num_experts, bool e4m3) {
   const double rows = (double)numel / (double)(numel < num_experts ? (numel > 0 ? numel : 1) : num_experts);
   return rows <= 40.0 ? 64 : (rows <= 88.0 && !e4m3 ? 128 : 256);
 }
-constexpr int kSplitCounters = 256;  // tail-split arrival counters of one launch: one per CTA
+// tail-split arrival counters of one launch: 8 per split tile, of which there are at most half as many as workers (<= 128)
+constexpr int kSplitCounters = 512;
 
 // int32 words of the expert table: first row [E], rows [E], exclusive prefix sum of the token tiles [E + 1]
 __host__ __device__ constexpr int pair_table_words(int num_experts) { return 3 * num_experts + 1; }
@@ -205,10 +206,11 @@ __device__ __forceinline__ void zero_block_rows(const PairTile& tl, void* out, i
 
 // Work units of one worker (a CTA pair).  Tiles are dealt round-robin; when the last round has work for at most half of
 // the workers (they are bound by their own rate, so a part-filled round costs as much as a full one), each of its tiles
-// is cut into S slices along K (S a power of two) that S neighbouring workers compute.  The S partial accumulators are
-// then summed by all S workers together: worker s owns the s-th strip of the tile's columns, publishes the other strips
-// of its partial in global memory, waits until all S have done so, adds the others' partials of its strip in slice
-// order (a fixed order: results do not depend on timing) and runs the epilogue on the strip.
+// is cut into S slices along K (S a power of two) that S neighbouring workers compute.  Every worker leaves its partial
+// accumulator in global memory; whichever arrives last (counted per group of four epilogue warps) adds all S in slice order (a
+// fixed order: results do not depend on timing) and runs the epilogue.  Nobody waits: workers may start in any order, and
+// none needs another to be resident.  (Workers that wait for one another and finish a strip of the columns each need all of
+// them resident; the times are the same: Mixtral rank, 333 tokens, 268 and 269 us per layer, 288 without the split.)
 struct UnitPlan {
   int64_t total, rounds, left;
   int grid, b, S, k_steps;

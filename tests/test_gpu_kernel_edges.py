@@ -1,4 +1,6 @@
 """GPU: the kernels at the sizes where a tile, a chunk or a dispatch rule ends, against the CPU oracle."""
+import ctypes
+
 import numpy as np
 import pytest
 import torch
@@ -152,6 +154,57 @@ def test_decode_layers_on_streams_of_two_priorities(fg, kind):
                 outs[i].append(calls[i]())
     torch.cuda.synchronize()
     assert all(torch.equal(o, refs[i]) for i in range(2) for o in outs[i])
+
+
+def _slices(lib, tiles, k_steps, most):
+    out = (ctypes.c_int64 * 5)()
+    assert lib.fmoe_debug_tail_plan(tiles, k_steps, most, lib.fmoe_sm_count() // 2, 0, 0, out) == 1
+    return out[4]
+
+
+# one tile per expert: 16 gate/up tiles in 4 slices (32 down tiles of 8 K steps: not cut), 8 down tiles in 8 slices of 8 K steps
+# (64 gate/up tiles: not cut)
+@pytest.mark.parametrize("E,H,I,k", [(4, 2048, 512, 2), (2, 1024, 4096, 1)])
+@pytest.mark.parametrize("T", [30, 300])
+@pytest.mark.parametrize("kind", ["bf16", "n_major", "bias", "channel"])
+def test_tail_split_is_finished_by_the_last_to_arrive(fg, kind, T, E, H, I, k):
+    """Tiles of a part-filled last round are cut along K; the worker that arrives last adds the partials in slice order, so
+    the bits do not depend on which one that is, nor on calls on a stream of another priority beside it."""
+    from flaggems_sglang_b200 import _C
+
+    step = 128 if kind == "channel" else 64  # channels of a K step
+    slices = _slices(_C.lib(), E * (I // 128), H // step, 4), _slices(_C.lib(), E * (H // 256), I // step, 8)
+    assert slices == ((4 // (step // 64), 1) if E == 4 else (1, 8 // (step // 64)))
+    x, w1, w2, g = _layer(T, H, I, E, 130 + T)
+    tw, ids = OR.softmax_topk(torch.randn(T, E, generator=g), k, True)
+    idx = torch.linspace(0, T - 1, 48).long().unique()
+    d, kw = [x.cuda(), w1.cuda(), w2.cuda()], dict(variant="tcgen05")
+    ref = OE.fused_experts(x[idx], w1, w2, tw[idx], ids[idx])
+    if kind == "n_major":
+        d[1:], kw = [w.transpose(1, 2).contiguous() for w in d[1:]], dict(weights_n_major=True)
+    elif kind == "bias":
+        b1, b2 = torch.randn(E, 2 * I, generator=g), torch.randn(E, H, generator=g)
+        kw.update(b1=b1.cuda(), b2=b2.cuda(), activation="swiglu_oai", gemm1_clamp_limit=7.0)
+        ref = OE.fused_experts_with_bias(x[idx], w1, b1, w2, b2, tw[idx], ids[idx], limit=7.0)
+    elif kind == "channel":
+        (w1q, s1), (w2q, s2) = OQ.quant_weight_per_channel(w1), OQ.quant_weight_per_channel(w2)
+        d[1:], kw = [w1q.cuda(), w2q.cuda()], dict(use_fp8_w8a8=True, per_channel_quant=True, w1_scale=s1.cuda(), w2_scale=s2.cuda())
+        ref = OE.fused_experts_fp8_per_channel(x[idx], w1q, s1, w2q, s2, tw[idx], ids[idx])
+    twd, idd = tw.cuda(), ids.cuda()
+    call = lambda: fg.fused_experts(*d, twd, idd, **kw)  # noqa: E731
+    out = call()
+    assert_close_moe(out[idx.cuda()], ref, "fp8" if kind == "channel" else "bf16", f"tail split {kind} T={T}")
+    decode = _decode_call(fg, "bf16", 8, 5, E=32, H=1024, I=1024)
+    dref = decode()
+    torch.cuda.synchronize()
+    streams = [torch.cuda.Stream(priority=p) for p in (0, -1, 0)]
+    outs = []
+    for _ in range(30):
+        for st, fn, want in zip(streams, (call, call, decode), (out, out, dref)):
+            with torch.cuda.stream(st):
+                outs.append((fn(), want))
+    torch.cuda.synchronize()
+    assert all(torch.equal(o, want) for o, want in outs)
 
 
 @pytest.mark.parametrize("E", [1, 8, 255, 257])
