@@ -180,8 +180,10 @@ int plan_fused(const fmoe_fused_args& a, const RouteArgs& route, FusedPlan* pl) 
   } else if (fp8) {
     p.off_xs = take((tc ? p.cap : a.T) * a.H);
     p.off_xs_scale = take(a.T * (a.H / 128) * 4);
-    // the wide tensor-core kernel quantises its 128-channel groups itself; the others write fp32 for the quantiser
-    p.off_act = take(p.cap * a.I * 4);
+    // fp32 rows for the quantiser.  The wide tensor-core kernel quantises its 128-channel groups itself, so with both kernels
+    // at work only experts of at most kNarrowRows rows have any (DeepSeek-V3, 16384 tokens: 134 MB, a row per position 1.34 GB)
+    const bool both = tc && !fold_narrow_only(p.numel, a.num_experts);
+    p.off_act = take((both ? (int64_t)a.num_experts * kNarrowRows : p.cap) * a.I * 4);
     p.off_actq = take(p.cap * a.I);
     p.off_actq_scale = take(p.cap * (a.I / 128) * 4);
   } else {
@@ -396,6 +398,7 @@ int run_fused(const fmoe_fused_args& args, const RouteArgs& route, const FusedPl
   }
   const bool both_folds = fold && tc && !fold_narrow_only(p.numel, a.num_experts);
   mark(2);
+  g1.fold_by_expert = both_folds;
   if (both_folds) g1.fold = FoldKernel::kNarrow;
   rc = run_gemm(g1, true, st);
   if (rc) return rc;

@@ -11,12 +11,14 @@ namespace fmoe {
 // different outputs from them asks for one at a time.
 enum class FoldKernel { kBoth, kNarrow, kWide };
 
+
 // Arguments of one grouped GEMM: the public ones, and what only the one-call layer hands over (fused.cu).
 struct GemmParams : fmoe_gemm_args {
   const int32_t* expert_table = nullptr;  // pair_table_words(E) words written by moe_align (see pair.cuh); NULL: derived
   int token_tile = 0;                     // the tile width that table was made for; 0: chosen by the launcher
   int32_t* split_counters = nullptr;      // zeroed arrival counters of the tail split; NULL: cleared by the launcher
   FoldKernel fold = FoldKernel::kBoth;
+  bool fold_by_expert = false;            // kNarrow, gate/up: the output has kNarrowRows rows per expert, not one per position
   bool skip_padding = false;              // gate/up: rows between an expert's last row and its block's end stay unwritten
 };
 

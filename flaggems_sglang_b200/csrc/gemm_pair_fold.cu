@@ -94,6 +94,7 @@ struct FoldParams {
   int32_t out_dtype;  // gate/up: FMOE_F32, FMOE_BF16 or (wide) FMOE_E4M3 with out_scale
   float* out_scale;   // [rows, n / 128]
   int32_t min_rows, max_rows;  // experts of this launch
+  bool by_expert;              // narrow, fp32 gate/up output: kNarrowRows rows per expert instead of one per position
 };
 
 __device__ __forceinline__ void report(int code) { atomicCAS(&g_device_status_fp8, 0, code); }
@@ -521,7 +522,8 @@ grouped_gemm_pair_fold_kernel(const __grid_constant__ CUtensorMap map_t, const _
 #pragma unroll
             for (int j = 0; j < 8; ++j) lo[j] = act_mul(lo[j] * rs[2 * (j >> 2) + (j & 1)], hi[j] * rs[2 * (j >> 2) + (j & 1)], p.activation);
             if (p.out_dtype == FMOE_F32) {  // eight lanes store one token's 32 bytes
-              float* out = reinterpret_cast<float*>(p.out) + (int64_t)(tl.row0 + tok0) * p.n + ch0 + (lane >> 2);
+              const int row0 = p.by_expert ? tl.row0 - table[tl.expert] + tl.expert * kNarrowRows : tl.row0;
+              float* out = reinterpret_cast<float*>(p.out) + (int64_t)(row0 + tok0) * p.n + ch0 + (lane >> 2);
 #pragma unroll
               for (int j = 0; j < 8; ++j) {
                 const int u = 8 * (j >> 2) + 2 * t + (j & 1);
@@ -1068,6 +1070,7 @@ int launch(const GemmParams& g, int min_rows, int max_rows, cudaStream_t st) {
   p.zero_padding = !g.skip_padding;
   p.out_dtype = g.out_dtype;
   p.out_scale = g.out_scale;
+  p.by_expert = g.fold_by_expert && max_rows <= kNarrowRows;
   p.min_rows = min_rows;
   p.max_rows = max_rows;
 

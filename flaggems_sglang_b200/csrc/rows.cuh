@@ -15,7 +15,7 @@ int run_quant_scatter(const void* x, int64_t T, int k, int64_t K, const int32_t*
 int run_quant_rows(const void* x, int64_t numel, int64_t K, const int32_t* slot_pos, void* q, float* scale, cudaStream_t st);
 // sorted f32 rows -> e4m3 with a scale per 128 channels, likewise
 int run_quant_slots(const float* x, int64_t numel, int64_t K, const int32_t* slot_pos, void* q, float* scale, cudaStream_t st);
-// the same, only the experts with up to max_rows rows (table: pair.cuh): CTAs per expert, so that the other experts cost nothing
+// the same from max_rows f32 rows per expert to the experts' positions, only the experts with up to max_rows rows (table: pair.cuh): CTAs per expert, so that the other experts cost nothing
 // (DeepSeek-V3, 4096 tokens, a third of the experts: 21 us against 105 us of looking at every slot)
 int run_quant_experts(const float* x, int64_t numel, int64_t K, int num_experts, const int32_t* table, int max_rows, void* q,
                       float* scale, cudaStream_t st);

@@ -50,6 +50,20 @@ def test_struct_layout_matches_header():
     assert _C.FusedArgs(T=3).struct_size == ctypes.sizeof(_C.FusedArgs)
 
 
+@pytest.mark.parametrize("T", [1024, 4096, 16384])
+def test_block_scale_workspace_has_no_row_per_position_in_fp32(lib, T):
+    """DeepSeek-V3 with both e4m3 kernels at work: fp32 rows only for experts of up to 64 rows, the rest of the workspace is
+    the quantised rows, the per-slot results and tables."""
+    from flaggems_sglang_b200 import _C
+
+    E, H, I, k = 256, 7168, 2048, 8
+    a = _C.FusedArgs(dtype=_C.E4M3, num_experts=E, top_k=k, T=T, H=H, I=I)
+    numel = T * k
+    cap = numel + E * 127
+    rest = cap * (H + I + I // 128 * 4) + numel * H * 2 + T * H // 128 * 4
+    assert lib.fmoe_fused_experts_workspace_bytes(a) <= rest + E * 64 * I * 4 + (4 << 20)
+
+
 def test_unknown_struct_size_is_refused(lib):
     """A binding compiled against another version of the header is caught before any field is trusted."""
     import ctypes
