@@ -262,25 +262,6 @@ def time_steps(step, steps, warmup, flush=False):
     return e0.elapsed_time(e1) / steps
 
 
-def stage_times(step, steps):
-    """Average device time per stage (ms) with events around each launch, in a pass of its own (the kernels are
-    launched one by one from Python): used for the CUDA-graph / L2-flushed points, whose timed loop cannot
-    carry events."""
-    import importlib
-
-    FM = importlib.import_module("flaggems_sglang_b200.ops.fused_moe")
-
-    FM.STAGE_EVENTS = []
-    for _ in range(steps):
-        step()
-    torch.cuda.synchronize()
-    acc = {}
-    for name, a, b in FM.STAGE_EVENTS:
-        acc.setdefault(name, []).append(a.elapsed_time(b))
-    FM.STAGE_EVENTS = None
-    return {k: sum(v) / len(v) for k, v in acc.items()}
-
-
 def time_steps_staged(step, steps, warmup, names):
     """Device time of `steps` production calls AND the average duration of every stage inside those same calls:
     the library records caller-provided events at its stage boundaries (fmoe_debug_stage_events), so the
@@ -316,14 +297,24 @@ def time_steps_staged(step, steps, warmup, names):
     return ms, st
 
 
-def stage_names(cfg, T):
-    from flaggems_sglang_b200.ops.fused_moe import _pick_variant
+def layer_kernels(cfg, T):
+    """Kernel family that the timed call (router logits in, one library call) takes."""
+    from flaggems_sglang_b200 import _C
+    from flaggems_sglang_b200.ops.fused_moe import layer_variant
 
-    dt = {"fp32": torch.float32, "bf16": torch.bfloat16, "fp8": torch.float8_e4m3fn}[cfg.dtype]
-    name, _ = _pick_variant(dt, T * cfg.top_k, cfg.E, cfg.I, cfg.H, None)
-    fp8 = cfg.dtype == "fp8"
-    if fp8 and cfg.fp8_scales == "channel":
-        name = "tcgen05"  # the only kernel family of the per-channel format
+    fa = _C.FusedArgs(dtype={"fp32": _C.F32, "bf16": _C.BF16, "fp8": _C.E4M3}[cfg.dtype], num_experts=cfg.E, top_k=cfg.top_k,
+                      T=T, H=cfg.H, I=cfg.I,
+                      scale_mode=_C.SCALE_CHANNEL if cfg.dtype == "fp8" and cfg.fp8_scales == "channel" else _C.SCALE_BLOCK128)
+    grouped = cfg.router == "grouped"
+    route = _C.RouteArgs(logits=16, grouped=int(grouped), renormalize=1, n_group=cfg.n_group if grouped else 1,
+                         topk_group=cfg.topk_group if grouped else 1)  # logits: present, not read
+    return layer_variant(fa, route)[0]
+
+
+def stage_names(cfg, T):
+    name, fp8 = layer_kernels(cfg, T), cfg.dtype == "fp8"
+    if name == "decode":
+        return ["decode_layer"] + [None] * 5
     g = ("gemm1_fp8_" if fp8 else "gemm1_") + name, ("gemm2_fp8_" if fp8 else "gemm2_") + name
     prep = "quant_input" if fp8 else ("gather_rows" if name.startswith("tcgen05") else None)
     return ["align", prep, g[0], "quant_act" if fp8 else None, g[1], "moe_sum"]
@@ -343,8 +334,8 @@ def measure_point(cfg, wts, T, steps, warmup, peaks, seed=0, skew=False):
     flush = nbytes < 2 * torch.cuda.get_device_properties(0).L2_cache_size
     if use_graph or flush:
         ms = time_steps(graphed(step) if use_graph else step, steps, warmup, flush=flush)
-        st = stage_times(step, max(3, steps // 2))
-        st_src = "separate pass, one launch per stage from the host"
+        st = time_steps_staged(step, max(3, steps // 2), 2, stage_names(cfg, T))[1]
+        st_src = "events inside the call, separate pass of the same call outside the graph"
     else:
         ms, st = time_steps_staged(step, steps, warmup, stage_names(cfg, T))
         st_src = "events inside the timed loop"

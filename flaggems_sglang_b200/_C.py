@@ -22,6 +22,7 @@ SCALE_BLOCK128, SCALE_CHANNEL = 0, 1
 VARIANTS = {"auto": 0, "simt": 1, "stream": 2, "tcgen05": 3}
 ACTIVATIONS = {"silu": 0, "gelu": 1, "swiglu_oai": 2}
 VARIANT_NAMES = {v: k for k, v in VARIANTS.items()}
+FUSED_DECODE = 4
 
 DTYPE_CODE = {torch.float32: F32, torch.bfloat16: BF16, torch.float8_e4m3fn: E4M3}
 
@@ -109,6 +110,7 @@ SIGNATURES = {
     "fmoe_pick_variant": (c_int, [c_int, c_int64, c_int, c_int64, c_int64, c_int, POINTER(c_int), POINTER(c_int)]),
     "fmoe_fused_experts_workspace_bytes": (c_int64, [POINTER(FusedArgs)]),
     "fmoe_fused_experts": (c_int, [POINTER(FusedArgs), c_void_p]),
+    "fmoe_fused_variant": (c_int, [POINTER(FusedArgs), POINTER(RouteArgs), POINTER(c_int), POINTER(c_int)]),
     "fmoe_fused_moe_workspace_bytes": (c_int64, [POINTER(FusedArgs), POINTER(RouteArgs)]),
     "fmoe_fused_moe": (c_int, [POINTER(FusedArgs), POINTER(RouteArgs), c_void_p]),
     "fmoe_fused_experts_sorted_workspace_bytes": (c_int64, [POINTER(FusedArgs)]),

@@ -529,6 +529,21 @@ extern "C" int fmoe_fused_experts_sorted(const fmoe_fused_args* args, const int3
   return fmoe::run_with_workspace(*args, r, stream);
 }
 
+extern "C" int fmoe_fused_variant(const fmoe_fused_args* args, const fmoe_route_args* route, int* variant_out, int* block_out) {
+  using namespace fmoe;
+  if (!args || !variant_out || !block_out) return fail(FMOE_ERR_INVALID_ARG, "fused_variant: null pointer");
+  if (route) {
+    const int rc = check_route(*args, *route);
+    if (rc) return rc;
+  }
+  FusedPlan p;
+  const int rc = plan_fused(*args, route ? route_args(*route) : RouteArgs{}, &p);
+  if (rc) return rc;
+  *variant_out = p.use_decode ? FMOE_FUSED_DECODE : p.variant;
+  *block_out = p.use_decode ? 0 : p.block;
+  return FMOE_OK;
+}
+
 extern "C" int64_t fmoe_fused_moe_workspace_bytes(const fmoe_fused_args* args, const fmoe_route_args* route) {
   if (!args || !route) {
     fmoe::fail(FMOE_ERR_INVALID_ARG, "fused_moe: args or route is null");

@@ -107,7 +107,8 @@ def standard_topk_to_routing(topk_weights: torch.Tensor, topk_ids: torch.Tensor,
 # kernel selection
 # --------------------------------------------------------------------------
 def _pick_variant(dtype, numel: int, E: int, I: int, H: int, forced: Optional[str]):
-    """-> (kernel family name, moe_align block size); the choice is made by the library (fmoe_pick_variant)."""
+    """-> (kernel family name, moe_align block size) of GEMMs that are launched one by one; the choice is made by the library
+    (fmoe_pick_variant)."""
     import ctypes
 
     forced = forced or os.environ.get("FMOE_VARIANT") or "auto"
@@ -119,6 +120,15 @@ def _pick_variant(dtype, numel: int, E: int, I: int, H: int, forced: Optional[st
     if rc != _C.OK:
         raise ValueError(_C.lib().fmoe_last_error().decode())
     return _C.VARIANT_NAMES[v.value], b.value
+
+
+def layer_variant(fa: _C.FusedArgs, route: Optional[_C.RouteArgs] = None):
+    """-> (kernel family name or "decode", moe_align block size) that the one-call layer takes for these arguments."""
+    import ctypes
+
+    v, b = ctypes.c_int(0), ctypes.c_int(0)
+    _C.check(_C.lib().fmoe_fused_variant(fa, route, ctypes.byref(v), ctypes.byref(b)))
+    return "decode" if v.value == _C.FUSED_DECODE else _C.VARIANT_NAMES[v.value], b.value
 
 
 def _gemm_args(**kw) -> _C.GemmArgs:
@@ -275,24 +285,26 @@ def _experts(hidden_states, w1, w2, topk_weights, topk_ids, route, k, inplace=Fa
 
     lib = _C.lib()
     st = _C.stream_ptr(dev)
-    if STAGE_EVENTS is None:
+    forced = variant or os.environ.get("FMOE_VARIANT") or "auto"
+    if forced not in _C.VARIANTS:
+        raise ValueError(f"unknown variant {forced!r}")
+    fa = _C.FusedArgs(
+        w_layout=_C.W_N_MAJOR if weights_n_major else _C.W_K_MAJOR,
+        scale_mode=_C.SCALE_CHANNEL if per_channel_quant else _C.SCALE_BLOCK128,
+        dtype=_C.E4M3 if use_fp8_w8a8 else _C.DTYPE_CODE[out_dtype], variant=_C.VARIANTS[forced], num_experts=E,
+        top_k=k, apply_router_weight_on_input=int(apply_router_weight_on_input), no_combine=int(no_combine),
+        zero_dropped=int(expert_map is not None), activation=_C.ACTIVATIONS[activation], T=T, H=H, I=I,
+        routed_scaling_factor=1.0 if routed_scaling_factor is None else float(routed_scaling_factor),
+        hidden=x.data_ptr(), w1=w1.data_ptr(), w2=w2.data_ptr(), w1_scale=_C.ptr(w1_scale),
+        w2_scale=_C.ptr(w2_scale), topk_weights=None if routed_here else wts.data_ptr(),
+        topk_ids=None if routed_here else ids.data_ptr(),
+        out_rows=_C.ptr(out_rows), b1=_C.ptr(b1), b2=_C.ptr(b2), act_alpha=act_alpha, act_limit=act_limit)
+    name, block = (None, 0) if STAGE_EVENTS is None else layer_variant(fa)
+    if STAGE_EVENTS is None or name == "decode":
         # production path: one library call, intermediates in one workspace tensor
-        forced = variant or os.environ.get("FMOE_VARIANT") or "auto"
-        if forced not in _C.VARIANTS:
-            raise ValueError(f"unknown variant {forced!r}")
         out = None if out_rows is not None else torch.empty((T, k, H) if no_combine else (T, H), dtype=out_dtype,
                                                             device=dev)
-        fa = _C.FusedArgs(
-            w_layout=_C.W_N_MAJOR if weights_n_major else _C.W_K_MAJOR,
-            scale_mode=_C.SCALE_CHANNEL if per_channel_quant else _C.SCALE_BLOCK128,
-            dtype=_C.E4M3 if use_fp8_w8a8 else _C.DTYPE_CODE[out_dtype], variant=_C.VARIANTS[forced], num_experts=E,
-            top_k=k, apply_router_weight_on_input=int(apply_router_weight_on_input), no_combine=int(no_combine),
-            zero_dropped=int(expert_map is not None), activation=_C.ACTIVATIONS[activation], T=T, H=H, I=I,
-            routed_scaling_factor=1.0 if routed_scaling_factor is None else float(routed_scaling_factor),
-            hidden=x.data_ptr(), w1=w1.data_ptr(), w2=w2.data_ptr(), w1_scale=_C.ptr(w1_scale),
-            w2_scale=_C.ptr(w2_scale), topk_weights=None if routed_here else wts.data_ptr(),
-            topk_ids=None if routed_here else ids.data_ptr(), out=_C.ptr(out),
-            out_rows=_C.ptr(out_rows), b1=_C.ptr(b1), b2=_C.ptr(b2), act_alpha=act_alpha, act_limit=act_limit)
+        fa.out = _C.ptr(out)
         if triple is not None:
             need = lib.fmoe_fused_experts_sorted_workspace_bytes(fa)
         else:
@@ -301,18 +313,18 @@ def _experts(hidden_states, w1, w2, topk_weights, topk_ids, route, k, inplace=Fa
             _C.check(_C.ERR_INVALID_ARG)
         ws = torch.empty(max(int(need), 256), dtype=torch.uint8, device=dev)
         fa.workspace, fa.workspace_bytes = ws.data_ptr(), ws.numel()
-        if triple is not None:
+        if name is not None:
+            with _stage("decode_layer"):  # routed slots: the triple and the router's logits do not come this way
+                _C.check(lib.fmoe_fused_experts(fa, st))
+        elif triple is not None:
             slot_of, hist, gate = triple
             _C.check(lib.fmoe_fused_experts_sorted(fa, slot_of.data_ptr(), hist.data_ptr(), gate.data_ptr(), st))
         else:
             _C.check(lib.fmoe_fused_experts(fa, st) if route is None else lib.fmoe_fused_moe(fa, route, st))
         return out
 
-    # profiling path (STAGE_EVENTS set): the same kernels launched one by one with events around each launch
-    if per_channel_quant:
-        name, block = "tcgen05", 128  # the one kernel family of this format
-    else:
-        name, block = _pick_variant(w1.dtype if not use_fp8_w8a8 else torch.float8_e4m3fn, numel, E, I, H, variant)
+    # kernel-by-kernel path (STAGE_EVENTS set): the family that the one call takes, its GEMMs launched one by one through
+    # their own entry points with events around each launch
     vcode = _C.VARIANTS[name]
 
     with _stage("align"):

@@ -282,7 +282,9 @@ typedef struct fmoe_fused_args {
                             out + slot*H (see fmoe_gemm_args.out_rows); `out` may then be NULL            */
 } fmoe_fused_args;
 
-/* Kernel family and moe_align block the AUTO choice takes for a shape.  forced_variant may be AUTO. */
+/* Kernel family and moe_align block the AUTO choice takes for a shape when the GEMMs are launched one by one
+ * (fmoe_gemm1_silu / fmoe_gemm2).  forced_variant may be AUTO.  The one-call layer has more to choose from and goes by the
+ * cost of the whole call: fmoe_fused_variant. */
 int fmoe_pick_variant(int dtype, int64_t numel, int E, int64_t I, int64_t H, int forced_variant,
                       int* variant_out, int* block_out);
 /* Bytes of workspace fmoe_fused_experts needs for these arguments (pointers are not read); < 0 on error. */
@@ -301,6 +303,11 @@ typedef struct fmoe_route_args {
   int32_t renormalize;
   int32_t n_group, topk_group;  /* grouped only                                                           */
 } fmoe_route_args;
+/* Kernels that fmoe_fused_moe (route == NULL: fmoe_fused_experts) takes for these arguments: FMOE_VARIANT_* or
+ * FMOE_FUSED_DECODE (at most 8 tokens: the GEMMs and the combine are one kernel), and the moe_align block (FMOE_FUSED_DECODE:
+ * 0).  Pointers are not read; route->logits only says that there is a router to run. */
+#define FMOE_FUSED_DECODE 4
+int fmoe_fused_variant(const fmoe_fused_args* args, const fmoe_route_args* route, int* variant_out, int* block_out);
 int64_t fmoe_fused_moe_workspace_bytes(const fmoe_fused_args* args, const fmoe_route_args* route);
 int fmoe_fused_moe(const fmoe_fused_args* args, const fmoe_route_args* route, void* stream);
 
@@ -424,6 +431,7 @@ int fmoe_selftest_bounded_wait(int64_t limit_cycles, void* stream);
  * boundaries and forgets the array:
  *   [0] start  [1] align done  [2] input rows gathered / quantised  [3] gate/up GEMM done
  *   [4] activations quantised (e4m3 only)  [5] down GEMM done  [6] sum done
+ * A call that the decode kernels take (fmoe_fused_variant: FMOE_FUSED_DECODE) is one stage, [0] to [1].
  * n = 0 cancels.  No counterpart in the reference (it times whole calls, benchmark/performance_utils.py:365-377).
  */
 #define FMOE_STAGE_EVENTS 7

@@ -64,6 +64,22 @@ def test_block_scale_workspace_has_no_row_per_position_in_fp32(lib, T):
     assert lib.fmoe_fused_experts_workspace_bytes(a) <= rest + E * 64 * I * 4 + (4 << 20)
 
 
+@pytest.mark.parametrize("dtype,T,E,H,I,k,want", [
+    ("BF16", 1, 128, 2048, 768, 8, "decode"), ("BF16", 9, 128, 2048, 768, 8, "stream"), ("BF16", 16, 8, 4096, 14336, 2, "tcgen05"),
+    ("E4M3", 8, 256, 7168, 2048, 8, "decode"), ("E4M3", 64, 256, 7168, 2048, 8, "tcgen05"), ("F32", 3, 8, 256, 512, 2, "simt")])
+def test_layer_variant_is_what_the_one_call_layer_takes(lib, dtype, T, E, H, I, k, want):
+    """Stage names come from here: the choice of the one-call layer, which is not that of GEMMs launched one by one
+    (fmoe_pick_variant says "stream" for the Mixtral, DeepSeek-V3 and decode-sized calls of this list)."""
+    from flaggems_sglang_b200 import _C
+    from flaggems_sglang_b200.ops.fused_moe import layer_variant
+
+    fa = _C.FusedArgs(dtype=getattr(_C, dtype), num_experts=E, top_k=k, T=T, H=H, I=I)
+    route = _C.RouteArgs(logits=16, grouped=0, renormalize=1, n_group=1, topk_group=1)
+    for r in (None, route):
+        name, block = layer_variant(fa, r)
+        assert name == want and block == {"decode": 0, "stream": 8, "tcgen05": 128, "simt": 16}[want]
+
+
 def test_unknown_struct_size_is_refused(lib):
     """A binding compiled against another version of the header is caught before any field is trusted."""
     import ctypes

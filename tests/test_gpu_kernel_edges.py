@@ -219,6 +219,25 @@ def test_align_at_chunk_edges(fg, numel, E):
     np.testing.assert_array_equal(e.cpu().numpy(), oe)
 
 
+@pytest.mark.parametrize("kind,T,names", [("bf16", 5, ["decode_layer"]), ("block", 5, ["decode_layer"]),
+                                          ("block", 12, ["gemm1_fp8_tcgen05", "gemm2_fp8_tcgen05"]), ("bf16", 12, ["gemm1_stream", "gemm2_stream"])])
+def test_stages_are_those_of_the_call(fg, kind, T, names):
+    """With stage events on, the kernel family is the one that the same call takes without them."""
+    import importlib
+
+    FM = importlib.import_module("flaggems_sglang_b200.ops.fused_moe")
+    call = _decode_call(fg, kind, T, 150)
+    ref = call()
+    FM.STAGE_EVENTS = []
+    try:
+        out = call()
+        seen = [n for n, _, _ in FM.STAGE_EVENTS if n.startswith(("gemm", "decode"))]
+    finally:
+        FM.STAGE_EVENTS = None
+    assert seen == names
+    assert_close_moe(out, ref.cpu(), "fp8" if kind == "block" else "bf16", f"stages {kind} T={T}")
+
+
 @pytest.mark.parametrize("T", [1, 8, 9, 100, 2049])
 def test_sorted_routing_equals_routing_by_slot(fg, T):
     """The routing triple goes to the kernels as it is; the results are those of the same routing by slot."""
