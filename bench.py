@@ -265,7 +265,8 @@ def time_steps(step, steps, warmup, flush=False):
 def time_steps_staged(step, steps, warmup, names):
     """Device time of `steps` production calls AND the average duration of every stage inside those same calls:
     the library records caller-provided events at its stage boundaries (fmoe_debug_stage_events), so the
-    per-kernel times and the step time come from one timed region."""
+    per-kernel times and the step time come from one timed region.  The third result is the number of kernels that the
+    library launched in it."""
     import ctypes
 
     from flaggems_sglang_b200 import _C
@@ -282,11 +283,13 @@ def time_steps_staged(step, steps, warmup, names):
         step()
     torch.cuda.synchronize()
     e0, e1 = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
+    lib.fmoe_debug_launches()
     e0.record()
     for i in range(steps):
         _C.check(lib.fmoe_debug_stage_events(arrs[i], n))
         step()
     e1.record()
+    launches = lib.fmoe_debug_launches()
     torch.cuda.synchronize()
     ms = e0.elapsed_time(e1) / steps
     st = {}
@@ -294,7 +297,7 @@ def time_steps_staged(step, steps, warmup, names):
         if name is None:
             continue
         st[name] = sum(row[j].elapsed_time(row[j + 1]) for row in evs) / steps
-    return ms, st
+    return ms, st, launches
 
 
 def layer_kernels(cfg, T):
@@ -334,10 +337,12 @@ def measure_point(cfg, wts, T, steps, warmup, peaks, seed=0, skew=False):
     flush = nbytes < 2 * torch.cuda.get_device_properties(0).L2_cache_size
     if use_graph or flush:
         ms = time_steps(graphed(step) if use_graph else step, steps, warmup, flush=flush)
-        st = time_steps_staged(step, max(3, steps // 2), 2, stage_names(cfg, T))[1]
+        n = max(3, steps // 2)
+        _, st, launches = time_steps_staged(step, n, 2, stage_names(cfg, T))
+        launches = launches // n * steps  # a graph replays the launches of one call
         st_src = "events inside the call, separate pass of the same call outside the graph"
     else:
-        ms, st = time_steps_staged(step, steps, warmup, stage_names(cfg, T))
+        ms, st, launches = time_steps_staged(step, steps, warmup, stage_names(cfg, T))
         st_src = "events inside the timed loop"
     p_tensor = peaks["bf16_tflops"] * (2.0 if cfg.dtype == "fp8" else 1.0)
     t_hbm = nbytes / (peaks["hbm_gbs"] * 1e9)
@@ -347,7 +352,7 @@ def measure_point(cfg, wts, T, steps, warmup, peaks, seed=0, skew=False):
     return {"T": T, "ms": ms, "cuda_graph": use_graph, "l2_flush": flush, "tokens_per_s": T / (ms * 1e-3), "active_experts": active, "bound": bound,
             "roofline_ms": t_roof * 1e3, "roofline_frac": t_roof / (ms * 1e-3),
             "achieved_gbs": nbytes / (ms * 1e-3) / 1e9, "achieved_tflops": flops / (ms * 1e-3) / 1e12,
-            "stages_ms": st, "stages_source": st_src, "alg_bytes": nbytes, "alg_flops": flops, "skew": skew, "tok": tok}
+            "stages_ms": st, "stages_source": st_src, "gpu_launches": launches, "alg_bytes": nbytes, "alg_flops": flops, "skew": skew, "tok": tok}
 
 
 # DRAM traffic of the gate/up GEMM per launch (dram__bytes_read.sum + dram__bytes_write.sum of one ncu capture; the
@@ -442,23 +447,6 @@ def e2e_run(cfg, wts, T, steps, warmup, seed=0):
     h2d = h_host.numel() * h_host.element_size() + l_host.numel() * l_host.element_size()
     d2h = out_host[0].numel() * out_host[0].element_size()
     return ms, h2d, d2h
-
-
-def launches_per_step(cfg, T):
-    from flaggems_sglang_b200.ops.fused_moe import _pick_variant
-
-    dt = {"fp32": torch.float32, "bf16": torch.bfloat16, "fp8": torch.float8_e4m3fn}[cfg.dtype]
-    name, _ = _pick_variant(dt, T * cfg.top_k, cfg.E, cfg.I, cfg.H, None)
-    numel = T * cfg.top_k
-    n = 1 + (3 if numel >= 8192 else 1) + 2 + 1  # router, align (count/scan/scatter above 8192 slots), two GEMMs, sum
-    if cfg.dtype == "fp8":
-        n += 1  # quantisation of the input rows
-        if name == "tcgen05" and cfg.top_k >= 2 and cfg.H % 512 == 0:
-            n += 2  # token rows quantised once, then bytes and scales copied into the sorted order
-        n += 1  # quantisation of the activations between the two GEMMs
-    elif name == "tcgen05":
-        n += 1  # row gather into sorted order
-    return n
 
 
 def sweep_entry(cfg, T, pt, peaks):
@@ -695,7 +683,7 @@ def main():
         "parity": parity,
         "e2e": {"value": T / (e2e_ms * 1e-3), "unit": UNIT, "ms_per_step": e2e_ms, "h2d_bytes_per_step": h2d,
                 "d2h_bytes_per_step": d2h, "copies": "pinned host buffers, side streams, double-buffered"},
-        "gpu_launches": launches_per_step(cfg, T) * args.steps,
+        "gpu_launches": point["gpu_launches"],
         "clocks": clocks,
         "stages_ms": {k: round(v, 4) for k, v in point["stages_ms"].items()},
         "sweep": sweep,

@@ -19,6 +19,11 @@ char* last_error_buffer() {
   return buf;
 }
 
+int64_t& launch_counter() {
+  static thread_local int64_t n = 0;
+  return n;
+}
+
 namespace {
 
 int validate_gemm(const GemmParams& a, bool gated, const char* who) {
@@ -117,6 +122,12 @@ extern "C" int fmoe_debug_tail_plan(int64_t total_tiles, int k_steps, int max_sp
 }
 
 extern "C" const char* fmoe_last_error(void) { return fmoe::last_error_buffer(); }
+
+extern "C" int64_t fmoe_debug_launches(void) {
+  const int64_t n = fmoe::launch_counter();
+  fmoe::launch_counter() = 0;
+  return n;
+}
 
 extern "C" int fmoe_sm_count(void) {
   int dev = 0, n = 0;

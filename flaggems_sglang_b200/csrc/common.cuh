@@ -38,9 +38,14 @@ inline int fail(int code, const char* fmt, ...) {
       return ::fmoe::fail(FMOE_ERR_CUDA, "%s failed: %s", #expr, cudaGetErrorString(err__)); \
   } while (0)
 
+// Kernels launched by the calling thread since it last asked (fmoe_debug_launches).
+int64_t& launch_counter();
+
+// After every kernel launch.
 inline int launch_status(const char* what) {
   cudaError_t err = cudaGetLastError();
   if (err != cudaSuccess) return fail(FMOE_ERR_CUDA, "launch of %s failed: %s", what, cudaGetErrorString(err));
+  ++launch_counter();
   return FMOE_OK;
 }
 

@@ -150,7 +150,9 @@ def run(args, cfg, rank: int, world: int, local: int, clock_sampler=None) -> Non
             clock_sampler.start()
         warm = max(args.warmup, 3)
         t_wall = time.perf_counter()
+        _C.lib().fmoe_debug_launches()
         ms_v = _timed(step, args.steps, warm, dev)
+        launches = _C.lib().fmoe_debug_launches() // (warm + args.steps)
         t_wall = time.perf_counter() - t_wall
         _C.check_device_status(dev)
 
@@ -274,8 +276,7 @@ def run(args, cfg, rank: int, world: int, local: int, clock_sampler=None) -> Non
                         "h2d_bytes_per_step": (h_host.numel() * h_host.element_size() + l_host.numel() * 4) * world,
                         "d2h_bytes_per_step": out_host[0].numel() * out_host[0].element_size() * world,
                         "copies": "pinned host buffers, side streams, double-buffered"},
-                # router, route, sort, dispatch, mask, align, row copy, 2 GEMMs, combine, sum (NCCL's not counted)
-                "gpu_launches": (11 if mode == "p2p" else 9) * args.steps * world,
+                "gpu_launches": launches * args.steps * world,  # this package's, counted on rank 0
                 "wall_ms_per_step": t_wall * 1e3 / (args.steps + warm),
                 "clocks": clocks,
                 "c5": c5,

@@ -437,6 +437,9 @@ int fmoe_selftest_bounded_wait(int64_t limit_cycles, void* stream);
 #define FMOE_STAGE_EVENTS 7
 int fmoe_debug_stage_events(void* const* events, int n);
 
+/* Diagnostic: kernels of this library that the calling thread has launched since it last asked. */
+int64_t fmoe_debug_launches(void);
+
 /*
  * Diagnostic: the decode layer kernel of the calling thread's NEXT call of at most 8 tokens is launched with at most `ctas`
  * CTAs (0: one per SM as usual).  Its work is the same, so this shows the call as it runs when other streams hold the rest

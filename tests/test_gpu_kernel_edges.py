@@ -238,6 +238,17 @@ def test_stages_are_those_of_the_call(fg, kind, T, names):
     assert_close_moe(out, ref.cpu(), "fp8" if kind == "block" else "bf16", f"stages {kind} T={T}")
 
 
+@pytest.mark.parametrize("kind,T,launches", [("bf16", 5, 2), ("block", 5, 2), ("bf16", 12, 5), ("bf16", 200, 6), ("block", 12, 7)])
+def test_launches_are_counted(fg, kind, T, launches):
+    """Decode: prepare and layer.  Otherwise router, block list, two GEMMs, sum, and the passes over rows in between."""
+    from flaggems_sglang_b200 import _C
+
+    call = _decode_call(fg, kind, T, 160)
+    _C.lib().fmoe_debug_launches()
+    call()
+    assert _C.lib().fmoe_debug_launches() == launches and _C.lib().fmoe_debug_launches() == 0
+
+
 @pytest.mark.parametrize("T", [1, 8, 9, 100, 2049])
 def test_sorted_routing_equals_routing_by_slot(fg, T):
     """The routing triple goes to the kernels as it is; the results are those of the same routing by slot."""
