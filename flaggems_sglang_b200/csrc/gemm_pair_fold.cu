@@ -24,6 +24,7 @@
 #include "pair.cuh"
 #include "rows.cuh"
 
+#include <atomic>
 #include <cstdlib>
 #include <type_traits>
 
@@ -148,7 +149,8 @@ __device__ __forceinline__ unsigned long long add2(unsigned long long a, unsigne
 }
 
 // PROF: instrumented build with wait-time counters (reading the clock is slow enough to distort the fold loop).
-template <bool GATED, bool PROF>
+// MOVE: registers move from the other warps to the fold warps (setmaxnreg); see launch().
+template <bool GATED, bool PROF, bool MOVE>
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 1)
 grouped_gemm_pair_fold_kernel(const __grid_constant__ CUtensorMap map_t, const __grid_constant__ CUtensorMap map_w,
                               const FoldParams p) {
@@ -213,7 +215,7 @@ grouped_gemm_pair_fold_kernel(const __grid_constant__ CUtensorMap map_t, const _
   PairCursor cursor;
   PairTile tl;
 
-  if (warp >= kFoldWarps) asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(kOtherRegs));
+  if (MOVE && warp >= kFoldWarps) asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(kOtherRegs));
   if (warp == kFoldWarps) {
     // ---------------- TMA producer (both CTAs) ----------------
     if (ptx::elect_one()) {
@@ -394,7 +396,7 @@ grouped_gemm_pair_fold_kernel(const __grid_constant__ CUtensorMap map_t, const _
     }
   } else {
     // ---------------- fold + epilogue (warps 0-15) ----------------
-    asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(kFoldRegs));
+    if constexpr (MOVE) asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(kFoldRegs));
     const int quarter = warp & 3, half = (warp >> 2) & 1, kgroup = warp >> 3;
     const int t = lane & 3;
     const uint32_t factor_addr = ptx::smem_u32(factors) + (16 * half + 2 * t) * 4;
@@ -618,7 +620,7 @@ struct WideGeo {
 };
 static_assert(WideGeo::bytes(1024) <= kMaxSmem, "shared memory");
 
-template <bool GATED, bool PROF>
+template <bool GATED, bool PROF, bool MOVE>
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 1)
 grouped_gemm_pair_fold_wide_kernel(const __grid_constant__ CUtensorMap map_t, const __grid_constant__ CUtensorMap map_w,
                                    const FoldParams p) {
@@ -681,7 +683,7 @@ grouped_gemm_pair_fold_wide_kernel(const __grid_constant__ CUtensorMap map_t, co
   PairCursor cursor;
   PairTile tl;
 
-  if (warp >= kFoldWarps) asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(kOtherRegs));
+  if (MOVE && warp >= kFoldWarps) asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(kOtherRegs));
   if (warp == kFoldWarps) {
     // ---------------- TMA producer (both CTAs): its half of the tile's tokens, its 128 weight rows ----------------
     if (ptx::elect_one()) {
@@ -876,7 +878,7 @@ grouped_gemm_pair_fold_wide_kernel(const __grid_constant__ CUtensorMap map_t, co
     }
   } else {
     // ---------------- fold + epilogue (warps 0-15) ----------------
-    asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(kFoldRegs));
+    if constexpr (MOVE) asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(kFoldRegs));
     // This loop runs at the 96 registers that 20 warps leave a thread: the tile is described by its meta entry, shared
     // memory addresses are constants, everything else is derived from three counters.
     const uint32_t lane_addr = tmem_base + ((uint32_t)((warp & 3) * 32) << 16) + 128 * (warp >> 3) + 32 * ((warp >> 2) & 1);
@@ -1026,15 +1028,22 @@ grouped_gemm_pair_fold_wide_kernel(const __grid_constant__ CUtensorMap map_t, co
 
 template <bool GATED, bool WIDE, bool PROF>
 int launch(const GemmParams& g, int min_rows, int max_rows, cudaStream_t st) {
-  auto kernel = WIDE ? grouped_gemm_pair_fold_wide_kernel<GATED, PROF> : grouped_gemm_pair_fold_kernel<GATED, PROF>;
   constexpr int TILE = WIDE ? 256 : TOK;
+  auto kernel = WIDE ? grouped_gemm_pair_fold_wide_kernel<GATED, PROF, true> : grouped_gemm_pair_fold_kernel<GATED, PROF, true>;
+  auto plain = WIDE ? grouped_gemm_pair_fold_wide_kernel<GATED, PROF, false> : grouped_gemm_pair_fold_kernel<GATED, PROF, false>;
+  // setmaxnreg waits for good when the launch has fewer registers than the warps' shares add up to.  The compiler gives these
+  // kernels the 96 per thread that 640 threads leave; one that gives fewer gets the kernels without the move
+  // (DeepSeek-V3, 4096 tokens: 3.33 ms per layer with it, 3.40 without).
+  static std::atomic<int> moves{-1};
+  if (moves < 0) {
+    cudaFuncAttributes fa;
+    FMOE_CUDA_OK(cudaFuncGetAttributes(&fa, kernel));
+    const char* env = getenv("FMOE_FOLD_MOVE_REGISTERS");  // "0": as with such a compiler
+    moves = fa.numRegs * kThreads >= (kFoldWarps * kFoldRegs + 4 * kOtherRegs) * 32 && !(env && env[0] == '0');
+  }
+  if (!moves) kernel = plain;
   static PerDeviceOnce once_attr;  // the opt-in to > 48 KB of dynamic shared memory is per device
   const cudaError_t attr_err = per_device_once(once_attr, [&] {
-    // setmaxnreg waits for good when the launch has fewer registers than the warps' shares add up to
-    cudaFuncAttributes fa;
-    const cudaError_t err = cudaFuncGetAttributes(&fa, kernel);
-    if (err != cudaSuccess) return err;
-    if (fa.numRegs * kThreads < (kFoldWarps * kFoldRegs + 4 * kOtherRegs) * 32) return cudaErrorInvalidConfiguration;
     return cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kMaxSmem);
   });
   if (attr_err != cudaSuccess)

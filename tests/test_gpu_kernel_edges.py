@@ -1,5 +1,8 @@
 """GPU: the kernels at the sizes where a tile, a chunk or a dispatch rule ends, against the CPU oracle."""
 import ctypes
+import os
+import subprocess
+import sys
 
 import numpy as np
 import pytest
@@ -74,6 +77,34 @@ def test_rows_per_expert_at_tile_edges(fg, tile, kind):
                                w2_scale=w2s.cuda(), **kw)
         ref = (OE.fused_experts_fp8_per_channel if kind == "channel" else OE.fused_experts_fp8)(x, w1q, w1s, w2q, w2s, tw, ids)
     assert_close_moe(out, ref, "fp8" if kind in ("channel", "block") else "bf16", f"{kind} tile {tile}")
+
+
+def test_e4m3_kernels_without_the_register_move(tmp_path):
+    """The e4m3 block-scale kernels as they are launched where the compiler left too few registers for setmaxnreg: same sums
+    in the same order, so the same bits."""
+    code = """
+import sys, torch
+import flaggems_sglang_b200 as fg
+g = torch.Generator(device="cuda").manual_seed(1)
+E, H, I, k, outs = 8, 512, 384, 2, []
+w1, w2 = (torch.randn(E, *s, generator=g, device="cuda") * s[1] ** -0.5 for s in ((2 * I, H), (H, I)))
+q = [fg.quant_weight_block128(torch.cat(list(w))) for w in (w1, w2)]
+w1q, s1 = q[0][0].view(E, 2 * I, H), q[0][1].view(E, 2 * I // 128, H // 128)
+w2q, s2 = q[1][0].view(E, H, I), q[1][1].view(E, H // 128, I // 128)
+for T in (20, 300, 900):
+    x, logits = torch.randn(T, H, generator=g, device="cuda").bfloat16(), torch.randn(T, E, generator=g, device="cuda")
+    outs.append(fg.fused_moe(x, w1q, w2q, logits, k, True, use_fp8_w8a8=True, w1_scale=s1, w2_scale=s2,
+                             block_shape=[128, 128], variant="tcgen05").cpu())
+fg._C.check_device_status()
+torch.save(outs, sys.argv[1])
+"""
+    outs = []
+    for move in ("1", "0"):
+        path = str(tmp_path / f"out{move}.pt")
+        env = dict(os.environ, FMOE_FOLD_MOVE_REGISTERS=move, PYTHONPATH=os.pathsep.join(sys.path))
+        subprocess.run([sys.executable, "-c", code, path], check=True, env=env, timeout=300)
+        outs.append(torch.load(path))
+    assert all(torch.equal(a, b) for a, b in zip(*outs))
 
 
 @pytest.mark.parametrize("T", [1, 2, 3, 5, 8, 9])
