@@ -56,13 +56,6 @@ int pick_variant(int dtype, int64_t numel, int E, int64_t I, int64_t H, int forc
 namespace {
 inline int64_t up256(int64_t v) { return (v + 255) & ~int64_t(255); }
 
-// The bf16 gate/up GEMM can fetch its input rows by TMA gather4 instead of reading a sorted copy of the hidden states.  The
-// gather costs about 12 cycles per row and K step, more than the copy (gate/up GEMM at Mixtral T=4096 2.4 times slower), so
-// the copy is the default and FMOE_TC_GATHER4=1 selects the gather (it saves the cap x H workspace).
-inline bool tc_gathers_input(int variant, int dtype) {
-  static const bool gather4 = getenv("FMOE_TC_GATHER4") != nullptr;
-  return variant == FMOE_VARIANT_TCGEN05 && dtype == FMOE_BF16 && gather4;
-}
 }
 
 // The whole layer on the CTA-pair GEMMs although an expert has few rows.  Both families read the weights once; the pair
@@ -187,7 +180,7 @@ int plan_fused(const fmoe_fused_args& a, const RouteArgs& route, FusedPlan* pl) 
     p.off_actq = take(p.cap * a.I);
     p.off_actq_scale = take(p.cap * (a.I / 128) * 4);
   } else {
-    if (tc && !(tc_gathers_input(p.variant, a.dtype) && !n_major)) p.off_xs = take(p.cap * a.H * eb);
+    if (tc) p.off_xs = take(p.cap * a.H * eb);
     if (tc && a.dtype == FMOE_BF16) {
       p.split_bytes = fmoe_gemm_split_workspace_bytes();
       p.off_split = take(p.split_bytes);
@@ -307,7 +300,7 @@ int run_fused(const fmoe_fused_args& args, const RouteArgs& route, const FusedPl
   al.num_zero = counters ? 2 * kSplitCounters : 0;
   int32_t* slot_pos = tc ? reinterpret_cast<int32_t*>(ws + p.off_slot_pos) : nullptr;
   al.slot_pos = slot_pos;
-  al.rows_only = tc && (fp8 || p.off_xs >= 0);  // the GEMMs go by the table, the row passes by slot_pos
+  al.rows_only = tc;  // the GEMMs go by the table, the row passes by slot_pos
   al.from_sorted = route.slot_of != nullptr;
   int rc = route.slot_of ? run_align_sorted(al, slots, st) : run_align(al, st);
   if (rc) return rc;
@@ -360,7 +353,7 @@ int run_fused(const fmoe_fused_args& args, const RouteArgs& route, const FusedPl
 
   if (!fp8) {
     g1.dtype = g1.out_dtype = g2.dtype = a.dtype;
-    if (tc && p.off_xs >= 0) {
+    if (tc) {
       void* xs = ws + p.off_xs;
       rc = run_scatter_rows(a.hidden, (int)eb, a.T, a.top_k, a.H, slot_pos, xs, st);
       if (rc) return rc;

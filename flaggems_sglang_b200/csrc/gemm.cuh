@@ -1,7 +1,6 @@
 // Internal interface between the C-ABI entry points (api.cu) and the three
 // grouped-GEMM kernel families.
 #pragma once
-#include <cstdlib>
 
 #include "common.cuh"
 
@@ -41,10 +40,6 @@ bool gemm_pair_fold_supports(const GemmParams& p, bool gated);
 
 // Token tiles per group: the group's token rows should stay around 16 MB (hot in L2 across the weight tiles).
 inline int pick_group_m(int64_t block_rows, int64_t k_bytes_per_row) {
-  if (const char* env = getenv("FMOE_TC_GROUP_M")) {  // tuning aid
-    const int g = atoi(env);
-    if (g >= 1 && g <= 1024) return g;
-  }
   const int64_t per_block = block_rows * k_bytes_per_row;
   int64_t g = (16ll << 20) / (per_block > 0 ? per_block : 1);
   return (int)(g < 8 ? 8 : (g > 64 ? 64 : g));

@@ -13,7 +13,6 @@
 // items to fill the GPU, 2/4/8 warps of a CTA share an item, split K in chunks of 128 and
 // are reduced through shared memory in a fixed order (bit-reproducible).  gemm1 pairs 16
 // gate rows with the matching 16 up rows so that silu(gate)*up is applied in registers.
-#include <cstdlib>
 
 #include "gemm.cuh"
 
@@ -284,11 +283,6 @@ grouped_gemm_stream_kernel(GemmParams p, int W, int n_slabs) {
 
 // Warps per item: enough warps in flight to cover HBM latency, but at least two 128-k chunks per warp.
 int pick_ksplit(int64_t items, int64_t kblocks, int elem_bytes) {
-  // FMOE_STREAM_W=1|2|4|8 forces the split (tuning aid)
-  if (const char* env = getenv("FMOE_STREAM_W")) {
-    int w = atoi(env);
-    if (w == 1 || w == 2 || w == 4 || w == 8) return w;
-  }
   // Measured on B200: with 2-byte elements a warp touches 256 contiguous bytes of a row per step and, for long
   // reductions (Mixtral: 32 and 112 chunks of 128), HBM streams best when the warps of a CTA walk one row range
   // together (W = 8 gives 2 KB runs).  For short reductions (Qwen3 2048 / 768, the reference's test shape 1280 /

@@ -347,8 +347,7 @@ def _experts(hidden_states, w1, w2, topk_weights, topk_ids, route, k, inplace=Fa
     z_args = dict(out=_C.ptr(z), out_rows=_C.ptr(out_rows))
 
     if not use_fp8_w8a8:
-        if name == "tcgen05" and not os.environ.get("FMOE_TC_GATHER4"):
-            # sorted copy of the input rows (FMOE_TC_GATHER4=1: the gate/up GEMM gathers them by TMA instead)
+        if name == "tcgen05":  # sorted copy of the input rows
             xs = torch.empty((cap, H), dtype=out_dtype, device=dev)
             with _stage("gather_rows"):
                 _C.check(lib.fmoe_gather_rows(x.data_ptr(), x.element_size(), cap, H, sorted_ids.data_ptr(), k, numel,
