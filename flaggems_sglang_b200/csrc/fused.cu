@@ -27,9 +27,11 @@ int pick_variant(int dtype, int64_t numel, int E, int64_t I, int64_t H, int forc
                                         : (I % 128 == 0 && H % 128 == 0);
   int v = forced;
   if (v == FMOE_VARIANT_AUTO) {
-    // measured on B200: up to 4 rows per expert the two families tie (both stream the weights once at ~90 % of
-    // HBM bandwidth) and the streaming kernel wins on tile quantisation for a handful of experts; above that the
-    // 128-row tensor-core tiles win (DeepSeek-V3 T=256: 1.49 against 2.11 ms)
+    // Both families read the weights of every expert once, at about 90 % of the HBM rate, up to the rows of a streaming block:
+    // from 4 to 5 rows that block doubles and the streaming kernel slows down.  Layer calls, stream / pairs in us, at 4, 5 and
+    // 6 rows: Qwen3 212/207, 254/219, 262/209; half of it 117/129, 137/140, 142/132; a quarter of Mixtral 133/136, 165/136,
+    // 165/136.  (The one-call layer takes the pairs at fewer rows too where they win: layer_prefers_pairs, every e4m3 call
+    // among them.  The expert-parallel layer lays its receive area out by this choice.)
     if (stream_ok && ((dtype == FMOE_BF16 ? rows <= 4.0 : rows < 4.0) || !tc_ok)) v = FMOE_VARIANT_STREAM;
     else if (tc_ok) v = FMOE_VARIANT_TCGEN05;
     else v = FMOE_VARIANT_SIMT;
@@ -59,20 +61,23 @@ inline int64_t up256(int64_t v) { return (v + 255) & ~int64_t(255); }
 }
 
 // The whole layer on the CTA-pair GEMMs although an expert has few rows.  Both families read the weights once; the pair
-// kernels stream them 3-15 % faster but cost a row copy and a longer prologue, 5-15 us.  Measured per layer, stream / pairs
+// kernels stream them up to 15 % faster but cost a row copy and a longer prologue, 5-15 us.  Measured per layer, stream / pairs
 // in us:
-//   e4m3            DeepSeek-V3 9 tokens 510 / 447, 64 tokens 1203 / 1031, a rank's quarter with 20 tokens 239 / 223
+//   e4m3            DeepSeek-V3 9 tokens 510 / 447, 64 tokens 1203 / 1031, a rank's eighth with 9 to 16 tokens 262 / 243
 //   not x128        (the streaming kernel masks its loads) GPT-OSS 9 tokens 257 / 220, half of it 135 / 126
-//   2.8 GB          Mixtral 4 tokens 364 / 360, 16 tokens 486 / 460
-//   1.2-1.5 GB      3 rows and more: Qwen3 52 tokens 210 / 205, reference shape 24 tokens 253 / 252; below: Qwen3 40 tokens
-//                   198 / 200, reference shape 17 tokens 232 / 235, 10 tokens 193 / 199
-//   0.6-0.7 GB      half of Qwen3, 64 tokens 119 / 134; a quarter of Mixtral, 12 tokens 137 / 140
+//   0.6-0.7 GB      half of Qwen3, 64 tokens 119 / 134; a quarter of Mixtral, 12 tokens 117 / 122
+//   1.2 GB and more, 3 rows and more: Qwen3 64 tokens 212 / 207, reference shape 24 tokens 248 / 243, 64 experts of 2560 x 2048
+//                   313 / 313, 16 of 4096 x 6144 385 / 351, Mixtral 12 tokens 467 / 438
+//   1.2 GB and more, below: H or I of 4096 and more (the streaming kernel cuts its K loop between 8 warps) 8 experts of 4096 x
+//                   6144 200 / 191, x 9216 311 / 291, Mixtral 459 / 436, 16 of 4096 x 4096 266 / 253, 32 of 2048 x 4096
+//                   215 / 207, 8 of 2048 x 12288 181 / 182; smaller 64 of 2048 x 2048 228 / 237, of 3072 x 2304 369 / 371,
+//                   32 of 3072 x 3072 229 / 236, Qwen3 191 / 191, 128 of 2048 x 1536 277 / 278 and 329 / 324
 bool layer_prefers_pairs(const fmoe_fused_args& a, int64_t numel) {
   if (a.dtype == FMOE_E4M3) return true;  // sizes are multiples of 128
   if (a.H % 32 || a.I % 32) return false;
   if (a.H % 128 || a.I % 128) return true;
   const int64_t active = std::min<int64_t>(a.num_experts, numel), bytes = active * 6 * a.H * a.I;
-  return bytes >= 2400000000ll || (bytes >= 1200000000ll && numel >= 3 * active);
+  return bytes >= 1200000000ll && (numel >= 3 * active || std::max(a.H, a.I) >= 4096);
 }
 
 int plan_fused(const fmoe_fused_args& a, const RouteArgs& route, FusedPlan* pl) {

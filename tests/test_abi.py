@@ -66,6 +66,9 @@ def test_block_scale_workspace_has_no_row_per_position_in_fp32(lib, T):
 
 @pytest.mark.parametrize("dtype,T,E,H,I,k,want", [
     ("BF16", 1, 128, 2048, 768, 8, "decode"), ("BF16", 9, 128, 2048, 768, 8, "stream"), ("BF16", 16, 8, 4096, 14336, 2, "tcgen05"),
+    # fewer than 3 rows per expert: long rows, short rows, little weight; 3 rows
+    ("BF16", 10, 8, 4096, 7168, 2, "tcgen05"), ("BF16", 16, 64, 3072, 2304, 8, "stream"), ("BF16", 10, 8, 4096, 3584, 2, "stream"),
+    ("BF16", 24, 64, 3072, 2304, 8, "tcgen05"),
     ("E4M3", 8, 256, 7168, 2048, 8, "decode"), ("E4M3", 64, 256, 7168, 2048, 8, "tcgen05"), ("F32", 3, 8, 256, 512, 2, "simt")])
 def test_layer_variant_is_what_the_one_call_layer_takes(lib, dtype, T, E, H, I, k, want):
     """Stage names come from here: the choice of the one-call layer, which is not that of GEMMs launched one by one
