@@ -31,7 +31,10 @@ int validate_gemm(const GemmParams& a, bool gated, const char* who) {
   FMOE_REQUIRE(a.num_experts >= 1 && a.top_k >= 1 && a.block_size >= 1, "%s: bad E/top_k/block_size", who);
   FMOE_REQUIRE(a.activation == FMOE_ACT_SILU || a.activation == FMOE_ACT_GELU || a.activation == FMOE_ACT_SWIGLU_OAI,
                "%s: unknown activation %d", who, a.activation);
-  FMOE_REQUIRE(a.w_layout == FMOE_W_K_MAJOR || a.w_layout == FMOE_W_N_MAJOR, "%s: unknown w_layout %d", who, a.w_layout);
+  FMOE_REQUIRE(a.w_layout == FMOE_W_K_MAJOR || a.w_layout == FMOE_W_N_MAJOR || a.w_layout == FMOE_W_INTERLEAVED,
+               "%s: unknown w_layout %d", who, a.w_layout);
+  if (a.w_layout == FMOE_W_INTERLEAVED && (!gated || a.dtype == FMOE_E4M3))
+    return fail(FMOE_ERR_UNSUPPORTED, "%s: interleaved gate and up rows (FMOE_W_INTERLEAVED) are read by gemm1 with bf16 or f32", who);
   if (a.w_layout == FMOE_W_N_MAJOR) {
     if (a.dtype != FMOE_BF16 || (a.variant != FMOE_VARIANT_AUTO && a.variant != FMOE_VARIANT_TCGEN05))
       return fail(FMOE_ERR_UNSUPPORTED, "%s: [E,K,N] weights (FMOE_W_N_MAJOR) are read by the bf16 TCGEN05 kernel only", who);

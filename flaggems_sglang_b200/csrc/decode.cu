@@ -202,7 +202,7 @@ struct LayerParams {
   int32_t* tickets;        // next share: gate/up [0, shares), down [shares, 2 shares)
   int64_t H, I;
   int T, k, E, shares;
-  int on_input, activation, no_combine;
+  int on_input, activation, no_combine, interleaved;
   float act_alpha, act_limit, scale;
   int stages, x_bytes;
   int n_red, n_epi, tp, red_bytes;  // partial sums in the ring, epilogue warps at work, token columns of a partial sum
@@ -358,7 +358,9 @@ decode_layer_kernel(const __grid_constant__ CUtensorMap map1, const __grid_const
               break;
             }
             ptx::mbar_arrive_expect_tx(&full_bar[stage], STAGE_BYTES);
-            if (sh.gemm == 0) tma_load_5d(ring + stage * STAGE_BYTES, &map1, 0, 0, 2 * e, s, piece, &full_bar[stage]);
+            if (sh.gemm == 0)
+              tma_load_5d(ring + stage * STAGE_BYTES, &map1, 0, 0, p.interleaved ? 0 : 2 * e, p.interleaved ? e * units1 + s : s, piece,
+                          &full_bar[stage]);
             else tma_load_4d(ring + stage * STAGE_BYTES, &map2, 0, 0, e * units2 + s, piece, &full_bar[stage]);
             if (++stage == stages) {
               stage = 0;
@@ -438,9 +440,9 @@ decode_layer_kernel(const __grid_constant__ CUtensorMap map1, const __grid_const
           for (int i = 0; i < 2; ++i) {
             if (slot >= 0 && lane + 32 * i < outs) {
               const int64_t ch = (int64_t)s * 8 + row_i + row_step * i;
-              const float* bias = p.b1 ? p.b1 + (int64_t)expert * 2 * p.I + ch : nullptr;
-              const float o = gated_output<false>(sum[i], sum_up[i], bias ? bias[0] : 0.f, bias ? bias[p.I] : 0.f, wt, p.activation,
-                                                  p.act_alpha, p.act_limit);
+              const float* bias = p.b1 ? p.b1 + (int64_t)expert * 2 * p.I + (p.interleaved ? 2 * ch : ch) : nullptr;
+              const float o = gated_output<false>(sum[i], sum_up[i], bias ? bias[0] : 0.f, bias ? bias[p.interleaved ? 1 : p.I] : 0.f, wt,
+                                                  p.activation, p.act_alpha, p.act_limit);
               const int64_t at = ((int64_t)block * 8 + tok_i) * p.I + ch;
               if constexpr (EB == 2) reinterpret_cast<__nv_bfloat16*>(p.act)[at] = __float2bfloat16_rn(o);
               else reinterpret_cast<float*>(p.act)[at] = o;
@@ -660,11 +662,14 @@ int launch_layer(const fmoe_fused_args& a, const LayerParams& p, int smem, cudaS
     return cudaFuncSetAttribute(decode_layer_kernel<EB>, cudaFuncAttributeMaxDynamicSharedMemorySize, kMaxSmem);
   });
   if (err != cudaSuccess) return fail(FMOE_ERR_CUDA, "cudaFuncSetAttribute failed: %s", cudaGetErrorString(err));
-  // 128-byte pieces of 8 gate rows and their 8 up rows (gate and up halves of all experts in one dimension) / of 16 rows
+  // 128-byte pieces of 8 gate rows and their 8 up rows (gate and up halves of all experts in one dimension; where they
+  // alternate, the groups of 16 rows of all experts) / of 16 rows
   constexpr int PIECE = 128 / EB;
   const cuuint64_t row1 = (cuuint64_t)a.H * EB, row2 = (cuuint64_t)a.I * EB;
-  const cuuint64_t dims1[5] = {PIECE, 8, 2 * (cuuint64_t)a.num_experts, (cuuint64_t)a.I / 8, row1 / 128};
-  const cuuint64_t strides1[4] = {row1, row1 * a.I, row1 * 8, 128};
+  const cuuint64_t E = a.num_experts, groups = (cuuint64_t)a.I / 8;
+  const cuuint64_t dims1[5] = {PIECE, 8, p.interleaved ? 2 : 2 * E, p.interleaved ? E * groups : groups, row1 / 128};
+  const cuuint64_t strides1[4] = {p.interleaved ? row1 * 2 : row1, p.interleaved ? row1 : row1 * a.I,
+                                  p.interleaved ? row1 * 16 : row1 * 8, 128};
   const cuuint32_t box1[5] = {PIECE, 8, 2, 1, PIECES};
   const cuuint64_t dims2[4] = {PIECE, 16, (cuuint64_t)a.num_experts * (a.H / 16), row2 / 128};
   const cuuint64_t strides2[3] = {row2, row2 * 16, 128};
@@ -694,7 +699,7 @@ int status_word_decode(int* out, bool clear) {
 
 bool plan_decode(const fmoe_fused_args& a, const RouteArgs& r, DecodePlan* pl) {
   const bool fp8 = a.dtype == FMOE_E4M3;
-  if (a.variant != FMOE_VARIANT_AUTO || a.w_layout != FMOE_W_K_MAJOR || a.out_rows) return false;
+  if (a.variant != FMOE_VARIANT_AUTO || (a.w_layout != FMOE_W_K_MAJOR && a.w_layout != FMOE_W_INTERLEAVED) || a.out_rows) return false;
   if (a.dtype != FMOE_BF16 && !(fp8 && a.scale_mode == FMOE_SCALE_BLOCK128)) return false;
   if (a.no_combine && a.zero_dropped) return false;
   if (a.T < 1 || a.T > kDecodeTokens || a.top_k > 32 || a.num_experts > 1024) return false;
@@ -800,6 +805,7 @@ int run_decode(const fmoe_fused_args& a, const RouteArgs& r, const DecodePlan& p
   p.on_input = a.apply_router_weight_on_input;
   p.activation = a.activation;
   p.no_combine = a.no_combine;
+  p.interleaved = a.w_layout == FMOE_W_INTERLEAVED;
   p.act_alpha = a.act_alpha;
   p.act_limit = a.act_limit;
   p.scale = a.routed_scaling_factor == 0.f ? 1.0f : a.routed_scaling_factor;

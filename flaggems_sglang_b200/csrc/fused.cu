@@ -106,7 +106,10 @@ int plan_fused(const fmoe_fused_args& a, const RouteArgs& route, FusedPlan* pl) 
       FMOE_REQUIRE(a.H % 128 == 0 && a.I % 128 == 0, "fused_experts: e4m3 needs H and I to be multiples of 128");
     }
   }
-  FMOE_REQUIRE(a.w_layout == FMOE_W_K_MAJOR || a.w_layout == FMOE_W_N_MAJOR, "fused_experts: unknown w_layout %d", a.w_layout);
+  FMOE_REQUIRE(a.w_layout == FMOE_W_K_MAJOR || a.w_layout == FMOE_W_N_MAJOR || a.w_layout == FMOE_W_INTERLEAVED,
+               "fused_experts: unknown w_layout %d", a.w_layout);
+  if (a.w_layout == FMOE_W_INTERLEAVED && a.dtype == FMOE_E4M3)
+    return fail(FMOE_ERR_UNSUPPORTED, "fused_experts: interleaved gate and up rows (FMOE_W_INTERLEAVED) need bf16 or f32 weights");
   const bool n_major = a.w_layout == FMOE_W_N_MAJOR;
   if (n_major && (a.dtype != FMOE_BF16 || a.b1 || a.b2 || a.activation == FMOE_ACT_SWIGLU_OAI ||
                   (a.variant != FMOE_VARIANT_AUTO && a.variant != FMOE_VARIANT_TCGEN05)))
@@ -334,6 +337,7 @@ int run_fused(const fmoe_fused_args& args, const RouteArgs& route, const FusedPl
   g.token_tile = al.token_tile;
   g.skip_padding = true;  // nothing below reads a padding row's values
   GemmParams g1 = g, g2 = g;
+  if (a.w_layout == FMOE_W_INTERLEAVED) g2.w_layout = FMOE_W_K_MAJOR;
   g1.split_counters = counters;
   g2.split_counters = counters ? counters + kSplitCounters : nullptr;
   g1.n = a.I;

@@ -65,6 +65,7 @@ struct PairParams {
   const float* a_scale;   // F8: one scale per row of the sorted order, or per token (a_scale_gather)
   const float* w_scale;   // F8: [E, w_rows], one scale per output channel
   const float* bias;      // optional [E, w_rows]
+  int32_t vec_step, vec_up;  // gate/up: entry of channel c in w_scale / bias is c * vec_step, its up entry vec_up further
   void* out;
   void* const* out_rows;  // down projection: optional per-slot row addresses (may be peer memory)
   float* split_partials;    // tail split: [workers][2 CTAs][128][256] f32 partial accumulators (NULL: no split)
@@ -335,7 +336,7 @@ grouped_gemm_pair_kernel(const __grid_constant__ CUtensorMap map_t, const __grid
 #pragma unroll
           for (int i = 0; i < 4; ++i) {
             const int64_t c = GATED ? ch0 + g + 8 * (i & 1) : ch0 + g + 8 * i;
-            if (c < p.n) cv[i] = vec[c + (GATED && i >= 2 ? p.n : 0)];
+            if (c < p.n) cv[i] = GATED ? vec[c * p.vec_step + (i >= 2 ? p.vec_up : 0)] : vec[c];
           }
         }
       }
@@ -611,12 +612,15 @@ int pair_map_tokens(CUtensorMap* map, const void* base, int64_t rows, int64_t co
 }
 
 // weights [E, rows, K], K contiguous.  gated: rows = n gate rows then n up rows; the box takes 4 groups of 16 gate rows and
-// the 16 matching up rows (K, 16 rows, gate/up, row groups, expert: rows past n read as zeros).  plain: rows = n, 128 rows.
-int pair_map_weights(CUtensorMap* map, const void* base, int64_t experts, int64_t n, int64_t k, int elem_bytes, bool gated) {
+// the 16 matching up rows (K, 16 rows, gate/up, row groups, expert: rows past n read as zeros); interleaved: gate and up rows
+// alternate, the box is the same.  plain: rows = n, 128 rows.
+int pair_map_weights(CUtensorMap* map, const void* base, int64_t experts, int64_t n, int64_t k, int elem_bytes, bool gated,
+                     bool interleaved) {
   const cuuint64_t row = (cuuint64_t)k * elem_bytes;
   if (gated) {
     const cuuint64_t dims[5] = {(cuuint64_t)k, 16, 2, (cuuint64_t)(n / 16), (cuuint64_t)experts};
-    const cuuint64_t strides[4] = {row, row * n, row * 16, row * 2 * n};
+    const cuuint64_t strides[4] = {interleaved ? row * 2 : row, interleaved ? row : row * n, interleaved ? row * 32 : row * 16,
+                                   row * 2 * n};
     const cuuint32_t box[5] = {(cuuint32_t)(KBYTES / elem_bytes), 16, 2, 4, 1};
     return encode_tensor_map(map, base, elem_bytes, 5, dims, strides, box, true, "gate/up weights");
   }
@@ -650,11 +654,12 @@ int launch(const GemmParams& g, cudaStream_t st) {
     return fail(FMOE_ERR_CUDA, "cudaFuncSetAttribute(smem=%d) failed: %s", MAX_SMEM, cudaGetErrorString(attr_err));
 
   const int64_t w_rows = GATED ? 2 * g.n : g.n;
+  const bool interleaved = GATED && g.w_layout == FMOE_W_INTERLEAVED;
   CUtensorMap map_t, map_w;
   int rc = pair_map_tokens(&map_t, g.a, g.a_rows, g.k, ELEM, GATHER ? 1 : BOX_TOKENS);
   if (rc) return rc;
   if constexpr (WMN) rc = pair_map_weights_nmajor(&map_w, g.w, g.num_experts, g.k, w_rows);
-  else rc = pair_map_weights(&map_w, g.w, g.num_experts, g.n, g.k, ELEM, GATED);
+  else rc = pair_map_weights(&map_w, g.w, g.num_experts, g.n, g.k, ELEM, GATED, interleaved);
   if (rc) return rc;
 
   PairParams p;
@@ -667,6 +672,8 @@ int launch(const GemmParams& g, cudaStream_t st) {
   p.a_scale_gather = g.a_scale_gather;
   p.w_scale = g.w_scale;
   p.bias = g.bias;
+  p.vec_step = interleaved ? 2 : 1;
+  p.vec_up = interleaved ? 1 : (int32_t)g.n;
   p.act_alpha = g.act_alpha;
   p.act_limit = g.act_limit;
   p.out = g.out;
@@ -724,7 +731,7 @@ bool gemm_pair_supports(const GemmParams& p, bool gated) {
   if (p.block_size != 128) return false;
   // gather mode: gate/up GEMM only; one int4 of sorted ids per lane
   if (p.a_gather && (!gated || p.top_k < 1 || !aligned16(p.sorted_token_ids))) return false;
-  if (p.w_layout != FMOE_W_K_MAJOR && p.w_layout != FMOE_W_N_MAJOR) return false;
+  if (p.w_layout != FMOE_W_K_MAJOR && p.w_layout != FMOE_W_N_MAJOR && !(p.w_layout == FMOE_W_INTERLEAVED && gated)) return false;
   // weights in the reference operator's [E, K, N] layout: plain kernels only (no row gather, bias or swiglu_oai)
   if (p.w_layout == FMOE_W_N_MAJOR && (p.a_gather || p.bias || (gated && p.activation == FMOE_ACT_SWIGLU_OAI))) return false;
   if (p.k <= 0 || (p.k * (f8 ? 1 : 2)) % 16 != 0) return false;  // TMA row stride must be a multiple of 16 bytes

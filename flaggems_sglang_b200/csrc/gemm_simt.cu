@@ -27,8 +27,10 @@ grouped_gemm_simt_kernel(GemmParams p) {
   if (c >= p.n) return;
   const int64_t w_rows = GATED ? 2 * p.n : p.n;  // rows of w per expert
   const AT* w = reinterpret_cast<const AT*>(p.w) + (int64_t)e * w_rows * p.k;
-  const AT* wg = w + c * p.k;
-  const AT* wu = GATED ? w + (p.n + c) * p.k : nullptr;
+  const int64_t row_g = GATED && p.w_layout == FMOE_W_INTERLEAVED ? 2 * c : c;
+  const int64_t row_u = p.w_layout == FMOE_W_INTERLEAVED ? 2 * c + 1 : p.n + c;
+  const AT* wg = w + row_g * p.k;
+  const AT* wu = GATED ? w + row_u * p.k : nullptr;
   const int64_t kblocks = ceil_div<int64_t>(p.k, 128);
   const float* swg = nullptr;
   const float* swu = nullptr;
@@ -65,7 +67,7 @@ grouped_gemm_simt_kernel(GemmParams p) {
     const float* bias = p.bias ? p.bias + (int64_t)e * w_rows : nullptr;
     if constexpr (GATED) {
       reinterpret_cast<OutT*>(p.out)[pos * p.n + c] = from_f32<OutT>(gated_output<false>(
-          acc_g, acc_u, bias ? bias[c] : 0.f, bias ? bias[p.n + c] : 0.f, rs, p.activation, p.act_alpha, p.act_limit));
+          acc_g, acc_u, bias ? bias[row_g] : 0.f, bias ? bias[row_u] : 0.f, rs, p.activation, p.act_alpha, p.act_limit));
     } else {
       reinterpret_cast<OutT*>(p.out)[(int64_t)slot * p.n + c] = from_f32<OutT>((acc_g + (bias ? bias[c] : 0.f)) * rs);
     }

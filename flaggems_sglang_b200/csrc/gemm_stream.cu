@@ -72,6 +72,7 @@ grouped_gemm_stream_kernel(GemmParams p, int W, int n_slabs) {
   const int64_t n0 = (int64_t)slab * (GATED ? 16 : 32);
   const int64_t kblocks = (K + 127) / 128;  // bf16: the last chunk may be partial (its loads past K read as zero)
   const int64_t row_bytes = K * EB;
+  const bool interleaved = EB == 2 && p.w_layout == FMOE_W_INTERLEAVED;  // gate and up rows alternate
 
   float acc[RT][NTG][4];
 #pragma unroll
@@ -96,7 +97,9 @@ grouped_gemm_stream_kernel(GemmParams p, int W, int n_slabs) {
       slab_row0[rt] = GATED ? (rt == 0 ? n0 : p.n + n0) : n0 + 16 * rt;
 #pragma unroll
       for (int h = 0; h < 2; ++h) {
-        int64_t row = min(slab_row0[rt] + g + 8 * h, w_rows - 1);
+        int64_t row = slab_row0[rt] + g + 8 * h;
+        if (GATED && interleaved) row = 2 * (n0 + g + 8 * h) + rt;
+        row = min(row, w_rows - 1);
         wptr[rt][h] = reinterpret_cast<const uint8_t*>(p.w) + (((int64_t)e * w_rows + row) * K) * EB + t * 16;
       }
     }
@@ -265,10 +268,12 @@ grouped_gemm_stream_kernel(GemmParams p, int W, int n_slabs) {
       const int col = g + 8 * (i >> 1);
       const float* bias = p.bias ? p.bias + (int64_t)e * w_rows : nullptr;
       if constexpr (GATED) {
-        if (n0 + col < p.n)
-          out[(b * BM + q * 8 + 2 * t + (i & 1)) * p.n + n0 + col] = from_f32<OutT>(gated_output<false>(
-              acc[0][q][i], acc[1][q][i], bias ? bias[n0 + col] : 0.f, bias ? bias[p.n + n0 + col] : 0.f, rs,
-              p.activation, p.act_alpha, p.act_limit));
+        if (n0 + col < p.n) {
+          const int64_t c = n0 + col;
+          out[(b * BM + q * 8 + 2 * t + (i & 1)) * p.n + c] = from_f32<OutT>(gated_output<false>(
+              acc[0][q][i], acc[1][q][i], bias ? bias[interleaved ? 2 * c : c] : 0.f,
+              bias ? bias[interleaved ? 2 * c + 1 : p.n + c] : 0.f, rs, p.activation, p.act_alpha, p.act_limit));
+        }
       } else {
         OutT* orow = p.out_rows ? reinterpret_cast<OutT*>(p.out_rows[slot]) : out + (int64_t)slot * p.n;
         if (!orow) continue;

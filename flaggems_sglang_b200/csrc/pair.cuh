@@ -252,7 +252,8 @@ struct UnitPlan {
 int encode_tensor_map(CUtensorMap* map, const void* base, int elem_bytes, int rank, const cuuint64_t* dims,
                       const cuuint64_t* strides, const cuuint32_t* box, bool weights, const char* what);
 int pair_map_tokens(CUtensorMap* map, const void* base, int64_t rows, int64_t cols, int elem_bytes, int box_rows);
-int pair_map_weights(CUtensorMap* map, const void* base, int64_t experts, int64_t n, int64_t k, int elem_bytes, bool gated);
+int pair_map_weights(CUtensorMap* map, const void* base, int64_t experts, int64_t n, int64_t k, int elem_bytes, bool gated,
+                     bool interleaved = false);
 int pair_map_weights_nmajor(CUtensorMap* map, const void* base, int64_t experts, int64_t k, int64_t w_rows);
 int device_sm_count();
 

@@ -168,6 +168,7 @@ def fused_experts(
     gemm1_alpha: Optional[float] = None,
     gemm1_clamp_limit: Optional[float] = None,
     weights_n_major: bool = False,
+    w1_interleaved: bool = False,
 ) -> torch.Tensor:
     """Expert computation for already-routed tokens.
 
@@ -190,18 +191,20 @@ def fused_experts(
     `weights_n_major=True`: w1 is [E,H,2I] and w2 [E,I,H] (the layout the reference operator takes,
     src/flaggems_sglang/ops/fused_moe.py:192-199), read in place by the bf16 tensor-core kernels as an N-major
     operand; see `n_major_supported` for the shapes this covers.
+    `w1_interleaved=True`: gate and up rows of w1 (and entries of b1) alternate, gate first, as the layers of the bias
+    variant hold them; read in place.  bf16 / fp32 weights.
     """
     return _experts(hidden_states, w1, w2, topk_weights, topk_ids, None, topk_ids.shape[1] if topk_ids.ndim == 2 else 0, inplace,
                     activation, apply_router_weight_on_input, use_fp8_w8a8, per_channel_quant, w1_scale, w2_scale, a1_scale,
                     a2_scale, block_shape, no_combine, routed_scaling_factor, expert_map, variant, out_rows, b1, b2, gemm1_alpha,
-                    gemm1_clamp_limit, weights_n_major)
+                    gemm1_clamp_limit, weights_n_major, w1_interleaved=w1_interleaved)
 
 
 def _experts(hidden_states, w1, w2, topk_weights, topk_ids, route, k, inplace=False, activation="silu",
              apply_router_weight_on_input=False, use_fp8_w8a8=False, per_channel_quant=False, w1_scale=None, w2_scale=None,
              a1_scale=None, a2_scale=None, block_shape=None, no_combine=False, routed_scaling_factor=None, expert_map=None,
              variant=None, out_rows=None, b1=None, b2=None, gemm1_alpha=None, gemm1_clamp_limit=None, weights_n_major=False,
-             triple=None):
+             triple=None, w1_interleaved=False):
     """`fused_experts`; with `route` (a filled _C.RouteArgs: logits of [T,E]) the router and the experts in one call, with
     `triple` (positions -> slots, rows per expert, weights of the sorted positions) a routing that is already in expert order."""
     logger.debug("FLAGGEMS_SGLANG_B200 FUSED_EXPERTS")
@@ -225,6 +228,8 @@ def _experts(hidden_states, w1, w2, topk_weights, topk_ids, route, k, inplace=Fa
     I = twoI // 2
     assert Hw == H, "hidden size mismatch"
     assert w2.shape[0] == E and w2.shape[1] == H and w2.shape[2] == I, "intermediate size mismatch"
+    assert not (w1_interleaved and (weights_n_major or use_fp8_w8a8)), "w1_interleaved needs bf16 or fp32 [E,2I,H] weights"
+    w_layout = _C.W_N_MAJOR if weights_n_major else (_C.W_INTERLEAVED if w1_interleaved else _C.W_K_MAJOR)
     routed_here = route is not None or triple is not None
     assert routed_here or (topk_ids.shape == topk_weights.shape and topk_ids.shape[0] == T), "topk shape mismatch"
     numel = T * k
@@ -289,7 +294,7 @@ def _experts(hidden_states, w1, w2, topk_weights, topk_ids, route, k, inplace=Fa
     if forced not in _C.VARIANTS:
         raise ValueError(f"unknown variant {forced!r}")
     fa = _C.FusedArgs(
-        w_layout=_C.W_N_MAJOR if weights_n_major else _C.W_K_MAJOR,
+        w_layout=w_layout,
         scale_mode=_C.SCALE_CHANNEL if per_channel_quant else _C.SCALE_BLOCK128,
         dtype=_C.E4M3 if use_fp8_w8a8 else _C.DTYPE_CODE[out_dtype], variant=_C.VARIANTS[forced], num_experts=E,
         top_k=k, apply_router_weight_on_input=int(apply_router_weight_on_input), no_combine=int(no_combine),
@@ -356,7 +361,7 @@ def _experts(hidden_states, w1, w2, topk_weights, topk_ids, route, k, inplace=Fa
         else:
             a_ptr, a_rows, gather = x.data_ptr(), T, 1
         act = torch.empty((cap, I), dtype=out_dtype, device=dev)
-        g1 = _gemm_args(dtype=code, out_dtype=code, a_gather=gather, n=I, k=H, a_rows=a_rows, a=a_ptr,
+        g1 = _gemm_args(w_layout=w_layout, dtype=code, out_dtype=code, a_gather=gather, n=I, k=H, a_rows=a_rows, a=a_ptr,
                         w=w1.data_ptr(), row_scale=row_w if apply_router_weight_on_input else None,
                         out=act.data_ptr(), bias=_C.ptr(b1), act_alpha=act_alpha, act_limit=act_limit, **common)
         with _stage("gemm1_" + name):
@@ -448,7 +453,7 @@ def _experts(hidden_states, w1, w2, topk_weights, topk_ids, route, k, inplace=Fa
 # fused_experts' options that the one-call layer takes (global_num_experts is accepted there and has no effect)
 _EXPERT_OPTIONS = frozenset(("inplace", "activation", "apply_router_weight_on_input", "use_fp8_w8a8", "per_channel_quant",
                              "w1_scale", "w2_scale", "a1_scale", "a2_scale", "block_shape", "no_combine", "variant", "b1", "b2",
-                             "gemm1_alpha", "gemm1_clamp_limit", "weights_n_major"))
+                             "gemm1_alpha", "gemm1_clamp_limit", "weights_n_major", "w1_interleaved"))
 
 
 def fused_moe(
@@ -592,14 +597,6 @@ def triton_kernel_fused_experts(
                         apply_router_weight_on_input=apply_router_weight_on_input)
 
 
-def _split_interleaved(w13_rows: torch.Tensor, b13: Optional[torch.Tensor]):
-    """[E,2I,H] with gate and linear rows interleaved (even = gate), b13 [E,2I] likewise -> the same tensors with
-    the I gate rows first, the layout of this package's gate/up kernels.  One copy of w13."""
-    w = torch.cat((w13_rows[:, 0::2], w13_rows[:, 1::2]), dim=1).contiguous()
-    b = None if b13 is None else torch.cat((b13[:, 0::2], b13[:, 1::2]), dim=1)
-    return w, b
-
-
 def triton_kernel_fused_experts_with_bias(
     hidden_states: torch.Tensor,
     w1: torch.Tensor,
@@ -629,7 +626,7 @@ def triton_kernel_fused_experts_with_bias(
         z[p,:] = (y[p,:] . w2[e] + b2[e]) * g_out[p],      out[t] = sum over the k rows of token t
 
     w1 [E,H,2I] holds gate and linear columns interleaved (even = gate), b1 [E,2I] likewise, as that library
-    expects; they are split into the [gate rows; up rows] layout of this package's kernels once per call.
+    expects, and is read in place when it is the transposed view of a serving-side [E,2I,H] weight.
     `activation="silu"` names this swiglu, as in the reference; alpha defaults to 1.702.  The precision
     configs are accepted for signature compatibility and must be None (bf16 only).
     """
@@ -641,30 +638,14 @@ def triton_kernel_fused_experts_with_bias(
         raise ValueError(f"Unsupported FusedMoe activation: {activation}")
     assert w1.dtype == torch.bfloat16 and w2.dtype == torch.bfloat16, "w1/w2 must be bfloat16"
     assert hidden_states.shape[-1] == w1.shape[-2], "hidden size mismatch"
-    w1_split, b1_split = _split_interleaved(w1.transpose(1, 2), b1)
-    return _from_triple(hidden_states, w1_split, _k_major(w2), routing_data, gather_indx, scatter_indx, "swiglu_oai",
-                        apply_router_weight_on_input=apply_router_weight_on_input, b1=b1_split, b2=b2,
-                        gemm1_alpha=gemm1_alpha, gemm1_clamp_limit=gemm1_clamp_limit)
+    return _from_triple(hidden_states, _k_major(w1), _k_major(w2), routing_data, gather_indx, scatter_indx, "swiglu_oai",
+                        apply_router_weight_on_input=apply_router_weight_on_input, b1=b1, b2=b2,
+                        gemm1_alpha=gemm1_alpha, gemm1_clamp_limit=gemm1_clamp_limit, w1_interleaved=True)
 
 
 @dataclass
 class StandardCombineInput:
     hidden_states: torch.Tensor
-
-
-def _split_interleaved_cached(layer, b13):
-    """`_split_interleaved` of the layer's w13 / bias, kept on the layer until either tensor is replaced or
-    modified in place (data pointer and version counter), so that the copy is not repeated on every call."""
-    w = layer.w13_weight
-    key = (w.data_ptr(), w._version, tuple(w.shape), b13.data_ptr(), b13._version)
-    cached = getattr(layer, "_fmoe_split_w13", None)
-    if cached is None or cached[0] != key:
-        cached = (key, _split_interleaved(w, b13))
-        try:
-            layer._fmoe_split_w13 = cached
-        except Exception:  # noqa: BLE001  (a layer object that refuses new attributes: split per call)
-            pass
-    return cached[1]
 
 
 def _standard_output_type():
@@ -703,12 +684,11 @@ def fused_moe_flagos(obj, layer: torch.nn.Module, dispatch_output):
         assert b13 is not None and b2 is not None, "Bias execution requires both w13_bias and w2_bias"
         alpha, limit = getattr(cfg, "gemm1_alpha", None), getattr(cfg, "gemm1_clamp_limit", None)
         if hasattr(topk_output, "topk_weights"):
-            w13, b13s = _split_interleaved_cached(layer, b13)
             out = fused_experts(
-                hidden_states, w13, layer.w2_weight, topk_output.topk_weights, topk_output.topk_ids,
+                hidden_states, layer.w13_weight, layer.w2_weight, topk_output.topk_weights, topk_output.topk_ids,
                 activation="swiglu_oai", apply_router_weight_on_input=cfg.apply_router_weight_on_input,
                 routed_scaling_factor=cfg.routed_scaling_factor,
-                b1=b13s, b2=b2, gemm1_alpha=alpha, gemm1_clamp_limit=limit,
+                b1=b13, b2=b2, gemm1_alpha=alpha, gemm1_clamp_limit=limit, w1_interleaved=True,
             )
         else:
             routing_data, gather_indx, scatter_indx = topk_output

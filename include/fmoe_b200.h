@@ -159,10 +159,13 @@ int fmoe_gather_rows(const void* x, int elem_bytes, int64_t rows_out, int64_t K,
 #define FMOE_SCALE_CHANNEL 1
 #define FMOE_W_K_MAJOR 0
 #define FMOE_W_N_MAJOR 1
+#define FMOE_W_INTERLEAVED 2 /* as FMOE_W_K_MAJOR, but gate and up rows of w1 (and entries of its bias) alternate, gate first:
+                                the serving-side layout of the bias variant (src/flaggems_sglang/ops/fused_moe.py:380-398).
+                                bf16 and f32; gemm1 only, w2 is as with FMOE_W_K_MAJOR                           */
 typedef struct fmoe_gemm_args {
   uint32_t struct_size;/* sizeof(fmoe_gemm_args) as the CALLER compiled it; a size the library does not know is
                           refused with FMOE_ERR_INVALID_ARG before any other field is read   */
-  int32_t w_layout;    /* FMOE_W_K_MAJOR (0) | FMOE_W_N_MAJOR: see `w`                   */
+  int32_t w_layout;    /* FMOE_W_K_MAJOR (0) | FMOE_W_N_MAJOR: see `w` | FMOE_W_INTERLEAVED */
   int32_t dtype;       /* FMOE_F32 | FMOE_BF16 | FMOE_E4M3: type of a and w            */
   int32_t out_dtype;   /* FMOE_F32 | FMOE_BF16 | FMOE_E4M3 (gemm1+TCGEN05 fp8 only)     */
   int32_t variant;     /* FMOE_VARIANT_*                                                 */
@@ -250,7 +253,8 @@ int fmoe_moe_sum_add(const void* z, int dtype, int64_t T, int k, int64_t H, floa
 typedef struct fmoe_fused_args {
   uint32_t struct_size; /* sizeof(fmoe_fused_args) as the caller compiled it (checked like fmoe_gemm_args.struct_size) */
   int32_t w_layout;     /* FMOE_W_K_MAJOR: w1 [E,2I,H], w2 [E,H,I]; FMOE_W_N_MAJOR: w1 [E,H,2I], w2 [E,I,H] (bf16,
-                           TCGEN05 kernels, no bias / swiglu_oai)                                          */
+                           TCGEN05 kernels, no bias / swiglu_oai); FMOE_W_INTERLEAVED: gate and up rows of w1 and entries
+                           of b1 alternate (bf16, f32)                                                      */
   int32_t dtype;        /* FMOE_F32 | FMOE_BF16: type of hidden/w1/w2/out; FMOE_E4M3: e4m3 weights with
                            128x128 scales, bf16 hidden/out, activations quantised per token per 128 channels */
   int32_t variant;      /* FMOE_VARIANT_* (AUTO: chosen from the shape)                                   */

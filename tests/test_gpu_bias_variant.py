@@ -107,6 +107,46 @@ def test_bias_variant_is_refused_with_fp8_weights(fg):
                          w2_scale=s2.cuda(), block_shape=[128, 128], b1=b1.cuda())
 
 
+@pytest.mark.parametrize("variant,T,H,I,dtype", [
+    ("simt", 9, 96, 160, torch.float32), ("simt", 9, 96, 160, torch.bfloat16), ("stream", 20, 352, 160, torch.bfloat16),
+    ("stream", 20, 256, 128, torch.bfloat16), ("tcgen05", 70, 352, 160, torch.bfloat16), ("tcgen05", 300, 256, 384, torch.bfloat16),
+    (None, 1, 256, 128, torch.bfloat16), (None, 8, 640, 320, torch.bfloat16)])
+def test_interleaved_rows_are_the_same_layer(fg, variant, T, H, I, dtype):
+    """Gate and up rows that alternate are read in place by every kernel family (None: the decode kernels): same products, same
+    order, so the bits of the layer with the gate rows first."""
+    E, k = 8, 2
+    x, w1, w2, b1, b2, logits = _layer(T, H, I, E, 50 + T, dtype)
+    tw, ti = OR.softmax_topk(logits, k, True)
+    alternate = lambda v: torch.stack((v[:, :I], v[:, I:]), dim=2).flatten(1, 2).contiguous()  # noqa: E731
+    run = lambda w, b, **kw: fg.fused_experts(x.cuda(), w.cuda(), w2.cuda(), tw.cuda(), ti.cuda(), variant=variant, **kw,  # noqa: E731
+                                              **({} if b is None else dict(b1=b.cuda(), b2=b2.cuda(), gemm1_clamp_limit=7.0)))
+    for b, act in ((b1, "swiglu_oai"), (None, "silu")):
+        ref = run(w1, b, activation=act)
+        assert torch.equal(run(alternate(w1), None if b is None else alternate(b), activation=act, w1_interleaved=True), ref)
+    assert_close_moe(ref, OE.fused_experts(x, w1, w2, tw, ti), "bf16" if dtype == torch.bfloat16 else "fp32", f"interleaved {variant} T={T}")
+
+
+@pytest.mark.parametrize("T", [1, 21, 300])
+def test_hook_reads_the_weights_that_the_layer_holds_now(fg, T):
+    """Weights written in place through `.data`, which no version counter sees (how weights are loaded anew while serving)."""
+    from types import SimpleNamespace as NS
+
+    E, H, I, k = 8, 256, 128, 2
+    a, b = (_layer(T, H, I, E, s) for s in (60, 61))
+    tw, ti = OR.softmax_topk(a[5], k, True)
+    cfg = NS(num_experts=E, activation="silu", apply_router_weight_on_input=False, no_combine=False, routed_scaling_factor=None,
+             gemm1_alpha=1.702, gemm1_clamp_limit=7.0)
+    layer = lambda v: NS(**{n: torch.nn.Parameter(t.cuda(), requires_grad=False) for n, t in  # noqa: E731
+                            zip(("w13_weight", "w2_weight", "w13_weight_bias", "w2_weight_bias"), v[1:5])})
+    run = lambda lay: fg.fused_moe_flagos(NS(runner=NS(config=cfg)), lay, NS(  # noqa: E731
+        hidden_states=a[0].cuda(), topk_output=NS(topk_weights=tw.cuda(), topk_ids=ti.cuda()))).hidden_states
+    held, fresh = layer(a), layer(b)
+    run(held)
+    for n in vars(held):
+        getattr(held, n).data.copy_(getattr(fresh, n).data)
+    assert torch.equal(run(held), run(fresh))
+
+
 def test_hook_routes_biased_layers_to_the_bias_variant(fg):
     """`fused_moe_flagos` with `w13_weight_bias` / `w2_weight_bias` on the layer (reference hook :380-398): the
     serving-side w13 [E,2I,H] holds gate and linear rows interleaved."""
