@@ -1,4 +1,5 @@
-// Decode-sized layer: up to 8 tokens, bf16 or e4m3 (128x128 block scales) weights with K contiguous, two kernels.
+// Decode-sized layer: up to 8 tokens, bf16 or e4m3 (128x128 block scales) weights with K contiguous, two kernels.  Gate and up rows
+// of w1 may alternate (FMOE_W_INTERLEAVED): the gate/up tensor map then has other strides, the box is the same.
 //
 // A call of this size is the reading of the chosen experts' weights and little else: 75 MB for one token of a layer with
 // 8 x (2048, 768) experts, 11.7 us at the copy rate of the card.  As five or six kernels (router, align, quantiser, two
@@ -6,9 +7,9 @@
 //
 //   decode_prepare_kernel : CTA 0 routes the tokens (or takes the given ids) and lists the active experts with their slots;
 //                           it clears the counters; the other CTAs quantise the hidden rows (e4m3)
-//   decode_layer_kernel   : one CTA per SM: 8 compute warps, a producer warp, 8 epilogue warps.  Both GEMMs in one kernel: the weights of
-//                           a CTA's share of the gate/up GEMM, then of the down GEMM, stream through ONE ring of bulk
-//                           copies in shared memory that keeps filling across the dependency between the two, so HBM
+//   decode_layer_kernel   : one CTA per SM: 12 compute warps, a producer warp, 8 epilogue warps.  Both GEMMs in one kernel: the
+//                           weights of a CTA's share of the gate/up GEMM, then of the down GEMM, stream through ONE ring of
+//                           bulk copies in shared memory that keeps filling across the dependency between the two, so HBM
 //                           does not idle there.  A down unit waits for its expert's activations only (a counter per
 //                           expert), and the last unit of a 16-channel slab sums the slab over the slots (moe_sum).
 //

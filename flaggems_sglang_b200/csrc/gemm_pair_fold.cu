@@ -18,7 +18,7 @@
 //               2190 -> 2005 us per layer.)  The gate/up output is fp32, for the quantiser behind it
 //   warp 16   : TMA producer      warp 17 : MMA issuer (CTA 0)
 //   warps 18-19: factors.  For four K blocks at a time they multiply the tokens' scales with the tile's one or two weight
-//               scales and leave the products in a 3-slot ring in shared memory, next to the tile's slots and row weights:
+//               scales and leave the products in a 4-slot ring in shared memory, next to the tile's slots and row weights:
 //               the fold warps read one 8-byte pair per two tokens and keep no pointers
 // What bounds it: HBM (the weights stream through a ring of 20 KB stages) up to about 8 rows per expert, the fold above.
 #include "pair.cuh"
@@ -879,7 +879,7 @@ grouped_gemm_pair_fold_wide_kernel(const __grid_constant__ CUtensorMap map_t, co
   } else {
     // ---------------- fold + epilogue (warps 0-15) ----------------
     if constexpr (MOVE) asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(kFoldRegs));
-    // This loop runs at the 96 registers that 20 warps leave a thread: the tile is described by its meta entry, shared
+    // This loop runs at 104 registers (96 where the move is left out): the tile is described by its meta entry, shared
     // memory addresses are constants, everything else is derived from three counters.
     const uint32_t lane_addr = tmem_base + ((uint32_t)((warp & 3) * 32) << 16) + 128 * (warp >> 3) + 32 * ((warp >> 2) & 1);
     const uint32_t my_full = ptx::smem_u32(part_full) + 8 * (warp >> 3);  // the warp's half of the even K blocks

@@ -210,7 +210,8 @@ __device__ __forceinline__ void zero_block_rows(const PairTile& tl, void* out, i
 // accumulator in global memory; whichever arrives last (counted per group of four epilogue warps) adds all S in slice order (a
 // fixed order: results do not depend on timing) and runs the epilogue.  Nobody waits: workers may start in any order, and
 // none needs another to be resident.  (Workers that wait for one another and finish a strip of the columns each need all of
-// them resident; the times are the same: Mixtral rank, 333 tokens, 268 and 269 us per layer, 288 without the split.)
+// them resident; the times are the same: Mixtral rank, 333 tokens, 282 us per layer both ways, 287 against 281 without the
+// split on another card.)
 struct UnitPlan {
   int64_t total, rounds, left;
   int grid, b, S, k_steps;

@@ -581,7 +581,7 @@ def test_fp8_per_channel_quant(fg, T, H, I, E, k):
 @pytest.mark.parametrize("T,H,I,E,k", [(700, 1024, 768, 8, 2), (1024, 4096, 1024, 4, 2)])
 def test_tail_split_on_and_off(fg, monkeypatch, T, H, I, E, k):
     """A last round of tiles that fills at most half of the CTAs is cut along K over the idle CTAs (fp32 partials summed
-    strip-wise in a fixed order).  On and off are both deterministic, both match the oracle, and differ from each other
+    in slice order by whichever worker arrives last).  On and off are both deterministic, both match the oracle, and differ from each other
     by summation order only."""
     x, w1, w2, logits = _layer(T, H, I, E, k, torch.bfloat16, 900 + T)
     tw, ti = OR.softmax_topk(logits, k, True)
