@@ -204,16 +204,17 @@ def _experts(hidden_states, w1, w2, topk_weights, topk_ids, route, k, inplace=Fa
              apply_router_weight_on_input=False, use_fp8_w8a8=False, per_channel_quant=False, w1_scale=None, w2_scale=None,
              a1_scale=None, a2_scale=None, block_shape=None, no_combine=False, routed_scaling_factor=None, expert_map=None,
              variant=None, out_rows=None, b1=None, b2=None, gemm1_alpha=None, gemm1_clamp_limit=None, weights_n_major=False,
-             triple=None, w1_interleaved=False):
+             triple=None, w1_interleaved=False, also=()):
     """`fused_experts`; with `route` (a filled _C.RouteArgs: logits of [T,E]) the router and the experts in one call, with
-    `triple` (positions -> slots, rows per expert, weights of the sorted positions) a routing that is already in expert order."""
+    `triple` (positions -> slots, rows per expert, weights of the sorted positions) a routing that is already in expert order.
+    `also`: the tensors behind `route`, which have to be on the same device."""
     logger.debug("FLAGGEMS_SGLANG_B200 FUSED_EXPERTS")
     assert inplace is False, "Inplace is not supported"
     assert a1_scale is None, _UNSUPPORTED_FEATURE_MSG.format(name="a1_scale")
     assert a2_scale is None, _UNSUPPORTED_FEATURE_MSG.format(name="a2_scale")
     if activation not in _C.ACTIVATIONS:
         raise ValueError(f"Unsupported FusedMoe activation: {activation}")
-    dev = _C.require_cuda(hidden_states, w1, w2, topk_weights, topk_ids, w1_scale, w2_scale, expert_map)
+    dev = _C.require_cuda(hidden_states, w1, w2, topk_weights, topk_ids, w1_scale, w2_scale, expert_map, *also)
     assert hidden_states.ndim == 2, "hidden_states must be 2D"
     T, H = hidden_states.shape
     if weights_n_major:
@@ -485,13 +486,13 @@ def fused_moe(
             raise ValueError("Number of tokens mismatch")
         bias = None
         if use_grouped_topk and correction_bias is not None:
-            _C.require_cuda(correction_bias)
             bias = correction_bias.float().contiguous()
             if bias.numel() != E:
                 raise ValueError("correction_bias must have num_experts entries")
         route = _C.RouteArgs(g.data_ptr(), _C.ptr(bias), int(use_grouped_topk), int(renormalize),
                              num_expert_group if use_grouped_topk else 1, topk_group if use_grouped_topk else 1)
-        return _experts(hidden_states, w1, w2, None, None, route, topk, routed_scaling_factor=routed_scaling_factor, **kwargs)
+        return _experts(hidden_states, w1, w2, None, None, route, topk, routed_scaling_factor=routed_scaling_factor,
+                        also=(g, bias), **kwargs)
     w, ids = _route(hidden_states, gating_output, topk, renormalize, use_grouped_topk, num_expert_group,
                     topk_group, correction_bias, None)
     return fused_experts(hidden_states, w1, w2, w, ids, routed_scaling_factor=routed_scaling_factor, **kwargs)

@@ -63,7 +63,7 @@ def grouped_topk(
         raise ValueError("Number of tokens mismatch")
     bias = None
     if correction_bias is not None:
-        _C.require_cuda(correction_bias)
+        _C.require_cuda(gating_output, correction_bias)
         bias = correction_bias.float().contiguous()
         if bias.numel() != E:
             raise ValueError("correction_bias must have num_experts entries")

@@ -83,6 +83,28 @@ def test_layer_variant_is_what_the_one_call_layer_takes(lib, dtype, T, E, H, I, 
         assert name == want and block == {"decode": 0, "stream": 8, "tcgen05": 128, "simt": 16}[want]
 
 
+@pytest.mark.parametrize("stray", ["logits", "bias"])
+def test_one_call_moe_refuses_a_router_input_on_another_device(monkeypatch, stray):
+    """The router's inputs go into the library call as plain pointers: they have to be on the layer's device (devices are
+    played by the CPU and the meta device here)."""
+    import importlib
+
+    FM = importlib.import_module("flaggems_sglang_b200.ops.fused_moe")
+
+    def require(*tensors):
+        devs = {t.device for t in tensors if t is not None}
+        if len(devs) > 1:
+            raise RuntimeError("tensors on different devices")
+        return devs.pop()
+
+    monkeypatch.setattr(FM._C, "require_cuda", require)  # (one module: the router's ops call the same)
+    h, w1, w2 = torch.zeros(3, 64), torch.zeros(4, 256, 64), torch.zeros(4, 64, 128)
+    logits = torch.zeros(3, 4, device="meta" if stray == "logits" else "cpu")
+    bias = torch.zeros(4, device="meta" if stray == "bias" else "cpu")
+    with pytest.raises(RuntimeError, match="different devices"):
+        FM.fused_moe(h, w1, w2, logits, 2, use_grouped_topk=True, num_expert_group=2, topk_group=1, correction_bias=bias)
+
+
 def test_unknown_struct_size_is_refused(lib):
     """A binding compiled against another version of the header is caught before any field is trusted."""
     import ctypes
