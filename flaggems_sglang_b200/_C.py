@@ -167,8 +167,33 @@ def ptr(t) -> int | None:
     return None if t is None else t.data_ptr()
 
 
-def stream_ptr(device=None) -> int:
-    return torch.cuda.current_stream(device).cuda_stream
+def stream_ptr(device: torch.device | None = None) -> int:
+    """The device's current stream as the library takes it (with a Stream object around it a decode call takes 2 us more)."""
+    return torch._C._cuda_getCurrentRawStream(current_device() if device is None else device.index)
+
+
+def current_device() -> int:
+    return torch._C._cuda_getDevice()
+
+
+class on_device:
+    """`with on_device(dev):` — `dev` is the current device inside.  The library launches on the current device; a default
+    stream's handle does not say whose it is, so a call for tensors of another GPU would run here and read that GPU's memory."""
+
+    __slots__ = ("want", "before")
+
+    def __init__(self, dev: torch.device):
+        self.want = dev.index
+
+    def __enter__(self):
+        self.before = current_device()
+        if self.before != self.want:
+            torch._C._cuda_setDevice(self.want)
+
+    def __exit__(self, *exc):
+        if self.before != self.want:
+            torch._C._cuda_setDevice(self.before)
+        return False
 
 
 def require_cuda(*tensors) -> torch.device:
@@ -192,4 +217,8 @@ def require_cuda(*tensors) -> torch.device:
 
 def check_device_status(device=None) -> None:
     """Synchronises the current stream and raises if a bounded wait inside a tcgen05 kernel gave up."""
-    check(lib().fmoe_check_device_status(stream_ptr(device)))
+    dev = torch.device("cuda") if device is None else torch.device(device)
+    if dev.index is None:
+        dev = torch.device("cuda", current_device())
+    with on_device(dev):
+        check(lib().fmoe_check_device_status(stream_ptr(dev)))

@@ -215,6 +215,12 @@ def _experts(hidden_states, w1, w2, topk_weights, topk_ids, route, k, inplace=Fa
     if activation not in _C.ACTIVATIONS:
         raise ValueError(f"Unsupported FusedMoe activation: {activation}")
     dev = _C.require_cuda(hidden_states, w1, w2, topk_weights, topk_ids, w1_scale, w2_scale, expert_map, *also)
+    if dev.index != _C.current_device():  # the library launches on the current device
+        with _C.on_device(dev):
+            return _experts(hidden_states, w1, w2, topk_weights, topk_ids, route, k, inplace, activation,
+                            apply_router_weight_on_input, use_fp8_w8a8, per_channel_quant, w1_scale, w2_scale, a1_scale, a2_scale,
+                            block_shape, no_combine, routed_scaling_factor, expert_map, variant, out_rows, b1, b2, gemm1_alpha,
+                            gemm1_clamp_limit, weights_n_major, triple, w1_interleaved, also)
     assert hidden_states.ndim == 2, "hidden_states must be 2D"
     T, H = hidden_states.shape
     if weights_n_major:

@@ -35,9 +35,10 @@ def moe_align_block_size(topk_ids: torch.Tensor, block_size: int, num_experts: i
     lib = _C.lib()
     ws_bytes = lib.fmoe_moe_align_workspace_bytes(numel, num_experts) if numel >= 16384 else 0
     ws = torch.empty(ws_bytes, dtype=torch.uint8, device=dev) if ws_bytes else None
-    _C.check(lib.fmoe_moe_align_block_size_ws(ids.data_ptr(), numel, num_experts, block_size, sorted_ids.data_ptr(),
-                                              cap, expert_ids.data_ptr(), nblk, num_post.data_ptr(), _C.ptr(ws),
-                                              ws_bytes, _C.stream_ptr(dev)))
+    with _C.on_device(dev):
+        _C.check(lib.fmoe_moe_align_block_size_ws(ids.data_ptr(), numel, num_experts, block_size, sorted_ids.data_ptr(),
+                                                  cap, expert_ids.data_ptr(), nblk, num_post.data_ptr(), _C.ptr(ws),
+                                                  ws_bytes, _C.stream_ptr(dev)))
     return sorted_ids, expert_ids, num_post
 
 

@@ -28,8 +28,9 @@ def moe_sum(input: torch.Tensor, output: torch.Tensor, routed_scaling_factor: fl
         raise ValueError("moe_sum needs contiguous tensors")
     T, k, H = input.shape
     scale = 1.0 if routed_scaling_factor is None else float(routed_scaling_factor)
-    _C.check(_C.lib().fmoe_moe_sum_add(input.data_ptr(), _C.DTYPE_CODE[input.dtype], T, k, H, scale,
-                                       _C.ptr(shared_output), output.data_ptr(), _C.stream_ptr(dev)))
+    with _C.on_device(dev):
+        _C.check(_C.lib().fmoe_moe_sum_add(input.data_ptr(), _C.DTYPE_CODE[input.dtype], T, k, H, scale,
+                                           _C.ptr(shared_output), output.data_ptr(), _C.stream_ptr(dev)))
     return output
 
 

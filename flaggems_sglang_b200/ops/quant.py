@@ -23,8 +23,9 @@ def per_token_group_quant_fp8(x: torch.Tensor, group_size: int = 128):
     rows, K = x.shape
     q = torch.empty(rows, K, dtype=torch.float8_e4m3fn, device=dev)
     s = torch.empty(rows, K // 128, dtype=torch.float32, device=dev)
-    _C.check(_C.lib().fmoe_quant_fp8_group128(x.data_ptr(), _C.DTYPE_CODE[x.dtype], rows, K, None, 1, 0, None,
-                                              q.data_ptr(), s.data_ptr(), _C.stream_ptr(dev)))
+    with _C.on_device(dev):
+        _C.check(_C.lib().fmoe_quant_fp8_group128(x.data_ptr(), _C.DTYPE_CODE[x.dtype], rows, K, None, 1, 0, None,
+                                                  q.data_ptr(), s.data_ptr(), _C.stream_ptr(dev)))
     return q, s
 
 
@@ -55,8 +56,9 @@ def per_token_quant_fp8(x: torch.Tensor):
     rows, K = x.shape
     q = torch.empty(rows, K, dtype=torch.float8_e4m3fn, device=dev)
     s = torch.empty(rows, dtype=torch.float32, device=dev)
-    _C.check(_C.lib().fmoe_quant_fp8_per_token(x.data_ptr(), _C.BF16, rows, K, None, 1, 0, None, q.data_ptr(),
-                                               s.data_ptr(), _C.stream_ptr(dev)))
+    with _C.on_device(dev):
+        _C.check(_C.lib().fmoe_quant_fp8_per_token(x.data_ptr(), _C.BF16, rows, K, None, 1, 0, None, q.data_ptr(),
+                                                   s.data_ptr(), _C.stream_ptr(dev)))
     return q, s
 
 

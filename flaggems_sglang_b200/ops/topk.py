@@ -35,8 +35,9 @@ def fused_topk(hidden_states, gating_output: torch.Tensor, topk: int, renormaliz
         raise ValueError("Number of tokens mismatch")
     w = torch.empty(T, topk, dtype=torch.float32, device=g.device)
     ids = torch.empty(T, topk, dtype=torch.int32, device=g.device)
-    _C.check(_C.lib().fmoe_topk_softmax(g.data_ptr(), T, E, topk, int(bool(renormalize)), w.data_ptr(),
-                                        ids.data_ptr(), _C.stream_ptr(g.device)))
+    with _C.on_device(g.device):
+        _C.check(_C.lib().fmoe_topk_softmax(g.data_ptr(), T, E, topk, int(bool(renormalize)), w.data_ptr(),
+                                            ids.data_ptr(), _C.stream_ptr(g.device)))
     return w, ids
 
 
@@ -70,9 +71,10 @@ def grouped_topk(
     w = torch.empty(T, topk, dtype=torch.float32, device=g.device)
     ids = torch.empty(T, topk, dtype=torch.int32, device=g.device)
     scale = 1.0 if routed_scaling_factor is None else float(routed_scaling_factor)
-    _C.check(_C.lib().fmoe_topk_grouped(g.data_ptr(), _C.ptr(bias), T, E, topk, num_expert_group, topk_group,
-                                        int(bool(renormalize)), scale, w.data_ptr(), ids.data_ptr(),
-                                        _C.stream_ptr(g.device)))
+    with _C.on_device(g.device):
+        _C.check(_C.lib().fmoe_topk_grouped(g.data_ptr(), _C.ptr(bias), T, E, topk, num_expert_group, topk_group,
+                                            int(bool(renormalize)), scale, w.data_ptr(), ids.data_ptr(),
+                                            _C.stream_ptr(g.device)))
     return w, ids
 
 

@@ -105,6 +105,28 @@ def test_one_call_moe_refuses_a_router_input_on_another_device(monkeypatch, stra
         FM.fused_moe(h, w1, w2, logits, 2, use_grouped_topk=True, num_expert_group=2, topk_group=1, correction_bias=bias)
 
 
+def test_calls_run_on_the_device_of_their_tensors(monkeypatch):
+    """With another device current, a call switches to the tensors' device and back (two devices are played here)."""
+    import importlib
+
+    FM = importlib.import_module("flaggems_sglang_b200.ops.fused_moe")
+    now, seen = [0], []
+    monkeypatch.setattr(torch._C, "_cuda_getDevice", lambda: now[0], raising=False)
+    monkeypatch.setattr(torch._C, "_cuda_setDevice", lambda d: (seen.append(d), now.__setitem__(0, d)), raising=False)
+    monkeypatch.setattr(FM._C, "require_cuda", lambda *t: torch.device("cuda", 1))
+    x, w1, w2 = torch.zeros(0, 64), torch.zeros(4, 256, 64), torch.zeros(4, 64, 128)
+    out = FM.fused_experts(x, w1, w2, torch.zeros(0, 2), torch.zeros(0, 2, dtype=torch.int32), no_combine=True)
+    assert out.shape == (0, 2, 64) and seen == [1, 0]
+    with pytest.raises(ZeroDivisionError):
+        with FM._C.on_device(torch.device("cuda", 1)):
+            assert now == [1]
+            1 / 0
+    assert now == [0]
+    with FM._C.on_device(torch.device("cuda", 0)):
+        pass
+    assert seen == [1, 0, 1, 0]
+
+
 def test_unknown_struct_size_is_refused(lib):
     """A binding compiled against another version of the header is caught before any field is trusted."""
     import ctypes
