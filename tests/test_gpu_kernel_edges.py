@@ -172,6 +172,17 @@ def test_decode_layer_needs_no_cta_that_has_not_started(fg, kind, T, ctas):
     assert torch.equal(out, ref) and torch.equal(call(), ref)
 
 
+@pytest.mark.parametrize("ctas", [0, 3])
+def test_decode_layer_without_an_active_expert(fg, ctas):
+    """No slot has an expert: every share of the work is empty, the sums are zero."""
+    from flaggems_sglang_b200 import _C
+
+    x, w1, w2, _ = _layer(3, 256, 128, 4, 1)
+    _C.check(_C.lib().fmoe_debug_decode_ctas(ctas))
+    out = fg.fused_experts(x.cuda(), w1.cuda(), w2.cuda(), torch.ones(3, 2, device="cuda"), torch.full((3, 2), -1, dtype=torch.int32, device="cuda"))
+    assert not out.any()
+
+
 @pytest.mark.parametrize("kind", ["bf16", "block"])
 def test_decode_layers_on_streams_of_two_priorities(fg, kind):
     calls = [_decode_call(fg, kind, T, 110 + T, E=32, H=1024, I=1024) for T in (1, 8)]
