@@ -292,19 +292,32 @@ align_scatter_kernel(const int32_t* __restrict__ topk_ids, int numel, int E, con
 // The triple is the caller's memory and only the device sees it.  Rows past the last position are clipped, a position whose
 // slot is outside [0, numel) is left out, and ids and slot_pos are -1 for a slot that no position names: no later kernel
 // forms an address from a word that was not written in this call.  Both misuses are recorded for fmoe_check_device_status.
-// The grid is one cluster, so that all of ids and slot_pos can be set to -1 before the first position is stored.
+// Up to kSortedThreads slots one CTA sets them first, up to kClusterSlots a cluster, whose barrier stands between that and the
+// first store of a position; above that a kernel before this one does it, because eight SMs take too long over the scattered
+// stores.  64 experts of 1280 x 256, us per call, one CTA / cluster / two kernels: 8 slots 24.7 / 26.6 / -, 136 slots 45.1 /
+// 45.2 / -, 2056 slots - / 52.9 / 51.3, 8192 slots - / 71.6 / 67.5, 32768 slots - / 176.2 / 155.5.
 // ---------------------------------------------------------------------------------------------
-constexpr int kSortedThreads = 1024;
+constexpr int kSortedThreads = 256;
 constexpr int kSortedCtas = 8;
+constexpr int kClusterSlots = kSortedCtas * kSortedThreads;
 
 __device__ __forceinline__ void report_triple(int code) { atomicCAS(&g_device_status_align, 0, code); }
 
-__global__ void __cluster_dims__(kSortedCtas, 1, 1) __launch_bounds__(kSortedThreads)
+__global__ void __launch_bounds__(kSortedThreads)
+clear_slots_kernel(int numel, int32_t* __restrict__ ids, int32_t* __restrict__ slot_pos) {
+  pdl_entry();
+  for (int i = blockIdx.x * kSortedThreads + threadIdx.x; i < numel; i += gridDim.x * kSortedThreads) {
+    ids[i] = -1;
+    if (slot_pos) slot_pos[i] = -1;
+  }
+}
+
+__global__ void __launch_bounds__(kSortedThreads)
 align_sorted_kernel(const int32_t* __restrict__ slot_of, const int32_t* __restrict__ hist, const float* __restrict__ gate, int numel,
                     int E, int block, int32_t* __restrict__ sorted_ids, int sorted_cap, int32_t* __restrict__ expert_ids,
                     int expert_cap, int32_t* __restrict__ num_post_pad, int32_t* __restrict__ table, int token_tile,
                     int32_t* __restrict__ zero_words, int num_zero, int32_t* __restrict__ ids, float* __restrict__ weights,
-                    int32_t* __restrict__ slot_pos, int rows_only) {
+                    int32_t* __restrict__ slot_pos, int rows_only, int clear) {
   pdl_entry();
   extern __shared__ int s_mem[];
   int* s_total = s_mem;            // [E]
@@ -312,10 +325,12 @@ align_sorted_kernel(const int32_t* __restrict__ slot_of, const int32_t* __restri
   int* s_first = s_start + E + 1;  // [E+1] unpadded
   __shared__ int s_sum[2 * kSortedThreads / 32];
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, block_id = blockIdx.x;
-  constexpr int stride = kSortedCtas * kSortedThreads;
-  for (int i = block_id * kSortedThreads + tid; i < numel; i += stride) {
-    ids[i] = -1;
-    if (slot_pos) slot_pos[i] = -1;
+  const int stride = gridDim.x * kSortedThreads;
+  if (clear) {
+    for (int i = block_id * kSortedThreads + tid; i < numel; i += stride) {
+      ids[i] = -1;
+      if (slot_pos) slot_pos[i] = -1;
+    }
   }
   for (int e = tid; e < E; e += kSortedThreads) s_total[e] = hist[e];
   __syncthreads();
@@ -348,7 +363,7 @@ align_sorted_kernel(const int32_t* __restrict__ slot_of, const int32_t* __restri
   __syncthreads();
   scan_experts<kSortedThreads / 32>(s_total, s_start, E, block, block_id == 0 ? num_post_pad : nullptr,
                                     block_id == 0 ? table : nullptr, token_tile, s_sum);
-  ptx::cluster_sync_all();
+  if (clear) ptx::cluster_sync_all();
   for (int p = block_id * kSortedThreads + tid; p < numel; p += stride) {
     const int slot = slot_of[p];
     const bool named = slot >= 0 && slot < numel;
@@ -434,9 +449,19 @@ int run_align_sorted(const AlignArgs& a, const SortedSlots& s, cudaStream_t st) 
     const int rc = check_align(a);
     if (rc) return rc;
   }
-  launch_pdl(align_sorted_kernel, dim3(kSortedCtas), dim3(kSortedThreads), (3 * (size_t)a.E + 2) * sizeof(int), st, s.slot_of, s.hist, s.gate,
-             (int)a.numel, a.E, a.block, a.sorted_ids, (int)a.sorted_cap, a.expert_ids, (int)a.expert_cap, a.num_post_pad, a.table,
-             a.token_tile, a.zero_words, a.num_zero, s.ids, s.weights, a.slot_pos, (int)a.rows_only);
+  const bool clear = a.numel <= kClusterSlots;
+  if (!clear) {
+    launch_pdl(clear_slots_kernel, dim3(148), dim3(kSortedThreads), 0, st, (int)a.numel, s.ids, a.slot_pos);
+    const int rc = launch_status("clear_slots_kernel");
+    if (rc) return rc;
+  }
+  const int64_t items = std::max(a.numel, a.sorted_ids && !a.rows_only ? a.sorted_cap / 4 : 0);
+  const unsigned cluster = !clear || a.numel <= kSortedThreads ? 1 : kSortedCtas;
+  const unsigned grid = clear ? cluster : (unsigned)std::min<int64_t>(ceil_div<int64_t>(items, kSortedThreads), 148);
+  launch_pdl_cluster(align_sorted_kernel, cluster, dim3(grid), dim3(kSortedThreads),
+                     (3 * (size_t)a.E + 2) * sizeof(int), st, s.slot_of, s.hist, s.gate, (int)a.numel, a.E, a.block, a.sorted_ids,
+                     (int)a.sorted_cap, a.expert_ids, (int)a.expert_cap, a.num_post_pad, a.table, a.token_tile, a.zero_words,
+                     a.num_zero, s.ids, s.weights, a.slot_pos, (int)a.rows_only, (int)clear);
   return launch_status("align_sorted_kernel");
 }
 

@@ -291,7 +291,7 @@ def test_launches_are_counted(fg, kind, T, launches):
     assert _C.lib().fmoe_debug_launches() == launches and _C.lib().fmoe_debug_launches() == 0
 
 
-@pytest.mark.parametrize("T", [1, 8, 9, 100, 2049])
+@pytest.mark.parametrize("T", [1, 8, 9, 85, 86, 100, 682, 683, 2049])
 def test_sorted_routing_equals_routing_by_slot(fg, T):
     """The routing triple goes to the kernels as it is; the results are those of the same routing by slot."""
     E, H, I, k = 24, 256, 192, 3
@@ -313,7 +313,8 @@ def test_sorted_routing_equals_routing_by_slot(fg, T):
     assert torch.equal(rows, ref)
 
 
-@pytest.mark.parametrize("T", [2, 30, 700, 3000])
+# 3 slots per token: both sides of 256 and 2048 slots, where a cluster and then two kernels make the block list
+@pytest.mark.parametrize("T", [2, 30, 85, 86, 682, 683, 3000])
 @pytest.mark.parametrize("fault", ["slot", "duplicate", "hist_over", "hist_negative", "hist_short"])
 def test_inconsistent_triple_stays_inside_its_buffers(fg, fault, T):
     """Entries of a routing triple that only the device sees: the workspace is filled with words that would be addresses if a
