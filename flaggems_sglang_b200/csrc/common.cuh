@@ -58,10 +58,21 @@ inline int launch_status(const char* what) {
 // FMOE_PDL=0 turns the launch attribute off (plain stream serialisation).
 bool pdl_enabled();
 
+//
+// The row passes and the CTA-pair GEMMs of a layer call let their successor start only after their own wait
+// (pdl_entry_late, or pdl_wait and then pdl_trigger).  A kernel that finds itself started then knows that everything
+// before its predecessor is complete, and may read that ahead of its own wait, past L1 (ld.global.cg, TMA): the GEMMs copy
+// the expert table and fill their ring with weights while the row pass, or the last tiles of the GEMM before, still run.
 #if defined(__CUDACC__)
+__device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+__device__ __forceinline__ void pdl_trigger() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 __device__ __forceinline__ void pdl_entry() {
-  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
-  asm volatile("griddepcontrol.wait;" ::: "memory");
+  pdl_trigger();
+  pdl_wait();
+}
+__device__ __forceinline__ void pdl_entry_late() {
+  pdl_wait();
+  pdl_trigger();
 }
 
 // cluster: CTAs per cluster, in x (1: as the kernel is compiled)

@@ -147,8 +147,11 @@ grouped_gemm_pair_kernel(const __grid_constant__ CUtensorMap map_t, const __grid
     ptx::tmem_relinquish_pair();
   }
   ptx::tc_fence_before_sync();
-  pdl_entry();  // everything above is independent of the kernels before this one on the stream
-  const int used_blocks = min((int)(*p.num_tokens_post_padded / 128), p.max_blocks);
+  // Everything above is independent of the kernels before this one on the stream.  A given table is complete by now (see
+  // pdl_entry_late): only the rows and what the epilogue reads and writes have to wait for the kernel before.
+  const bool early = p.expert_table != nullptr;
+  if (!early) pdl_wait();
+  const int used_blocks = early ? 0 : min((int)(*p.num_tokens_post_padded / 128), p.max_blocks);
   pair_build_table(table, p.num_experts, p.expert_table, p.expert_ids, p.sorted_token_ids, p.numel, 128,
                    p.token_tile, used_blocks);
   ptx::cluster_sync_all();  // the other CTA's barriers exist before anything is signalled across
@@ -178,18 +181,10 @@ grouped_gemm_pair_kernel(const __grid_constant__ CUtensorMap map_t, const __grid
         const int boxes = (half_n + BOX_TOKENS - 1) / BOX_TOKENS;
         const uint32_t t_bytes = GATHER ? half_n * KBYTES : boxes * (BOX_TOKENS * KBYTES);
         const int32_t c0 = GATED ? tl.w_tile * 128 + rank * 64 : tl.w_tile * 256 + rank * 128;
-        for (int ks = ks0; ks < ks1; ++ks) {
-          const long long tp0 = p.profile ? clock64() : 0;
-          const bool okp = ptx::mbar_wait(&empty_bar[stage], phase ^ 1);
-          if (p.profile) prof_p += clock64() - tp0;
-          if (!okp) {
-            report(0x100 | stage);
-            alive = false;
-            break;
-          }
-          const uint32_t sw = ring + stage * stage_size, stok = sw + W_BYTES, bar0 = bar_full0 + stage * 8;
+        auto load_weights = [&](int ks, int s) {  // K step ks into stage s; arms the stage for the bytes of all its loads
+          const uint32_t sw = ring + s * stage_size, bar0 = bar_full0 + s * 8;
           const int32_t x = ks * (KBYTES / (F8 ? 1 : 2));  // element coordinate along K
-          if (rank == 0) ptx::mbar_arrive_expect_tx(&full_bar[stage], 2 * (W_BYTES + t_bytes));
+          if (rank == 0) ptx::mbar_arrive_expect_tx(&full_bar[s], 2 * (W_BYTES + t_bytes));
           if constexpr (WMN) {
             ptx::tma_load_3d_pair(sw, &map_w, c0, x, tl.expert, bar0);
             ptx::tma_load_3d_pair(sw + W_BYTES / 2, &map_w, GATED ? c0 + (int32_t)p.n : c0 + 64, x, tl.expert, bar0);
@@ -198,16 +193,43 @@ grouped_gemm_pair_kernel(const __grid_constant__ CUtensorMap map_t, const __grid
           } else {
             ptx::tma_load_3d_pair(sw, &map_w, x, c0, tl.expert, bar0);
           }
+        };
+        auto load_tokens = [&](int ks, int s) {
+          const uint32_t stok = ring + s * stage_size + W_BYTES, bar0 = bar_full0 + s * 8;
+          const int32_t x = ks * (KBYTES / (F8 ? 1 : 2));
           if constexpr (GATHER) {
             auto row = [&](int32_t slot) { return (slot >= 0 && slot < p.numel) ? slot / p.top_k : p.a_rows; };
             for (int r = 0; r < half_n; r += 4) {
-              const int4 s = *reinterpret_cast<const int4*>(p.sorted_token_ids + row_t + r);
-              ptx::tma_gather4_pair(stok + r * KBYTES, &map_t, x, row(s.x), row(s.y), row(s.z), row(s.w), bar0);
+              const int4 id = *reinterpret_cast<const int4*>(p.sorted_token_ids + row_t + r);
+              ptx::tma_gather4_pair(stok + r * KBYTES, &map_t, x, row(id.x), row(id.y), row(id.z), row(id.w), bar0);
             }
           } else {
             for (int b = 0; b < boxes; ++b)
               ptx::tma_load_2d_pair(stok + b * (BOX_TOKENS * KBYTES), &map_t, x, row_t + b * BOX_TOKENS, bar0);
           }
+        };
+        int ks = ks0;
+        if (it == 0) {
+          // the first tile's weights are on their way before the rows are there: as many K steps as the ring has stages
+          const int ahead = early ? min(stages, ks1 - ks0) : 0;
+          for (int s = 0; s < ahead; ++s) load_weights(ks0 + s, s);
+          pdl_wait();
+          for (int s = 0; s < ahead; ++s) load_tokens(ks0 + s, s);
+          ks += ahead;
+          stage = ahead == stages ? 0 : ahead;
+          phase = ahead == stages;
+        }
+        for (; ks < ks1; ++ks) {
+          const long long tp0 = p.profile ? clock64() : 0;
+          const bool okp = ptx::mbar_wait(&empty_bar[stage], phase ^ 1);
+          if (p.profile) prof_p += clock64() - tp0;
+          if (!okp) {
+            report(0x100 | stage);
+            alive = false;
+            break;
+          }
+          load_weights(ks, stage);
+          load_tokens(ks, stage);
           if (++stage == stages) {
             stage = 0;
             phase ^= 1;
@@ -292,6 +314,7 @@ grouped_gemm_pair_kernel(const __grid_constant__ CUtensorMap map_t, const __grid
     }
   } else {
     // ---------------- epilogue (both CTAs, each its CTA's 128 weight rows) ----------------
+    pdl_entry_late();
     const int quarter = warp & 3, half = warp >> 2;
     const int g = lane >> 2, t = lane & 3;
     uint8_t* strip = strips + warp * STRIP_BYTES;

@@ -203,8 +203,10 @@ grouped_gemm_pair_fold_kernel(const __grid_constant__ CUtensorMap map_t, const _
     ptx::tmem_relinquish_pair();
   }
   ptx::tc_fence_before_sync();
-  pdl_entry();  // everything above is independent of the kernels before this one on the stream
-  const int used_blocks = min((int)(*p.num_tokens_post_padded / 128), p.max_blocks);
+  // a given table is complete by now (see pdl_entry_late): only rows, scales and outputs wait for the kernel before
+  const bool early = p.expert_table != nullptr;
+  if (!early) pdl_wait();
+  const int used_blocks = early ? 0 : min((int)(*p.num_tokens_post_padded / 128), p.max_blocks);
   pair_build_table(table, p.num_experts, p.expert_table, p.expert_ids, p.sorted_token_ids, p.numel, 128, TOK,
                    used_blocks, p.min_rows, p.max_rows);
   ptx::cluster_sync_all();
@@ -230,19 +232,36 @@ grouped_gemm_pair_fold_kernel(const __grid_constant__ CUtensorMap map_t, const _
         const int boxes = (half_n + BOX_TOKENS - 1) / BOX_TOKENS;
         const uint32_t bytes = 2 * (W_BYTES + boxes * (BOX_TOKENS * KBYTES));
         const int32_t c0 = GATED ? tl.w_tile * 128 + rank * 64 : tl.w_tile * 256 + rank * 128;
-        for (int kb = 0; kb < kblocks; ++kb) {
+        auto load_weights = [&](int kb, int s) {  // arms the stage for the bytes of all its loads
+          const uint32_t sw = ring + s * STAGE_BYTES, bar0 = bar_full0 + s * 8;
+          const int32_t x = kb * KBYTES;  // element coordinate (1-byte elements)
+          if (rank == 0) ptx::mbar_arrive_expect_tx(&full_bar[s], bytes);
+          if constexpr (GATED) ptx::tma_load_5d_pair(sw, &map_w, x, 0, 0, c0 >> 4, tl.expert, bar0);
+          else ptx::tma_load_3d_pair(sw, &map_w, x, c0, tl.expert, bar0);
+        };
+        auto load_tokens = [&](int kb, int s) {
+          for (int b = 0; b < boxes; ++b)
+            ptx::tma_load_2d_pair(ring + s * STAGE_BYTES + W_BYTES + b * (BOX_TOKENS * KBYTES), &map_t, kb * KBYTES,
+                                  row_t + b * BOX_TOKENS, bar_full0 + s * 8);
+        };
+        int kb = 0;
+        if (tile == worker) {
+          // the first tile's weights are on their way before the rows are there
+          const int ahead = early ? min(STAGES, kblocks) : 0;
+          for (; kb < ahead; ++kb) load_weights(kb, kb);
+          pdl_wait();
+          for (int s = 0; s < ahead; ++s) load_tokens(s, s);
+          stage = ahead == STAGES ? 0 : ahead;
+          phase = ahead == STAGES;
+        }
+        for (; kb < kblocks; ++kb) {
           if (!ptx::mbar_wait(&empty_bar[stage], phase ^ 1)) {
             report(0x500 | stage);
             alive = false;
             break;
           }
-          const uint32_t sw = ring + stage * STAGE_BYTES, stok = sw + W_BYTES, bar0 = bar_full0 + stage * 8;
-          const int32_t x = kb * KBYTES;  // element coordinate (1-byte elements)
-          if (rank == 0) ptx::mbar_arrive_expect_tx(&full_bar[stage], bytes);
-          if constexpr (GATED) ptx::tma_load_5d_pair(sw, &map_w, x, 0, 0, c0 >> 4, tl.expert, bar0);
-          else ptx::tma_load_3d_pair(sw, &map_w, x, c0, tl.expert, bar0);
-          for (int b = 0; b < boxes; ++b)
-            ptx::tma_load_2d_pair(stok + b * (BOX_TOKENS * KBYTES), &map_t, x, row_t + b * BOX_TOKENS, bar0);
+          load_weights(kb, stage);
+          load_tokens(kb, stage);
           if (++stage == STAGES) {
             stage = 0;
             phase ^= 1;
@@ -315,6 +334,7 @@ grouped_gemm_pair_fold_kernel(const __grid_constant__ CUtensorMap map_t, const _
     // ---------------- factors: two warps take alternate groups of four K blocks, one tile after the other ----------------
     constexpr int LANES = TOK / 32;  // tokens per lane
     const int me = warp - (kFoldWarps + 2);
+    pdl_wait();
     uint32_t group = 0;  // groups so far (selects the slot and its phase)
     bool alive = true;
     int ltile = 0;
@@ -397,6 +417,7 @@ grouped_gemm_pair_fold_kernel(const __grid_constant__ CUtensorMap map_t, const _
   } else {
     // ---------------- fold + epilogue (warps 0-15) ----------------
     if constexpr (MOVE) asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(kFoldRegs));
+    pdl_entry_late();
     const int quarter = warp & 3, half = (warp >> 2) & 1, kgroup = warp >> 3;
     const int t = lane & 3;
     const uint32_t factor_addr = ptx::smem_u32(factors) + (16 * half + 2 * t) * 4;
@@ -671,8 +692,9 @@ grouped_gemm_pair_fold_wide_kernel(const __grid_constant__ CUtensorMap map_t, co
     ptx::tmem_relinquish_pair();
   }
   ptx::tc_fence_before_sync();
-  pdl_entry();
-  const int used_blocks = min((int)(*p.num_tokens_post_padded / 128), p.max_blocks);
+  const bool early = p.expert_table != nullptr;
+  if (!early) pdl_wait();
+  const int used_blocks = early ? 0 : min((int)(*p.num_tokens_post_padded / 128), p.max_blocks);
   pair_build_table(table, p.num_experts, p.expert_table, p.expert_ids, p.sorted_token_ids, p.numel, 128, 256, used_blocks,
                    p.min_rows, p.max_rows);
   ptx::cluster_sync_all();
@@ -698,18 +720,34 @@ grouped_gemm_pair_fold_wide_kernel(const __grid_constant__ CUtensorMap map_t, co
         const int boxes = (half_n + BOX_TOKENS - 1) / BOX_TOKENS;  // lanes past them multiply what an earlier stage left
         const uint32_t bytes = 2 * (W_BYTES + boxes * (BOX_TOKENS * KBYTES));
         const int32_t row_w = GATED ? tl.w_tile * 128 + rank * (int32_t)p.n : tl.w_tile * 256 + rank * 128;
-        for (int kb = 0; kb < kblocks; ++kb) {
+        auto load_weights = [&](int kb, int s) {
+          const uint32_t sw = ring + s * STAGE_BYTES + W_BYTES, bar0 = bar_full0 + s * 8;
+          if (rank == 0) ptx::mbar_arrive_expect_tx(&full_bar[s], bytes);
+          ptx::tma_load_3d_pair(sw, &map_w, kb * KBYTES, row_w, tl.expert, bar0);
+        };
+        auto load_tokens = [&](int kb, int s) {
+          for (int b = 0; b < boxes; ++b)
+            ptx::tma_load_2d_pair(ring + s * STAGE_BYTES + b * (BOX_TOKENS * KBYTES), &map_t, kb * KBYTES, row_t + b * BOX_TOKENS,
+                                  bar_full0 + s * 8);
+        };
+        int kb = 0;
+        if (tile == worker) {
+          // the first tile's weights are on their way before the rows are there
+          const int ahead = early ? min(STAGES, kblocks) : 0;
+          for (; kb < ahead; ++kb) load_weights(kb, kb);
+          pdl_wait();
+          for (int s = 0; s < ahead; ++s) load_tokens(s, s);
+          stage = ahead == STAGES ? 0 : ahead;
+          phase = ahead == STAGES;
+        }
+        for (; kb < kblocks; ++kb) {
           if (!ptx::mbar_wait(&empty_bar[stage], phase ^ 1)) {
             report(0x500 | stage);
             alive = false;
             break;
           }
-          const uint32_t stok = ring + stage * STAGE_BYTES, bar0 = bar_full0 + stage * 8;
-          const int32_t x = kb * KBYTES;
-          if (rank == 0) ptx::mbar_arrive_expect_tx(&full_bar[stage], bytes);
-          ptx::tma_load_3d_pair(stok + W_BYTES, &map_w, x, row_w, tl.expert, bar0);
-          for (int b = 0; b < boxes; ++b)
-            ptx::tma_load_2d_pair(stok + b * (BOX_TOKENS * KBYTES), &map_t, x, row_t + b * BOX_TOKENS, bar0);
+          load_weights(kb, stage);
+          load_tokens(kb, stage);
           if (++stage == STAGES) {
             stage = 0;
             phase ^= 1;
@@ -781,6 +819,7 @@ grouped_gemm_pair_fold_wide_kernel(const __grid_constant__ CUtensorMap map_t, co
   } else if (warp >= kFoldWarps + 2) {
     // ---------------- factors: two warps take alternate groups of eight K blocks ----------------
     const int me = warp - (kFoldWarps + 2);
+    pdl_wait();
     uint32_t group = 0;
     bool alive = true;
     int ltile = 0;
@@ -879,6 +918,7 @@ grouped_gemm_pair_fold_wide_kernel(const __grid_constant__ CUtensorMap map_t, co
   } else {
     // ---------------- fold + epilogue (warps 0-15) ----------------
     if constexpr (MOVE) asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(kFoldRegs));
+    pdl_entry_late();
     // This loop runs at 104 registers (96 where the move is left out): the tile is described by its meta entry, shared
     // memory addresses are constants, everything else is derived from three counters.
     const uint32_t lane_addr = tmem_base + ((uint32_t)((warp & 3) * 32) << 16) + 128 * (warp >> 3) + 32 * ((warp >> 2) & 1);

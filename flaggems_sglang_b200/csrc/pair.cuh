@@ -67,7 +67,7 @@ __device__ __forceinline__ void pair_build_table(int32_t* table, int num_experts
   if (global_table) {
     const bool all = min_rows <= 0 && max_rows == 0x7fffffff;
     for (int i = threadIdx.x; i < pair_table_words(num_experts); i += blockDim.x) {
-      const int32_t v = global_table[i];
+      const int32_t v = __ldcg(global_table + i);  // possibly ahead of griddepcontrol.wait: not from L1
       table[i] = !all && i >= num_experts && i < 2 * num_experts && (v < min_rows || v > max_rows) ? 0 : v;
     }
     __syncthreads();

@@ -40,7 +40,8 @@ __global__ void __launch_bounds__(256)
 quant_group128_kernel(const InT* __restrict__ x, int64_t rows_out, int64_t K, const int32_t* __restrict__ row_map,
                       int map_div, int64_t sentinel, const int32_t* __restrict__ num_rows_dev,
                       uint8_t* __restrict__ q, float* __restrict__ scale, const int32_t* __restrict__ pos) {
-  pdl_entry();
+  if constexpr (MODE == RowMode::kMap) pdl_entry();
+  else pdl_entry_late();
   constexpr int kIlp = 4;
   const int sub = threadIdx.x & 15;  // lane inside the 16-lane team
   const unsigned hmask = (threadIdx.x & 16) ? 0xffff0000u : 0x0000ffffu;
@@ -143,7 +144,8 @@ __global__ void __launch_bounds__(256)
 quant_row_kernel(const __nv_bfloat16* __restrict__ x, int64_t rows_out, int64_t K, const int32_t* __restrict__ row_map,
                  int map_div, int64_t sentinel, const int32_t* __restrict__ num_rows_dev, uint8_t* __restrict__ q,
                  float* __restrict__ scale, const int32_t* __restrict__ pos) {
-  pdl_entry();
+  if constexpr (MODE == RowMode::kMap) pdl_entry();
+  else pdl_entry_late();
   __shared__ float s_max[8];
   constexpr int kTeams = 256 / TEAM;
   const int lane = threadIdx.x % TEAM;
@@ -250,7 +252,7 @@ gather_rows_kernel(const uint4* __restrict__ x, int64_t rows_out, int64_t vec_pe
 __global__ void __launch_bounds__(256)
 scatter_rows_kernel(const uint4* __restrict__ x, int64_t T, int k, int vec_per_row, int pieces, const int32_t* __restrict__ pos,
                     uint4* __restrict__ out) {
-  pdl_entry();
+  pdl_entry_late();
   constexpr int kIlp = 4;
   const int lane = threadIdx.x & 31;
   const int64_t items = T * pieces;
