@@ -6,7 +6,7 @@
 //   pipeline  : 192 KB ring of 6, 8 or 9 stages (16 KB of weights + 16, 8 or 4 KB of tokens) per CTA
 //   TMEM      : 512 columns per CTA = two 128 x 256 fp32 accumulators, so the epilogue of a tile overlaps the next tile
 //   warps     : 0-15 epilogue (TMEM lane quarter = warp % 4; the four of a quarter take 16-token chunks in turn),
-//               16 TMA producer (each CTA its own weight rows and its own half of the tokens), 17 MMA issuer (CTA 0)
+//               16-17 TMA producers (each CTA its own weight rows and its own half of the tokens), 18 MMA issuer (CTA 0)
 //
 // Why pairs: with one CTA per 128 x 256 tile an MMA reads 12 KB of shared memory for every 8 KB here, and TMA writes as
 // much; fill and operand reads of one SM together ran into its 128 bytes per clock.  Why weights on M: see pair.cuh.
@@ -46,6 +46,12 @@ constexpr int ACC_COLS = 256;
 // with 8 a short main loop waited for them (7.3k cycles per tile against 6.1k of MMAs at K = 768).  The gate/up exchange of
 // M-major weights needs shared memory per group of four, so that kernel keeps 8.
 constexpr int epi_warps(bool exchange) { return exchange ? 8 : 16; }
+// TMA warps: they take the K steps in turn.  Waiting for a stage, arming it and issuing two to five copies takes one thread
+// about 430 cycles, and with one warp that was the pace of every tile whose MMAs need less (SM cycles per K step with 64, 128,
+// 192 and 256 tokens per tile: 431, 470, 493, 508; two warps: 288 tokens in two tiles 500 -> 405, 256 tokens 508 -> 465; a
+// third one changes nothing).  Qwen3, 128 experts of 288 rows: gate/up GEMM 270 -> 251 us; Mixtral 549 -> 513 us.
+constexpr int kProducers = 2;
+constexpr int pair_threads(bool exchange) { return (epi_warps(exchange) + kProducers + 1) * 32; }
 constexpr int BOX_TOKENS = 32;                      // token rows per TMA box
 constexpr int STRIP_BYTES = kStripBytes;
 constexpr int EX_PITCH = 20;                        // floats per lane row of the gate/up exchange (16 tokens + padding)
@@ -108,10 +114,11 @@ __device__ __forceinline__ bool any_of_four_warps(int bar, bool pred) {
 }
 
 template <bool GATED, bool F8, bool EXTRA, bool WMN, bool GATHER>
-__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__((epi_warps(GATED && WMN) + 2) * 32, 1)
+__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(pair_threads(GATED && WMN), 1)
 grouped_gemm_pair_kernel(const __grid_constant__ CUtensorMap map_t, const __grid_constant__ CUtensorMap map_w,
                          const PairParams p) {
   constexpr int kEpiWarps = epi_warps(GATED && WMN), HALVES = kEpiWarps / 4;  // warps per lane quarter
+  constexpr int kMmaWarp = kEpiWarps + kProducers;
   extern __shared__ __align__(1024) uint8_t smem[];  // aligned by declaration: every address below is a constant
   const int stages = p.stages, stage_size = p.stage_bytes;
   uint64_t* bars = reinterpret_cast<uint64_t*>(smem + RING_BYTES);
@@ -142,7 +149,7 @@ grouped_gemm_pair_kernel(const __grid_constant__ CUtensorMap map_t, const __grid
     ptx::prefetch_tensormap(&map_t);
     ptx::prefetch_tensormap(&map_w);
   }
-  if (warp == kEpiWarps + 1) {
+  if (warp == kMmaWarp) {
     ptx::tmem_alloc_pair(tmem_slot, TMEM_COLS);
     ptx::tmem_relinquish_pair();
   }
@@ -164,11 +171,23 @@ grouped_gemm_pair_kernel(const __grid_constant__ CUtensorMap map_t, const __grid
   PairCursor cursor;
   PairTile tl;
 
-  if (warp == kEpiWarps) {
-    // ---------------- TMA producer (both CTAs) ----------------
+  if (warp >= kEpiWarps && warp < kMmaWarp) {
+    // ---------------- TMA producers (both CTAs): K steps me, me + kProducers, .. of all the worker's tiles ----------------
     if (ptx::elect_one()) {
-      int stage = 0;
+      const int me = warp - kEpiWarps;
+      int stage = me, mine = me;  // mine: this warp's next K step, counted from the tile's first
       uint32_t phase = 0;
+      int last_stage = -1;
+      uint32_t last_phase = 0;
+      auto advance = [&]() {
+        last_stage = stage;
+        last_phase = phase;
+        stage += kProducers;
+        if (stage >= stages) {
+          stage -= stages;
+          phase ^= 1;
+        }
+      };
       bool alive = true;
       long long prof_p = 0;
       int64_t tile;
@@ -208,18 +227,18 @@ grouped_gemm_pair_kernel(const __grid_constant__ CUtensorMap map_t, const __grid
               ptx::tma_load_2d_pair(stok + b * (BOX_TOKENS * KBYTES), &map_t, x, row_t + b * BOX_TOKENS, bar0);
           }
         };
-        int ks = ks0;
+        int ks = ks0 + mine;
         if (it == 0) {
           // the first tile's weights are on their way before the rows are there: as many K steps as the ring has stages
           const int ahead = early ? min(stages, ks1 - ks0) : 0;
-          for (int s = 0; s < ahead; ++s) load_weights(ks0 + s, s);
+          for (int i = me; i < ahead; i += kProducers) load_weights(ks0 + i, i);
           pdl_wait();
-          for (int s = 0; s < ahead; ++s) load_tokens(ks0 + s, s);
-          ks += ahead;
-          stage = ahead == stages ? 0 : ahead;
-          phase = ahead == stages;
+          for (; ks - ks0 < ahead; ks += kProducers) {
+            load_tokens(ks, stage);
+            advance();
+          }
         }
-        for (; ks < ks1; ++ks) {
+        for (; ks < ks1; ks += kProducers) {
           const long long tp0 = p.profile ? clock64() : 0;
           const bool okp = ptx::mbar_wait(&empty_bar[stage], phase ^ 1);
           if (p.profile) prof_p += clock64() - tp0;
@@ -230,27 +249,15 @@ grouped_gemm_pair_kernel(const __grid_constant__ CUtensorMap map_t, const __grid
           }
           load_weights(ks, stage);
           load_tokens(ks, stage);
-          if (++stage == stages) {
-            stage = 0;
-            phase ^= 1;
-          }
+          advance();
         }
+        mine = ks - ks1;
       }
       if (p.profile && blockIdx.x < 256) g_wait_prof[blockIdx.x * 8 + 3] = prof_p;
-      if (alive) {  // drain: every stage this CTA filled has been consumed before the CTA may end
-        for (int s = 0; s < stages; ++s) {
-          if (!ptx::mbar_wait(&empty_bar[stage], phase ^ 1)) {
-            report(0x180 | stage);
-            break;
-          }
-          if (++stage == stages) {
-            stage = 0;
-            phase ^= 1;
-          }
-        }
-      }
+      // drain: what this warp filled has been consumed (in order) before the CTA may end
+      if (alive && last_stage >= 0 && !ptx::mbar_wait(&empty_bar[last_stage], last_phase)) report(0x180 | last_stage);
     }
-  } else if (warp == kEpiWarps + 1) {
+  } else if (warp == kMmaWarp) {
     // ---------------- MMA issuer (CTA 0 only) ----------------
     if (rank == 0 && ptx::elect_one()) {
       int stage = 0;
@@ -550,7 +557,7 @@ grouped_gemm_pair_kernel(const __grid_constant__ CUtensorMap map_t, const __grid
   ptx::tc_fence_before_sync();
   __syncthreads();
   ptx::cluster_sync_all();  // nobody signals into a CTA that has left, and both are done with TMEM
-  if (warp == kEpiWarps + 1) {
+  if (warp == kMmaWarp) {
     ptx::tc_fence_after_sync();
     ptx::tmem_dealloc_pair(tmem_base, TMEM_COLS);
   }
@@ -738,7 +745,7 @@ int launch(const GemmParams& g, cudaStream_t st) {
       FMOE_CUDA_OK(cudaMemsetAsync(g.split_ws, 0, kSplitCounters * 4, st));
     }
   }
-  launch_pdl(kernel, dim3(2 * workers), dim3((epi_warps(GATED && WMN) + 2) * 32), smem, st, map_t, map_w, p);
+  launch_pdl(kernel, dim3(2 * workers), dim3(pair_threads(GATED && WMN)), smem, st, map_t, map_w, p);
   return launch_status("grouped_gemm_pair_kernel");
 }
 
