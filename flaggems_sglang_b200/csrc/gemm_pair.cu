@@ -6,7 +6,8 @@
 //   pipeline  : 192 KB ring of 6, 8 or 9 stages (16 KB of weights + 16, 8 or 4 KB of tokens) per CTA
 //   TMEM      : 512 columns per CTA = two 128 x 256 fp32 accumulators, so the epilogue of a tile overlaps the next tile
 //   warps     : 0-15 epilogue (TMEM lane quarter = warp % 4; the four of a quarter take 16-token chunks in turn),
-//               16-17 TMA producers (each CTA its own weight rows and its own half of the tokens), 18 MMA issuer (CTA 0)
+//               16-17 TMA producers (each CTA its own weight rows and its own half of the tokens), 18 MMA issuer (CTA 0),
+//               19 list of the worker's tiles
 //
 // Why pairs: with one CTA per 128 x 256 tile an MMA reads 12 KB of shared memory for every 8 KB here, and TMA writes as
 // much; fill and operand reads of one SM together ran into its 128 bytes per clock.  Why weights on M: see pair.cuh.
@@ -51,14 +52,14 @@ constexpr int epi_warps(bool exchange) { return exchange ? 8 : 16; }
 // 192 and 256 tokens per tile: 431, 470, 493, 508; two warps: 288 tokens in two tiles 500 -> 405, 256 tokens 508 -> 465; a
 // third one changes nothing).  Qwen3, 128 experts of 288 rows: gate/up GEMM 270 -> 251 us; Mixtral 549 -> 513 us.
 constexpr int kProducers = 2;
-constexpr int pair_threads(bool exchange) { return (epi_warps(exchange) + kProducers + 1) * 32; }
+constexpr int pair_threads(bool exchange) { return (epi_warps(exchange) + kProducers + 2) * 32; }
 constexpr int BOX_TOKENS = 32;                      // token rows per TMA box
 constexpr int STRIP_BYTES = kStripBytes;
 constexpr int EX_PITCH = 20;                        // floats per lane row of the gate/up exchange (16 tokens + padding)
 constexpr int EX_BYTES = 128 * EX_PITCH * 4;        // per half of the epilogue warps
 constexpr int BAR_BYTES = 256;
 constexpr int smem_bytes(int num_experts, bool exchange) {
-  return RING_BYTES + BAR_BYTES + (exchange ? 2 * EX_BYTES : epi_warps(false) * STRIP_BYTES) + pair_table_bytes(num_experts);
+  return RING_BYTES + BAR_BYTES + kListBytes + (exchange ? 2 * EX_BYTES : epi_warps(false) * STRIP_BYTES) + pair_table_bytes(num_experts);
 }
 static_assert(smem_bytes(1024, true) <= 227 * 1024, "shared memory");
 
@@ -127,7 +128,9 @@ grouped_gemm_pair_kernel(const __grid_constant__ CUtensorMap map_t, const __grid
   uint64_t* acc_full = bars + 2 * MAX_STAGES;       // [2] per CTA: MMA -> this CTA's epilogue
   uint64_t* acc_empty = bars + 2 * MAX_STAGES + 2;  // [2] used in CTA 0: both epilogues -> MMA
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 2 * MAX_STAGES + 4);
-  uint8_t* strips = smem + RING_BYTES + BAR_BYTES;
+  uint64_t* list_bars = bars + 2 * MAX_STAGES + 5;   // [4] (PairList)
+  int4* list = reinterpret_cast<int4*>(smem + RING_BYTES + BAR_BYTES);
+  uint8_t* strips = smem + RING_BYTES + BAR_BYTES + kListBytes;
   int32_t* table = reinterpret_cast<int32_t*>(strips + (GATED && WMN ? 2 * EX_BYTES : kEpiWarps * STRIP_BYTES));
 
   const int warp = ptx::uniform_warp_id(), lane = threadIdx.x & 31;
@@ -143,6 +146,7 @@ grouped_gemm_pair_kernel(const __grid_constant__ CUtensorMap map_t, const __grid
       ptx::mbar_init(&acc_full[a], 1);
       ptx::mbar_init(&acc_empty[a], 2 * kEpiWarps);  // one arrival per epilogue warp of both CTAs
     }
+    PairList::init_barriers(list_bars, kEpiWarps + kProducers + (rank == 0));
     ptx::fence_barrier_init();
   }
   if (warp == kEpiWarps && lane == 0) {
@@ -166,10 +170,10 @@ grouped_gemm_pair_kernel(const __grid_constant__ CUtensorMap map_t, const __grid
   const uint32_t tmem_base = *tmem_slot;
 
   const int k_steps = p.k_steps;
-  UnitPlan plan;
-  plan.init((int64_t)table[3 * p.num_experts] * p.w_tiles, k_steps, p.split_max, workers, worker);
-  PairCursor cursor;
-  PairTile tl;
+  PairList units(list, list_bars);
+  PairUnit unit;
+  const PairTile& tl = unit.tl;
+  auto first_step = [&](int slice) { return (int)((int64_t)k_steps * slice >> unit.log2_s); };  // of a slice of this unit's tile
 
   if (warp >= kEpiWarps && warp < kMmaWarp) {
     // ---------------- TMA producers (both CTAs): K steps me, me + kProducers, .. of all the worker's tiles ----------------
@@ -190,11 +194,14 @@ grouped_gemm_pair_kernel(const __grid_constant__ CUtensorMap map_t, const __grid
       };
       bool alive = true;
       long long prof_p = 0;
-      int64_t tile;
-      int ks0, ks1, slice;
       const uint32_t ring = ptx::smem_u32(smem), bar_full0 = ptx::smem_u32(full_bar) & ~ptx::kPeerRankBit;
-      for (int64_t it = 0; alive && plan.get(it, &tile, &ks0, &ks1, &slice); ++it) {
-        cursor.locate(tile, p.w_tiles, p.group, p.num_experts, table, &tl);
+      for (bool first = true; alive; first = false) {
+        const int got = units.next<false>(&unit);
+        if (got <= 0) {
+          if (got < 0) report(0x400);
+          break;
+        }
+        const int ks0 = first_step(unit.slice), ks1 = first_step(unit.slice + 1);
         const int half_n = tl.n >> 1;                       // tokens this CTA loads
         const int row_t = tl.row0 + rank * half_n;
         const int boxes = (half_n + BOX_TOKENS - 1) / BOX_TOKENS;
@@ -228,7 +235,7 @@ grouped_gemm_pair_kernel(const __grid_constant__ CUtensorMap map_t, const __grid
           }
         };
         int ks = ks0 + mine;
-        if (it == 0) {
+        if (first) {
           // the first tile's weights are on their way before the rows are there: as many K steps as the ring has stages
           const int ahead = early ? min(stages, ks1 - ks0) : 0;
           for (int i = me; i < ahead; i += kProducers) load_weights(ks0 + i, i);
@@ -265,15 +272,18 @@ grouped_gemm_pair_kernel(const __grid_constant__ CUtensorMap map_t, const __grid
       int local = 0;
       bool alive = true;
       long long prof_acc = 0, prof_data = 0;
-      int64_t tile;
-      int ks0, ks1, slice;
       const uint32_t ring = ptx::smem_u32(smem);
       const uint64_t db0 = ptx::smem_desc_sw128(ring + W_BYTES);
       // M-major: 64 channels (128 B) x 8 K rows per swizzle atom; the next 8 K rows 1 KB on, the next 64 channels 8 KB on
       const uint64_t da0 = WMN ? ptx::smem_desc_sw128_lbo(ring, W_BYTES / 2, 1024) : ptx::smem_desc_sw128(ring);
       constexpr int a_step = WMN ? (2048 >> 4) : 2;  // one MMA's K: 16 K rows of 128 B, or 32 bytes of each row
-      for (int64_t it = 0; alive && plan.get(it, &tile, &ks0, &ks1, &slice); ++it) {
-        cursor.locate(tile, p.w_tiles, p.group, p.num_experts, table, &tl);
+      while (alive) {
+        const int got = units.next<false>(&unit);
+        if (got <= 0) {
+          if (got < 0) report(0x410);
+          break;
+        }
+        const int ks0 = first_step(unit.slice), ks1 = first_step(unit.slice + 1);
         // bit 15: the M-side operand is M-major
         const uint32_t idesc = ptx::make_idesc(F8 ? /*e4m3*/ 0 : /*bf16*/ 1, 256, (uint32_t)tl.n) | (WMN ? (1u << 15) : 0u);
         const int acc = local & 1;
@@ -319,6 +329,14 @@ grouped_gemm_pair_kernel(const __grid_constant__ CUtensorMap map_t, const __grid
         g_wait_prof[blockIdx.x * 8 + 2] = prof_data;
       }
     }
+  } else if (warp == kMmaWarp + 1) {
+    // ---------------- the worker's tiles ----------------
+    UnitPlan plan;
+    plan.init((int64_t)table[3 * p.num_experts] * p.w_tiles, k_steps, p.split_max, workers, worker);
+    int more = 1;
+    for (int batch = 0; more > 0; ++batch)
+      more = PairList::fill(list, list_bars, batch, plan, p.w_tiles, p.group, p.num_experts, table);
+    if (more < 0) report(0x430);
   } else {
     // ---------------- epilogue (both CTAs, each its CTA's 128 weight rows) ----------------
     pdl_entry_late();
@@ -328,10 +346,15 @@ grouped_gemm_pair_kernel(const __grid_constant__ CUtensorMap map_t, const __grid
     int local = 0;
     bool alive = true;
     long long prof_wait = 0, prof_busy = 0;
-    int64_t tile;
-    int ks0, ks1, slice;
-    for (int64_t it = 0; alive && plan.get(it, &tile, &ks0, &ks1, &slice); ++it) {
-      cursor.locate(tile, p.w_tiles, p.group, p.num_experts, table, &tl);
+    while (alive) {
+      const bool waits = units.n % kListUnits == 0;
+      int got = units.next<true>(&unit);
+      if (waits && any_of_four_warps(1 + half, got < 0)) got = -1;  // warps that meet at a barrier below leave together
+      if (got <= 0) {
+        if (got < 0) report(0x420);
+        break;
+      }
+      const int slice = unit.slice, S = 1 << unit.log2_s;
       const int acc = local & 1;
       const uint32_t acc_phase = (local >> 1) & 1;
       ++local;
@@ -371,7 +394,7 @@ grouped_gemm_pair_kernel(const __grid_constant__ CUtensorMap map_t, const __grid
         }
       }
       const long long te0 = p.profile ? clock64() : 0;
-      const bool split = plan.is_split(it);
+      const bool split = S > 1;
       bool oke = warp_wait_relaxed(&acc_full[acc], acc_phase);
       // warps that meet at a barrier below leave together or not at all
       if (split || (GATED && WMN)) oke = !any_of_four_warps(1 + half, !oke);
@@ -384,11 +407,10 @@ grouped_gemm_pair_kernel(const __grid_constant__ CUtensorMap map_t, const __grid
       }
       ptx::tc_fence_after_sync();
       const uint32_t taddr = tmem_base + acc * ACC_COLS + ((uint32_t)(quarter * 32) << 16);
-      const int S = split ? plan.S : 1;
       // fragment (slice o, chunk j) of this thread: four float4, 512 bytes apart so that a warp stores whole lines
       auto partial = [&](int o, int j) {
         return reinterpret_cast<float4*>(p.split_partials) +
-               ((((int64_t)(plan.b - slice + o) * 2 + rank) * 16 + j) * 4 + quarter) * 128 + lane;
+               ((((int64_t)(worker - slice + o) * 2 + rank) * 16 + j) * 4 + quarter) * 128 + lane;
       };
       bool finish = true;  // these four warps run the epilogue of their chunks
       if (split) {
@@ -409,7 +431,7 @@ grouped_gemm_pair_kernel(const __grid_constant__ CUtensorMap map_t, const __grid
         __threadfence();  // the partials are visible device-wide before these warps count as arrived
         asm volatile("bar.sync %0, 128;" ::"r"(1 + half) : "memory");
         finish = any_of_four_warps(1 + half, quarter == 0 && lane == 0 &&
-                                                 atomicAdd(p.split_counters + (plan.b / S * 2 + rank) * 4 + half, 1) == S - 1);
+                                                 atomicAdd(p.split_counters + ((worker >> unit.log2_s) * 2 + rank) * 4 + half, 1) == S - 1);
         __threadfence();  // the other slices' partials are read after the count
       }
       // the next chunk's TMEM read-out is in flight while a chunk is stored

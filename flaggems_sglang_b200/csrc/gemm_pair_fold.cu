@@ -17,7 +17,7 @@
 //               block: 722 SM cycles per K block; this split 572.  DeepSeek-V3, 128 tokens 1361 -> 1245 us, 1024 tokens
 //               2190 -> 2005 us per layer.)  The gate/up output is fp32, for the quantiser behind it
 //   warp 16   : TMA producer      warp 17 : MMA issuer (CTA 0)
-//   warps 18-19: factors.  For four K blocks at a time they multiply the tokens' scales with the tile's one or two weight
+//   warps 18-19: factors (and warp 18 the list of the worker's tiles).  For four K blocks at a time they multiply the tokens' scales with the tile's one or two weight
 //               scales and leave the products in a 4-slot ring in shared memory, next to the tile's slots and row weights:
 //               the fold warps read one 8-byte pair per two tokens and keep no pointers
 // What bounds it: HBM (the weights stream through a ring of 20 KB stages) up to about 8 rows per expert, the fold above.
@@ -64,7 +64,7 @@ struct Geo {
   static constexpr int EX_BYTES = 2 * 1024;                    // per fold warp: sums on their way to the partner warp
   static constexpr int META_BYTES = GATED ? 0 : META_TILES * TOK * 8;  // slots and row weights of the tile's tokens
   static constexpr int bytes(int num_experts) {
-    return STAGES * STAGE_BYTES + BAR_BYTES + kFoldWarps * (STRIP_BYTES + EX_BYTES) + FACTOR_BYTES + META_BYTES +
+    return STAGES * STAGE_BYTES + BAR_BYTES + kListBytes + kFoldWarps * (STRIP_BYTES + EX_BYTES) + FACTOR_BYTES + META_BYTES +
            pair_table_bytes(num_experts);
   }
 };
@@ -166,8 +166,10 @@ grouped_gemm_pair_fold_kernel(const __grid_constant__ CUtensorMap map_t, const _
   uint64_t* sc_full = part_empty + BUFS;                // [slots] factor warps -> fold
   uint64_t* sc_empty = sc_full + SC_SLOTS;              // [slots] fold -> factor warps
   uint64_t* pair_bar = sc_empty + SC_SLOTS;             // [8] the two warps that exchange sums
-  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(pair_bar + 8);
-  uint8_t* strips = smem + STAGES * STAGE_BYTES + BAR_BYTES;
+  uint64_t* list_bars = pair_bar + 8;                   // [4] (PairList)
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(list_bars + 4);
+  int4* list = reinterpret_cast<int4*>(smem + STAGES * STAGE_BYTES + BAR_BYTES);
+  uint8_t* strips = smem + STAGES * STAGE_BYTES + BAR_BYTES + kListBytes;
   uint8_t* factors = strips + kFoldWarps * G::STRIP_BYTES;                      // [slot][K block][gate | up][token]
   int32_t* meta = reinterpret_cast<int32_t*>(factors + G::FACTOR_BYTES);        // [tile][slot ids | row weights]
   uint8_t* exchange = factors + G::FACTOR_BYTES + G::META_BYTES;                 // [warp][round parity][4][lane] f32 pairs
@@ -192,6 +194,7 @@ grouped_gemm_pair_fold_kernel(const __grid_constant__ CUtensorMap map_t, const _
       ptx::mbar_init(&sc_empty[s], kFoldWarps);
     }
     for (int w = 0; w < 8; ++w) ptx::mbar_init(&pair_bar[w], 2);
+    PairList::init_barriers(list_bars, kFoldWarps + 3 + (rank == 0));  // TMA, two factor warps, MMA
     ptx::fence_barrier_init();
   }
   if (warp == kFoldWarps && lane == 0) {
@@ -214,8 +217,9 @@ grouped_gemm_pair_fold_kernel(const __grid_constant__ CUtensorMap map_t, const _
   const uint32_t tmem_base = *tmem_slot;
   const int kblocks = p.kblocks;
   const int total_tiles = table[3 * p.num_experts] * p.w_tiles;
-  PairCursor cursor;
-  PairTile tl;
+  PairList units(list, list_bars);
+  PairUnit unit;
+  const PairTile& tl = unit.tl;
 
   if (MOVE && warp >= kFoldWarps) asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(kOtherRegs));
   if (warp == kFoldWarps) {
@@ -225,8 +229,12 @@ grouped_gemm_pair_fold_kernel(const __grid_constant__ CUtensorMap map_t, const _
       uint32_t phase = 0;
       bool alive = true;
       const uint32_t ring = ptx::smem_u32(smem), bar_full0 = ptx::smem_u32(full_bar) & ~ptx::kPeerRankBit;
-      for (int tile = worker; tile < total_tiles && alive; tile += workers) {
-        cursor.locate(tile, p.w_tiles, p.group, p.num_experts, table, &tl);
+      for (bool first = true; alive; first = false) {
+        const int got = units.next<false>(&unit);
+        if (got <= 0) {
+          if (got < 0) report(0x5c0);
+          break;
+        }
         const int half_n = tl.n >> 1;
         const int row_t = tl.row0 + rank * half_n;
         const int boxes = (half_n + BOX_TOKENS - 1) / BOX_TOKENS;
@@ -245,7 +253,7 @@ grouped_gemm_pair_fold_kernel(const __grid_constant__ CUtensorMap map_t, const _
                                   row_t + b * BOX_TOKENS, bar_full0 + s * 8);
         };
         int kb = 0;
-        if (tile == worker) {
+        if (first) {
           // the first tile's weights are on their way before the rows are there
           const int ahead = early ? min(STAGES, kblocks) : 0;
           for (; kb < ahead; ++kb) load_weights(kb, kb);
@@ -290,8 +298,12 @@ grouped_gemm_pair_fold_kernel(const __grid_constant__ CUtensorMap map_t, const _
       long long prof_mp = 0, prof_md = 0;
       const uint32_t ring = ptx::smem_u32(smem);
       const uint64_t da0 = ptx::smem_desc_sw128(ring), db0 = ptx::smem_desc_sw128(ring + W_BYTES);
-      for (int tile = worker; tile < total_tiles && alive; tile += workers) {
-        cursor.locate(tile, p.w_tiles, p.group, p.num_experts, table, &tl);
+      while (alive) {
+        const int got = units.next<false>(&unit);
+        if (got <= 0) {
+          if (got < 0) report(0x5d0);
+          break;
+        }
         const uint32_t idesc = ptx::make_idesc(/*e4m3*/ 0, 256, (uint32_t)tl.n);
         for (int kb = 0; kb < kblocks; ++kb, ++step) {
           const int buf = step % BUFS;
@@ -334,14 +346,28 @@ grouped_gemm_pair_fold_kernel(const __grid_constant__ CUtensorMap map_t, const _
     // ---------------- factors: two warps take alternate groups of four K blocks, one tile after the other ----------------
     constexpr int LANES = TOK / 32;  // tokens per lane
     const int me = warp - (kFoldWarps + 2);
+    int more = 0;  // the list goes on
+    auto add_units = [&](int batch) {
+      UnitPlan plan;
+      plan.init(total_tiles, kblocks, 0, workers, worker);
+      more = PairList::fill(list, list_bars, batch, plan, p.w_tiles, p.group, p.num_experts, table);
+      if (more < 0) report(0x5b0);
+    };
+    if (me == 0) add_units(0);
     pdl_wait();
     uint32_t group = 0;  // groups so far (selects the slot and its phase)
     bool alive = true;
     int ltile = 0;
     const bool vec = (kblocks & 3) == 0 && aligned16(p.a_scale) && aligned16(p.w_scale);
     const int wblocks = (int)(p.w_rows / 128);
-    for (int tile = worker; tile < total_tiles && alive; tile += workers, ++ltile) {
-      cursor.locate(tile, p.w_tiles, p.group, p.num_experts, table, &tl);
+    for (; alive; ++ltile) {
+      // half a batch ahead: every reader is at most a few tiles (of the factor ring) behind, so nobody is waited for
+      if (more > 0 && ltile % kListUnits == kListUnits / 2) add_units(ltile / kListUnits + 1);
+      const int got = units.next<true>(&unit);
+      if (got <= 0) {
+        if (got < 0) report(0x5e0);
+        break;
+      }
       int32_t ids[LANES], row[LANES];  // slot and scale row of token lane + 32 j
 #pragma unroll
       for (int j = 0; j < LANES; ++j) {
@@ -429,8 +455,12 @@ grouped_gemm_pair_fold_kernel(const __grid_constant__ CUtensorMap map_t, const _
     int ltile = 0;
     bool alive = true;
     long long prof_fw = 0, prof_fb = 0, prof_sw = 0, prof_epi = 0;
-    for (int tile = worker; tile < total_tiles && alive; tile += workers, ++ltile) {
-      cursor.locate(tile, p.w_tiles, p.group, p.num_experts, table, &tl);
+    for (; alive; ++ltile) {
+      const int got = units.next<true>(&unit);
+      if (got <= 0) {
+        if (got < 0) report(0x5f0);
+        break;
+      }
       const int pieces = max(0, ((tl.n >> 4) - half + 1) >> 1);  // 16-token pieces half, half + 2, ..
       unsigned long long acc[PIECES][8];  // [0..3] rows 0-15 of the quarter, [4..7] rows 16-31
 #pragma unroll
@@ -636,7 +666,7 @@ struct WideGeo {
   static constexpr int META_BYTES = META_TILES * META_WORDS * 4;
   static constexpr int AMAX_BYTES = 2 * 4 * 128 * 4;  // two tiles' [column piece][token] largest magnitudes
   static constexpr int bytes(int num_experts) {
-    return STAGES * STAGE_BYTES + BAR_BYTES + SC_SLOTS * SLOT_BYTES + META_BYTES + AMAX_BYTES + pair_table_bytes(num_experts);
+    return STAGES * STAGE_BYTES + BAR_BYTES + kListBytes + SC_SLOTS * SLOT_BYTES + META_BYTES + AMAX_BYTES + pair_table_bytes(num_experts);
   }
 };
 static_assert(WideGeo::bytes(1024) <= kMaxSmem, "shared memory");
@@ -656,8 +686,10 @@ grouped_gemm_pair_fold_wide_kernel(const __grid_constant__ CUtensorMap map_t, co
   uint64_t* sc_full = part_empty + 4;        // [slots] scale warps -> fold
   uint64_t* sc_empty = sc_full + SC_SLOTS;   // [slots] fold -> scale warps
   uint64_t* amax_bar = sc_empty + SC_SLOTS;  // [4] the four warps that hold a token's 128 channels
-  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(amax_bar + 4);
-  uint8_t* scales = smem + STAGES * STAGE_BYTES + BAR_BYTES;  // [slot][K block][half][token]
+  uint64_t* list_bars = amax_bar + 4;        // [4] (PairList)
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(list_bars + 4);
+  int4* list = reinterpret_cast<int4*>(smem + STAGES * STAGE_BYTES + BAR_BYTES);
+  uint8_t* scales = smem + STAGES * STAGE_BYTES + BAR_BYTES + kListBytes;  // [slot][K block][half][token]
   int32_t* meta = reinterpret_cast<int32_t*>(scales + SC_SLOTS * G::SLOT_BYTES);  // [tile]
   float* amax_buf = reinterpret_cast<float*>(scales + SC_SLOTS * G::SLOT_BYTES + G::META_BYTES);
   int32_t* table = reinterpret_cast<int32_t*>(scales + SC_SLOTS * G::SLOT_BYTES + G::META_BYTES + G::AMAX_BYTES);
@@ -681,6 +713,7 @@ grouped_gemm_pair_fold_wide_kernel(const __grid_constant__ CUtensorMap map_t, co
       ptx::mbar_init(&sc_full[s], 1);
       ptx::mbar_init(&sc_empty[s], kFoldWarps);
     }
+    PairList::init_barriers(list_bars, 3);  // TMA, two factor warps
     ptx::fence_barrier_init();
   }
   if (warp == kFoldWarps && lane == 0) {
@@ -702,8 +735,9 @@ grouped_gemm_pair_fold_wide_kernel(const __grid_constant__ CUtensorMap map_t, co
   const uint32_t tmem_base = *tmem_slot;
   const int kblocks = p.kblocks;
   const int total_tiles = table[3 * p.num_experts] * p.w_tiles;
-  PairCursor cursor;
-  PairTile tl;
+  PairList units(list, list_bars);
+  PairUnit unit;
+  const PairTile& tl = unit.tl;
 
   if (MOVE && warp >= kFoldWarps) asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(kOtherRegs));
   if (warp == kFoldWarps) {
@@ -713,8 +747,12 @@ grouped_gemm_pair_fold_wide_kernel(const __grid_constant__ CUtensorMap map_t, co
       uint32_t phase = 0;
       bool alive = true;
       const uint32_t ring = ptx::smem_u32(smem), bar_full0 = ptx::smem_u32(full_bar) & ~ptx::kPeerRankBit;
-      for (int tile = worker; tile < total_tiles && alive; tile += workers) {
-        cursor.locate(tile, p.w_tiles, p.group, p.num_experts, table, &tl);
+      for (bool first = true; alive; first = false) {
+        const int got = units.next<false>(&unit);
+        if (got <= 0) {
+          if (got < 0) report(0x5c0);
+          break;
+        }
         const int half_n = tl.n >> 1;
         const int row_t = tl.row0 + rank * half_n;
         const int boxes = (half_n + BOX_TOKENS - 1) / BOX_TOKENS;  // lanes past them multiply what an earlier stage left
@@ -731,7 +769,7 @@ grouped_gemm_pair_fold_wide_kernel(const __grid_constant__ CUtensorMap map_t, co
                                   bar_full0 + s * 8);
         };
         int kb = 0;
-        if (tile == worker) {
+        if (first) {
           // the first tile's weights are on their way before the rows are there
           const int ahead = early ? min(STAGES, kblocks) : 0;
           for (; kb < ahead; ++kb) load_weights(kb, kb);
@@ -819,14 +857,28 @@ grouped_gemm_pair_fold_wide_kernel(const __grid_constant__ CUtensorMap map_t, co
   } else if (warp >= kFoldWarps + 2) {
     // ---------------- factors: two warps take alternate groups of eight K blocks ----------------
     const int me = warp - (kFoldWarps + 2);
+    int more = 0;
+    auto add_units = [&](int batch) {
+      UnitPlan plan;
+      plan.init(total_tiles, kblocks, 0, workers, worker);
+      more = PairList::fill(list, list_bars, batch, plan, p.w_tiles, p.group, p.num_experts, table);
+      if (more < 0) report(0x5b0);
+    };
+    if (me == 0) add_units(0);
     pdl_wait();
     uint32_t group = 0;
     bool alive = true;
     int ltile = 0;
     const bool vec = (kblocks & 3) == 0 && aligned16(p.a_scale) && aligned16(p.w_scale);
     const int wblocks = (int)(p.w_rows / 128);
-    for (int tile = worker; tile < total_tiles && alive; tile += workers, ++ltile) {
-      cursor.locate(tile, p.w_tiles, p.group, p.num_experts, table, &tl);
+    for (; alive; ++ltile) {
+      // half a batch ahead: every reader is at most a few tiles (of the factor ring) behind, so nobody is waited for
+      if (more > 0 && ltile % kListUnits == kListUnits / 2) add_units(ltile / kListUnits + 1);
+      const int got = units.next<true>(&unit);
+      if (got <= 0) {
+        if (got < 0) report(0x5e0);
+        break;
+      }
       const int half_n = tl.n >> 1, first = tl.row0 + rank * half_n;
       int32_t ids[4], row[4];  // slot and scale row of this CTA's token lane + 32 j
 #pragma unroll

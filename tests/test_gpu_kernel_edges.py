@@ -79,6 +79,25 @@ def test_rows_per_expert_at_tile_edges(fg, tile, kind):
     assert_close_moe(out, ref, "fp8" if kind in ("channel", "block") else "bf16", f"{kind} tile {tile}")
 
 
+@pytest.mark.parametrize("H,I", [(128, 9600), (19200, 128)])
+@pytest.mark.parametrize("kind", ["bf16", "block"])
+def test_many_tiles_per_worker(fg, H, I, kind):
+    """CTA-pair GEMMs (gate/up, then down) whose workers have 65 tiles each: their list of tiles is refilled twice."""
+    E = 64
+    x, w1, w2, g = _layer(E + 32, H, I, E, 9)
+    ids = torch.cat([torch.arange(E), torch.arange(32)]).to(torch.int32).view(-1, 1)
+    tw = torch.rand(E + 32, 1, generator=g) + 0.5
+    if kind == "bf16":
+        out = fg.fused_experts(x.cuda(), w1.cuda(), w2.cuda(), tw.cuda(), ids.cuda(), variant="tcgen05")
+        ref = OE.fused_experts(x, w1, w2, tw, ids)
+    else:
+        (w1q, w1s), (w2q, w2s) = OQ.quant_weight_block128(w1), OQ.quant_weight_block128(w2)
+        out = fg.fused_experts(x.cuda(), w1q.cuda(), w2q.cuda(), tw.cuda(), ids.cuda(), use_fp8_w8a8=True, w1_scale=w1s.cuda(),
+                               w2_scale=w2s.cuda(), block_shape=[128, 128], variant="tcgen05")
+        ref = OE.fused_experts_fp8(x, w1q, w1s, w2q, w2s, tw, ids)
+    assert_close_moe(out, ref, "fp8" if kind == "block" else "bf16", f"{kind} H={H} I={I}")
+
+
 def test_e4m3_kernels_without_the_register_move(tmp_path):
     """The e4m3 block-scale kernels as they are launched where the compiler left too few registers for setmaxnreg: same sums
     in the same order, so the same bits."""
