@@ -44,24 +44,21 @@ constexpr int stage_bytes(int token_tile) { return W_BYTES + token_tile / 2 * KB
 constexpr int TMEM_COLS = 512;
 constexpr int ACC_COLS = 256;
 // Epilogue warps: 16 (4 per TMEM lane quarter), so that their TMEM, shuffle, shared-memory and store latencies overlap;
-// with 8 a short main loop waited for them (7.3k cycles per tile against 6.1k of MMAs at K = 768).  The gate/up exchange of
-// M-major weights needs shared memory per group of four, so that kernel keeps 8.
-constexpr int epi_warps(bool exchange) { return exchange ? 8 : 16; }
+// with 8 a short main loop waited for them (7.3k cycles per tile against 6.1k of MMAs at K = 768).
+constexpr int kEpiWarps = 16;
 // TMA warps: they take the K steps in turn.  Waiting for a stage, arming it and issuing two to five copies takes one thread
 // about 430 cycles, and with one warp that was the pace of every tile whose MMAs need less (SM cycles per K step with 64, 128,
 // 192 and 256 tokens per tile: 431, 470, 493, 508; two warps: 288 tokens in two tiles 500 -> 405, 256 tokens 508 -> 465; a
 // third one changes nothing).  Qwen3, 128 experts of 288 rows: gate/up GEMM 270 -> 251 us; Mixtral 549 -> 513 us.
 constexpr int kProducers = 2;
-constexpr int pair_threads(bool exchange) { return (epi_warps(exchange) + kProducers + 2) * 32; }
+constexpr int kThreads = (kEpiWarps + kProducers + 2) * 32;
 constexpr int BOX_TOKENS = 32;                      // token rows per TMA box
-constexpr int STRIP_BYTES = kStripBytes;
-constexpr int EX_PITCH = 20;                        // floats per lane row of the gate/up exchange (16 tokens + padding)
-constexpr int EX_BYTES = 128 * EX_PITCH * 4;        // per half of the epilogue warps
+constexpr int STRIP_BYTES = kStripBytes;             // per epilogue warp; also holds its 1 KB of the gate/up exchange
 constexpr int BAR_BYTES = 256;
-constexpr int smem_bytes(int num_experts, bool exchange) {
-  return RING_BYTES + BAR_BYTES + kListBytes + (exchange ? 2 * EX_BYTES : epi_warps(false) * STRIP_BYTES) + pair_table_bytes(num_experts);
+constexpr int smem_bytes(int num_experts) {
+  return RING_BYTES + BAR_BYTES + kListBytes + kEpiWarps * STRIP_BYTES + pair_table_bytes(num_experts);
 }
-static_assert(smem_bytes(1024, true) <= 227 * 1024, "shared memory");
+static_assert(smem_bytes(1024) <= 227 * 1024, "shared memory");
 
 struct PairParams {
   const int32_t* sorted_token_ids;
@@ -104,6 +101,9 @@ __device__ __forceinline__ bool warp_wait_relaxed(uint64_t* bar, uint32_t parity
   return __all_sync(0xffffffffu, ptx::mbar_wait_relaxed(bar, parity));
 }
 
+// Two epilogue warps (gate rows, up rows) meet.  Barriers 5-12; 1-4 are the groups of four, 0 is __syncthreads.
+__device__ __forceinline__ void pair_of_warps_sync(int pair) { asm volatile("bar.sync %0, 64;" ::"r"(5 + pair) : "memory"); }
+
 // Whether `pred` holds for any thread of the four epilogue warps (one of each TMEM lane quarter) that share barrier `bar`.
 __device__ __forceinline__ bool any_of_four_warps(int bar, bool pred) {
   int v = pred;
@@ -115,10 +115,10 @@ __device__ __forceinline__ bool any_of_four_warps(int bar, bool pred) {
 }
 
 template <bool GATED, bool F8, bool EXTRA, bool WMN, bool GATHER>
-__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(pair_threads(GATED && WMN), 1)
+__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 1)
 grouped_gemm_pair_kernel(const __grid_constant__ CUtensorMap map_t, const __grid_constant__ CUtensorMap map_w,
                          const PairParams p) {
-  constexpr int kEpiWarps = epi_warps(GATED && WMN), HALVES = kEpiWarps / 4;  // warps per lane quarter
+  constexpr int HALVES = kEpiWarps / 4;  // warps per lane quarter
   constexpr int kMmaWarp = kEpiWarps + kProducers;
   extern __shared__ __align__(1024) uint8_t smem[];  // aligned by declaration: every address below is a constant
   const int stages = p.stages, stage_size = p.stage_bytes;
@@ -131,7 +131,7 @@ grouped_gemm_pair_kernel(const __grid_constant__ CUtensorMap map_t, const __grid
   uint64_t* list_bars = bars + 2 * MAX_STAGES + 5;   // [4] (PairList)
   int4* list = reinterpret_cast<int4*>(smem + RING_BYTES + BAR_BYTES);
   uint8_t* strips = smem + RING_BYTES + BAR_BYTES + kListBytes;
-  int32_t* table = reinterpret_cast<int32_t*>(strips + (GATED && WMN ? 2 * EX_BYTES : kEpiWarps * STRIP_BYTES));
+  int32_t* table = reinterpret_cast<int32_t*>(strips + kEpiWarps * STRIP_BYTES);
 
   const int warp = ptx::uniform_warp_id(), lane = threadIdx.x & 31;
   const int rank = (int)ptx::cluster_ctarank();
@@ -380,7 +380,8 @@ grouped_gemm_pair_kernel(const __grid_constant__ CUtensorMap map_t, const __grid
       }
       // first output channel of this warp, and per-channel factors / biases of its rows: gated {gate g, gate g+8, up g,
       // up g+8}, plain {g, g+8, g+16, g+24}
-      const int ch0 = GATED ? tl.w_tile * 128 + rank * 64 + quarter * 16 : tl.w_tile * 256 + rank * 128 + quarter * 32;
+      const int quarter_ch = WMN ? 32 * (quarter & 1) + 16 * (quarter >> 1) : 16 * quarter;
+      const int ch0 = GATED ? tl.w_tile * 128 + rank * 64 + quarter_ch : tl.w_tile * 256 + rank * 128 + quarter * 32;
       float cv[4] = {0.f, 0.f, 0.f, 0.f};
       if constexpr ((F8 || EXTRA) && !WMN) {
         const float* vec = F8 ? p.w_scale : p.bias;
@@ -485,78 +486,75 @@ grouped_gemm_pair_kernel(const __grid_constant__ CUtensorMap map_t, const __grid
           }
         }
         const int src_lane = (c & 1) * 16;
-        if constexpr (GATED && WMN) {
-          // gate rows are lanes 0-63, up rows 64-127: the four warps of a half meet in shared memory
-          float* ex = reinterpret_cast<float*>(strips + half * EX_BYTES);
+        float rs[4];  // columns 2t, 2t+1, 8+2t, 9+2t
 #pragma unroll
-          for (int q = 0; q < 4; ++q) {
-            const int row = quarter * 32 + g + 8 * (q & 1) + 16 * (q >> 1);
-            const uint32_t* v = (q >> 1) ? hi : lo;
-            *reinterpret_cast<float2*>(ex + row * EX_PITCH + 2 * t) =
-                make_float2(__uint_as_float(v[2 * (q & 1)]), __uint_as_float(v[2 * (q & 1) + 1]));
-            *reinterpret_cast<float2*>(ex + row * EX_PITCH + 8 + 2 * t) =
-                make_float2(__uint_as_float(v[4 + 2 * (q & 1)]), __uint_as_float(v[4 + 2 * (q & 1) + 1]));
-          }
-          asm volatile("bar.sync %0, 128;" ::"r"(1 + half) : "memory");
-          const int i = quarter * 32 + lane, u = i >> 3, oct = i & 7;  // token of the chunk, 8 channels
-          const int tok = j * 16 + u;
-          const float rs = __shfl_sync(0xffffffffu, rs_c, src_lane + u);
-          const int64_t ch = tl.w_tile * 128 + rank * 64 + oct * 8;
-          if (tok < tl.cols && ch < p.n) {
-            uint32_t w[4];
+        for (int q = 0; q < 4; ++q) rs[q] = __shfl_sync(0xffffffffu, rs_c, src_lane + (q >> 1) * 8 + 2 * t + (q & 1));
+        if constexpr (GATED) {
+          if constexpr (WMN) {
+            // M-major gate rows are in lanes 0-63 and the up rows of the same channels in lanes 64-127: two warps swap halves
+            // through shared memory, lane by lane.  The gate warp finishes its first 16 channels, the up warp the other 16.
+            // (Four warps that met twice a chunk and read back by token, eight such warps: 8500 cycles for 128 tokens, more than
+            // the 20 K steps of the reference shape.  1024 tokens of it through the operator: 348 -> 326 us.)
+            const bool gate = quarter < 2;
+            float4* mine = reinterpret_cast<float4*>(strip) + lane;
+            const float4* theirs = reinterpret_cast<const float4*>(strips + (warp ^ 2) * STRIP_BYTES) + lane;
 #pragma unroll
-            for (int v = 0; v < 4; ++v) {
-              const float* e0 = ex + (oct * 8 + 2 * v) * EX_PITCH + u;
-              const float g0 = e0[0], g1 = e0[EX_PITCH], u0 = e0[64 * EX_PITCH], u1 = e0[65 * EX_PITCH];
-              w[v] = pack_bf16x2(act_mul_fast(g0 * rs, u0 * rs, p.activation), act_mul_fast(g1 * rs, u1 * rs, p.activation));
+            for (int q = 0; q < 2; ++q) {
+              uint32_t o[4];
+#pragma unroll
+              for (int i = 0; i < 4; ++i) o[i] = gate ? hi[4 * q + i] : lo[4 * q + i];
+              mine[32 * q] = make_float4(__uint_as_float(o[0]), __uint_as_float(o[1]), __uint_as_float(o[2]), __uint_as_float(o[3]));
             }
-            *reinterpret_cast<uint4*>(reinterpret_cast<__nv_bfloat16*>(p.out) + (int64_t)(tl.row0 + tok) * p.n + ch) =
-                make_uint4(w[0], w[1], w[2], w[3]);
-          }
-          asm volatile("bar.sync %0, 128;" ::"r"(1 + half) : "memory");
-        } else {
-          float rs[4];  // columns 2t, 2t+1, 8+2t, 9+2t
+            pair_of_warps_sync(half * 2 + (quarter & 1));
 #pragma unroll
-          for (int q = 0; q < 4; ++q) rs[q] = __shfl_sync(0xffffffffu, rs_c, src_lane + (q >> 1) * 8 + 2 * t + (q & 1));
-          if constexpr (GATED) {
+            for (int q = 0; q < 2; ++q) {
+              const float4 v = theirs[32 * q];
+              const uint32_t got[4] = {__float_as_uint(v.x), __float_as_uint(v.y), __float_as_uint(v.z), __float_as_uint(v.w)};
+#pragma unroll
+              for (int i = 0; i < 4; ++i) {
+                if (gate) hi[4 * q + i] = got[i];
+                else lo[4 * q + i] = got[i];
+              }
+            }
+            pair_of_warps_sync(half * 2 + (quarter & 1));  // both have read: the strips are free
+          }
+          uint32_t m[4];
+#pragma unroll
+          for (int q = 0; q < 4; ++q) {  // q = 2 * (column group) + (row half)
+            const int i = 4 * (q >> 1) + 2 * (q & 1);
+            float o[2];
+#pragma unroll
+            for (int v = 0; v < 2; ++v) {
+              const float gv = __uint_as_float(lo[i + v]), uv = __uint_as_float(hi[i + v]), r = rs[2 * (q >> 1) + v];
+              if constexpr (EXTRA)
+                o[v] = gated_output<true>(gv, uv, cv[q & 1], cv[2 + (q & 1)], r, p.activation, p.act_alpha, p.act_limit);
+              else if constexpr (F8)  // (accumulator * row scale) * channel scale, then the activation
+                o[v] = act_mul_fast(gv * r * cv[q & 1], uv * r * cv[2 + (q & 1)], p.activation);
+              else
+                o[v] = act_mul_fast(gv * r, uv * r, p.activation);
+            }
+            m[q] = pack_bf16x2(o[0], o[1]);
+          }
+          strip_put16(strip, 48, 0, lane, m);
+          strip_store_sorted(strip, lane, reinterpret_cast<__nv_bfloat16*>(p.out) + (int64_t)(tl.row0 + j * 16) * p.n, p.n, ch0,
+                             tl.cols - j * 16);
+        } else {
+#pragma unroll
+          for (int h = 0; h < 2; ++h) {
             uint32_t m[4];
 #pragma unroll
-            for (int q = 0; q < 4; ++q) {  // q = 2 * (column group) + (row half)
+            for (int q = 0; q < 4; ++q) {
               const int i = 4 * (q >> 1) + 2 * (q & 1);
-              float o[2];
-#pragma unroll
-              for (int v = 0; v < 2; ++v) {
-                const float gv = __uint_as_float(lo[i + v]), uv = __uint_as_float(hi[i + v]), r = rs[2 * (q >> 1) + v];
-                if constexpr (EXTRA)
-                  o[v] = gated_output<true>(gv, uv, cv[q & 1], cv[2 + (q & 1)], r, p.activation, p.act_alpha, p.act_limit);
-                else if constexpr (F8)  // (accumulator * row scale) * channel scale, then the activation
-                  o[v] = act_mul_fast(gv * r * cv[q & 1], uv * r * cv[2 + (q & 1)], p.activation);
-                else
-                  o[v] = act_mul_fast(gv * r, uv * r, p.activation);
-              }
-              m[q] = pack_bf16x2(o[0], o[1]);
+              const uint32_t* a = h ? hi : lo;
+              const float v0 = __uint_as_float(a[i]), v1 = __uint_as_float(a[i + 1]);
+              const float r0 = rs[2 * (q >> 1)], r1 = rs[2 * (q >> 1) + 1], c0 = cv[2 * h + (q & 1)];
+              if constexpr (F8) m[q] = pack_bf16x2(v0 * r0 * c0, v1 * r1 * c0);
+              else m[q] = pack_bf16x2((v0 + c0) * r0, (v1 + c0) * r1);
             }
-            strip_put16(strip, 48, 0, lane, m);
-            strip_store_sorted(strip, lane, reinterpret_cast<__nv_bfloat16*>(p.out) + (int64_t)(tl.row0 + j * 16) * p.n, p.n, ch0,
-                               tl.cols - j * 16);
-          } else {
-#pragma unroll
-            for (int h = 0; h < 2; ++h) {
-              uint32_t m[4];
-#pragma unroll
-              for (int q = 0; q < 4; ++q) {
-                const int i = 4 * (q >> 1) + 2 * (q & 1);
-                const uint32_t* a = h ? hi : lo;
-                const float v0 = __uint_as_float(a[i]), v1 = __uint_as_float(a[i + 1]);
-                const float r0 = rs[2 * (q >> 1)], r1 = rs[2 * (q >> 1) + 1], c0 = cv[2 * h + (q & 1)];
-                if constexpr (F8) m[q] = pack_bf16x2(v0 * r0 * c0, v1 * r1 * c0);
-                else m[q] = pack_bf16x2((v0 + c0) * r0, (v1 + c0) * r1);
-              }
-              strip_put16(strip, 80, 16 * h, lane, m);
-            }
-            strip_store_slots(strip, lane, p.out, p.out_rows, p.n, ch0, __shfl_sync(0xffffffffu, slot_c, src_lane + (lane >> 2)),
-                              __shfl_sync(0xffffffffu, slot_c, src_lane + 8 + (lane >> 2)));
+            strip_put16(strip, 80, 16 * h, lane, m);
           }
+          strip_store_slots(strip, lane, p.out, p.out_rows, p.n, ch0, __shfl_sync(0xffffffffu, slot_c, src_lane + (lane >> 2)),
+                            __shfl_sync(0xffffffffu, slot_c, src_lane + 8 + (lane >> 2)));
         }
       }
       // the accumulator may be overwritten from here on: tell CTA 0's MMA warp
@@ -695,9 +693,9 @@ namespace {
 template <bool GATED, bool F8, bool EXTRA, bool WMN, bool GATHER>
 int launch(const GemmParams& g, cudaStream_t st) {
   constexpr int ELEM = F8 ? 1 : 2;
-  constexpr int MAX_SMEM = smem_bytes(1024, GATED && WMN);
+  constexpr int MAX_SMEM = smem_bytes(1024);
   auto kernel = grouped_gemm_pair_kernel<GATED, F8, EXTRA, WMN, GATHER>;
-  const int smem = smem_bytes(g.num_experts, GATED && WMN);
+  const int smem = smem_bytes(g.num_experts);
   static PerDeviceOnce once_attr;  // the opt-in to > 48 KB of dynamic shared memory is per device
   const cudaError_t attr_err = per_device_once(once_attr, [&] {
     return cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, MAX_SMEM);
@@ -767,7 +765,7 @@ int launch(const GemmParams& g, cudaStream_t st) {
       FMOE_CUDA_OK(cudaMemsetAsync(g.split_ws, 0, kSplitCounters * 4, st));
     }
   }
-  launch_pdl(kernel, dim3(2 * workers), dim3(pair_threads(GATED && WMN)), smem, st, map_t, map_w, p);
+  launch_pdl(kernel, dim3(2 * workers), dim3(kThreads), smem, st, map_t, map_w, p);
   return launch_status("grouped_gemm_pair_kernel");
 }
 
