@@ -262,3 +262,30 @@ def test_header_compiles_as_plain_c_and_cpp(tmp_path):
     subprocess.run([gcc, "-std=c99", "-I", os.path.join(ROOT, "include"), str(src), "-o", str(exe)], check=True)
     out = subprocess.run([str(exe)], check=True, capture_output=True, text=True).stdout.split()
     assert [int(v) for v in out] == [ctypes.sizeof(_C.GemmArgs), ctypes.sizeof(_C.FusedArgs), _C.W_N_MAJOR, _C.SCALE_CHANNEL]
+
+
+def test_hook_output_type_follows_the_serving_stack(monkeypatch):
+    """Without sglang the import path is searched once; a serving stack that is loaded later is found all the same."""
+    import importlib
+    import sys
+    import types
+
+    fm = importlib.import_module("flaggems_sglang_b200.ops.fused_moe")
+    searched = []
+
+    class Finder:
+        def find_spec(self, name, path=None, target=None):
+            searched.append(name)
+
+    for name in [m for m in sys.modules if m.split(".")[0] == "sglang"]:
+        monkeypatch.delitem(sys.modules, name)
+    monkeypatch.setattr(sys, "meta_path", [Finder()])
+    monkeypatch.setattr(fm, "_sglang_missing", False)
+    for _ in range(3):
+        assert fm._standard_output_type() is fm.StandardCombineInput
+    assert searched == ["sglang"]
+    path = "sglang.srt.layers.moe.token_dispatcher.standard".split(".")
+    for i in range(len(path)):
+        monkeypatch.setitem(sys.modules, ".".join(path[:i + 1]), types.ModuleType(path[i]))
+    sys.modules[".".join(path)].StandardCombineInput = dict
+    assert fm._standard_output_type() is dict
