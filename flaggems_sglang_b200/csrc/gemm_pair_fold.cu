@@ -95,6 +95,7 @@ struct FoldParams {
   int32_t out_dtype;  // gate/up: FMOE_F32, FMOE_BF16 or (wide) FMOE_E4M3 with out_scale
   float* out_scale;   // [rows, n / 128]
   int32_t min_rows, max_rows;  // experts of this launch
+  bool stores_of_32;           // rows of the output start at multiples of 32 bytes
   bool by_expert;              // narrow, fp32 gate/up output: kNarrowRows rows per expert instead of one per position
 };
 
@@ -128,14 +129,27 @@ __device__ __forceinline__ unsigned long long lds64(uint32_t addr) {
   return v;
 }
 
+// One 32-byte store where the destination is aligned to it, else two of 16 bytes.  The wide kernel's lanes store to 32 rows at
+// once, so that every instruction touches 32 lines whatever it writes.  (Down GEMM, 64 experts of 512 rows,
+// H = 7168, I = 2048: 650 us with 16-byte stores, 550 with 32.)
+__device__ __forceinline__ void store_32_bytes(void* dst, const uint32_t (&w)[8], bool whole) {
+  if (whole) {
+    asm volatile("st.global.v8.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8};" ::"l"(dst), "r"(w[0]), "r"(w[1]), "r"(w[2]), "r"(w[3]), "r"(w[4]),
+                 "r"(w[5]), "r"(w[6]), "r"(w[7])
+                 : "memory");
+  } else {
+    reinterpret_cast<uint4*>(dst)[0] = make_uint4(w[0], w[1], w[2], w[3]);
+    reinterpret_cast<uint4*>(dst)[1] = make_uint4(w[4], w[5], w[6], w[7]);
+  }
+}
 // 32 values times s as bf16
-__device__ __forceinline__ void store32(__nv_bfloat16* dst, const float* v, float s) {
+__device__ __forceinline__ void store32(__nv_bfloat16* dst, const float* v, float s, bool whole) {
 #pragma unroll
-  for (int q = 0; q < 4; ++q) {
-    uint32_t w[4];
+  for (int q = 0; q < 2; ++q) {
+    uint32_t w[8];
 #pragma unroll
-    for (int j = 0; j < 4; ++j) w[j] = pack_bf16x2(v[8 * q + 2 * j] * s, v[8 * q + 2 * j + 1] * s);
-    reinterpret_cast<uint4*>(dst)[q] = make_uint4(w[0], w[1], w[2], w[3]);
+    for (int j = 0; j < 8; ++j) w[j] = pack_bf16x2(v[16 * q + 2 * j] * s, v[16 * q + 2 * j + 1] * s);
+    store_32_bytes(dst + 16 * q, w, whole);
   }
 }
 
@@ -1060,19 +1074,17 @@ grouped_gemm_pair_fold_wide_kernel(const __grid_constant__ CUtensorMap map_t, co
           amax = fmaxf(fmaxf(am[0], am[128]), fmaxf(am[256], am[384]));
           if (mine && slot >= 0) {
             const float s = group_scale(amax), r = __frcp_rn(s);
-            uint4* dst = reinterpret_cast<uint4*>(reinterpret_cast<uint8_t*>(p.out) + at);
+            uint32_t w[8];
 #pragma unroll
-            for (int h = 0; h < 2; ++h) {
+            for (int u = 0; u < 4; ++u) {
               float v[8];
-              uint2 q[2];
 #pragma unroll
-              for (int u = 0; u < 2; ++u) {
-#pragma unroll
-                for (int i = 0; i < 8; ++i) v[i] = acc[16 * h + 8 * u + i];
-                q[u] = quant8(v, s, r, amax <= 3.0e38f);
-              }
-              dst[h] = make_uint4(q[0].x, q[0].y, q[1].x, q[1].y);
+              for (int i = 0; i < 8; ++i) v[i] = acc[8 * u + i];
+              const uint2 q = quant8(v, s, r, amax <= 3.0e38f);
+              w[2 * u] = q.x;
+              w[2 * u + 1] = q.y;
             }
+            store_32_bytes(reinterpret_cast<uint8_t*>(p.out) + at, w, p.stores_of_32);
             if (cpart == 0) p.out_scale[at >> 7] = s;  // n is a multiple of 128
           }
         } else if (mine && slot >= 0) {
@@ -1081,7 +1093,7 @@ grouped_gemm_pair_fold_wide_kernel(const __grid_constant__ CUtensorMap map_t, co
 #pragma unroll
             for (int v = 0; v < 8; ++v) dst[v] = make_float4(acc[4 * v], acc[4 * v + 1], acc[4 * v + 2], acc[4 * v + 3]);
           } else {
-            store32(reinterpret_cast<__nv_bfloat16*>(p.out) + at, acc, 1.0f);
+            store32(reinterpret_cast<__nv_bfloat16*>(p.out) + at, acc, 1.0f, p.stores_of_32);
           }
         }
       } else if (mine && slot >= 0) {
@@ -1091,7 +1103,7 @@ grouped_gemm_pair_fold_wide_kernel(const __grid_constant__ CUtensorMap map_t, co
 #pragma unroll
         for (int h = 0; h < 2; ++h) {
           const int64_t colg = (int64_t)m[258] * 256 + 128 * h + 32 * cpart;
-          if (obase && colg < p.n) store32(obase + colg, &acc[32 * h], rs);
+          if (obase && colg < p.n) store32(obase + colg, &acc[32 * h], rs, p.stores_of_32);
         }
       }
       if (PROF) prof_epi += clock64() - te0;
@@ -1172,6 +1184,7 @@ int launch(const GemmParams& g, int min_rows, int max_rows, cudaStream_t st) {
   p.out_dtype = g.out_dtype;
   p.out_scale = g.out_scale;
   p.by_expert = g.fold_by_expert && max_rows <= kNarrowRows;
+  p.stores_of_32 = !p.out_rows && reinterpret_cast<uintptr_t>(g.out) % 32 == 0;  // n is a multiple of 128
   p.min_rows = min_rows;
   p.max_rows = max_rows;
 

@@ -98,6 +98,37 @@ def test_many_tiles_per_worker(fg, H, I, kind):
     assert_close_moe(out, ref, "fp8" if kind == "block" else "bf16", f"{kind} H={H} I={I}")
 
 
+@pytest.mark.parametrize("gated", [True, False])
+def test_wide_e4m3_kernel_stores_to_rows_at_16_bytes(fg, gated):
+    """The wide block-scale kernel stores 32 bytes at a time where the output is aligned to that, and 16 where it is not: the
+    same bits."""
+    from flaggems_sglang_b200 import _C
+    from flaggems_sglang_b200.ops.fused_moe import _gemm_args
+
+    g = torch.Generator().manual_seed(3)
+    rows, n, k = [70, 0, 300, 129], 384, 256
+    E, numel = len(rows), sum(rows)
+    ids = torch.repeat_interleave(torch.arange(E), torch.tensor(rows)).to(torch.int32).view(-1, 1).cuda()
+    sorted_ids, expert_ids, num_post = fg.moe_align_block_size(ids, 128, E)
+    cap = sorted_ids.numel()
+    a = torch.randn(cap, k, generator=g).to(torch.float8_e4m3fn).cuda()
+    w = torch.randn(E, (2 if gated else 1) * n, k, generator=g).to(torch.float8_e4m3fn).cuda()
+    a_scale, w_scale = torch.rand(cap, k // 128, generator=g).cuda(), torch.rand(E, w.shape[1] // 128, k // 128, generator=g).cuda()
+    out_rows, outs = cap if gated else numel, []
+    for shift in (0, 8, 16):  # bf16 elements
+        buf = torch.zeros(out_rows * n + 16, dtype=torch.bfloat16, device="cuda")
+        args = _gemm_args(variant=_C.VARIANTS["tcgen05"], activation=0, num_experts=E, top_k=1, block_size=128, numel=numel,
+                          sorted_cap=cap, max_blocks=cap // 128, sorted_token_ids=sorted_ids.data_ptr(),
+                          expert_ids=expert_ids.data_ptr(), num_tokens_post_padded=num_post.data_ptr(), dtype=_C.E4M3,
+                          out_dtype=_C.BF16, n=n, k=k, a_rows=cap, a=a.data_ptr(), a_scale=a_scale.data_ptr(), w=w.data_ptr(),
+                          w_scale=w_scale.data_ptr(), out=buf[shift:].data_ptr())
+        lib = _C.lib()
+        _C.check((lib.fmoe_gemm1_silu if gated else lib.fmoe_gemm2)(args, _C.stream_ptr()))
+        outs.append(buf[shift:shift + out_rows * n].clone())
+    assert float(outs[0].float().abs().sum()) > 0
+    assert torch.equal(outs[0], outs[1]) and torch.equal(outs[0], outs[2])
+
+
 def test_e4m3_kernels_without_the_register_move(tmp_path):
     """The e4m3 block-scale kernels as they are launched where the compiler left too few registers for setmaxnreg: same sums
     in the same order, so the same bits."""
