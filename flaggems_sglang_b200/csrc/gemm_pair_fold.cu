@@ -142,15 +142,12 @@ __device__ __forceinline__ void store_32_bytes(void* dst, const uint32_t (&w)[8]
     reinterpret_cast<uint4*>(dst)[1] = make_uint4(w[4], w[5], w[6], w[7]);
   }
 }
-// 32 values times s as bf16
-__device__ __forceinline__ void store32(__nv_bfloat16* dst, const float* v, float s, bool whole) {
+// 16 values times s as bf16
+__device__ __forceinline__ void store16(__nv_bfloat16* dst, const float* v, float s, bool whole) {
+  uint32_t w[8];
 #pragma unroll
-  for (int q = 0; q < 2; ++q) {
-    uint32_t w[8];
-#pragma unroll
-    for (int j = 0; j < 8; ++j) w[j] = pack_bf16x2(v[16 * q + 2 * j] * s, v[16 * q + 2 * j + 1] * s);
-    store_32_bytes(dst + 16 * q, w, whole);
-  }
+  for (int j = 0; j < 8; ++j) w[j] = pack_bf16x2(v[2 * j] * s, v[2 * j + 1] * s);
+  store_32_bytes(dst, w, whole);
 }
 
 __device__ __forceinline__ void sts64(uint32_t addr, unsigned long long v) {
@@ -649,26 +646,32 @@ grouped_gemm_pair_fold_kernel(const __grid_constant__ CUtensorMap map_t, const _
 }
 
 // ---------------------------------------------------------------------------------------------------------------------
-// Wide tiles (experts with many rows): the same fold with the TOKENS on the M side, 256 of one expert (128 in each CTA) x
-// 256 weight rows (CTA 0 loads the first 128: gate, or the tile's first half; CTA 1 the other 128).  A thread of the fold
-// then owns one token: its activation scale is ONE value per K block and the weight scale one value per 128 columns, and
-// TMEM is read 32 lanes wide.  With tokens on N every thread needs one factor per column: a 16-lane read-out with packed
-// factors takes 512 cycles of TMEM and 128-256 shared-memory loads per 128 x 256 partial, a 32-lane one 256 cycles and 1024
-// cycles of broadcast loads (both measured), against 310 cycles and 32 loads here.  In exchange M is always 256: tokens short
-// of that are lanes without work, so experts with few rows stay on the narrow kernel.
-//   TMEM: four partials of 128 columns.  A K block's MMAs go to two of them: the first holds rows 0-63 of both CTAs' weights,
-//   the second rows 64-127.
+// Wide tiles (experts with many rows): the same fold with the TOKENS on the M side, up to 256 of one expert (128 in each CTA)
+// x 256 weight rows (CTA 0 loads the tile's first 64 gate and 64 up channels, in turns of 16, or its first 128 rows; CTA 1
+// the others).  A thread of the fold then owns one token: its activation scale is ONE value per K block and the weight scale
+// one value per 128 rows, and TMEM is read 32 lanes wide (136 cycles for a 128 x 256 partial, its FMAs 256).  With tokens on N
+// every thread needs one factor per column: a 16-lane read-out with packed factors takes 128-256 shared-memory loads per
+// partial, a 32-lane one 1024 cycles of broadcast loads, against 32 loads here.
+//   M = 256, or 128 where the tile has at most 128 tokens (an expert's last or only tile: all others have 256).  An MMA of
+//   M = 128 takes as long, but leaves half as much to fold, half the lanes' power unspent and a third of shared memory's
+//   traffic: 0.50 us per K block and tile against 0.66 (DeepSeek-V3, 64 experts of 128 rows, both GEMMs: 717 -> 610 us; as
+//   M = 256 with lanes to spare such a tile took as long as a full one).  Its layout: lanes 0-63 hold the CTA's 64 tokens x
+//   CTA 0's weight rows, lanes 64-127 the same tokens x CTA 1's.
+//   TMEM: four partials of 128 columns (M = 128: the first 64 of each).  A K block's MMAs go to two of them: the first holds
+//   rows 0-63 of both CTAs' weights, the second rows 64-127.
 //   warps 0-15: fold + epilogue.  Eight warps fold each half, so that one half's TMEM reads run beside the other's FMAs and a
 //   partial is handed back while the other half is still being multiplied (one partial of 256 columns per K block, folded by
 //   all sixteen warps at once: gate/up + down of DeepSeek-V3, 4096 tokens, 3.43 ms; this split 3.25 ms).  Warp w: TMEM lanes
-//   32 * (w % 4).., half w / 8, columns 32 * (w / 4 % 2).. of gate and of up: 64 accumulators per thread.  The loop keeps
-//   its addresses in two registers; every spill inside it shows (44 bytes of them: 3.76 ms)
+//   32 * (w % 4).., half w / 8, the 64 columns of CTA w / 4 % 2's weight rows (M = 128: 32 columns): 64 accumulators per
+//   thread.  (Eight warps with 128 accumulators each spill: 530 -> 700 us and more.)
 //   warp 16 TMA, warp 17 MMA (CTA 0), warps 18-19 factors: products of token and weight scales in a ring of 4 slots of 8 K
-//   blocks, one slot wait per 8 K blocks of the fold
-// The gate/up kernel quantises its output: the tile's 128 channels of a token are one group, spread over four warps, which
-// exchange their largest magnitudes through shared memory.  (A bf16 activation and a quantiser pass took 135 us of that case.)
-// What bounds it: the power limit (980 W, SM clock 1.4 GHz of 1.965) and the fold, about 800 cycles per K block against 512
-// of MMA.
+//   blocks, one slot wait per 8 K blocks of the fold.  Their loop over the slot's halves is not unrolled: it would not fit
+//   their 64 registers (gate/up GEMM, 256 rows, 545 us with it, 519 without).
+// The gate/up kernel quantises its output: the tile's 128 channels of a token are one group, spread over four warps (M = 128:
+// eight), which exchange their largest magnitudes through shared memory.  (A bf16 activation and a quantiser pass took 135 us
+// of that case.)
+// What bounds it: shared memory (M = 256: 32 KB in and 48 KB of operand reads per K block, 640 cycles; the fold's round trip
+// through two partials makes it about 800), at the SM clock that the power limit leaves (1.4 GHz of 1.965).
 // ---------------------------------------------------------------------------------------------------------------------
 struct WideGeo {
   static constexpr int STAGE_BYTES = 2 * W_BYTES;  // 128 token rows + 128 weight rows per CTA
@@ -678,7 +681,8 @@ struct WideGeo {
   static constexpr int SLOT_BYTES = GROUP * KB_BYTES;
   static constexpr int META_WORDS = 2 * 128 + 4;   // slot ids, row weights, {first row, rows of this CTA, weight tile}
   static constexpr int META_BYTES = META_TILES * META_WORDS * 4;
-  static constexpr int AMAX_BYTES = 2 * 4 * 128 * 4;  // two tiles' [column piece][token] largest magnitudes
+  // two tiles' [column piece][token] largest magnitudes: four pieces of 128 tokens, then eight of 64 (M = 128)
+  static constexpr int AMAX_BYTES = 2 * (4 * 128 + 8 * 64) * 4;
   static constexpr int bytes(int num_experts) {
     return STAGES * STAGE_BYTES + BAR_BYTES + kListBytes + SC_SLOTS * SLOT_BYTES + META_BYTES + AMAX_BYTES + pair_table_bytes(num_experts);
   }
@@ -700,7 +704,8 @@ grouped_gemm_pair_fold_wide_kernel(const __grid_constant__ CUtensorMap map_t, co
   uint64_t* sc_full = part_empty + 4;        // [slots] scale warps -> fold
   uint64_t* sc_empty = sc_full + SC_SLOTS;   // [slots] fold -> scale warps
   uint64_t* amax_bar = sc_empty + SC_SLOTS;  // [4] the four warps that hold a token's 128 channels
-  uint64_t* list_bars = amax_bar + 4;        // [4] (PairList)
+  uint64_t* small_bar = amax_bar + 4;        // [2] M = 128: the eight warps that hold a token's 128 channels
+  uint64_t* list_bars = small_bar + 2;       // [4] (PairList)
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(list_bars + 4);
   int4* list = reinterpret_cast<int4*>(smem + STAGES * STAGE_BYTES + BAR_BYTES);
   uint8_t* scales = smem + STAGES * STAGE_BYTES + BAR_BYTES + kListBytes;  // [slot][K block][half][token]
@@ -727,7 +732,8 @@ grouped_gemm_pair_fold_wide_kernel(const __grid_constant__ CUtensorMap map_t, co
       ptx::mbar_init(&sc_full[s], 1);
       ptx::mbar_init(&sc_empty[s], kFoldWarps);
     }
-    PairList::init_barriers(list_bars, 3);  // TMA, two factor warps
+    for (int b = 0; b < 2; ++b) ptx::mbar_init(&small_bar[b], 8);
+    PairList::init_barriers(list_bars, 3 + (rank == 0));  // TMA, two factor warps, MMA
     ptx::fence_barrier_init();
   }
   if (warp == kFoldWarps && lane == 0) {
@@ -771,11 +777,12 @@ grouped_gemm_pair_fold_wide_kernel(const __grid_constant__ CUtensorMap map_t, co
         const int row_t = tl.row0 + rank * half_n;
         const int boxes = (half_n + BOX_TOKENS - 1) / BOX_TOKENS;  // lanes past them multiply what an earlier stage left
         const uint32_t bytes = 2 * (W_BYTES + boxes * (BOX_TOKENS * KBYTES));
-        const int32_t row_w = GATED ? tl.w_tile * 128 + rank * (int32_t)p.n : tl.w_tile * 256 + rank * 128;
+        const int32_t c0 = GATED ? tl.w_tile * 128 + rank * 64 : tl.w_tile * 256 + rank * 128;
         auto load_weights = [&](int kb, int s) {
           const uint32_t sw = ring + s * STAGE_BYTES + W_BYTES, bar0 = bar_full0 + s * 8;
           if (rank == 0) ptx::mbar_arrive_expect_tx(&full_bar[s], bytes);
-          ptx::tma_load_3d_pair(sw, &map_w, kb * KBYTES, row_w, tl.expert, bar0);
+          if constexpr (GATED) ptx::tma_load_5d_pair(sw, &map_w, kb * KBYTES, 0, 0, c0 >> 4, tl.expert, bar0);
+          else ptx::tma_load_3d_pair(sw, &map_w, kb * KBYTES, c0, tl.expert, bar0);
         };
         auto load_tokens = [&](int kb, int s) {
           for (int b = 0; b < boxes; ++b)
@@ -822,14 +829,19 @@ grouped_gemm_pair_fold_wide_kernel(const __grid_constant__ CUtensorMap map_t, co
   } else if (warp == kFoldWarps + 1) {
     // ---------------- MMA issuer (CTA 0): one fresh partial per K block ----------------
     if (rank == 0 && ptx::elect_one()) {
-      constexpr uint32_t idesc = ptx::make_idesc(/*e4m3*/ 0, 256, 128);
       int stage = 0;
       uint32_t phase = 0, step = 0;
       bool alive = true;
       long long prof_mp = 0, prof_md = 0;
       const uint32_t ring = ptx::smem_u32(smem);
       const uint64_t da0 = ptx::smem_desc_sw128(ring), db0 = ptx::smem_desc_sw128(ring + W_BYTES);
-      for (int tile = worker; tile < total_tiles && alive; tile += workers) {
+      while (alive) {
+        const int got = units.next<false>(&unit);
+        if (got <= 0) {
+          if (got < 0) report(0x5d0);
+          break;
+        }
+        const uint32_t idesc = ptx::make_idesc(/*e4m3*/ 0, tl.n <= 128 ? 128 : 256, 128);
         for (int kb = 0; kb < kblocks; ++kb, ++step) {
           const long long tm0 = PROF ? clock64() : 0;
           if (!ptx::mbar_wait(&full_bar[stage], phase)) {  // the data is there long before the partial is folded
@@ -875,7 +887,7 @@ grouped_gemm_pair_fold_wide_kernel(const __grid_constant__ CUtensorMap map_t, co
     auto add_units = [&](int batch) {
       UnitPlan plan;
       plan.init(total_tiles, kblocks, 0, workers, worker);
-      more = PairList::fill(list, list_bars, batch, plan, p.w_tiles, p.group, p.num_experts, table);
+      more = PairList::fill(list, list_bars, batch, plan, p.w_tiles, p.group, p.num_experts, table, 256);
       if (more < 0) report(0x5b0);
     };
     if (me == 0) add_units(0);
@@ -912,7 +924,7 @@ grouped_gemm_pair_fold_wide_kernel(const __grid_constant__ CUtensorMap map_t, co
         if ((int)(group & 1) != me) continue;
         const int slot = group % SC_SLOTS;
         bool granted = false;
-#pragma unroll
+#pragma unroll 1
         for (int q = 0; q < G::GROUP / 4; ++q) {
           const int kb = kb0 + 4 * q, left = kblocks - kb;
           if (left <= 0) break;
@@ -987,18 +999,22 @@ grouped_gemm_pair_fold_wide_kernel(const __grid_constant__ CUtensorMap map_t, co
     pdl_entry_late();
     // This loop runs at 104 registers (96 where the move is left out): the tile is described by its meta entry, shared
     // memory addresses are constants, everything else is derived from three counters.
-    const uint32_t lane_addr = tmem_base + ((uint32_t)((warp & 3) * 32) << 16) + 128 * (warp >> 3) + 32 * ((warp >> 2) & 1);
     const uint32_t my_full = ptx::smem_u32(part_full) + 8 * (warp >> 3);  // the warp's half of the even K blocks
     constexpr uint32_t kToEmpty = 4 * 8;                                   // from part_full to part_empty
     uint32_t step = 0, group = 0;  // K blocks folded so far; factor slots used
     int ltile = 0;
+    int small_tiles = 0;  // of them: the barriers of the two kinds of quantisation group have phases of their own
     bool alive = true;
     long long prof_fw = 0, prof_fb = 0, prof_sw = 0, prof_epi = 0;
-    for (; worker + ltile * workers < total_tiles; ++ltile) {
-      float acc[64];  // 32 columns of the first 128 weight rows (gate), then the same 32 of the second (up)
+    const volatile int32_t* tiles = table + 3 * p.num_experts;
+    for (; worker + ltile * workers < *tiles * p.w_tiles; ++ltile) {
+      // Gate/up: 16 gate channels, the same 16 of up, and 16 further of both; down: 64 channels (M = 128: the first half)
+      float acc[64];
 #pragma unroll
       for (int i = 0; i < 64; ++i) acc[i] = 0.f;
-      bool mine = false;  // some of this warp's lanes hold tokens
+      bool mine = false;   // some of this warp's lanes hold tokens
+      bool small = false;  // M = 128: lanes 0-63 hold this CTA's 64 tokens x CTA 0's weight rows, lanes 64-127 x CTA 1's
+      const int piece = (warp >> 2) & 1;
 #pragma unroll 1
       for (int left = kblocks; left > 0; left -= G::GROUP, ++group) {
         const long long tf0 = PROF ? clock64() : 0;
@@ -1008,40 +1024,49 @@ grouped_gemm_pair_fold_wide_kernel(const __grid_constant__ CUtensorMap map_t, co
           break;
         }
         if (PROF) prof_sw += clock64() - tf0;
-        mine = (warp & 3) * 32 < meta[(ltile % META_TILES) * G::META_WORDS + 257];
-        uint32_t src = ptx::smem_u32(scales) + (group % SC_SLOTS) * G::SLOT_BYTES + ((warp & 3) * 32 + lane) * 4;
+        const int tokens = meta[(ltile % META_TILES) * G::META_WORDS + 257];
+        small = tokens <= 64;
+        mine = (small ? warp & 1 : warp & 3) * 32 < tokens;
+        uint32_t src = ptx::smem_u32(scales) + (group % SC_SLOTS) * G::SLOT_BYTES + ((small ? warp & 1 : warp & 3) * 32 + lane) * 4;
+        if constexpr (!GATED) src += 512 * (small ? (warp >> 1) & 1 : piece);
+        const uint32_t from = *reinterpret_cast<volatile uint32_t*>(tmem_slot) + ((uint32_t)((warp & 3) * 32) << 16) + 128 * (warp >> 3) +
+                              (small ? 32 : 64) * piece;
         const uint32_t end = step + min(left, G::GROUP);
+        // 16 columns at a time keeps the staging registers few (the 64 accumulators stay live)
+        auto fold = [&](auto chunks_c) {
+          constexpr int CHUNKS = decltype(chunks_c)::value;
 #pragma unroll 1
-        for (; step != end; ++step, src += G::KB_BYTES) {
-          const uint32_t odd = step & 1;
-          const long long tf1 = PROF ? clock64() : 0;
-          if (!__all_sync(0xffffffffu, ptx::mbar_wait_addr(my_full + odd * 16, (step >> 1) & 1))) {
-            report(0x700);
-            alive = false;
-            break;
-          }
-          const long long tf2 = PROF ? clock64() : 0;
-          ptx::tc_fence_after_sync();
-          if (mine) {
+          for (; step != end; ++step, src += G::KB_BYTES) {
+            const uint32_t odd = step & 1;
+            const long long tf1 = PROF ? clock64() : 0;
+            if (!__all_sync(0xffffffffu, ptx::mbar_wait_addr(my_full + odd * 16, (step >> 1) & 1))) {
+              report(0x700);
+              alive = false;
+              break;
+            }
+            const long long tf2 = PROF ? clock64() : 0;
+            ptx::tc_fence_after_sync();
 #pragma unroll
-            for (int c = 0; c < 4; ++c) {
-              // 16 columns at a time keeps the staging registers few (the 64 accumulators stay live)
-              const float f = lds32(src + (c >> 1) * 512);
+            for (int c = 0; c < CHUNKS; ++c) {
+              const float f = lds32(src + (GATED ? (c & 1) * 512 : 0));
               uint32_t v[16];
-              ptx::tmem_ld_32x32b_x16(lane_addr + odd * 256 + (c >> 1) * 64 + (c & 1) * 16, v);
+              ptx::tmem_ld_32x32b_x16(from + odd * 256 + c * 16, v);
               ptx::tmem_ld_wait();
 #pragma unroll
               for (int i = 0; i < 16; ++i) acc[16 * c + i] = fmaf(__uint_as_float(v[i]), f, acc[16 * c + i]);
             }
+            ptx::tc_fence_before_sync();
+            __syncwarp();
+            if (ptx::elect_one()) ptx::mbar_arrive_cluster(((my_full + odd * 16) & ~ptx::kPeerRankBit) + kToEmpty);
+            if (PROF) {
+              prof_fw += tf2 - tf1;
+              prof_fb += clock64() - tf2;
+            }
           }
-          ptx::tc_fence_before_sync();
-          __syncwarp();
-          if (ptx::elect_one()) ptx::mbar_arrive_cluster(((my_full + odd * 16) & ~ptx::kPeerRankBit) + kToEmpty);
-          if (PROF) {
-            prof_fw += tf2 - tf1;
-            prof_fb += clock64() - tf2;
-          }
-        }
+        };
+        if (!mine) fold(std::integral_constant<int, 0>{});
+        else if (small) fold(std::integral_constant<int, 2>{});
+        else fold(std::integral_constant<int, 4>{});
         if (!alive) break;
         if (lane == 0) ptx::mbar_arrive(&sc_empty[group % SC_SLOTS]);
       }
@@ -1049,29 +1074,41 @@ grouped_gemm_pair_fold_wide_kernel(const __grid_constant__ CUtensorMap map_t, co
 
       const long long te0 = PROF ? clock64() : 0;
       const int32_t* m = meta + (ltile % META_TILES) * G::META_WORDS;
-      const int32_t slot = m[(warp & 3) * 32 + lane];
-      const float rs = __int_as_float(m[128 + (warp & 3) * 32 + lane]);
-      const int cpart = warp >> 2;
+      const int tok = (small ? warp & 1 : warp & 3) * 32 + lane, half = warp >> 3;
+      const int32_t slot = m[tok];
+      const float rs = __int_as_float(m[128 + tok]);
+      const int side = small ? (warp >> 1) & 1 : piece;  // whose weight rows: CTA 0's or CTA 1's
       if constexpr (GATED) {
-        // output columns w_tile * 128 + 32 cpart + [0,32), in place of the gate accumulators
-        const int64_t at = (int64_t)(m[256] + (warp & 3) * 32 + lane) * p.n + m[258] * 128 + 32 * cpart;
+        // output channels of the tile: 16 or 32 from here, in place of the gate accumulators
+        const int ch = 64 * side + 32 * half + (small ? 16 * piece : 0);
+        const int64_t at = (int64_t)(m[256] + tok) * p.n + m[258] * 128 + ch;
         float amax = 0.f;
 #pragma unroll
-        for (int i = 0; i < 32; ++i) {
-          acc[i] = act_mul_fast(acc[i] * rs, acc[32 + i] * rs, p.activation);
-          amax = fmaxf(amax, fabsf(acc[i]));
+        for (int h = 0; h < 2; ++h) {
+          if (h == 1 && small) break;
+#pragma unroll
+          for (int i = 0; i < 16; ++i) {
+            acc[32 * h + i] = act_mul_fast(acc[32 * h + i] * rs, acc[32 * h + 16 + i] * rs, p.activation);
+            amax = fmaxf(amax, fabsf(acc[32 * h + i]));
+          }
         }
         if (p.out_dtype == FMOE_E4M3) {
-          // the tile's 128 channels are one quantisation group, held by four warps
-          float* am = amax_buf + (ltile & 1) * 512 + (warp & 3) * 32 + lane;
-          am[cpart * 128] = amax;
+          // the tile's 128 channels are one quantisation group, held by four warps (M = 128: by eight)
+          const int part = (small ? 4 * side : 0) + 2 * half + piece;
+          float* am = amax_buf + (small ? 1024 + (small_tiles & 1) * 512 : ((ltile - small_tiles) & 1) * 512) + tok;
+          const int pitch = small ? 64 : 128;
+          uint64_t* bar = small ? &small_bar[warp & 1] : &amax_bar[warp & 3];
+          am[part * pitch] = amax;
           __syncwarp();
-          if (lane == 0) ptx::mbar_arrive(&amax_bar[warp & 3]);
-          if (!warp_wait(&amax_bar[warp & 3], ltile & 1)) {
+          if (lane == 0) ptx::mbar_arrive(bar);
+          if (!warp_wait(bar, (small ? small_tiles : ltile - small_tiles) & 1)) {
             report(0x7c0);
             break;
           }
-          amax = fmaxf(fmaxf(am[0], am[128]), fmaxf(am[256], am[384]));
+#pragma unroll
+          for (int j = 0; j < 8; ++j)
+            if (j < 4 || small) amax = fmaxf(amax, am[j * pitch]);
+          small_tiles += small;
           if (mine && slot >= 0) {
             const float s = group_scale(amax), r = __frcp_rn(s);
             uint32_t w[8];
@@ -1079,31 +1116,40 @@ grouped_gemm_pair_fold_wide_kernel(const __grid_constant__ CUtensorMap map_t, co
             for (int u = 0; u < 4; ++u) {
               float v[8];
 #pragma unroll
-              for (int i = 0; i < 8; ++i) v[i] = acc[8 * u + i];
+              for (int i = 0; i < 8; ++i) v[i] = acc[32 * (u >> 1) + 8 * (u & 1) + i];
               const uint2 q = quant8(v, s, r, amax <= 3.0e38f);
               w[2 * u] = q.x;
               w[2 * u + 1] = q.y;
             }
-            store_32_bytes(reinterpret_cast<uint8_t*>(p.out) + at, w, p.stores_of_32);
-            if (cpart == 0) p.out_scale[at >> 7] = s;  // n is a multiple of 128
+            uint8_t* dst = reinterpret_cast<uint8_t*>(p.out) + at;
+            if (small) *reinterpret_cast<uint4*>(dst) = make_uint4(w[0], w[1], w[2], w[3]);
+            else store_32_bytes(dst, w, p.stores_of_32);
+            if (part == 0) p.out_scale[at >> 7] = s;  // n is a multiple of 128
           }
         } else if (mine && slot >= 0) {
-          if (p.out_dtype == FMOE_F32) {
-            float4* dst = reinterpret_cast<float4*>(reinterpret_cast<float*>(p.out) + at);
 #pragma unroll
-            for (int v = 0; v < 8; ++v) dst[v] = make_float4(acc[4 * v], acc[4 * v + 1], acc[4 * v + 2], acc[4 * v + 3]);
-          } else {
-            store32(reinterpret_cast<__nv_bfloat16*>(p.out) + at, acc, 1.0f, p.stores_of_32);
+          for (int h = 0; h < 2; ++h) {
+            if (h == 1 && small) break;
+            if (p.out_dtype == FMOE_F32) {
+              float4* dst = reinterpret_cast<float4*>(reinterpret_cast<float*>(p.out) + at + 16 * h);
+#pragma unroll
+              for (int v = 0; v < 4; ++v)
+                dst[v] = make_float4(acc[32 * h + 4 * v], acc[32 * h + 4 * v + 1], acc[32 * h + 4 * v + 2], acc[32 * h + 4 * v + 3]);
+            } else {
+              store16(reinterpret_cast<__nv_bfloat16*>(p.out) + at + 16 * h, &acc[32 * h], 1.0f, p.stores_of_32);
+            }
           }
         }
       } else if (mine && slot >= 0) {
-        // columns w_tile * 256 + 32 cpart + [0,32), and the same 128 further
         __nv_bfloat16* obase = p.out_rows ? reinterpret_cast<__nv_bfloat16*>(p.out_rows[slot])
                                           : reinterpret_cast<__nv_bfloat16*>(p.out) + (int64_t)slot * p.n;
+        const int64_t colg = (int64_t)m[258] * 256 + 128 * side + 64 * half + (small ? 32 * piece : 0);
+        if (obase && colg < p.n) {
 #pragma unroll
-        for (int h = 0; h < 2; ++h) {
-          const int64_t colg = (int64_t)m[258] * 256 + 128 * h + 32 * cpart;
-          if (obase && colg < p.n) store32(obase + colg, &acc[32 * h], rs, p.stores_of_32);
+          for (int c = 0; c < 4; ++c) {
+            if (c >= 2 && small) break;
+            store16(obase + colg + 16 * c, &acc[16 * c], rs, p.stores_of_32);
+          }
         }
       }
       if (PROF) prof_epi += clock64() - te0;
@@ -1156,8 +1202,7 @@ int launch(const GemmParams& g, int min_rows, int max_rows, cudaStream_t st) {
   CUtensorMap map_t, map_w;
   int rc = pair_map_tokens(&map_t, g.a, g.a_rows, g.k, 1, BOX_TOKENS);
   if (rc) return rc;
-  // wide: gate and up rows are whole boxes of 128 of one [w_rows, K] matrix per expert
-  rc = pair_map_weights(&map_w, g.w, g.num_experts, WIDE ? w_rows : g.n, g.k, 1, GATED && !WIDE);
+  rc = pair_map_weights(&map_w, g.w, g.num_experts, g.n, g.k, 1, GATED);
   if (rc) return rc;
   FoldParams p;
   p.sorted_token_ids = g.sorted_token_ids;

@@ -27,8 +27,8 @@ constexpr int kSplitCounters = 512;
 __host__ __device__ constexpr int pair_table_words(int num_experts) { return 3 * num_experts + 1; }
 __host__ __device__ constexpr int pair_table_bytes(int num_experts) { return (pair_table_words(num_experts) * 4 + 15) & ~15; }
 // The e4m3 block-scale GEMMs (gemm_pair_fold.cu): experts with up to kNarrowRows rows go to the narrow kernel (one 64-token
-// tile: 0.36 us per K block and tile), the others to the wide one (256 tokens: 0.65 us).  A call whose experts have few rows
-// on average is left to the narrow kernel alone: the wide one would find next to nothing.
+// tile: 0.45 us per K block and tile, 0.36 with 16 rows), the others to the wide one (up to 128 tokens 0.50 us, 256 0.66 us).
+// A call whose experts have few rows on average is left to the narrow kernel alone: the wide one would find next to nothing.
 constexpr int kNarrowRows = 64;
 inline bool fold_narrow_only(int64_t numel, int num_experts) {
   return numel <= 16 * (numel < num_experts ? numel : (int64_t)num_experts);
@@ -121,7 +121,9 @@ struct PairTile {
 
 // Tile order: expert by expert, inside an expert in groups of at most `group` token tiles, inside a group the token tile
 // varies fastest: the tiles that run at the same time share weight rows through L2, and the group's token rows stay hot.
-__device__ __forceinline__ PairTile pair_locate(int64_t tile, int w_tiles, int group, int num_experts, const int32_t* table) {
+// Tokens per tile: the expert's in equal tiles, or, given a fixed number, as many per tile and the rest in the last.
+__device__ __forceinline__ PairTile pair_locate(int64_t tile, int w_tiles, int group, int num_experts, const int32_t* table,
+                                                int fixed = 0) {
   const int32_t* prefix = table + 2 * num_experts;
   const int q = (int)(tile / w_tiles);
   int expert = 0, hi = num_experts - 1;  // last expert whose prefix is <= q (one with tiles, as q < prefix[E])
@@ -136,8 +138,10 @@ __device__ __forceinline__ PairTile pair_locate(int64_t tile, int w_tiles, int g
   const int64_t per_group = (int64_t)group * w_tiles;
   const int g = (int)(local / per_group), r = (int)(local % per_group);
   const int in_group = min(group, tiles - g * group);
-  const int t = g * group + r % in_group;
-  const int step = (((rows + tiles - 1) / tiles) + 15) & ~15;  // the expert's tokens in equal tiles
+  // where the last tile is a short one, the order changes from weight tile to weight tile: an even number of workers would
+  // deal all short ones to half of them
+  const int t = g * group + (fixed ? (r + r / in_group) % in_group : r % in_group);
+  const int step = fixed ? fixed : (((rows + tiles - 1) / tiles) + 15) & ~15;
   PairTile tl;
   tl.w_tile = r / in_group;
   tl.row0 = table[expert] + t * step;
@@ -298,7 +302,7 @@ struct PairList {
   }
   // A whole warp adds a batch.  1: there are more, 0: the list ends in it, -1: time-out.
   static __device__ __forceinline__ int fill(int4* units, uint64_t* bars, int batch, const UnitPlan& plan, int w_tiles, int group,
-                                             int num_experts, const int32_t* table) {
+                                             int num_experts, const int32_t* table, int fixed = 0) {
     const int slot = batch & 1, lane = threadIdx.x & 31;
     if (batch >= 2 && !__all_sync(0xffffffffu, ptx::mbar_wait_relaxed(&bars[2 + slot], ((batch >> 1) & 1) ^ 1))) return -1;
     int64_t tile;
@@ -308,7 +312,7 @@ struct PairList {
     const bool any = plan.get(it, &tile, &ks0, &ks1, &u.slice);
     int4 d = make_int4(0, 0, 0, 0);
     if (any) {
-      u.tl = pair_locate(tile, w_tiles, group, num_experts, table);
+      u.tl = pair_locate(tile, w_tiles, group, num_experts, table, fixed);
       u.log2_s = plan.is_split(it) ? 31 - __clz(plan.S) : 0;
       d = u.pack();
     }

@@ -129,6 +129,21 @@ def test_wide_e4m3_kernel_stores_to_rows_at_16_bytes(fg, gated):
     assert torch.equal(outs[0], outs[1]) and torch.equal(outs[0], outs[2])
 
 
+@pytest.mark.parametrize("H,I", [(128, 256), (256, 128)])
+def test_wide_e4m3_kernel_mixes_tile_heights(fg, H, I):
+    """Block-scale layers whose experts end in tiles of M = 128 and of M = 256, one and two K blocks long: the warps that share a
+    quantisation group change from tile to tile, and a tile is over before the slowest warp has left the one before."""
+    rows = [300, 65, 129, 256, 400, 128, 257, 640, 70, 512, 0, 384] * 3
+    E, T = len(rows), sum(rows)
+    x, w1, w2, g = _layer(T, H, I, E, 11)
+    ids = torch.repeat_interleave(torch.arange(E), torch.tensor(rows))[torch.randperm(T, generator=g)].to(torch.int32).view(T, 1)
+    tw = torch.rand(T, 1, generator=g) + 0.5
+    (w1q, w1s), (w2q, w2s) = OQ.quant_weight_block128(w1), OQ.quant_weight_block128(w2)
+    out = fg.fused_experts(x.cuda(), w1q.cuda(), w2q.cuda(), tw.cuda(), ids.cuda(), use_fp8_w8a8=True, w1_scale=w1s.cuda(),
+                           w2_scale=w2s.cuda(), block_shape=[128, 128])
+    assert_close_moe(out, OE.fused_experts_fp8(x, w1q, w1s, w2q, w2s, tw, ids), "fp8", f"H={H} I={I}")
+
+
 def test_e4m3_kernels_without_the_register_move(tmp_path):
     """The e4m3 block-scale kernels as they are launched where the compiler left too few registers for setmaxnreg: same sums
     in the same order, so the same bits."""
