@@ -61,23 +61,23 @@ inline int64_t up256(int64_t v) { return (v + 255) & ~int64_t(255); }
 }
 
 // The whole layer on the CTA-pair GEMMs although an expert has few rows.  Both families read the weights once; the pair
-// kernels stream them up to 15 % faster but cost a row copy and a longer prologue, 5-15 us.  Measured per layer, stream / pairs
-// in us:
-//   e4m3            DeepSeek-V3 9 tokens 510 / 447, 64 tokens 1203 / 1031, a rank's eighth with 9 to 16 tokens 262 / 243
-//   not x128        (the streaming kernel masks its loads) GPT-OSS 9 tokens 257 / 220, half of it 135 / 126
-//   0.6-0.7 GB      half of Qwen3, 64 tokens 119 / 134; a quarter of Mixtral, 12 tokens 117 / 122
-//   1.2 GB and more, 3 rows and more: Qwen3 64 tokens 212 / 207, reference shape 24 tokens 248 / 243, 64 experts of 2560 x 2048
-//                   313 / 313, 16 of 4096 x 6144 385 / 351, Mixtral 12 tokens 467 / 438
-//   1.2 GB and more, below: H or I of 4096 and more (the streaming kernel cuts its K loop between 8 warps) 8 experts of 4096 x
-//                   6144 200 / 191, x 9216 311 / 291, Mixtral 459 / 436, 16 of 4096 x 4096 266 / 253, 32 of 2048 x 4096
-//                   215 / 207, 8 of 2048 x 12288 181 / 182; smaller 64 of 2048 x 2048 228 / 237, of 3072 x 2304 369 / 371,
-//                   32 of 3072 x 3072 229 / 236, Qwen3 191 / 191, 128 of 2048 x 1536 277 / 278 and 329 / 324
+// kernels stream them up to 15 % faster but cost a row copy, a launch more and a longer prologue, 3-5 us.  Measured per layer,
+// stream / pairs in us:
+//   e4m3        DeepSeek-V3 9 tokens 510 / 447, 64 tokens 1203 / 1031, a rank's eighth with 9 to 16 tokens 262 / 243
+//   not x128    (the streaming kernel masks its loads) GPT-OSS 9 tokens 232 / 183, 64 tokens 363 / 253
+//   0.3 GB and more of weights (of as many experts as there are slots), 3 rows and more per expert
+//               Qwen3 48 tokens 202 / 190, half of it 116 / 110; reference shape 24 tokens 248 / 233, half of it 140 / 131, a
+//               quarter 87 / 79; Mixtral 12 tokens 473 / 426, a quarter 137 / 126
+//   1.2 GB and more, fewer rows: H or I of 4096 and more (the streaming kernel cuts its K loop between 8 warps): 8 experts of
+//               4096 x 6144 200 / 191, x 9216 311 / 291, Mixtral 431 / 388
+//   0.2 GB      128 experts of 2048 x 128, 64 tokens 58 / 63; 16 of 2048 x 1024 24 tokens 50 / 52
+//   below       (launches count) 32 of 1024 x 512, 24 tokens 31 / 34; 8 of 1024 x 1024 33 / 33
 bool layer_prefers_pairs(const fmoe_fused_args& a, int64_t numel) {
   if (a.dtype == FMOE_E4M3) return true;  // sizes are multiples of 128
   if (a.H % 32 || a.I % 32) return false;
   if (a.H % 128 || a.I % 128) return true;
   const int64_t active = std::min<int64_t>(a.num_experts, numel), bytes = active * 6 * a.H * a.I;
-  return bytes >= 1200000000ll && (numel >= 3 * active || std::max(a.H, a.I) >= 4096);
+  return numel >= 3 * active ? bytes >= 300000000ll : bytes >= 1200000000ll && std::max(a.H, a.I) >= 4096;
 }
 
 int plan_fused(const fmoe_fused_args& a, const RouteArgs& route, FusedPlan* pl) {

@@ -54,13 +54,20 @@ extern "C" int fmoe_fused_experts_static(const fmoe_fused_args* args, void* stre
   if (rc) return rc;
   fmoe_fused_args a = *args;
   if (plan.total > kStaticScratchBytes && a.variant == FMOE_VARIANT_AUTO) {
-    // the streaming kernels need no padded copies: with few rows per expert their plan may fit where the faster one does not
+    // The decode and the streaming kernels need no padded copies: with few rows per expert their plans may fit where the faster
+    // one does not.
+    RouteArgs small;
+    small.small_scratch = true;
     int variant = 0, block = 0;
-    FusedPlan streamed;
-    a.variant = FMOE_VARIANT_STREAM;
-    if (pick_variant(a.dtype, a.T * a.top_k, a.num_experts, a.I, a.H, FMOE_VARIANT_STREAM, &variant, &block) == FMOE_OK &&
-        plan_fused(a, RouteArgs{}, &streamed) == FMOE_OK && streamed.total <= kStaticScratchBytes)
-      plan = streamed;
+    FusedPlan other;
+    if (plan_fused(a, small, &other) == FMOE_OK && other.use_decode && other.total <= kStaticScratchBytes) {
+      plan = other;
+    } else {
+      a.variant = FMOE_VARIANT_STREAM;
+      if (pick_variant(a.dtype, a.T * a.top_k, a.num_experts, a.I, a.H, FMOE_VARIANT_STREAM, &variant, &block) == FMOE_OK &&
+          plan_fused(a, RouteArgs{}, &other) == FMOE_OK && other.total <= kStaticScratchBytes)
+        plan = other;
+    }
   }
   if (plan.total > kStaticScratchBytes)
     return fail(FMOE_ERR_UNSUPPORTED,

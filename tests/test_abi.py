@@ -83,6 +83,18 @@ def test_layer_variant_is_what_the_one_call_layer_takes(lib, dtype, T, E, H, I, 
         assert name == want and block == {"decode": 0, "stream": 8, "tcgen05": 128, "simt": 16}[want]
 
 
+@pytest.mark.parametrize("dtype,T,E,H,I,k,want", [
+    # 3 rows per expert from 0.3 GB of weights on
+    ("BF16", 48, 128, 2048, 384, 8, "tcgen05"), ("BF16", 47, 128, 2048, 384, 8, "stream"), ("BF16", 24, 64, 1280, 768, 8, "tcgen05"),
+    ("BF16", 24, 16, 2048, 1024, 2, "stream"),
+    # e4m3 tokens times row length, by the length of the down rows
+    ("E4M3", 3, 256, 7168, 1024, 8, "decode"), ("E4M3", 4, 256, 7168, 1024, 8, "tcgen05"), ("E4M3", 3, 256, 7168, 512, 8, "decode"),
+    ("E4M3", 4, 256, 7168, 512, 8, "tcgen05"), ("E4M3", 2, 256, 7168, 256, 8, "decode"), ("E4M3", 3, 256, 7168, 256, 8, "tcgen05"),
+    ("E4M3", 6, 64, 4096, 1536, 6, "decode"), ("E4M3", 7, 64, 4096, 1536, 6, "tcgen05"), ("E4M3", 8, 128, 2048, 384, 8, "decode")])
+def test_layer_variant_on_both_sides_of_its_lines(lib, dtype, T, E, H, I, k, want):
+    test_layer_variant_is_what_the_one_call_layer_takes(lib, dtype, T, E, H, I, k, want)
+
+
 @pytest.mark.parametrize("stray", ["logits", "bias"])
 def test_one_call_moe_refuses_a_router_input_on_another_device(monkeypatch, stray):
     """The router's inputs go into the library call as plain pointers: they have to be on the layer's device (devices are

@@ -442,6 +442,42 @@ def test_combine_slot_counts(fg, k):
         assert torch.equal(out.cpu(), OE.moe_sum(z.to(dt)).to(dt))
 
 
+@pytest.mark.parametrize("T", [2, 3, 8])
+def test_e4m3_layer_around_the_decode_line(fg, T):
+    """Short down rows: two tokens take the decode kernels, three the CTA-pair GEMMs, in every form of the call.  Eight need more
+    than the allocation-free entry holds for the pairs: it keeps the decode kernels."""
+    from flaggems_sglang_b200 import _C
+
+    E, H, I, k = 64, 7168, 256, 8
+    x, w1, w2, g = _layer(T, H, I, E, 30 + T)
+    logits = torch.randn(T, E, generator=g)
+    tw, ids = OR.softmax_topk(logits, k, True)
+    (w1q, s1), (w2q, s2) = OQ.quant_weight_block128(w1), OQ.quant_weight_block128(w2)
+    d = [x.cuda(), w1q.cuda(), w2q.cuda()]
+    s1d, s2d = s1.cuda(), s2.cuda()
+    kw = dict(use_fp8_w8a8=True, w1_scale=s1d, w2_scale=s2d, block_shape=[128, 128])
+    ref = OE.fused_experts_fp8(x, w1q, s1, w2q, s2, tw, ids)
+    twd, idd = tw.cuda(), ids.cuda()
+    assert_close_moe(fg.fused_experts(*d, twd, idd, **kw), ref, "fp8", f"T={T}")
+    assert_close_moe(fg.fused_moe(*d, logits.cuda(), k, True, routed_scaling_factor=1.5, **kw), ref.float() * 1.5, "fp8", f"T={T} router")
+    rows = fg.fused_experts(*d, twd, idd, no_combine=True, **kw)
+    assert_close_moe(rows.float().sum(1), ref, "fp8", f"T={T} rows")
+    first = [fg.fused_experts(*d, twd, idd, apply_router_weight_on_input=True, variant=v, **kw) for v in (None, "stream")]
+    assert_close_moe(first[0], first[1].cpu(), "fp8", f"T={T} weight first")
+    local = torch.arange(E, dtype=torch.int32)
+    local[::2] = -1
+    kept = OE.fused_experts_fp8(x, w1q, s1, w2q, s2, torch.where(ids % 2 == 1, tw, torch.zeros(())), ids)
+    assert_close_moe(fg.fused_experts(*d, twd, idd, expert_map=local.cuda(), **kw), kept, "fp8", f"T={T} expert map")
+    out = torch.empty(T, H, dtype=torch.bfloat16, device="cuda")
+    a = _C.FusedArgs(dtype=_C.E4M3, num_experts=E, top_k=k, T=T, H=H, I=I, routed_scaling_factor=1.0, hidden=d[0].data_ptr(),
+                     w1=d[1].data_ptr(), w2=d[2].data_ptr(), w1_scale=s1d.data_ptr(), w2_scale=s2d.data_ptr(),
+                     topk_weights=twd.data_ptr(), topk_ids=idd.data_ptr(), out=out.data_ptr())
+    lib = _C.lib()
+    assert (lib.fmoe_fused_experts_workspace_bytes(a) > lib.fmoe_static_scratch_bytes()) == (T == 8)
+    _C.check(lib.fmoe_fused_experts_static(a, _C.stream_ptr()))
+    assert_close_moe(out, ref, "fp8", f"T={T} static")
+
+
 def test_static_entry_streams_what_does_not_fit(fg):
     """e4m3 layers with few rows per expert take the padded tensor-core plan; the allocation-free entry keeps the streaming
     one where only that fits its array."""
