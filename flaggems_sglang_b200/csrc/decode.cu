@@ -84,7 +84,8 @@ struct PrepareParams {
   int64_t H;
 };
 
-constexpr int kPrepThreads = 512;
+constexpr int kPrepThreads = 256;  // one per slot, of which there are at most kMaxBlocks; 8 warps route 8 tokens
+static_assert(kPrepThreads >= kMaxBlocks, "one thread per slot");
 
 template <int VPT>
 __global__ void __launch_bounds__(kPrepThreads)
@@ -117,12 +118,9 @@ decode_prepare_kernel(const PrepareParams p) {
   }
   extern __shared__ float s_dyn[];  // grouped: per token score[E], choice[E]
   __shared__ int s_sel[kDecodeTokens][32];
-  __shared__ int s_cnt[1024];
-  __shared__ int s_block[1024];
-  __shared__ int s_ids[kMaxBlocks];
+  __shared__ int s_ids[kMaxBlocks], s_quot[kMaxBlocks], s_rem[kMaxBlocks];
   const int numel = p.T * p.k;
   for (int i = tid; i < p.num_counters; i += kPrepThreads) p.counters[i] = 0;
-  for (int e = tid; e < p.E; e += kPrepThreads) s_cnt[e] = 0;
   if (p.logits) {
     if (p.grouped) {
       for (int i = tid; i < p.T * p.E; i += kPrepThreads) {
@@ -146,41 +144,35 @@ decode_prepare_kernel(const PrepareParams p) {
     for (int i = tid; i < numel; i += kPrepThreads) s_ids[i] = p.ids_in[i];
   }
   __syncthreads();
-  for (int i = tid; i < numel; i += kPrepThreads) {
-    const int e = s_ids[i];
-    if (e >= 0 && e < p.E) atomicAdd(&s_cnt[e], 1);
-  }
-  __syncthreads();
-  // blocks of at most T rows of one expert, experts ascending (one block per active expert, unless the caller's ids name
-  // an expert twice for a token)
-  if (warp == 0) {
-    int run = 0;
-    for (int base = 0; base < p.E; base += 32) {
-      const int e = base + lane;
-      const int n = e < p.E ? (s_cnt[e] + p.T - 1) / p.T : 0;
-      int incl = n;
-#pragma unroll
-      for (int off = 1; off < 32; off <<= 1) {
-        const int v = __shfl_up_sync(0xffffffffu, incl, off);
-        if (lane >= off) incl += v;
-      }
-      if (n > 0) s_block[e] = run + incl - n;
-      for (int i = 0; i < n; ++i) {
-        const int b = run + incl - n + i;
-        p.plan[plan_expert(b)] = e;
-        p.plan[plan_rows(b)] = min(s_cnt[e] - i * p.T, p.T);
-      }
-      run += __shfl_sync(0xffffffffu, incl, 31);
+  // Blocks of at most T rows of one expert, experts ascending (one block per active expert, unless the caller's ids name
+  // an expert twice for a token).  A thread per slot counts: its place among its expert's slots, then the blocks before its own.
+  // (Counting by expert and a prefix sum over all of them is a chain of 8 x 5 shuffles for 256.)
+  int e = -1, quot = 0, rem = -1;  // block of the expert, row in it
+  if (tid < numel) {
+    e = s_ids[tid];
+    int before = 0;
+    for (int j = 0; j < tid; ++j) before += s_ids[j] == e;
+    if (e >= 0 && e < p.E) {
+      quot = before / p.T;
+      rem = before - quot * p.T;
     }
-    if (lane == 0) p.plan[0] = run;
+    s_quot[tid] = quot;
+    s_rem[tid] = rem;
   }
-  __syncthreads();
-  for (int i = tid; i < numel; i += kPrepThreads) {
-    const int e = s_ids[i];
-    if (e < 0 || e >= p.E) continue;
-    int rank = 0;
-    for (int j = 0; j < i; ++j) rank += s_ids[j] == e;
-    p.plan[plan_slot(s_block[e] + rank / p.T, rank % p.T)] = i;
+  const int blocks = __syncthreads_count(rem == 0);
+  if (tid == 0) p.plan[0] = blocks;
+  if (rem >= 0) {
+    int block = 0, rows = 0;
+    for (int j = 0; j < numel; ++j) {
+      const int ej = s_ids[j], qj = s_quot[j], rj = s_rem[j];
+      block += rj == 0 && (ej < e || (ej == e && qj < quot));
+      rows += rj >= 0 && ej == e && qj == quot;
+    }
+    p.plan[plan_slot(block, rem)] = tid;
+    if (rem == 0) {
+      p.plan[plan_expert(block)] = e;
+      p.plan[plan_rows(block)] = rows;
+    }
   }
 }
 

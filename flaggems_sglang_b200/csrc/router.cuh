@@ -127,23 +127,29 @@ __device__ __forceinline__ void route_grouped(const float* s_score, const float*
     int e = lane + 32 * i;
     key[i] = (e < E) ? s_choice[e] : kNegInf;
   }
-  // group score: sum of the two largest choices of the group (lane g scans group g)
+  // group score: sum of the two largest choices of the group.  The warp's lanes are shared out among the groups, as many to
+  // each as the next power of two allows, and meet by shuffles (one lane per group: 32 dependent steps for 8 groups of 32).
   const int gsz = E / n_group;
-  float gscore = kNegInf;
-  if (lane < n_group) {
-    float m1 = kNegInf, m2 = kNegInf;
-    for (int i = 0; i < gsz; ++i) {
-      float c = s_choice[lane * gsz + ((i + lane) % gsz)];  // rotate start: spreads banks
-      if (c > m1) {
-        m2 = m1;
-        m1 = c;
-      } else if (c > m2) {
-        m2 = c;
-      }
+  int per = 1;
+  while (2 * per * n_group <= 32) per *= 2;
+  const int group = lane / per;
+  float m1 = kNegInf, m2 = kNegInf;
+  if (group < n_group) {
+    for (int i = lane % per; i < gsz; i += per) {
+      const float c = s_choice[group * gsz + i];
+      m2 = fmaxf(m2, fminf(m1, c));
+      m1 = fmaxf(m1, c);
     }
-    gscore = (gsz >= 2) ? (m1 + m2) : m1;
-    if (gscore != gscore) gscore = kNegInf;  // +inf + -inf
   }
+  for (int off = per >> 1; off > 0; off >>= 1) {
+    const float o1 = __shfl_xor_sync(0xffffffffu, m1, off), o2 = __shfl_xor_sync(0xffffffffu, m2, off);
+    m2 = fmaxf(fminf(m1, o1), fmaxf(m2, o2));
+    m1 = fmaxf(m1, o1);
+  }
+  float gscore = (gsz >= 2) ? (m1 + m2) : m1;
+  if (gscore != gscore) gscore = kNegInf;  // +inf + -inf
+  gscore = __shfl_sync(0xffffffffu, gscore, min(lane, n_group - 1) * per);  // lane g: group g
+  if (lane >= n_group) gscore = kNegInf;
   // keep the topk_group best groups (ties -> lower group index)
   uint32_t keep = 0;
   for (int j = 0; j < topk_group; ++j) {
