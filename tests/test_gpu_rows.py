@@ -4,6 +4,8 @@ import torch
 
 from oracle import experts as OE
 from oracle import quant as OQ
+from oracle import routing as OR
+from tests.util import assert_close_moe
 
 pytestmark = pytest.mark.gpu
 
@@ -93,6 +95,25 @@ def test_moe_sum_bit_exact(fg, T, k, H, dtype, scale):
     if scale is not None:
         ref = (ref.float() * scale).to(dtype)
     assert torch.equal(out.cpu(), ref)
+
+
+@pytest.mark.parametrize("k", [1, 3, 4, 5, 7, 8, 9, 17])
+def test_moe_sum_at_the_edges_of_its_rounds_of_slots(fg, k):
+    test_moe_sum_bit_exact(fg, 19, k, 264, torch.bfloat16, None)
+
+
+@pytest.mark.parametrize("H", [256, 4352])
+def test_per_channel_layer_with_more_slots_than_fetched_ahead(fg, H):
+    """Ten slots per token: the scatter of a quantised row fetches eight positions ahead and looks the others up."""
+    T, E, I, k = 23, 12, 128, 10
+    g = torch.Generator().manual_seed(H)
+    x = torch.randn(T, H, generator=g).to(torch.bfloat16)
+    (w1, s1), (w2, s2) = (OQ.quant_weight_per_channel((torch.randn(E, *s, generator=g) * s[1] ** -0.5).to(torch.bfloat16))
+                          for s in ((2 * I, H), (H, I)))
+    tw, ids = OR.softmax_topk(torch.randn(T, E, generator=g), k, True)
+    out = fg.fused_experts(x.cuda(), w1.cuda(), w2.cuda(), tw.cuda(), ids.cuda(), use_fp8_w8a8=True, per_channel_quant=True,
+                           w1_scale=s1.cuda(), w2_scale=s2.cuda())
+    assert_close_moe(out, OE.fused_experts_fp8_per_channel(x, w1, s1, w2, s2, tw, ids), "fp8", f"H={H}")
 
 
 @pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
