@@ -28,8 +28,6 @@ __device__ __forceinline__ int64_t mapped_row(const int32_t* row_map, int map_di
 // inside the loop.
 // With `pos` (position of every slot in the expert-sorted order) the layer walks what is there instead of the padded order,
 // most of which is padding when experts have few rows:
-//   RowMode::kScatter : row p is token p, read and quantised once and stored at the positions of its map_div slots; its
-//                       scales stay by token (the GEMM looks them up)
 //   RowMode::kInPlace : row p is slot p; the row at its position is quantised into the same position
 //   RowMode::kExpert  : blockIdx.y is an expert, its rows start at map_div times that and go to its positions; experts with
 //                       more than map_div rows are left out.  `pos` is the expert table (first row [E], rows [E], ..)
@@ -44,7 +42,6 @@ quant_group128_kernel(const InT* __restrict__ x, int64_t rows_out, int64_t K, co
   else pdl_entry_late();
   constexpr int kIlp = 4;
   const int sub = threadIdx.x & 15;  // lane inside the 16-lane team
-  const unsigned hmask = (threadIdx.x & 16) ? 0xffff0000u : 0x0000ffffu;
   const int groups = (int)(K / 128);
   int64_t limit = num_rows_dev ? min((int64_t)*num_rows_dev, rows_out) : rows_out;
   int64_t base = 0;
@@ -59,7 +56,7 @@ quant_group128_kernel(const InT* __restrict__ x, int64_t rows_out, int64_t K, co
   const int step_g = (int)(teams % groups);
   int64_t p = team / groups;  // item of this team: (row p, group g); the next one is `teams` items further
   int g = (int)(team % groups);
-  while (p < limit) {
+  while (__any_sync(0xffffffffu, p < limit)) {  // the warp stays together: shuffles of half a warp each take their own turn
     float v[kIlp][8];
     int64_t pu[kIlp];
     int gu[kIlp];
@@ -72,8 +69,8 @@ quant_group128_kernel(const InT* __restrict__ x, int64_t rows_out, int64_t K, co
 #pragma unroll
       for (int i = 0; i < 8; ++i) v[u][i] = 0.f;
       if (p < limit) {
-        const int64_t r = MODE == RowMode::kScatter ? p : (MODE == RowMode::kExpert ? (int64_t)blockIdx.y * map_div + p
-                          : (MODE == RowMode::kInPlace ? pos[p] : mapped_row(row_map, map_div, sentinel, p)));
+        const int64_t r = MODE == RowMode::kExpert ? (int64_t)blockIdx.y * map_div + p
+                          : (MODE == RowMode::kInPlace ? pos[p] : mapped_row(row_map, map_div, sentinel, p));
         if constexpr (MODE == RowMode::kExpert) pu[u] = base + p;
         if constexpr (MODE == RowMode::kInPlace) pu[u] = r;
         real[u] = r >= 0;
@@ -108,13 +105,13 @@ quant_group128_kernel(const InT* __restrict__ x, int64_t rows_out, int64_t K, co
 #pragma unroll
       for (int i = 0; i < 8; ++i) amax = fmaxf(amax, fabsf(v[u][i]));
 #pragma unroll
-      for (int off = 8; off > 0; off >>= 1) amax = fmaxf(amax, __shfl_xor_sync(hmask, amax, off));
+      for (int off = 8; off > 0; off >>= 1) amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, off));
       if constexpr (MODE != RowMode::kMap) {
         if (!real[u]) continue;
       } else if (pu[u] >= limit) {  // uniform over the 16 lanes of the team
         continue;
       }
-      [[maybe_unused]] uint2* dst = reinterpret_cast<uint2*>(q + pu[u] * K + (int64_t)gu[u] * 128 + sub * 8);
+      uint2* dst = reinterpret_cast<uint2*>(q + pu[u] * K + (int64_t)gu[u] * 128 + sub * 8);
       if (!real[u]) {  // padding position: zeros with a unit scale
         *dst = make_uint2(0, 0);
         if (sub == 0) scale[pu[u] * groups + gu[u]] = 1.0f;
@@ -122,13 +119,71 @@ quant_group128_kernel(const InT* __restrict__ x, int64_t rows_out, int64_t K, co
       }
       const float s = group_scale(amax);
       const uint2 bytes = quant8(v[u], s, __frcp_rn(s), amax <= 3.0e38f);
-      if constexpr (MODE == RowMode::kScatter) {
-        for (int j = 0; j < map_div; ++j) {
-          const int32_t to = pos[pu[u] * map_div + j];
-          if (to >= 0) *reinterpret_cast<uint2*>(q + (int64_t)to * K + (int64_t)gu[u] * 128 + sub * 8) = bytes;
+      *dst = bytes;
+      if (sub == 0) scale[pu[u] * groups + gu[u]] = s;
+    }
+  }
+}
+
+// Token rows quantised once and stored at the positions of their k slots, scales by token.  Eight lanes own a group of 128
+// channels, 32 bytes each, and store 16: most of what this kernel does is storing, and its stores bound it (sixteen lanes and
+// 8-byte stores, shuffles by half warps: DeepSeek-V3, 4096 tokens, 70 us; this one 47 us).
+__global__ void __launch_bounds__(256)
+quant_scatter128_kernel(const __nv_bfloat16* __restrict__ x, int64_t T, int64_t K, int k, const int32_t* __restrict__ pos,
+                        uint8_t* __restrict__ q, float* __restrict__ scale) {
+  pdl_entry_late();
+  constexpr int kIlp = 2;
+  const int sub = threadIdx.x & 7;
+  const int groups = (int)(K / 128);
+  const int64_t teams = (int64_t)gridDim.x * 32, team = (int64_t)blockIdx.x * 32 + (threadIdx.x >> 3);
+  const int64_t step_p = teams / groups;
+  const int step_g = (int)(teams % groups);
+  int64_t p = team / groups;  // item of this team: (token p, group g); the next one is `teams` items further
+  int g = (int)(team % groups);
+  while (__any_sync(0xffffffffu, p < T)) {  // the warp stays together for its shuffles
+    uint4 raw[kIlp][2];
+    int64_t pu[kIlp];
+    int gu[kIlp];
+#pragma unroll
+    for (int u = 0; u < kIlp; ++u) {
+      pu[u] = p;
+      gu[u] = g;
+      raw[u][0] = raw[u][1] = make_uint4(0, 0, 0, 0);
+      if (p < T) {
+        const uint4* src = reinterpret_cast<const uint4*>(x + p * K + g * 128 + sub * 16);
+        raw[u][0] = __ldg(src);
+        raw[u][1] = __ldg(src + 1);
+      }
+      p += step_p;
+      g += step_g;
+      if (g >= groups) {
+        g -= groups;
+        ++p;
+      }
+    }
+#pragma unroll
+    for (int u = 0; u < kIlp; ++u) {
+      float v[2][8], amax = 0.f;
+#pragma unroll
+      for (int h = 0; h < 2; ++h) {
+        const __nv_bfloat162* e = reinterpret_cast<const __nv_bfloat162*>(&raw[u][h]);
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+          v[h][2 * i] = __low2float(e[i]);
+          v[h][2 * i + 1] = __high2float(e[i]);
         }
-      } else {
-        *dst = bytes;
+#pragma unroll
+        for (int i = 0; i < 8; ++i) amax = fmaxf(amax, fabsf(v[h][i]));
+      }
+#pragma unroll
+      for (int off = 4; off > 0; off >>= 1) amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, off));
+      if (pu[u] >= T) continue;
+      const float s = group_scale(amax), r = __frcp_rn(s);
+      const uint2 lo = quant8(v[0], s, r, amax <= 3.0e38f), hi = quant8(v[1], s, r, amax <= 3.0e38f);
+      uint8_t* at = q + (int64_t)gu[u] * 128 + sub * 16;
+      for (int j = 0; j < k; ++j) {
+        const int32_t to = pos[pu[u] * k + j];
+        if (to >= 0) *reinterpret_cast<uint4*>(at + (int64_t)to * K) = make_uint4(lo.x, lo.y, hi.x, hi.y);
       }
       if (sub == 0) scale[pu[u] * groups + gu[u]] = s;
     }
@@ -394,13 +449,16 @@ int fmoe::run_scatter_rows(const void* x, int elem_bytes, int64_t T, int k, int6
 int fmoe::run_quant_scatter(const void* x, int64_t T, int k, int64_t K, const int32_t* slot_pos, bool per_row, void* q,
                             float* scale, cudaStream_t st) {
   FMOE_REQUIRE(K > 0 && K % (per_row ? 8 : 128) == 0 && (!per_row || K <= 16384), "quant_scatter: bad K %lld", (long long)K);
-  FMOE_REQUIRE(x && q && scale && aligned16(x) && (reinterpret_cast<uintptr_t>(q) & 7u) == 0, "quant_scatter: null or misaligned pointer");
+  FMOE_REQUIRE(x && q && scale && aligned16(x) && aligned16(q), "quant_scatter: null or misaligned pointer");
   auto go = [&](auto kernel, int64_t ctas) {
     launch_pdl(kernel, dim3((unsigned)std::min<int64_t>(std::max<int64_t>(ctas, 1), 148 * 8)), dim3(256), 0, st,
                (const __nv_bfloat16*)x, T, K, nullptr, k, 0, nullptr, (uint8_t*)q, scale, slot_pos);
   };
-  if (!per_row) go(quant_group128_kernel<__nv_bfloat16, RowMode::kScatter>, ceil_div<int64_t>(T * (K / 128), 64));
-  else if (K <= 2048) go(quant_row_kernel<32, 8, RowMode::kScatter>, ceil_div<int64_t>(T, 8));
+  if (!per_row) {
+    const int64_t ctas = std::min<int64_t>(std::max<int64_t>(ceil_div<int64_t>(T * (K / 128), 64), 1), 148 * 8);
+    launch_pdl(quant_scatter128_kernel, dim3((unsigned)ctas), dim3(256), 0, st, (const __nv_bfloat16*)x, T, K, k, slot_pos, (uint8_t*)q,
+               scale);
+  } else if (K <= 2048) go(quant_row_kernel<32, 8, RowMode::kScatter>, ceil_div<int64_t>(T, 8));
   else if (K <= 4096) go(quant_row_kernel<32, 16, RowMode::kScatter>, ceil_div<int64_t>(T, 8));
   else go(quant_row_kernel<256, 8, RowMode::kScatter>, T);
   return launch_status("quant_scatter");
