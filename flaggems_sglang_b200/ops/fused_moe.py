@@ -21,6 +21,7 @@ from __future__ import annotations
 import logging
 import os
 import sys
+import time
 from dataclasses import dataclass
 from typing import Optional
 
@@ -656,23 +657,27 @@ class StandardCombineInput:
     hidden_states: torch.Tensor
 
 
-_sglang_missing = False
+_SGLANG_RETRY_S = 0.2
+_sglang_missing = False  # or, after a failed import: the import path it searched and when to search again
 
 
 def _standard_output_type():
     """The combine-input container of the serving stack when it is importable (the reference imports it at
-    src/flaggems_sglang/ops/fused_moe.py:337-339), this module's stand-in with the same field otherwise.  A failed import is
-    not repeated until something has loaded sglang: each search of the import path takes 75 us of the calling thread, three
-    times what the rest of a hook call takes."""
+    src/flaggems_sglang/ops/fused_moe.py:337-339), this module's stand-in with the same field otherwise.  Each search of the
+    import path takes 75 us of the calling thread, three times what the rest of a hook call takes, so a failed import is
+    repeated only when something has loaded sglang, when the path or its finders are others, or after 0.2 s (files may have
+    come, or a finder learnt of them)."""
     global _sglang_missing
-    if _sglang_missing and "sglang" not in sys.modules:
+    path = (*sys.path, *sys.meta_path)
+    missing = _sglang_missing
+    if missing and "sglang" not in sys.modules and missing[0] == path and time.monotonic() < missing[1]:
         return StandardCombineInput
     try:
         from sglang.srt.layers.moe.token_dispatcher.standard import StandardCombineInput as _Sgl
 
         return _Sgl
     except Exception:  # noqa: BLE001
-        _sglang_missing = True
+        _sglang_missing = path, time.monotonic() + _SGLANG_RETRY_S
         return StandardCombineInput
 
 

@@ -301,3 +301,33 @@ def test_hook_output_type_follows_the_serving_stack(monkeypatch):
         monkeypatch.setitem(sys.modules, ".".join(path[:i + 1]), types.ModuleType(path[i]))
     sys.modules[".".join(path)].StandardCombineInput = dict
     assert fm._standard_output_type() is dict
+
+
+@pytest.mark.parametrize("how", ["path", "files"])
+def test_hook_output_type_finds_a_serving_stack_that_comes_later(monkeypatch, tmp_path, how):
+    """sglang becomes importable after a search has failed, and nobody else imports it: by a new entry of the import path, at
+    once; by files in a directory that was on it, at the next search."""
+    import importlib
+    import sys
+    import time
+
+    fm = importlib.import_module("flaggems_sglang_b200.ops.fused_moe")
+    for name in [m for m in sys.modules if m.split(".")[0] == "sglang"]:
+        monkeypatch.delitem(sys.modules, name)
+    monkeypatch.setattr(sys, "path", ([str(tmp_path)] if how == "files" else []) + [p for p in sys.path if p])
+    monkeypatch.setattr(fm, "_sglang_missing", False)
+    if fm._standard_output_type() is not fm.StandardCombineInput:
+        pytest.skip("sglang is installed")
+    d = tmp_path / "sglang" / "srt" / "layers" / "moe" / "token_dispatcher"
+    d.mkdir(parents=True)
+    (d / "standard.py").write_text("class StandardCombineInput:\n    pass\n")
+    if how == "path":
+        sys.path.insert(0, str(tmp_path))
+    else:
+        importlib.invalidate_caches()
+        monkeypatch.setattr(time, "monotonic", lambda: 1e12)
+    try:
+        assert fm._standard_output_type().__module__ == "sglang.srt.layers.moe.token_dispatcher.standard"
+    finally:
+        for name in [m for m in sys.modules if m.split(".")[0] == "sglang"]:
+            del sys.modules[name]
