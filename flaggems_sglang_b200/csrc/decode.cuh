@@ -15,7 +15,7 @@ struct RouteArgs {
   const int32_t* slot_of = nullptr;
   const int32_t* hist = nullptr;
   const float* gate = nullptr;
-  bool small_scratch = false;  // the caller's scratch is fixed: the decode kernels wherever they can take the call
+  bool small_scratch = false;  // the caller's scratch does not hold a faster family's plan: the decode kernels wherever they can take the call
 };
 
 struct DecodePlan {

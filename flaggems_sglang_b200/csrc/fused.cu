@@ -436,9 +436,25 @@ int run_fused(const fmoe_fused_args& args, const RouteArgs& route, const FusedPl
   return rc;
 }
 
+int plan_within(const fmoe_fused_args& a, const RouteArgs& route, int64_t limit, FusedPlan* plan) {
+  const int rc = plan_fused(a, route, plan);
+  if (rc || plan->total <= limit || a.variant != FMOE_VARIANT_AUTO) return rc;
+  RouteArgs small = route;
+  small.small_scratch = true;
+  FusedPlan other;
+  if (plan_fused(a, small, &other) == FMOE_OK && other.use_decode && other.total <= limit) {
+    *plan = other;
+    return FMOE_OK;
+  }
+  fmoe_fused_args stream = a;
+  stream.variant = FMOE_VARIANT_STREAM;
+  if (plan_fused(stream, route, &other) == FMOE_OK && other.total <= limit) *plan = other;
+  return FMOE_OK;
+}
+
 int run_with_workspace(const fmoe_fused_args& args, const RouteArgs& route, void* stream) {
   FusedPlan p;
-  int rc = plan_fused(args, route, &p);
+  int rc = plan_within(args, route, args.workspace_bytes, &p);
   if (rc) return rc;
   if (args.T == 0) return FMOE_OK;
   FMOE_REQUIRE(args.workspace && (reinterpret_cast<uintptr_t>(args.workspace) & 255u) == 0,

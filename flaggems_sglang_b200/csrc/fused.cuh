@@ -20,6 +20,9 @@ struct FusedPlan {
 
 int pick_variant(int dtype, int64_t numel, int E, int64_t I, int64_t H, int forced, int* variant, int* block);
 int plan_fused(const fmoe_fused_args& a, const RouteArgs& route, FusedPlan* plan);
+// plan_fused for scratch of `limit` bytes: where the fastest family's plan is larger, that of the decode or the streaming kernels
+// (no padded copies) if it fits.  When none does, the plan is the first one, and its total is above the limit.
+int plan_within(const fmoe_fused_args& a, const RouteArgs& route, int64_t limit, FusedPlan* plan);
 // Enqueues the whole computation using `ws` (at least plan.total bytes, 256-byte aligned) as scratch.
 int run_fused(const fmoe_fused_args& a, const RouteArgs& route, const FusedPlan& plan, uint8_t* ws, void* stream);
 

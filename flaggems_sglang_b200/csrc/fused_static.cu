@@ -50,25 +50,8 @@ extern "C" int fmoe_fused_experts_static(const fmoe_fused_args* args, void* stre
   using namespace fmoe;
   if (!args) return fail(FMOE_ERR_INVALID_ARG, "fused_experts_static: args is null");
   FusedPlan plan;
-  int rc = plan_fused(*args, RouteArgs{}, &plan);
+  int rc = plan_within(*args, RouteArgs{}, kStaticScratchBytes, &plan);
   if (rc) return rc;
-  fmoe_fused_args a = *args;
-  if (plan.total > kStaticScratchBytes && a.variant == FMOE_VARIANT_AUTO) {
-    // The decode and the streaming kernels need no padded copies: with few rows per expert their plans may fit where the faster
-    // one does not.
-    RouteArgs small;
-    small.small_scratch = true;
-    int variant = 0, block = 0;
-    FusedPlan other;
-    if (plan_fused(a, small, &other) == FMOE_OK && other.use_decode && other.total <= kStaticScratchBytes) {
-      plan = other;
-    } else {
-      a.variant = FMOE_VARIANT_STREAM;
-      if (pick_variant(a.dtype, a.T * a.top_k, a.num_experts, a.I, a.H, FMOE_VARIANT_STREAM, &variant, &block) == FMOE_OK &&
-          plan_fused(a, RouteArgs{}, &other) == FMOE_OK && other.total <= kStaticScratchBytes)
-        plan = other;
-    }
-  }
   if (plan.total > kStaticScratchBytes)
     return fail(FMOE_ERR_UNSUPPORTED,
                 "fused_experts_static: this problem needs %lld bytes of scratch, the built-in array holds %lld; "
@@ -78,5 +61,5 @@ extern "C" int fmoe_fused_experts_static(const fmoe_fused_args* args, void* stre
   uint8_t* scratch = nullptr;
   rc = static_scratch_for_current_device(&scratch);
   if (rc) return rc;
-  return run_fused(a, RouteArgs{}, plan, scratch, stream);
+  return run_fused(*args, RouteArgs{}, plan, scratch, stream);
 }

@@ -247,8 +247,9 @@ int fmoe_moe_sum_add(const void* z, int dtype, int64_t T, int k, int64_t H, floa
  * [quantisation] -> gemm2 * weight -> moe_sum.  Takes over src/flaggems_sglang/ops/fused_moe.py:197-232
  * (`triton_kernel_fused_experts` body) and, with b1/b2 and FMOE_ACT_SWIGLU_OAI, :235-325
  * (`triton_kernel_fused_experts_with_bias`) on the serving-side layouts w1 [E,2I,H], w2 [E,H,I].
- * All intermediates live in the caller's `workspace` (size from fmoe_fused_experts_workspace_bytes);
- * nothing is allocated and the host is never synchronised.
+ * All intermediates live in the caller's `workspace` (size from fmoe_fused_experts_workspace_bytes: what the fastest
+ * kernels for the shape need; with less, an AUTO call takes the decode or the streaming kernels where those have room, and is
+ * refused otherwise); nothing is allocated and the host is never synchronised.
  */
 typedef struct fmoe_fused_args {
   uint32_t struct_size; /* sizeof(fmoe_fused_args) as the caller compiled it (checked like fmoe_gemm_args.struct_size) */
@@ -307,7 +308,7 @@ typedef struct fmoe_route_args {
   int32_t renormalize;
   int32_t n_group, topk_group;  /* grouped only                                                           */
 } fmoe_route_args;
-/* Kernels that fmoe_fused_moe (route == NULL: fmoe_fused_experts) takes for these arguments: FMOE_VARIANT_* or
+/* Kernels that fmoe_fused_moe (route == NULL: fmoe_fused_experts) takes for these arguments and a full workspace: FMOE_VARIANT_* or
  * FMOE_FUSED_DECODE (at most 8 tokens: the GEMMs and the combine are one kernel), and the moe_align block (FMOE_FUSED_DECODE:
  * 0).  Pointers are not read; route->logits only says that there is a router to run. */
 #define FMOE_FUSED_DECODE 4
@@ -340,7 +341,7 @@ int fmoe_fused_experts_sorted(const fmoe_fused_args* args, const int32_t* topk_i
  * array of FMOE_STATIC_SCRATCH_BYTES that is part of the library image, so every GPU that loads the
  * library gives up that much memory until the process exits.
  *
- *   - Problems whose workspace (fmoe_fused_experts_workspace_bytes) exceeds FMOE_STATIC_SCRATCH_BYTES are
+ *   - Problems that no kernels can run in FMOE_STATIC_SCRATCH_BYTES (as with a workspace of that size) are
  *     refused with FMOE_ERR_UNSUPPORTED; nothing is launched.
  *   - The first call on each device looks up the array's device address (cudaGetSymbolAddress, with that
  *     device current) and remembers it.

@@ -95,6 +95,37 @@ def test_layer_variant_on_both_sides_of_its_lines(lib, dtype, T, E, H, I, k, wan
     test_layer_variant_is_what_the_one_call_layer_takes(lib, dtype, T, E, H, I, k, want)
 
 
+@pytest.mark.parametrize("dtype,T,E,H,I,k,small", [
+    ("E4M3", 3, 256, 7168, 256, 8, "decode"), ("E4M3", 64, 256, 7168, 2048, 8, "stream"), ("BF16", 48, 128, 2048, 384, 8, "stream"),
+    ("BF16", 300, 128, 2048, 384, 8, "stream")])
+def test_workspace_of_the_smaller_kernels_is_taken(lib, dtype, T, E, H, I, k, small):
+    """A caller that brings less than the fastest kernels need keeps the ones that need less, down to what those need (found here
+    by halving; without pointers a call whose workspace is large enough ends at the check of its pointers)."""
+    from flaggems_sglang_b200 import _C
+
+    a = _C.FusedArgs(dtype=getattr(_C, dtype), num_experts=E, top_k=k, T=T, H=H, I=I, workspace=256)
+    need = lib.fmoe_fused_experts_workspace_bytes(a)
+
+    def taken(size):
+        a.workspace_bytes = size
+        assert lib.fmoe_fused_experts(a, None) == _C.ERR_INVALID_ARG
+        msg = lib.fmoe_last_error()
+        assert (b"too small" in msg) != (b"null pointer" in msg), msg
+        return b"null pointer" in msg
+
+    lo, hi = 0, need
+    assert taken(hi) and not taken(lo)
+    while hi - lo > 1:
+        mid = (lo + hi) // 2
+        lo, hi = (lo, mid) if taken(mid) else (mid, hi)
+    # what holds the per-slot results and the activation; the streaming kernels' blocks hold up to 32 rows
+    rows = T * k * 8 if small == "decode" else T * k + min(E, T * k) * 31
+    eb = 2 if dtype == "BF16" else 1 + 4 / 128 + 4
+    assert hi <= min(need - 1, T * k * H * 2 + rows * I * eb + T * H * 2 + (1 << 20))
+    a.variant = _C.VARIANTS["tcgen05"]
+    assert not taken(need - 1)
+
+
 @pytest.mark.parametrize("stray", ["logits", "bias"])
 def test_one_call_moe_refuses_a_router_input_on_another_device(monkeypatch, stray):
     """The router's inputs go into the library call as plain pointers: they have to be on the layer's device (devices are

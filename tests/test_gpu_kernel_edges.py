@@ -502,3 +502,45 @@ def test_static_entry_streams_what_does_not_fit(fg):
     _C.check(lib.fmoe_fused_experts_static(a, _C.stream_ptr()))
     assert torch.equal(out, ref)
     assert_close_moe(auto, ref.cpu(), "fp8", "auto against stream")
+
+
+@pytest.mark.parametrize("entry", ["experts", "moe", "sorted"])
+@pytest.mark.parametrize("kind,T,E,H,I,limit", [("block", 3, 64, 2048 + 7168, 256, 1 << 20), ("bf16", 24, 64, 1280, 768, 1 << 22)])
+def test_workspace_that_holds_only_the_smaller_kernels(fg, entry, kind, T, E, H, I, limit):
+    """The C entries with less workspace than the fastest kernels need: the decode or the streaming kernels run in it, nothing
+    outside it is written."""
+    from flaggems_sglang_b200 import _C
+
+    k = 8
+    x, w1, w2, g = _layer(T, H, I, E, 40 + T)
+    logits = torch.randn(T, E, generator=g)
+    tw, ids = OR.softmax_topk(logits, k, True)
+    idx = torch.arange(0, T, 8)
+    if kind == "block":
+        (w1, s1), (w2, s2) = OQ.quant_weight_block128(w1), OQ.quant_weight_block128(w2)
+        ref = OE.fused_experts_fp8(x[idx], w1, s1, w2, s2, tw[idx], ids[idx])
+        scales = s1.cuda(), s2.cuda()
+    else:
+        ref, scales = OE.fused_experts(x[idx], w1, w2, tw[idx], ids[idx]), (None, None)
+    lib, d = _C.lib(), [x.cuda(), w1.cuda(), w2.cuda(), tw.cuda(), ids.cuda(), logits.cuda()]
+    out = torch.full((T, H), float("nan"), dtype=torch.bfloat16, device="cuda")
+    a = _C.FusedArgs(dtype=_C.E4M3 if kind == "block" else _C.BF16, num_experts=E, top_k=k, T=T, H=H, I=I, routed_scaling_factor=1.0,
+                     hidden=d[0].data_ptr(), w1=d[1].data_ptr(), w2=d[2].data_ptr(), w1_scale=_C.ptr(scales[0]),
+                     w2_scale=_C.ptr(scales[1]), topk_weights=d[3].data_ptr(), topk_ids=d[4].data_ptr(), out=out.data_ptr())
+    assert lib.fmoe_fused_experts_workspace_bytes(a) > limit
+    area = torch.full((limit + 512 + 4096,), 0x5A, dtype=torch.uint8, device="cuda")
+    start = -(-(area.data_ptr() + 2048) // 256) * 256
+    a.workspace, a.workspace_bytes = start, limit
+    st = _C.stream_ptr()
+    if entry == "experts":
+        _C.check(lib.fmoe_fused_experts(a, st))
+    elif entry == "moe":
+        _C.check(lib.fmoe_fused_moe(a, _C.RouteArgs(logits=d[5].data_ptr(), grouped=0, renormalize=1, n_group=1, topk_group=1), st))
+    else:
+        rd, gi, _ = fg.standard_topk_to_routing(d[3], d[4], E)
+        slot_of, hist, gate = (v.contiguous() for v in (gi.src_indx, rd.expt_hist, rd.gate_scal))
+        _C.check(lib.fmoe_fused_experts_sorted(a, slot_of.data_ptr(), hist.data_ptr(), gate.data_ptr(), st))
+    torch.cuda.synchronize()
+    lo = start - area.data_ptr()
+    assert bool((area[:lo] == 0x5A).all()) and bool((area[lo + limit:] == 0x5A).all())
+    assert_close_moe(out[idx.cuda()], ref, "fp8" if kind == "block" else "bf16", f"{entry} {kind} small workspace")
