@@ -7,7 +7,7 @@
 //   TMEM      : 512 columns per CTA = two 128 x 256 fp32 accumulators, so the epilogue of a tile overlaps the next tile
 //   warps     : 0-15 epilogue (TMEM lane quarter = warp % 4; the four of a quarter take 16-token chunks in turn),
 //               16-17 TMA producers (each CTA its own weight rows and its own half of the tokens), 18 MMA issuer (CTA 0),
-//               19 list of the worker's tiles
+//               19 the worker's tiles (long launches: tickets, so that all workers stay near one another)
 //
 // Why pairs: with one CTA per 128 x 256 tile an MMA reads 12 KB of shared memory for every 8 KB here, and TMA writes as
 // much; fill and operand reads of one SM together ran into its 128 bytes per clock.  Why weights on M: see pair.cuh.
@@ -47,14 +47,15 @@ constexpr int ACC_COLS = 256;
 // with 8 a short main loop waited for them (7.3k cycles per tile against 6.1k of MMAs at K = 768).
 constexpr int kEpiWarps = 16;
 // TMA warps: they take the K steps in turn.  Waiting for a stage, arming it and issuing two to five copies takes one thread
-// about 430 cycles, and with one warp that was the pace of every tile whose MMAs need less (SM cycles per K step with 64, 128,
-// 192 and 256 tokens per tile: 431, 470, 493, 508; two warps: 288 tokens in two tiles 500 -> 405, 256 tokens 508 -> 465; a
-// third one changes nothing).  Qwen3, 128 experts of 288 rows: gate/up GEMM 270 -> 251 us; Mixtral 549 -> 513 us.
+// 430 to 500 cycles, and with one warp that was the pace of every tile whose MMAs need less.  SM cycles per K step, counted by the
+// MMA warp, one / two warps: Mixtral gate/up with 192 tokens per tile 499 / 392 (their MMAs: 384), 256 tokens 515 / 513 (512);
+// Qwen3 with 144 tokens 523 / 446.  A third warp changes nothing.  Qwen3, 128 experts of 288 rows: gate/up GEMM 270 -> 251 us.
 constexpr int kProducers = 2;
 constexpr int kThreads = (kEpiWarps + kProducers + 2) * 32;
 constexpr int BOX_TOKENS = 32;                      // token rows per TMA box
 constexpr int STRIP_BYTES = kStripBytes;             // per epilogue warp; also holds its 1 KB of the gate/up exchange
-constexpr int BAR_BYTES = 256;
+constexpr int BAR_BYTES = 768;
+constexpr int kMaxTicketWorkers = (kSplitCounters - 1) / 8 * 2;  // the tail split leaves its last counter to the tickets
 constexpr int smem_bytes(int num_experts) {
   return RING_BYTES + BAR_BYTES + kListBytes + kEpiWarps * STRIP_BYTES + pair_table_bytes(num_experts);
 }
@@ -74,6 +75,7 @@ struct PairParams {
   void* const* out_rows;  // down projection: optional per-slot row addresses (may be peer memory)
   float* split_partials;    // tail split: [workers][2 CTAs][128][256] f32 partial accumulators (NULL: no split)
   int32_t* split_counters;  // tail split: [tiles][2 CTAs][4 warp groups] arrivals, zero at launch
+  int32_t* tickets;         // units taken beyond the workers' first ones, zero at launch (NULL: units are dealt round-robin)
   int64_t numel;
   int64_t n;              // gemm1: I, gemm2: H
   int64_t w_rows;         // rows of W per expert
@@ -114,6 +116,54 @@ __device__ __forceinline__ bool any_of_four_warps(int bar, bool pred) {
   return v != 0;
 }
 
+// A worker's units in shared memory, two halves of kListUnits.  Dealt round-robin, each CTA's list warp works them out 32 at a
+// time (as PairList).  Taken by ticket, CTA 0's does, one at a time and one unit ahead of the TMA warps, and hands them to the
+// roles of both CTAs.
+// Why tickets: workers with tiles of their own drift apart, by 108 us after 48 tiles of 27 us (Mixtral gate/up, 875 rows), since
+// one that is behind finds its weights gone from L2 and falls further behind.  The four that share a weight tile were 37 us
+// apart and read it from DRAM more than once; by ticket they are 2.4 us apart.  DRAM bytes read by that GEMM at 4096 tokens: 2.70 ->
+// 1.95 GB, of which 1.95 are its weights and rows.  (With one TMA warp, whose pace held the workers together, 1.99.  Dealt, it was
+// 3.1 and 4.1 GB on other cards.)
+struct PairFeed {
+  const int4* units;  // [2 * kListUnits]; one without columns ends the work
+  uint64_t* full;     // [2 * kListUnits] the unit, or (dealt) the 32 from it, are there
+  uint32_t empty;     // [2] every reader has read a half: readers of this CTA, or (tickets) of both, in CTA 0
+  uint64_t* ask;      // tickets, used in CTA 0: a TMA warp has begun a unit
+  bool tickets;
+  int n = 0;          // units read so far
+  __device__ __forceinline__ PairFeed(const void* units_, uint64_t* bars, bool tickets_)
+      : units(reinterpret_cast<const int4*>(units_)), full(bars), ask(bars + 2 * kListUnits + 2), tickets(tickets_) {
+    empty = ptx::smem_u32(bars + 2 * kListUnits) & (tickets ? ~ptx::kPeerRankBit : ~0u);
+  }
+  __device__ __forceinline__ void init_barriers(int readers) {
+    for (int i = 0; i < 2 * kListUnits; ++i) ptx::mbar_init(&full[i], 1);
+    for (int i = 0; i < 2; ++i) ptx::mbar_init(full + 2 * kListUnits + i, readers);
+    ptx::mbar_init(ask, 1);
+  }
+  __device__ __forceinline__ bool waits() const { return tickets || n % kListUnits == 0; }  // the next next() waits
+  // Next unit, for a role that one thread runs, or (WARP) a whole warp.  1: there is one, 0: the work has ended, -1: time-out.
+  template <bool WARP>
+  __device__ __forceinline__ int next(PairUnit* u) {
+    const int half = n / kListUnits, slot = n % (2 * kListUnits);
+    if (n && n % kListUnits == 0) {
+      if (WARP) __syncwarp();
+      if (!WARP || (threadIdx.x & 31) == 0) ptx::mbar_arrive_cluster(empty + 8 * ((half & 1) ^ 1));
+    }
+    if (waits()) {
+      bool ok = ptx::mbar_wait(&full[slot], (half >> 1) & 1);
+      if (WARP) ok = __all_sync(0xffffffffu, ok);
+      if (!ok) return -1;
+    }
+    u->unpack(units[slot]);
+    ++n;
+    return u->tl.cols != 0;
+  }
+  // The list warp, before it writes the first unit of a half: its readers have read what was there.
+  __device__ __forceinline__ bool wait_half(int half) const {
+    return half < 2 || __all_sync(0xffffffffu, ptx::mbar_wait_relaxed(full + 2 * kListUnits + (half & 1), ((half >> 1) & 1) ^ 1));
+  }
+};
+
 template <bool GATED, bool F8, bool EXTRA, bool WMN, bool GATHER>
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 1)
 grouped_gemm_pair_kernel(const __grid_constant__ CUtensorMap map_t, const __grid_constant__ CUtensorMap map_w,
@@ -128,8 +178,7 @@ grouped_gemm_pair_kernel(const __grid_constant__ CUtensorMap map_t, const __grid
   uint64_t* acc_full = bars + 2 * MAX_STAGES;       // [2] per CTA: MMA -> this CTA's epilogue
   uint64_t* acc_empty = bars + 2 * MAX_STAGES + 2;  // [2] used in CTA 0: both epilogues -> MMA
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 2 * MAX_STAGES + 4);
-  uint64_t* list_bars = bars + 2 * MAX_STAGES + 5;   // [4] (PairList)
-  int4* list = reinterpret_cast<int4*>(smem + RING_BYTES + BAR_BYTES);
+  PairFeed units(smem + RING_BYTES + BAR_BYTES, bars + 2 * MAX_STAGES + 5, p.tickets != nullptr);
   uint8_t* strips = smem + RING_BYTES + BAR_BYTES + kListBytes;
   int32_t* table = reinterpret_cast<int32_t*>(strips + kEpiWarps * STRIP_BYTES);
 
@@ -146,7 +195,7 @@ grouped_gemm_pair_kernel(const __grid_constant__ CUtensorMap map_t, const __grid
       ptx::mbar_init(&acc_full[a], 1);
       ptx::mbar_init(&acc_empty[a], 2 * kEpiWarps);  // one arrival per epilogue warp of both CTAs
     }
-    PairList::init_barriers(list_bars, kEpiWarps + kProducers + (rank == 0));
+    units.init_barriers(units.tickets ? 2 * (kEpiWarps + kProducers) + 1 : kEpiWarps + kProducers + (rank == 0));
     ptx::fence_barrier_init();
   }
   if (warp == kEpiWarps && lane == 0) {
@@ -170,7 +219,6 @@ grouped_gemm_pair_kernel(const __grid_constant__ CUtensorMap map_t, const __grid
   const uint32_t tmem_base = *tmem_slot;
 
   const int k_steps = p.k_steps;
-  PairList units(list, list_bars);
   PairUnit unit;
   const PairTile& tl = unit.tl;
   auto first_step = [&](int slice) { return (int)((int64_t)k_steps * slice >> unit.log2_s); };  // of a slice of this unit's tile
@@ -201,6 +249,7 @@ grouped_gemm_pair_kernel(const __grid_constant__ CUtensorMap map_t, const __grid
           if (got < 0) report(0x400);
           break;
         }
+        if (units.tickets && rank == 0 && me == 0) ptx::mbar_arrive(units.ask);
         const int ks0 = first_step(unit.slice), ks1 = first_step(unit.slice + 1);
         const int half_n = tl.n >> 1;                       // tokens this CTA loads
         const int row_t = tl.row0 + rank * half_n;
@@ -330,13 +379,58 @@ grouped_gemm_pair_kernel(const __grid_constant__ CUtensorMap map_t, const __grid
       }
     }
   } else if (warp == kMmaWarp + 1) {
-    // ---------------- the worker's tiles ----------------
+    // ---------------- the worker's units ----------------
     UnitPlan plan;
     plan.init((int64_t)table[3 * p.num_experts] * p.w_tiles, k_steps, p.split_max, workers, worker);
-    int more = 1;
-    for (int batch = 0; more > 0; ++batch)
-      more = PairList::fill(list, list_bars, batch, plan, p.w_tiles, p.group, p.num_experts, table);
-    if (more < 0) report(0x430);
+    auto unit_at = [&](int64_t it, int4* d) {
+      int64_t tile;
+      int ks0, ks1;
+      PairUnit u;
+      const bool any = plan.get(it, &tile, &ks0, &ks1, &u.slice);
+      *d = make_int4(0, 0, 0, 0);
+      if (any) {
+        u.tl = pair_locate(tile, p.w_tiles, p.group, p.num_experts, table);
+        u.log2_s = plan.is_split(it) ? 31 - __clz(plan.S) : 0;
+        u.b = plan.b;
+        *d = u.pack();
+      }
+      return any;
+    };
+    int4* list = const_cast<int4*>(units.units);
+    int4 d;
+    if (!units.tickets) {
+      bool more = true;
+      for (int half = 0; more; ++half) {
+        if (!units.wait_half(half)) {
+          report(0x430);
+          break;
+        }
+        more = __all_sync(0xffffffffu, unit_at((int64_t)half * kListUnits + lane, &d));
+        list[(half & 1) * kListUnits + lane] = d;
+        __syncwarp();
+        if (lane == 0) ptx::mbar_arrive(&units.full[(half & 1) * kListUnits]);
+      }
+    } else if (rank == 0) {
+      bool more = true;
+      for (int i = 0, ticket = worker; more; ++i) {
+        if (i) {
+          if (!__all_sync(0xffffffffu, ptx::mbar_wait_relaxed(units.ask, (i - 1) & 1))) {
+            report(0x431);
+            break;
+          }
+          if (lane == 0) ticket = workers + atomicAdd(p.tickets, 1);
+          ticket = __shfl_sync(0xffffffffu, ticket, 0);
+        }
+        if (i % kListUnits == 0 && !units.wait_half(i / kListUnits)) {
+          report(0x432);
+          break;
+        }
+        plan.b = ticket % workers;
+        more = unit_at(ticket / workers, &d);
+        const int slot = i % (2 * kListUnits);
+        if (lane < 2) ptx::st_async_16(ptx::mapa(ptx::smem_u32(list + slot), lane), d, ptx::mapa(ptx::smem_u32(&units.full[slot]), lane));
+      }
+    }
   } else {
     // ---------------- epilogue (both CTAs, each its CTA's 128 weight rows) ----------------
     pdl_entry_late();
@@ -347,7 +441,7 @@ grouped_gemm_pair_kernel(const __grid_constant__ CUtensorMap map_t, const __grid
     bool alive = true;
     long long prof_wait = 0, prof_busy = 0;
     while (alive) {
-      const bool waits = units.n % kListUnits == 0;
+      const bool waits = units.waits();
       int got = units.next<true>(&unit);
       if (waits && any_of_four_warps(1 + half, got < 0)) got = -1;  // warps that meet at a barrier below leave together
       if (got <= 0) {
@@ -411,7 +505,7 @@ grouped_gemm_pair_kernel(const __grid_constant__ CUtensorMap map_t, const __grid
       // fragment (slice o, chunk j) of this thread: four float4, 512 bytes apart so that a warp stores whole lines
       auto partial = [&](int o, int j) {
         return reinterpret_cast<float4*>(p.split_partials) +
-               ((((int64_t)(worker - slice + o) * 2 + rank) * 16 + j) * 4 + quarter) * 128 + lane;
+               ((((int64_t)(unit.b - slice + o) * 2 + rank) * 16 + j) * 4 + quarter) * 128 + lane;
       };
       bool finish = true;  // these four warps run the epilogue of their chunks
       if (split) {
@@ -432,7 +526,7 @@ grouped_gemm_pair_kernel(const __grid_constant__ CUtensorMap map_t, const __grid
         __threadfence();  // the partials are visible device-wide before these warps count as arrived
         asm volatile("bar.sync %0, 128;" ::"r"(1 + half) : "memory");
         finish = any_of_four_warps(1 + half, quarter == 0 && lane == 0 &&
-                                                 atomicAdd(p.split_counters + ((worker >> unit.log2_s) * 2 + rank) * 4 + half, 1) == S - 1);
+                                                 atomicAdd(p.split_counters + ((unit.b >> unit.log2_s) * 2 + rank) * 4 + half, 1) == S - 1);
         __threadfence();  // the other slices' partials are read after the count
       }
       // the next chunk's TMEM read-out is in flight while a chunk is stored
@@ -752,6 +846,7 @@ int launch(const GemmParams& g, cudaStream_t st) {
   p.split_partials = nullptr;
   p.split_counters = nullptr;
   p.split_max = 0;
+  p.tickets = nullptr;
   const char* split_env = getenv("FMOE_TC_SPLIT_TAIL");  // "0": off (read per launch, tests flip it)
   const bool split_off = split_env && split_env[0] == '0';
   const bool split_fits = g.split_ws_bytes >= kSplitCounters * 4 + (int64_t)workers * 2 * 128 * 256 * 4 && workers <= 128;
@@ -765,6 +860,15 @@ int launch(const GemmParams& g, cudaStream_t st) {
       FMOE_CUDA_OK(cudaMemsetAsync(g.split_ws, 0, kSplitCounters * 4, st));
     }
   }
+  // Units by ticket from 800 K steps a worker on (by the rows an expert has on average), and where there is a zeroed word.  Layers
+  // dealt / by ticket in us: Mixtral 2048 tokens 1407 / 1390, 3000 2054 / 1919, 3500 2419 / 2196, 4096 2650 / 2516, 8192 5146 /
+  // 4804; Qwen3 16384 tokens 1478 / 1425; DeepSeek-V3 per channel 8192 tokens 4251 / 4047, 2048 1855 / 1851, 16 544 / 540.  Below,
+  // what a ticket takes shows and there is no drift to save: half of Mixtral 333 tokens 266.6 / 268.2, Mixtral 19 tokens 437.2 /
+  // 439.7, a quarter of Qwen3 (down GEMM of 3 K steps a tile) 387 / 397.
+  int32_t* counters = g.split_counters ? g.split_counters : p.split_counters;
+  const int64_t active = std::min<int64_t>(g.num_experts, g.numel);
+  const int64_t tiles = std::max(active, g.numel / p.token_tile + active / 2) * p.w_tiles;
+  if (counters && workers <= kMaxTicketWorkers && tiles * p.k_steps >= 800 * workers) p.tickets = counters + kSplitCounters - 1;
   launch_pdl(kernel, dim3(2 * workers), dim3(kThreads), smem, st, map_t, map_w, p);
   return launch_status("grouped_gemm_pair_kernel");
 }

@@ -22,7 +22,8 @@ inline int pick_token_tile(int64_t numel, int num_experts, bool e4m3) {
   const double rows = (double)numel / (double)(numel < num_experts ? (numel > 0 ? numel : 1) : num_experts);
   return rows <= 40.0 ? 64 : (rows <= 88.0 && !e4m3 ? 128 : 256);
 }
-// tail-split arrival counters of one launch: 8 per split tile, of which there are at most half as many as workers (<= 128)
+// tail-split arrival counters of one launch: 8 per split tile, of which there are at most half as many as workers (<= 128); up to
+// 126 workers the last word is free and counts the tickets (gemm_pair.cu)
 constexpr int kSplitCounters = 512;
 
 // int32 words of the expert table: first row [E], rows [E], exclusive prefix sum of the token tiles [E + 1]
@@ -205,7 +206,8 @@ __device__ __forceinline__ void zero_block_rows(const PairTile& tl, void* out, i
 }
 #endif
 
-// Work units of one worker (a CTA pair).  Tiles are dealt round-robin; when the last round has work for at most half of
+// Work units of one worker (a CTA pair).  Tiles are dealt round-robin (long launches of gemm_pair.cu: taken by ticket in the same
+// order, a unit being that of worker ticket % workers in round ticket / workers); when the last round has work for at most half of
 // the workers (they are bound by their own rate, so a part-filled round costs as much as a full one), each of its tiles
 // is cut into S slices along K (S a power of two) that S neighbouring workers compute.  Every worker leaves its partial
 // accumulator in global memory; whichever arrives last (counted per group of four epilogue warps) adds all S in slice order (a
@@ -261,8 +263,9 @@ constexpr int kListBytes = 2 * kListUnits * 16;
 struct PairUnit {
   PairTile tl;
   int slice, log2_s;  // slice of a tile that is cut into 2^log2_s along K
+  int b;              // place in its round (UnitPlan)
   __device__ __forceinline__ int4 pack() const {
-    return make_int4(tl.row0, tl.cols | (int)tl.last << 9 | log2_s << 10 | slice << 14, tl.w_tile, tl.expert);
+    return make_int4(tl.row0, tl.cols | (int)tl.last << 9 | log2_s << 10 | slice << 14, tl.w_tile, tl.expert | b << 16);
   }
   __device__ __forceinline__ void unpack(const int4& d) {
     tl.row0 = d.x;
@@ -272,7 +275,8 @@ struct PairUnit {
     log2_s = d.y >> 10 & 15;
     slice = d.y >> 14;
     tl.w_tile = d.z;
-    tl.expert = d.w;
+    tl.expert = d.w & 0xffff;
+    b = d.w >> 16;
   }
 };
 
@@ -316,6 +320,7 @@ struct PairList {
     if (any) {
       u.tl = pair_locate(tile, w_tiles, group, num_experts, table, fixed);
       u.log2_s = plan.is_split(it) ? 31 - __clz(plan.S) : 0;
+      u.b = plan.b;
       d = u.pack();
     }
     units[slot * kListUnits + lane] = d;

@@ -122,6 +122,19 @@ __device__ __forceinline__ void cluster_sync_all() {  // every thread of every C
 __device__ __forceinline__ void mbar_arrive_cluster(uint32_t cluster_addr) {
   asm volatile("mbarrier.arrive.shared::cluster.b64 _, [%0];" ::"r"(cluster_addr) : "memory");
 }
+// Cluster-wide address of a CTA's copy of this CTA's shared memory address
+__device__ __forceinline__ uint32_t mapa(uint32_t addr, uint32_t cta) {
+  uint32_t out;
+  asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(out) : "r"(addr), "r"(cta));
+  return out;
+}
+// 16 bytes to shared memory of the cluster, and the one arrival of the mbarrier (of the same CTA) that waits for them
+__device__ __forceinline__ void st_async_16(uint32_t dst, const int4& v, uint32_t bar) {
+  asm volatile("mbarrier.arrive.expect_tx.release.cluster.shared::cluster.b64 _, [%0], 16;" ::"r"(bar) : "memory");
+  asm volatile("st.async.shared::cluster.mbarrier::complete_tx::bytes.v4.b32 [%0], {%1, %2, %3, %4}, [%5];" ::"r"(dst), "r"(v.x),
+               "r"(v.y), "r"(v.z), "r"(v.w), "r"(bar)
+               : "memory");
+}
 // Tiled TMA loads into THIS CTA's shared memory whose completion bytes are credited to an mbarrier that may live in the
 // pair's other CTA (cluster-wide address).  Plain loads: one destination CTA.
 __device__ __forceinline__ void tma_load_2d_pair(uint32_t smem_dst, const CUtensorMap* map, int32_t x, int32_t y,

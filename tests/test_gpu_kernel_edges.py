@@ -544,3 +544,98 @@ def test_workspace_that_holds_only_the_smaller_kernels(fg, entry, kind, T, E, H,
     lo = start - area.data_ptr()
     assert bool((area[:lo] == 0x5A).all()) and bool((area[lo + limit:] == 0x5A).all())
     assert_close_moe(out[idx.cuda()], ref, "fp8" if kind == "block" else "bf16", f"{entry} {kind} small workspace")
+
+
+@pytest.mark.parametrize("gated", [True, False])
+@pytest.mark.parametrize("kind", ["bf16", "n_major", "channel"])
+def test_units_by_ticket_are_those_dealt(fg, kind, gated):
+    """Long launches of the CTA-pair GEMM take their units by ticket.  Some 70 (e4m3: 140) a worker, so that the list's places are
+    used again, and tiles that are too short along K to be cut: the bits are those of units dealt round-robin, which a call without
+    scratch keeps.  Beside another stream's calls too, when workers start late."""
+    from flaggems_sglang_b200 import _C
+    from flaggems_sglang_b200.ops.fused_moe import _gemm_args
+
+    rows = [1, 256, 257, 900, 0, 513, 64, 511] * 3
+    E, numel, k = len(rows), sum(rows), 768
+    e4m3 = kind == "channel"
+    steps, w_tiles = k * (1 if e4m3 else 2) // 128, 248 if e4m3 else 124
+    n, lib = w_tiles * (128 if gated else 256), _C.lib()
+    assert (numel // 256 + E // 2) * w_tiles * steps >= 800 * (lib.fmoe_sm_count() // 2) and steps < 16
+    g = torch.Generator(device="cuda").manual_seed(5)
+    ids = torch.repeat_interleave(torch.arange(E), torch.tensor(rows)).to(torch.int32).view(-1, 1).cuda()
+    sorted_ids, expert_ids, num_post = fg.moe_align_block_size(ids, 128, E)
+    cap = sorted_ids.numel()
+    dt, w_rows = torch.float8_e4m3fn if e4m3 else torch.bfloat16, (2 if gated else 1) * n
+    a = torch.randn(cap, k, generator=g, device="cuda").to(dt)
+    w = torch.empty(E, *((k, w_rows) if kind == "n_major" else (w_rows, k)), dtype=dt, device="cuda")
+    for e in range(E):
+        w[e] = (torch.randn(*w.shape[1:], generator=g, device="cuda") * k ** -0.5).to(dt)
+    scales = {}
+    if e4m3:
+        s = torch.rand(cap, generator=g, device="cuda"), torch.rand(E, w_rows, generator=g, device="cuda")
+        scales = dict(a_scale=s[0].data_ptr(), w_scale=s[1].data_ptr(), scale_mode=_C.SCALE_CHANNEL)
+    split_ws = torch.empty(int(lib.fmoe_gemm_split_workspace_bytes()), dtype=torch.uint8, device="cuda")
+
+    def call(tickets):
+        out = torch.zeros(cap if gated else numel, n, dtype=torch.bfloat16, device="cuda")
+        ws = dict(split_ws=split_ws.data_ptr(), split_ws_bytes=split_ws.numel()) if tickets else {}
+        args = _gemm_args(variant=_C.VARIANTS["tcgen05"], activation=0, num_experts=E, top_k=1, block_size=128, numel=numel,
+                          sorted_cap=cap, max_blocks=cap // 128, sorted_token_ids=sorted_ids.data_ptr(),
+                          expert_ids=expert_ids.data_ptr(), num_tokens_post_padded=num_post.data_ptr(),
+                          dtype=_C.E4M3 if e4m3 else _C.BF16, out_dtype=_C.BF16, n=n, k=k, a_rows=cap, a=a.data_ptr(),
+                          w=w.data_ptr(), out=out.data_ptr(), w_layout=_C.W_N_MAJOR if kind == "n_major" else _C.W_K_MAJOR,
+                          **scales, **ws)
+        _C.check((lib.fmoe_gemm1_silu if gated else lib.fmoe_gemm2)(args, _C.stream_ptr()))
+        return out
+
+    ref = call(False)
+    assert float(ref.float().abs().sum()) > 0
+    other = _decode_call(fg, "bf16", 8, 5, E=32, H=1024, I=1024)
+    other()
+    torch.cuda.synchronize()
+    streams = [torch.cuda.Stream(priority=p) for p in (0, -1)]
+    outs = []
+    for _ in range(3):
+        with torch.cuda.stream(streams[1]):
+            for _ in range(8):
+                other()
+        with torch.cuda.stream(streams[0]):
+            outs.append(call(True))
+    torch.cuda.synchronize()
+    assert all(torch.equal(o, ref) for o in outs)
+
+
+# the gate/up GEMM (H = 32 K steps), then the down GEMM (I = 126 K steps) by ticket with the tiles of its last round cut along K
+@pytest.mark.parametrize("H,I,gated", [(2048, 14336, True), (7168, 8064, False)])
+@pytest.mark.parametrize("kind", ["bf16", "n_major", "channel"])
+def test_units_by_ticket_with_a_cut_last_round(fg, kind, H, I, gated):
+    from flaggems_sglang_b200 import _C
+
+    lib, E, T, step = _C.lib(), 2, 4096, 64
+    if kind == "channel":
+        H, I, step = (2 * H, I, 128) if gated else (H, 2 * I, 128)
+    steps, w_tiles = (H // step, I // 128) if gated else (I // step, H // 256)
+    assert (T // 256 + E // 2) * w_tiles * steps >= 800 * (lib.fmoe_sm_count() // 2)
+    slices = (ctypes.c_int64 * 5)()
+    tiles, workers = T // 256 * w_tiles, lib.fmoe_sm_count() // 2
+    assert lib.fmoe_debug_tail_plan(tiles, steps, 4 if gated else 8, workers, 0, -(-tiles // workers) - 1, slices) == 1 and slices[4] > 1
+    gd = torch.Generator(device="cuda").manual_seed(18)
+    w1 = torch.stack([(torch.randn(2 * I, H, generator=gd, device="cuda") * H ** -0.5).bfloat16() for _ in range(E)])
+    w2 = torch.stack([(torch.randn(H, I, generator=gd, device="cuda") * I ** -0.5).bfloat16() for _ in range(E)])
+    g = torch.Generator().manual_seed(17)
+    x, tw = torch.randn(T, H, generator=g).bfloat16(), torch.rand(T, 1, generator=g) + 0.5
+    ids = torch.arange(E).repeat(T // E).to(torch.int32).view(T, 1)
+    idx = torch.linspace(0, T - 1, 8).long()
+    d, kw = [x.cuda(), w1, w2], dict(variant="tcgen05")
+    c1, c2 = w1.cpu(), w2.cpu()
+    if kind == "n_major":
+        d[1:], kw = [w.transpose(1, 2).contiguous() for w in d[1:]], dict(weights_n_major=True)
+    if kind == "channel":
+        (q1, s1), (q2, s2) = OQ.quant_weight_per_channel(c1), OQ.quant_weight_per_channel(c2)
+        ref = OE.fused_experts_fp8_per_channel(x[idx], q1, s1, q2, s2, tw[idx], ids[idx])
+        d[1:], kw = [q1.cuda(), q2.cuda()], dict(use_fp8_w8a8=True, per_channel_quant=True, w1_scale=s1.cuda(), w2_scale=s2.cuda())
+    else:
+        ref = OE.fused_experts(x[idx], c1, c2, tw[idx], ids[idx])
+    outs = [fg.fused_experts(*d, tw.cuda(), ids.cuda(), **kw) for _ in range(3)]
+    assert_close_moe(outs[0][idx.cuda()], ref, "fp8" if kind == "channel" else "bf16", f"tickets {kind} H={H}")
+    assert all(torch.equal(o, outs[0]) for o in outs)
