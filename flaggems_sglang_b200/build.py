@@ -25,6 +25,7 @@ NVCC_FLAGS = [
     "-O3", "-std=c++17", "-lineinfo",
     "-Xcompiler", "-fPIC",
     "--expt-relaxed-constexpr",
+    "-Xptxas", "-v",
     "-I", INCLUDE,
 ]
 
@@ -46,6 +47,11 @@ def _deps_mtime() -> float:
     return max(os.path.getmtime(h) for h in hdrs)
 
 
+def ptxas_report(src: str) -> str:
+    """Where the registers and spills of a source file's kernels are kept, as the compiler printed them."""
+    return os.path.join(OBJ_DIR, src[:-3] + ".ptxas")
+
+
 def build(force: bool = False, verbose: bool = False) -> str:
     os.makedirs(OBJ_DIR, exist_ok=True)
     nvcc = _nvcc()
@@ -56,12 +62,8 @@ def build(force: bool = False, verbose: bool = False) -> str:
         s = os.path.join(CSRC, src)
         o = os.path.join(OBJ_DIR, src[:-3] + ".o")
         objs.append(o)
-        if force or not os.path.exists(o) or os.path.getmtime(o) < max(os.path.getmtime(s), hdr_m):
-            cmd = [nvcc, *NVCC_FLAGS, "-c", s, "-o", o]
-            if verbose:
-                cmd.insert(1, "-Xptxas")
-                cmd.insert(2, "-v")
-            jobs.append(cmd)
+        if force or not os.path.exists(o) or not os.path.exists(ptxas_report(src)) or os.path.getmtime(o) < max(os.path.getmtime(s), hdr_m):
+            jobs.append([nvcc, *NVCC_FLAGS, "-c", s, "-o", o])
 
     def run(cmd):
         r = subprocess.run(cmd, capture_output=True, text=True)
@@ -74,6 +76,8 @@ def build(force: bool = False, verbose: bool = False) -> str:
                     sys.stderr.write(" ".join(cmd) + "\n" + r.stdout + r.stderr)
                 if r.returncode != 0:
                     raise RuntimeError(f"nvcc failed for {cmd[-3]}")
+                with open(ptxas_report(os.path.basename(cmd[-3])), "w") as f:
+                    f.write(r.stderr)
     if jobs or force or not os.path.exists(LIB_PATH):
         cmd = [nvcc, "-shared", "-o", LIB_PATH, *objs, "-gencode", "arch=compute_100a,code=sm_100a", "--cudart", "shared"]
         r = subprocess.run(cmd, capture_output=True, text=True)

@@ -359,9 +359,7 @@ grouped_gemm_pair_fold_kernel(const __grid_constant__ CUtensorMap map_t, const _
     const int me = warp - (kFoldWarps + 2);
     int more = 0;  // the list goes on
     auto add_units = [&](int batch) {
-      UnitPlan plan;
-      plan.init(total_tiles, kblocks, 0, workers, worker);
-      more = PairList::fill(list, list_bars, batch, plan, p.w_tiles, p.group, p.num_experts, table);
+      more = PairList::fill(list, list_bars, batch, worker, workers, total_tiles, p.w_tiles, p.group, p.num_experts, table);
       if (more < 0) report(0x5b0);
     };
     if (me == 0) add_units(0);
@@ -665,8 +663,11 @@ grouped_gemm_pair_fold_kernel(const __grid_constant__ CUtensorMap map_t, const _
 //   32 * (w % 4).., half w / 8, the 64 columns of CTA w / 4 % 2's weight rows (M = 128: 32 columns): 64 accumulators per
 //   thread.  (Eight warps with 128 accumulators each spill: 530 -> 700 us and more.)
 //   warp 16 TMA, warp 17 MMA (CTA 0), warps 18-19 factors: products of token and weight scales in a ring of 4 slots of 8 K
-//   blocks, one slot wait per 8 K blocks of the fold.  Their loop over the slot's halves is not unrolled: it would not fit
-//   their 64 registers (gate/up GEMM, 256 rows, 545 us with it, 519 without).
+//   blocks, one slot wait per 8 K blocks of the fold.  What would not fit their 64 registers is left out of their loop: it is not
+//   unrolled over the slot's halves (gate/up GEMM, 256 rows, 545 us with it, 519 without), and the path for scales that 16-byte
+//   loads cannot take is a kernel of its own (VEC; with both in one, and the epilogue as it was, 116 and 88 bytes were
+//   loaded back: DeepSeek-V3, 4096 tokens, 3150 -> 2985 us without, 1024 1680 -> 1633, 16384 8913 -> 8362).  The fold warps' 104
+//   registers hold the epilogue because the activation is chosen once for a tile, not per value.
 // The gate/up kernel quantises its output: the tile's 128 channels of a token are one group, spread over four warps (M = 128:
 // eight), which exchange their largest magnitudes through shared memory.  (A bf16 activation and a quantiser pass took 135 us
 // of that case.)
@@ -689,7 +690,8 @@ struct WideGeo {
 };
 static_assert(WideGeo::bytes(1024) <= kMaxSmem, "shared memory");
 
-template <bool GATED, bool PROF, bool MOVE>
+// VEC: the scales of four K blocks are one 16-byte load
+template <bool GATED, bool PROF, bool MOVE, bool VEC>
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 1)
 grouped_gemm_pair_fold_wide_kernel(const __grid_constant__ CUtensorMap map_t, const __grid_constant__ CUtensorMap map_w,
                                    const FoldParams p) {
@@ -885,9 +887,7 @@ grouped_gemm_pair_fold_wide_kernel(const __grid_constant__ CUtensorMap map_t, co
     const int me = warp - (kFoldWarps + 2);
     int more = 0;
     auto add_units = [&](int batch) {
-      UnitPlan plan;
-      plan.init(total_tiles, kblocks, 0, workers, worker);
-      more = PairList::fill(list, list_bars, batch, plan, p.w_tiles, p.group, p.num_experts, table, 256);
+      more = PairList::fill(list, list_bars, batch, worker, workers, total_tiles, p.w_tiles, p.group, p.num_experts, table, 256);
       if (more < 0) report(0x5b0);
     };
     if (me == 0) add_units(0);
@@ -895,7 +895,6 @@ grouped_gemm_pair_fold_wide_kernel(const __grid_constant__ CUtensorMap map_t, co
     uint32_t group = 0;
     bool alive = true;
     int ltile = 0;
-    const bool vec = (kblocks & 3) == 0 && aligned16(p.a_scale) && aligned16(p.w_scale);
     const int wblocks = (int)(p.w_rows / 128);
     for (; alive; ++ltile) {
       // half a batch ahead: every reader is at most a few tiles (of the factor ring) behind, so nobody is waited for
@@ -929,7 +928,7 @@ grouped_gemm_pair_fold_wide_kernel(const __grid_constant__ CUtensorMap map_t, co
           const int kb = kb0 + 4 * q, left = kblocks - kb;
           if (left <= 0) break;
           float4 a[4], f0, f1;
-          if (vec) {
+          if constexpr (VEC) {
             f0 = __ldg(reinterpret_cast<const float4*>(sw0 + kb));
             f1 = __ldg(reinterpret_cast<const float4*>(sw1 + kb));
 #pragma unroll
@@ -1083,15 +1082,19 @@ grouped_gemm_pair_fold_wide_kernel(const __grid_constant__ CUtensorMap map_t, co
         const int ch = 64 * side + 32 * half + (small ? 16 * piece : 0);
         const int64_t at = (int64_t)(m[256] + tok) * p.n + m[258] * 128 + ch;
         float amax = 0.f;
+        auto activate = [&](auto activation) {
 #pragma unroll
-        for (int h = 0; h < 2; ++h) {
-          if (h == 1 && small) break;
+          for (int h = 0; h < 2; ++h) {
+            if (h == 1 && small) break;
 #pragma unroll
-          for (int i = 0; i < 16; ++i) {
-            acc[32 * h + i] = act_mul_fast(acc[32 * h + i] * rs, acc[32 * h + 16 + i] * rs, p.activation);
-            amax = fmaxf(amax, fabsf(acc[32 * h + i]));
+            for (int i = 0; i < 16; ++i) {
+              acc[32 * h + i] = act_mul_fast(acc[32 * h + i] * rs, acc[32 * h + 16 + i] * rs, decltype(activation)::value);
+              amax = fmaxf(amax, fabsf(acc[32 * h + i]));
+            }
           }
-        }
+        };
+        if (p.activation == FMOE_ACT_GELU) activate(std::integral_constant<int, FMOE_ACT_GELU>{});
+        else activate(std::integral_constant<int, FMOE_ACT_SILU>{});
         if (p.out_dtype == FMOE_E4M3) {
           // the tile's 128 channels are one quantisation group, held by four warps (M = 128: by eight)
           const int part = (small ? 4 * side : 0) + 2 * half + piece;
@@ -1176,11 +1179,11 @@ grouped_gemm_pair_fold_wide_kernel(const __grid_constant__ CUtensorMap map_t, co
     g_wait_prof_fp8[(GATED ? 2048 : 0) + blockIdx.x * 8 + 5] = clock64() - t_kernel0;
 }
 
-template <bool GATED, bool WIDE, bool PROF>
+template <bool GATED, bool WIDE, bool PROF, bool VEC>
 int launch(const GemmParams& g, int min_rows, int max_rows, cudaStream_t st) {
   constexpr int TILE = WIDE ? 256 : TOK;
-  auto kernel = WIDE ? grouped_gemm_pair_fold_wide_kernel<GATED, PROF, true> : grouped_gemm_pair_fold_kernel<GATED, PROF, true>;
-  auto plain = WIDE ? grouped_gemm_pair_fold_wide_kernel<GATED, PROF, false> : grouped_gemm_pair_fold_kernel<GATED, PROF, false>;
+  auto kernel = WIDE ? grouped_gemm_pair_fold_wide_kernel<GATED, PROF, true, VEC> : grouped_gemm_pair_fold_kernel<GATED, PROF, true>;
+  auto plain = WIDE ? grouped_gemm_pair_fold_wide_kernel<GATED, PROF, false, VEC> : grouped_gemm_pair_fold_kernel<GATED, PROF, false>;
   // setmaxnreg waits for good when the launch has fewer registers than the warps' shares add up to.  The compiler gives these
   // kernels the 96 per thread that 640 threads leave; one that gives fewer gets the kernels without the move
   // (DeepSeek-V3, 4096 tokens: 3.33 ms per layer with it, 3.40 without).
@@ -1277,8 +1280,15 @@ int gemm_pair_fold(const GemmParams& p, bool gated, cudaStream_t st) {
   static const bool profile = getenv("FMOE_TC_PROFILE") != nullptr;
   auto go = [&](auto wide_c, int min_rows, int max_rows) {
     constexpr bool W = decltype(wide_c)::value;
-    if (profile) return gated ? launch<true, W, true>(p, min_rows, max_rows, st) : launch<false, W, true>(p, min_rows, max_rows, st);
-    return gated ? launch<true, W, false>(p, min_rows, max_rows, st) : launch<false, W, false>(p, min_rows, max_rows, st);
+    auto with = [&](auto vec_c) {
+      constexpr bool V = decltype(vec_c)::value;
+      if (profile) return gated ? launch<true, W, true, V>(p, min_rows, max_rows, st) : launch<false, W, true, V>(p, min_rows, max_rows, st);
+      return gated ? launch<true, W, false, V>(p, min_rows, max_rows, st) : launch<false, W, false, V>(p, min_rows, max_rows, st);
+    };
+    if constexpr (W) {
+      if (p.k % 512 != 0 || !aligned16(p.a_scale) || !aligned16(p.w_scale)) return with(std::false_type{});
+    }
+    return with(std::true_type{});
   };
   constexpr int kAll = 0x7fffffff;
   // e4m3 output is the wide kernel's: a narrow tile's 128 channels are spread over both CTAs

@@ -125,7 +125,9 @@ struct PairTile {
 // Tile order: expert by expert, inside an expert in groups of at most `group` token tiles, inside a group the token tile
 // varies fastest: the tiles that run at the same time share weight rows through L2, and the group's token rows stay hot.
 // Tokens per tile: the expert's in equal tiles, or, given a fixed number, as many per tile and the rest in the last.
-__device__ __forceinline__ PairTile pair_locate(int64_t tile, int w_tiles, int group, int num_experts, const int32_t* table,
+// Int: int64_t, or int where the launch's tiles fit.
+template <typename Int>
+__device__ __forceinline__ PairTile pair_locate(Int tile, int w_tiles, int group, int num_experts, const int32_t* table,
                                                 int fixed = 0) {
   const int32_t* prefix = table + 2 * num_experts;
   const int q = (int)(tile / w_tiles);
@@ -137,8 +139,8 @@ __device__ __forceinline__ PairTile pair_locate(int64_t tile, int w_tiles, int g
   }
   const int tiles = prefix[expert + 1] - prefix[expert];
   const int rows = table[num_experts + expert];
-  const int64_t local = tile - (int64_t)prefix[expert] * w_tiles;
-  const int64_t per_group = (int64_t)group * w_tiles;
+  const Int local = tile - (Int)prefix[expert] * w_tiles;
+  const Int per_group = (Int)group * w_tiles;
   const int g = (int)(local / per_group), r = (int)(local % per_group);
   const int in_group = min(group, tiles - g * group);
   // where the last tile is a short one, the order changes from weight tile to weight tile: an even number of workers would
@@ -306,27 +308,24 @@ struct PairList {
     ++n;
     return u->tl.cols != 0;
   }
-  // A whole warp adds a batch.  1: there are more, 0: the list ends in it, -1: time-out.
-  static __device__ __forceinline__ int fill(int4* units, uint64_t* bars, int batch, const UnitPlan& plan, int w_tiles, int group,
-                                             int num_experts, const int32_t* table, int fixed = 0) {
+  // A whole warp adds a batch of whole tiles: worker, worker + workers, .. below total.  1: there are more, 0: the list ends in it,
+  // -1: time-out.
+  static __device__ __forceinline__ int fill(int4* units, uint64_t* bars, int batch, int worker, int workers, int total, int w_tiles,
+                                             int group, int num_experts, const int32_t* table, int fixed = 0) {
     const int slot = batch & 1, lane = threadIdx.x & 31;
     if (batch >= 2 && !__all_sync(0xffffffffu, ptx::mbar_wait_relaxed(&bars[2 + slot], ((batch >> 1) & 1) ^ 1))) return -1;
-    int64_t tile;
-    int ks0, ks1;
-    PairUnit u;
-    const int64_t it = (int64_t)batch * kListUnits + lane;
-    const bool any = plan.get(it, &tile, &ks0, &ks1, &u.slice);
+    const int tile = worker + (batch * kListUnits + lane) * workers;
     int4 d = make_int4(0, 0, 0, 0);
-    if (any) {
+    if (tile < total) {
+      PairUnit u;
       u.tl = pair_locate(tile, w_tiles, group, num_experts, table, fixed);
-      u.log2_s = plan.is_split(it) ? 31 - __clz(plan.S) : 0;
-      u.b = plan.b;
+      u.slice = u.log2_s = u.b = 0;
       d = u.pack();
     }
     units[slot * kListUnits + lane] = d;
     __syncwarp();
     if (lane == 0) ptx::mbar_arrive(&bars[slot]);
-    return __all_sync(0xffffffffu, any);
+    return __all_sync(0xffffffffu, tile < total);
   }
 };
 #endif

@@ -278,6 +278,20 @@ def test_variant_selection_is_shape_only():
     assert _pick_variant(torch.float8_e4m3fn, 131072, 256, 2048, 7168, None) == ("tcgen05", 128)
 
 
+@pytest.mark.parametrize("src,kernel,count", [
+    ("gemm_pair_fold.cu", r"fold_wide_kernelILb[01]ELb0ELb1ELb[01]E", 4), ("gemm_pair_fold.cu", r"fold_kernelILb[01]ELb0ELb1E", 2),
+    ("gemm_pair.cu", r"pair_kernelI", 10)])
+def test_tensor_core_kernels_keep_their_registers(lib, src, kernel, count):
+    """No kernel of the tensor-core GEMMs spills (the e4m3 ones: as they are launched, with the register move and without the
+    profile): their warps run at 64, 96 or 104 registers, and a spill is a local-memory access per K block."""
+    from flaggems_sglang_b200.build import ptxas_report
+
+    found = re.findall(r"Compiling entry function '(\S+)'.*?(\d+) bytes spill stores, (\d+) bytes spill loads",
+                       open(ptxas_report(src)).read(), flags=re.S)
+    mine = [f for f in found if re.search(kernel, f[0])]
+    assert len(mine) == count and all(f[1:] == ("0", "0") for f in mine), mine
+
+
 def test_header_compiles_as_plain_c_and_cpp(tmp_path):
     """The boundary is a C ABI: the public header must be self-contained C99 (and valid C++), and a C translation unit
     that fills both argument structs must agree with the ctypes mirrors on their sizes."""
