@@ -31,7 +31,8 @@
 namespace fmoe {
 
 __device__ int g_device_status = 0;  // 0 = fine; otherwise (role << 8 | site) of the first wait that gave up
-// Optional wait-time profile (FMOE_TC_PROFILE=1): per CTA {tiles, mma wait acc, mma wait data, producer wait, epilogue wait, epilogue busy}
+// Optional wait-time profile (FMOE_TC_PROFILE=1): per CTA {tiles, mma wait acc, mma wait data, first producer's waits, epilogue wait,
+// epilogue busy, second producer's waits}
 __device__ long long g_wait_prof[256 * 8];
 
 namespace {
@@ -309,7 +310,7 @@ grouped_gemm_pair_kernel(const __grid_constant__ CUtensorMap map_t, const __grid
         }
         mine = ks - ks1;
       }
-      if (p.profile && blockIdx.x < 256) g_wait_prof[blockIdx.x * 8 + 3] = prof_p;
+      if (p.profile && blockIdx.x < 256) g_wait_prof[blockIdx.x * 8 + 3 + 3 * me] = prof_p;
       // drain: what this warp filled has been consumed (in order) before the CTA may end
       if (alive && last_stage >= 0 && !ptx::mbar_wait(&empty_bar[last_stage], last_phase)) report(0x180 | last_stage);
     }

@@ -73,9 +73,9 @@ def main():
     tiles = lead[:, 0].sum()
     all_tiles = tiles * (sms / len(lead))
     print(f"  down GEMM: {len(lead)} CTAs issue MMAs, {tiles / len(lead):.1f} tiles each; per tile (clock cycles):")
-    print("    MMA warp waits for its accumulator %.0f, for TMA data %.0f; producer waits for a free stage %.0f; "
+    print("    MMA warp waits for its accumulator %.0f, for TMA data %.0f; the two producers wait for a free stage %.0f and %.0f; "
           "epilogue waits %.0f, busy %.0f" % (lead[:, 1].sum() / tiles, lead[:, 2].sum() / tiles, a[:, 3].sum() / all_tiles,
-                                             a[:, 4].sum() / all_tiles, a[:, 5].sum() / all_tiles))
+                                             a[:, 6].sum() / all_tiles, a[:, 4].sum() / all_tiles, a[:, 5].sum() / all_tiles))
 
 
 if __name__ == "__main__":

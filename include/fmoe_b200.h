@@ -454,8 +454,8 @@ int fmoe_debug_decode_ctas(int ctas);
 
 /*
  * Diagnostic: with the environment variable FMOE_TC_PROFILE set, the bf16 tcgen05 kernel records, per
- * CTA, clock cycles spent waiting {tiles, MMA on accumulator, MMA on data, producer on free stage,
- * epilogue on accumulator, epilogue busy, -, -}.  Copies the last launch's n values (8 per CTA, at most
+ * CTA, clock cycles spent waiting {tiles, MMA on accumulator, MMA on data, first producer on free stage,
+ * epilogue on accumulator, epilogue busy, second producer on free stage, -}.  Copies the last launch's n values (8 per CTA, at most
  * 256 CTAs) to HOST memory.  No counterpart in the reference.
  */
 int fmoe_debug_tcgen05_wait_profile(int64_t* host_out, int n);

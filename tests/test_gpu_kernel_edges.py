@@ -639,3 +639,24 @@ def test_units_by_ticket_with_a_cut_last_round(fg, kind, H, I, gated):
     outs = [fg.fused_experts(*d, tw.cuda(), ids.cuda(), **kw) for _ in range(3)]
     assert_close_moe(outs[0][idx.cuda()], ref, "fp8" if kind == "channel" else "bf16", f"tickets {kind} H={H}")
     assert all(torch.equal(o, outs[0]) for o in outs)
+
+
+def test_wait_profile_has_a_word_for_each_producer():
+    """FMOE_TC_PROFILE: both TMA warps of a CTA leave their waits, in words of their own."""
+    code = """
+import ctypes, torch
+import flaggems_sglang_b200 as fg
+from flaggems_sglang_b200 import _C
+E, H, I, T = 8, 2048, 2048, 2048
+w1, w2 = (torch.randn(E, *s, device="cuda").mul_(0.02).bfloat16() for s in ((2 * I, H), (H, I)))
+x, logits = torch.randn(T, H, device="cuda").bfloat16(), torch.randn(T, E, device="cuda")
+fg.fused_moe(x, w1, w2, logits, 2, True, variant="tcgen05")
+_C.check_device_status()
+n = _C.lib().fmoe_sm_count() // 2 * 2
+buf = (ctypes.c_int64 * (n * 8))()
+_C.check(_C.lib().fmoe_debug_wait_profile(_C.VARIANTS["tcgen05"], buf, n * 8))
+a = torch.tensor(list(buf)).view(n, 8)
+assert bool((a[:, 3] > 0).all()) and bool((a[:, 6] > 0).all()), a[:4]
+"""
+    env = dict(os.environ, FMOE_TC_PROFILE="1", PYTHONPATH=os.pathsep.join(sys.path))
+    subprocess.run([sys.executable, "-c", code], check=True, env=env, timeout=300)
