@@ -660,3 +660,69 @@ assert bool((a[:, 3] > 0).all()) and bool((a[:, 6] > 0).all()), a[:4]
 """
     env = dict(os.environ, FMOE_TC_PROFILE="1", PYTHONPATH=os.pathsep.join(sys.path))
     subprocess.run([sys.executable, "-c", code], check=True, env=env, timeout=300)
+
+
+def test_calls_in_one_workspace_whose_routing_changes(tmp_path):
+    """The CTA-pair GEMMs read the expert table and weights, and take tickets, ahead of their wait for the kernel before.  Calls of
+    one workspace follow one another without a synchronisation, each with another routing (few hot experts, other ones, all, a
+    different number of tokens), so that a table or a counter of the call before would give other rows: the bits are those of calls
+    that are waited for, with programmatic launches and with plain ones."""
+    code = """
+import sys, torch
+import flaggems_sglang_b200 as fg
+from flaggems_sglang_b200 import _C
+lib, st = _C.lib(), _C.stream_ptr()
+g = torch.Generator(device="cuda").manual_seed(1)
+rand = lambda *s: torch.randn(*s, generator=g, device="cuda")
+E, k, outs = 16, 4, []
+for kind, H, I, sizes in (("bf16", 1024, 1024, (700, 301)), ("bf16", 4096, 7168, (2048, 1500)), ("n_major", 1024, 1024, (700, 301)),
+                          ("channel", 1024, 1024, (700, 301)), ("block", 1024, 1024, (700, 301)), ("block", 1024, 512, (90, 40))):
+    w1, w2 = rand(E, 2 * I, H) * H ** -0.5, rand(E, H, I) * I ** -0.5
+    s1 = s2 = None
+    if kind in ("block", "channel"):
+        quant = fg.quant_weight_block128 if kind == "block" else fg.quant_weight_per_channel
+        (w1, s1), (w2, s2) = (tuple(torch.stack(v) for v in zip(*(quant(e) for e in w))) for w in (w1, w2))
+    else:
+        w1, w2 = w1.bfloat16(), w2.bfloat16()
+    if kind == "n_major":
+        w1, w2 = w1.transpose(1, 2).contiguous(), w2.transpose(1, 2).contiguous()
+    calls = []
+    for i in range(8):
+        T = sizes[i % 2]
+        logits = rand(T, E)
+        if i % 4 != 3:
+            logits[:, (5 * i + torch.arange(6, device="cuda")) % E] += 4.0  # six hot experts, others in each call
+        x, out = rand(T, H).bfloat16(), torch.empty(T, H, dtype=torch.bfloat16, device="cuda")
+        a = _C.FusedArgs(dtype=_C.E4M3 if s1 is not None else _C.BF16, variant=_C.VARIANTS["tcgen05"], num_experts=E, top_k=k, T=T, H=H, I=I,
+                         routed_scaling_factor=1.0, hidden=x.data_ptr(), w1=w1.data_ptr(), w2=w2.data_ptr(), w1_scale=_C.ptr(s1),
+                         w2_scale=_C.ptr(s2), out=out.data_ptr(), w_layout=_C.W_N_MAJOR if kind == "n_major" else _C.W_K_MAJOR,
+                         scale_mode=_C.SCALE_CHANNEL if kind == "channel" else _C.SCALE_BLOCK128)
+        calls.append((a, _C.RouteArgs(logits=logits.data_ptr(), grouped=0, renormalize=1, n_group=1, topk_group=1), out, (x, logits)))
+    need = max(lib.fmoe_fused_moe_workspace_bytes(a, r) for a, r, _, _ in calls)
+    ws = torch.empty(need, dtype=torch.uint8, device="cuda")
+    refs = []
+    for a, r, out, _ in calls:
+        a.workspace, a.workspace_bytes = ws.data_ptr(), need
+        _C.check(lib.fmoe_fused_moe(a, r, st))
+        torch.cuda.synchronize()
+        refs.append(out.clone())
+        assert float(refs[-1].float().abs().sum()) > 0
+    for _ in range(12):
+        for _, _, out, _ in calls:
+            out.fill_(float("nan"))
+        torch.cuda._sleep(2000000)  # the calls queue up behind it
+        for a, r, _, _ in calls:
+            _C.check(lib.fmoe_fused_moe(a, r, st))
+        torch.cuda.synchronize()
+        assert all(torch.equal(out, ref) for (_, _, out, _), ref in zip(calls, refs)), (kind, H, I)
+    outs += [r.cpu() for r in refs]
+fg._C.check_device_status()
+torch.save(outs, sys.argv[1])
+"""
+    outs = []
+    for pdl in ("1", "0"):
+        path = str(tmp_path / f"out{pdl}.pt")
+        env = dict(os.environ, FMOE_PDL=pdl, PYTHONPATH=os.pathsep.join(sys.path))
+        subprocess.run([sys.executable, "-c", code, path], check=True, env=env, timeout=300)
+        outs.append(torch.load(path))
+    assert all(torch.equal(a, b) for a, b in zip(*outs))
