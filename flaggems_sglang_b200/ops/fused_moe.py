@@ -658,7 +658,7 @@ class StandardCombineInput:
 
 
 _SGLANG_RETRY_S = 0.2
-_sglang_missing = False  # or, after a failed import: the import path it searched and when to search again
+_sglang_missing = False  # or, after a failed import: when to search again, and the import path and finders that were searched
 
 
 def _standard_output_type():
@@ -668,16 +668,16 @@ def _standard_output_type():
     repeated only when something has loaded sglang, when the path or its finders are others, or after 0.2 s (files may have
     come, or a finder learnt of them)."""
     global _sglang_missing
-    path = (*sys.path, *sys.meta_path)
-    missing = _sglang_missing
-    if missing and "sglang" not in sys.modules and missing[0] == path and time.monotonic() < missing[1]:
-        return StandardCombineInput
+    if _sglang_missing:
+        until, path, finders = _sglang_missing
+        if "sglang" not in sys.modules and time.monotonic() < until and sys.path == path and sys.meta_path == finders:
+            return StandardCombineInput
     try:
         from sglang.srt.layers.moe.token_dispatcher.standard import StandardCombineInput as _Sgl
 
         return _Sgl
     except Exception:  # noqa: BLE001
-        _sglang_missing = path, time.monotonic() + _SGLANG_RETRY_S
+        _sglang_missing = time.monotonic() + _SGLANG_RETRY_S, list(sys.path), list(sys.meta_path)
         return StandardCombineInput
 
 
