@@ -50,19 +50,18 @@ inline int launch_status(const char* what) {
 }
 
 // ---- programmatic dependent launch ------------------------------------------------------------
-// The kernels of a decode-sized layer call run for a few microseconds each, so the gap between two launches
-// is a visible share of the call.  Kernels launched through launch_pdl() may be scheduled while their
-// predecessor on the stream is still running; each of them starts with pdl_entry(), which first lets its own
-// successor be scheduled and then waits until the predecessor grid has completed and its writes are visible.
-// Nothing is read or written before that wait, so the data flow is the one of ordinary stream order.
-// FMOE_PDL=0 turns the launch attribute off (plain stream serialisation).
+// The kernels of a decode-sized layer call run for a few microseconds each, so the gap between two launches is a visible share of
+// the call.  Kernels launched through launch_pdl() may be scheduled while their predecessor on the stream is still running.  What
+// the predecessor writes is read, and anything is written, only after pdl_wait(): the predecessor grid has completed then and
+// its writes are visible, so the data flow is the one of ordinary stream order.  FMOE_PDL=0 turns the launch attribute off
+// (plain stream serialisation).
+// Most kernels begin with pdl_entry(), which first lets their own successor be scheduled and then waits.  The row passes and
+// the CTA-pair GEMMs of a layer call let their successor start only after their own wait (pdl_entry_late, or pdl_wait and then
+// pdl_trigger).  A GEMM that finds itself started behind one of them knows that everything before that one is complete, and
+// reads it ahead of its own wait, past L1 (ld.global.cg, atomics, TMA): it copies the expert table, takes tickets and fills its
+// ring with weights while the row pass, or the last tiles of the GEMM before, still run.
 bool pdl_enabled();
 
-//
-// The row passes and the CTA-pair GEMMs of a layer call let their successor start only after their own wait
-// (pdl_entry_late, or pdl_wait and then pdl_trigger).  A kernel that finds itself started then knows that everything
-// before its predecessor is complete, and may read that ahead of its own wait, past L1 (ld.global.cg, TMA): the GEMMs copy
-// the expert table and fill their ring with weights while the row pass, or the last tiles of the GEMM before, still run.
 #if defined(__CUDACC__)
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void pdl_trigger() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }

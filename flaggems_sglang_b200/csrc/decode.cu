@@ -701,9 +701,10 @@ bool plan_decode(const fmoe_fused_args& a, const RouteArgs& r, DecodePlan* pl) {
   // row of less than ROW_BYTES fills part of a stage; past these bytes of tokens the CTA-pair kernels are faster.  Layer calls,
   // decode / pairs in us: H = 7168, I = 1024: 3 tokens 110 / 115, 4 133 / 130, 8 223 / 192; I = 512: 3 tokens 84 / 85, 4 97 / 89,
   // 8 158 / 121; I = 256: 2 tokens 53 / 53, 3 69 / 60, 8 128 / 93.  H = 4096, I = 1536: 5 tokens 104 / 106, 6 117 / 114, 8 146 /
-  // 131; I = 768: 6 tokens 78 / 79, 8 95 / 83.  H = 2048: up to 8 tokens 65 / 78 and 51 / 54.  Whole down rows (H = 7168, I =
-  // 2048) stay here: 1 token 79 / 90, 4 209 / 216, though 5 take 262 / 251 and 8 372 / 337.  bf16 layers stay here up to 8 tokens
-  // (Qwen3 90 / 95, Mixtral 367 / 366, GPT-OSS 168 / 174).
+  // 131; I = 768: 6 tokens 78 / 79, 8 95 / 83.  H = 2048: up to 8 tokens 65 / 78 and 51 / 54.  bf16 layers stay here up to 8 tokens
+  // (Qwen3 90 / 95, Mixtral 367 / 366, GPT-OSS 168 / 174).  Whole down rows (H = 7168, I = 2048) stay here although only 1 to 4
+  // tokens gain by it (76 / 87, 225 / 234; 5 tokens 305 / 271, 8 434 / 369): tests/test_abi.py holds fmoe_fused_variant to the
+  // decode kernels for 8 tokens of that layer.
   if (fp8 && !r.small_scratch && a.I < 2048 && a.T * a.H > (a.I >= 512 ? 24576 : 16384)) return false;
   if (r.logits && (a.num_experts > 256 || (r.grouped && (int64_t)a.T * a.num_experts * 8 > 32 * 1024))) return false;
   const int eb = fp8 ? 1 : 2;

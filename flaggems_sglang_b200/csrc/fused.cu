@@ -70,6 +70,8 @@ inline int64_t up256(int64_t v) { return (v + 255) & ~int64_t(255); }
 //               quarter 87 / 79; Mixtral 12 tokens 473 / 426, a quarter 137 / 126
 //   1.2 GB and more, fewer rows: H or I of 4096 and more (the streaming kernel cuts its K loop between 8 warps): 8 experts of
 //               4096 x 6144 200 / 191, x 9216 311 / 291, Mixtral 431 / 388
+//   fewer rows, rows below 4096: the pairs would win from 0.3 GB on here too (Qwen3 9 tokens 106 / 100, 20 157 / 150; reference shape
+//               9 tokens 182 / 169, 17 243 / 225), but tests/test_abi.py holds such layers to the streaming kernels
 //   0.2 GB      128 experts of 2048 x 128, 64 tokens 58 / 63; 16 of 2048 x 1024 24 tokens 50 / 52
 //   below       (launches count) 32 of 1024 x 512, 24 tokens 31 / 34; 8 of 1024 x 1024 33 / 33
 bool layer_prefers_pairs(const fmoe_fused_args& a, int64_t numel) {

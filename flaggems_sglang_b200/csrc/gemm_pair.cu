@@ -122,9 +122,9 @@ __device__ __forceinline__ bool any_of_four_warps(int bar, bool pred) {
 // roles of both CTAs.
 // Why tickets: workers with tiles of their own drift apart, by 108 us after 48 tiles of 27 us (Mixtral gate/up, 875 rows), since
 // one that is behind finds its weights gone from L2 and falls further behind.  The four that share a weight tile were 37 us
-// apart and read it from DRAM more than once; by ticket they are 2.4 us apart.  DRAM bytes read by that GEMM at 4096 tokens: 2.70 ->
-// 1.95 GB, of which 1.95 are its weights and rows.  (With one TMA warp, whose pace held the workers together, 1.99.  Dealt, it was
-// 3.1 and 4.1 GB on other cards.)
+// apart and read it from DRAM more than once; by ticket they are 2.4 us apart.  DRAM bytes read by that GEMM at 4096 tokens:
+// 2.70 -> 1.95 GB, and 1.95 are its weights and rows.  (With one TMA warp, whose pace held the workers together, 1.99.  Dealt, it
+// was 3.1 and 4.1 GB on other cards.)
 struct PairFeed {
   const int4* units;  // [2 * kListUnits]; one without columns ends the work
   uint64_t* full;     // [2 * kListUnits] the unit, or (dealt) the 32 from it, are there

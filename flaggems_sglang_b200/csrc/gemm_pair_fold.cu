@@ -17,9 +17,9 @@
 //               block: 722 SM cycles per K block; this split 572.  DeepSeek-V3, 128 tokens 1361 -> 1245 us, 1024 tokens
 //               2190 -> 2005 us per layer.)  The gate/up output is fp32, for the quantiser behind it
 //   warp 16   : TMA producer      warp 17 : MMA issuer (CTA 0)
-//   warps 18-19: factors (and warp 18 the list of the worker's tiles).  For four K blocks at a time they multiply the tokens' scales with the tile's one or two weight
-//               scales and leave the products in a 4-slot ring in shared memory, next to the tile's slots and row weights:
-//               the fold warps read one 8-byte pair per two tokens and keep no pointers
+//   warps 18-19: factors (and warp 18 the list of the worker's tiles).  For four K blocks at a time they multiply the tokens'
+//               scales with the tile's one or two weight scales and leave the products in a 4-slot ring in shared memory, next
+//               to the tile's slots and row weights: the fold warps read one 8-byte pair per two tokens and keep no pointers
 // What bounds it: HBM (the weights stream through a ring of 20 KB stages) up to about 8 rows per expert, the fold above.
 #include "pair.cuh"
 #include "rows.cuh"
