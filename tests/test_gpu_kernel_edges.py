@@ -129,19 +129,24 @@ def test_wide_e4m3_kernel_stores_to_rows_at_16_bytes(fg, gated):
     assert torch.equal(outs[0], outs[1]) and torch.equal(outs[0], outs[2])
 
 
-@pytest.mark.parametrize("H,I", [(128, 256), (256, 128)])
-def test_wide_e4m3_kernel_mixes_tile_heights(fg, H, I):
-    """Block-scale layers whose experts end in tiles of M = 128 and of M = 256, one and two K blocks long: the warps that share a
+# then 73 tiles a worker in the gate/up GEMM or in the down GEMM: every ring and list wraps round, both kinds of tile in turn
+@pytest.mark.parametrize("H,I,per_worker", [(128, 256, 1), (256, 128, 1), (128, 12800, 64), (25600, 128, 64), (384, 6528, 32)])
+def test_wide_e4m3_kernel_mixes_tile_heights(fg, H, I, per_worker):
+    """Block-scale layers whose experts end in tiles of M = 128 and of M = 256, one to three K blocks long: the warps that share a
     quantisation group change from tile to tile, and a tile is over before the slowest warp has left the one before."""
     rows = [300, 65, 129, 256, 400, 128, 257, 640, 70, 512, 0, 384] * 3
     E, T = len(rows), sum(rows)
+    workers, tiles = fg._C.lib().fmoe_sm_count() // 2, sum(-(-r // 256) for r in rows) * max(I // 128, H // 256)
+    if per_worker > 1:
+        assert tiles > per_worker * workers
     x, w1, w2, g = _layer(T, H, I, E, 11)
     ids = torch.repeat_interleave(torch.arange(E), torch.tensor(rows))[torch.randperm(T, generator=g)].to(torch.int32).view(T, 1)
     tw = torch.rand(T, 1, generator=g) + 0.5
     (w1q, w1s), (w2q, w2s) = OQ.quant_weight_block128(w1), OQ.quant_weight_block128(w2)
-    out = fg.fused_experts(x.cuda(), w1q.cuda(), w2q.cuda(), tw.cuda(), ids.cuda(), use_fp8_w8a8=True, w1_scale=w1s.cuda(),
-                           w2_scale=w2s.cuda(), block_shape=[128, 128])
-    assert_close_moe(out, OE.fused_experts_fp8(x, w1q, w1s, w2q, w2s, tw, ids), "fp8", f"H={H} I={I}")
+    d = [v.cuda() for v in (x, w1q, w2q, tw, ids, w1s, w2s)]
+    outs = [fg.fused_experts(*d[:5], use_fp8_w8a8=True, w1_scale=d[5], w2_scale=d[6], block_shape=[128, 128]) for _ in range(3)]
+    assert_close_moe(outs[0], OE.fused_experts_fp8(x, w1q, w1s, w2q, w2s, tw, ids), "fp8", f"H={H} I={I}")
+    assert all(torch.equal(o, outs[0]) for o in outs)
 
 
 def test_e4m3_kernels_without_the_register_move(tmp_path):
