@@ -336,6 +336,7 @@ int run_fused(const fmoe_fused_args& args, const RouteArgs& route, const FusedPl
     g.split_ws_bytes = p.split_bytes;
   }
   g.expert_table = table;
+  g.behind_late_trigger = tc;  // below, a row pass or another pair GEMM stands before each of them
   g.token_tile = al.token_tile;
   g.skip_padding = true;  // nothing below reads a padding row's values
   GemmParams g1 = g, g2 = g;

@@ -14,6 +14,8 @@ enum class FoldKernel { kBoth, kNarrow, kWide };
 // Arguments of one grouped GEMM: the public ones, and what only the one-call layer hands over (fused.cu).
 struct GemmParams : fmoe_gemm_args {
   const int32_t* expert_table = nullptr;  // pair_table_words(E) words written by moe_align (see pair.cuh); NULL: derived
+  bool behind_late_trigger = false;       // the launch before lets this one start only after its own wait (pdl_entry_late): the
+                                          // table is complete then, and is read ahead of this kernel's wait
   int token_tile = 0;                     // the tile width that table was made for; 0: chosen by the launcher
   int32_t* split_counters = nullptr;      // zeroed arrival counters of the tail split; NULL: cleared by the launcher
   FoldKernel fold = FoldKernel::kBoth;

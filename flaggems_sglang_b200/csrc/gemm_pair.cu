@@ -67,6 +67,7 @@ struct PairParams {
   const int32_t* expert_ids;
   const int32_t* num_tokens_post_padded;
   const int32_t* expert_table;  // written by moe_align (NULL: derived from the block tables)
+  bool early;                   // it is complete when the kernel starts
   const float* row_scale;
   const float* a_scale;   // F8: one scale per row of the sorted order, or per token (a_scale_gather)
   const float* w_scale;   // F8: [E, w_rows], one scale per output channel
@@ -208,11 +209,11 @@ grouped_gemm_pair_kernel(const __grid_constant__ CUtensorMap map_t, const __grid
     ptx::tmem_relinquish_pair();
   }
   ptx::tc_fence_before_sync();
-  // Everything above is independent of the kernels before this one on the stream.  A given table is complete by now (see
-  // pdl_entry_late): only the rows and what the epilogue reads and writes have to wait for the kernel before.
-  const bool early = p.expert_table != nullptr;
+  // Everything above is independent of the kernels before this one on the stream.  Behind a late trigger a given table is
+  // complete by now (see pdl_entry_late): only the rows and what the epilogue reads and writes wait for the kernel before.
+  const bool early = p.early;
   if (!early) pdl_wait();
-  const int used_blocks = early ? 0 : min((int)(*p.num_tokens_post_padded / 128), p.max_blocks);
+  const int used_blocks = p.expert_table ? 0 : min((int)(*p.num_tokens_post_padded / 128), p.max_blocks);
   pair_build_table(table, p.num_experts, p.expert_table, p.expert_ids, p.sorted_token_ids, p.numel, 128,
                    p.token_tile, used_blocks);
   ptx::cluster_sync_all();  // the other CTA's barriers exist before anything is signalled across
@@ -812,6 +813,7 @@ int launch(const GemmParams& g, cudaStream_t st) {
   p.expert_ids = g.expert_ids;
   p.num_tokens_post_padded = g.num_tokens_post_padded;
   p.expert_table = g.expert_table;
+  p.early = g.expert_table && g.behind_late_trigger;
   p.row_scale = g.row_scale;
   p.a_scale = g.a_scale;
   p.a_scale_gather = g.a_scale_gather;

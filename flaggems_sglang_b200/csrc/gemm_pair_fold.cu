@@ -96,6 +96,7 @@ struct FoldParams {
   float* out_scale;   // [rows, n / 128]
   int32_t min_rows, max_rows;  // experts of this launch
   bool stores_of_32;           // rows of the output start at multiples of 32 bytes
+  bool early;                  // the table is complete when the kernel starts
   bool by_expert;              // narrow, fp32 gate/up output: kNarrowRows rows per expert instead of one per position
 };
 
@@ -217,10 +218,10 @@ grouped_gemm_pair_fold_kernel(const __grid_constant__ CUtensorMap map_t, const _
     ptx::tmem_relinquish_pair();
   }
   ptx::tc_fence_before_sync();
-  // a given table is complete by now (see pdl_entry_late): only rows, scales and outputs wait for the kernel before
-  const bool early = p.expert_table != nullptr;
+  // behind a late trigger a given table is complete by now (see pdl_entry_late): only rows, scales and outputs wait
+  const bool early = p.early;
   if (!early) pdl_wait();
-  const int used_blocks = early ? 0 : min((int)(*p.num_tokens_post_padded / 128), p.max_blocks);
+  const int used_blocks = p.expert_table ? 0 : min((int)(*p.num_tokens_post_padded / 128), p.max_blocks);
   pair_build_table(table, p.num_experts, p.expert_table, p.expert_ids, p.sorted_token_ids, p.numel, 128, TOK,
                    used_blocks, p.min_rows, p.max_rows);
   ptx::cluster_sync_all();
@@ -747,9 +748,9 @@ grouped_gemm_pair_fold_wide_kernel(const __grid_constant__ CUtensorMap map_t, co
     ptx::tmem_relinquish_pair();
   }
   ptx::tc_fence_before_sync();
-  const bool early = p.expert_table != nullptr;
+  const bool early = p.early;
   if (!early) pdl_wait();
-  const int used_blocks = early ? 0 : min((int)(*p.num_tokens_post_padded / 128), p.max_blocks);
+  const int used_blocks = p.expert_table ? 0 : min((int)(*p.num_tokens_post_padded / 128), p.max_blocks);
   pair_build_table(table, p.num_experts, p.expert_table, p.expert_ids, p.sorted_token_ids, p.numel, 128, 256, used_blocks,
                    p.min_rows, p.max_rows);
   ptx::cluster_sync_all();
@@ -1212,6 +1213,7 @@ int launch(const GemmParams& g, int min_rows, int max_rows, cudaStream_t st) {
   p.expert_ids = g.expert_ids;
   p.num_tokens_post_padded = g.num_tokens_post_padded;
   p.expert_table = g.expert_table;
+  p.early = g.expert_table && g.behind_late_trigger;
   p.row_scale = g.row_scale;
   p.a_scale = g.a_scale;
   p.w_scale = g.w_scale;
