@@ -690,6 +690,34 @@ int status_word_decode(int* out, bool clear) {
   return FMOE_OK;
 }
 
+namespace {
+
+// e4m3 layers of up to 8 tokens that the CTA-pair kernels run faster.  They need a list, a row copy, a quantiser and a combine pass
+// more, some 15 us, and nearly the same time whatever the tokens.  The decode kernels pay for token rows: long ones leave the ring
+// few stages, every token column has scale products of its own, a down row of less than ROW_BYTES fills part of a stage, and every
+// active expert costs 1-3 us of waits.  With cold weights, decode / pairs in us:
+//   k = 8, E = 256 (token rows decide): H = 7168, I = 1024: 3 tokens 110 / 115, 4 135 / 135, 8 263 / 226; I = 512: 2 61 / 56, 4 101 /
+//               82, 8 181 / 136; I = 256: 2 53 / 46, 4 81 / 60; H = 4096, I = 1536: 4 109 / 115, 8 210 / 189
+//   few slots   (launches and prologues count): H = 7168, I = 256: E = 8, k = 2, 3 tokens 30 / 36, 4 33 / 37, 5 37 / 37, 8 41 / 38; E = 16,
+//               k = 1, 3 tokens 23 / 35, 8 36 / 37; I = 128: E = 8, k = 2, 5 tokens 31 / 36, 8 36 / 36; E = 32, k = 4, 3 tokens 41 / 38;
+//               I = 1024: E = 16, k = 1, 5 tokens 41 / 41, 6 46 / 43; I = 1792: 8 tokens 61 / 65
+//               H = 4096, I = 256: E = 8, k = 2, 8 tokens 29 / 31; E = 16, k = 2, 6 tokens 30 / 31, 8 32 / 31; E = 32, k = 4, 5 tokens 38 / 33
+// Of 741 calls past the first line (H of 4096 to 7168, I of 128 to 1792, k of 1 to 8), 252 took 2 to 69 % longer on the pairs.  By
+// the lines below 21 still do, 2 to 8 %, and 17 take 2 to 7 % longer on the decode kernels.
+// Whole down rows (H = 7168, I = 2048) stay with the decode kernels although only 1 to 4 tokens gain by it (76 / 87, 225 / 234; 5
+// tokens 305 / 271, 8 434 / 369): tests/test_abi.py holds fmoe_fused_variant to them for 8 tokens of that layer.  bf16 layers
+// stay too (Qwen3 90 / 95, Mixtral 367 / 366, GPT-OSS 168 / 174 with 8 tokens).
+bool pairs_are_faster(const fmoe_fused_args& a) {
+  if (a.I >= 2048 || a.T * a.H <= (a.I >= 512 ? 24576 : 16384)) return false;
+  // channels of the token rows and of the slots' rows; from I = 1536 on the pairs' tiles need a second round
+  const int64_t rows = a.T * (a.top_k + 1) * a.H;
+  if (rows <= (a.I >= 1536 ? 112 : (a.I > 512 ? 76 : 88)) * 1024) return false;
+  const int64_t weights = std::min<int64_t>(a.num_experts, a.T * a.top_k) * 3 * a.H * a.I;
+  return weights > 28000000 || rows > 128 * 1024;
+}
+
+}  // namespace
+
 bool plan_decode(const fmoe_fused_args& a, const RouteArgs& r, DecodePlan* pl) {
   const bool fp8 = a.dtype == FMOE_E4M3;
   if (a.variant != FMOE_VARIANT_AUTO || (a.w_layout != FMOE_W_K_MAJOR && a.w_layout != FMOE_W_INTERLEAVED) || a.out_rows) return false;
@@ -697,15 +725,7 @@ bool plan_decode(const fmoe_fused_args& a, const RouteArgs& r, DecodePlan* pl) {
   if (a.no_combine && a.zero_dropped) return false;
   if (a.T < 1 || a.T > kDecodeTokens || a.top_k > 32 || a.num_experts > 1024) return false;
   if (a.H % (fp8 ? 128 : 64) || a.I % (fp8 ? 128 : 64)) return false;  // rows of whole 128-byte pieces
-  // e4m3, I below 2048: long token rows leave the ring few stages, every token column has scale products of its own, and a down
-  // row of less than ROW_BYTES fills part of a stage; past these bytes of tokens the CTA-pair kernels are faster.  Layer calls,
-  // decode / pairs in us: H = 7168, I = 1024: 3 tokens 110 / 115, 4 133 / 130, 8 223 / 192; I = 512: 3 tokens 84 / 85, 4 97 / 89,
-  // 8 158 / 121; I = 256: 2 tokens 53 / 53, 3 69 / 60, 8 128 / 93.  H = 4096, I = 1536: 5 tokens 104 / 106, 6 117 / 114, 8 146 /
-  // 131; I = 768: 6 tokens 78 / 79, 8 95 / 83.  H = 2048: up to 8 tokens 65 / 78 and 51 / 54.  bf16 layers stay here up to 8 tokens
-  // (Qwen3 90 / 95, Mixtral 367 / 366, GPT-OSS 168 / 174).  Whole down rows (H = 7168, I = 2048) stay here although only 1 to 4
-  // tokens gain by it (76 / 87, 225 / 234; 5 tokens 305 / 271, 8 434 / 369): tests/test_abi.py holds fmoe_fused_variant to the
-  // decode kernels for 8 tokens of that layer.
-  if (fp8 && !r.small_scratch && a.I < 2048 && a.T * a.H > (a.I >= 512 ? 24576 : 16384)) return false;
+  if (fp8 && !r.small_scratch && pairs_are_faster(a)) return false;
   if (r.logits && (a.num_experts > 256 || (r.grouped && (int64_t)a.T * a.num_experts * 8 > 32 * 1024))) return false;
   const int eb = fp8 ? 1 : 2;
   // token rows of the gate/up GEMM; rows of one block (at most T) of the down GEMM

@@ -95,6 +95,17 @@ def test_layer_variant_on_both_sides_of_its_lines(lib, dtype, T, E, H, I, k, wan
     test_layer_variant_is_what_the_one_call_layer_takes(lib, dtype, T, E, H, I, k, want)
 
 
+@pytest.mark.parametrize("T,E,H,I,k,want", [
+    (4, 8, 7168, 256, 2, "decode"), (5, 8, 7168, 256, 2, "tcgen05"),                                            # channels of the rows
+    (5, 16, 7168, 1024, 1, "decode"), (6, 16, 7168, 1024, 1, "tcgen05"), (8, 16, 7168, 1792, 1, "decode"), (6, 8, 5120, 1792, 2, "decode"),
+    (7, 8, 5120, 1536, 2, "decode"), (8, 8, 5120, 1536, 2, "tcgen05"),
+    (6, 8, 7168, 128, 2, "decode"), (7, 8, 7168, 128, 2, "tcgen05"), (8, 16, 4096, 128, 2, "decode"),           # bytes of the weights
+    (5, 32, 4096, 128, 4, "tcgen05"), (5, 64, 4096, 128, 4, "tcgen05"), (8, 8, 4096, 256, 2, "decode")])
+def test_small_e4m3_layers_keep_the_decode_kernels(lib, T, E, H, I, k, want):
+    """Few slots or few bytes of weights: the CTA-pair kernels' launches and prologues would be most of the call."""
+    test_layer_variant_is_what_the_one_call_layer_takes(lib, "E4M3", T, E, H, I, k, want)
+
+
 @pytest.mark.parametrize("dtype,T,E,H,I,k,small", [
     ("E4M3", 3, 256, 7168, 256, 8, "decode"), ("E4M3", 64, 256, 7168, 2048, 8, "stream"), ("BF16", 48, 128, 2048, 384, 8, "stream"),
     ("BF16", 300, 128, 2048, 384, 8, "stream")])
