@@ -358,7 +358,7 @@ def measure_point(cfg, wts, T, steps, warmup, peaks, seed=0, skew=False):
 # DRAM traffic of the gate/up GEMM per launch (dram__bytes_read.sum + dram__bytes_write.sum of one ncu capture; the
 # summaries with the full commands are under profiles/).  Keyed by (config, T).
 MEASURED_TRAFFIC = {
-    ("mixtral", 4096): (2.27e9, "profiles/grouped_gemm_pair_b200.md, full-size capture of the same launch"),
+    ("mixtral", 4096): (2.18e9, "profiles/grouped_gemm_pair_b200.md, full-size capture of the same launch"),
 }
 
 

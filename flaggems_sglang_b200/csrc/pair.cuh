@@ -15,8 +15,8 @@ namespace fmoe {
 // weights (what a launch needs whose time is the reading of weights); a wide one reads the weights from L2 less often.
 // Experts well above the average are cut into several tiles either way.  bf16, layers with tiles of 128 / 256 in us, uniform
 // routing: Mixtral rank, 83 rows 265 / 272, 115 rows 262 / 280, 130 rows 315 / 293; Qwen3 116 rows 263 / 269, 128 rows 304 / 287;
-// with Zipf-1.2 routing: GPT-OSS 112 rows 372 / 346, Qwen3 94 rows 243 / 229.  The line of 88 costs uniform routing up to 5 % for
-// some 30 rows and saves skewed routing 4-10 %.  e4m3 multiplies a weight byte in half the time,
+// with Zipf-1.2 routing: GPT-OSS 112 rows 372 / 346, Qwen3 94 rows 243 / 229.  The line of 88 costs uniform routing 2 to 7 % up to
+// some 120 rows and saves skewed routing 6 to 7 %.  e4m3 multiplies a weight byte in half the time,
 // so that the second reading is what counts (DeepSeek-V3, 64 rows on average: 128 tokens 2108 us, 256 tokens 1939 us).
 inline int pick_token_tile(int64_t numel, int num_experts, bool e4m3) {
   const double rows = (double)numel / (double)(numel < num_experts ? (numel > 0 ? numel : 1) : num_experts);
