@@ -439,7 +439,7 @@ int run_fused(const fmoe_fused_args& args, const RouteArgs& route, const FusedPl
   return rc;
 }
 
-int plan_within(const fmoe_fused_args& a, const RouteArgs& route, int64_t limit, FusedPlan* plan) {
+int plan_within(const fmoe_fused_args& a, const RouteArgs& route, int64_t limit, bool any_rows, FusedPlan* plan) {
   const int rc = plan_fused(a, route, plan);
   if (rc || plan->total <= limit || a.variant != FMOE_VARIANT_AUTO) return rc;
   RouteArgs small = route;
@@ -449,6 +449,10 @@ int plan_within(const fmoe_fused_args& a, const RouteArgs& route, int64_t limit,
     *plan = other;
     return FMOE_OK;
   }
+  int variant = 0, block = 0;
+  if (pick_variant(a.dtype, a.T * a.top_k, a.num_experts, a.I, a.H, FMOE_VARIANT_AUTO, &variant, &block) != FMOE_OK ||
+      (variant != FMOE_VARIANT_STREAM && !any_rows))
+    return FMOE_OK;
   fmoe_fused_args stream = a;
   stream.variant = FMOE_VARIANT_STREAM;
   if (plan_fused(stream, route, &other) == FMOE_OK && other.total <= limit) *plan = other;
@@ -457,7 +461,7 @@ int plan_within(const fmoe_fused_args& a, const RouteArgs& route, int64_t limit,
 
 int run_with_workspace(const fmoe_fused_args& args, const RouteArgs& route, void* stream) {
   FusedPlan p;
-  int rc = plan_within(args, route, args.workspace_bytes, &p);
+  int rc = plan_within(args, route, args.workspace_bytes, false, &p);
   if (rc) return rc;
   if (args.T == 0) return FMOE_OK;
   FMOE_REQUIRE(args.workspace && (reinterpret_cast<uintptr_t>(args.workspace) & 255u) == 0,

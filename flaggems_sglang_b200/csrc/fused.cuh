@@ -21,8 +21,10 @@ struct FusedPlan {
 int pick_variant(int dtype, int64_t numel, int E, int64_t I, int64_t H, int forced, int* variant, int* block);
 int plan_fused(const fmoe_fused_args& a, const RouteArgs& route, FusedPlan* plan);
 // plan_fused for scratch of `limit` bytes: where the fastest family's plan is larger, that of the decode or the streaming kernels
-// (no padded copies) if it fits.  When none does, the plan is the first one, and its total is above the limit.
-int plan_within(const fmoe_fused_args& a, const RouteArgs& route, int64_t limit, FusedPlan* plan);
+// (no padded copies) if it fits.  The streaming ones only for calls of few rows per expert (pick_variant), or for `any_rows`: with
+// many they would take many times as long, and a caller whose workspace is a little short is told so instead.  When none fits,
+// the plan is the first one, and its total is above the limit.
+int plan_within(const fmoe_fused_args& a, const RouteArgs& route, int64_t limit, bool any_rows, FusedPlan* plan);
 // Enqueues the whole computation using `ws` (at least plan.total bytes, 256-byte aligned) as scratch.
 int run_fused(const fmoe_fused_args& a, const RouteArgs& route, const FusedPlan& plan, uint8_t* ws, void* stream);
 

@@ -50,7 +50,7 @@ extern "C" int fmoe_fused_experts_static(const fmoe_fused_args* args, void* stre
   using namespace fmoe;
   if (!args) return fail(FMOE_ERR_INVALID_ARG, "fused_experts_static: args is null");
   FusedPlan plan;
-  int rc = plan_within(*args, RouteArgs{}, kStaticScratchBytes, &plan);
+  int rc = plan_within(*args, RouteArgs{}, kStaticScratchBytes, true, &plan);
   if (rc) return rc;
   if (plan.total > kStaticScratchBytes)
     return fail(FMOE_ERR_UNSUPPORTED,

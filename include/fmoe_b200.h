@@ -248,8 +248,8 @@ int fmoe_moe_sum_add(const void* z, int dtype, int64_t T, int k, int64_t H, floa
  * (`triton_kernel_fused_experts` body) and, with b1/b2 and FMOE_ACT_SWIGLU_OAI, :235-325
  * (`triton_kernel_fused_experts_with_bias`) on the serving-side layouts w1 [E,2I,H], w2 [E,H,I].
  * All intermediates live in the caller's `workspace` (size from fmoe_fused_experts_workspace_bytes: what the fastest
- * kernels for the shape need; with less, an AUTO call takes the decode or the streaming kernels where those have room, and is
- * refused otherwise); nothing is allocated and the host is never synchronised.
+ * kernels for the shape need; with less, an AUTO call of up to 8 tokens or of few rows per expert takes the decode or the
+ * streaming kernels where those have room, and other calls are refused); nothing is allocated and the host is never synchronised.
  */
 typedef struct fmoe_fused_args {
   uint32_t struct_size; /* sizeof(fmoe_fused_args) as the caller compiled it (checked like fmoe_gemm_args.struct_size) */

@@ -108,10 +108,11 @@ def test_small_e4m3_layers_keep_the_decode_kernels(lib, T, E, H, I, k, want):
 
 @pytest.mark.parametrize("dtype,T,E,H,I,k,small", [
     ("E4M3", 3, 256, 7168, 256, 8, "decode"), ("E4M3", 64, 256, 7168, 2048, 8, "stream"), ("BF16", 48, 128, 2048, 384, 8, "stream"),
-    ("BF16", 300, 128, 2048, 384, 8, "stream")])
+    ("BF16", 300, 128, 2048, 384, 8, None), ("E4M3", 4096, 256, 7168, 2048, 8, None), ("BF16", 65, 128, 2048, 384, 8, None)])
 def test_workspace_of_the_smaller_kernels_is_taken(lib, dtype, T, E, H, I, k, small):
     """A caller that brings less than the fastest kernels need keeps the ones that need less, down to what those need (found here
-    by halving; without pointers a call whose workspace is large enough ends at the check of its pointers)."""
+    by halving; without pointers a call whose workspace is large enough ends at the check of its pointers).  With many rows per
+    expert the streaming kernels would take many times as long: a workspace that is a byte short is refused."""
     from flaggems_sglang_b200 import _C
 
     a = _C.FusedArgs(dtype=getattr(_C, dtype), num_experts=E, top_k=k, T=T, H=H, I=I, workspace=256)
@@ -124,6 +125,9 @@ def test_workspace_of_the_smaller_kernels_is_taken(lib, dtype, T, E, H, I, k, sm
         assert (b"too small" in msg) != (b"null pointer" in msg), msg
         return b"null pointer" in msg
 
+    if small is None:
+        assert taken(need) and not taken(need - 1)
+        return
     lo, hi = 0, need
     assert taken(hi) and not taken(lo)
     while hi - lo > 1:
